@@ -15,7 +15,7 @@
 //    costs a 32-lane register write per weight, more than the FMA they feed; instead the weights of the (up to
 //    four) channels being processed are staged in __constant__ memory, where an FMA reads them as an operand.
 //
-//   forward     : logits -> A (raw logits are parked in A, then normalised in a second walk by the same thread)
+//   forward     : logits -> A (a first kernel parks the raw logits in A, a second one normalises them in place)
 //   logit grads : gL = A * (gA - sum_d gA*A), in place over gA; per-block sums of gL for the bias gradient
 //   input grads : gX = transposed stencil of gL (+ an optional addend: the direct gradient of the max/avg channels)
 //   weight grads: gW[k,c,tap] = sum X(shifted by tap) * gL, per-block partial sums, reduced in a fixed order by
@@ -72,17 +72,23 @@ struct PlaneRing {
   static constexpr size_t bytes() { return (size_t)STAGES * NV * AT_THREADS * sizeof(float); }
 };
 
-// ---- forward ------------------------------------------------------------------------------------------
-// grid (ceil(N1/128), B), block 128.  Channels k0 .. k0+KC-1 of Kc, whose weights are in c_att_weights.
+// ---- forward: logits --------------------------------------------------------------------------------------
+// The walk along d is cut into pieces of `dc` displacements, one block each (a piece re-reads one plane on either
+// side): a walk is a serial chain, and a single 55 x 128 image has 56 pixel tiles for 148 SMs.  A logit is the same
+// sum in the same order whatever the cut.  The softmax has a kernel of its own (attention_softmax_kernel), which
+// keeps the online maximum, its branch and its exponential out of this issue-bound loop.
+// Gather form: grid (ceil(N1/128), B * pieces), block 128.  Channels k0 .. k0+KC-1 of Kc, weights in c_att_weights.
 constexpr int FW_STAGES = 4;
 
 template <int KC>
 __global__ void __launch_bounds__(AT_THREADS)
-attention_forward_kernel(const float* __restrict__ x, long long x_sb, const float* __restrict__ bias,
-                         float* __restrict__ a, int Kc, int k0, int D, int H1, int W1) {
+attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float* __restrict__ bias,
+                        float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1) {
   __shared__ float ring_mem[FW_STAGES * 18 * AT_THREADS];
   const int N1 = H1 * W1;
-  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y;
+  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y % B, d0 = (blockIdx.y / B) * dc;
+  const int d1 = min(d0 + dc, D);                              // this block's logits: d0 <= d < d1
+  const int e0 = max(d0 - 1, 0), e1 = min(d1 + 1, D);          // the planes they need
   if (p >= N1) return;
   const int h = p / W1, w = p - h * W1;
   const Neighbourhood nb(h, w, H1, W1);
@@ -93,7 +99,7 @@ attention_forward_kernel(const float* __restrict__ x, long long x_sb, const floa
   float* out = a + ((size_t)b * Kc + k0) * D * plane + p;
 
   auto issue = [&](int e) {  // neighbourhoods of plane e (both channels) -> stage e % FW_STAGES
-    if (e < D) {
+    if (e < e1) {
       const int s = e % FW_STAGES;
       const float* q0 = x0 + (size_t)e * plane;
       const float* q1 = x1 + (size_t)e * plane;
@@ -106,26 +112,19 @@ attention_forward_kernel(const float* __restrict__ x, long long x_sb, const floa
     cp_async_commit();
   };
 
-  float bk[KC], acc[3][KC], m[KC], l[KC];
+  float bk[KC], acc[3][KC];
 #pragma unroll
   for (int k = 0; k < KC; ++k) {
     bk[k] = __ldg(bias + k0 + k);
     acc[0][k] = acc[1][k] = acc[2][k] = bk[k];
-    m[k] = -INFINITY;
-    l[k] = 0.f;
   }
   auto emit = [&](int d) {  // logit d is complete in acc[0]
 #pragma unroll
-    for (int k = 0; k < KC; ++k) {
-      const float L = acc[0][k];
-      out[((size_t)k * D + d) * plane] = L;
-      if (L > m[k]) { l[k] = l[k] * __expf(m[k] - L) + 1.f; m[k] = L; }
-      else l[k] += __expf(L - m[k]);
-    }
+    for (int k = 0; k < KC; ++k) out[((size_t)k * D + d) * plane] = acc[0][k];
   };
 #pragma unroll
-  for (int s = 0; s < FW_STAGES - 1; ++s) issue(s);
-  for (int e = 0; e < D; ++e) {  // plane e feeds logits e+1 (tap td=0), e (td=1), e-1 (td=2)
+  for (int s = 0; s < FW_STAGES - 1; ++s) issue(e0 + s);
+  for (int e = e0; e < e1; ++e) {  // plane e feeds logits e+1 (tap td=0), e (td=1), e-1 (td=2)
     issue(e + FW_STAGES - 1);
     cp_async_wait<FW_STAGES - 1>();
     const int s = e % FW_STAGES;
@@ -141,37 +140,21 @@ attention_forward_kernel(const float* __restrict__ x, long long x_sb, const floa
           acc[0][k] = fmaf(xv, c_att_weights[(k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
         }
       }
-    if (e >= 1) emit(e - 1);
+    if (e > d0) emit(e - 1);
 #pragma unroll
     for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
   }
-  emit(D - 1);
-#pragma unroll
-  for (int k = 0; k < KC; ++k) l[k] = 1.f / l[k];
-  // the thread re-reads its own stores, four displacements at a time so that the loads overlap
-  constexpr int DB = 4;
-  for (int d0 = 0; d0 < D; d0 += DB) {
-    float v[DB][KC];
-#pragma unroll
-    for (int i = 0; i < DB; ++i)
-#pragma unroll
-      for (int k = 0; k < KC; ++k) v[i][k] = d0 + i < D ? out[((size_t)k * D + d0 + i) * plane] : 0.f;
-#pragma unroll
-    for (int i = 0; i < DB; ++i)
-#pragma unroll
-      for (int k = 0; k < KC; ++k)
-        if (d0 + i < D) out[((size_t)k * D + d0 + i) * plane] = __expf(v[i][k] - m[k]) * l[k];
-  }
+  if (d1 == D) emit(D - 1);
 }
 
-// ---- forward, pixel tiles fetched by TMA -----------------------------------------------------------------
+// ---- logits, pixel tiles fetched by TMA -----------------------------------------------------------------
 // A block owns a tile of AT_TW x AT_TH image-1 pixels.  A producer warp fetches, plane by plane, the tile of both
 // input channels with its one-pixel halo as ONE tiled TMA load into a ring of stages (the box starts 4 pixels to the
 // left so that its x coordinate is a multiple of 16 bytes; pixels outside the image arrive as zeros, which is the
 // convolution's zero padding), and the 128 pixel threads read their 18 neighbours from shared memory at constant
 // offsets.  Against the gather above this removes the 18 per-thread copies per plane and their address arithmetic,
 // which were a third of the instructions of an issue-bound kernel.  Needs W1 % 4 == 0 (TMA strides are multiples of
-// 16 bytes).  grid (ceil(W1/32), ceil(H1/4), B), block 128 + 32.
+// 16 bytes).  grid (ceil(W1/32), ceil(H1/4), B * pieces), block 128 + 32.
 constexpr int AT_TW = 32, AT_TH = 4;
 constexpr int AT_BOX_W = AT_TW + 8, AT_BOX_H = AT_TH + 2;
 constexpr int AT_TSTAGES = 6;
@@ -193,11 +176,14 @@ struct AttentionTileSmem {
 
 template <int KC>
 __global__ void __launch_bounds__(AT_THREADS + 32)
-attention_forward_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const float* __restrict__ bias,
-                               float* __restrict__ a, int Kc, int k0, int D, int H1, int W1, int* status) {
+attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const float* __restrict__ bias,
+                              float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1,
+                              int* status) {
   if (*reinterpret_cast<volatile int*>(status) != 0) return;
   __shared__ __align__(128) AttentionTileSmem<2> sm;
-  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z;
+  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z % B, d0 = (blockIdx.z / B) * dc;
+  const int d1 = min(d0 + dc, D);
+  const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, D) - e0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
@@ -208,11 +194,11 @@ attention_forward_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const f
   __syncthreads();
   if (warp == AT_THREADS / 32) {  // producer
     if (lane == 0) {
-      for (int e = 0; e < D; ++e) {
-        const uint32_t s = e % AT_TSTAGES, ph = (e / AT_TSTAGES) & 1u;
+      for (int i = 0; i < n_planes; ++i) {
+        const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
         if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES);
-        tma_load_5d(sm.x[s].v, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e, 0, b);
+        tma_load_5d(sm.x[s].v, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
       }
     }
     return;
@@ -223,25 +209,20 @@ attention_forward_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const f
   const size_t plane = (size_t)H1 * W1;
   float* out = a + ((size_t)b * Kc + k0) * D * plane + (size_t)(valid ? h * W1 + w : 0);
 
-  float bk[KC], acc[3][KC], m[KC], l[KC];
+  float bk[KC], acc[3][KC];
 #pragma unroll
   for (int k = 0; k < KC; ++k) {
     bk[k] = __ldg(bias + k0 + k);
     acc[0][k] = acc[1][k] = acc[2][k] = bk[k];
-    m[k] = -INFINITY;
-    l[k] = 0.f;
   }
   auto emit = [&](int d) {  // logit d is complete in acc[0]
 #pragma unroll
-    for (int k = 0; k < KC; ++k) {
-      const float L = acc[0][k];
-      if (valid) out[((size_t)k * D + d) * plane] = L;
-      if (L > m[k]) { l[k] = l[k] * __expf(m[k] - L) + 1.f; m[k] = L; }
-      else l[k] += __expf(L - m[k]);
-    }
+    for (int k = 0; k < KC; ++k)
+      if (valid) out[((size_t)k * D + d) * plane] = acc[0][k];
   };
-  for (int e = 0; e < D; ++e) {  // plane e feeds logits e+1 (tap td=0), e (td=1), e-1 (td=2)
-    const uint32_t s = e % AT_TSTAGES, ph = (e / AT_TSTAGES) & 1u;
+  for (int i = 0; i < n_planes; ++i) {  // plane e feeds logits e+1 (tap td=0), e (td=1), e-1 (td=2)
+    const int e = e0 + i;
+    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
     const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
     if (!__all_sync(0xffffffffu, ok)) return;
     float xv[2][9];
@@ -262,27 +243,75 @@ attention_forward_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const f
           acc[0][k] = fmaf(xv[c][n], c_att_weights[(k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
         }
       }
-    if (e >= 1) emit(e - 1);
+    if (e > d0) emit(e - 1);
 #pragma unroll
     for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
   }
-  emit(D - 1);
-  if (!valid) return;
+  if (d1 == D) emit(D - 1);
+}
+
+// ---- softmax over d, in place -------------------------------------------------------------------------------
+// A block owns 32 consecutive pixels of one (sample, channel); warp g takes displacements g, g + 8, ... and keeps its
+// V = ceil(D / 8) values in registers, so that every logit is read once and every weight written once (HBM-bound, all
+// loads of a thread in flight together).  V = 0: any D, the values are read again in each of the three walks.  The
+// order of the sums depends on D only.  grid ceil(N1/32) * planes (= B * Kc), block 256.
+constexpr int SM_GROUPS = 8;
+constexpr int SM_THREADS = SM_GROUPS * 32;
+
+template <int V>
+__global__ void __launch_bounds__(SM_THREADS)
+attention_softmax_kernel(float* __restrict__ a, int D, int N1, unsigned pixel_blocks) {
+  __shared__ float red[2][SM_GROUPS][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const unsigned row = blockIdx.x / pixel_blocks;
+  const int p = (int)(blockIdx.x - row * pixel_blocks) * 32 + lane;
+  const bool in = p < N1;
+  float* base = a + (size_t)row * D * N1 + (in ? p : 0);
+  constexpr int NV = V > 0 ? V : 1;
+  float v[NV];
+  float m = -INFINITY;
+  if constexpr (V > 0) {
 #pragma unroll
-  for (int k = 0; k < KC; ++k) l[k] = 1.f / l[k];
-  // the thread re-reads its own stores, four displacements at a time so that the loads overlap
-  constexpr int DB = 4;
-  for (int d0 = 0; d0 < D; d0 += DB) {
-    float v[DB][KC];
+    for (int i = 0; i < V; ++i) {
+      const int d = g + i * SM_GROUPS;
+      v[i] = in && d < D ? base[(size_t)d * N1] : -INFINITY;
+    }
 #pragma unroll
-    for (int i = 0; i < DB; ++i)
+    for (int i = 0; i < V; ++i) m = fmaxf(m, v[i]);
+  } else {
+    for (int d = g; d < D; d += SM_GROUPS) m = fmaxf(m, in ? base[(size_t)d * N1] : 0.f);
+  }
+  red[0][g][lane] = m;
+  __syncthreads();
 #pragma unroll
-      for (int k = 0; k < KC; ++k) v[i][k] = d0 + i < D ? out[((size_t)k * D + d0 + i) * plane] : 0.f;
+  for (int i = 0; i < SM_GROUPS; ++i) m = fmaxf(m, red[0][i][lane]);
+  float l = 0.f;
+  if constexpr (V > 0) {
 #pragma unroll
-    for (int i = 0; i < DB; ++i)
+    for (int i = 0; i < V; ++i) {
+      if (g + i * SM_GROUPS < D) {
+        v[i] = __expf(v[i] - m);
+        l += v[i];
+      }
+    }
+  } else {
+    for (int d = g; d < D; d += SM_GROUPS) l += __expf((in ? base[(size_t)d * N1] : 0.f) - m);
+  }
+  red[1][g][lane] = l;
+  __syncthreads();
+  l = 0.f;
 #pragma unroll
-      for (int k = 0; k < KC; ++k)
-        if (d0 + i < D) out[((size_t)k * D + d0 + i) * plane] = __expf(v[i][k] - m[k]) * l[k];
+  for (int i = 0; i < SM_GROUPS; ++i) l += red[1][i][lane];
+  const float inv = 1.f / l;
+  if (!in) return;
+  if constexpr (V > 0) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int d = g + i * SM_GROUPS;
+      if (d < D) base[(size_t)d * N1] = v[i] * inv;
+    }
+  } else {
+    for (int d = g; d < D; d += SM_GROUPS) base[(size_t)d * N1] = __expf(base[(size_t)d * N1] - m) * inv;
   }
 }
 
@@ -568,7 +597,7 @@ attention_reduce_partials_kernel(const float* __restrict__ partial, int rows, in
 }
 
 // ---- input and weight gradients, pixel tiles fetched by TMA -------------------------------------------------
-// Same arithmetic as the two gather kernels above with the tile scheme of attention_forward_tiled_kernel.
+// Same arithmetic as the two gather kernels above with the tile scheme of attention_logits_tiled_kernel.
 // Input gradients: the stage holds the tile (with halo) of the KC logit-gradient channels of one plane.
 template <int KC>
 __global__ void __launch_bounds__(AT_THREADS + 32)
@@ -810,32 +839,61 @@ size_t attention_partial_floats(const AttentionDims& d) {  // bias partials per 
   return (size_t)d.B * d.Kc * (blocks + 2 * AT_TAPS * (blocks > tiles ? blocks : tiles));
 }
 
+// Displacements per block of a stencil walk: enough blocks (AT_BLOCKS_TARGET) to fill the 148 SMs several times over,
+// but at least AT_MIN_WALK displacements, because every block also reads a plane on either side of its own.
+constexpr int AT_BLOCKS_TARGET = 148 * 8, AT_MIN_WALK = 8;
+static int walk_length(size_t blocks, int D) {
+  const int pieces = (int)((AT_BLOCKS_TARGET + blocks - 1) / blocks);
+  const int dc = (D + pieces - 1) / pieces;
+  const int least = D < AT_MIN_WALK ? D : AT_MIN_WALK;
+  return dc > least ? dc : least;
+}
+
+static cudaError_t launch_softmax(float* a, size_t planes, int D, int N1, cudaStream_t st) {
+  const unsigned pb = (unsigned)((N1 + 31) / 32);
+  if ((unsigned long long)pb * planes > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+  const unsigned blocks = (unsigned)(pb * planes);
+  const int v = (D + SM_GROUPS - 1) / SM_GROUPS;
+  if (v <= 4) attention_softmax_kernel<4><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  else if (v <= 8) attention_softmax_kernel<8><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  else if (v <= 16) attention_softmax_kernel<16><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  else if (v <= 32) attention_softmax_kernel<32><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  else attention_softmax_kernel<0><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
                                      const float* bias, float* a, cudaStream_t st, int* status) {
-  const dim3 grid = pixel_grid(d);
   const bool tiled = status != nullptr && tileable(d, x, x_sb);
   CUtensorMap tm_x;
   if (tiled) {
     cudaError_t err = tile_map(&tm_x, x, x_sb, 2, 2, d, true);
     if (err != cudaSuccess) return err;
   }
-  const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B);
-  StagedWeights staged(st);
-  for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
-    const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
-    cudaError_t err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
-    if (err != cudaSuccess) return err;
-    if (tiled) {
-#define SFB_AT_FWD_T(KC) attention_forward_tiled_kernel<KC><<<tgrid, AT_THREADS + 32, 0, st>>>(tm_x, bias, a, d.Kc, k0, d.D, d.H1, d.W1, status)
-      if (kc == 1) SFB_AT_FWD_T(1); else if (kc == 2) SFB_AT_FWD_T(2); else if (kc == 3) SFB_AT_FWD_T(3); else SFB_AT_FWD_T(4);
+  const int dc = walk_length((tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B, d.D);
+  const unsigned pieces = (unsigned)((d.D + dc - 1) / dc);
+  const dim3 grid(pixel_grid(d).x, d.B * pieces);
+  const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * pieces);
+  {
+    StagedWeights staged(st);
+    for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
+      const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
+      cudaError_t err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
+      if (err != cudaSuccess) return err;
+      if (tiled) {
+#define SFB_AT_FWD_T(KC) attention_logits_tiled_kernel<KC><<<tgrid, AT_THREADS + 32, 0, st>>>(tm_x, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1, status)
+        if (kc == 1) SFB_AT_FWD_T(1); else if (kc == 2) SFB_AT_FWD_T(2); else if (kc == 3) SFB_AT_FWD_T(3); else SFB_AT_FWD_T(4);
 #undef SFB_AT_FWD_T
-      continue;
-    }
-#define SFB_AT_FWD(KC) attention_forward_kernel<KC><<<grid, AT_THREADS, 0, st>>>(x, x_sb, bias, a, d.Kc, k0, d.D, d.H1, d.W1)
-    if (kc == 1) SFB_AT_FWD(1); else if (kc == 2) SFB_AT_FWD(2); else if (kc == 3) SFB_AT_FWD(3); else SFB_AT_FWD(4);
+        continue;
+      }
+#define SFB_AT_FWD(KC) attention_logits_kernel<KC><<<grid, AT_THREADS, 0, st>>>(x, x_sb, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1)
+      if (kc == 1) SFB_AT_FWD(1); else if (kc == 2) SFB_AT_FWD(2); else if (kc == 3) SFB_AT_FWD(3); else SFB_AT_FWD(4);
 #undef SFB_AT_FWD
+    }
   }
-  return cudaGetLastError();
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  return launch_softmax(a, (size_t)d.B * d.Kc, d.D, d.H1 * d.W1, st);
 }
 
 template <int KC>

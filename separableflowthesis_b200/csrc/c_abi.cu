@@ -1077,7 +1077,7 @@ int sfb_attention_forward(const float* X, int64_t x_batch_stride, const float* w
   if (X == nullptr || weight == nullptr || bias == nullptr || A == nullptr)
     return fail(SFB_ERR_INVALID_ARGUMENT, "X, weight, bias and A must not be NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SFB_CUDA(timed(KID_ATTENTION_FWD, (Kc + 3) / 4, st,
+  SFB_CUDA(timed(KID_ATTENTION_FWD, (Kc + 3) / 4 + 1, st,
                  [&] { return launch_attention_forward(ad, X, x_batch_stride, weight, bias, A, st); }));
   return SFB_OK;
 }
@@ -1176,7 +1176,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   a.status = w.status;
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
-  SFB_CUDA(timed(KID_ATTENTION_FWD, 2 * ((K + 3) / 4), st, [&] {
+  SFB_CUDA(timed(KID_ATTENTION_FWD, 2 * ((K + 3) / 4 + 1), st, [&] {
     launch_attention_forward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + (size_t)c0 * d.W2 * N1, sb_u, weight_u,
                              bias_u, A_u, st, w.status);
     return launch_attention_forward(AttentionDims{d.B, K, d.H2, d.H1, d.W1}, SEP_v + (size_t)c0 * d.H2 * N1, sb_v,

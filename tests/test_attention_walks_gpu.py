@@ -1,0 +1,55 @@
+"""The attention kernels where their work is cut along the displacement axis and where the softmax changes the number of
+values a thread keeps: one displacement, the shortest piece, the edges of the register variants (32, 64, 128, 256
+displacements) and beyond, for the gather form and for the TMA tiles (image-1 widths that are a multiple of 4)."""
+import pytest
+import torch
+
+from oracle import separation_oracle as orc
+from separableflowthesis_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+# FP32 stencils of 54 products, softmax with __expf (2 ulp at |x| < 10) and sums of up to 300 weights: a few 1e-6
+TOL = 2e-5
+DS = [1, 2, 7, 8, 9, 17, 32, 33, 64, 65, 128, 129, 256, 257, 300]
+
+
+def relerr(a, b):
+    return ((a.double().cpu() - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("D", DS)
+@pytest.mark.parametrize("shape", [(1, 2, 3, 5), (2, 5, 6, 33)])
+def test_gather_form(shape, D, cuda_device):
+    B, Kc, H1, W1 = shape
+    g = torch.Generator().manual_seed(100 + D)
+    x = torch.randn(B, 2, D, H1, W1, generator=g)
+    weight, bias = torch.randn(Kc, 2, 3, 3, 3, generator=g) * 0.3, torch.randn(Kc, generator=g)
+    a = ops.attention_forward(x.to(cuda_device), weight.to(cuda_device), bias.to(cuda_device))
+    ref = orc.attention_forward(x.double(), weight.double(), bias.double())
+    assert relerr(a, ref) < TOL
+    assert (a.sum(dim=2) - 1).abs().max().item() < 1e-5
+    ga, add = torch.randn(a.shape, generator=g), torch.randn(x.shape, generator=g)
+    gx, gw, gb = ops.attention_backward(x.to(cuda_device), weight.to(cuda_device), a, ga.to(cuda_device),
+                                        add.to(cuda_device))
+    r_gx, r_gw, r_gb = orc.attention_backward(x.double(), weight.double(), a.double().cpu(), ga.double(), add.double())
+    assert relerr(gx, r_gx) < TOL
+    if D > 1:   # a softmax over one entry has no gradient: the reference is zero up to rounding
+        assert relerr(gw, r_gw) < TOL
+    assert (gb.double().cpu() - r_gb).abs().max().item() < TOL * max(r_gw.abs().max().item(), 1.0)
+
+
+@pytest.mark.parametrize("size", [(5, 36, 1, 7), (8, 32, 9, 33), (4, 4, 17, 65), (6, 68, 64, 129), (9, 40, 130, 257)])
+@pytest.mark.parametrize("Kc", [1, 3, 4, 6])
+def test_tiles(size, Kc, cuda_device):
+    """The weights a level call returns against the oracle's attention of the max/mean channels it returns."""
+    H1, W1, H2, W2 = size
+    g = torch.Generator().manual_seed(7 * Kc + H2)
+    F1, F2 = torch.randn(1, H1, W1, 16, generator=g) / 4, torch.randn(1, H2, W2, 16, generator=g)
+    params = [torch.randn(Kc, 2, 3, 3, 3, generator=g) * 0.3, torch.randn(Kc, generator=g),
+              torch.randn(Kc, 2, 3, 3, 3, generator=g) * 0.3, torch.randn(Kc, generator=g)]
+    sep_u, sep_v, _, _, a_u, a_v = ops.separation_level_forward(F1.to(cuda_device), F2.to(cuda_device),
+                                                                *[p.to(cuda_device) for p in params])
+    for sep, a, w, b in ((sep_u, a_u, params[0], params[1]), (sep_v, a_v, params[2], params[3])):
+        ref = orc.attention_forward(sep[:, :2].double().cpu(), w.double(), b.double())
+        assert relerr(a, ref) < TOL
