@@ -329,99 +329,89 @@ static bool tileable(const AttentionDims& d, const void* x, long long sb) {
   return d.W1 % 4 == 0 && sb % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
 }
 
-// ---- sums over a block, written to dst[i] -------------------------------------------------------------
-template <int N>
-__device__ void block_sums_to(float (&v)[N], float* smem /* [AT_THREADS/32][N] */, float* dst) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    float s = v[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    v[i] = s;
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) smem[warp * N + i] = v[i];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < N; i += AT_THREADS) {
-    float s = 0.f;
-#pragma unroll
-    for (int wv = 0; wv < AT_THREADS / 32; ++wv) s += smem[wv * N + i];
-    dst[i] = s;
-  }
-}
-
 // ---- logit gradients (softmax backward), in place -------------------------------------------------------
-// grid (ceil(N1/128), B), block 128.  bias_partial: (B * gridDim.x, Kc).
-template <int KC>
-__global__ void __launch_bounds__(AT_THREADS)
+// gL = A * (gA - sum_d gA*A), with the split of attention_softmax_kernel: 32 pixels of one (sample, channel) per block,
+// V = ceil(D / 8) displacements per thread, both arrays read once into registers (V = 0: any D, read twice).  HBM-bound.
+// bias_partial: (Kc, B * pixel_blocks), the block's sum of gL.  grid ceil(N1/32) * B * Kc, block 256.
+template <int V>
+__global__ void __launch_bounds__(SM_THREADS, V > 16 ? 2 : (V > 8 ? 3 : 6))
 attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, float* __restrict__ bias_partial,
-                            int Kc, int k0, int D, int N1) {
-  __shared__ float red[(AT_THREADS / 32) * KC];
-  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y;
-  const size_t plane = (size_t)N1;
-  float bsum[KC];
+                            int Kc, int D, int N1, unsigned pixel_blocks) {
+  __shared__ float red[SM_GROUPS][32];
+  __shared__ float bred[SM_GROUPS];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const unsigned row = blockIdx.x / pixel_blocks;   // sample * Kc + channel
+  const unsigned pb = blockIdx.x - row * pixel_blocks;
+  const int p = (int)pb * 32 + lane;
+  const bool in = p < N1;
+  const size_t base = (size_t)row * D * N1 + (in ? p : 0);
+  constexpr int NV = V > 0 ? V : 1;
+  float gv[NV], av[NV];
+  float s = 0.f;
+  if constexpr (V > 0) {
 #pragma unroll
-  for (int k = 0; k < KC; ++k) bsum[k] = 0.f;
-  if (p < N1) {
-    const size_t base = ((size_t)b * Kc + k0) * D * plane + p;
-    float s[KC];
-#pragma unroll
-    for (int k = 0; k < KC; ++k) s[k] = 0.f;
-    constexpr int DB = 4;  // displacements per batch: all loads of a batch are issued before they are used
-    for (int d0 = 0; d0 < D; d0 += DB) {
-      float gv[DB][KC], av[DB][KC];
-#pragma unroll
-      for (int i = 0; i < DB; ++i)
-#pragma unroll
-        for (int k = 0; k < KC; ++k) {
-          const size_t idx = base + ((size_t)k * D + d0 + i) * plane;
-          gv[i][k] = d0 + i < D ? g[idx] : 0.f;
-          av[i][k] = d0 + i < D ? __ldg(a + idx) : 0.f;
-        }
-#pragma unroll
-      for (int i = 0; i < DB; ++i)
-#pragma unroll
-        for (int k = 0; k < KC; ++k) s[k] = fmaf(gv[i][k], av[i][k], s[k]);
+    for (int i = 0; i < V; ++i) {
+      const int d = grp + i * SM_GROUPS;
+      const bool ok = in && d < D;
+      gv[i] = ok ? g[base + (size_t)d * N1] : 0.f;
+      av[i] = ok ? __ldg(a + base + (size_t)d * N1) : 0.f;
     }
-    for (int d0 = 0; d0 < D; d0 += DB) {
-      float gv[DB][KC], av[DB][KC];
 #pragma unroll
-      for (int i = 0; i < DB; ++i)
+    for (int i = 0; i < V; ++i) s = fmaf(gv[i], av[i], s);
+  } else if (in) {
+    for (int d = grp; d < D; d += SM_GROUPS) s = fmaf(g[base + (size_t)d * N1], __ldg(a + base + (size_t)d * N1), s);
+  }
+  red[grp][lane] = s;
+  __syncthreads();
+  s = 0.f;
 #pragma unroll
-        for (int k = 0; k < KC; ++k) {
-          const size_t idx = base + ((size_t)k * D + d0 + i) * plane;
-          gv[i][k] = d0 + i < D ? g[idx] : 0.f;
-          av[i][k] = d0 + i < D ? __ldg(a + idx) : 0.f;
-        }
+  for (int i = 0; i < SM_GROUPS; ++i) s += red[i][lane];
+  float bsum = 0.f;
+  if constexpr (V > 0) {
 #pragma unroll
-      for (int i = 0; i < DB; ++i)
-#pragma unroll
-        for (int k = 0; k < KC; ++k) {
-          const float gl = av[i][k] * (gv[i][k] - s[k]);
-          if (d0 + i < D) g[base + ((size_t)k * D + d0 + i) * plane] = gl;
-          bsum[k] += gl;
-        }
+    for (int i = 0; i < V; ++i) {
+      const int d = grp + i * SM_GROUPS;
+      if (in && d < D) {
+        const float gl = av[i] * (gv[i] - s);
+        g[base + (size_t)d * N1] = gl;
+        bsum += gl;
+      }
+    }
+  } else if (in) {
+    for (int d = grp; d < D; d += SM_GROUPS) {
+      const float gl = __ldg(a + base + (size_t)d * N1) * (g[base + (size_t)d * N1] - s);
+      g[base + (size_t)d * N1] = gl;
+      bsum += gl;
     }
   }
-  block_sums_to<KC>(bsum, red, bias_partial + ((size_t)b * gridDim.x + blockIdx.x) * Kc + k0);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
+  if (lane == 0) bred[grp] = bsum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < SM_GROUPS; ++i) t += bred[i];
+    const unsigned k = row % Kc, b = row / Kc, rows = gridDim.x / Kc;   // rows = B * pixel_blocks
+    bias_partial[(size_t)k * rows + (size_t)b * pixel_blocks + pb] = t;
+  }
 }
 
 // ---- input gradients -----------------------------------------------------------------------------------
 // gX[c, d, h, w] = add[c, d, h, w] + sum_{k, td, th, tw} W[k, c, td, th, tw] * gL[k, d - td + 1, h - th + 1, w - tw + 1]
 // Channels k0 .. k0+KC-1 (weights in c_att_weights); a later chunk adds to what the earlier ones stored.
-// grid (ceil(N1/128), B), block 128, dynamic shared memory PlaneRing<9*KC, IG_STAGES>::bytes().
+// The walk is cut into pieces of `dc` displacements like the forward's.
+// grid (ceil(N1/128), B * pieces), block 128, dynamic shared memory PlaneRing<9*KC, IG_STAGES>::bytes().
 constexpr int IG_STAGES = 3;
 
 template <int KC>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_input_grad_kernel(const float* __restrict__ gl, const float* __restrict__ add, long long add_sb,
-                            float* __restrict__ gx, int accumulate, int Kc, int k0, int D, int H1, int W1) {
+                            float* __restrict__ gx, int accumulate, int Kc, int k0, int B, int D, int dc, int H1, int W1) {
   extern __shared__ float ring_dyn[];
   const int N1 = H1 * W1;
-  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y;
+  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y % B, d0 = (blockIdx.y / B) * dc;
+  const int d1 = min(d0 + dc, D), e0 = max(d0 - 1, 0), e1 = min(d1 + 1, D);
   if (p >= N1) return;
   const int h = p / W1, w = p - h * W1;
   const Neighbourhood nb(h, w, H1, W1);
@@ -432,7 +422,7 @@ attention_input_grad_kernel(const float* __restrict__ gl, const float* __restric
   const float* ad = add != nullptr ? add + (size_t)b * add_sb + p : nullptr;
 
   auto issue = [&](int e) {
-    if (e < D) {
+    if (e < e1) {
       const int s = e % IG_STAGES;
 #pragma unroll
       for (int k = 0; k < KC; ++k) {
@@ -457,8 +447,8 @@ attention_input_grad_kernel(const float* __restrict__ gl, const float* __restric
     }
   };
 #pragma unroll
-  for (int s = 0; s < IG_STAGES - 1; ++s) issue(s);
-  for (int e = 0; e < D; ++e) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
+  for (int s = 0; s < IG_STAGES - 1; ++s) issue(e0 + s);
+  for (int e = e0; e < e1; ++e) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
     issue(e + IG_STAGES - 1);
     cp_async_wait<IG_STAGES - 1>();
     const int s = e % IG_STAGES;
@@ -475,29 +465,30 @@ attention_input_grad_kernel(const float* __restrict__ gl, const float* __restric
           for (int td = 0; td < 3; ++td)
             acc[c][td] = fmaf(v, c_att_weights[(k * 2 + c) * AT_TAPS + td * 9 + t], acc[c][td]);
       }
-    if (e >= 1) emit(e - 1);
+    if (e > d0) emit(e - 1);
 #pragma unroll
     for (int c = 0; c < 2; ++c) { acc[c][0] = acc[c][1]; acc[c][1] = acc[c][2]; acc[c][2] = 0.f; }
   }
-  emit(D - 1);
+  if (d1 == D) emit(D - 1);
 }
 
 // ---- weight gradients ----------------------------------------------------------------------------------
 // gW[k, c, td, th, tw] = sum_{b, d, h, w} gL[k, d, h, w] * X[c, d + td - 1, h + th - 1, w + tw - 1]
-// grid (ceil(N1/128), B, 2 * ceil(Kc/KW)), block 128: a thread owns input channel c and KW output channels;
-// its KW*27 sums live in registers, every X value it reads feeds 3*KW of them.
-// partial: (B * gridDim.x, Kc, 2, 27).
+// grid (ceil(N1/128), B * pieces, 2 * ceil(Kc/KW)), block 128: a thread owns input channel c and KW output channels;
+// its KW*27 sums live in registers, every X value it reads feeds 3*KW of them.  A piece is `dc` planes of X.
+// partial: (Kc * 2 * 27, gridDim.x * gridDim.y), one column per block, so that the reduction reads consecutive values.
 constexpr int WG_STAGES = 4;
 
 template <int KW>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const float* __restrict__ gl,
-                             float* __restrict__ partial, int Kc, int D, int H1, int W1) {
+                             float* __restrict__ partial, int Kc, int B, int D, int dc, int H1, int W1) {
   constexpr int NV = 9 + KW;
   __shared__ float ring_mem[WG_STAGES * NV * AT_THREADS];
   __shared__ float red[(AT_THREADS / 32) * KW * AT_TAPS];
   const int N1 = H1 * W1;
-  const int b = blockIdx.y, c = blockIdx.z & 1, k0 = (blockIdx.z >> 1) * KW;
+  const int b = blockIdx.y % B, c = blockIdx.z & 1, k0 = (blockIdx.z >> 1) * KW;
+  const int e0 = (blockIdx.y / B) * dc, e1 = min(e0 + dc, D);
   const size_t plane = (size_t)N1;
   const int p = blockIdx.x * AT_THREADS + threadIdx.x;
   float acc[KW * AT_TAPS];  // [k][td][neighbour]
@@ -510,7 +501,7 @@ attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const 
     const float* xc = x + (size_t)b * x_sb + (size_t)c * D * plane + p;
     const float* g = gl + ((size_t)b * Kc + k0) * D * plane + p;
     auto issue = [&](int e) {  // X neighbourhood of plane e and gL of plane e+1
-      if (e < D) {
+      if (e < e1) {
         const int s = e % WG_STAGES;
         const float* q = xc + (size_t)e * plane;
 #pragma unroll
@@ -526,12 +517,12 @@ attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const 
     float g_prev[KW], g_cur[KW], g_next[KW];
 #pragma unroll
     for (int k = 0; k < KW; ++k) {
-      g_prev[k] = 0.f;
-      g_cur[k] = k0 + k < Kc ? __ldg(g + (size_t)k * D * plane) : 0.f;
+      g_prev[k] = (e0 > 0 && k0 + k < Kc) ? __ldg(g + ((size_t)k * D + e0 - 1) * plane) : 0.f;
+      g_cur[k] = k0 + k < Kc ? __ldg(g + ((size_t)k * D + e0) * plane) : 0.f;
     }
 #pragma unroll
-    for (int s = 0; s < WG_STAGES - 1; ++s) issue(s);
-    for (int e = 0; e < D; ++e) {  // plane e of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2)
+    for (int s = 0; s < WG_STAGES - 1; ++s) issue(e0 + s);
+    for (int e = e0; e < e1; ++e) {  // plane e of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2)
       issue(e + WG_STAGES - 1);
       cp_async_wait<WG_STAGES - 1>();
       const int s = e % WG_STAGES;
@@ -566,26 +557,27 @@ attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const 
     for (int i = 0; i < KW * AT_TAPS; ++i) red[warp * KW * AT_TAPS + i] = acc[i];
   }
   __syncthreads();
-  float* dst = partial + ((size_t)b * gridDim.x + blockIdx.x) * Kc * 2 * AT_TAPS;
+  const size_t rows = (size_t)gridDim.x * gridDim.y;
+  float* dst = partial + (size_t)blockIdx.y * gridDim.x + blockIdx.x;
   for (int i = threadIdx.x; i < KW * AT_TAPS; i += AT_THREADS) {
     const int k = i / AT_TAPS, t = i - k * AT_TAPS;
     if (k0 + k >= Kc) continue;
     float s = 0.f;
 #pragma unroll
     for (int wv = 0; wv < AT_THREADS / 32; ++wv) s += red[wv * KW * AT_TAPS + i];
-    dst[((size_t)(k0 + k) * 2 + c) * AT_TAPS + t] = s;
+    dst[(((size_t)(k0 + k) * 2 + c) * AT_TAPS + t) * rows] = s;
   }
 }
 
-// out[i] = sum over rows of partial[row][i].  One block per column: thread t adds rows t, t + 256, ... in order, then
+// out[i] = sum over rows of partial[i][row].  One block per column: thread t adds rows t, t + 256, ... in order, then
 // the 256 partial sums are combined in a fixed tree, so the result does not depend on scheduling (bit-reproducible).
 constexpr int RP_THREADS = 256;
 __global__ void __launch_bounds__(RP_THREADS)
-attention_reduce_partials_kernel(const float* __restrict__ partial, int rows, int cols, float* __restrict__ out) {
+attention_reduce_partials_kernel(const float* __restrict__ partial, int rows, float* __restrict__ out) {
   __shared__ float red[RP_THREADS];
   const int i = blockIdx.x;
   float s = 0.f;
-  for (int r = threadIdx.x; r < rows; r += RP_THREADS) s += __ldg(partial + (size_t)r * cols + i);
+  for (int r = threadIdx.x; r < rows; r += RP_THREADS) s += __ldg(partial + (size_t)i * rows + r);
   red[threadIdx.x] = s;
   __syncthreads();
 #pragma unroll
@@ -602,11 +594,13 @@ attention_reduce_partials_kernel(const float* __restrict__ partial, int rows, in
 template <int KC>
 __global__ void __launch_bounds__(AT_THREADS + 32)
 attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, const float* __restrict__ add,
-                                  long long add_sb, float* __restrict__ gx, int accumulate, int k0, int D, int H1,
-                                  int W1, int* status) {
+                                  long long add_sb, float* __restrict__ gx, int accumulate, int k0, int B, int D,
+                                  int dc, int H1, int W1, int* status) {
   if (*reinterpret_cast<volatile int*>(status) != 0) return;
   __shared__ __align__(128) AttentionTileSmem<KC> sm;
-  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z;
+  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z % B, d0 = (blockIdx.z / B) * dc;
+  const int d1 = min(d0 + dc, D);
+  const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, D) - e0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
@@ -617,11 +611,11 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
   __syncthreads();
   if (warp == AT_THREADS / 32) {  // producer
     if (lane == 0) {
-      for (int e = 0; e < D; ++e) {
-        const uint32_t s = e % AT_TSTAGES, ph = (e / AT_TSTAGES) & 1u;
+      for (int i = 0; i < n_planes; ++i) {
+        const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
         if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&sm.full[s], KC * AT_TILE_BYTES);
-        tma_load_5d(sm.x[s].v, &tm_gl, &sm.full[s], w0 - 4, h0 - 1, e, k0, b);
+        tma_load_5d(sm.x[s].v, &tm_gl, &sm.full[s], w0 - 4, h0 - 1, e0 + i, k0, b);
       }
     }
     return;
@@ -646,8 +640,9 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
       o0[i] = v;
     }
   };
-  for (int e = 0; e < D; ++e) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
-    const uint32_t s = e % AT_TSTAGES, ph = (e / AT_TSTAGES) & 1u;
+  for (int i = 0; i < n_planes; ++i) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
+    const int e = e0 + i;
+    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
     const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
     if (!__all_sync(0xffffffffu, ok)) return;
     float v[KC][9];
@@ -669,117 +664,151 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
           for (int td = 0; td < 3; ++td)
             acc[c][td] = fmaf(v[k][n], c_att_weights[(k * 2 + c) * AT_TAPS + td * 9 + t], acc[c][td]);
       }
-    if (e >= 1) emit(e - 1);
+    if (e > d0) emit(e - 1);
 #pragma unroll
     for (int c = 0; c < 2; ++c) { acc[c][0] = acc[c][1]; acc[c][1] = acc[c][2]; acc[c][2] = 0.f; }
   }
-  emit(D - 1);
+  if (d1 == D) emit(D - 1);
 }
 
-// Weight gradients: a thread owns input channel c and KW output channels; the stage holds the tile (with halo) of
-// plane e of X[c] and the tile (without halo) of plane e+1 of the KW logit-gradient channels.
-// grid (ceil(W1/32), ceil(H1/4), B * 2 * chunks); partial: (B * tiles, Kc, 2, 27).
+// Weight gradients: warps 0-3 own input channel 0, warps 4-7 input channel 1, each thread KW output channels of its
+// pixel; the stage holds the tile (with halo) of plane e of both X channels and the tile (without halo) of plane e+1 of
+// the KW logit-gradient channels, which the two halves share.  The sums of two output channels are one packed pair
+// (fma.rn.f32x2 with the X value in both halves), which halves the multiply-add instructions; KW odd leaves one
+// channel on scalar ones.  A piece is `dc` planes of X.
+// grid (ceil(W1/32), ceil(H1/4), B * chunks * pieces); partial: (Kc * 2 * 27, tiles * B * pieces).
+constexpr int WG_WARPS = 8;
 template <int KW>
 struct WeightGradTileSmem {
   struct alignas(128) Stage {   // both parts are TMA destinations: 128-byte aligned
-    alignas(128) float x[AT_BOX_H][AT_BOX_W];
+    alignas(128) float x[2][AT_BOX_H][AT_BOX_W];
     alignas(128) float g[KW][AT_TH][AT_TW];
   } st[AT_TSTAGES];
   uint64_t full[AT_TSTAGES];
   uint64_t empty[AT_TSTAGES];
   WaitCtl ctl;
-  float red[(AT_THREADS / 32) * KW * AT_TAPS];
+  float red[WG_WARPS * KW * AT_TAPS];
 };
 
 template <int KW>
-__global__ void __launch_bounds__(AT_THREADS + 32)
+__global__ void __launch_bounds__(WG_WARPS * 32 + 32, 1)
 attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_gl,
                                    const float* __restrict__ gl, float* __restrict__ partial, int Kc, int B, int D,
-                                   int H1, int W1, int* status) {
+                                   int dc, int chunks, int H1, int W1, int* status) {
   if (*reinterpret_cast<volatile int*>(status) != 0) return;
   __shared__ __align__(128) WeightGradTileSmem<KW> sm;
+  constexpr int KP = KW / 2;   // packed channel pairs
   const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH;
-  const int b = blockIdx.z % B, zc = blockIdx.z / B, c = zc & 1, k0 = (zc >> 1) * KW;
+  const int b = blockIdx.z % B, zr = blockIdx.z / B, k0 = (zr % chunks) * KW, piece = zr / chunks;
+  const int e0 = piece * dc, n_planes = min(dc, D - e0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
+    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], WG_WARPS); }
     wait_ctl_init(&sm.ctl, 0);
     fence_barrier_init();
     prefetch_tensormap(&tm_x);
     prefetch_tensormap(&tm_gl);
   }
   __syncthreads();
-  if (warp == AT_THREADS / 32) {  // producer
+  if (warp == WG_WARPS) {  // producer
     if (lane == 0) {
-      for (int e = 0; e < D; ++e) {
-        const uint32_t s = e % AT_TSTAGES, ph = (e / AT_TSTAGES) & 1u;
+      for (int i = 0; i < n_planes; ++i) {
+        const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
         if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.full[s], AT_TILE_BYTES + KW * AT_TH * AT_TW * (uint32_t)sizeof(float));
-        tma_load_5d(sm.st[s].x, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e, c, b);
-        tma_load_5d(sm.st[s].g, &tm_gl, &sm.full[s], w0, h0, e + 1, k0, b);  // plane D and channels >= Kc read as zero
+        mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES + KW * AT_TH * AT_TW * (uint32_t)sizeof(float));
+        tma_load_5d(sm.st[s].x, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
+        tma_load_5d(sm.st[s].g, &tm_gl, &sm.full[s], w0, h0, e0 + i + 1, k0, b);  // plane D, channels >= Kc read as zero
       }
     }
     return;
   }
-  const int tx = lane, ty = warp;
+  const int tx = lane, ty = warp & 3, c = warp >> 2;
   const int h = h0 + ty, w = w0 + tx;
   const bool valid = h < H1 && w < W1;
   const size_t plane = (size_t)H1 * W1;
-  float acc[KW * AT_TAPS];  // [k][td][neighbour]
+  uint64_t acc2[KP > 0 ? KP * AT_TAPS : 1];         // [pair][td][neighbour]
+  float acc1[(KW & 1) != 0 ? AT_TAPS : 1];          // the odd channel
 #pragma unroll
-  for (int i = 0; i < KW * AT_TAPS; ++i) acc[i] = 0.f;
+  for (int i = 0; i < KP * AT_TAPS; ++i) acc2[i] = 0ull;
+  if constexpr ((KW & 1) != 0) {
+#pragma unroll
+    for (int i = 0; i < AT_TAPS; ++i) acc1[i] = 0.f;
+  }
   float g_prev[KW], g_cur[KW], g_next[KW];
 #pragma unroll
   for (int k = 0; k < KW; ++k) {
-    g_prev[k] = 0.f;
-    g_cur[k] = (valid && k0 + k < Kc) ? __ldg(gl + (((size_t)b * Kc + k0 + k) * D) * plane + (size_t)h * W1 + w) : 0.f;
+    const bool ok = valid && k0 + k < Kc;
+    const float* gp = gl + (((size_t)b * Kc + (ok ? k0 + k : 0)) * D + e0) * plane + (ok ? (size_t)h * W1 + w : 0);
+    g_prev[k] = (ok && e0 > 0) ? __ldg(gp - plane) : 0.f;
+    g_cur[k] = ok ? __ldg(gp) : 0.f;
   }
   bool alive = true;
-  for (int e = 0; e < D; ++e) {  // plane e of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2)
-    const uint32_t s = e % AT_TSTAGES, ph = (e / AT_TSTAGES) & 1u;
+  for (int i = 0; i < n_planes; ++i) {  // plane e of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2)
+    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
     const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
     if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
     float v[9];
 #pragma unroll
-    for (int n = 0; n < 9; ++n) v[n] = sm.st[s].x[ty + n / 3][tx + 3 + n % 3];
+    for (int n = 0; n < 9; ++n) v[n] = sm.st[s].x[c][ty + n / 3][tx + 3 + n % 3];
 #pragma unroll
     for (int k = 0; k < KW; ++k) g_next[k] = sm.st[s].g[k][ty][tx];
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.empty[s]);
 #pragma unroll
-    for (int k = 0; k < KW; ++k)
+    for (int q = 0; q < KP; ++q) {
+      const uint64_t gn = pack2(g_next[2 * q], g_next[2 * q + 1]), gc = pack2(g_cur[2 * q], g_cur[2 * q + 1]),
+                     gp = pack2(g_prev[2 * q], g_prev[2 * q + 1]);
 #pragma unroll
       for (int n = 0; n < 9; ++n) {
-        acc[k * AT_TAPS + n] = fmaf(g_next[k], v[n], acc[k * AT_TAPS + n]);
-        acc[k * AT_TAPS + 9 + n] = fmaf(g_cur[k], v[n], acc[k * AT_TAPS + 9 + n]);
-        acc[k * AT_TAPS + 18 + n] = fmaf(g_prev[k], v[n], acc[k * AT_TAPS + 18 + n]);
+        const uint64_t vv = pack2(v[n], v[n]);
+        acc2[q * AT_TAPS + n] = fma2(gn, vv, acc2[q * AT_TAPS + n]);
+        acc2[q * AT_TAPS + 9 + n] = fma2(gc, vv, acc2[q * AT_TAPS + 9 + n]);
+        acc2[q * AT_TAPS + 18 + n] = fma2(gp, vv, acc2[q * AT_TAPS + 18 + n]);
       }
+    }
+    if constexpr ((KW & 1) != 0) {
+#pragma unroll
+      for (int n = 0; n < 9; ++n) {
+        acc1[n] = fmaf(g_next[KW - 1], v[n], acc1[n]);
+        acc1[9 + n] = fmaf(g_cur[KW - 1], v[n], acc1[9 + n]);
+        acc1[18 + n] = fmaf(g_prev[KW - 1], v[n], acc1[18 + n]);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < KW; ++k) { g_prev[k] = g_cur[k]; g_cur[k] = g_next[k]; }
   }
-  // reduce over the block's 128 pixel threads (named barrier 1: the producer warp has left);
-  // thread i < KW*27 then holds column (k, td, n) and stores it at [k0 + k][c][td*9 + n]
-#pragma unroll
-  for (int i = 0; i < KW * AT_TAPS; ++i) {
-    float sum = alive ? acc[i] : 0.f;
+  // reduce over the 128 pixel threads of each input channel (named barrier 1: the producer warp has left);
+  // column (k, c, td, n) goes to row (k0 + k) * 54 + c * 27 + td * 9 + n of the partial sums
+  auto put = [&](int i, float sum) {
+    if (!alive) sum = 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    acc[i] = sum;
-  }
-  if (lane == 0) {
+    if (lane == 0) sm.red[warp * KW * AT_TAPS + i] = sum;
+  };
 #pragma unroll
-    for (int i = 0; i < KW * AT_TAPS; ++i) sm.red[warp * KW * AT_TAPS + i] = acc[i];
+  for (int q = 0; q < KP; ++q)
+#pragma unroll
+    for (int t = 0; t < AT_TAPS; ++t) {
+      float lo, hi;
+      unpack2(acc2[q * AT_TAPS + t], lo, hi);
+      put(2 * q * AT_TAPS + t, lo);
+      put((2 * q + 1) * AT_TAPS + t, hi);
+    }
+  if constexpr ((KW & 1) != 0) {
+#pragma unroll
+    for (int t = 0; t < AT_TAPS; ++t) put((KW - 1) * AT_TAPS + t, acc1[t]);
   }
-  named_bar_sync(1, AT_THREADS);
+  named_bar_sync(1, WG_WARPS * 32);
   const int tiles = gridDim.x * gridDim.y;
-  float* dst = partial + ((size_t)b * tiles + blockIdx.y * gridDim.x + blockIdx.x) * Kc * 2 * AT_TAPS;
-  for (int i = threadIdx.x; i < KW * AT_TAPS; i += AT_THREADS) {
-    const int k = i / AT_TAPS, t = i - k * AT_TAPS;
+  const size_t rows = (size_t)tiles * (gridDim.z / chunks);
+  float* dst = partial + ((size_t)piece * B + b) * tiles + blockIdx.y * gridDim.x + blockIdx.x;
+  for (int i = threadIdx.x; i < 2 * KW * AT_TAPS; i += WG_WARPS * 32) {
+    const int cc = i / (KW * AT_TAPS), j = i - cc * KW * AT_TAPS, k = j / AT_TAPS, t = j - k * AT_TAPS;
     if (k0 + k >= Kc) continue;
     float sum = 0.f;
 #pragma unroll
-    for (int wv = 0; wv < AT_THREADS / 32; ++wv) sum += sm.red[wv * KW * AT_TAPS + i];
-    dst[((size_t)(k0 + k) * 2 + c) * AT_TAPS + t] = sum;
+    for (int wv = 0; wv < 4; ++wv) sum += sm.red[(cc * 4 + wv) * KW * AT_TAPS + j];
+    dst[(((size_t)(k0 + k) * 2 + cc) * AT_TAPS + t) * rows] = sum;
   }
 }
 
@@ -834,19 +863,32 @@ static dim3 pixel_grid(const AttentionDims& d) { return dim3((d.H1 * d.W1 + AT_T
 static size_t tile_count(const AttentionDims& d) {
   return (size_t)((d.W1 + AT_TW - 1) / AT_TW) * ((d.H1 + AT_TH - 1) / AT_TH);
 }
-size_t attention_partial_floats(const AttentionDims& d) {  // bias partials per pixel block, weight partials per block / tile
-  const size_t blocks = (size_t)pixel_grid(d).x, tiles = tile_count(d);
-  return (size_t)d.B * d.Kc * (blocks + 2 * AT_TAPS * (blocks > tiles ? blocks : tiles));
-}
-
 // Displacements per block of a stencil walk: enough blocks (AT_BLOCKS_TARGET) to fill the 148 SMs several times over,
 // but at least AT_MIN_WALK displacements, because every block also reads a plane on either side of its own.
+// The weight gradients pay for a reduction over the block at the end of a walk as well and keep one or two blocks on an
+// SM, hence fewer and longer pieces.
 constexpr int AT_BLOCKS_TARGET = 148 * 8, AT_MIN_WALK = 8;
-static int walk_length(size_t blocks, int D) {
-  const int pieces = (int)((AT_BLOCKS_TARGET + blocks - 1) / blocks);
+constexpr int WG_BLOCKS_TARGET = 148 * 3, WG_MIN_WALK = 16;
+static int walk_length(size_t blocks, int D, int target = AT_BLOCKS_TARGET, int min_walk = AT_MIN_WALK) {
+  const int pieces = (int)((target + blocks - 1) / blocks);
   const int dc = (D + pieces - 1) / pieces;
-  const int least = D < AT_MIN_WALK ? D : AT_MIN_WALK;
+  const int least = D < min_walk ? D : min_walk;
   return dc > least ? dc : least;
+}
+// No walk of at most D displacements over these blocks has more pieces than this.
+static size_t walk_pieces_bound(size_t blocks, int D, int target, int min_walk) {
+  const size_t pieces = (target + blocks - 1) / blocks, most = (size_t)(D + min_walk - 1) / min_walk;
+  return pieces < most ? pieces : most;
+}
+
+// Bias partials per 32-pixel block, weight partials per block / tile and piece of the walk.  An upper bound that does
+// not fall when D grows: a level's two calls share one buffer sized for the larger D.
+size_t attention_partial_floats(const AttentionDims& d) {
+  const size_t blocks = (size_t)pixel_grid(d).x * d.B, tiles = tile_count(d) * d.B;
+  const size_t gather = blocks * walk_pieces_bound(2 * blocks, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
+  const size_t tiled = tiles * walk_pieces_bound(tiles, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
+  const size_t bias = (size_t)d.B * (((size_t)d.H1 * d.W1 + 31) / 32);
+  return d.Kc * (bias + 2 * AT_TAPS * (gather > tiled ? gather : tiled));
 }
 
 static cudaError_t launch_softmax(float* a, size_t planes, int D, int N1, cudaStream_t st) {
@@ -898,7 +940,7 @@ cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, lon
 
 template <int KC>
 static cudaError_t launch_input_grad(const dim3 grid, const float* g, const float* add, long long add_sb, float* gx,
-                                     int accumulate, const AttentionDims& d, int k0, cudaStream_t st) {
+                                     int accumulate, const AttentionDims& d, int dc, int k0, cudaStream_t st) {
   constexpr size_t smem = PlaneRing<9 * KC, IG_STAGES>::bytes();
   static bool configured[AT_MAX_DEVICES] = {false};  // benign race: setting the attribute twice is harmless
   int dev = 0;
@@ -909,8 +951,21 @@ static cudaError_t launch_input_grad(const dim3 grid, const float* g, const floa
     if (err != cudaSuccess) return err;
     configured[dev] = true;
   }
-  attention_input_grad_kernel<KC><<<grid, AT_THREADS, smem, st>>>(g, add, add_sb, gx, accumulate, d.Kc, k0, d.D, d.H1,
-                                                                  d.W1);
+  attention_input_grad_kernel<KC><<<grid, AT_THREADS, smem, st>>>(g, add, add_sb, gx, accumulate, d.Kc, k0, d.B, d.D, dc,
+                                                                  d.H1, d.W1);
+  return cudaGetLastError();
+}
+
+static cudaError_t launch_logit_grad(const AttentionDims& d, const float* a, float* g, float* bias_partial,
+                                     cudaStream_t st) {
+  const int N1 = d.H1 * d.W1, v = (d.D + SM_GROUPS - 1) / SM_GROUPS;
+  const unsigned pb = (unsigned)((N1 + 31) / 32);
+  if ((unsigned long long)pb * d.B * d.Kc > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+  const unsigned blocks = pb * (unsigned)(d.B * d.Kc);
+#define SFB_AT_LG(V) attention_logit_grad_kernel<V><<<blocks, SM_THREADS, 0, st>>>(a, g, bias_partial, d.Kc, d.D, N1, pb)
+  if (v <= 4) SFB_AT_LG(4); else if (v <= 8) SFB_AT_LG(8); else if (v <= 16) SFB_AT_LG(16);
+  else if (v <= 32) SFB_AT_LG(32); else SFB_AT_LG(0);
+#undef SFB_AT_LG
   return cudaGetLastError();
 }
 
@@ -918,24 +973,23 @@ cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, lo
                                       const float* a, float* g, const float* add, long long add_sb, float* gx,
                                       float* gweight, float* gbias, float* partial, cudaStream_t st, int* status) {
   const int N1 = d.H1 * d.W1;
-  const dim3 grid = pixel_grid(d);
-  const int rows = (int)(grid.x * grid.y);
-  float* bias_partial = partial;                            // (rows, Kc)
-  float* weight_partial = partial + (size_t)rows * d.Kc;    // (rows or tiles, Kc, 54)
+  const size_t blocks = (size_t)pixel_grid(d).x * d.B, tiles = tile_count(d) * d.B;
+  const int bias_rows = d.B * ((N1 + 31) / 32);
+  float* bias_partial = partial;                               // (Kc, bias_rows)
+  float* weight_partial = partial + (size_t)bias_rows * d.Kc;  // (Kc * 54, blocks or tiles times pieces)
   const long long g_sb = (long long)d.Kc * d.D * N1;
   const bool tiled = status != nullptr && tileable(d, x, x_sb) && tileable(d, g, g_sb);
-  const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B);
-  for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
-    const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
-#define SFB_AT_LG(KC) attention_logit_grad_kernel<KC><<<grid, AT_THREADS, 0, st>>>(a, g, bias_partial, d.Kc, k0, d.D, N1)
-    if (kc == 1) SFB_AT_LG(1); else if (kc == 2) SFB_AT_LG(2); else if (kc == 3) SFB_AT_LG(3); else SFB_AT_LG(4);
-#undef SFB_AT_LG
-  }
+  cudaError_t err = launch_logit_grad(d, a, g, bias_partial, st);
+  if (err != cudaSuccess) return err;
   {
+    const int dc = walk_length(tiled ? tiles : blocks, d.D);
+    const unsigned pieces = (unsigned)((d.D + dc - 1) / dc);
+    const dim3 grid(pixel_grid(d).x, d.B * pieces);
+    const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * pieces);
     StagedWeights staged(st);
     for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
       const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
-      cudaError_t err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
+      err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
       if (err != cudaSuccess) return err;
       const float* ad = k0 == 0 ? add : nullptr;
       const int accumulate = k0 == 0 ? 0 : 1;
@@ -943,38 +997,41 @@ cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, lo
         CUtensorMap tm_gl;
         err = tile_map(&tm_gl, g, g_sb, d.Kc, kc, d, true);
         if (err != cudaSuccess) return err;
-#define SFB_AT_IG_T(KC) attention_input_grad_tiled_kernel<KC><<<tgrid, AT_THREADS + 32, 0, st>>>(tm_gl, ad, add_sb, gx, accumulate, k0, d.D, d.H1, d.W1, status)
+#define SFB_AT_IG_T(KC) attention_input_grad_tiled_kernel<KC><<<tgrid, AT_THREADS + 32, 0, st>>>(tm_gl, ad, add_sb, gx, accumulate, k0, d.B, d.D, dc, d.H1, d.W1, status)
         if (kc == 1) SFB_AT_IG_T(1); else if (kc == 2) SFB_AT_IG_T(2); else if (kc == 3) SFB_AT_IG_T(3); else SFB_AT_IG_T(4);
 #undef SFB_AT_IG_T
         continue;
       }
-      if (kc == 1) err = launch_input_grad<1>(grid, g, ad, add_sb, gx, accumulate, d, k0, st);
-      else if (kc == 2) err = launch_input_grad<2>(grid, g, ad, add_sb, gx, accumulate, d, k0, st);
-      else if (kc == 3) err = launch_input_grad<3>(grid, g, ad, add_sb, gx, accumulate, d, k0, st);
-      else err = launch_input_grad<4>(grid, g, ad, add_sb, gx, accumulate, d, k0, st);
+      if (kc == 1) err = launch_input_grad<1>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
+      else if (kc == 2) err = launch_input_grad<2>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
+      else if (kc == 3) err = launch_input_grad<3>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
+      else err = launch_input_grad<4>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
       if (err != cudaSuccess) return err;
     }
   }
   const int kw = d.Kc >= 4 ? 4 : d.Kc, chunks = (d.Kc + kw - 1) / kw;
-  int wrows = rows;
+  const int dc = walk_length(tiled ? tiles : 2 * blocks, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
+  const int pieces = (d.D + dc - 1) / dc;
+  int wrows;
   if (tiled) {
     CUtensorMap tm_x, tm_gl;
-    cudaError_t err = tile_map(&tm_x, x, x_sb, 2, 1, d, true);
+    err = tile_map(&tm_x, x, x_sb, 2, 2, d, true);
     if (err == cudaSuccess) err = tile_map(&tm_gl, g, g_sb, d.Kc, kw, d, false);
     if (err != cudaSuccess) return err;
-    const dim3 wgrid(tgrid.x, tgrid.y, d.B * 2 * chunks);
-    wrows = (int)(tile_count(d) * d.B);
-#define SFB_AT_WG_T(KW) attention_weight_grad_tiled_kernel<KW><<<wgrid, AT_THREADS + 32, 0, st>>>(tm_x, tm_gl, g, weight_partial, d.Kc, d.B, d.D, d.H1, d.W1, status)
+    const dim3 wgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * chunks * pieces);
+    wrows = (int)(tiles * pieces);
+#define SFB_AT_WG_T(KW) attention_weight_grad_tiled_kernel<KW><<<wgrid, WG_WARPS * 32 + 32, 0, st>>>(tm_x, tm_gl, g, weight_partial, d.Kc, d.B, d.D, dc, chunks, d.H1, d.W1, status)
     if (kw == 1) SFB_AT_WG_T(1); else if (kw == 2) SFB_AT_WG_T(2); else if (kw == 3) SFB_AT_WG_T(3); else SFB_AT_WG_T(4);
 #undef SFB_AT_WG_T
   } else {
-#define SFB_AT_WG(KW) attention_weight_grad_kernel<KW><<<dim3(grid.x, grid.y, 2 * chunks), AT_THREADS, 0, st>>>(x, x_sb, g, weight_partial, d.Kc, d.D, d.H1, d.W1)
+    const dim3 wgrid(pixel_grid(d).x, d.B * pieces, 2 * chunks);
+    wrows = (int)(blocks * pieces);
+#define SFB_AT_WG(KW) attention_weight_grad_kernel<KW><<<wgrid, AT_THREADS, 0, st>>>(x, x_sb, g, weight_partial, d.Kc, d.B, d.D, dc, d.H1, d.W1)
     if (kw == 1) SFB_AT_WG(1); else if (kw == 2) SFB_AT_WG(2); else if (kw == 3) SFB_AT_WG(3); else SFB_AT_WG(4);
 #undef SFB_AT_WG
   }
-  const int wcols = d.Kc * 2 * AT_TAPS;
-  attention_reduce_partials_kernel<<<wcols, RP_THREADS, 0, st>>>(weight_partial, wrows, wcols, gweight);
-  attention_reduce_partials_kernel<<<d.Kc, RP_THREADS, 0, st>>>(bias_partial, rows, d.Kc, gbias);
+  attention_reduce_partials_kernel<<<d.Kc * 2 * AT_TAPS, RP_THREADS, 0, st>>>(weight_partial, wrows, gweight);
+  attention_reduce_partials_kernel<<<d.Kc, RP_THREADS, 0, st>>>(bias_partial, bias_rows, gbias);
   return cudaGetLastError();
 }
 
