@@ -6,7 +6,8 @@
 // HBM-bound gathers.  The volumes stay in the layout the rest of the path produces, (B, dim, D, H1, W1): the
 // displacement axis of one pixel is strided by the plane size, a warp handles 32 neighbouring pixels, and because
 // neighbouring pixels have similar displacements their gathers mostly fall into the same 128-byte lines.  (The
-// reference first permutes to (B*H1*W1, dim, 1, D), core/corr.py:531-541.)
+// reference first permutes to (B*H1*W1, dim, 1, D), core/corr.py:531-541.)  Every warp takes one pyramid level of its
+// pixels, so that a pixel's levels are gathered side by side and not one after the other.
 // Backward: every (b, channel, displacement, pixel) element of a level's gradient is touched by one thread only,
 // so the scatter needs no atomics; the levels are then folded into the gradient of the volume in one pass.
 #include "kernels.h"
@@ -42,30 +43,43 @@ struct LookupLevelsMut {
   int D[LOOKUP_MAX_LEVELS];
 };
 
-// out (B, levels*dim*(2r+1), N1): channel (l*dim + ch)*(2r+1) + t.  grid (ceil(N1/128), B)
-__global__ void lookup_forward_kernel(const LookupLevels lv, const float* __restrict__ coord, long long coord_sb,
-                                      float* __restrict__ out, int dim, int N1, int levels, int radius,
-                                      int clamp_unit) {
-  const int p = blockIdx.x * LK_THREADS + threadIdx.x, b = blockIdx.y;
+// out (B, levels*dim*(2r+1), N1): channel (l*dim + ch)*(2r+1) + t.  Block: 32 pixels x LK_WARPS levels at a time;
+// TAPS = 2r+1 when known at compile time (all loads of a thread in flight together), else 0.  grid (ceil(N1/32), B)
+constexpr int LK_WARPS = 4;
+template <int TAPS>
+__global__ void __launch_bounds__(32 * LK_WARPS)
+lookup_forward_kernel(const LookupLevels lv, const float* __restrict__ coord, long long coord_sb,
+                      float* __restrict__ out, int dim, int N1, int levels, int radius, int clamp_unit) {
+  const int p = blockIdx.x * 32 + (threadIdx.x & 31), b = blockIdx.y;
   if (p >= N1) return;
   const float c = __ldg(coord + (size_t)b * coord_sb + p);
-  const int taps = 2 * radius + 1;
+  const int taps = TAPS > 0 ? TAPS : 2 * radius + 1;
   float* o = out + (size_t)b * levels * dim * taps * N1 + p;
-  for (int l = 0; l < levels; ++l) {
+  for (int l = threadIdx.x >> 5; l < levels; l += LK_WARPS) {
     const int Dl = lv.D[l];
-    for (int t = 0; t < taps; ++t) {
-      const float ix = lookup_position(c, l, t, radius, clamp_unit, Dl);
-      const float fl = floorf(ix);
-      const float w1 = ix - fl, w0 = 1.f - w1;
-      // a position far outside the volume (or NaN) samples zeros; clamp before the conversion to int
-      const int i0 = (int)fminf(fmaxf(fl, -2.f), (float)Dl), i1 = i0 + 1;
-      const bool in0 = i0 >= 0 && i0 < Dl && fl == (float)i0, in1 = i1 >= 0 && i1 < Dl && fl == (float)i0;
-      for (int ch = 0; ch < dim; ++ch) {
-        const float* v = lv.ptr[l] + ((size_t)(b * dim + ch) * Dl) * N1 + p;
+    for (int ch = 0; ch < dim; ++ch) {
+      const float* v = lv.ptr[l] + ((size_t)(b * dim + ch) * Dl) * N1 + p;
+      float* ol = o + (size_t)(l * dim + ch) * taps * N1;
+      auto tap = [&](int t) {
+        const float ix = lookup_position(c, l, t, radius, clamp_unit, Dl);
+        const float fl = floorf(ix);
+        const float w1 = ix - fl, w0 = 1.f - w1;
+        // a position far outside the volume (or NaN) samples zeros; clamp before the conversion to int
+        const int i0 = (int)fminf(fmaxf(fl, -2.f), (float)Dl), i1 = i0 + 1;
+        const bool in0 = i0 >= 0 && i0 < Dl && fl == (float)i0, in1 = i1 >= 0 && i1 < Dl && fl == (float)i0;
         float r = 0.f;
         if (in0) r = w0 * __ldg(v + (size_t)i0 * N1);
         if (in1) r = fmaf(w1, __ldg(v + (size_t)i1 * N1), r);
-        o[(size_t)((l * dim + ch) * taps + t) * N1] = r;
+        return r;
+      };
+      if constexpr (TAPS > 0) {
+        float r[TAPS];
+#pragma unroll
+        for (int t = 0; t < TAPS; ++t) r[t] = tap(t);
+#pragma unroll
+        for (int t = 0; t < TAPS; ++t) ol[(size_t)t * N1] = r[t];
+      } else {
+        for (int t = 0; t < taps; ++t) ol[(size_t)t * N1] = tap(t);
       }
     }
   }
@@ -120,62 +134,77 @@ __global__ void lookup_fold_kernel(const LookupLevelsMut gl, int N1, int levels)
 }
 
 // Backward in one pass for radius <= LK_RMAX: per level, the taps of a pixel touch a window of at most 2r+3
-// consecutive rows, which the thread accumulates in shared memory (its own column, no barrier); it then writes its
-// whole displacement column of the volume gradient once, folding the levels in as it goes (a level-l entry spreads
-// evenly over the 2^l level-0 entries it averaged).  No memset, no read-modify-write, no pyramid scratch.
-// grid (ceil(N1/128), B * dim)
+// consecutive rows, which one thread accumulates in shared memory (its own column); after a barrier the block's warps
+// write the whole displacement columns of its 32 pixels once, eight consecutive rows at a time, folding the levels in as
+// they go (a level-l entry spreads evenly over the 2^l level-0 entries it averaged).  No memset, no read-modify-write, no
+// pyramid scratch.  What bounds it is the write of the volume gradient, so the column is spread over the block's warps: with
+// one thread per pixel doing levels and rows in turn, 58 656 pixels (8 x 47 x 156) were too few threads to cover it.
+// grid (ceil(N1/32), B * dim), block 256.
 constexpr int LK_RMAX = 4;
 constexpr int LK_WIN = 2 * LK_RMAX + 4;
+constexpr int LK_BWARPS = 8;
+constexpr int LK_ROWS = 8;
 
-__global__ void __launch_bounds__(LK_THREADS)
+template <int TAPS>
+__global__ void __launch_bounds__(32 * LK_BWARPS)
 lookup_backward_window_kernel(const float* __restrict__ coord, long long coord_sb, const float* __restrict__ gout,
                               float* __restrict__ gcorr, int dim, int D, int N1, int levels, int radius,
                               int clamp_unit) {
-  __shared__ float win[LOOKUP_MAX_LEVELS][LK_WIN][LK_THREADS];
-  const int p = blockIdx.x * LK_THREADS + threadIdx.x, b = blockIdx.y / dim, ch = blockIdx.y - b * dim;
-  if (p >= N1) return;
-  const int tid = threadIdx.x;
-  const float c = __ldg(coord + (size_t)b * coord_sb + p);
-  const int taps = 2 * radius + 1;
-  const float* go = gout + (size_t)b * levels * dim * taps * N1 + p;
-  int wbase[LOOKUP_MAX_LEVELS], Dl[LOOKUP_MAX_LEVELS];
-  int Dcur = D;
-  for (int l = 0; l < levels; ++l, Dcur /= 2) {
-    Dl[l] = Dcur;
-    for (int s = 0; s < LK_WIN; ++s) win[l][s][tid] = 0.f;
-    for (int t = 0; t < taps; ++t) {
-      const float ix = lookup_position(c, l, t, radius, clamp_unit, Dcur);
-      const float fl = floorf(ix);
-      const float w1 = ix - fl, w0 = 1.f - w1;
-      const int i0 = (int)fminf(fmaxf(fl, -2.f), (float)Dcur);
-      if (t == 0) wbase[l] = i0;
-      const float g = __ldg(go + (size_t)((l * dim + ch) * taps + t) * N1);
-      const int s0 = i0 - wbase[l];   // positions grow with t: 0 <= s0 <= 2r+1 (+1 of rounding slack)
-      if (s0 >= 0 && s0 + 1 < LK_WIN) {
-        win[l][s0][tid] += w0 * g;      // rows outside the volume are dropped when the column is written
-        win[l][s0 + 1][tid] += w1 * g;
+  __shared__ float win[LOOKUP_MAX_LEVELS][LK_WIN][32];
+  __shared__ int wbase[LOOKUP_MAX_LEVELS][32];
+  constexpr int MAX_TAPS = TAPS > 0 ? TAPS : 2 * LK_RMAX + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane, b = blockIdx.y / dim, ch = blockIdx.y - b * dim;
+  const bool in = p < N1;
+  const int taps = TAPS > 0 ? TAPS : 2 * radius + 1;
+  const float c = in ? __ldg(coord + (size_t)b * coord_sb + p) : 0.f;
+  const float* go = gout + (size_t)b * levels * dim * taps * N1 + (in ? p : 0);
+  for (int l = warp; l < levels; l += LK_BWARPS) {
+    const int Dl = D >> l;
+    for (int s = 0; s < LK_WIN; ++s) win[l][s][lane] = 0.f;
+    const float* gl = go + (size_t)(l * dim + ch) * taps * N1;
+    float g[MAX_TAPS];
+#pragma unroll
+    for (int t = 0; t < MAX_TAPS; ++t) g[t] = (in && t < taps) ? __ldg(gl + (size_t)t * N1) : 0.f;
+    int base = 0;
+#pragma unroll
+    for (int t = 0; t < MAX_TAPS; ++t) {
+      if (t < taps) {
+        const float ix = lookup_position(c, l, t, radius, clamp_unit, Dl);
+        const float fl = floorf(ix);
+        const float w1 = ix - fl, w0 = 1.f - w1;
+        const int i0 = (int)fminf(fmaxf(fl, -2.f), (float)Dl);
+        if (t == 0) base = i0;
+        const int s0 = i0 - base;   // positions grow with t: 0 <= s0 <= 2r+1 (+1 of rounding slack)
+        if (s0 >= 0 && s0 + 1 < LK_WIN) {
+          win[l][s0][lane] += w0 * g[t];      // rows outside the volume are dropped when the column is written
+          win[l][s0 + 1][lane] += w1 * g[t];
+        }
       }
     }
+    wbase[l][lane] = base;
   }
+  __syncthreads();
+  if (!in) return;
   float* dst = gcorr + ((size_t)(b * dim + ch) * D) * N1 + p;
-  // rows below / above every level's window get no gradient: plain zero stores
-  int lo = D, hi = 0;
-  for (int l = 0; l < levels; ++l) {
-    lo = min(lo, max(wbase[l], 0) << l);
-    hi = max(hi, min((wbase[l] + LK_WIN) << l, D));
-  }
-  lo = min(lo, D);
-  for (int i = 0; i < lo; ++i) dst[(size_t)i * N1] = 0.f;
-  for (int i = max(hi, lo); i < D; ++i) dst[(size_t)i * N1] = 0.f;
-  for (int i = lo; i < max(hi, lo); ++i) {
-    float acc = 0.f, scale = 1.f;
+  for (int i0 = warp * LK_ROWS; i0 < D; i0 += LK_BWARPS * LK_ROWS) {
+    float acc[LK_ROWS];
+#pragma unroll
+    for (int r = 0; r < LK_ROWS; ++r) acc[r] = 0.f;
+    float scale = 1.f;
     for (int l = 0; l < levels; ++l, scale *= 0.5f) {
-      const int j = i >> l;
-      if (j >= Dl[l]) break;            // dropped by the floor of an odd size: no coarser level sees it either
-      const int s = j - wbase[l];
-      if (s >= 0 && s < LK_WIN) acc = fmaf(scale, win[l][s][tid], acc);
+      const int wb = wbase[l][lane], Dl = D >> l;
+      // rows i0 .. i0+7 meet entries (i0 >> l) .. ((i0 + 7) >> l) of this level
+      if ((i0 >> l) - wb >= LK_WIN || ((i0 + LK_ROWS - 1) >> l) < wb) continue;
+#pragma unroll
+      for (int r = 0; r < LK_ROWS; ++r) {
+        const int j = (i0 + r) >> l, s = j - wb;   // j >= Dl: dropped by the floor of an odd size
+        if (j < Dl && s >= 0 && s < LK_WIN) acc[r] = fmaf(scale, win[l][s][lane], acc[r]);
+      }
     }
-    dst[(size_t)i * N1] = acc;
+#pragma unroll
+    for (int r = 0; r < LK_ROWS; ++r)
+      if (i0 + r < D) dst[(size_t)(i0 + r) * N1] = acc[r];
   }
 }
 
@@ -217,8 +246,9 @@ cudaError_t launch_lookup_forward(const LookupDims& d, const float* corr, const 
   LookupLevels lv;
   fill_levels(lv, d, corr, pyramid);
   const int N1 = d.H1 * d.W1;
-  const dim3 grid((N1 + LK_THREADS - 1) / LK_THREADS, d.B);
-  lookup_forward_kernel<<<grid, LK_THREADS, 0, st>>>(lv, coord, coord_sb, out, d.dim, N1, d.levels, d.radius, clamp_unit);
+  const dim3 grid((N1 + 31) / 32, d.B);
+  auto kern = d.radius == LK_RMAX ? lookup_forward_kernel<2 * LK_RMAX + 1> : lookup_forward_kernel<0>;
+  kern<<<grid, 32 * LK_WARPS, 0, st>>>(lv, coord, coord_sb, out, d.dim, N1, d.levels, d.radius, clamp_unit);
   return cudaGetLastError();
 }
 
@@ -226,9 +256,9 @@ cudaError_t launch_lookup_backward(const LookupDims& d, const float* gout, const
                                    float* gcorr, float* gpyramid, int clamp_unit, cudaStream_t st) {
   const int N1 = d.H1 * d.W1;
   if (d.radius <= LK_RMAX) {
-    const dim3 wgrid((N1 + LK_THREADS - 1) / LK_THREADS, d.B * d.dim);
-    lookup_backward_window_kernel<<<wgrid, LK_THREADS, 0, st>>>(coord, coord_sb, gout, gcorr, d.dim, d.D, N1, d.levels,
-                                                               d.radius, clamp_unit);
+    const dim3 wgrid((N1 + 31) / 32, d.B * d.dim);
+    auto kern = d.radius == LK_RMAX ? lookup_backward_window_kernel<2 * LK_RMAX + 1> : lookup_backward_window_kernel<0>;
+    kern<<<wgrid, 32 * LK_BWARPS, 0, st>>>(coord, coord_sb, gout, gcorr, d.dim, d.D, N1, d.levels, d.radius, clamp_unit);
     return cudaGetLastError();
   }
   LookupLevelsMut gl;
