@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -238,7 +239,10 @@ struct Workspace {
   float* gm_v;
   float* at_partial;  // ... and the attention backward's per-block partial sums
   int n1p;
-  size_t bytes;
+  size_t bytes;        // without the scratch of the tail pieces, which a caller's buffer may lack (the kernels then
+  int* tail_count;     // do whole tiles only)
+  float* part;
+  size_t part_bytes;
 };
 
 int padded_pixels(const Dims& d) { return (d.N1() + TILE_M - 1) / TILE_M * TILE_M; }
@@ -255,6 +259,7 @@ PixView cf_view(const void* base, int slots, int D, int N1) {
 // What an op keeps in the workspace: the mean rows of F2, Rx packed input slots, Ro packed output slots.
 struct WsPlan { bool aux; int Rx; int Ro; int Rg; bool level_bwd; bool bf16; };
 constexpr int MAXAVG_SLOTS = 3;  // max, mean, argmax bits
+constexpr int MAXAVG_PART_SLOTS = 2;  // of a tail piece: max, argmax bits
 int chunk_channels(int Kc) { return Kc < KC_MAX_PER_SWEEP ? Kc : KC_MAX_PER_SWEEP; }
 int grad_slots(int kc) { return 2 * kc <= 4 ? 4 : 8; }  // two slots per channel, rounded up to a multiple of 4
 
@@ -318,7 +323,24 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
     w.at_partial = take(attention_partial_floats(AttentionDims{d.B, d.Kc, d.H2 > d.W2 ? d.H2 : d.W2, d.H1, d.W1}));
   }
   w.bytes = off;
+  w.tail_count = reinterpret_cast<int*>(p + WS_TAIL_OFFSET);
+  size_t part = 0;
+  if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS).part_floats);
+  if (d.Kc > 0 && plan.bf16) part = std::max(part, sweep_split(d, chunk_channels(d.Kc)).part_floats);
+  w.part = reinterpret_cast<float*>(p + off);
+  w.part_bytes = part * sizeof(float);
   return w;
+}
+
+// A sweep's cut into whole tiles and pieces, as far as the workspace has scratch for the pieces.
+void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
+  const TileSplit s = sweep_split(a.d, slots);
+  const bool cut = s.pieces > 1 && s.part_floats * sizeof(float) <= w.part_bytes;
+  a.whole_tiles = cut ? s.whole_tiles : s.tiles;
+  a.pieces = cut ? s.pieces : 1;
+  a.part_slots = slots;
+  a.part = w.part;
+  a.tail_count = w.tail_count;
 }
 
 int check_shape(const sfb_shape* s, bool need_kc, Dims* d) {
@@ -372,6 +394,7 @@ int check_workspace(const Dims& d, void* ws, size_t ws_bytes, int op, Workspace*
   *out = carve(d, ws, plan_for(op, d));
   if (ws_bytes < out->bytes)
     return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", ws_bytes, out->bytes);
+  if (ws_bytes < out->bytes + out->part_bytes) out->part_bytes = 0;
   return SFB_OK;
 }
 
@@ -468,6 +491,7 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   a.pu_arg = packed_view(w.ou, d.H2, MAXAVG_SLOTS, w.n1p, 2);
   a.pv_arg = packed_view(w.ov, d.W2, MAXAVG_SLOTS, w.n1p, 2);
   a.status = w.status;
+  set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   // packed (displacement, slot, pixel) -> the reference's (pixel, channel, displacement) tensors
   const int N1 = d.N1(), R = MAXAVG_SLOTS;
@@ -485,7 +509,7 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
 
 // ou(b,u,k,p) = sum_v S * w_u[k], ov(b,v,k,p) = sum_u S * w_v[k] for all Kc channels, at most KC_MAX_PER_SWEEP
 // channels per sweep.  Weight k is slot (slot0 + k*stride) of the views xu (per u: w_v) / xv (per v: w_u).
-int run_compress_sweeps(const Dims& d, int* status, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2, PixView xu,
+int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2, PixView xu,
                         PixView xv, int wu_slot0, int wv_slot0, int w_stride, PixView ou, PixView ov, int n_valid,
                         cudaStream_t st, int op16 = 0, const float* out_scale = nullptr) {
   for (int k0 = 0; k0 < d.Kc; k0 += KC_MAX_PER_SWEEP) {
@@ -501,7 +525,8 @@ int run_compress_sweeps(const Dims& d, int* status, const CUtensorMap& tm_f1, co
     a.ou = ou; a.ov = ov;
     a.op16 = op16;
     a.out_scale = out_scale;
-    a.status = status;
+    a.status = w.status;
+    set_sweep_split(a, w, chunk_channels(d.Kc));
     SFB_CUDA(timed(KID_SWEEP_COMPRESS, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_f2 /* unused */, st); }));
   }
   return SFB_OK;
@@ -645,7 +670,7 @@ int run_attention_grads(const Dims& d, const Workspace& w, const float* gC_u, co
     launch_pack(gC_v, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st);
     return launch_pack(gC_u, w.xu, d.B, N1, w.n1p, K, 0, K, d.H2, K, 0, 1, 0.f, st);
   }));
-  SFB_TRY(run_compress_sweeps(d, w.status, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
+  SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
                               0, 0, 1, packed_view(w.ou, d.H2, K, w.n1p), packed_view(w.ov, d.W2, K, w.n1p), w.n1p, st, op16, sweep_out_scale(w, op16)));
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
     launch_unpack(w.ou, gA_v, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st);
@@ -656,7 +681,9 @@ int run_attention_grads(const Dims& d, const Workspace& w, const float* gC_u, co
 
 // ---- scratch that lives in the library image, for callers that must not allocate ----
 constexpr size_t STATIC_SCRATCH_BYTES = 32u << 20;
-static __device__ __align__(256) unsigned char g_static_scratch[STATIC_SCRATCH_BYTES];
+// The counters of the tail tiles, which the header holds beside its first 256 bytes, come on top.
+constexpr size_t STATIC_ARRAY_BYTES = STATIC_SCRATCH_BYTES + WS_HEADER_BYTES - 256;
+static __device__ __align__(256) unsigned char g_static_scratch[STATIC_ARRAY_BYTES];
 
 constexpr int MAX_DEVICES = 64;
 std::mutex g_static_mu;
@@ -691,7 +718,8 @@ size_t sfb_workspace_bytes(int op, const sfb_shape* shape) {
                        op == SFB_OP_SEPARATION_FEATURE_BACKWARD_CF || op == SFB_OP_SEPARATION_LEVEL_FORWARD ||
                        op == SFB_OP_SEPARATION_LEVEL_BACKWARD;
   if (check_shape(shape, need_kc, &d) != SFB_OK) return 0;
-  return carve(d, nullptr, plan_for(op, d)).bytes;
+  const Workspace w = carve(d, nullptr, plan_for(op, d));
+  return w.bytes + w.part_bytes;
 }
 
 int sfb_max_avg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, const sfb_shape* shape,
@@ -707,13 +735,14 @@ int sfb_max_avg_forward_static(const float* F1, const float* F2, float* MA_u, fl
   WsPlan plan = plan_for(SFB_OP_MAX_AVG_FORWARD, d);
   plan.bf16 = false;  // this entry point always computes with TF32 operands: no room is set aside for 16-bit copies
   const size_t need = carve(d, nullptr, plan).bytes;
-  if (need > STATIC_SCRATCH_BYTES)
+  if (need > STATIC_ARRAY_BYTES)
     return fail(SFB_ERR_UNSUPPORTED_SHAPE,
                 "this shape needs %zu bytes of scratch but the built-in scratch holds %zu; use sfb_max_avg_forward "
                 "with a caller-provided workspace", need, (size_t)STATIC_SCRATCH_BYTES);
   void* scratch = nullptr;
   SFB_TRY(static_scratch(&scratch));
-  const Workspace w = carve(d, scratch, plan);
+  Workspace w = carve(d, scratch, plan);
+  if (need + w.part_bytes > STATIC_ARRAY_BYTES) w.part_bytes = 0;  // no room for the tail pieces: whole tiles only
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_f1_rows(&tm_f1, d, w.F1r, TILE_M));
@@ -730,6 +759,7 @@ int sfb_max_avg_forward_static(const float* F1, const float* F2, float* MA_u, fl
   a.pu = packed_view(w.ou, d.H2, MAXAVG_SLOTS, w.n1p);
   a.pv = packed_view(w.ov, d.W2, MAXAVG_SLOTS, w.n1p);
   a.status = w.status;
+  set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st));
   SFB_CUDA(launch_unpack(w.ou, MA_u, d.B, d.N1(), w.n1p, 2, d.H2, MAXAVG_SLOTS, 0, 1, 2, 0, st));
   SFB_CUDA(launch_unpack(w.ov, MA_v, d.B, d.N1(), w.n1p, 2, d.W2, MAXAVG_SLOTS, 0, 1, 2, 0, st));
@@ -769,7 +799,7 @@ int sfb_compression_forward(const float* F1, const float* F2, const float* A_u, 
     launch_pack(A_u, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st);         // w_u[k][v] = XV slot k
     return launch_pack(A_v, w.xu, d.B, N1, w.n1p, K, 0, K, d.H2, K, 0, 1, 0.f, st);  // w_v[k][u] = XU slot k
   }));
-  SFB_TRY(run_compress_sweeps(d, w.status, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
+  SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
                               0, 0, 1, packed_view(w.ou, d.H2, K, w.n1p), packed_view(w.ov, d.W2, K, w.n1p), w.n1p, st, op16, sweep_out_scale(w, op16)));
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
     launch_unpack(w.ou, C_u, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st);
@@ -958,6 +988,7 @@ int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v
   a.pu_arg = cf_view(AM_u, 1, d.H2, N1);
   a.pv_arg = cf_view(AM_v, 1, d.W2, N1);
   a.status = w.status;
+  set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   return SFB_OK;
 }
@@ -979,7 +1010,7 @@ static int run_compress_cf(const float* F1, const float* F2, const float* W_u, c
   SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
   const int N1 = d.N1(), K = d.Kc;
   // W_u (B,K,W2,N1) weights per v, W_v (B,K,H2,N1) per u; O_u (B,K,H2,N1), O_v (B,K,W2,N1)
-  return run_compress_sweeps(d, w.status, tm_f1, tm_f2, cf_view(W_v, K, d.H2, N1), cf_view(W_u, K, d.W2, N1), 0, 0, 1,
+  return run_compress_sweeps(d, w, tm_f1, tm_f2, cf_view(W_v, K, d.H2, N1), cf_view(W_u, K, d.W2, N1), 0, 0, 1,
                              cf_view(O_u, K, d.H2, N1), cf_view(O_v, K, d.W2, N1), N1, st, op16, sweep_out_scale(w, op16));
 }
 
@@ -1174,6 +1205,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   a.op16 = op16;
   a.out_scale = sweep_out_scale(w, op16);
   a.status = w.status;
+  set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
   SFB_CUDA(timed(KID_ATTENTION_FWD, 2 * ((K + 3) / 4 + 1), st, [&] {
@@ -1183,7 +1215,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
                                     weight_v, bias_v, A_v, st, w.status);
   }));
   // C_u (per u, weights A_u per v) -> SEP_v channels 2.., C_v -> SEP_u channels 2..
-  return run_compress_sweeps(d, w.status, tm_f1, tm_f2, cf_view(A_v, K, d.H2, N1), cf_view(A_u, K, d.W2, N1), 0, 0, 1,
+  return run_compress_sweeps(d, w, tm_f1, tm_f2, cf_view(A_v, K, d.H2, N1), cf_view(A_u, K, d.W2, N1), 0, 0, 1,
                              cf_channels(SEP_v, Kt, c0 + 2, d.H2, N1), cf_channels(SEP_u, Kt, c0 + 2, d.W2, N1), N1, st,
                              op16, sweep_out_scale(w, op16));
 }
@@ -1237,7 +1269,7 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
   // attention gradients: gA_v(b,k,u,p) = sum_v S * gC_v(b,k,v,p), gA_u(b,k,v,p) = sum_u S * gC_u(b,k,u,p), with
   // gC_u = gSEP_v[:, 2:] (per u) and gC_v = gSEP_u[:, 2:] (per v) in the role of the weights
-  SFB_TRY(run_compress_sweeps(d, w.status, tm_f1, tm_f2, cf_channels(gSEP_v, Kt, c0 + 2, d.H2, N1),
+  SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, cf_channels(gSEP_v, Kt, c0 + 2, d.H2, N1),
                               cf_channels(gSEP_u, Kt, c0 + 2, d.W2, N1), 0, 0, 1, cf_view(w.ga_v, K, d.H2, N1),
                               cf_view(w.ga_u, K, d.W2, N1), N1, st, op16, sweep_out_scale(w, op16)));
   // through softmax and Conv3d: parameter gradients, and the total gradients of the max/avg channels
@@ -1454,6 +1486,8 @@ int sfb_corr_volume(const float* F1, const float* F2, float* S, const sfb_shape*
   a.n_valid = w.n1p;
   a.dump = S;
   a.status = w.status;
+  a.whole_tiles = d.B * ((d.N1() + TILE_M - 1) / TILE_M);
+  a.pieces = 1;
   SFB_CUDA(timed(KID_SWEEP_DUMP, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_f2 /* unused */, st); }));
   return SFB_OK;
 }

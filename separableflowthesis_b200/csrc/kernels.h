@@ -93,7 +93,18 @@ struct SweepArgs {
   int* status;           // device status word
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
   int drop_last_load;    // test hook: the producer leaves out its last F2 block, so that one wait runs out
+  // Tiles past `whole_tiles` are done by `pieces` CTAs each (TileSplit); part / tail_count are unused when pieces is 1.
+  int whole_tiles, pieces, part_slots;
+  float* part;
+  int* tail_count;       // one zero per tail tile; every launch leaves them zero
 };
+
+// How a launch of equal tiles fills the SMs: whole_tiles CTAs do one tile each, every further tile is done by `pieces`
+// CTAs, which need part_floats floats of scratch.
+constexpr int SM_COUNT = 148;
+constexpr int MAX_PIECES = 16;
+struct TileSplit { int tiles, whole_tiles, pieces; size_t part_floats; };
+TileSplit sweep_split(const Dims& d, int slots);  // slots: row results per pixel (max and argmax; channels of a launch)
 
 // Gradient GEMM.  G = dLoss/dS is generated from two "interleaved" operand sets: for every displacement
 // and image-1 pixel the R4 values (slots) that pixel contributes, in groups of four:
@@ -149,7 +160,9 @@ cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, i
 
 // Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, all cleared by
 // launch_prepare.  amax slots hold float bits (atomicMax), the others floats; every scale is a power of two.
-constexpr size_t WS_HEADER_BYTES = 256, WS_SCALES_OFFSET = 64, WS_HEADER_CLEAR_BYTES = 128;
+// From WS_TAIL_OFFSET on, SM_COUNT counters of the tail tiles (SweepArgs::tail_count).
+constexpr size_t WS_HEADER_BYTES = 1024, WS_SCALES_OFFSET = 64, WS_TAIL_OFFSET = 256, WS_HEADER_CLEAR_BYTES = 1024;
+static_assert(WS_TAIL_OFFSET + SM_COUNT * sizeof(int) <= WS_HEADER_CLEAR_BYTES, "tail counters");
 enum : int {
   SCALE_AMAX_F1 = 0, SCALE_AMAX_F2 = 1, SCALE_AMAX_G = 2, SCALE_AMAX_A = 3,
   SCALE_F1 = 4, SCALE_F2 = 5, SCALE_INV_F1F2 = 6,   // F1h = fp16(s1 F1), F2h = fp16(s2 F2), sweep outputs * 1/(s1 s2)

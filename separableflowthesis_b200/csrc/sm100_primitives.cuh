@@ -374,6 +374,29 @@ __device__ __forceinline__ float sum2(uint64_t v) {
   return lo + hi;
 }
 
+// Four consecutive floats of which the first n exist (n < 1: none), as one 16-byte access when all do and the address allows
+// it.  Loads bypass L1, so that they see what other SMs stored.
+__device__ __forceinline__ float4 load4_cg(const float* p, int n) {
+  if (n >= 4 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) return __ldcg(reinterpret_cast<const float4*>(p));
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (n > 0) v.x = __ldcg(p);
+  if (n > 1) v.y = __ldcg(p + 1);
+  if (n > 2) v.z = __ldcg(p + 2);
+  if (n > 3) v.w = __ldcg(p + 3);
+  return v;
+}
+__device__ __forceinline__ void store4(float* p, const float4& v, int n) {
+  if (n >= 4 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+    *reinterpret_cast<float4*>(p) = v;
+    return;
+  }
+  if (n > 0) p[0] = v.x;
+  if (n > 1) p[1] = v.y;
+  if (n > 2) p[2] = v.z;
+  if (n > 3) p[3] = v.w;
+}
+__device__ __forceinline__ void add4(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+
 // Byte offset of element (row, col) inside a [rows][32 fp32] tile stored with the 128-byte swizzle
 // (16-byte chunk index XOR row mod 8); the tile base must be 1024-byte aligned.
 __device__ __forceinline__ uint32_t sw128_offset(int row, int col) {

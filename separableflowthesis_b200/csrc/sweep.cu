@@ -17,6 +17,10 @@
 //                  once per column block), row-direction max(+argmax) merged through the packed output
 //                  once per tile.  The two mean channels come from extra tiles whose "image-2 pixels"
 //                  are the row-mean and column-mean feature rows of F2 (mean_v S[u,v] = F1 . mean_v F2[u,v]).
+// Tail tiles: a grid that is not a multiple of 148 tiles leaves SMs idle in its last wave (and a single 55 x 128 pair has
+// 55 tiles in all), so the tiles past the last full wave are cut into `pieces` CTAs, each a range of column blocks.  Column
+// results are complete within a piece; row results of pieces 1.. go to scratch, and the CTA that finishes a tile last (a
+// counter per tile, nobody waits) folds them into piece 0's results in piece order, so the result does not depend on timing.
 //   compression  : group g takes channel g.  OU[k,u] = sum_v S*w_u[k,v] (reduced per tile, accumulated
 //                  with red.add), OV[k,v] = sum_u S*w_v[k,u] (register accumulators across the inner loop).
 // Replaces the reference kernels MemorySaver_kernel_forward.cu:128-313, :328-533, :550-753.
@@ -55,13 +59,22 @@ struct SweepSmem {
   uint64_t acc_empty[SW_NACC];
   uint64_t merge[SW_NMERGE];              // group 1 -> group 0: partial column results are in memory
   uint32_t tmem_base;
+  int last_piece;                         // this CTA finished its tail tile last: it folds the pieces together
   WaitCtl ctl;
 };
 constexpr size_t SW_SMEM_BYTES = sizeof(SweepSmem) + 1024;  // + slack to align the base to 1024 B
 
 struct SweepSched {
-  int b, m0, nkb, n_ub, n_vb, t_main, t_total;
+  int b, m0, nkb, n_ub;
+  int vb0;              // first column block of this CTA
+  int t_main, t_total;  // tiles of its column blocks; the same plus the tiles of the mean rows
+  int tail, piece;      // tail tile this CTA has a piece of (-1: a whole tile) and which piece
 };
+
+// Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][slot][row u][128 pixels]
+__device__ __forceinline__ float* sweep_part(const SweepArgs& a, int tail, int piece, int slot) {
+  return a.part + (((size_t)tail * (a.pieces - 1) + piece - 1) * a.part_slots + slot) * a.d.H2 * TILE_M;
+}
 
 // ---------------------------------------------------------------------------------- producer
 __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const CUtensorMap* tm_f1,
@@ -70,7 +83,7 @@ __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSch
   mbar_expect_tx(&sm.f1_full, sc.nkb * SW_F1_BLOCK_BYTES);
   for (int kb = 0; kb < sc.nkb; ++kb) tma_load_3d(sm.f1[kb], tm_f1, &sm.f1_full, kb * kel, sc.m0, sc.b);
   uint32_t it = 0;
-  int vb = 0, ub = 0;
+  int vb = sc.vb0, ub = 0;
   for (int t = 0; t < sc.t_total; ++t) {
     const bool main_tile = t < sc.t_main;
     for (int kb = 0; kb < sc.nkb; ++kb, ++it) {
@@ -169,14 +182,21 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
   // per-thread views: value of (displacement d, slot) at ptr[d*sd + slot*ss]
   float* pu = a.pu.base + sc.b * a.pu.sb + e.p;
   float* pv = a.pv.base + sc.b * a.pv.sb + e.p;
+  float* pum = pu + a.pu.ss;   // the mean channel: written by one piece, straight to its place
   float* pua = ARG ? a.pu_arg.base + sc.b * a.pu_arg.sb + e.p : nullptr;
   float* pva = ARG ? a.pv_arg.base + sc.b * a.pv_arg.sb + e.p : nullptr;
-  const uint32_t usd = a.pu.sd, uss = a.pu.ss, vsd = a.pv.sd, vss = a.pv.ss, uasd = a.pu_arg.sd, vasd = a.pv_arg.sd;
+  uint32_t usd = a.pu.sd, uasd = a.pu_arg.sd;
+  const uint32_t umsd = a.pu.sd, vsd = a.pv.sd, vss = a.pv.ss, vasd = a.pv_arg.sd;
+  if (sc.piece > 0) {          // row maxima of a later piece: scratch slots 0 (value) and 1 (arg-max)
+    pu = sweep_part(a, sc.tail, sc.piece, 0) + (e.p - sc.m0);
+    if (ARG) pua = sweep_part(a, sc.tail, sc.piece, 1) + (e.p - sc.m0);
+    usd = uasd = TILE_M;
+  }
   const bool valid = e.valid;
 
   float cm[SWEEP_VT];
   int ca[SWEEP_VT];
-  int vb = 0, ub = 0;
+  int vb = sc.vb0, ub = 0;
   for (int t = 0; t < sc.t_main; ++t) {
     const int v0 = vb * SWEEP_VT, ubase = ub * SWEEP_UT + e.wg * SW_RW;
     const int nu = min(SW_RW, H2 - ubase), nv = min(SWEEP_VT, W2 - v0);  // nu may be <= 0
@@ -188,7 +208,7 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
     float rold[SW_RW];
 #pragma unroll
     for (int ul = 0; ul < SW_RW; ++ul)
-      rold[ul] = (valid && vb > 0 && ul < nu) ? pu[(ubase + ul) * usd] : -CUDART_INF_F;
+      rold[ul] = (valid && vb > sc.vb0 && ul < nu) ? pu[(ubase + ul) * usd] : -CUDART_INF_F;
 
     if (!epi_wait(sm, a, t)) return;
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * (SW_RW * SWEEP_VT);
@@ -225,7 +245,7 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
             for (int j = 0; j < SWEEP_VT; ++j) cm[j] = fmaxf(cm[j], r[j]);
           }
           m *= e.osc;  // memory holds scaled-back values; compare and store in that domain
-          if (valid && (vb == 0 || m > rold[ul])) {  // strict: the lowest column block wins ties
+          if (valid && (vb == sc.vb0 || m > rold[ul])) {  // strict: the lowest column block wins ties
             pu[u * usd] = m;
             if (ARG) pua[u * uasd] = __int_as_float(v0 + arg);
           }
@@ -234,7 +254,7 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
     }
     if (ub == sc.n_ub - 1) {
       // end of a column block: group 1 publishes its partial column maxima, group 0 merges and stores
-      uint64_t* bar = &sm.merge[vb % SW_NMERGE];
+      uint64_t* bar = &sm.merge[(vb - sc.vb0) % SW_NMERGE];
       if (e.wg == 1) {
 #pragma unroll
         for (int j = 0; j < SWEEP_VT; ++j) {
@@ -247,7 +267,7 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
         __syncwarp();
         if (e.lane == 0) mbar_arrive(bar);
       } else {
-        const bool ok = mbar_wait(bar, (vb / SW_NMERGE) & 1u, &sm.ctl, a.status, DEV_TIMEOUT_EPILOGUE);
+        const bool ok = mbar_wait(bar, ((vb - sc.vb0) / SW_NMERGE) & 1u, &sm.ctl, a.status, DEV_TIMEOUT_EPILOGUE);
         if (!__all_sync(0xffffffffu, ok)) return;
 #pragma unroll
         for (int j = 0; j < SWEEP_VT; ++j) {
@@ -286,7 +306,7 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
         for (int j = 0; j < 64; ++j) {
           const int r = r0 + j;
           if (!valid) continue;
-          if (r < H2) pu[r * usd + uss] = s[j] * e.osc;
+          if (r < H2) pum[r * umsd] = s[j] * e.osc;
           else if (r < naux) pv[(r - H2) * vsd + vss] = s[j] * e.osc;
         }
       }
@@ -299,13 +319,18 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
   const int H2 = a.d.H2, W2 = a.d.W2;
   const bool active = e.wg < a.kc;            // this warpgroup's channel exists (warp-uniform)
   const bool valid = e.valid && active;
-  const uint32_t xusd = a.xu.sd, xvsd = a.xv.sd, ousd = a.ou.sd, ovsd = a.ov.sd;
+  const uint32_t xusd = a.xu.sd, xvsd = a.xv.sd, ovsd = a.ov.sd;
+  uint32_t ousd = a.ou.sd;
   // this thread's pixel and channel in sample b of each view; displacement d at ptr[d*sd], 32-bit offsets
   const int k = a.k0 + e.wg;
   const float* wu = a.xv.base + sc.b * a.xv.sb + e.p + (a.wu_slot0 + k * a.w_stride) * a.xv.ss;  // w_u[k][v]
   const float* wv = a.xu.base + sc.b * a.xu.sb + e.p + (a.wv_slot0 + k * a.w_stride) * a.xu.ss;  // w_v[k][u]
   float* ou = a.ou.base + sc.b * a.ou.sb + e.p + k * a.ou.ss;
   float* ov = a.ov.base + sc.b * a.ov.sb + e.p + k * a.ov.ss;
+  if (sc.piece > 0 && active) {  // row sums of a later piece: scratch slot = channel of this launch
+    ou = sweep_part(a, sc.tail, sc.piece, e.wg) + (e.p - sc.m0);
+    ousd = TILE_M;
+  }
 
   // Both sums run on packed FP32 pairs (two neighbouring columns per fma.rn.f32x2), which halves the
   // instructions per cell: the epilogue warps share their schedulers' issue slots, and with scalar FMAs
@@ -315,7 +340,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
   // Cells outside the image hold S = 0 (TMA zero-fills the missing F2 rows) and get weight 0, so every
   // tile is processed whole and only the loads and stores at the edges are predicated.
   uint64_t au2[SWEEP_VT / 2], cv2[SWEEP_VT / 2];
-  int vb = 0, ub = 0;
+  int vb = sc.vb0, ub = 0;
   for (int t = 0; t < sc.t_main; ++t) {
     const int v0 = vb * SWEEP_VT, u0 = ub * SWEEP_UT;
     const int nu = min(SWEEP_UT, H2 - u0), nv = min(SWEEP_VT, W2 - v0);
@@ -340,7 +365,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N;
     if (active) {
       float* ou_t = ou + u0 * ousd;
-      const bool first = vb == 0;  // the first column block initialises the output, later ones accumulate
+      const bool first = vb == sc.vb0;  // the first column block initialises the output, later ones accumulate
 #pragma unroll
       for (int pr = 0; pr < SWEEP_UT / 2; ++pr) {
         float s[2 * SWEEP_VT];
@@ -412,8 +437,81 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
   }
 }
 
-// ---------------------------------------------------------------------------------- kernel
+// Pieces 1.. of a finished tail tile folded into piece 0's row results, in piece order (all threads of the CTA that
+// finished last).  Maxima: a later piece has the higher columns, so only a strictly larger value replaces.  One SM's loads
+// are all that moves these bytes, so a thread takes four pixels of up to FOLD_ROWS rows at once and asks for all pieces'
+// values before it uses any (with one 4-byte load at a time a fold of 135 rows x 4 channels took as long as the sweep).
+__device__ __forceinline__ void max4_first(float& v, float& arg, float o, float oarg) {
+  if (o > v) { v = o; arg = oarg; }
+}
 template <int MODE>
+__device__ void sweep_fold_pieces(const SweepArgs& a, const SweepSched& sc) {
+  constexpr int NT = sw_threads(MODE), QUADS = TILE_M / 4, FOLD_ROWS = MODE == SWEEP_MAXARGAVG ? 2 : 4, FOLD_PIECES = 2;
+  const int H2 = a.d.H2, n = (MODE == SWEEP_COMPRESS ? a.kc : 1) * H2 * QUADS;
+  for (int i0 = threadIdx.x; i0 < n; i0 += FOLD_ROWS * NT) {
+    float* dst[FOLD_ROWS];
+    float* arg_dst[FOLD_ROWS];
+    const float* part[FOLD_ROWS];   // piece 1's values; piece s is (s - 1) * part_slots slots further on
+    int cnt[FOLD_ROWS];
+    float4 v[FOLD_ROWS], va[FOLD_ROWS];
+#pragma unroll
+    for (int r = 0; r < FOLD_ROWS; ++r) {
+      const int i = i0 + r * NT, px = i % QUADS * 4, q = i / QUADS, k = q / H2, u = q - k * H2, p = sc.m0 + px;
+      cnt[r] = i < n ? min(4, a.n_valid - p) : 0;
+      if (cnt[r] <= 0) { cnt[r] = 0; dst[r] = arg_dst[r] = nullptr; part[r] = a.part; continue; }
+      if (MODE == SWEEP_COMPRESS) dst[r] = a.ou.base + sc.b * a.ou.sb + p + (a.k0 + k) * a.ou.ss + u * a.ou.sd;
+      else dst[r] = a.pu.base + sc.b * a.pu.sb + p + u * a.pu.sd;
+      arg_dst[r] = MODE == SWEEP_MAXARGAVG ? a.pu_arg.base + sc.b * a.pu_arg.sb + p + u * a.pu_arg.sd : nullptr;
+      part[r] = sweep_part(a, sc.tail, 1, k) + (size_t)u * TILE_M + px;
+      v[r] = load4_cg(dst[r], cnt[r]);
+      if (MODE == SWEEP_MAXARGAVG) va[r] = load4_cg(arg_dst[r], cnt[r]);
+    }
+    const size_t slot = (size_t)H2 * TILE_M, step = slot * a.part_slots;
+    for (int s0 = 1; s0 < a.pieces; s0 += FOLD_PIECES) {
+      float4 o[FOLD_PIECES][FOLD_ROWS], oa[MODE == SWEEP_MAXARGAVG ? FOLD_PIECES : 1][FOLD_ROWS];
+#pragma unroll
+      for (int j = 0; j < FOLD_PIECES; ++j)
+#pragma unroll
+        for (int r = 0; r < FOLD_ROWS; ++r) {
+          const bool ok = s0 + j < a.pieces && cnt[r] > 0;
+          const float* src = part[r] + (s0 + j - 1) * step;
+          // lanes past the image were never written: their values are loaded and dropped
+          o[j][r] = ok ? __ldcg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (MODE == SWEEP_MAXARGAVG)
+            oa[j][r] = ok ? __ldcg(reinterpret_cast<const float4*>(src + slot)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+      for (int j = 0; j < FOLD_PIECES; ++j) {
+        if (s0 + j >= a.pieces) break;
+#pragma unroll
+        for (int r = 0; r < FOLD_ROWS; ++r) {
+          if (MODE == SWEEP_COMPRESS) {
+            add4(v[r], o[j][r]);
+          } else if (MODE == SWEEP_MAXARGAVG) {
+            max4_first(v[r].x, va[r].x, o[j][r].x, oa[j][r].x);
+            max4_first(v[r].y, va[r].y, o[j][r].y, oa[j][r].y);
+            max4_first(v[r].z, va[r].z, o[j][r].z, oa[j][r].z);
+            max4_first(v[r].w, va[r].w, o[j][r].w, oa[j][r].w);
+          } else {
+            v[r] = make_float4(o[j][r].x > v[r].x ? o[j][r].x : v[r].x, o[j][r].y > v[r].y ? o[j][r].y : v[r].y,
+                               o[j][r].z > v[r].z ? o[j][r].z : v[r].z, o[j][r].w > v[r].w ? o[j][r].w : v[r].w);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < FOLD_ROWS; ++r) {
+      if (cnt[r] == 0) continue;
+      store4(dst[r], v[r], cnt[r]);
+      if (MODE == SWEEP_MAXARGAVG) store4(arg_dst[r], va[r], cnt[r]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------- kernel
+// CUT: the launch has tail pieces.  A launch without any runs the kernel without their bookkeeping, whose registers cost
+// the compression epilogue 10 % (it is at its register limit: 897 -> 990 us at 135 x 240).
+template <int MODE, bool CUT>
 __global__ void __launch_bounds__(sw_threads(MODE), 1)
 sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ CUtensorMap tm_f2,
              const __grid_constant__ CUtensorMap tm_aux, const SweepArgs a) {
@@ -427,14 +525,27 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
 
   SweepSched sc;
-  sc.b = blockIdx.x / tiles_per_sample;
-  sc.m0 = (blockIdx.x - sc.b * tiles_per_sample) * TILE_M;
+  int tile = blockIdx.x;
+  sc.tail = -1;
+  sc.piece = 0;
+  if (CUT && tile >= a.whole_tiles) {  // pieces of the tail tiles follow the whole tiles
+    const int r = tile - a.whole_tiles;
+    sc.tail = r / a.pieces;
+    sc.piece = r - sc.tail * a.pieces;
+    tile = a.whole_tiles + sc.tail;
+  }
+  sc.b = tile / tiles_per_sample;
+  sc.m0 = (tile - sc.b * tiles_per_sample) * TILE_M;
   sc.nkb = a.op16 ? (a.d.C + 2 * KBLK - 1) / (2 * KBLK) : (a.d.C + KBLK - 1) / KBLK;
   sc.n_ub = (a.d.H2 + SWEEP_UT - 1) / SWEEP_UT;
-  sc.n_vb = (a.d.W2 + SWEEP_VT - 1) / SWEEP_VT;
-  sc.t_main = sc.n_ub * sc.n_vb;
+  const int n_vb = (a.d.W2 + SWEEP_VT - 1) / SWEEP_VT;
+  const int n_pieces = CUT && sc.tail >= 0 ? a.pieces : 1;
+  const int per = n_vb / n_pieces, extra = n_vb - per * n_pieces;  // the first `extra` pieces have one block more
+  sc.vb0 = sc.piece * per + min(sc.piece, extra);
+  sc.t_main = sc.n_ub * (per + (sc.piece < extra ? 1 : 0));
   const bool has_aux = (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG);
-  sc.t_total = sc.t_main + (has_aux ? (a.d.H2 + a.d.W2 + SW_TILE_N - 1) / SW_TILE_N : 0);
+  const bool does_aux = has_aux && sc.piece == n_pieces - 1;       // the mean rows go to the last, smallest piece
+  sc.t_total = sc.t_main + (does_aux ? (a.d.H2 + a.d.W2 + SW_TILE_N - 1) / SW_TILE_N : 0);
 
   if (threadIdx.x == 0) {
     mbar_init(&sm.f1_full, 1);
@@ -488,32 +599,76 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     tc_fence_after();
     tmem_dealloc(sm.tmem_base, SW_TMEM_COLS);
   }
+  if (n_pieces > 1 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
+    __threadfence();  // this thread's results before the count ...
+    __syncthreads();
+    if (threadIdx.x == 0) sm.last_piece = atomicAdd(a.tail_count + sc.tail, 1) == n_pieces - 1;
+    __syncthreads();
+    if (sm.last_piece) {
+      __threadfence();  // ... and the count before the other pieces' results
+      sweep_fold_pieces<MODE>(a, sc);
+      if (threadIdx.x == 0) a.tail_count[sc.tail] = 0;  // as the next launch expects it
+    }
+  }
 }
 
-template <int MODE>
+// How the tail tiles are cut, in units of one 256-column tile's time: a CTA costs about two tiles of prologue, a fold
+// reads pieces * slots * H2 rows of 128 values through one SM (about 677 rows per tile time).  Pieces must save a quarter
+// of the tail and a whole tile to be used: a wave with idle SMs runs its tiles faster than a full one, so little is left of
+// smaller predicted savings (106 tail tiles of 135 x 240 in four pieces, predicted 0.86: max/avg sweep 588 -> 551 us, but
+// the compression sweep no faster; 55 tiles of 55 x 128 in two pieces, predicted 0.56: 108 -> 76 and 86 -> 58 us).
+TileSplit sweep_split(const Dims& d, int slots) {
+  const long long tiles = (long long)d.B * ((d.N1() + TILE_M - 1) / TILE_M);
+  const int n_ub = (d.H2 + SWEEP_UT - 1) / SWEEP_UT, n_vb = (d.W2 + SWEEP_VT - 1) / SWEEP_VT;
+  const int rest = (int)(tiles % SM_COUNT);
+  TileSplit r{(int)tiles, (int)tiles, 1, 0};
+  if (rest == 0) return r;
+  double best = 0, whole = 0;
+  for (int n = 1; n <= n_vb && n <= MAX_PIECES; ++n) {
+    const double waves = (rest * n + SM_COUNT - 1) / SM_COUNT;
+    const double cost = waves * ((n_vb + n - 1) / n * n_ub + 2) + (n > 1 ? n * (double)slots * d.H2 / 677.0 + 0.5 : 0.0);
+    if (n == 1) best = whole = cost;
+    if (cost < best && cost < 0.75 * whole && cost < whole - 1) { best = cost; r.pieces = n; }
+  }
+  if (r.pieces > 1) {
+    r.whole_tiles = (int)tiles - rest;
+    r.part_floats = (size_t)rest * (r.pieces - 1) * slots * d.H2 * TILE_M;
+  }
+  return r;
+}
+
+template <int MODE, bool CUT>
 static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                               const CUtensorMap& tm_aux, cudaStream_t stream) {
-  auto kern = sweep_kernel<MODE>;
+  auto kern = sweep_kernel<MODE, CUT>;
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM_BYTES);
   });
   if (err != cudaSuccess) return err;
   const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
-  const dim3 grid(a.d.B * tiles_per_sample);
+  const int tiles = a.d.B * tiles_per_sample;
+  const dim3 grid(a.whole_tiles + (tiles - a.whole_tiles) * a.pieces);
   kern<<<grid, sw_threads(MODE), SW_SMEM_BYTES, stream>>>(tm_f1, tm_f2, tm_aux, a);
   return cudaGetLastError();
+}
+
+template <int MODE>
+static cudaError_t launch_mode(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
+                               const CUtensorMap& tm_aux, cudaStream_t stream) {
+  return a.pieces > 1 ? launch_one<MODE, true>(a, tm_f1, tm_f2, tm_aux, stream)
+                      : launch_one<MODE, false>(a, tm_f1, tm_f2, tm_aux, stream);
 }
 
 cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                          const CUtensorMap& tm_aux, cudaStream_t stream) {
   switch (a.mode) {
-    case SWEEP_MAXAVG: return launch_one<SWEEP_MAXAVG>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_MAXARGAVG: return launch_one<SWEEP_MAXARGAVG>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_DUMP: return launch_one<SWEEP_DUMP>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_MAXAVG: return launch_mode<SWEEP_MAXAVG>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_MAXARGAVG: return launch_mode<SWEEP_MAXARGAVG>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_DUMP: return launch_one<SWEEP_DUMP, false>(a, tm_f1, tm_f2, tm_aux, stream);
     case SWEEP_COMPRESS:
       if (a.kc < 1 || a.kc > KC_MAX_PER_SWEEP) return cudaErrorInvalidValue;
-      return launch_one<SWEEP_COMPRESS>(a, tm_f1, tm_f2, tm_aux, stream);
+      return launch_mode<SWEEP_COMPRESS>(a, tm_f1, tm_f2, tm_aux, stream);
     default: return cudaErrorInvalidValue;
   }
 }
