@@ -327,6 +327,7 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   size_t part = 0;
   if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS).part_floats);
   if (d.Kc > 0 && plan.bf16) part = std::max(part, sweep_split(d, chunk_channels(d.Kc)).part_floats);
+  if (plan.Rg) part = std::max(part, std::max(grad_split(d, 0).part_floats, grad_split(d, 1).part_floats));
   w.part = reinterpret_cast<float*>(p + off);
   w.part_bytes = part * sizeof(float);
   return w;
@@ -339,6 +340,16 @@ void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
   a.whole_tiles = cut ? s.whole_tiles : s.tiles;
   a.pieces = cut ? s.pieces : 1;
   a.part_slots = slots;
+  a.part = w.part;
+  a.tail_count = w.tail_count;
+}
+
+// The same for a gradient GEMM.
+void set_grad_split(GradArgs& a, const Workspace& w) {
+  const TileSplit s = grad_split(a.d, a.image2_major);
+  const bool cut = s.pieces > 1 && s.part_floats * sizeof(float) <= w.part_bytes;
+  a.whole_tiles = cut ? s.whole_tiles : s.tiles;
+  a.pieces = cut ? s.pieces : 1;
   a.part = w.part;
   a.tail_count = w.tail_count;
 }
@@ -581,6 +592,7 @@ int run_grad_pair(const Dims& d, const Workspace& w, int mode, int R4, int accum
   a.out = gF1;
   a.out_scale = scale1;
   a.dev_scale = op16 == OP16_FP16 ? w.scales + SCALE_INV_GF1 : nullptr;
+  set_grad_split(a, w);
   SFB_CUDA(timed(kid, 1, st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xu /* unused */, st); }));
   // gF2 = G^T * F1 : rows are an 8 x 16 block of image-2 pixels, the K sweep streams 32 pixels of F1, XU and XV.
   {  // (N1, C, B) with rows padded to n1p; box = 32 pixels x all channels
@@ -594,6 +606,7 @@ int run_grad_pair(const Dims& d, const Workspace& w, int mode, int R4, int accum
   a.out = gF2;
   a.out_scale = 1.f;
   a.dev_scale = op16 == OP16_FP16 ? w.scales + SCALE_INV_GF2 : nullptr;
+  set_grad_split(a, w);
   SFB_CUDA(timed(kid + 1, 1, st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xv, st); }));
   return SFB_OK;
 }

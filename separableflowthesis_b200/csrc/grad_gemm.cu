@@ -30,6 +30,10 @@
 // 16-bit (64-byte rows, 64-byte swizzle), so a block is two instructions of K = 16 instead of four of K = 8.
 // Accumulation stays FP32.  With FP16 the operands carry power-of-two scales (kernels.h, SCALE_*) that the drain undoes.
 //
+// Tail tiles: like the correlation sweeps, the tiles past the last full wave of 148 CTAs are cut into `pieces` CTAs, each
+// a range of the K sweep.  Piece 0 drains to the output, the others to scratch, and the CTA that finishes a tile last
+// (a counter per tile, nobody waits) adds them to the output in piece order: deterministic.
+//
 // Warp roles: warp 0 feature (B operand) producer, warp 1 TMEM allocation + MMA issue, warps 2..9 generate G
 // and, at the end, drain the accumulator (two warps per TMEM lane quarter, alternating 16-column chunks),
 // warp 10 producer of the XU / XV blocks.
@@ -86,11 +90,14 @@ struct GradSmem {
   uint64_t xv_empty[Cfg::NXV];
   uint64_t acc_full;
   uint32_t tmem_base;
+  int last_piece;                             // this CTA finished its tail tile last: it adds the pieces up
   WaitCtl ctl;
 };
 
 struct GradSched {
-  int b, nkb, n_blocks;
+  int b, nkb;
+  int t0, n_blocks;  // first block of the K sweep this CTA does, and how many
+  int tail, piece;   // tail tile this CTA has a piece of (-1: a whole tile) and which piece
   int m0;            // image-1-major: first pixel of the row tile
   int u0, v0;        // image-2-major: origin of the 8 x 16 row tile
   int n_ub2;         // image-1-major: number of 2-row blocks along u
@@ -166,12 +173,12 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
   // (BF16: two values per column, so the thread's 8 values of a row are 4 columns)
   const uint32_t ta0 = sm.tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + GG_ACC_COLS +
                        vh * (BF16 ? GG_VH / 2 : GG_VH);
-  int vb = 0, ub2 = 0;
+  int vb = sc.t0 / sc.n_ub2, ub2 = sc.t0 - vb * sc.n_ub2;
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t so = t % Cfg::NXU, pho = (t / Cfg::NXU) & 1u;
     const uint32_t s = t % Cfg::NG, ph = (t / Cfg::NG) & 1u;
     const int vbase = vb * GG_VT + vh * GG_VH;
-    if (ub2 == 0) {
+    if (ub2 == 0 || t == 0) {
 #pragma unroll
       for (int i = 0; i < GG_VH; ++i)
         xv[i].load_global(xv_p + (size_t)(vbase + i) * row_stride, group_stride, vbase + i < W2);
@@ -306,6 +313,7 @@ __device__ void feature_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, co
                                  const CUtensorMap* tm_y) {
   using Cfg = GradCfg<Q, I2MAJOR>;
   int vb = 0, ub2 = 0;
+  if (I2MAJOR == 0) { vb = sc.t0 / sc.n_ub2; ub2 = sc.t0 - vb * sc.n_ub2; }
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t s = t % Cfg::NY, ph = (t / Cfg::NY) & 1u;
     if (!mbar_wait(&sm.y_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
@@ -314,7 +322,7 @@ __device__ void feature_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, co
       tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (vb * sc.h2p + ub2 * GG_UT) * GG_VT, 0, sc.b);
       if (++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
     } else {
-      tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], t * GG_KJ, 0, sc.b);
+      tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (sc.t0 + t) * GG_KJ, 0, sc.b);
     }
   }
 }
@@ -326,7 +334,7 @@ __device__ void operand_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, co
                                  const CUtensorMap* tm_xu, const CUtensorMap* tm_xv) {
   using Cfg = GradCfg<Q, I2MAJOR>;
   using Smem = GradSmem<Q, I2MAJOR>;
-  int ub2 = 0;
+  int ub2 = I2MAJOR == 0 ? sc.t0 % sc.n_ub2 : 0;
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t su = t % Cfg::NXU, phu = (t / Cfg::NXU) & 1u;
     if (!mbar_wait(&sm.xu_empty[su], phu ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
@@ -336,11 +344,11 @@ __device__ void operand_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, co
       tma_load_4d(sm.xu[su] + Smem::XU_FLOATS / 2, tm_xu, &sm.xu_full[su], (sc.m0 + 64) * 4, 0, ub2 * GG_UT, sc.b);
       if (++ub2 == sc.n_ub2) ub2 = 0;
     } else {
-      tma_load_4d(sm.xu[su], tm_xu, &sm.xu_full[su], t * GG_KJ * 4, 0, sc.u0, sc.b);
+      tma_load_4d(sm.xu[su], tm_xu, &sm.xu_full[su], (sc.t0 + t) * GG_KJ * 4, 0, sc.u0, sc.b);
       const uint32_t sv = t % Cfg::NXV, phv = (t / Cfg::NXV) & 1u;
       if (!mbar_wait(&sm.xv_empty[sv], phv ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
       mbar_expect_tx(&sm.xv_full[sv], Smem::XV_FLOATS * 4);
-      tma_load_4d(sm.xv[sv], tm_xv, &sm.xv_full[sv], t * GG_KJ * 4, 0, sc.v0, sc.b);
+      tma_load_4d(sm.xv[sv], tm_xv, &sm.xv_full[sv], (sc.t0 + t) * GG_KJ * 4, 0, sc.v0, sc.b);
     }
   }
 }
@@ -385,6 +393,29 @@ __device__ void grad_mma(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Grad
   umma_commit(&sm.acc_full);
 }
 
+// Where output row m of this CTA's tile lives (null: past the image); consecutive channels are cstride floats apart.
+template <int I2MAJOR>
+__device__ float* grad_row(const GradArgs& a, const GradSched& sc, int m, size_t& cstride) {
+  const int C = a.d.C;
+  cstride = 1;
+  if (I2MAJOR == 0) {
+    const int p = sc.m0 + m;
+    if (p >= a.d.N1()) return nullptr;
+    if (!a.out_cf) return a.out + ((size_t)sc.b * a.d.N1() + p) * C;
+    cstride = (size_t)a.d.N1();
+    return a.out + (size_t)sc.b * C * a.d.N1() + p;
+  }
+  const int u = sc.u0 + m / GG_ROW_VT, v = sc.v0 + m % GG_ROW_VT;
+  if (u >= a.d.H2 || v >= a.d.W2) return nullptr;
+  if (!a.out_cf) return a.out + (((size_t)sc.b * a.d.H2 + u) * a.d.W2 + v) * C;
+  cstride = (size_t)a.d.N2();
+  return a.out + (size_t)sc.b * C * a.d.N2() + (size_t)u * a.d.W2 + v;
+}
+// Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][channel][128 rows]
+__device__ __forceinline__ float* grad_part(const GradArgs& a, int tail, int piece) {
+  return a.part + ((size_t)tail * (a.pieces - 1) + piece - 1) * a.d.C * TILE_M;
+}
+
 template <int Q, int I2MAJOR>
 __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc, int warp, int gw, int lane) {
   const bool ok = mbar_wait(&sm.acc_full, 0, &sm.ctl, a.status, DEV_TIMEOUT_EPILOGUE);
@@ -393,20 +424,14 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
   const int C = a.d.C;
   const int q = warp & 3;  // TMEM lane quarter this warp may read
   const int m = q * 32 + lane;
-  float* dst = nullptr;
-  size_t cstride = 1;  // elements between consecutive channels of this row
-  if (I2MAJOR == 0) {
-    const int p = sc.m0 + m;
-    if (p < a.d.N1()) {
-      if (a.out_cf) { dst = a.out + (size_t)sc.b * C * a.d.N1() + p; cstride = (size_t)a.d.N1(); }
-      else dst = a.out + ((size_t)sc.b * a.d.N1() + p) * C;
-    }
-  } else {
-    const int u = sc.u0 + m / GG_ROW_VT, v = sc.v0 + m % GG_ROW_VT;
-    if (u < a.d.H2 && v < a.d.W2) {
-      if (a.out_cf) { dst = a.out + (size_t)sc.b * C * a.d.N2() + (size_t)u * a.d.W2 + v; cstride = (size_t)a.d.N2(); }
-      else dst = a.out + (((size_t)sc.b * a.d.H2 + u) * a.d.W2 + v) * C;
-    }
+  size_t cstride;
+  float* dst = grad_row<I2MAJOR>(a, sc, m, cstride);
+  bool channel_major = a.out_cf != 0, accumulate = a.accumulate != 0;
+  if (sc.piece > 0) {
+    if (dst != nullptr) dst = grad_part(a, sc.tail, sc.piece) + m;
+    cstride = TILE_M;
+    channel_major = true;
+    accumulate = false;
   }
   const uint32_t tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
   const float osc = a.out_scale * (a.dev_scale != nullptr ? __ldg(a.dev_scale) : 1.f);
@@ -416,13 +441,13 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
     float s[16];
     tmem_ld16(tbase + c0, s);
     if (dst == nullptr) continue;
-    if (a.out_cf) {  // channel-major output: a warp's 32 rows are 32 neighbouring pixels of one channel plane
+    if (channel_major) {  // a warp's 32 rows are 32 neighbouring pixels of one channel plane
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         if (c0 + j < C) {
           float* d1 = dst + (size_t)(c0 + j) * cstride;
           float v1 = s[j] * osc;
-          if (a.accumulate) v1 += *d1;
+          if (accumulate) v1 += *d1;
           *d1 = v1;
         }
       }
@@ -432,13 +457,74 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
         if (c0 + j < C) {
           float4* d4 = reinterpret_cast<float4*>(dst + c0 + j);
           float4 v4 = make_float4(s[j] * osc, s[j + 1] * osc, s[j + 2] * osc, s[j + 3] * osc);
-          if (a.accumulate) {
+          if (accumulate) {
             const float4 o = *d4;
             v4.x += o.x; v4.y += o.y; v4.z += o.z; v4.w += o.w;
           }
           *d4 = v4;
         }
       }
+    }
+  }
+}
+
+// Pieces 1.. of a finished tail tile added to the output, in piece order (all threads of the CTA that finished last).  One
+// SM's loads move all of it, so a thread takes four rows x four channels at once and asks for several pieces' values
+// before it uses any.
+template <int I2MAJOR>
+__device__ void grad_fold_pieces(const GradArgs& a, const GradSched& sc) {
+  constexpr int QUADS = TILE_M / 4, FOLD_PIECES = 2;
+  const int C = a.d.C;
+  for (int i = threadIdx.x; i < C / 4 * QUADS; i += GG_THREADS) {  // C is a multiple of 4
+    const int m = i % QUADS * 4, c0 = i / QUADS * 4;
+    size_t cstride, unused;
+    float* row[4];   // the four rows are neighbours in the image: the ones that exist come first
+    row[0] = grad_row<I2MAJOR>(a, sc, m, cstride);
+    if (row[0] == nullptr) continue;
+    int cnt = 1;
+#pragma unroll
+    for (int r = 1; r < 4; ++r) {
+      row[r] = grad_row<I2MAJOR>(a, sc, m + r, unused);
+      cnt += row[r] != nullptr;
+    }
+    float4 v[4];     // channel-major output: [channel] over the rows; pixel-major: [row] over the channels
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[j] = a.out_cf ? load4_cg(row[0] + (c0 + j) * cstride, cnt) : load4_cg(row[j] + c0, j < cnt ? 4 : 0);
+    float4 sum[4];   // [channel] over the rows
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[j] = a.out_cf ? v[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!a.out_cf) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        (&sum[j].x)[0] = (&v[0].x)[j]; (&sum[j].x)[1] = (&v[1].x)[j];
+        (&sum[j].x)[2] = (&v[2].x)[j]; (&sum[j].x)[3] = (&v[3].x)[j];
+      }
+    }
+    const float* part = grad_part(a, sc.tail, 1) + (size_t)c0 * TILE_M + m;
+    const size_t step = (size_t)C * TILE_M;
+    for (int s0 = 1; s0 < a.pieces; s0 += FOLD_PIECES) {
+      float4 o[FOLD_PIECES][4];
+#pragma unroll
+      for (int q = 0; q < FOLD_PIECES; ++q)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          o[q][j] = s0 + q < a.pieces ? __ldcg(reinterpret_cast<const float4*>(part + (s0 + q - 1) * step + j * TILE_M))
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < FOLD_PIECES; ++q) {
+        if (s0 + q >= a.pieces) break;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) add4(sum[j], o[q][j]);
+      }
+    }
+    if (a.out_cf) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) store4(row[0] + (c0 + j) * cstride, sum[j], cnt);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (r < cnt) store4(row[r] + c0, make_float4((&sum[0].x)[r], (&sum[1].x)[r], (&sum[2].x)[r], (&sum[3].x)[r]), 4);
     }
   }
 }
@@ -458,24 +544,40 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
 
   GradSched sc;
   sc.nkb = (a.d.C + KBLK - 1) / KBLK;
+  int tile = blockIdx.x;
+  sc.tail = -1;
+  sc.piece = 0;
+  if (tile >= a.whole_tiles) {  // pieces of the tail tiles follow the whole tiles
+    const int r = tile - a.whole_tiles;
+    sc.tail = r / a.pieces;
+    sc.piece = r - sc.tail * a.pieces;
+    tile = a.whole_tiles + sc.tail;
+  }
+  int all_blocks;
   if (I2MAJOR == 0) {
     const int tiles = (a.d.N1() + TILE_M - 1) / TILE_M;
-    sc.b = blockIdx.x / tiles;
-    sc.m0 = (blockIdx.x - sc.b * tiles) * TILE_M;
+    sc.b = tile / tiles;
+    sc.m0 = (tile - sc.b * tiles) * TILE_M;
     sc.u0 = sc.v0 = 0;
     sc.n_ub2 = (a.d.H2 + GG_UT - 1) / GG_UT;
     sc.h2p = sc.n_ub2 * GG_UT;
-    sc.n_blocks = sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT);
+    all_blocks = sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT);
   } else {
     const int n_ub = (a.d.H2 + GG_ROW_UT - 1) / GG_ROW_UT, n_vb = (a.d.W2 + GG_ROW_VT - 1) / GG_ROW_VT;
-    sc.b = blockIdx.x / (n_ub * n_vb);
-    const int r = blockIdx.x - sc.b * (n_ub * n_vb);
+    sc.b = tile / (n_ub * n_vb);
+    const int r = tile - sc.b * (n_ub * n_vb);
     sc.u0 = (r / n_vb) * GG_ROW_UT;
     sc.v0 = (r % n_vb) * GG_ROW_VT;
     sc.m0 = 0;
     sc.n_ub2 = 0;
     sc.h2p = 0;
-    sc.n_blocks = (a.d.N1() + GG_KJ - 1) / GG_KJ;
+    all_blocks = (a.d.N1() + GG_KJ - 1) / GG_KJ;
+  }
+  const int n_pieces = sc.tail >= 0 ? a.pieces : 1;
+  {
+    const int per = all_blocks / n_pieces, extra = all_blocks - per * n_pieces;  // the first `extra` pieces have one more
+    sc.t0 = sc.piece * per + min(sc.piece, extra);
+    sc.n_blocks = per + (sc.piece < extra ? 1 : 0);
   }
 
   if (threadIdx.x == 0) {
@@ -525,6 +627,45 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
     tc_fence_after();
     tmem_dealloc(sm.tmem_base, gg_tmem_cols<I2MAJOR>());
   }
+  if (n_pieces > 1 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
+    __threadfence();  // this thread's results before the count ...
+    __syncthreads();
+    if (threadIdx.x == 0) sm.last_piece = atomicAdd(a.tail_count + sc.tail, 1) == n_pieces - 1;
+    __syncthreads();
+    if (sm.last_piece) {
+      __threadfence();  // ... and the count before the other pieces' results
+      grad_fold_pieces<I2MAJOR>(a, sc);
+      if (threadIdx.x == 0) a.tail_count[sc.tail] = 0;  // as the next launch expects it
+    }
+  }
+}
+
+static int grad_tiles(const Dims& d, int image2_major) {
+  return image2_major ? d.B * ((d.H2 + GG_ROW_UT - 1) / GG_ROW_UT) * ((d.W2 + GG_ROW_VT - 1) / GG_ROW_VT)
+                      : d.B * ((d.N1() + TILE_M - 1) / TILE_M);
+}
+
+// How the tail tiles are cut, in units of one K block's time (32 values, about 0.6 us): a CTA costs about eight blocks of
+// prologue and drain, a fold reads 128 KB per piece through one SM (about two blocks).  Pieces must save a quarter of the
+// tail (see sweep_split) and at least four blocks to be used.
+TileSplit grad_split(const Dims& d, int image2_major) {
+  const int tiles = grad_tiles(d, image2_major), rest = tiles % SM_COUNT;
+  const int blocks = image2_major ? (d.N1() + GG_KJ - 1) / GG_KJ
+                                  : ((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT);
+  TileSplit r{tiles, tiles, 1, 0};
+  if (rest == 0) return r;
+  double best = 0, whole = 0;
+  for (int n = 1; n <= blocks && n <= MAX_PIECES; ++n) {
+    const double waves = (rest * n + SM_COUNT - 1) / SM_COUNT;
+    const double cost = waves * ((blocks + n - 1) / n + 8) + (n > 1 ? 2.0 * n * d.C / MAX_C + 2 : 0.0);
+    if (n == 1) best = whole = cost;
+    if (cost < best && cost < 0.75 * whole && cost < whole - 4) { best = cost; r.pieces = n; }
+  }
+  if (r.pieces > 1) {
+    r.whole_tiles = tiles - rest;
+    r.part_floats = (size_t)rest * (r.pieces - 1) * d.C * TILE_M;
+  }
+  return r;
 }
 
 template <int MODE, int Q, int I2MAJOR, int BF16>
@@ -538,9 +679,7 @@ static cudaError_t launch_one(const GradArgs& a, const CUtensorMap& tm_y, const 
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
   });
   if (err != cudaSuccess) return err;
-  int ctas;
-  if (I2MAJOR == 0) ctas = a.d.B * ((a.d.N1() + TILE_M - 1) / TILE_M);
-  else ctas = a.d.B * ((a.d.H2 + GG_ROW_UT - 1) / GG_ROW_UT) * ((a.d.W2 + GG_ROW_VT - 1) / GG_ROW_VT);
+  const int ctas = a.whole_tiles + (grad_tiles(a.d, I2MAJOR) - a.whole_tiles) * a.pieces;
   kern<<<dim3(ctas), GG_THREADS, smem_bytes, stream>>>(tm_y, tm_xu, tm_xv, a);
   return cudaGetLastError();
 }

@@ -134,7 +134,11 @@ struct GradArgs {
   float* out;            // gF1 (B,N1,C) or gF2 (B,N2,C)
   int* status;
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
+  int whole_tiles, pieces;           // as in SweepArgs, here with pieces of the K sweep (TileSplit)
+  float* part;
+  int* tail_count;
 };
+TileSplit grad_split(const Dims& d, int image2_major);
 
 // One source of an interleaved slot: dst[b][d][slot/4][p][slot%4] = scale * src[b][p][k][d] (raw copy when scale == 0);
 // src is (B, N1, Ksrc, D).  A null src makes the slot the constant `scale` (zero by default) for every valid pixel.
