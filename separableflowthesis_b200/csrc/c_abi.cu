@@ -468,13 +468,34 @@ int map_sweep_operands(const Dims& d, const Workspace& w, int op16, CUtensorMap*
   return SFB_OK;
 }
 
-// Rounded copies of a call's features (and of the mean rows of image 2 when with_aux), plus 16-bit copies of kind op16.
-cudaError_t prepare_operands(const Dims& d, const Workspace& w, const float* F1, const float* F2, bool with_aux,
-                             int op16, cudaStream_t st) {
+// The features of a call as the caller holds them: pixel-major (B, pixels, C), or (fmaps) the model's feature maps
+// (B, C, pixels) with a factor for image 1.
+struct Features {
+  const float* F1;
+  const float* F2;
+  bool fmaps;
+  float scale1;
+};
+
+// Operand copies of a call's features (and of the mean rows of image 2 when with_aux) for operands of kind op16.
+cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& f, bool with_aux, int op16, cudaStream_t st) {
   // (an op without sweeps has no 16-bit copies in its workspace, but its gradient GEMMs still need the feature scales)
-  return launch_prepare(d, F1, F2, w.F1r, w.F2r, with_aux ? w.aux : nullptr, w.status, st, op16 ? w.F1h : nullptr,
-                        op16 ? w.F2h : nullptr, op16 && with_aux ? w.auxh : nullptr, op16, w.scales);
+  float* const F1r = op16 ? nullptr : w.F1r;
+  float* const F2r = op16 ? nullptr : w.F2r;
+  float* const aux = op16 || !with_aux ? nullptr : w.aux;
+  uint16_t* const F1h = op16 ? w.F1h : nullptr;
+  uint16_t* const F2h = op16 ? w.F2h : nullptr;
+  uint16_t* const auxh = op16 && with_aux ? w.auxh : nullptr;
+  return f.fmaps ? launch_prepare_cf(d, f.F1, f.F2, f.scale1, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales)
+                 : launch_prepare(d, f.F1, f.F2, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales);
 }
+// Launches of the above: FP16 operands add the search for the magnitudes.
+int prepare_launches(const Workspace& w, bool fmaps, bool with_aux, int op16) {
+  const bool copies = !op16 || w.F1h != nullptr;
+  return (copies ? (fmaps ? 1 : 2) : 0) + (with_aux ? 1 : 0) + (op16 == OP16_FP16 ? 1 : 0);
+}
+#define SFB_PREPARE(f, with_aux) \
+  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, (f).fmaps, with_aux, op16), st, [&] { return prepare_operands(d, w, f, with_aux, op16, st); }))
 
 int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, int32_t* AM_u, int32_t* AM_v,
                        bool with_argmax, const sfb_shape* shape, void* ws, size_t ws_bytes, void* stream) {
@@ -489,7 +510,8 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
-  SFB_CUDA(timed(KID_PREPARE, 3 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, true, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, true);
   SweepArgs a;
   memset(&a, 0, sizeof(a));
   a.d = d;
@@ -544,7 +566,7 @@ int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm
 }
 
 // out_cf: the gradients are written channel-major, (B, C, pixels), gF1 multiplied by scale1.
-int run_grad_pair(const Dims& d, const Workspace& w, int mode, int R4, int accumulate, float* gF1, float* gF2,
+int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int mode, int R4, int accumulate, float* gF1, float* gF2,
                   cudaStream_t st, int out_cf = 0, float scale1 = 1.f) {
   // 16-bit form when the operand switch says so (callers have refused feature dimensions that do not allow it); with
   // FP16 the callers have run grad_operand_scales and packed the operands with those scales
@@ -575,9 +597,13 @@ int run_grad_pair(const Dims& d, const Workspace& w, int mode, int R4, int accum
   const size_t f2t_per_sample = (size_t)d.C * ((d.W2 + GG_VT - 1) / GG_VT) * w.h2p * GG_VT;
   if (!accumulate) {  // later passes over further channel chunks reuse the copies of the first
     SFB_CUDA(timed(KID_PREPARE, 2, st, [&] {
+      if (op16 && feat.fmaps) {  // already channel-major
+        launch_channel_major_cf(feat.F1, reinterpret_cast<uint16_t*>(w.F1t), d.B, 1, d.N1(), w.n1p, d.C, 0, feat.scale1, op16, s1, st);
+        return launch_channel_major_cf(feat.F2, reinterpret_cast<uint16_t*>(w.F2t), d.B, d.H2, d.W2, w.h2p, d.C, 1, 1.f, op16, s2, st);
+      }
       cudaMemsetAsync(w.F2t, 0, (size_t)d.B * f2t_per_sample * (op16 ? 2 : sizeof(float)), st);
-      launch_channel_major(w.F1r, w.F1t, d.B, 1, d.N1(), w.n1p, d.C, 0, op16, s1, st);
-      return launch_channel_major(w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
+      launch_channel_major(op16 ? feat.F1 : w.F1r, w.F1t, d.B, 1, d.N1(), w.n1p, d.C, 0, op16, s1, st);
+      return launch_channel_major(op16 ? feat.F2 : w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
     }));
   }
   // gF1 = G * F2 : rows are image-1 pixels, the K sweep streams 2 x 16 blocks of F2 and 2-row blocks of XU.
@@ -662,11 +688,11 @@ struct AbsmaxSrc { const float* p; size_t n; };
 int grad_operand_scales(const Workspace& w, int op16, std::initializer_list<AbsmaxSrc> grads,
                         std::initializer_list<AbsmaxSrc> weights, cudaStream_t st) {
   if (op16 != OP16_FP16) return SFB_OK;
-  SFB_CUDA(timed(KID_PREPARE, (int)(grads.size() + weights.size()) + 1, st, [&] {
-    for (const AbsmaxSrc& g : grads) launch_absmax(g.p, g.n, 1.f, w.scales + SCALE_AMAX_G, st);
-    for (const AbsmaxSrc& a : weights) launch_absmax(a.p, a.n, 1.f, w.scales + SCALE_AMAX_A, st);
-    return launch_grad_scales(w.scales, st);
-  }));
+  AbsmaxSource src[ABSMAX_MAX];
+  int n = 0;
+  for (const AbsmaxSrc& g : grads) src[n++] = AbsmaxSource{g.p, g.n, 1.f, SCALE_AMAX_G};
+  for (const AbsmaxSrc& a : weights) src[n++] = AbsmaxSource{a.p, a.n, 1.f, SCALE_AMAX_A};
+  SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_absmax(src, n, w.scales, true, st); }));
   return SFB_OK;
 }
 const float* grad_slot_scales(const Workspace& w, int op16) { return op16 == OP16_FP16 ? w.scales : nullptr; }
@@ -806,7 +832,8 @@ int sfb_compression_forward(const float* F1, const float* F2, const float* A_u, 
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
     launch_pack(A_u, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st);         // w_u[k][v] = XV slot k
@@ -833,7 +860,8 @@ int sfb_max_argmax_avg_backward(const float* F1, const float* F2, const int32_t*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   const size_t pix = (size_t)d.B * d.N1();
   SFB_TRY(grad_operand_scales(w, op16, {{gMA_u, pix * 2 * d.H2}, {gMA_v, pix * 2 * d.W2}}, {}, st));
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
@@ -842,7 +870,7 @@ int sfb_max_argmax_avg_backward(const float* F1, const float* F2, const int32_t*
     launch_pack_interleaved(su, w.gxu, d.B, d.N1(), w.n1p, d.H2, 4, 1, 0, st);
     return launch_pack_interleaved(sv, w.gxv, d.B, d.N1(), w.n1p, d.W2, 4, 1, 0, st);
   }));
-  return run_grad_pair(d, w, GRAD_MAXAVG, 4, 0, gF1, gF2, st);
+  return run_grad_pair(d, w, feat, GRAD_MAXAVG, 4, 0, gF1, gF2, st);
 }
 
 int sfb_compression_backward(const float* F1, const float* F2, const float* A_u, const float* A_v,
@@ -858,7 +886,8 @@ int sfb_compression_backward(const float* F1, const float* F2, const float* A_u,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   SFB_TRY(run_attention_grads(d, w, gC_u, gC_v, gA_u, gA_v, st, op16));
   {
@@ -874,7 +903,7 @@ int sfb_compression_backward(const float* F1, const float* F2, const float* A_u,
       launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st);
       return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
     }));
-    SFB_TRY(run_grad_pair(d, w, GRAD_COMPRESS, R4, k0 > 0 ? 1 : 0, gF1, gF2, st));
+    SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, k0 > 0 ? 1 : 0, gF1, gF2, st));
   }
   return SFB_OK;
 }
@@ -890,13 +919,14 @@ int sfb_compression_attention_backward(const float* F1, const float* F2, const f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   return run_attention_grads(d, w, gC_u, gC_v, gA_u, gA_v, st, op16);
 }
 
 // Feature gradients of both backward ops from one GEMM pair (plus accumulated passes for channels beyond
-// KC_MAX_PER_SWEEP).  F1r / F2r must already hold the rounded features.
-static int run_fused_feature_grads(const Dims& d, const Workspace& w, const int32_t* AM_u, const int32_t* AM_v,
+// KC_MAX_PER_SWEEP).  The call's prepare_operands has run.
+static int run_fused_feature_grads(const Dims& d, const Workspace& w, const Features& feat, const int32_t* AM_u, const int32_t* AM_v,
                                    const float* gMA_u, const float* gMA_v, const float* A_u, const float* A_v,
                                    const float* gC_u, const float* gC_v, float* gF1, float* gF2, cudaStream_t st) {
   const int N1 = d.N1(), K = d.Kc;
@@ -920,7 +950,7 @@ static int run_fused_feature_grads(const Dims& d, const Workspace& w, const int3
       launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st);
       return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4 * Qc, Q, 1, st);
     }));
-    SFB_TRY(run_grad_pair(d, w, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st));
+    SFB_TRY(run_grad_pair(d, w, feat, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st));
   }
   for (int k0 = KC_MAX_PER_SWEEP; k0 < K; k0 += KC_MAX_PER_SWEEP) {  // remaining channels: compression form, accumulated
     const int kc = chunk_channels(K - k0), R4 = grad_slots(kc);
@@ -930,7 +960,7 @@ static int run_fused_feature_grads(const Dims& d, const Workspace& w, const int3
       launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st);
       return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
     }));
-    SFB_TRY(run_grad_pair(d, w, GRAD_COMPRESS, R4, 1, gF1, gF2, st));
+    SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, 1, gF1, gF2, st));
   }
   return SFB_OK;
 }
@@ -948,8 +978,9 @@ int sfb_separation_feature_backward(const float* F1, const float* F2, const int3
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
-  return run_fused_feature_grads(d, w, AM_u, AM_v, gMA_u, gMA_v, A_u, A_v, gC_u, gC_v, gF1, gF2, st);
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
+  return run_fused_feature_grads(d, w, feat, AM_u, AM_v, gMA_u, gMA_v, A_u, A_v, gC_u, gC_v, gF1, gF2, st);
 }
 
 int sfb_separation_backward(const float* F1, const float* F2, const int32_t* AM_u, const int32_t* AM_v,
@@ -967,9 +998,10 @@ int sfb_separation_backward(const float* F1, const float* F2, const int32_t* AM_
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   SFB_TRY(run_attention_grads(d, w, gC_u, gC_v, gA_u, gA_v, st, op16));
-  return run_fused_feature_grads(d, w, AM_u, AM_v, gMA_u, gMA_v, A_u, A_v, gC_u, gC_v, gF1, gF2, st);
+  return run_fused_feature_grads(d, w, feat, AM_u, AM_v, gMA_u, gMA_v, A_u, A_v, gC_u, gC_v, gF1, gF2, st);
 }
 
 int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v, float* SEP_u, int32_t* AM_u,
@@ -987,7 +1019,8 @@ int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
-  SFB_CUDA(timed(KID_PREPARE, 3 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, true, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, true);
   const int N1 = d.N1();
   SweepArgs a;
   memset(&a, 0, sizeof(a));
@@ -1020,7 +1053,8 @@ static int run_compress_cf(const float* F1, const float* F2, const float* W_u, c
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   // W_u (B,K,W2,N1) weights per v, W_v (B,K,H2,N1) per u; O_u (B,K,H2,N1), O_v (B,K,W2,N1)
   return run_compress_sweeps(d, w, tm_f1, tm_f2, cf_view(W_v, K, d.H2, N1), cf_view(W_u, K, d.W2, N1), 0, 0, 1,
@@ -1042,7 +1076,7 @@ int sfb_compression_attention_backward_cf(const float* F1, const float* F2, cons
 
 // Channels-first form of run_fused_feature_grads: gMA sources gM_v (B,2,H2,N1) / gM_u (B,2,W2,N1); the compression
 // gradients are channels g0.. of tensors with gK channels.
-static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const int32_t* AM_u, const int32_t* AM_v,
+static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const Features& feat, const int32_t* AM_u, const int32_t* AM_v,
                                       const float* gM_v, const float* gM_u, const float* A_u, const float* A_v,
                                       const float* gC_u, const float* gC_v, int gK, int g0, float* gF1, float* gF2,
                                       cudaStream_t st, int out_cf = 0, float scale1 = 1.f, bool unit_weights = false) {
@@ -1071,7 +1105,7 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const i
       launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st);
       return launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4 * Qc, Q, 1, st);
     }));
-    SFB_TRY(run_grad_pair(d, w, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st, out_cf, scale1));
+    SFB_TRY(run_grad_pair(d, w, feat, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st, out_cf, scale1));
   }
   for (int k0 = KC_MAX_PER_SWEEP; k0 < K; k0 += KC_MAX_PER_SWEEP) {
     const int kc = chunk_channels(K - k0), R4 = grad_slots(kc);
@@ -1081,7 +1115,7 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const i
       launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st);
       return launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
     }));
-    SFB_TRY(run_grad_pair(d, w, GRAD_COMPRESS, R4, 1, gF1, gF2, st, out_cf, scale1));
+    SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, 1, gF1, gF2, st, out_cf, scale1));
   }
   return SFB_OK;
 }
@@ -1100,8 +1134,9 @@ int sfb_separation_feature_backward_cf(const float* F1, const float* F2, const i
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
-  return run_fused_feature_grads_cf(d, w, AM_u, AM_v, gSEP_v, gSEP_u, A_u, A_v, gC_u, gC_v, d.Kc, 0, gF1, gF2, st);
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
+  return run_fused_feature_grads_cf(d, w, feat, AM_u, AM_v, gSEP_v, gSEP_u, A_u, A_v, gC_u, gC_v, d.Kc, 0, gF1, gF2, st);
 }
 
 // ---- attention weights: Conv3d(2 -> Kc, 3, padding 1) + softmax over the displacement axis ----
@@ -1198,13 +1233,8 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
-  uint16_t* const F1h = op16 ? w.F1h : nullptr;
-  uint16_t* const F2h = op16 ? w.F2h : nullptr;
-  uint16_t* const auxh = op16 ? w.auxh : nullptr;
-  SFB_CUDA(timed(KID_PREPARE, 3 + (op16 == OP16_FP16 ? 3 : 0), st, [&] {
-    return fmaps ? launch_prepare_cf(d, F1, F2, scale1, w.F1r, w.F2r, w.aux, w.status, st, F1h, F2h, auxh, op16, w.scales)
-                 : launch_prepare(d, F1, F2, w.F1r, w.F2r, w.aux, w.status, st, F1h, F2h, auxh, op16, w.scales);
-  }));
+  const Features feat{F1, F2, fmaps != 0, scale1};
+  SFB_PREPARE(feat, true);
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
   SweepArgs a;
   memset(&a, 0, sizeof(a));
@@ -1273,12 +1303,8 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  uint16_t* const F1h = op16 ? w.F1h : nullptr;
-  uint16_t* const F2h = op16 ? w.F2h : nullptr;
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] {
-    return fmaps ? launch_prepare_cf(d, F1, F2, scale1, w.F1r, w.F2r, nullptr, w.status, st, F1h, F2h, nullptr, op16, w.scales)
-                 : launch_prepare(d, F1, F2, w.F1r, w.F2r, nullptr, w.status, st, F1h, F2h, nullptr, op16, w.scales);
-  }));
+  const Features feat{F1, F2, fmaps != 0, fmaps ? scale1 : 1.f};
+  SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
   // attention gradients: gA_v(b,k,u,p) = sum_v S * gC_v(b,k,v,p), gA_u(b,k,v,p) = sum_u S * gC_u(b,k,u,p), with
   // gC_u = gSEP_v[:, 2:] (per u) and gC_v = gSEP_u[:, 2:] (per v) in the role of the weights
@@ -1294,7 +1320,7 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
     return launch_attention_backward(AttentionDims{d.B, K, d.H2, d.H1, d.W1}, SEP_v + ov, sb_v, weight_v, A_v, w.ga_v,
                                      gSEP_v + ov, sb_v, w.gm_v, gweight_v, gbias_v, w.at_partial, st, w.status);
   }));
-  return run_fused_feature_grads_cf(d, w, AM_u, AM_v, w.gm_v, w.gm_u, A_u, A_v, gSEP_v, gSEP_u, Kt, c0 + 2, gF1, gF2, st,
+  return run_fused_feature_grads_cf(d, w, feat, AM_u, AM_v, w.gm_v, w.gm_u, A_u, A_v, gSEP_v, gSEP_u, Kt, c0 + 2, gF1, gF2, st,
                                     fmaps, fmaps ? scale1 : 1.f, /*unit_weights=*/true);
 }
 
@@ -1491,7 +1517,8 @@ int sfb_corr_volume(const float* F1, const float* F2, float* S, const sfb_shape*
   const int op16 = OP16_NONE;  // this test aid always computes with TF32 operands (its workspace has no 16-bit copies)
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  SFB_CUDA(timed(KID_PREPARE, 2 + (op16 == OP16_FP16 ? 3 : 0), st, [&] { return prepare_operands(d, w, F1, F2, false, op16, st); }));
+  const Features feat{F1, F2, false, 1.f};
+  SFB_PREPARE(feat, false);
   SweepArgs a;
   memset(&a, 0, sizeof(a));
   a.d = d;

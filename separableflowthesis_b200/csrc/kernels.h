@@ -171,12 +171,13 @@ enum : int {
   SCALE_AMAX_F1 = 0, SCALE_AMAX_F2 = 1, SCALE_AMAX_G = 2, SCALE_AMAX_A = 3,
   SCALE_F1 = 4, SCALE_F2 = 5, SCALE_INV_F1F2 = 6,   // F1h = fp16(s1 F1), F2h = fp16(s2 F2), sweep outputs * 1/(s1 s2)
   SCALE_GA = 7, SCALE_G = 8, SCALE_A = 9,           // gradient slots * sg (* sa when no weight multiplies them), weights * sa
-  SCALE_INV_GF1 = 10, SCALE_INV_GF2 = 11            // gF1 * 1/(sg sa s2), gF2 * 1/(sg sa s1)
+  SCALE_INV_GF1 = 10, SCALE_INV_GF2 = 11,           // gF1 * 1/(sg sa s2), gF2 * 1/(sg sa s1)
+  SCALE_TICKET = 12                                 // blocks of a running magnitude search that are done
 };
-// Rounds F1/F2 to TF32 (round-to-nearest) into the workspace copies, optionally builds the
-// row/column mean rows of F2, and clears the workspace header.
-// F1h / F2h / auxh (optional): the same three arrays as 16-bit operands of kind `op16` from the unrounded values: BF16,
-// or FP16 after scaling by the powers of two this call derives from the arrays' largest magnitudes (scales[]).
+// Makes the operand copies of a call's features and clears the workspace header.  TF32 operands (op16 = 0): F1r / F2r,
+// rounded to nearest, and the row/column mean rows of F2 in aux.  16-bit operands: F1h / F2h / auxh, from the unrounded
+// values (BF16, or FP16 after scaling by the powers of two this call derives from the arrays' largest magnitudes,
+// scales[]).  Null arrays are left out.
 cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, float* F1r, float* F2r, float* aux,
                            int* status, cudaStream_t stream, uint16_t* F1h = nullptr, uint16_t* F2h = nullptr,
                            uint16_t* auxh = nullptr, int op16 = 0, float* scales = nullptr);
@@ -186,11 +187,15 @@ cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, floa
 cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fmap2, float scale1, float* F1r,
                               float* F2r, float* aux, int* status, cudaStream_t stream, uint16_t* F1h = nullptr,
                               uint16_t* F2h = nullptr, uint16_t* auxh = nullptr, int op16 = 0, float* scales = nullptr);
-// Largest |x| * premul of n floats, combined into the amax slot; the gradient-operand scales from the amax slots.
-cudaError_t launch_absmax(const float* x, size_t n, float premul, float* slot, cudaStream_t stream);
-cudaError_t launch_feature_scales(float* scales, cudaStream_t stream);
-cudaError_t launch_grad_scales(float* scales, cudaStream_t stream);
-// Channel-major copy of a (rounded) pixel-major feature array (B, rows*width, C), as FP32 or (op16 != 0) as 16-bit
+// Largest |x| * premul of each array, combined into its amax slot, and then the multipliers that follow from the slots:
+// those of the features or (gradients) those of the gradient operands.
+constexpr int ABSMAX_MAX = 6;
+struct AbsmaxSource { const float* p; size_t n; float premul; int slot; };
+cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, bool gradients, cudaStream_t stream);
+// 16-bit channel-major copy from a (B, C, rows*width) feature map times `scale`, padding zeroed (layouts below).
+cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
+                                    int blocked, float scale, int op16, const float* scale16, cudaStream_t stream);
+// Channel-major copy of a pixel-major feature array (B, rows*width, C), as FP32 (of rounded values) or (op16 != 0) as 16-bit
 // operands (FP16: times the device scalar *scale16); padding is not written.
 //   blocked = 0: dst (B, C, pitch) with pixel index row*width + x (rows = 1)
 //   blocked = 1: dst (B, C, ceil(width/16), pitch, 16), element (row, x) at ((x/16)*pitch + row)*16 + x%16

@@ -8,7 +8,9 @@
 //  * 16-bit operand copies (BF16, or FP16 for the operand type with TF32's mantissa at twice its tensor-core rate).
 //    FP16 has a narrow exponent range, so every tensor that becomes an FP16 operand is first multiplied by a power
 //    of two that brings its largest magnitude next to 1 (exact, undone when results are stored): absmax_kernel
-//    finds the magnitudes, *_scales_kernel turn them into the multipliers, all on the device.
+//    finds the magnitudes and its last block turns them into the multipliers, all on the device.
+// The FP32 copies are made for TF32 operands only; with 16-bit operands every reader takes the 16-bit copies or the
+// caller's features themselves.
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -17,32 +19,6 @@
 #include "sm100_primitives.cuh"
 
 namespace sfb {
-
-// Largest |x| * premul of an array, as the bits of a non-negative float, combined into *out with atomicMax (integer
-// order = float order for non-negative values; NaNs are ignored).  n4 = number of float4.
-__global__ void absmax_kernel(const float4* __restrict__ x, size_t n4, int tail, float premul,
-                              unsigned* __restrict__ out) {
-  float m = 0.f;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    const float4 v = __ldg(x + i);
-    m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-  }
-  if (blockIdx.x == 0 && (int)threadIdx.x < tail) m = fmaxf(m, fabsf(__ldg(reinterpret_cast<const float*>(x + n4) + threadIdx.x)));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(out, __float_as_uint(m * fabsf(premul)));
-}
-
-cudaError_t launch_absmax(const float* x, size_t n, float premul, float* slot, cudaStream_t stream) {
-  if (n == 0) return cudaSuccess;
-  const size_t n4 = n / 4;  // the arrays are 16-byte aligned; up to three trailing values are read one by one
-  const int threads = 256;
-  const unsigned blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((n4 + threads - 1) / threads, 148 * 8));
-  absmax_kernel<<<blocks, threads, 0, stream>>>(reinterpret_cast<const float4*>(x), n4, (int)(n - 4 * n4), premul,
-                                                reinterpret_cast<unsigned*>(slot));
-  return cudaGetLastError();
-}
 
 // The power of two that brings a largest magnitude (float bits in `amax_bits`) into [target, 2*target); 1 when the
 // magnitude is zero, not finite or subnormal, and never beyond 2^+-40, so that products of three scales stay finite
@@ -57,29 +33,84 @@ __device__ __forceinline__ float pow2_scale(unsigned amax_bits, int target_log2)
 }
 
 // scales[] (SCALE_* in kernels.h): feature scales from the two magnitudes found by absmax_kernel.
-__global__ void feature_scales_kernel(float* scales) {
-  const float s1 = pow2_scale(__float_as_uint(scales[SCALE_AMAX_F1]), 0);
-  const float s2 = pow2_scale(__float_as_uint(scales[SCALE_AMAX_F2]), 0);
+__device__ void feature_scales(float* scales) {
+  const float s1 = pow2_scale(__float_as_uint(__ldcg(scales + SCALE_AMAX_F1)), 0);
+  const float s2 = pow2_scale(__float_as_uint(__ldcg(scales + SCALE_AMAX_F2)), 0);
   scales[SCALE_F1] = s1;
   scales[SCALE_F2] = s2;
   scales[SCALE_INV_F1F2] = 1.f / (s1 * s2);
 }
-// Gradient-operand scales (after feature_scales_kernel of the same call): G is generated as (sg * sa) * G.
-__global__ void grad_scales_kernel(float* scales) {
-  const float sg = pow2_scale(__float_as_uint(scales[SCALE_AMAX_G]), 7);   // largest gradient value -> [128, 256)
-  const float sa = pow2_scale(__float_as_uint(scales[SCALE_AMAX_A]), 0);   // largest weight -> [1, 2)
+// Gradient-operand scales (after the feature scales of the same call): G is generated as (sg * sa) * G.
+__device__ void grad_scales(float* scales) {
+  const float sg = pow2_scale(__float_as_uint(__ldcg(scales + SCALE_AMAX_G)), 7);   // largest gradient value -> [128, 256)
+  const float sa = pow2_scale(__float_as_uint(__ldcg(scales + SCALE_AMAX_A)), 0);   // largest weight -> [1, 2)
   scales[SCALE_GA] = sg * sa;
   scales[SCALE_G] = sg;
   scales[SCALE_A] = sa;
   scales[SCALE_INV_GF1] = 1.f / (sg * sa * scales[SCALE_F2]);   // gF1 = G * F2
   scales[SCALE_INV_GF2] = 1.f / (sg * sa * scales[SCALE_F1]);   // gF2 = G^T * F1
 }
-cudaError_t launch_feature_scales(float* scales, cudaStream_t stream) {
-  feature_scales_kernel<<<1, 1, 0, stream>>>(scales);
-  return cudaGetLastError();
+
+// Largest |x| * premul of up to ABSMAX_MAX arrays, each as the bits of a non-negative float combined into its slot of
+// scales[] with atomicMax (integer order = float order for non-negative values; NaNs are ignored), one atomic per
+// block; the block that finishes last (SCALE_TICKET counts them, and is left at zero) turns the magnitudes into the
+// multipliers.  One launch in place of one per array and one for the multipliers.  grid (blocks, arrays), block 256.
+constexpr int AM_THREADS = 256, AM_UNROLL = 4;
+struct AbsmaxJobs {
+  const float* p[ABSMAX_MAX];
+  size_t n[ABSMAX_MAX];
+  float premul[ABSMAX_MAX];
+  int slot[ABSMAX_MAX];
+};
+__global__ void __launch_bounds__(AM_THREADS)
+absmax_kernel(const AbsmaxJobs jobs, float* scales, int gradients) {
+  __shared__ float red[AM_THREADS / 32];
+  const int job = blockIdx.y;
+  const float* x = jobs.p[job];
+  const size_t n = jobs.n[job], n4 = n / 4, stride = (size_t)gridDim.x * AM_THREADS;
+  const float4* x4 = reinterpret_cast<const float4*>(x);  // the arrays are 16-byte aligned
+  float m = 0.f;
+  for (size_t i = (size_t)blockIdx.x * AM_THREADS + threadIdx.x; i < n4; i += AM_UNROLL * stride) {
+    float4 v[AM_UNROLL];
+#pragma unroll
+    for (int j = 0; j < AM_UNROLL; ++j) v[j] = i + j * stride < n4 ? __ldg(x4 + i + j * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < AM_UNROLL; ++j)
+      m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+  }
+  if (blockIdx.x == 0 && threadIdx.x < n - 4 * n4) m = fmaxf(m, fabsf(__ldg(x + 4 * n4 + threadIdx.x)));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int i = 1; i < AM_THREADS / 32; ++i) m = fmaxf(m, red[i]);
+  if (m > 0.f) atomicMax(reinterpret_cast<unsigned*>(scales) + jobs.slot[job], __float_as_uint(m * fabsf(jobs.premul[job])));
+  __threadfence();
+  unsigned* ticket = reinterpret_cast<unsigned*>(scales) + SCALE_TICKET;
+  if (atomicAdd(ticket, 1u) != gridDim.x * gridDim.y - 1) return;
+  __threadfence();
+  if (gradients) grad_scales(scales);
+  else feature_scales(scales);
+  *ticket = 0;
 }
-cudaError_t launch_grad_scales(float* scales, cudaStream_t stream) {
-  grad_scales_kernel<<<1, 1, 0, stream>>>(scales);
+
+cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, bool gradients, cudaStream_t stream) {
+  if (count < 1 || count > ABSMAX_MAX) return cudaErrorInvalidValue;
+  AbsmaxJobs jobs;
+  size_t most = 0;
+  for (int i = 0; i < ABSMAX_MAX; ++i) {
+    const AbsmaxSource& s = src[i < count ? i : 0];
+    jobs.p[i] = s.p;
+    jobs.n[i] = s.n;
+    jobs.premul[i] = s.premul;
+    jobs.slot[i] = s.slot;
+    most = std::max(most, s.n);
+  }
+  const size_t per_block = (size_t)AM_THREADS * 4 * AM_UNROLL;
+  const unsigned blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((most + per_block - 1) / per_block, 148 * 8));
+  absmax_kernel<<<dim3(blocks, count), AM_THREADS, 0, stream>>>(jobs, scales, gradients ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -95,31 +126,93 @@ __global__ void round_copy_kernel(const float4* __restrict__ in, float4* __restr
       if (op16 == OP16_FP16) outh[i] = make_uint2(pack_fp16x2(v.x * sc, v.y * sc), pack_fp16x2(v.z * sc, v.w * sc));
       else outh[i] = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
     }
-    v.x = round_tf32(v.x); v.y = round_tf32(v.y); v.z = round_tf32(v.z); v.w = round_tf32(v.w);
-    out[i] = v;
+    if (out != nullptr) {
+      v.x = round_tf32(v.x); v.y = round_tf32(v.y); v.z = round_tf32(v.z); v.w = round_tf32(v.w);
+      out[i] = v;
+    }
   }
 }
 
-// grid (H2 + W2, B), block = min(C, 256) threads over channels.
-__global__ void f2_means_kernel(const float* __restrict__ F2, float* __restrict__ aux, int H2, int W2, int C,
-                                uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
-  const int r = blockIdx.x, b = blockIdx.y;
-  const float* base = F2 + (size_t)b * H2 * W2 * C;
-  float* dst = aux + ((size_t)b * (H2 + W2) + r) * C;
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    float acc = 0.f;
-    if (r < H2) {
-      const float* row = base + (size_t)r * W2 * C + c;
-      for (int v = 0; v < W2; ++v) acc += __ldg(row + (size_t)v * C);
-      acc /= (float)W2;
-    } else {
-      const float* col = base + (size_t)(r - H2) * C + c;
-      for (int u = 0; u < H2; ++u) acc += __ldg(col + (size_t)u * W2 * C);
-      acc /= (float)H2;
+// One mean row, in the two forms the sweeps may read it: TF32 in `aux` or 16-bit in `auxh` (each may be null).
+__device__ __forceinline__ void store_mean(float mean, size_t at, float* aux, uint16_t* auxh, int op16, float sc16) {
+  if (aux != nullptr) aux[at] = round_tf32(mean);
+  if (auxh != nullptr) auxh[at] = to_op16(mean * sc16, op16);
+}
+
+// From pixel-major features.  A block owns one mean row; four groups of 64 threads take every fourth pixel of it, a
+// thread four channels at a time, so that the pixels' loads are in flight side by side.  grid (H2 + W2, B), block 256.
+constexpr int FM_GROUPS = 4, FM_QUADS = 64;
+__global__ void __launch_bounds__(FM_GROUPS * FM_QUADS)
+f2_means_kernel(const float* __restrict__ F2, float* __restrict__ aux, int H2, int W2, int C,
+                uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
+  __shared__ float4 red[FM_GROUPS][FM_QUADS];
+  const int r = blockIdx.x, b = blockIdx.y, g = threadIdx.x / FM_QUADS, q = threadIdx.x % FM_QUADS;
+  const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
+  const int count = r < H2 ? W2 : H2;
+  const size_t step = r < H2 ? (size_t)C : (size_t)W2 * C;   // between the pixels of the row / column
+  const float* base = F2 + (size_t)b * H2 * W2 * C + (r < H2 ? (size_t)r * W2 * C : (size_t)(r - H2) * C);
+  for (int c0 = 0; c0 < C; c0 += 4 * FM_QUADS) {   // C is a multiple of 4
+    const int c = c0 + 4 * q;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < C) {
+#pragma unroll 4
+      for (int i = g; i < count; i += FM_GROUPS) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(base + i * step + c));
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
     }
-    dst[c] = round_tf32(acc);
-    if (auxh != nullptr)
-      auxh[((size_t)b * (H2 + W2) + r) * C + c] = to_op16(op16 == OP16_FP16 && scale16 != nullptr ? acc * __ldg(scale16) : acc, op16);
+    red[g][q] = acc;
+    __syncthreads();
+    if (g == 0 && c < C) {
+#pragma unroll
+      for (int i = 1; i < FM_GROUPS; ++i) {
+        const float4 v = red[i][q];
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
+      const float n = (float)count;
+      const size_t at = ((size_t)b * (H2 + W2) + r) * C + c;
+      store_mean(acc.x / n, at, aux, auxh, op16, sc16);
+      store_mean(acc.y / n, at + 1, aux, auxh, op16, sc16);
+      store_mean(acc.z / n, at + 2, aux, auxh, op16, sc16);
+      store_mean(acc.w / n, at + 3, aux, auxh, op16, sc16);
+    }
+    __syncthreads();
+  }
+}
+
+// From channel-major feature maps: a block owns one channel plane, whose rows and columns it sums in two walks (the
+// second finds the plane in L2).  grid (C, B), block 256.
+__global__ void __launch_bounds__(256)
+f2_means_cf_kernel(const float* __restrict__ fmap2, float* __restrict__ aux, int H2, int W2, int C,
+                   uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
+  __shared__ float red[8][33];
+  const int c = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
+  const float* plane = fmap2 + ((size_t)b * C + c) * H2 * W2;
+  const size_t out0 = (size_t)b * (H2 + W2) * C + c;
+  for (int u = warp; u < H2; u += 8) {
+    float acc = 0.f;
+#pragma unroll 4
+    for (int v = lane; v < W2; v += 32) acc += __ldg(plane + (size_t)u * W2 + v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) store_mean(acc / (float)W2, out0 + (size_t)u * C, aux, auxh, op16, sc16);
+  }
+  for (int v0 = 0; v0 < W2; v0 += 32) {
+    const int v = v0 + lane;
+    float acc = 0.f;
+    if (v < W2) {
+#pragma unroll 4
+      for (int u = warp; u < H2; u += 8) acc += __ldg(plane + (size_t)u * W2 + v);
+    }
+    red[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && v < W2) {
+#pragma unroll
+      for (int i = 1; i < 8; ++i) acc += red[i][lane];
+      store_mean(acc / (float)H2, out0 + (size_t)(H2 + v) * C, aux, auxh, op16, sc16);
+    }
+    __syncthreads();
   }
 }
 
@@ -300,30 +393,68 @@ cudaError_t launch_unpack(const float* src, void* dst, int B, int N1, int n1p, i
   return cudaGetLastError();
 }
 
-// (B, C, N) -> (B, N, C), scaled and rounded to TF32.  32 x 32 tiles through shared memory; grid
-// (ceil(N/32), ceil(C/32), B), block (32, 8).
-__global__ void transpose_round_kernel(const float* __restrict__ in, float* __restrict__ out, int C, int N,
-                                       float scale, uint16_t* __restrict__ outh, int op16,
-                                       const float* __restrict__ scale16) {
-  __shared__ float tile[32][33];
-  const float sc16 = (outh != nullptr && op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
-  const int b = blockIdx.z, p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+// (B, C, N) -> (B, N, C) for both images in one launch, scaled: as TF32 in `out` or as 16-bit operands in `outh` (the one
+// that is not wanted is null).  Tiles of 64 channels x 32 pixels through shared memory, so that a warp writes 64 channels
+// of a pixel, two per lane; the first t1 blocks of a row do image 1.  grid (t1 + t2, ceil(C/64), B), block (32, 8).
+struct TransposeJob { const float* in; float* out; uint16_t* outh; const float* scale16; float scale; int N; };
+__global__ void __launch_bounds__(256)
+transpose_round_kernel(const TransposeJob j1, const TransposeJob j2, int t1, int C, int op16) {
+  __shared__ float tile[64][33];
+  const bool first = (int)blockIdx.x < t1;
+  const TransposeJob& j = first ? j1 : j2;
+  const int N = j.N;
+  const float sc16 = (j.outh != nullptr && op16 == OP16_FP16 && j.scale16 != nullptr) ? __ldg(j.scale16) : 1.f;
+  const int b = blockIdx.z, p0 = ((int)blockIdx.x - (first ? 0 : t1)) * 32, c0 = blockIdx.y * 64;
   const int tx = threadIdx.x, ty = threadIdx.y;
 #pragma unroll
-  for (int j = ty; j < 32; j += 8) {
-    const int c = c0 + j, p = p0 + tx;
-    tile[j][tx] = (c < C && p < N) ? __ldg(in + ((size_t)b * C + c) * N + p) : 0.f;
+  for (int i = 0; i < 8; ++i) {
+    const int c = c0 + ty + 8 * i, p = p0 + tx;
+    tile[ty + 8 * i][tx] = (c < C && p < N) ? __ldg(j.in + ((size_t)b * C + c) * N + p) * j.scale : 0.f;
   }
   __syncthreads();
 #pragma unroll
-  for (int j = ty; j < 32; j += 8) {
-    const int p = p0 + j, c = c0 + tx;
+  for (int i = 0; i < 4; ++i) {
+    const int p = p0 + ty + 8 * i, c = c0 + 2 * tx;   // C is even
     if (p < N && c < C) {
-      const float v = tile[tx][j] * scale;
-      out[((size_t)b * N + p) * C + c] = round_tf32(v);
-      if (outh != nullptr) outh[((size_t)b * N + p) * C + c] = to_op16(v * sc16, op16);
+      const float lo = tile[2 * tx][ty + 8 * i], hi = tile[2 * tx + 1][ty + 8 * i];
+      const size_t at = ((size_t)b * N + p) * C + c;
+      if (j.out != nullptr) *reinterpret_cast<float2*>(j.out + at) = make_float2(round_tf32(lo), round_tf32(hi));
+      if (j.outh != nullptr)
+        *reinterpret_cast<uint32_t*>(j.outh + at) = op16 == OP16_FP16 ? pack_fp16x2(lo * sc16, hi * sc16) : pack_bf16x2(lo, hi);
     }
   }
+}
+
+// 16-bit channel-major copies straight from the model's feature maps (B, C, rows*width), times `scale` and, for FP16, the
+// device scalar: the layouts of channel_major_kernel, padding included (zeros), two values per store.  One grid row per
+// channel of a sample: grid (ceil(pairs per channel / 256), C, B).
+__global__ void __launch_bounds__(256)
+channel_major_cf_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, int rows, int width, int pitch, int C,
+                        int blocked, float scale, int op16, const float* __restrict__ scale16) {
+  const int per_channel = blocked ? (width + 15) / 16 * pitch * 16 : pitch;
+  const int i = (blockIdx.x * 256 + threadIdx.x) * 2;
+  if (i >= per_channel) return;
+  const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
+  int row = 0, x = i;
+  if (blocked) {
+    const int xb = i / (pitch * 16), r = i - xb * pitch * 16;
+    row = r / 16;
+    x = xb * 16 + (r & 15);
+  }
+  const size_t chan = (size_t)blockIdx.z * C + blockIdx.y;
+  const float* src = in + (chan * rows + row) * width + x;
+  const bool ok = row < rows;
+  const float lo = ok && x < width ? __ldg(src) * scale : 0.f, hi = ok && x + 1 < width ? __ldg(src + 1) * scale : 0.f;
+  out[(chan * per_channel + i) / 2] = op16 == OP16_FP16 ? pack_fp16x2(lo * sc16, hi * sc16) : pack_bf16x2(lo, hi);
+}
+
+cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
+                                    int blocked, float scale, int op16, const float* scale16, cudaStream_t stream) {
+  const int per_channel = blocked ? (width + 15) / 16 * pitch * 16 : pitch;
+  const dim3 grid((per_channel / 2 + 255) / 256, C, B);
+  channel_major_cf_kernel<<<grid, 256, 0, stream>>>(src, reinterpret_cast<uint32_t*>(dst), rows, width, pitch, C, blocked,
+                                                    scale, op16, scale16);
+  return cudaGetLastError();
 }
 
 // Channel-major copies of a pixel-major feature array (B, rows*width, C), the K-major B operands of the gradient GEMMs.
@@ -370,14 +501,14 @@ cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, i
   return cudaGetLastError();
 }
 
-// Clears the workspace header (status word and scale slots) and, for FP16 operands, finds the two feature scales.
+// Clears the workspace header (status word, scale slots, counters) and, for FP16 operands, finds the two feature scales.
 static cudaError_t begin_prepare(const Dims& d, const float* F1, const float* F2, float premul1, int* status, int op16,
                                  float* scales, cudaStream_t stream) {
   cudaError_t err = cudaMemsetAsync(status, 0, WS_HEADER_CLEAR_BYTES, stream);
   if (err != cudaSuccess || op16 != OP16_FP16 || scales == nullptr) return err;
-  launch_absmax(F1, (size_t)d.B * d.N1() * d.C, premul1, scales + SCALE_AMAX_F1, stream);
-  launch_absmax(F2, (size_t)d.B * d.N2() * d.C, 1.f, scales + SCALE_AMAX_F2, stream);
-  return launch_feature_scales(scales, stream);
+  const AbsmaxSource src[2] = {{F1, (size_t)d.B * d.N1() * d.C, premul1, SCALE_AMAX_F1},
+                               {F2, (size_t)d.B * d.N2() * d.C, 1.f, SCALE_AMAX_F2}};
+  return launch_absmax(src, 2, scales, false, stream);
 }
 
 cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fmap2, float scale1, float* F1r,
@@ -387,15 +518,13 @@ cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fm
   if (err != cudaSuccess) return err;
   const float* s1 = (op16 == OP16_FP16 && scales != nullptr) ? scales + SCALE_F1 : nullptr;
   const float* s2 = (op16 == OP16_FP16 && scales != nullptr) ? scales + SCALE_F2 : nullptr;
-  const dim3 block(32, 8);
-  transpose_round_kernel<<<dim3((d.N1() + 31) / 32, (d.C + 31) / 32, d.B), block, 0, stream>>>(
-      fmap1, F1r, d.C, d.N1(), scale1, F1h, op16, s1);
-  transpose_round_kernel<<<dim3((d.N2() + 31) / 32, (d.C + 31) / 32, d.B), block, 0, stream>>>(
-      fmap2, F2r, d.C, d.N2(), 1.f, F2h, op16, s2);
-  if (aux != nullptr) {  // mean rows from the transposed copy (already rounded: the means differ by < 2^-12 relative)
-    const dim3 grid(d.H2 + d.W2, d.B);
-    f2_means_kernel<<<grid, std::min(d.C, 256), 0, stream>>>(F2r, aux, d.H2, d.W2, d.C, auxh, op16, s2);
+  if (F1r != nullptr || F1h != nullptr) {
+    const int t1 = (d.N1() + 31) / 32, t2 = (d.N2() + 31) / 32;
+    const TransposeJob j1{fmap1, F1r, F1h, s1, scale1, d.N1()}, j2{fmap2, F2r, F2h, s2, 1.f, d.N2()};
+    transpose_round_kernel<<<dim3(t1 + t2, (d.C + 63) / 64, d.B), dim3(32, 8), 0, stream>>>(j1, j2, t1, d.C, op16);
   }
+  if (aux != nullptr || auxh != nullptr)
+    f2_means_cf_kernel<<<dim3(d.C, d.B), 256, 0, stream>>>(fmap2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
   return cudaGetLastError();
 }
 
@@ -409,16 +538,16 @@ cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, floa
   const size_t n1 = (size_t)d.B * d.N1() * d.C / 4, n2 = (size_t)d.B * d.N2() * d.C / 4;  // C % 4 == 0
   const int threads = 256;
   auto blocks = [&](size_t n) { return (unsigned)std::min<size_t>((n + threads - 1) / threads, 148 * 16); };
-  round_copy_kernel<<<blocks(n1), threads, 0, stream>>>(reinterpret_cast<const float4*>(F1),
-                                                        reinterpret_cast<float4*>(F1r), n1,
-                                                        reinterpret_cast<uint2*>(F1h), op16, s1);
-  round_copy_kernel<<<blocks(n2), threads, 0, stream>>>(reinterpret_cast<const float4*>(F2),
-                                                        reinterpret_cast<float4*>(F2r), n2,
-                                                        reinterpret_cast<uint2*>(F2h), op16, s2);
-  if (aux != nullptr) {
-    const dim3 grid(d.H2 + d.W2, d.B);
-    f2_means_kernel<<<grid, std::min(d.C, 256), 0, stream>>>(F2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
+  if (F1r != nullptr || F1h != nullptr) {
+    round_copy_kernel<<<blocks(n1), threads, 0, stream>>>(reinterpret_cast<const float4*>(F1),
+                                                          reinterpret_cast<float4*>(F1r), n1,
+                                                          reinterpret_cast<uint2*>(F1h), op16, s1);
+    round_copy_kernel<<<blocks(n2), threads, 0, stream>>>(reinterpret_cast<const float4*>(F2),
+                                                          reinterpret_cast<float4*>(F2r), n2,
+                                                          reinterpret_cast<uint2*>(F2h), op16, s2);
   }
+  if (aux != nullptr || auxh != nullptr)
+    f2_means_kernel<<<dim3(d.H2 + d.W2, d.B), FM_GROUPS * FM_QUADS, 0, stream>>>(F2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
   return cudaGetLastError();
 }
 
