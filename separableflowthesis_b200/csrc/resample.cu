@@ -20,43 +20,82 @@ __device__ __forceinline__ void resample_source(int d, float scale, int Dl, int&
   l0 = 1.f - l1;
 }
 
-// grid (ceil(N1/128), ceil(D0/RS_DB), B*K): a thread produces RS_DB output rows of its pixel, all loads first
+// A thread produces RS_DB output rows of its VEC neighbouring pixels, all loads first.  VEC = 4 (16-byte loads and stores)
+// when the planes allow it: a row is a coalesced store of two interpolated loads, and with 4-byte accesses the number of
+// instructions, not HBM, set the pace.  grid (ceil(N1/(128*VEC)), ceil(D0/RS_DB), B*K)
 constexpr int RS_DB = 8;
 
-__global__ void upsample_displacement_kernel(const float* __restrict__ in, float* __restrict__ out, long long out_sb,
-                                             int K, int Dl, int D0, int N1, float scale) {
-  const int p = blockIdx.x * RS_THREADS + threadIdx.x, d0 = blockIdx.y * RS_DB;
+template <int VEC> struct RsVec;
+template <> struct RsVec<1> { typedef float type; };
+template <> struct RsVec<4> { typedef float4 type; };
+__device__ __forceinline__ float rs_mix(float a, float b, float l0, float l1) { return l0 * a + l1 * b; }
+__device__ __forceinline__ float4 rs_mix(const float4& a, const float4& b, float l0, float l1) {
+  return make_float4(rs_mix(a.x, b.x, l0, l1), rs_mix(a.y, b.y, l0, l1), rs_mix(a.z, b.z, l0, l1), rs_mix(a.w, b.w, l0, l1));
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(RS_THREADS)
+upsample_displacement_kernel(const float* __restrict__ in, float* __restrict__ out, long long out_sb, int K, int Dl,
+                             int D0, int N1, float scale) {
+  typedef typename RsVec<VEC>::type V;
+  const int p = (blockIdx.x * RS_THREADS + threadIdx.x) * VEC, d0 = blockIdx.y * RS_DB;
   if (p >= N1) return;
   const int b = blockIdx.z / K, k = blockIdx.z - b * K;
   const float* src = in + ((size_t)blockIdx.z * Dl) * N1 + p;
-  float v0[RS_DB], v1[RS_DB], l0[RS_DB], l1[RS_DB];
+  V v0[RS_DB], v1[RS_DB];
+  float l0[RS_DB], l1[RS_DB];
 #pragma unroll
   for (int j = 0; j < RS_DB; ++j) {
     int i0, i1;
     resample_source(min(d0 + j, D0 - 1), scale, Dl, i0, i1, l0[j], l1[j]);
-    v0[j] = __ldg(src + (size_t)i0 * N1);
-    v1[j] = __ldg(src + (size_t)i1 * N1);
+    v0[j] = __ldg(reinterpret_cast<const V*>(src + (size_t)i0 * N1));
+    v1[j] = __ldg(reinterpret_cast<const V*>(src + (size_t)i1 * N1));
   }
   float* dst = out + (size_t)b * out_sb + ((size_t)k * D0 + d0) * N1 + p;
 #pragma unroll
   for (int j = 0; j < RS_DB; ++j)
-    if (d0 + j < D0) dst[(size_t)j * N1] = l0[j] * v0[j] + l1[j] * v1[j];
+    if (d0 + j < D0) *reinterpret_cast<V*>(dst + (size_t)j * N1) = rs_mix(v0[j], v1[j], l0[j], l1[j]);
 }
 
-// gin[b][k][i][p] = sum over d of the weights with which output row d read input row i.  grid (ceil(N1/128), B*K)
-__global__ void upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long gout_sb,
-                                                     float* __restrict__ gin, int K, int Dl, int D0, int N1,
-                                                     float scale) {
+// gin[b][k][i][p] = sum over d of the weights with which output row d read input row i, added in the order of d.  A
+// thread produces the RS_IB rows from r0 on: it walks the output rows whose lower neighbour is r0 - 1 .. r0 + RS_IB - 1
+// (one thread for a whole column was too few threads for small images).  grid (ceil(N1/128), B*K, ceil(Dl/RS_IB))
+constexpr int RS_IB = 8;
+
+__global__ void __launch_bounds__(RS_THREADS)
+upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long gout_sb, float* __restrict__ gin, int K,
+                                     int Dl, int D0, int N1, float scale) {
   const int p = blockIdx.x * RS_THREADS + threadIdx.x;
   if (p >= N1) return;
   const int b = blockIdx.y / K, k = blockIdx.y - b * K;
+  const int r0 = blockIdx.z * RS_IB, r1 = min(r0 + RS_IB, Dl);
   const float* g = gout + (size_t)b * gout_sb + ((size_t)k * D0) * N1 + p;
   float* dst = gin + ((size_t)blockIdx.y * Dl) * N1 + p;
+  // first output row with lower neighbour >= r0 - 1: an estimate, corrected with the exact rule (neighbours never fall
+  // as d grows)
+  int first = 0;
+  if (r0 > 1) {
+    int i0, i1;
+    float l0, l1;
+    first = max(0, min(D0 - 1, (int)((float)(r0 - 1) / scale) - 1));
+    for (; first > 0; --first) {
+      resample_source(first - 1, scale, Dl, i0, i1, l0, l1);
+      if (i0 < r0 - 1) break;
+    }
+    for (; first < D0; ++first) {
+      resample_source(first, scale, Dl, i0, i1, l0, l1);
+      if (i0 >= r0 - 1) break;
+    }
+  }
   // the source row grows by at most one per output row (Dl <= D0): two running sums cover rows cur and cur + 1
-  int cur = 0;
+  int cur = r0 > 0 ? r0 - 1 : 0;
   float acc0 = 0.f, acc1 = 0.f;
+  auto put = [&](int i, float v) {
+    if (i >= r0 && i < r1) dst[(size_t)i * N1] = v;
+  };
   constexpr int DB = 8;  // output rows loaded per batch
-  for (int d0 = 0; d0 < D0; d0 += DB) {
+  bool done = false;
+  for (int d0 = first; d0 < D0 && !done; d0 += DB) {
     float gv[DB];
 #pragma unroll
     for (int j = 0; j < DB; ++j) gv[j] = d0 + j < D0 ? __ldg(g + (size_t)(d0 + j) * N1) : 0.f;
@@ -66,8 +105,9 @@ __global__ void upsample_displacement_adjoint_kernel(const float* __restrict__ g
       int i0, i1;
       float l0, l1;
       resample_source(d0 + j, scale, Dl, i0, i1, l0, l1);
+      if (i0 >= r1) { done = true; break; }
       while (cur < i0) {  // at most one step
-        dst[(size_t)cur * N1] = acc0;
+        put(cur, acc0);
         acc0 = acc1;
         acc1 = 0.f;
         ++cur;
@@ -77,23 +117,26 @@ __global__ void upsample_displacement_adjoint_kernel(const float* __restrict__ g
       else acc0 = fmaf(l1, gv[j], acc0);
     }
   }
-  dst[(size_t)cur * N1] = acc0;
-  if (cur + 1 < Dl) dst[(size_t)(cur + 1) * N1] = acc1;
-  for (int i = cur + 2; i < Dl; ++i) dst[(size_t)i * N1] = 0.f;
+  put(cur, acc0);
+  put(cur + 1, acc1);
+  for (int i = cur + 2; i < r1; ++i) put(i, 0.f);
 }
 
 static float resample_scale(int Dl, int D0) { return D0 > 1 ? (float)(Dl - 1) / (float)(D0 - 1) : 0.f; }
 
 cudaError_t launch_upsample_displacement(const float* in, float* out, long long out_sb, int B, int K, int Dl, int D0,
                                          int N1, cudaStream_t st) {
-  const dim3 grid((N1 + RS_THREADS - 1) / RS_THREADS, (D0 + RS_DB - 1) / RS_DB, B * K);
-  upsample_displacement_kernel<<<grid, RS_THREADS, 0, st>>>(in, out, out_sb, K, Dl, D0, N1, resample_scale(Dl, D0));
+  const bool vec = N1 % 4 == 0 && out_sb % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+  const int px = RS_THREADS * (vec ? 4 : 1);
+  const dim3 grid((N1 + px - 1) / px, (D0 + RS_DB - 1) / RS_DB, B * K);
+  auto kern = vec ? upsample_displacement_kernel<4> : upsample_displacement_kernel<1>;
+  kern<<<grid, RS_THREADS, 0, st>>>(in, out, out_sb, K, Dl, D0, N1, resample_scale(Dl, D0));
   return cudaGetLastError();
 }
 
 cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
                                                  int D0, int N1, cudaStream_t st) {
-  const dim3 grid((N1 + RS_THREADS - 1) / RS_THREADS, B * K);
+  const dim3 grid((N1 + RS_THREADS - 1) / RS_THREADS, B * K, (Dl + RS_IB - 1) / RS_IB);
   upsample_displacement_adjoint_kernel<<<grid, RS_THREADS, 0, st>>>(gout, gout_sb, gin, K, Dl, D0, N1,
                                                                     resample_scale(Dl, D0));
   return cudaGetLastError();
