@@ -8,14 +8,13 @@
 // average-pooled image-2 features, so level l needs only the pooled features, never the volume.
 //
 // Work per (pixel, level): the (2r+2)^2 dot products of the pixel's feature row with the image-2 feature rows at
-// the integer positions under its window, then (2r+1)^2 bilinear combinations of them.  A gather bound by the
-// L1/L2 path of the image-2 rows (1 KB each at C = 256), so the kernel shares them: a warp takes four
-// neighbouring pixels, whose windows mostly overlap because neighbouring pixels move alike, walks the bounding box
-// of the four windows once, and uses every loaded image-2 row for all four pixels (feature rows of the four pixels
-// in registers, lanes split the channels).  Partial sums of 32 (position, pixel) pairs are reduced together with a
-// 31-shuffle transpose.  When the four windows lie far apart (a motion boundary, a wrap to the next image row) the
-// warp falls back to one pixel at a time.  A CTA covers 32 consecutive pixels and stages its outputs in shared
-// memory so that the (B, levels*(2r+1)^2, H1, W1) result is written in full 128-byte lines.
+// the integer positions under its window, then (2r+1)^2 bilinear combinations of them.  The image-2 rows (1 KB each at
+// C = 256) come through L1/L2, so the kernels share them: a walk serves a block of neighbouring pixels, whose windows
+// mostly overlap because neighbouring pixels move alike, visits the bounding box of their windows once, and uses every
+// loaded image-2 row for all of them (their feature rows in registers, lanes split the channels).  Partial sums of 32
+// (position, pixel) pairs are reduced together with a 31-shuffle transpose.  When the windows lie far apart (a motion
+// boundary) the walk is done for fewer pixels at a time.  A CTA covers 8 x 4 pixels and stages its outputs in shared
+// memory, so that the (B, levels*(2r+1)^2, H1, W1) result is written in runs of eight pixels (a 32-byte sector).
 //
 // Backward (features only: the model detaches the coordinates, core/sepflow.py:193): the same walk with the roles
 // swapped.  The gradient of a pixel's window is spread back onto the integer positions (each takes from at most four
@@ -24,22 +23,16 @@
 #include <climits>
 
 #include "kernels.h"
+#include "sm100_primitives.cuh"
 
 namespace sfb {
 
-constexpr int L4_THREADS = 256;
-constexpr int L4_WARPS = L4_THREADS / 32;
-constexpr int L4_PX = 4;                       // pixels per warp
-constexpr int L4_TILE = L4_WARPS * L4_PX;      // pixels per CTA
+constexpr int L4_TW = 8, L4_TH = 4;            // image-1 pixels of a CTA: two-dimensional, so that windows overlap
+constexpr int L4_TILE = L4_TW * L4_TH;
 constexpr int L4_RMAX = 4;
 constexpr int L4_WIN = 2 * L4_RMAX + 1;        // window side
-constexpr int L4_BW = 16, L4_BH = 12;          // largest bounding box a four-pixel pass accepts
-constexpr int L4_BMAX = L4_BW * L4_BH;
-#ifndef L4_BWD_STEP
-#define L4_BWD_STEP 2
-#endif
+constexpr int L4_SIDE = 2 * L4_RMAX + 2;       // integer positions under a window, per side
 static_assert(L4_TILE == 32, "the output staging assumes 32 pixels per CTA");
-static_assert((2 * L4_RMAX + 2) * (2 * L4_RMAX + 2) <= L4_BMAX, "one pixel's positions must fit the buffer");
 
 struct Lookup4dLevels {
   const float* f2[LOOKUP_MAX_LEVELS];   // level l: (B, H2_l, W2_l, C)
@@ -66,8 +59,23 @@ struct L4Pixel {     // geometry of one pixel at one level
   int bx, by;        // integer position under the window centre
 };
 
-__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
-  return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, acc))));
+// Bounding box of the integer positions of several pixels' windows.
+struct L4Box {
+  int ox, oy, bw, bh;
+};
+
+// Four channels as two packed pairs: one fma.rn.f32x2 per pair.
+struct L4Quad {
+  uint64_t lo, hi;
+};
+__device__ __forceinline__ L4Quad l4_load(const float* p, bool ok) {
+  L4Quad q{0ull, 0ull};
+  if (ok) {
+    const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(p));
+    q.lo = t.x;
+    q.hi = t.y;
+  }
+  return q;
 }
 
 // v[i] of all lanes summed; lane i keeps the total of v[i].  31 shuffles for 32 values.
@@ -93,44 +101,72 @@ __device__ __forceinline__ float l4_fraction(float c, int base, int t, int radiu
   return pos - (float)(base + t - radius);
 }
 
-__device__ __forceinline__ void l4_pixel_geometry(const float* __restrict__ coords, int b, int p, int N1, int level,
-                                                  int H2, int W2, L4Pixel& g) {
+__device__ __forceinline__ L4Pixel l4_pixel_geometry(const float* __restrict__ coords, int b, int p, int N1, int level,
+                                                     int H2, int W2) {
+  L4Pixel g;
   const float inv = 1.f / (float)(1 << level);
   g.cx = __ldg(coords + ((size_t)b * 2 + 0) * N1 + p) * inv;
   g.cy = __ldg(coords + ((size_t)b * 2 + 1) * N1 + p) * inv;
   g.bx = l4_floor(l4_unnormalise(g.cx, W2));
   g.by = l4_floor(l4_unnormalise(g.cy, H2));
+  return g;
 }
 
-// Dot products of NPX pixels' feature rows with the image-2 rows of a bounding box (ox, oy, bw x bh), scaled, into
-// S[px][row * bw + col]; zero outside the image.
+// Box of the pixels in `mask` (lanes hold one pixel each); every lane gets it.  An empty mask gives an empty box.
+__device__ __forceinline__ L4Box l4_box(const L4Pixel& g, unsigned mask, int radius, int lane) {
+  const bool in = (mask >> lane) & 1u;
+  const int xmin = __reduce_min_sync(0xffffffffu, in ? g.bx : INT_MAX), xmax = __reduce_max_sync(0xffffffffu, in ? g.bx : INT_MIN);
+  const int ymin = __reduce_min_sync(0xffffffffu, in ? g.by : INT_MAX), ymax = __reduce_max_sync(0xffffffffu, in ? g.by : INT_MIN);
+  if (mask == 0) return L4Box{0, 0, 0, 0};
+  return L4Box{xmin - radius, ymin - radius, xmax - xmin + 2 * radius + 2, ymax - ymin + 2 * radius + 2};
+}
+__device__ __forceinline__ bool l4_fits(const L4Box& box, int limit) {  // extents are at most 2e6 + 10: no overflow in 64 bits
+  return (long long)box.bw * box.bh <= limit;
+}
+
+// Image-2 row of every box position (-1: outside the image, or padding up to a multiple of 32), so that the walk below
+// spends one broadcast load per position instead of a division and four comparisons.
+__device__ __forceinline__ void l4_fill_rows(int* rows, const L4Box& box, int H2, int W2, int lane) {
+  const int nq = box.bw * box.bh;
+  for (int q = lane; q < (nq + 31) / 32 * 32; q += 32) {
+    const int row = q / box.bw, x = box.ox + q - row * box.bw, y = box.oy + row;
+    rows[q] = (q < nq && x >= 0 && x < W2 && y >= 0 && y < H2) ? y * W2 + x : -1;
+  }
+}
+
+// ---- forward ----------------------------------------------------------------------------------------------
+// A CTA owns 8 x 4 pixels at one level, a warp 2 x 2 of them: one walk over the box of their windows with the four
+// pixels' feature rows in registers (lanes split the channels).  Bound by instruction issue: the products are packed
+// pairs and the positions come from a table.
+constexpr int L4_THREADS = 256;
+constexpr int L4_WARPS = L4_THREADS / 32;
+constexpr int L4_PX = 4;
+constexpr int L4_BMAX = 224;                   // largest box a four-pixel walk accepts
+static_assert(L4_SIDE * L4_SIDE <= L4_BMAX && L4_BMAX % 32 == 0, "one pixel's positions must fit the table");
+
+// Dot products of NPX pixels' feature rows with the image-2 rows of a box, scaled, into S[px0 + px][position]; zero
+// outside the image.
 template <int NCH, int NPX>
-__device__ __forceinline__ void l4_box_products(const float4 (&f1)[L4_PX][NCH], const float* __restrict__ F2b, int H2,
-                                                int W2, int C, int ox, int oy, int bw, int bh, float scale,
-                                                float (*S)[L4_BMAX], int px0, int lane) {
+__device__ __forceinline__ void l4_box_products(const L4Quad (&f1)[NPX][NCH], const float* __restrict__ F2b, int C,
+                                                const int* rows, int nq, float scale, float (*S)[L4_BMAX], int px0,
+                                                int lane) {
   constexpr int QB = 32 / NPX;
-  const int nq = bw * bh;
   for (int q0 = 0; q0 < nq; q0 += QB) {
     float v[32];
 #pragma unroll
     for (int qi = 0; qi < QB; ++qi) {
-      const int q = q0 + qi;
-      const int row = q / bw, col = q - row * bw;
-      const int x = ox + col, y = oy + row;
-      const bool in = q < nq && x >= 0 && x < W2 && y >= 0 && y < H2;
-      float4 f2[NCH];
+      const int r = rows[q0 + qi];
+      const float* src = F2b + (size_t)(r < 0 ? 0 : r) * C + lane * 4;
+      L4Quad f2[NCH];
 #pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        const int c = ch * 128 + lane * 4;
-        f2[ch] = (in && c < C) ? __ldg(reinterpret_cast<const float4*>(F2b + ((size_t)y * W2 + x) * C + c))
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+      for (int ch = 0; ch < NCH; ++ch) f2[ch] = l4_load(src + ch * 128, r >= 0 && ch * 128 + lane * 4 < C);
 #pragma unroll
       for (int px = 0; px < NPX; ++px) {
-        float acc = 0.f;
+        uint64_t acc = mul2(f1[px][0].lo, f2[0].lo);
+        acc = fma2(f1[px][0].hi, f2[0].hi, acc);
 #pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) acc = dot4(f1[px][ch], f2[ch], acc);
-        v[qi * NPX + px] = acc;
+        for (int ch = 1; ch < NCH; ++ch) acc = fma2(f1[px][ch].hi, f2[ch].hi, fma2(f1[px][ch].lo, f2[ch].lo, acc));
+        v[qi * NPX + px] = sum2(acc);
       }
     }
     const float total = warp_transpose_reduce(v, lane);
@@ -139,187 +175,211 @@ __device__ __forceinline__ void l4_box_products(const float4 (&f1)[L4_PX][NCH], 
   }
 }
 
-// grid (ceil(N1 / 32), levels, B)
+// grid (ceil(W1/8) * ceil(H1/4), levels, B)
 template <int NCH>
 __global__ void __launch_bounds__(L4_THREADS, 2)
 lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
-                        float* __restrict__ out, int N1, int C, int radius, int levels, float scale) {
+                        float* __restrict__ out, int H1, int W1, int C, int radius, int levels, float scale) {
   __shared__ float s_S[L4_WARPS][L4_PX][L4_BMAX];
   __shared__ float s_out[L4_WIN * L4_WIN][L4_TILE + 1];
+  __shared__ int s_rows[L4_WARPS][L4_BMAX];
   __shared__ L4Pixel s_geo[L4_WARPS][L4_PX];
 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int level = blockIdx.y, b = blockIdx.z;
+  const int level = blockIdx.y, b = blockIdx.z, N1 = H1 * W1;
   const int H2 = lv.H2[level], W2 = lv.W2[level];
   const float* F2b = lv.f2[level] + (size_t)b * H2 * W2 * C;
-  const int p0 = blockIdx.x * L4_TILE + w * L4_PX;
+  const int tiles_x = (W1 + L4_TW - 1) / L4_TW;
+  const int h0 = (int)(blockIdx.x / tiles_x) * L4_TH, w0 = (int)(blockIdx.x % tiles_x) * L4_TW;
   const int win = 2 * radius + 1;
+  // warp w: columns 2*(w%4) .., rows 2*(w/4) .. of the tile; its pixel px: column px%2, row px/2
+  const int ph = h0 + 2 * (w >> 2), pw = w0 + 2 * (w & 3);
 
-  // geometry of the warp's pixels and the bounding box of their windows
-  int xmin = INT_MAX, xmax = INT_MIN, ymin = INT_MAX, ymax = INT_MIN;
-  if (lane < L4_PX && p0 + lane < N1) {
-    L4Pixel g;
-    l4_pixel_geometry(coords, b, p0 + lane, N1, level, H2, W2, g);
-    s_geo[w][lane] = g;
-    xmin = xmax = g.bx;
-    ymin = ymax = g.by;
-  }
-#pragma unroll
-  for (int off = 1; off < L4_PX; off <<= 1) {
-    xmin = min(xmin, __shfl_xor_sync(0xffffffffu, xmin, off));
-    xmax = max(xmax, __shfl_xor_sync(0xffffffffu, xmax, off));
-    ymin = min(ymin, __shfl_xor_sync(0xffffffffu, ymin, off));
-    ymax = max(ymax, __shfl_xor_sync(0xffffffffu, ymax, off));
-  }
-  xmin = __shfl_sync(0xffffffffu, xmin, 0); xmax = __shfl_sync(0xffffffffu, xmax, 0);
-  ymin = __shfl_sync(0xffffffffu, ymin, 0); ymax = __shfl_sync(0xffffffffu, ymax, 0);
-  __syncwarp();
-  const int npx = min(L4_PX, N1 - p0);   // <= 0: nothing to do for this warp
+  L4Pixel geo{0.f, 0.f, 0, 0};
+  const int mh = ph + ((lane >> 1) & 1), mw = pw + (lane & 1);
+  const bool mine = lane < L4_PX && mh < H1 && mw < W1;
+  if (mine) geo = l4_pixel_geometry(coords, b, mh * W1 + mw, N1, level, H2, W2);
+  if (lane < L4_PX) s_geo[w][lane] = geo;
+  const unsigned mask = __ballot_sync(0xffffffffu, mine);
 
-  if (npx > 0) {
-    float4 f1[L4_PX][NCH];
+  if (mask != 0) {
+    L4Quad f1[L4_PX][NCH];
 #pragma unroll
     for (int px = 0; px < L4_PX; ++px)
 #pragma unroll
       for (int ch = 0; ch < NCH; ++ch) {
         const int c = ch * 128 + lane * 4;
-        f1[px][ch] = (px < npx && c < C)
-                         ? __ldg(reinterpret_cast<const float4*>(F1 + ((size_t)b * N1 + p0 + px) * C + c))
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        const size_t p = (size_t)b * N1 + (size_t)(ph + px / 2) * W1 + pw + px % 2;
+        const bool ok = ((mask >> px) & 1u) && c < C;
+        f1[px][ch] = l4_load(F1 + (ok ? p * C + c : 0), ok);
       }
 
-    const int bw = xmax - xmin + 2 * radius + 2, bh = ymax - ymin + 2 * radius + 2;
-    const bool together = bw <= L4_BW && bh <= L4_BH;
+    L4Box box = l4_box(geo, mask, radius, lane);
+    const bool together = l4_fits(box, L4_BMAX);
     if (together) {
-      l4_box_products<NCH, L4_PX>(f1, F2b, H2, W2, C, xmin - radius, ymin - radius, bw, bh, scale, s_S[w], 0, lane);
-    } else {
+      l4_fill_rows(s_rows[w], box, H2, W2, lane);
+      __syncwarp();
+      l4_box_products<NCH, L4_PX>(f1, F2b, C, s_rows[w], box.bw * box.bh, scale, s_S[w], 0, lane);
+    } else {  // motion boundaries: one pixel at a time
 #pragma unroll
       for (int px = 0; px < L4_PX; ++px) {
-        if (px >= npx) break;
-        float4 one[L4_PX][NCH];
+        if (!((mask >> px) & 1u)) continue;
+        L4Quad one[1][NCH];
 #pragma unroll
         for (int ch = 0; ch < NCH; ++ch) one[0][ch] = f1[px][ch];
-        const L4Pixel g = s_geo[w][px];
-        l4_box_products<NCH, 1>(one, F2b, H2, W2, C, g.bx - radius, g.by - radius, 2 * radius + 2, 2 * radius + 2,
-                                scale, s_S[w], px, lane);
+        box = l4_box(geo, 1u << px, radius, lane);
+        __syncwarp();
+        l4_fill_rows(s_rows[w], box, H2, W2, lane);
+        __syncwarp();
+        l4_box_products<NCH, 1>(one, F2b, C, s_rows[w], box.bw * box.bh, scale, s_S[w], px, lane);
       }
     }
     __syncwarp();
 
     // bilinear combinations
-    for (int idx = lane; idx < npx * win * win; idx += 32) {
+    for (int idx = lane; idx < L4_PX * win * win; idx += 32) {
       const int px = idx / (win * win), o = idx - px * win * win;
+      if (!((mask >> px) & 1u)) continue;
       const int a = o / win, bb = o - a * win;
       const L4Pixel g = s_geo[w][px];
-      const int ox = together ? xmin - radius : g.bx - radius;
-      const int oy = together ? ymin - radius : g.by - radius;
-      const int sbw = together ? bw : 2 * radius + 2;
+      const int ox = together ? box.ox : g.bx - radius;
+      const int oy = together ? box.oy : g.by - radius;
+      const int sbw = together ? box.bw : 2 * radius + 2;
       const float fx = l4_fraction(g.cx, g.bx, a, radius, W2);
       const float fy = l4_fraction(g.cy, g.by, bb, radius, H2);
       const float* S = s_S[w][px] + (g.by + bb - radius - oy) * sbw + (g.bx + a - radius - ox);
       const float top = S[0] + fx * (S[1] - S[0]);
       const float bot = S[sbw] + fx * (S[sbw + 1] - S[sbw]);
-      s_out[o][w * L4_PX + px] = top + fy * (bot - top);
+      s_out[o][(2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2] = top + fy * (bot - top);
     }
   }
   __syncthreads();
-  const int pbase = blockIdx.x * L4_TILE;
   for (int i = threadIdx.x; i < win * win * L4_TILE; i += L4_THREADS) {
-    const int o = i / L4_TILE, pp = i % L4_TILE;
-    if (pbase + pp < N1)
-      out[(((size_t)b * levels + level) * win * win + o) * N1 + pbase + pp] = s_out[o][pp];
+    const int o = i / L4_TILE, pp = i % L4_TILE, h = h0 + pp / L4_TW, x = w0 + pp % L4_TW;
+    if (h < H1 && x < W1) out[(((size_t)b * levels + level) * win * win + o) * N1 + (size_t)h * W1 + x] = s_out[o][pp];
   }
 }
 
-__device__ __forceinline__ void red_add_v4(float* addr, const float4& v) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-               : "memory");
+// ---- backward ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void red_add_v4(float* addr, uint64_t lo, uint64_t hi) {
+  float x, y, z, w;
+  unpack2(lo, x, y);
+  unpack2(hi, z, w);
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
-// One walk of a bounding box in the backward: gS[px][q] (already scaled) is in shared memory.
+// One walk of a box for the pixels px0 .. px0+NPX-1: gS[px][position] (already scaled) is in shared memory.
 template <int NCH, int NPX>
-__device__ __forceinline__ void l4_box_gradients(const float4 (&f1)[L4_PX][NCH], float4 (&gf1)[L4_PX][NCH],
-                                                 const float* __restrict__ F2b, float* __restrict__ G2b, int H2, int W2,
-                                                 int C, int ox, int oy, int bw, int bh, float (*gS)[L4_BMAX], int px0,
-                                                 int lane) {
-  // L4_BWD_STEP positions of a row per step: their image-2 rows are all requested before any is used
-  constexpr int J = L4_BWD_STEP;
-  for (int row = 0; row < bh; ++row) {
-    const int y = oy + row;
-    if (y < 0 || y >= H2) continue;
-    for (int col = 0; col < bw; col += J) {
-      bool in[J];
-      float4 f2[J][NCH];
-      float g[J][NPX];
-      size_t at[J];
+__device__ __forceinline__ void l4_box_gradients(const L4Quad (&f1)[L4_PX][NCH], L4Quad (&gf1)[L4_PX][NCH],
+                                                 const float* __restrict__ F2b, float* __restrict__ G2b, int C,
+                                                 const int* rows, int nq, const float (*gS)[L4_BMAX], int px0, int lane) {
+  constexpr int J = NCH > 2 ? 1 : 4 / NCH;   // positions per step: their image-2 rows are all requested before any is used
+  for (int q0 = 0; q0 < nq; q0 += J) {
+    int r[J];
+    L4Quad f2[J][NCH];
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const int x = ox + col + j;
-        in[j] = col + j < bw && x >= 0 && x < W2;
-        at[j] = ((size_t)y * W2 + (in[j] ? x : 0)) * C;
+    for (int j = 0; j < J; ++j) {
+      r[j] = rows[q0 + j];   // -1 past the box
+      const float* src = F2b + (size_t)(r[j] < 0 ? 0 : r[j]) * C + lane * 4;
 #pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) {
-          const int c = ch * 128 + lane * 4;
-          f2[j][ch] = (in[j] && c < C) ? __ldg(reinterpret_cast<const float4*>(F2b + at[j] + c))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+      for (int ch = 0; ch < NCH; ++ch) f2[j][ch] = l4_load(src + ch * 128, r[j] >= 0 && ch * 128 + lane * 4 < C);
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      if (r[j] < 0) continue;
+      float g[NPX];
+      bool any = false;
+#pragma unroll
+      for (int k = 0; k < NPX; ++k) {
+        g[k] = gS[px0 + k][q0 + j];
+        any |= g[k] != 0.f;
       }
+      if (!any) continue;   // no pixel of the walk has this position in its window
+      uint64_t gg[NPX];
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
-        bool any = false;
+      for (int k = 0; k < NPX; ++k) gg[k] = pack2(g[k], g[k]);
+      float* dst = G2b + (size_t)r[j] * C + lane * 4;
 #pragma unroll
-        for (int px = 0; px < NPX; ++px) {
-          g[j][px] = in[j] ? gS[px0 + px][row * bw + col + j] : 0.f;
-          any |= g[j][px] != 0.f;
+      for (int ch = 0; ch < NCH; ++ch) {
+        L4Quad g2{0ull, 0ull};
+#pragma unroll
+        for (int k = 0; k < NPX; ++k) {
+          L4Quad& a = gf1[px0 + k][ch];   // a compile-time index once the caller's loop is unrolled
+          a.lo = fma2(gg[k], f2[j][ch].lo, a.lo);
+          a.hi = fma2(gg[k], f2[j][ch].hi, a.hi);
+          g2.lo = fma2(gg[k], f1[px0 + k][ch].lo, g2.lo);
+          g2.hi = fma2(gg[k], f1[px0 + k][ch].hi, g2.hi);
         }
-        if (!any) continue;   // outside the image, or no pixel of the pass has this position in its window
-#pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) {
-          const int c = ch * 128 + lane * 4;
-          float4 g2 = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int px = 0; px < NPX; ++px) {
-            float4& a = gf1[px0 + px][ch];   // a compile-time index once the caller's loop is unrolled
-            a.x = fmaf(g[j][px], f2[j][ch].x, a.x); a.y = fmaf(g[j][px], f2[j][ch].y, a.y);
-            a.z = fmaf(g[j][px], f2[j][ch].z, a.z); a.w = fmaf(g[j][px], f2[j][ch].w, a.w);
-            const float4& s = f1[px0 + px][ch];
-            g2.x = fmaf(g[j][px], s.x, g2.x); g2.y = fmaf(g[j][px], s.y, g2.y);
-            g2.z = fmaf(g[j][px], s.z, g2.z); g2.w = fmaf(g[j][px], s.w, g2.w);
-          }
-          if (c < C) red_add_v4(G2b + at[j] + c, g2);
-        }
+        if (ch * 128 + lane * 4 < C) red_add_v4(dst + ch * 128, g2.lo, g2.hi);
       }
     }
   }
 }
 
-// grid (ceil(N1 / 32), 1, B); every CTA walks all levels so that gF1 is stored once.
+// Gradient of the integer positions of pixel px over one box: position (i, j) of a pixel's (2r+2)^2 grid takes from window
+// entries a in {i-1, i}, b in {j-1, j} with the weight that entry gives it.
+__device__ __forceinline__ void l4_position_gradients(float* gS, const L4Pixel& g, bool live, const L4Box& box,
+                                                      const float (*s_g)[L4_TILE + 1], int pp, int radius, int H2, int W2,
+                                                      float scale, int lane) {
+  const int win = 2 * radius + 1, side = 2 * radius + 2, nq = box.bw * box.bh;
+  for (int q = lane; q < nq; q += 32) {
+    const int row = q / box.bw, col = q - row * box.bw;
+    const int i = box.ox + col - (g.bx - radius), j = box.oy + row - (g.by - radius);
+    float acc = 0.f;
+    if (live && i >= 0 && i < side && j >= 0 && j < side) {
+#pragma unroll
+      for (int da = 0; da < 2; ++da) {
+        const int a = i - da;
+        if (a < 0 || a >= win) continue;
+        const float fx = l4_fraction(g.cx, g.bx, a, radius, W2);
+        const float wx = da ? fx : 1.f - fx;
+#pragma unroll
+        for (int db = 0; db < 2; ++db) {
+          const int bb = j - db;
+          if (bb < 0 || bb >= win) continue;
+          const float fy = l4_fraction(g.cy, g.by, bb, radius, H2);
+          const float wy = db ? fy : 1.f - fy;
+          acc = fmaf(wx * wy, s_g[a * win + bb][pp], acc);
+        }
+      }
+    }
+    gS[q] = acc * scale;
+  }
+}
+
+// The forward's blocks of 8 x 4 and 2 x 2 pixels; every CTA walks all levels, so that gF1 is stored once.  Bound by
+// instruction issue like the forward.  A walk for 4 x 2 pixels with the channels split over two warps makes fewer
+// reductions into L2, but it reads every position's gradients twice and was slower (474 us, against 444 us for the scalar
+// kernel that took four pixels of a row).  grid (ceil(W1/8) * ceil(H1/4), 1, B)
 template <int NCH>
 __global__ void __launch_bounds__(L4_THREADS, 2)
 lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
-                         const float* __restrict__ gout, float* __restrict__ gF1, int N1, int C, int radius, int levels,
-                         float scale) {
+                         const float* __restrict__ gout, float* __restrict__ gF1, int H1, int W1, int C, int radius,
+                         int levels, float scale) {
   __shared__ float s_gS[L4_WARPS][L4_PX][L4_BMAX];
   __shared__ float s_g[L4_WIN * L4_WIN][L4_TILE + 1];
+  __shared__ int s_rows[L4_WARPS][L4_BMAX];
   __shared__ L4Pixel s_geo[L4_WARPS][L4_PX];
 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int b = blockIdx.z;
-  const int pbase = blockIdx.x * L4_TILE;
-  const int p0 = pbase + w * L4_PX;
-  const int win = 2 * radius + 1, side = 2 * radius + 2;
-  const int npx = min(L4_PX, N1 - p0);
+  const int b = blockIdx.z, N1 = H1 * W1, win = 2 * radius + 1;
+  const int tiles_x = (W1 + L4_TW - 1) / L4_TW;
+  const int h0 = (int)(blockIdx.x / tiles_x) * L4_TH, w0 = (int)(blockIdx.x % tiles_x) * L4_TW;
+  const int ph = h0 + 2 * (w >> 2), pw = w0 + 2 * (w & 3);
+  const int mh = ph + ((lane >> 1) & 1), mw = pw + (lane & 1);
+  const bool mine = lane < L4_PX && mh < H1 && mw < W1;
+  const unsigned mask = __ballot_sync(0xffffffffu, mine);
 
-  float4 f1[L4_PX][NCH], gf1[L4_PX][NCH];
+  L4Quad f1[L4_PX][NCH], gf1[L4_PX][NCH];
 #pragma unroll
   for (int px = 0; px < L4_PX; ++px)
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch) {
       const int c = ch * 128 + lane * 4;
-      f1[px][ch] = (px < npx && c < C)
-                       ? __ldg(reinterpret_cast<const float4*>(F1 + ((size_t)b * N1 + p0 + px) * C + c))
-                       : make_float4(0.f, 0.f, 0.f, 0.f);
-      gf1[px][ch] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const size_t p = (size_t)b * N1 + (size_t)(ph + px / 2) * W1 + pw + px % 2;
+      const bool ok = ((mask >> px) & 1u) && c < C;
+      f1[px][ch] = l4_load(F1 + (ok ? p * C + c : 0), ok);
+      gf1[px][ch] = L4Quad{0ull, 0ull};
     }
 
   for (int level = 0; level < levels; ++level) {
@@ -329,74 +389,36 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
 
     __syncthreads();   // the previous level's s_g is no longer read
     for (int i = threadIdx.x; i < win * win * L4_TILE; i += L4_THREADS) {
-      const int o = i / L4_TILE, pp = i % L4_TILE;
-      s_g[o][pp] = pbase + pp < N1 ? __ldg(gout + (((size_t)b * levels + level) * win * win + o) * N1 + pbase + pp)
-                                   : 0.f;
+      const int o = i / L4_TILE, pp = i % L4_TILE, h = h0 + pp / L4_TW, x = w0 + pp % L4_TW;
+      s_g[o][pp] = (h < H1 && x < W1)
+                       ? __ldg(gout + (((size_t)b * levels + level) * win * win + o) * N1 + (size_t)h * W1 + x)
+                       : 0.f;
     }
-    int xmin = INT_MAX, xmax = INT_MIN, ymin = INT_MAX, ymax = INT_MIN;
-    if (lane < L4_PX && p0 + lane < N1) {
-      L4Pixel g;
-      l4_pixel_geometry(coords, b, p0 + lane, N1, level, H2, W2, g);
-      s_geo[w][lane] = g;
-      xmin = xmax = g.bx;
-      ymin = ymax = g.by;
-    }
-#pragma unroll
-    for (int off = 1; off < L4_PX; off <<= 1) {
-      xmin = min(xmin, __shfl_xor_sync(0xffffffffu, xmin, off));
-      xmax = max(xmax, __shfl_xor_sync(0xffffffffu, xmax, off));
-      ymin = min(ymin, __shfl_xor_sync(0xffffffffu, ymin, off));
-      ymax = max(ymax, __shfl_xor_sync(0xffffffffu, ymax, off));
-    }
-    xmin = __shfl_sync(0xffffffffu, xmin, 0); xmax = __shfl_sync(0xffffffffu, xmax, 0);
-    ymin = __shfl_sync(0xffffffffu, ymin, 0); ymax = __shfl_sync(0xffffffffu, ymax, 0);
+    L4Pixel geo{0.f, 0.f, 0, 0};
+    if (mine) geo = l4_pixel_geometry(coords, b, mh * W1 + mw, N1, level, H2, W2);
+    if (lane < L4_PX) s_geo[w][lane] = geo;
     __syncthreads();
-    if (npx <= 0) continue;
+    if (mask == 0) continue;
 
-    const int bw = xmax - xmin + side, bh = ymax - ymin + side;
-    const bool together = bw <= L4_BW && bh <= L4_BH;
-    const int sbw = together ? bw : side, sbh = together ? bh : side;
-
-    // gradient of the integer positions: position (i, j) of a pixel's (2r+2)^2 grid takes from window entries
-    // a in {i-1, i}, b in {j-1, j} with the weight that entry gives it
-    for (int idx = lane; idx < npx * sbw * sbh; idx += 32) {
-      const int px = idx / (sbw * sbh), q = idx - px * sbw * sbh;
-      const int row = q / sbw, col = q - row * sbw;
-      const L4Pixel g = s_geo[w][px];
-      const int ox = together ? xmin - radius : g.bx - radius;
-      const int oy = together ? ymin - radius : g.by - radius;
-      const int i = ox + col - (g.bx - radius), j = oy + row - (g.by - radius);
-      float acc = 0.f;
-      if (i >= 0 && i < side && j >= 0 && j < side) {
-#pragma unroll
-        for (int da = 0; da < 2; ++da) {
-          const int a = i - da;
-          if (a < 0 || a >= win) continue;
-          const float fx = l4_fraction(g.cx, g.bx, a, radius, W2);
-          const float wx = da ? fx : 1.f - fx;
-#pragma unroll
-          for (int db = 0; db < 2; ++db) {
-            const int bb = j - db;
-            if (bb < 0 || bb >= win) continue;
-            const float fy = l4_fraction(g.cy, g.by, bb, radius, H2);
-            const float wy = db ? fy : 1.f - fy;
-            acc = fmaf(wx * wy, s_g[a * win + bb][w * L4_PX + px], acc);
-          }
-        }
-      }
-      s_gS[w][px][q] = acc * scale;
-    }
-    __syncwarp();
-
-    if (together) {
-      l4_box_gradients<NCH, L4_PX>(f1, gf1, F2b, G2b, H2, W2, C, xmin - radius, ymin - radius, bw, bh, s_gS[w], 0, lane);
-    } else {
+    L4Box box = l4_box(geo, mask, radius, lane);
+    if (l4_fits(box, L4_BMAX)) {
+      l4_fill_rows(s_rows[w], box, H2, W2, lane);
+      for (int px = 0; px < L4_PX; ++px)
+        l4_position_gradients(s_gS[w][px], s_geo[w][px], (mask >> px) & 1u, box, s_g,
+                              (2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2, radius, H2, W2, scale, lane);
+      __syncwarp();
+      l4_box_gradients<NCH, L4_PX>(f1, gf1, F2b, G2b, C, s_rows[w], box.bw * box.bh, s_gS[w], 0, lane);
+    } else {  // motion boundaries: one pixel at a time
 #pragma unroll
       for (int px = 0; px < L4_PX; ++px) {
-        if (px >= npx) break;
-        const L4Pixel g = s_geo[w][px];
-        l4_box_gradients<NCH, 1>(f1, gf1, F2b, G2b, H2, W2, C, g.bx - radius, g.by - radius, side, side, s_gS[w], px,
-                                 lane);
+        if (!((mask >> px) & 1u)) continue;
+        box = l4_box(geo, 1u << px, radius, lane);
+        __syncwarp();
+        l4_fill_rows(s_rows[w], box, H2, W2, lane);
+        l4_position_gradients(s_gS[w][px], s_geo[w][px], true, box, s_g,
+                              (2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2, radius, H2, W2, scale, lane);
+        __syncwarp();
+        l4_box_gradients<NCH, 1>(f1, gf1, F2b, G2b, C, s_rows[w], box.bw * box.bh, s_gS[w], px, lane);
       }
     }
     __syncwarp();
@@ -407,8 +429,10 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch) {
       const int c = ch * 128 + lane * 4;
-      if (px < npx && c < C)
-        *reinterpret_cast<float4*>(gF1 + ((size_t)b * N1 + p0 + px) * C + c) = gf1[px][ch];
+      if (((mask >> px) & 1u) && c < C) {
+        const size_t p = (size_t)b * N1 + (size_t)(ph + px / 2) * W1 + pw + px % 2;
+        *reinterpret_cast<ulonglong2*>(gF1 + p * C + c) = make_ulonglong2(gf1[px][ch].lo, gf1[px][ch].hi);
+      }
     }
 }
 
@@ -423,39 +447,45 @@ static Lookup4dLevels make_levels(const Lookup4dDims& d, const float* const* F2,
   return lv;
 }
 
+static unsigned l4_tiles(const Lookup4dDims& d) {
+  return (unsigned)((d.W1 + L4_TW - 1) / L4_TW) * (unsigned)((d.H1 + L4_TH - 1) / L4_TH);
+}
+
 cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                     const float* coords, float* out, float scale, cudaStream_t stream) {
-  const int N1 = d.H1 * d.W1;
   const Lookup4dLevels lv = make_levels(d, F2, nullptr);
-  const dim3 grid((N1 + L4_TILE - 1) / L4_TILE, d.levels, d.B);
+  const dim3 grid(l4_tiles(d), d.levels, d.B);
+#define SFB_L4_FWD(NCH) lookup4d_forward_kernel<NCH><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, out, d.H1, d.W1, d.C, d.radius, d.levels, scale)
   switch ((d.C + 127) / 128) {
-    case 1: lookup4d_forward_kernel<1><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, out, N1, d.C, d.radius, d.levels, scale); break;
-    case 2: lookup4d_forward_kernel<2><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, out, N1, d.C, d.radius, d.levels, scale); break;
-    case 3: lookup4d_forward_kernel<3><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, out, N1, d.C, d.radius, d.levels, scale); break;
-    case 4: lookup4d_forward_kernel<4><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, out, N1, d.C, d.radius, d.levels, scale); break;
+    case 1: SFB_L4_FWD(1); break;
+    case 2: SFB_L4_FWD(2); break;
+    case 3: SFB_L4_FWD(3); break;
+    case 4: SFB_L4_FWD(4); break;
     default: return cudaErrorInvalidValue;
   }
+#undef SFB_L4_FWD
   return cudaGetLastError();
 }
 
 cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                      const float* coords, const float* gout, float* gF1, float* const* gF2,
                                      float scale, cudaStream_t stream) {
-  const int N1 = d.H1 * d.W1;
   for (int l = 0; l < d.levels; ++l) {
     const cudaError_t err =
         cudaMemsetAsync(gF2[l], 0, (size_t)d.B * d.H2[l] * d.W2[l] * d.C * sizeof(float), stream);
     if (err != cudaSuccess) return err;
   }
   const Lookup4dLevels lv = make_levels(d, F2, gF2);
-  const dim3 grid((N1 + L4_TILE - 1) / L4_TILE, 1, d.B);
+  const dim3 grid(l4_tiles(d), 1, d.B);
+#define SFB_L4_BWD(NCH) lookup4d_backward_kernel<NCH><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, scale)
   switch ((d.C + 127) / 128) {
-    case 1: lookup4d_backward_kernel<1><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, gout, gF1, N1, d.C, d.radius, d.levels, scale); break;
-    case 2: lookup4d_backward_kernel<2><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, gout, gF1, N1, d.C, d.radius, d.levels, scale); break;
-    case 3: lookup4d_backward_kernel<3><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, gout, gF1, N1, d.C, d.radius, d.levels, scale); break;
-    case 4: lookup4d_backward_kernel<4><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, gout, gF1, N1, d.C, d.radius, d.levels, scale); break;
+    case 1: SFB_L4_BWD(1); break;
+    case 2: SFB_L4_BWD(2); break;
+    case 3: SFB_L4_BWD(3); break;
+    case 4: SFB_L4_BWD(4); break;
     default: return cudaErrorInvalidValue;
   }
+#undef SFB_L4_BWD
   return cudaGetLastError();
 }
 
