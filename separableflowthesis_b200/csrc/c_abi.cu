@@ -469,16 +469,20 @@ int map_sweep_operands(const Dims& d, const Workspace& w, int op16, CUtensorMap*
 }
 
 // The features of a call as the caller holds them: pixel-major (B, pixels, C), or (fmaps) the model's feature maps
-// (B, C, pixels) with a factor for image 1.
+// (B, C, pixels) with a factor for image 1; and the operand type of the call (OP16_*).  An entry point reads the
+// process-wide switch once, into op16, and every step of the call goes by that: the copies prepare_operands makes are
+// those of one type, and another thread may move the switch at any time.
 struct Features {
   const float* F1;
   const float* F2;
   bool fmaps;
   float scale1;
+  int op16;
 };
 
-// Operand copies of a call's features (and of the mean rows of image 2 when with_aux) for operands of kind op16.
-cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& f, bool with_aux, int op16, cudaStream_t st) {
+// Operand copies of a call's features (and of the mean rows of image 2 when with_aux).
+cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& f, bool with_aux, cudaStream_t st) {
+  const int op16 = f.op16;
   // (an op without sweeps has no 16-bit copies in its workspace, but its gradient GEMMs still need the feature scales)
   float* const F1r = op16 ? nullptr : w.F1r;
   float* const F2r = op16 ? nullptr : w.F2r;
@@ -495,7 +499,7 @@ int prepare_launches(const Workspace& w, bool fmaps, bool with_aux, int op16) {
   return (copies ? (fmaps ? 1 : 2) : 0) + (with_aux ? 1 : 0) + (op16 == OP16_FP16 ? 1 : 0);
 }
 #define SFB_PREPARE(f, with_aux) \
-  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, (f).fmaps, with_aux, op16), st, [&] { return prepare_operands(d, w, f, with_aux, op16, st); }))
+  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, (f).fmaps, with_aux, (f).op16), st, [&] { return prepare_operands(d, w, f, with_aux, st); }))
 
 int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, int32_t* AM_u, int32_t* AM_v,
                        bool with_argmax, const sfb_shape* shape, void* ws, size_t ws_bytes, void* stream) {
@@ -510,7 +514,7 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, true);
   SweepArgs a;
   memset(&a, 0, sizeof(a));
@@ -568,10 +572,9 @@ int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm
 // out_cf: the gradients are written channel-major, (B, C, pixels), gF1 multiplied by scale1.
 int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int mode, int R4, int accumulate, float* gF1, float* gF2,
                   cudaStream_t st, int out_cf = 0, float scale1 = 1.f) {
-  // 16-bit form when the operand switch says so (callers have refused feature dimensions that do not allow it); with
-  // FP16 the callers have run grad_operand_scales and packed the operands with those scales
-  int op16 = OP16_NONE;
-  SFB_TRY(operand_mode(d, &op16));
+  // 16-bit form when the call has 16-bit operands; with FP16 the callers have run grad_operand_scales and packed the
+  // operands with those scales
+  const int op16 = feat.op16;
   const float* const s1 = op16 == OP16_FP16 ? w.scales + SCALE_F1 : nullptr;
   const float* const s2 = op16 == OP16_FP16 ? w.scales + SCALE_F2 : nullptr;
   CUtensorMap tm_y, tm_xu, tm_xv;
@@ -832,7 +835,7 @@ int sfb_compression_forward(const float* F1, const float* F2, const float* A_u, 
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
@@ -860,7 +863,7 @@ int sfb_max_argmax_avg_backward(const float* F1, const float* F2, const int32_t*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   const size_t pix = (size_t)d.B * d.N1();
   SFB_TRY(grad_operand_scales(w, op16, {{gMA_u, pix * 2 * d.H2}, {gMA_v, pix * 2 * d.W2}}, {}, st));
@@ -886,7 +889,7 @@ int sfb_compression_backward(const float* F1, const float* F2, const float* A_u,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   SFB_TRY(run_attention_grads(d, w, gC_u, gC_v, gA_u, gA_v, st, op16));
@@ -919,7 +922,7 @@ int sfb_compression_attention_backward(const float* F1, const float* F2, const f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   return run_attention_grads(d, w, gC_u, gC_v, gA_u, gA_v, st, op16);
 }
@@ -930,8 +933,7 @@ static int run_fused_feature_grads(const Dims& d, const Workspace& w, const Feat
                                    const float* gMA_u, const float* gMA_v, const float* A_u, const float* A_v,
                                    const float* gC_u, const float* gC_v, float* gF1, float* gF2, cudaStream_t st) {
   const int N1 = d.N1(), K = d.Kc;
-  int op16;
-  SFB_TRY(operand_mode(d, &op16));
+  const int op16 = feat.op16;
   {
     const size_t pix = (size_t)d.B * N1;
     SFB_TRY(grad_operand_scales(w, op16,
@@ -978,7 +980,7 @@ int sfb_separation_feature_backward(const float* F1, const float* F2, const int3
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   return run_fused_feature_grads(d, w, feat, AM_u, AM_v, gMA_u, gMA_v, A_u, A_v, gC_u, gC_v, gF1, gF2, st);
 }
@@ -998,7 +1000,7 @@ int sfb_separation_backward(const float* F1, const float* F2, const int32_t* AM_
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   SFB_TRY(run_attention_grads(d, w, gC_u, gC_v, gA_u, gA_v, st, op16));
   return run_fused_feature_grads(d, w, feat, AM_u, AM_v, gMA_u, gMA_v, A_u, A_v, gC_u, gC_v, gF1, gF2, st);
@@ -1019,7 +1021,7 @@ int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, true);
   const int N1 = d.N1();
   SweepArgs a;
@@ -1053,7 +1055,7 @@ static int run_compress_cf(const float* F1, const float* F2, const float* W_u, c
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   // W_u (B,K,W2,N1) weights per v, W_v (B,K,H2,N1) per u; O_u (B,K,H2,N1), O_v (B,K,W2,N1)
@@ -1081,8 +1083,7 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const F
                                       const float* gC_u, const float* gC_v, int gK, int g0, float* gF1, float* gF2,
                                       cudaStream_t st, int out_cf = 0, float scale1 = 1.f, bool unit_weights = false) {
   const int N1 = d.N1(), K = d.Kc;
-  int op16;
-  SFB_TRY(operand_mode(d, &op16));
+  const int op16 = feat.op16;
   {  // FP16 operands: scales from the whole gradient tensors (an upper bound when only some channels are this level's);
      // unit_weights: A_u / A_v are softmax outputs
     const size_t bn = (size_t)d.B * N1;
@@ -1134,7 +1135,7 @@ int sfb_separation_feature_backward_cf(const float* F1, const float* F2, const i
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   return run_fused_feature_grads_cf(d, w, feat, AM_u, AM_v, gSEP_v, gSEP_u, A_u, A_v, gC_u, gC_v, d.Kc, 0, gF1, gF2, st);
 }
@@ -1233,7 +1234,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
-  const Features feat{F1, F2, fmaps != 0, scale1};
+  const Features feat{F1, F2, fmaps != 0, scale1, op16};
   SFB_PREPARE(feat, true);
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
   SweepArgs a;
@@ -1303,7 +1304,7 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  const Features feat{F1, F2, fmaps != 0, fmaps ? scale1 : 1.f};
+  const Features feat{F1, F2, fmaps != 0, fmaps ? scale1 : 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
   // attention gradients: gA_v(b,k,u,p) = sum_v S * gC_v(b,k,v,p), gA_u(b,k,v,p) = sum_u S * gC_u(b,k,u,p), with
@@ -1517,7 +1518,7 @@ int sfb_corr_volume(const float* F1, const float* F2, float* S, const sfb_shape*
   const int op16 = OP16_NONE;  // this test aid always computes with TF32 operands (its workspace has no 16-bit copies)
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
-  const Features feat{F1, F2, false, 1.f};
+  const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   SweepArgs a;
   memset(&a, 0, sizeof(a));
