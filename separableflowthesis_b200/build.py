@@ -18,6 +18,7 @@ HEADERS = ["kernels.h", "sm100_primitives.cuh", os.path.join("..", "..", "includ
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-Werror=unused-result",   # dropping the result of a launcher (kernels.h) does not compile
 ]
 
 

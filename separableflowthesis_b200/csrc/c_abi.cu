@@ -398,6 +398,14 @@ int check_ptr(const void* p, const char* name) {
     if (e_ != cudaSuccess) return fail(SFB_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_));  \
   } while (0)
 
+// Inside a step of several launches (a function returning cudaError_t): the first one that fails ends it.  A launcher
+// takes the error off the runtime when it reports it, so a result that is not passed on is lost.
+#define SFB_LAUNCH(expr)                       \
+  do {                                         \
+    cudaError_t e_ = (expr);                   \
+    if (e_ != cudaSuccess) return e_;          \
+  } while (0)
+
 int check_workspace(const Dims& d, void* ws, size_t ws_bytes, int op, Workspace* out) {
   if (ws == nullptr) return fail(SFB_ERR_INVALID_ARGUMENT, "workspace is NULL");
   if ((reinterpret_cast<uintptr_t>(ws) & 255u) != 0)
@@ -533,10 +541,10 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   // packed (displacement, slot, pixel) -> the reference's (pixel, channel, displacement) tensors
   const int N1 = d.N1(), R = MAXAVG_SLOTS;
   SFB_CUDA(timed(KID_PACK, with_argmax ? 4 : 2, st, [&] {
-    launch_unpack(w.ou, MA_u, d.B, N1, w.n1p, 2, d.H2, R, 0, 1, 2, 0, st);
+    SFB_LAUNCH(launch_unpack(w.ou, MA_u, d.B, N1, w.n1p, 2, d.H2, R, 0, 1, 2, 0, st));
     cudaError_t e = launch_unpack(w.ov, MA_v, d.B, N1, w.n1p, 2, d.W2, R, 0, 1, 2, 0, st);
     if (with_argmax) {
-      launch_unpack(w.ou, AM_u, d.B, N1, w.n1p, 1, d.H2, R, 2, 1, 1, 0, st);
+      SFB_LAUNCH(launch_unpack(w.ou, AM_u, d.B, N1, w.n1p, 1, d.H2, R, 2, 1, 1, 0, st));
       e = launch_unpack(w.ov, AM_v, d.B, N1, w.n1p, 1, d.W2, R, 2, 1, 1, 0, st);
     }
     return e;
@@ -601,11 +609,11 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
   if (!accumulate) {  // later passes over further channel chunks reuse the copies of the first
     SFB_CUDA(timed(KID_PREPARE, 2, st, [&] {
       if (op16 && feat.fmaps) {  // already channel-major
-        launch_channel_major_cf(feat.F1, reinterpret_cast<uint16_t*>(w.F1t), d.B, 1, d.N1(), w.n1p, d.C, 0, feat.scale1, op16, s1, st);
+        SFB_LAUNCH(launch_channel_major_cf(feat.F1, reinterpret_cast<uint16_t*>(w.F1t), d.B, 1, d.N1(), w.n1p, d.C, 0, feat.scale1, op16, s1, st));
         return launch_channel_major_cf(feat.F2, reinterpret_cast<uint16_t*>(w.F2t), d.B, d.H2, d.W2, w.h2p, d.C, 1, 1.f, op16, s2, st);
       }
-      cudaMemsetAsync(w.F2t, 0, (size_t)d.B * f2t_per_sample * (op16 ? 2 : sizeof(float)), st);
-      launch_channel_major(op16 ? feat.F1 : w.F1r, w.F1t, d.B, 1, d.N1(), w.n1p, d.C, 0, op16, s1, st);
+      SFB_LAUNCH(cudaMemsetAsync(w.F2t, 0, (size_t)d.B * f2t_per_sample * (op16 ? 2 : sizeof(float)), st));
+      SFB_LAUNCH(launch_channel_major(op16 ? feat.F1 : w.F1r, w.F1t, d.B, 1, d.N1(), w.n1p, d.C, 0, op16, s1, st));
       return launch_channel_major(op16 ? feat.F2 : w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
     }));
   }
@@ -709,13 +717,13 @@ int run_attention_grads(const Dims& d, const Workspace& w, const float* gC_u, co
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
   const int N1 = d.N1(), K = d.Kc;
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    launch_pack(gC_v, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st);
+    SFB_LAUNCH(launch_pack(gC_v, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st));
     return launch_pack(gC_u, w.xu, d.B, N1, w.n1p, K, 0, K, d.H2, K, 0, 1, 0.f, st);
   }));
   SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
                               0, 0, 1, packed_view(w.ou, d.H2, K, w.n1p), packed_view(w.ov, d.W2, K, w.n1p), w.n1p, st, op16, sweep_out_scale(w, op16)));
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    launch_unpack(w.ou, gA_v, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st);
+    SFB_LAUNCH(launch_unpack(w.ou, gA_v, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st));
     return launch_unpack(w.ov, gA_u, d.B, N1, w.n1p, K, d.W2, K, 0, 1, K, 0, st);
   }));
   return SFB_OK;
@@ -839,13 +847,13 @@ int sfb_compression_forward(const float* F1, const float* F2, const float* A_u, 
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    launch_pack(A_u, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st);         // w_u[k][v] = XV slot k
+    SFB_LAUNCH(launch_pack(A_u, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st));  // w_u[k][v] = XV slot k
     return launch_pack(A_v, w.xu, d.B, N1, w.n1p, K, 0, K, d.H2, K, 0, 1, 0.f, st);  // w_v[k][u] = XU slot k
   }));
   SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
                               0, 0, 1, packed_view(w.ou, d.H2, K, w.n1p), packed_view(w.ov, d.W2, K, w.n1p), w.n1p, st, op16, sweep_out_scale(w, op16)));
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    launch_unpack(w.ou, C_u, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st);
+    SFB_LAUNCH(launch_unpack(w.ou, C_u, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st));
     return launch_unpack(w.ov, C_v, d.B, N1, w.n1p, K, d.W2, K, 0, 1, K, 0, st);
   }));
   return SFB_OK;
@@ -870,7 +878,7 @@ int sfb_max_argmax_avg_backward(const float* F1, const float* F2, const int32_t*
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
     SlotSources su, sv;
     maxavg_slot_sources(d, AM_u, AM_v, gMA_u, gMA_v, &su, &sv, grad_slot_scales(w, op16));
-    launch_pack_interleaved(su, w.gxu, d.B, d.N1(), w.n1p, d.H2, 4, 1, 0, st);
+    SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, d.N1(), w.n1p, d.H2, 4, 1, 0, st));
     return launch_pack_interleaved(sv, w.gxv, d.B, d.N1(), w.n1p, d.W2, 4, 1, 0, st);
   }));
   return run_grad_pair(d, w, feat, GRAD_MAXAVG, 4, 0, gF1, gF2, st);
@@ -903,7 +911,7 @@ int sfb_compression_backward(const float* F1, const float* F2, const float* A_u,
     SFB_CUDA(timed(KID_PACK, 2, st, [&] {
       SlotSources su, sv;
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, grad_slot_scales(w, op16));
-      launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st);
+      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st));
       return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, k0 > 0 ? 1 : 0, gF1, gF2, st));
@@ -946,10 +954,10 @@ static int run_fused_feature_grads(const Dims& d, const Workspace& w, const Feat
     SFB_CUDA(timed(KID_PACK, 4, st, [&] {
       SlotSources su, sv;
       maxavg_slot_sources(d, AM_u, AM_v, gMA_u, gMA_v, &su, &sv, gs);
-      launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4, Q, 0, st);
-      launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4, Q, 0, st);
+      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4, Q, 0, st));
+      SFB_LAUNCH(launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4, Q, 0, st));
       compress_slot_sources(K, 0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs);
-      launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st);
+      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st));
       return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4 * Qc, Q, 1, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st));
@@ -959,7 +967,7 @@ static int run_fused_feature_grads(const Dims& d, const Workspace& w, const Feat
     SFB_CUDA(timed(KID_PACK, 2, st, [&] {
       SlotSources su, sv;
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs);
-      launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st);
+      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st));
       return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, 1, gF1, gF2, st));
@@ -1100,10 +1108,10 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const F
       SlotSources su, sv;
       // channel 0 = max gradient, channel 1 = mean gradient (same slots as the reference layout)
       maxavg_slot_sources(d, AM_u, AM_v, gM_v, gM_u, &su, &sv, gs);
-      launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4, Q, 0, st);
-      launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4, Q, 0, st);
+      SFB_LAUNCH(launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4, Q, 0, st));
+      SFB_LAUNCH(launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4, Q, 0, st));
       compress_slot_sources(K, 0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs, gK, g0);
-      launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st);
+      SFB_LAUNCH(launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st));
       return launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4 * Qc, Q, 1, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st, out_cf, scale1));
@@ -1113,7 +1121,7 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const F
     SFB_CUDA(timed(KID_PACK, 2, st, [&] {
       SlotSources su, sv;
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs, gK, g0);
-      launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st);
+      SFB_LAUNCH(launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st));
       return launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, 1, gF1, gF2, st, out_cf, scale1));
@@ -1253,8 +1261,8 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
   SFB_CUDA(timed(KID_ATTENTION_FWD, 2 * ((K + 3) / 4 + 1), st, [&] {
-    launch_attention_forward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + (size_t)c0 * d.W2 * N1, sb_u, weight_u,
-                             bias_u, A_u, st, w.status);
+    SFB_LAUNCH(launch_attention_forward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + (size_t)c0 * d.W2 * N1, sb_u, weight_u,
+                                        bias_u, A_u, st, w.status));
     return launch_attention_forward(AttentionDims{d.B, K, d.H2, d.H1, d.W1}, SEP_v + (size_t)c0 * d.H2 * N1, sb_v,
                                     weight_v, bias_v, A_v, st, w.status);
   }));
@@ -1316,8 +1324,8 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
   SFB_CUDA(timed(KID_ATTENTION_BWD, 2 * attention_backward_launches(K), st, [&] {
     const size_t ou = (size_t)c0 * d.W2 * N1, ov = (size_t)c0 * d.H2 * N1;  // first channel of this level
-    launch_attention_backward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + ou, sb_u, weight_u, A_u, w.ga_u,
-                              gSEP_u + ou, sb_u, w.gm_u, gweight_u, gbias_u, w.at_partial, st, w.status);
+    SFB_LAUNCH(launch_attention_backward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + ou, sb_u, weight_u, A_u, w.ga_u,
+                                         gSEP_u + ou, sb_u, w.gm_u, gweight_u, gbias_u, w.at_partial, st, w.status));
     return launch_attention_backward(AttentionDims{d.B, K, d.H2, d.H1, d.W1}, SEP_v + ov, sb_v, weight_v, A_v, w.ga_v,
                                      gSEP_v + ov, sb_v, w.gm_v, gweight_v, gbias_v, w.at_partial, st, w.status);
   }));

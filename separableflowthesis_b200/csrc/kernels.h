@@ -140,6 +140,9 @@ struct GradArgs {
 };
 TileSplit grad_split(const Dims& d, int image2_major);
 
+// Launchers, here and below: the returned error is taken off the runtime, so a caller must pass it on; dropping it does not
+// compile (unused results are errors in this build).
+
 // One source of an interleaved slot: dst[b][d][slot/4][p][slot%4] = scale * src[b][p][k][d] (raw copy when scale == 0);
 // src is (B, N1, Ksrc, D).  A null src makes the slot the constant `scale` (zero by default) for every valid pixel.
 struct SlotSource {
@@ -155,11 +158,11 @@ struct SlotSources {
   const float* dev_scales;  // may be null when no slot has dev != 0
 };
 // Same, from channels-first sources: dst[b][d][q][p][j] = scale * src[b][k][d][p], src is (B, Ksrc, D, N1).
-cudaError_t launch_pack_interleaved_cf(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
+[[nodiscard]] cudaError_t launch_pack_interleaved_cf(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
                                        int Qtot, int q0, cudaStream_t stream);
 // Writes R4 (4 or 8) slots = R4/4 groups starting at group q0 of dst (B, D, Qtot, n1p, 4); pixels N1 <= p < n1p
 // and slots without a source are zero.
-cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
+[[nodiscard]] cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
                                     int Qtot, int q0, cudaStream_t stream);
 
 // Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, all cleared by
@@ -178,41 +181,41 @@ enum : int {
 // rounded to nearest, and the row/column mean rows of F2 in aux.  16-bit operands: F1h / F2h / auxh, from the unrounded
 // values (BF16, or FP16 after scaling by the powers of two this call derives from the arrays' largest magnitudes,
 // scales[]).  Null arrays are left out.
-cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, float* F1r, float* F2r, float* aux,
+[[nodiscard]] cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, float* F1r, float* F2r, float* aux,
                            int* status, cudaStream_t stream, uint16_t* F1h = nullptr, uint16_t* F2h = nullptr,
                            uint16_t* auxh = nullptr, int op16 = 0, float* scales = nullptr);
 // The same from the model's feature maps fmap1 (B, C, H1, W1), fmap2 (B, C, H2, W2): F1r = round(scale1 * fmap1)
 // transposed to (B, H1, W1, C), F2r = round(fmap2) transposed (core/corr.py:419-422 does this with
 // permute().contiguous() and a division).
-cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fmap2, float scale1, float* F1r,
+[[nodiscard]] cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fmap2, float scale1, float* F1r,
                               float* F2r, float* aux, int* status, cudaStream_t stream, uint16_t* F1h = nullptr,
                               uint16_t* F2h = nullptr, uint16_t* auxh = nullptr, int op16 = 0, float* scales = nullptr);
 // Largest |x| * premul of each array, combined into its amax slot, and then the multipliers that follow from the slots:
 // those of the features or (gradients) those of the gradient operands.
 constexpr int ABSMAX_MAX = 6;
 struct AbsmaxSource { const float* p; size_t n; float premul; int slot; };
-cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, bool gradients, cudaStream_t stream);
+[[nodiscard]] cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, bool gradients, cudaStream_t stream);
 // 16-bit channel-major copy from a (B, C, rows*width) feature map times `scale`, padding zeroed (layouts below).
-cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
+[[nodiscard]] cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
                                     int blocked, float scale, int op16, const float* scale16, cudaStream_t stream);
 // Channel-major copy of a pixel-major feature array (B, rows*width, C), as FP32 (of rounded values) or (op16 != 0) as 16-bit
 // operands (FP16: times the device scalar *scale16); padding is not written.
 //   blocked = 0: dst (B, C, pitch) with pixel index row*width + x (rows = 1)
 //   blocked = 1: dst (B, C, ceil(width/16), pitch, 16), element (row, x) at ((x/16)*pitch + row)*16 + x%16
-cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, int width, int pitch, int C,
+[[nodiscard]] cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, int width, int pitch, int C,
                                  int blocked, int op16, const float* scale16, cudaStream_t stream);
 // Pack: dst[b][d][r0 + k*rstride][p] = scale * src[b][p][ksrc0 + k][d] for k < K (raw 32-bit copy when
 // scale == 0), zero for N1 <= p < n1p.  src is (B, N1, Ksrc, D), dst is (B, D, R, n1p).
-cudaError_t launch_pack(const void* src, float* dst, int B, int N1, int n1p, int Ksrc, int ksrc0, int K, int D,
+[[nodiscard]] cudaError_t launch_pack(const void* src, float* dst, int B, int N1, int n1p, int Ksrc, int ksrc0, int K, int D,
                         int R, int r0, int rstride, float scale, cudaStream_t stream);
 // Unpack: dst[b][p][kdst0 + k][d] = src[b][d][r0 + k*rstride][p] for k < K; dst is (B, N1, Kdst, D).
-cudaError_t launch_unpack(const float* src, void* dst, int B, int N1, int n1p, int K, int D, int R, int r0,
+[[nodiscard]] cudaError_t launch_unpack(const float* src, void* dst, int B, int N1, int n1p, int K, int D, int R, int r0,
                           int rstride, int Kdst, int kdst0, cudaStream_t stream);
-cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
+[[nodiscard]] cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                          const CUtensorMap& tm_aux, cudaStream_t stream);
 // tm_y: channel-major features of the other image (K-major B operand); tm_xu / tm_xv: interleaved operands (tm_xv is only read by the
 // image-2-major form; the image-1-major form keeps its (pixel, v) slots in registers).
-cudaError_t launch_grad_gemm(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
+[[nodiscard]] cudaError_t launch_grad_gemm(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
                              const CUtensorMap& tm_xv, cudaStream_t stream);
 
 
@@ -225,17 +228,17 @@ struct AttentionDims {
 // `status` (optional): a device status word for bounded waits.  With it, and when W1 is a multiple of 4 and x is
 // 16-byte aligned, the kernels fetch their pixel tiles (with the stencil's halo, zero-filled outside the image) by
 // TMA; otherwise every thread gathers its own neighbourhood.
-cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
+[[nodiscard]] cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
                                      const float* bias, float* a, cudaStream_t stream, int* status = nullptr);
 // Tiled fp32 tensor map without swizzle, zero fill out of bounds; dims / box innermost first, `strides_bytes` for
 // dimensions 1 .. rank-1.  Implemented next to the other tensor maps (c_abi.cu).
-cudaError_t encode_plain_map(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,
+[[nodiscard]] cudaError_t encode_plain_map(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,
                              const uint64_t* strides_bytes, const uint32_t* box);
 // Floats of scratch the backward needs for its per-block partial sums.
 size_t attention_partial_floats(const AttentionDims& d);
 // Backward: `g` holds dLoss/dA on entry and the logit gradients on return; gx (B, 2, D, H1, W1) = add + dLoss/dX
 // where `add` (same shape, `add_sb` elements between samples) may be null; gweight (Kc, 2, 3, 3, 3), gbias (Kc).
-cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
+[[nodiscard]] cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
                                       const float* a, float* g, const float* add, long long add_sb, float* gx,
                                       float* gweight, float* gbias, float* partial, cudaStream_t stream,
                                       int* status = nullptr);
@@ -243,10 +246,10 @@ cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, lo
 
 // Linear resampling along the displacement axis (core/corr.py:459-467: trilinear interpolate with unchanged H1, W1):
 // in (B, K, Dl, N1) -> K channels of a larger tensor, out[b] at out + b*out_sb, each (K, D0, N1); Dl <= D0.
-cudaError_t launch_upsample_displacement(const float* in, float* out, long long out_sb, int B, int K, int Dl, int D0,
+[[nodiscard]] cudaError_t launch_upsample_displacement(const float* in, float* out, long long out_sb, int B, int K, int Dl, int D0,
                                          int N1, cudaStream_t stream);
 // Its adjoint: gin (B, K, Dl, N1) from the gradient of those K channels.
-cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
+[[nodiscard]] cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
                                                  int D0, int N1, cudaStream_t stream);
 
 // Lookup on an aggregated 3D cost volume (the reference's CorrBlock1D, core/corr.py:513-624).
@@ -258,11 +261,11 @@ struct LookupDims {
   int B, dim, D, H1, W1, levels, radius;
 };
 size_t lookup_pyramid_floats(const LookupDims& d);
-cudaError_t launch_lookup_pyramid(const LookupDims& d, const float* corr, float* pyramid, cudaStream_t stream);
-cudaError_t launch_lookup_forward(const LookupDims& d, const float* corr, const float* pyramid, const float* coord,
+[[nodiscard]] cudaError_t launch_lookup_pyramid(const LookupDims& d, const float* corr, float* pyramid, cudaStream_t stream);
+[[nodiscard]] cudaError_t launch_lookup_forward(const LookupDims& d, const float* corr, const float* pyramid, const float* coord,
                                   long long coord_sb, float* out, int clamp_unit, cudaStream_t stream);
 // gcorr and gpyramid (same sizes as corr / pyramid) are overwritten; gpyramid is scratch.
-cudaError_t launch_lookup_backward(const LookupDims& d, const float* gout, const float* coord, long long coord_sb,
+[[nodiscard]] cudaError_t launch_lookup_backward(const LookupDims& d, const float* gout, const float* coord, long long coord_sb,
                                    float* gcorr, float* gpyramid, int clamp_unit, cudaStream_t stream);
 
 // Lookup on the 4D correlation volume without storing it (the call core/corr.py:491-510 leaves unimplemented; its
@@ -273,10 +276,10 @@ struct Lookup4dDims {
   int B, H1, W1, C, levels, radius;
   int H2[LOOKUP_MAX_LEVELS], W2[LOOKUP_MAX_LEVELS];
 };
-cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, const float* const* F2,
+[[nodiscard]] cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                     const float* coords, float* out, float scale, cudaStream_t stream);
 // gF1 (shape of F1) is overwritten; gF2[l] (shape of F2[l]) is zeroed and then accumulated with float reductions.
-cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, const float* const* F2,
+[[nodiscard]] cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                      const float* coords, const float* gout, float* gF1, float* const* gF2,
                                      float scale, cudaStream_t stream);
 
