@@ -245,8 +245,10 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
             for (int j = 0; j < SWEEP_VT; ++j) cm[j] = fmaxf(cm[j], r[j]);
           }
           m *= e.osc;  // memory holds scaled-back values; compare and store in that domain
-          if (valid && (vb == sc.vb0 || m > rold[ul])) {  // strict: the lowest column block wins ties
-            pu[u * usd] = m;
+          const bool better = m > rold[ul];              // strict: the lowest column block wins ties
+          if (valid && (vb == sc.vb0 || better)) {
+            // the first block of a later piece is compared too (with -inf): a NaN there must not stand in for its piece
+            pu[u * usd] = sc.piece > 0 && !better ? -CUDART_INF_F : m;
             if (ARG) pua[u * uasd] = __int_as_float(v0 + arg);
           }
         }
