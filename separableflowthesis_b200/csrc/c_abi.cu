@@ -325,8 +325,8 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   w.bytes = off;
   w.tail_count = reinterpret_cast<int*>(p + WS_TAIL_OFFSET);
   size_t part = 0;
-  if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS).part_floats);
-  if (d.Kc > 0 && plan.bf16) part = std::max(part, sweep_split(d, chunk_channels(d.Kc)).part_floats);
+  if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS, false).part_floats);
+  if (d.Kc > 0 && plan.bf16) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
   if (plan.Rg) part = std::max(part, std::max(grad_split(d, 0).part_floats, grad_split(d, 1).part_floats));
   w.part = reinterpret_cast<float*>(p + off);
   w.part_bytes = part * sizeof(float);
@@ -335,10 +335,11 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
 
 // A sweep's cut into whole tiles and pieces, as far as the workspace has scratch for the pieces.
 void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
-  const TileSplit s = sweep_split(a.d, slots);
+  const TileSplit s = sweep_split(a.d, slots, a.mode == SWEEP_COMPRESS);
   const bool cut = s.pieces > 1 && s.part_floats * sizeof(float) <= w.part_bytes;
   a.whole_tiles = cut ? s.whole_tiles : s.tiles;
   a.pieces = cut ? s.pieces : 1;
+  a.parts = cut ? s.parts : 0;
   a.part_slots = slots;
   a.part = w.part;
   a.tail_count = w.tail_count;

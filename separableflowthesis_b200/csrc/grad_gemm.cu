@@ -652,7 +652,7 @@ TileSplit grad_split(const Dims& d, int image2_major) {
   const int tiles = grad_tiles(d, image2_major), rest = tiles % SM_COUNT;
   const int blocks = image2_major ? (d.N1() + GG_KJ - 1) / GG_KJ
                                   : ((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT);
-  TileSplit r{tiles, tiles, 1, 0};
+  TileSplit r{tiles, tiles, 1, 0, 0};
   if (rest == 0) return r;
   double best = 0, whole = 0;
   for (int n = 1; n <= blocks && n <= MAX_PIECES; ++n) {
@@ -663,6 +663,7 @@ TileSplit grad_split(const Dims& d, int image2_major) {
   }
   if (r.pieces > 1) {
     r.whole_tiles = tiles - rest;
+    r.parts = r.pieces - 1;
     r.part_floats = (size_t)rest * (r.pieces - 1) * d.C * TILE_M;
   }
   return r;

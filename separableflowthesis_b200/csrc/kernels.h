@@ -94,7 +94,7 @@ struct SweepArgs {
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
   int drop_last_load;    // test hook: the producer leaves out its last F2 block, so that one wait runs out
   // Tiles past `whole_tiles` are done by `pieces` CTAs each (TileSplit); part / tail_count are unused when pieces is 1.
-  int whole_tiles, pieces, part_slots;
+  int whole_tiles, pieces, parts, part_slots;
   float* part;
   int* tail_count;       // one zero per tail tile; every launch leaves them zero
 };
@@ -103,8 +103,9 @@ struct SweepArgs {
 // CTAs, which need part_floats floats of scratch.
 constexpr int SM_COUNT = 148;
 constexpr int MAX_PIECES = 16;
-struct TileSplit { int tiles, whole_tiles, pieces; size_t part_floats; };
-TileSplit sweep_split(const Dims& d, int slots);  // slots: row results per pixel (max and argmax; channels of a launch)
+struct TileSplit { int tiles, whole_tiles, pieces, parts; size_t part_floats; };   // parts: results in scratch per tile and slot
+// slots: row results per pixel (max and argmax; channels of a launch); sums: they are added up, not compared
+TileSplit sweep_split(const Dims& d, int slots, bool sums);
 
 // Gradient GEMM.  G = dLoss/dS is generated from two "interleaved" operand sets: for every displacement
 // and image-1 pixel the R4 values (slots) that pixel contributes, in groups of four:

@@ -69,11 +69,47 @@ struct SweepSched {
   int vb0;              // first column block of this CTA
   int t_main, t_total;  // tiles of its column blocks; the same plus the tiles of the mean rows
   int tail, piece;      // tail tile this CTA has a piece of (-1: a whole tile) and which piece
+  int part_vb0;         // first column block of piece 1
 };
 
-// Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][slot][row u][128 pixels]
-__device__ __forceinline__ float* sweep_part(const SweepArgs& a, int tail, int piece, int slot) {
-  return a.part + (((size_t)tail * (a.pieces - 1) + piece - 1) * a.part_slots + slot) * a.d.H2 * TILE_M;
+// Scratch of the tail tiles: [tail][part][slot][row u][128 pixels].  The parts of a tile are its pieces 1.. (row maxima) or
+// the column blocks of its pieces 1.. (row sums, which are then folded block by block, in the order of a whole tile).
+__device__ __forceinline__ float* sweep_part(const SweepArgs& a, int tail, int part, int slot) {
+  return a.part + (((size_t)tail * a.parts + part) * a.part_slots + slot) * a.d.H2 * TILE_M;
+}
+// Column blocks of the pieces of a cut tile: the first n_vb % pieces have one more than the others.
+__host__ __device__ __forceinline__ int piece_start(int n_vb, int pieces, int piece) {
+  const int per = n_vb / pieces, extra = n_vb - per * pieces;
+  return piece * per + (piece < extra ? piece : extra);
+}
+
+// What the CTA of a block index does.
+template <int MODE, bool CUT>
+__device__ __forceinline__ SweepSched sweep_sched(const SweepArgs& a, int block) {
+  const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
+  SweepSched sc;
+  int tile = block;
+  sc.tail = -1;
+  sc.piece = 0;
+  if (CUT && tile >= a.whole_tiles) {  // pieces of the tail tiles follow the whole tiles
+    const int r = tile - a.whole_tiles;
+    sc.tail = r / a.pieces;
+    sc.piece = r - sc.tail * a.pieces;
+    tile = a.whole_tiles + sc.tail;
+  }
+  sc.b = tile / tiles_per_sample;
+  sc.m0 = (tile - sc.b * tiles_per_sample) * TILE_M;
+  sc.nkb = a.op16 ? (a.d.C + 2 * KBLK - 1) / (2 * KBLK) : (a.d.C + KBLK - 1) / KBLK;
+  sc.n_ub = (a.d.H2 + SWEEP_UT - 1) / SWEEP_UT;
+  const int n_vb = (a.d.W2 + SWEEP_VT - 1) / SWEEP_VT;
+  const int n_pieces = CUT && sc.tail >= 0 ? a.pieces : 1;
+  sc.vb0 = piece_start(n_vb, n_pieces, sc.piece);
+  sc.part_vb0 = piece_start(n_vb, n_pieces, 1);
+  sc.t_main = sc.n_ub * (piece_start(n_vb, n_pieces, sc.piece + 1) - sc.vb0);
+  const bool has_aux = (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG);
+  const bool does_aux = has_aux && sc.piece == n_pieces - 1;       // the mean rows go to the last, smallest piece
+  sc.t_total = sc.t_main + (does_aux ? (a.d.H2 + a.d.W2 + SW_TILE_N - 1) / SW_TILE_N : 0);
+  return sc;
 }
 
 // ---------------------------------------------------------------------------------- producer
@@ -176,7 +212,7 @@ __device__ __forceinline__ void max16_first(const float* r, float& m, int& arg) 
   arg = g ? i2[1] : i2[0];
 }
 
-template <bool ARG>
+template <bool ARG, bool CUT>
 __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
   const int H2 = a.d.H2, W2 = a.d.W2;
   // per-thread views: value of (displacement d, slot) at ptr[d*sd + slot*ss]
@@ -187,9 +223,9 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
   float* pva = ARG ? a.pv_arg.base + sc.b * a.pv_arg.sb + e.p : nullptr;
   uint32_t usd = a.pu.sd, uasd = a.pu_arg.sd;
   const uint32_t umsd = a.pu.sd, vsd = a.pv.sd, vss = a.pv.ss, vasd = a.pv_arg.sd;
-  if (sc.piece > 0) {          // row maxima of a later piece: scratch slots 0 (value) and 1 (arg-max)
-    pu = sweep_part(a, sc.tail, sc.piece, 0) + (e.p - sc.m0);
-    if (ARG) pua = sweep_part(a, sc.tail, sc.piece, 1) + (e.p - sc.m0);
+  if (CUT && sc.piece > 0) {   // row maxima of a later piece: scratch slots 0 (value) and 1 (arg-max)
+    pu = sweep_part(a, sc.tail, sc.piece - 1, 0) + (e.p - sc.m0);
+    if (ARG) pua = sweep_part(a, sc.tail, sc.piece - 1, 1) + (e.p - sc.m0);
     usd = uasd = TILE_M;
   }
   const bool valid = e.valid;
@@ -245,10 +281,10 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
             for (int j = 0; j < SWEEP_VT; ++j) cm[j] = fmaxf(cm[j], r[j]);
           }
           m *= e.osc;  // memory holds scaled-back values; compare and store in that domain
-          const bool better = m > rold[ul];              // strict: the lowest column block wins ties
-          if (valid && (vb == sc.vb0 || better)) {
-            // the first block of a later piece is compared too (with -inf): a NaN there must not stand in for its piece
-            pu[u * usd] = sc.piece > 0 && !better ? -CUDART_INF_F : m;
+          // the first block of a later piece is compared too (with -inf): a NaN there must not stand in for its piece
+          if (CUT && sc.piece > 0 && vb == sc.vb0 && !(m > -CUDART_INF_F)) m = -CUDART_INF_F;
+          if (valid && (vb == sc.vb0 || m > rold[ul])) {  // strict: the lowest column block wins ties
+            pu[u * usd] = m;
             if (ARG) pua[u * uasd] = __int_as_float(v0 + arg);
           }
         }
@@ -317,6 +353,7 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
   }
 }
 
+template <bool CUT>
 __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
   const int H2 = a.d.H2, W2 = a.d.W2;
   const bool active = e.wg < a.kc;            // this warpgroup's channel exists (warp-uniform)
@@ -329,9 +366,13 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
   const float* wv = a.xu.base + sc.b * a.xu.sb + e.p + (a.wv_slot0 + k * a.w_stride) * a.xu.ss;  // w_v[k][u]
   float* ou = a.ou.base + sc.b * a.ou.sb + e.p + k * a.ou.ss;
   float* ov = a.ov.base + sc.b * a.ov.sb + e.p + k * a.ov.ss;
-  if (sc.piece > 0 && active) {  // row sums of a later piece: scratch slot = channel of this launch
-    ou = sweep_part(a, sc.tail, sc.piece, e.wg) + (e.p - sc.m0);
+  // The first column block initialises the row sums, the others are added to them.  A later piece stores every block, into
+  // a part of its own (slot = channel of this launch).
+  uint32_t part_step = 0;
+  if (CUT && sc.piece > 0) {
+    ou = sweep_part(a, sc.tail, sc.vb0 - sc.part_vb0, e.wg) + (e.p - sc.m0);
     ousd = TILE_M;
+    part_step = (uint32_t)a.part_slots * H2 * TILE_M;
   }
 
   // Both sums run on packed FP32 pairs (two neighbouring columns per fma.rn.f32x2), which halves the
@@ -367,7 +408,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N;
     if (active) {
       float* ou_t = ou + u0 * ousd;
-      const bool first = vb == sc.vb0;  // the first column block initialises the output, later ones accumulate
+      const bool first = vb == 0 || part_step != 0;
 #pragma unroll
       for (int pr = 0; pr < SWEEP_UT / 2; ++pr) {
         float s[2 * SWEEP_VT];
@@ -405,7 +446,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         if (valid && 2 * j + 1 < nv) ov_t[(2 * j + 1) * ovsd] = hi * e.osc;
       }
     }
-    if (++ub == sc.n_ub) { ub = 0; ++vb; }
+    if (++ub == sc.n_ub) { ub = 0; ++vb; ou += part_step; }
   }
 }
 
@@ -439,21 +480,23 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
   }
 }
 
-// Pieces 1.. of a finished tail tile folded into piece 0's row results, in piece order (all threads of the CTA that
-// finished last).  Maxima: a later piece has the higher columns, so only a strictly larger value replaces.  One SM's loads
-// are all that moves these bytes, so a thread takes four pixels of up to FOLD_ROWS rows at once and asks for all pieces'
-// values before it uses any (with one 4-byte load at a time a fold of 135 rows x 4 channels took as long as the sweep).
+// The parts of a finished tail tile folded into piece 0's row results, in order (all threads of the CTA that finished last).
+// Maxima: a later piece has the higher columns, so only a strictly larger value replaces.  Sums: block by block, the order
+// in which a whole tile adds them, so that a sample's sums do not depend on the cut, which follows the batch and the row
+// range.  One SM's loads are all that moves these bytes, so a thread takes four pixels of up to FOLD_ROWS rows at once and
+// asks for several parts' values before it uses any (with one 4-byte load at a time a fold of 135 rows x 4 channels took as
+// long as the sweep).
 __device__ __forceinline__ void max4_first(float& v, float& arg, float o, float oarg) {
   if (o > v) { v = o; arg = oarg; }
 }
 template <int MODE>
 __device__ void sweep_fold_pieces(const SweepArgs& a, const SweepSched& sc) {
-  constexpr int NT = sw_threads(MODE), QUADS = TILE_M / 4, FOLD_ROWS = MODE == SWEEP_MAXARGAVG ? 2 : 4, FOLD_PIECES = 2;
+  constexpr int NT = sw_threads(MODE), QUADS = TILE_M / 4, FOLD_ROWS = MODE == SWEEP_MAXAVG ? 4 : 2, FOLD_PARTS = MODE == SWEEP_COMPRESS ? 6 : 2;
   const int H2 = a.d.H2, n = (MODE == SWEEP_COMPRESS ? a.kc : 1) * H2 * QUADS;
   for (int i0 = threadIdx.x; i0 < n; i0 += FOLD_ROWS * NT) {
     float* dst[FOLD_ROWS];
     float* arg_dst[FOLD_ROWS];
-    const float* part[FOLD_ROWS];   // piece 1's values; piece s is (s - 1) * part_slots slots further on
+    const float* part[FOLD_ROWS];   // the first part's values; part s is s * part_slots slots further on
     int cnt[FOLD_ROWS];
     float4 v[FOLD_ROWS], va[FOLD_ROWS];
 #pragma unroll
@@ -464,27 +507,27 @@ __device__ void sweep_fold_pieces(const SweepArgs& a, const SweepSched& sc) {
       if (MODE == SWEEP_COMPRESS) dst[r] = a.ou.base + sc.b * a.ou.sb + p + (a.k0 + k) * a.ou.ss + u * a.ou.sd;
       else dst[r] = a.pu.base + sc.b * a.pu.sb + p + u * a.pu.sd;
       arg_dst[r] = MODE == SWEEP_MAXARGAVG ? a.pu_arg.base + sc.b * a.pu_arg.sb + p + u * a.pu_arg.sd : nullptr;
-      part[r] = sweep_part(a, sc.tail, 1, k) + (size_t)u * TILE_M + px;
+      part[r] = sweep_part(a, sc.tail, 0, k) + (size_t)u * TILE_M + px;
       v[r] = load4_cg(dst[r], cnt[r]);
       if (MODE == SWEEP_MAXARGAVG) va[r] = load4_cg(arg_dst[r], cnt[r]);
     }
     const size_t slot = (size_t)H2 * TILE_M, step = slot * a.part_slots;
-    for (int s0 = 1; s0 < a.pieces; s0 += FOLD_PIECES) {
-      float4 o[FOLD_PIECES][FOLD_ROWS], oa[MODE == SWEEP_MAXARGAVG ? FOLD_PIECES : 1][FOLD_ROWS];
+    for (int s0 = 0; s0 < a.parts; s0 += FOLD_PARTS) {
+      float4 o[FOLD_PARTS][FOLD_ROWS], oa[MODE == SWEEP_MAXARGAVG ? FOLD_PARTS : 1][FOLD_ROWS];
 #pragma unroll
-      for (int j = 0; j < FOLD_PIECES; ++j)
+      for (int j = 0; j < FOLD_PARTS; ++j)
 #pragma unroll
         for (int r = 0; r < FOLD_ROWS; ++r) {
-          const bool ok = s0 + j < a.pieces && cnt[r] > 0;
-          const float* src = part[r] + (s0 + j - 1) * step;
+          const bool ok = s0 + j < a.parts && cnt[r] > 0;
+          const float* src = part[r] + (s0 + j) * step;
           // lanes past the image were never written: their values are loaded and dropped
           o[j][r] = ok ? __ldcg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
           if (MODE == SWEEP_MAXARGAVG)
             oa[j][r] = ok ? __ldcg(reinterpret_cast<const float4*>(src + slot)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-      for (int j = 0; j < FOLD_PIECES; ++j) {
-        if (s0 + j >= a.pieces) break;
+      for (int j = 0; j < FOLD_PARTS; ++j) {
+        if (s0 + j >= a.parts) break;
 #pragma unroll
         for (int r = 0; r < FOLD_ROWS; ++r) {
           if (MODE == SWEEP_COMPRESS) {
@@ -524,30 +567,7 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw + pad);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
-
-  SweepSched sc;
-  int tile = blockIdx.x;
-  sc.tail = -1;
-  sc.piece = 0;
-  if (CUT && tile >= a.whole_tiles) {  // pieces of the tail tiles follow the whole tiles
-    const int r = tile - a.whole_tiles;
-    sc.tail = r / a.pieces;
-    sc.piece = r - sc.tail * a.pieces;
-    tile = a.whole_tiles + sc.tail;
-  }
-  sc.b = tile / tiles_per_sample;
-  sc.m0 = (tile - sc.b * tiles_per_sample) * TILE_M;
-  sc.nkb = a.op16 ? (a.d.C + 2 * KBLK - 1) / (2 * KBLK) : (a.d.C + KBLK - 1) / KBLK;
-  sc.n_ub = (a.d.H2 + SWEEP_UT - 1) / SWEEP_UT;
-  const int n_vb = (a.d.W2 + SWEEP_VT - 1) / SWEEP_VT;
-  const int n_pieces = CUT && sc.tail >= 0 ? a.pieces : 1;
-  const int per = n_vb / n_pieces, extra = n_vb - per * n_pieces;  // the first `extra` pieces have one block more
-  sc.vb0 = sc.piece * per + min(sc.piece, extra);
-  sc.t_main = sc.n_ub * (per + (sc.piece < extra ? 1 : 0));
-  const bool has_aux = (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG);
-  const bool does_aux = has_aux && sc.piece == n_pieces - 1;       // the mean rows go to the last, smallest piece
-  sc.t_total = sc.t_main + (does_aux ? (a.d.H2 + a.d.W2 + SW_TILE_N - 1) / SW_TILE_N : 0);
+  const SweepSched sc = sweep_sched<MODE, CUT>(a, blockIdx.x);
 
   if (threadIdx.x == 0) {
     mbar_init(&sm.f1_full, 1);
@@ -558,7 +578,7 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     fence_barrier_init();
     prefetch_tensormap(&tm_f1);
     prefetch_tensormap(&tm_f2);
-    if (has_aux) prefetch_tensormap(&tm_aux);
+    if (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG) prefetch_tensormap(&tm_aux);
   }
   if (warp == 1) {
     tmem_alloc(&sm.tmem_base, SW_TMEM_COLS);
@@ -583,9 +603,9 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     e.valid = e.p < a.n_valid;
     e.tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
-    if (MODE == SWEEP_MAXAVG) epilogue_maxavg<false>(sm, a, sc, e);
-    else if (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true>(sm, a, sc, e);
-    else if (MODE == SWEEP_COMPRESS) epilogue_compress(sm, a, sc, e);
+    if (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT>(sm, a, sc, e);
+    else if (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT>(sm, a, sc, e);
+    else if (MODE == SWEEP_COMPRESS) epilogue_compress<CUT>(sm, a, sc, e);
     else epilogue_dump(sm, a, sc, e);
   }
 
@@ -601,40 +621,50 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     tc_fence_after();
     tmem_dealloc(sm.tmem_base, SW_TMEM_COLS);
   }
-  if (n_pieces > 1 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
-    __threadfence();  // this thread's results before the count ...
-    __syncthreads();
-    if (threadIdx.x == 0) sm.last_piece = atomicAdd(a.tail_count + sc.tail, 1) == n_pieces - 1;
-    __syncthreads();
-    if (sm.last_piece) {
-      __threadfence();  // ... and the count before the other pieces' results
-      sweep_fold_pieces<MODE>(a, sc);
-      if (threadIdx.x == 0) a.tail_count[sc.tail] = 0;  // as the next launch expects it
+  if constexpr (CUT) {
+    // the schedule is worked out again: kept over the epilogue, its registers would be spilled there
+    int block;
+    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
+    const SweepSched tail_sc = sweep_sched<MODE, CUT>(a, block);
+    if (tail_sc.tail >= 0 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
+      __threadfence();  // this thread's results before the count ...
+      __syncthreads();
+      if (threadIdx.x == 0) sm.last_piece = atomicAdd(a.tail_count + tail_sc.tail, 1) == a.pieces - 1;
+      __syncthreads();
+      if (sm.last_piece) {
+        __threadfence();  // ... and the count before the other pieces' results
+        sweep_fold_pieces<MODE>(a, tail_sc);
+        if (threadIdx.x == 0) a.tail_count[tail_sc.tail] = 0;  // as the next launch expects it
+      }
     }
   }
 }
 
 // How the tail tiles are cut, in units of one 256-column tile's time: a CTA costs about two tiles of prologue, a fold
-// reads pieces * slots * H2 rows of 128 values through one SM (about 677 rows per tile time).  Pieces must save a quarter
+// reads (parts + 1) * slots * H2 rows of 128 values through one SM (about 677 rows per tile time).  Pieces must save a quarter
 // of the tail and a whole tile to be used: a wave with idle SMs runs its tiles faster than a full one, so little is left of
 // smaller predicted savings (106 tail tiles of 135 x 240 in four pieces, predicted 0.86: max/avg sweep 588 -> 551 us, but
-// the compression sweep no faster; 55 tiles of 55 x 128 in two pieces, predicted 0.56: 108 -> 76 and 86 -> 58 us).
-TileSplit sweep_split(const Dims& d, int slots) {
+// the compression sweep no faster).  Whole and cut tiles measured (us per launch, C = 256, FP16, max/avg and compression):
+// 1 x 48 x 64: 65 and 44, 40 and 25; 1 x 55 x 128: 122 and 81, 113 and 83; 4 x 55 x 128: 240 and 199, 231 and 218;
+// 3 x 47 x 155: 246 and 171, 199 and 158; 8 x 47 x 156: 486 and 414, 349 and 339; 1 x 55 x 128 against 27 x 64: 54 and 46,
+// 37 and 31.  Adding the sums block by block costs a compression sweep 1 to 7 us against one sum per piece.
+TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   const long long tiles = (long long)d.B * ((d.N1() + TILE_M - 1) / TILE_M);
   const int n_ub = (d.H2 + SWEEP_UT - 1) / SWEEP_UT, n_vb = (d.W2 + SWEEP_VT - 1) / SWEEP_VT;
   const int rest = (int)(tiles % SM_COUNT);
-  TileSplit r{(int)tiles, (int)tiles, 1, 0};
+  TileSplit r{(int)tiles, (int)tiles, 1, 0, 0};
   if (rest == 0) return r;
   double best = 0, whole = 0;
   for (int n = 1; n <= n_vb && n <= MAX_PIECES; ++n) {
     const double waves = (rest * n + SM_COUNT - 1) / SM_COUNT;
-    const double cost = waves * ((n_vb + n - 1) / n * n_ub + 2) + (n > 1 ? n * (double)slots * d.H2 / 677.0 + 0.5 : 0.0);
+    const int parts = sums ? n_vb - piece_start(n_vb, n, 1) : n - 1;
+    const double cost = waves * ((n_vb + n - 1) / n * n_ub + 2) + (n > 1 ? (parts + 1) * (double)slots * d.H2 / 677.0 + 0.5 : 0.0);
     if (n == 1) best = whole = cost;
-    if (cost < best && cost < 0.75 * whole && cost < whole - 1) { best = cost; r.pieces = n; }
+    if (cost < best && cost < 0.75 * whole && cost < whole - 1) { best = cost; r.pieces = n; r.parts = parts; }
   }
   if (r.pieces > 1) {
     r.whole_tiles = (int)tiles - rest;
-    r.part_floats = (size_t)rest * (r.pieces - 1) * slots * d.H2 * TILE_M;
+    r.part_floats = (size_t)rest * r.parts * slots * d.H2 * TILE_M;
   }
   return r;
 }

@@ -83,6 +83,27 @@ def make_data(shape, dev):
 
 
 @pytest.mark.parametrize("operands", ["fp16", "tf32", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("name", list(OPS))
+def test_pieces_give_what_whole_tiles_give(name, shape, operands, cuda_device):
+    """Maxima, arg-maxima, means and the sums of the compression (its attention gradients are the same sums) bit for bit;
+    gradients, whose pieces accumulate apart, up to the order of an FP32 sum."""
+    with ops.sweep_operands(operands):
+        data = make_data(shape, cuda_device)
+        cut, whole = call_op(name, shape, 0, data), call_op(name, shape, 256, data)
+    assert whole is not None, "this shape is meant to be cut"
+    for x, y in zip(cut, whole):
+        if name in ("max/avg gradients", "feature gradients"):
+            # n products added in FP32 in two orders.  Each addition rounds its running sum by at most 2^-24 of it, and
+            # a running sum of terms of random sign stays near the largest result: sqrt(n) independent roundings of
+            # 2^-24 of that, the eightfold for the largest of some 10^6 values.
+            n = max(shape[1] * shape[2], shape[3] * shape[4])
+            assert (x - y).abs().max() <= 8 * n ** 0.5 * 2.0 ** -24 * y.abs().max()
+        else:
+            assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("operands", ["fp16", "tf32", "bf16"])
 @pytest.mark.parametrize("shape", [SHAPES[1], SHAPES[5], SHAPES[6], SHAPES[7]])
 def test_not_a_number_in_a_later_piece(shape, operands, cuda_device):
     """A NaN feature hides from the maxima what it hides in a whole tile and no more: not the rest of its piece."""
@@ -95,3 +116,16 @@ def test_not_a_number_in_a_later_piece(shape, operands, cuda_device):
     assert whole is not None
     for x, y in zip(cut, whole):
         assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x.nan_to_num(), y.nan_to_num())
+
+
+def test_a_sample_gives_the_same_in_any_batch(cuda_device):
+    """The number of pieces follows the number of tiles, hence the batch; the results of a sample do not (TF32 operands:
+    FP16 ones are scaled by the whole batch's magnitude)."""
+    B, H1, W1, H2, W2, C, Kc = shape = (5, 37, 128, 30, 90, 32, 3)
+    data = make_data(shape, cuda_device)
+    with ops.sweep_operands("tf32"):
+        full = ops.max_argmax_avg_forward(*data["f"]) + ops.compression_forward(*data["f"], *data["a"])
+        for b in range(B):
+            f1, f2, a_u, a_v = (t[b:b + 1].contiguous() for t in data["f"] + data["a"])
+            for x, y in zip(full, ops.max_argmax_avg_forward(f1, f2) + ops.compression_forward(f1, f2, a_u, a_v)):
+                assert torch.equal(x[b:b + 1], y)

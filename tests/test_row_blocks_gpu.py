@@ -87,7 +87,8 @@ def _row_blocks_combine(blocks, kind, cuda_device):
         for i in range(2):
             gw[i] += part[4][i]
             gb[i] += part[5][i]
-    # Same sweeps on the same features: with TF32 operands the outputs are identical.  With FP16 operands a block's
+    # Same sweeps on the same features: with TF32 operands the outputs are identical (also where the blocks' tiles are cut
+    # into other pieces than the whole image's: the test below).  With FP16 operands a block's
     # image-1 rows get their own power-of-two scale; scaling is exact except for the few values that land in FP16's
     # subnormal range under one scale and not the other, so the outputs agree to 1e-6 instead of bit for bit.  The
     # gradients are not bit-identical either way: at a block border dLoss/dS of a pixel is the sum of what two blocks
@@ -120,3 +121,22 @@ def _row_blocks_combine(blocks, kind, cuda_device):
                                        fw[5].double().cpu(), gu.double().cpu(), gv.double().cpu(), fmaps=True, scale1=scale)
     assert relerr(g1, rb[0]) < 2e-3 and relerr(g2, rb[1]) < 2e-3
     assert relerr(gw[0], rb[2]) < 2e-3 and relerr(gw[1], rb[4]) < 2e-3
+
+
+@pytest.mark.parametrize("blocks", [2, 3])
+def test_row_blocks_whose_tiles_are_cut_differently(blocks, cuda_device):
+    """55 x 128 is 55 pixel tiles, its blocks about 29 and 20: the sweeps cut them into other numbers of pieces, and the
+    outputs are the same bit for bit all the same."""
+    from separableflowthesis_b200 import ops
+    B, C, H, W, Kc = 1, 32, 55, 128, 4
+    g = torch.Generator().manual_seed(314)
+    f1, f2 = (torch.randn(B, C, H, W, generator=g).to(cuda_device) for _ in range(2))
+    params = [t.detach() for c in make_convs(Kc, g, cuda_device) for t in (c.weight, c.bias)]
+    with ops.sweep_operands("tf32"):
+        full = ops.separation_level_forward(f1, f2, *params, fmaps=True, scale1=0.2)
+        for ri in range(blocks):
+            sh = sharding.make_shard(B, H, blocks, ri, prefer="rows")
+            e0, e1, i0, i1 = sharding.halo_range(sh, H)
+            part = ops.separation_level_forward(f1[:, :, e0:e1].contiguous(), f2, *params, fmaps=True, scale1=0.2)
+            for x, y in zip(full, part):   # sep_u, sep_v, the arg-maxima, the attention weights: rows are the second axis from the end
+                assert torch.equal(x[..., sh.r0:sh.r1, :], y[..., i0:i1, :])
