@@ -58,23 +58,28 @@ upsample_displacement_kernel(const float* __restrict__ in, float* __restrict__ o
 }
 
 // gin[b][k][i][p] = sum over d of the weights with which output row d read input row i, added in the order of d.  A
-// thread produces the RS_IB rows from r0 on: it walks the output rows whose lower neighbour is r0 - 1 .. r0 + RS_IB - 1
-// (one thread for a whole column was too few threads for small images).  grid (ceil(N1/128), B*K, ceil(Dl/RS_IB))
-constexpr int RS_IB = 8;
+// thread walks its pixel's whole column, or (CUT) produces the RS_IB rows from r0 on by walking the output rows whose lower
+// neighbour is r0 - 1 .. r0 + RS_IB - 1.  Pieces re-read rows at their ends (twice the rows at Dl = D0, batches included),
+// so only launches of fewer than RS_CUT_BELOW blocks are cut, which on their own leave HBM idle.  Whole and cut, us:
+// 55 blocks (1 x 55 x 128, 128 -> 128 rows) 35 and 10, 464 (8 x 47 x 156, 156 rows) 50 and 39, 1016 (4 x 135 x 240, 240 rows)
+// 100 and 115, 2784 (six channels of 8 x 47 x 156) 153 and 197, 6096 (six of 4 x 135 x 240) 472 and 647.
+// grid (ceil(N1/128), B*K, CUT ? ceil(Dl/RS_IB) : 1)
+constexpr int RS_IB = 8, RS_CUT_BELOW = 6 * SM_COUNT;
 
+template <bool CUT>
 __global__ void __launch_bounds__(RS_THREADS)
 upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long gout_sb, float* __restrict__ gin, int K,
                                      int Dl, int D0, int N1, float scale) {
   const int p = blockIdx.x * RS_THREADS + threadIdx.x;
   if (p >= N1) return;
   const int b = blockIdx.y / K, k = blockIdx.y - b * K;
-  const int r0 = blockIdx.z * RS_IB, r1 = min(r0 + RS_IB, Dl);
+  const int r0 = CUT ? blockIdx.z * RS_IB : 0, r1 = CUT ? min(r0 + RS_IB, Dl) : Dl;
   const float* g = gout + (size_t)b * gout_sb + ((size_t)k * D0) * N1 + p;
   float* dst = gin + ((size_t)blockIdx.y * Dl) * N1 + p;
   // first output row with lower neighbour >= r0 - 1: an estimate, corrected with the exact rule (neighbours never fall
   // as d grows)
   int first = 0;
-  if (r0 > 1) {
+  if (CUT && r0 > 1) {
     int i0, i1;
     float l0, l1;
     first = max(0, min(D0 - 1, (int)((float)(r0 - 1) / scale) - 1));
@@ -88,10 +93,10 @@ upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long g
     }
   }
   // the source row grows by at most one per output row (Dl <= D0): two running sums cover rows cur and cur + 1
-  int cur = r0 > 0 ? r0 - 1 : 0;
+  int cur = CUT && r0 > 0 ? r0 - 1 : 0;
   float acc0 = 0.f, acc1 = 0.f;
   auto put = [&](int i, float v) {
-    if (i >= r0 && i < r1) dst[(size_t)i * N1] = v;
+    if (!CUT || (i >= r0 && i < r1)) dst[(size_t)i * N1] = v;
   };
   constexpr int DB = 8;  // output rows loaded per batch
   bool done = false;
@@ -105,7 +110,7 @@ upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long g
       int i0, i1;
       float l0, l1;
       resample_source(d0 + j, scale, Dl, i0, i1, l0, l1);
-      if (i0 >= r1) { done = true; break; }
+      if (CUT && i0 >= r1) { done = true; break; }
       while (cur < i0) {  // at most one step
         put(cur, acc0);
         acc0 = acc1;
@@ -118,7 +123,7 @@ upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long g
     }
   }
   put(cur, acc0);
-  put(cur + 1, acc1);
+  if (cur + 1 < r1) put(cur + 1, acc1);
   for (int i = cur + 2; i < r1; ++i) put(i, 0.f);
 }
 
@@ -136,9 +141,11 @@ cudaError_t launch_upsample_displacement(const float* in, float* out, long long 
 
 cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
                                                  int D0, int N1, cudaStream_t st) {
-  const dim3 grid((N1 + RS_THREADS - 1) / RS_THREADS, B * K, (Dl + RS_IB - 1) / RS_IB);
-  upsample_displacement_adjoint_kernel<<<grid, RS_THREADS, 0, st>>>(gout, gout_sb, gin, K, Dl, D0, N1,
-                                                                    resample_scale(Dl, D0));
+  const int blocks = (N1 + RS_THREADS - 1) / RS_THREADS;
+  const bool cut = Dl > RS_IB && (long long)blocks * B * K < RS_CUT_BELOW;
+  const dim3 grid(blocks, B * K, cut ? (Dl + RS_IB - 1) / RS_IB : 1);
+  auto kern = cut ? upsample_displacement_adjoint_kernel<true> : upsample_displacement_adjoint_kernel<false>;
+  kern<<<grid, RS_THREADS, 0, st>>>(gout, gout_sb, gin, K, Dl, D0, N1, resample_scale(Dl, D0));
   return cudaGetLastError();
 }
 

@@ -28,3 +28,16 @@ def test_rows(sizes, plane, cuda_device):
     gs = ops.upsample_displacement_backward(gd.to(cuda_device), 1, K, Dl)
     rs = orc.upsample_displacement_backward(gd.double(), 1, K, Dl)
     assert (gs.double().cpu() - rs).abs().max() < TOL * rs.abs().max()
+
+
+@pytest.mark.parametrize("sizes", [(8, 9), (9, 17), (16, 16), (17, 240), (33, 34)])
+def test_whole_columns_give_what_pieces_give(sizes, cuda_device):
+    """Launches with blocks enough to fill the GPU walk whole columns, smaller ones pieces of rows: the same sums."""
+    (Dl, D0), (H1, W1), (B, K) = sizes, (3, 5), (2, 444)   # 888 blocks: whole columns
+    g = torch.Generator().manual_seed(Dl)
+    gd = torch.randn(B, K + 1, D0, H1, W1, generator=g).to(cuda_device)
+    whole = ops.upsample_displacement_backward(gd, 1, K, Dl)
+    pieces = torch.cat([ops.upsample_displacement_backward(gd, 1 + k0, K // 4, Dl) for k0 in range(0, K, K // 4)], 1)
+    assert torch.equal(whole, pieces)
+    rs = orc.upsample_displacement_backward(gd.double().cpu(), 1, K, Dl)
+    assert (whole.double().cpu() - rs).abs().max() < TOL * rs.abs().max()
