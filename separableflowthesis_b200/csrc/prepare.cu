@@ -180,39 +180,81 @@ f2_means_kernel(const float* __restrict__ F2, float* __restrict__ aux, int H2, i
   }
 }
 
-// From channel-major feature maps: a block owns one channel plane, whose rows and columns it sums in two walks (the
-// second finds the plane in L2).  grid (C, B), block 256.
+// From channel-major feature maps: a block owns one channel plane; its warps take every eighth row, FC_ROWS rows at a time, a
+// lane every 32nd column.  NV = ceil(W2 / 32) rounded up to a power of two: the column sums of a lane stay in registers, so
+// that the plane is read once, with FC_ROWS * NV loads of a lane in flight (HBM-bound; one walk for the rows and one for the
+// columns took 162 us at 8 x 135 x 240, C = 256).  NV = 0: any width, in the two walks.  Both add in the same order.
+// grid (C, B), block 256.
+constexpr int FC_ROWS = 2;
+template <int NV>
 __global__ void __launch_bounds__(256)
 f2_means_cf_kernel(const float* __restrict__ fmap2, float* __restrict__ aux, int H2, int W2, int C,
                    uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
-  __shared__ float red[8][33];
+  __shared__ float red[8][NV > 0 ? NV : 1][33];
   const int c = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
   const float* plane = fmap2 + ((size_t)b * C + c) * H2 * W2;
   const size_t out0 = (size_t)b * (H2 + W2) * C + c;
-  for (int u = warp; u < H2; u += 8) {
-    float acc = 0.f;
-#pragma unroll 4
-    for (int v = lane; v < W2; v += 32) acc += __ldg(plane + (size_t)u * W2 + v);
+  auto store_row = [&](int u, float acc) {   // acc: this lane's share of row u
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) store_mean(acc / (float)W2, out0 + (size_t)u * C, aux, auxh, op16, sc16);
-  }
-  for (int v0 = 0; v0 < W2; v0 += 32) {
-    const int v = v0 + lane;
-    float acc = 0.f;
-    if (v < W2) {
-#pragma unroll 4
-      for (int u = warp; u < H2; u += 8) acc += __ldg(plane + (size_t)u * W2 + v);
-    }
-    red[warp][lane] = acc;
-    __syncthreads();
-    if (warp == 0 && v < W2) {
+  };
+  if constexpr (NV > 0) {
+    float col[NV];
 #pragma unroll
-      for (int i = 1; i < 8; ++i) acc += red[i][lane];
+    for (int i = 0; i < NV; ++i) col[i] = 0.f;
+    for (int u0 = warp; u0 < H2; u0 += 8 * FC_ROWS) {
+      float v[FC_ROWS][NV];
+#pragma unroll
+      for (int r = 0; r < FC_ROWS; ++r)
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+          v[r][i] = u0 + 8 * r < H2 && lane + 32 * i < W2 ? __ldg(plane + (size_t)(u0 + 8 * r) * W2 + lane + 32 * i) : 0.f;
+#pragma unroll
+      for (int r = 0; r < FC_ROWS; ++r) {
+        if (u0 + 8 * r >= H2) break;
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          acc += v[r][i];
+          col[i] += v[r][i];
+        }
+        store_row(u0 + 8 * r, acc);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) red[warp][i][lane] = col[i];
+    __syncthreads();
+    for (int v = threadIdx.x; v < W2; v += 256) {
+      float acc = red[0][v >> 5][v & 31];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) acc += red[i][v >> 5][v & 31];
       store_mean(acc / (float)H2, out0 + (size_t)(H2 + v) * C, aux, auxh, op16, sc16);
     }
-    __syncthreads();
+  } else {
+    for (int u = warp; u < H2; u += 8) {
+      float acc = 0.f;
+#pragma unroll 4
+      for (int v = lane; v < W2; v += 32) acc += __ldg(plane + (size_t)u * W2 + v);
+      store_row(u, acc);
+    }
+    for (int v0 = 0; v0 < W2; v0 += 32) {
+      const int v = v0 + lane;
+      float acc = 0.f;
+      if (v < W2) {
+#pragma unroll 4
+        for (int u = warp; u < H2; u += 8) acc += __ldg(plane + (size_t)u * W2 + v);
+      }
+      red[warp][0][lane] = acc;
+      __syncthreads();
+      if (warp == 0 && v < W2) {
+#pragma unroll
+        for (int i = 1; i < 8; ++i) acc += red[i][0][lane];
+        store_mean(acc / (float)H2, out0 + (size_t)(H2 + v) * C, aux, auxh, op16, sc16);
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -523,8 +565,14 @@ cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fm
     const TransposeJob j1{fmap1, F1r, F1h, s1, scale1, d.N1()}, j2{fmap2, F2r, F2h, s2, 1.f, d.N2()};
     transpose_round_kernel<<<dim3(t1 + t2, (d.C + 63) / 64, d.B), dim3(32, 8), 0, stream>>>(j1, j2, t1, d.C, op16);
   }
-  if (aux != nullptr || auxh != nullptr)
-    f2_means_cf_kernel<<<dim3(d.C, d.B), 256, 0, stream>>>(fmap2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
+  if (aux != nullptr || auxh != nullptr) {
+    auto kern = d.W2 <= 32    ? f2_means_cf_kernel<1>
+                : d.W2 <= 64  ? f2_means_cf_kernel<2>
+                : d.W2 <= 128 ? f2_means_cf_kernel<4>
+                : d.W2 <= 256 ? f2_means_cf_kernel<8>
+                              : f2_means_cf_kernel<0>;
+    kern<<<dim3(d.C, d.B), 256, 0, stream>>>(fmap2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
+  }
   return cudaGetLastError();
 }
 
