@@ -76,11 +76,43 @@ struct PlaneRing {
 // The walk along d is cut into pieces of `dc` displacements, one block each (a piece re-reads one plane on either
 // side): a walk is a serial chain, and a single 55 x 128 image has 56 pixel tiles for 148 SMs.  A logit is the same
 // sum in the same order whatever the cut.  The softmax has a kernel of its own (attention_softmax_kernel), which
-// keeps the online maximum, its branch and its exponential out of this issue-bound loop.
+// keeps the online maximum, its branch and its exponential out of this issue-bound loop; only a column of at most
+// AT_SOFT_MAX displacements walked in one piece is normalised at its end (SOFT, softmax_column): there the launch and the
+// idle warps of the other kernel cost more than the exponentials (8 x 47 x 156, four channels, D = 5, 8 and 16: 30, 36 and 44 us
+// with it, 21, 26 and 37 without).
 // Gather form: grid (ceil(N1/128), B * pieces), block 128.  Channels k0 .. k0+KC-1 of Kc, weights in c_att_weights.
 constexpr int FW_STAGES = 4;
+constexpr int AT_SOFT_MAX = 16;
 
-template <int KC>
+// Softmax of a pixel's column of D <= AT_SOFT_MAX logits, which the same thread has stored, in place.  The sum is formed as
+// attention_softmax_kernel forms it (SM_GROUPS partial sums of every SM_GROUPS-th value, then those in order), so that a
+// pixel's weights are the same whichever of the two its launch takes.
+constexpr int SM_GROUPS = 8;
+__device__ __forceinline__ void softmax_column(float* col, int D, size_t plane) {
+  float v[AT_SOFT_MAX], m = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int d = 0; d < AT_SOFT_MAX; ++d) v[d] = d < D ? col[d * plane] : -INFINITY;
+#pragma unroll
+  for (int d = 0; d < AT_SOFT_MAX; ++d) m = fmaxf(m, v[d]);
+#pragma unroll
+  for (int g = 0; g < SM_GROUPS; ++g) {
+    float s = 0.f;
+#pragma unroll
+    for (int d = g; d < AT_SOFT_MAX; d += SM_GROUPS) {
+      if (d < D) {
+        v[d] = __expf(v[d] - m);
+        s += v[d];
+      }
+    }
+    l += s;
+  }
+  const float inv = 1.f / l;
+#pragma unroll
+  for (int d = 0; d < AT_SOFT_MAX; ++d)
+    if (d < D) col[d * plane] = v[d] * inv;
+}
+
+template <int KC, bool SOFT>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float* __restrict__ bias,
                         float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1) {
@@ -145,6 +177,10 @@ attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float
     for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
   }
   if (d1 == D) emit(D - 1);
+  if constexpr (SOFT) {
+#pragma unroll 1
+    for (int k = 0; k < KC; ++k) softmax_column(out + (size_t)k * D * plane, D, plane);
+  }
 }
 
 // ---- logits, pixel tiles fetched by TMA -----------------------------------------------------------------
@@ -174,7 +210,7 @@ struct AttentionTileSmem {
   WaitCtl ctl;
 };
 
-template <int KC>
+template <int KC, bool SOFT>
 __global__ void __launch_bounds__(AT_THREADS + 32)
 attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const float* __restrict__ bias,
                               float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1,
@@ -248,6 +284,11 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
     for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
   }
   if (d1 == D) emit(D - 1);
+  if constexpr (SOFT) {
+    if (!valid) return;
+#pragma unroll 1
+    for (int k = 0; k < KC; ++k) softmax_column(out + (size_t)k * D * plane, D, plane);
+  }
 }
 
 // ---- softmax over d, in place -------------------------------------------------------------------------------
@@ -255,11 +296,10 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
 // V = ceil(D / 8) values in registers, so that every logit is read once and every weight written once (HBM-bound, all
 // loads of a thread in flight together).  V = 0: any D, the values are read again in each of the three walks.  The
 // order of the sums depends on D only.  grid ceil(N1/32) * planes (= B * Kc), block 256.
-constexpr int SM_GROUPS = 8;
 constexpr int SM_THREADS = SM_GROUPS * 32;
 
 template <int V>
-__global__ void __launch_bounds__(SM_THREADS)
+__global__ void __launch_bounds__(SM_THREADS, V == 0 ? 8 : (V <= 8 ? 6 : (V <= 20 ? 3 : 2)))
 attention_softmax_kernel(float* __restrict__ a, int D, int N1, unsigned pixel_blocks) {
   __shared__ float red[2][SM_GROUPS][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -330,19 +370,26 @@ static bool tileable(const AttentionDims& d, const void* x, long long sb) {
 }
 
 // ---- logit gradients (softmax backward), in place -------------------------------------------------------
-// gL = A * (gA - sum_d gA*A), with the split of attention_softmax_kernel: 32 pixels of one (sample, channel) per block,
-// V = ceil(D / 8) displacements per thread, both arrays read once into registers (V = 0: any D, read twice).  HBM-bound.
-// bias_partial: (Kc, B * pixel_blocks), the block's sum of gL.  grid ceil(N1/32) * B * Kc, block 256.
-template <int V>
-__global__ void __launch_bounds__(SM_THREADS, V > 16 ? 2 : (V > 8 ? 3 : 6))
+// gL = A * (gA - sum_d gA*A).  A column is shared by G warps: warp g of them takes displacements g, g + G, ... and keeps its
+// V = ceil(D / G) values of both arrays in registers, so that each is read once and all loads of a thread are in flight
+// together (HBM-bound).  A block is max(G, 8) warps, so short columns give it 8 / G groups of 32 pixels of one (sample,
+// channel).  V = 0: any D, both arrays read twice.  The order of the sums depends on D only.  Eight warps for every D
+// took 66 us for the attention backward of 2 x 135 x 240 and four channels at D = 5 and, spilling at V = 32, 635 us at
+// D = 135; 55 and 554 now.
+// bias_partial: (Kc, B * pixel_blocks), the block's sum of gL.  grid pixel_blocks * B * Kc, block 32 * max(G, 8).
+__host__ __device__ constexpr int lg_warps(int G) { return G > 8 ? G : 8; }
+__host__ __device__ constexpr int lg_pixels(int G) { return lg_warps(G) / G * 32; }
+template <int G, int V, int MIN_BLOCKS>
+__global__ void __launch_bounds__(32 * lg_warps(G), MIN_BLOCKS)
 attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, float* __restrict__ bias_partial,
                             int Kc, int D, int N1, unsigned pixel_blocks) {
-  __shared__ float red[SM_GROUPS][32];
-  __shared__ float bred[SM_GROUPS];
-  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  constexpr int WARPS = lg_warps(G);
+  __shared__ float red[WARPS][32];
+  __shared__ float bred[WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = warp % G;
   const unsigned row = blockIdx.x / pixel_blocks;   // sample * Kc + channel
   const unsigned pb = blockIdx.x - row * pixel_blocks;
-  const int p = (int)pb * 32 + lane;
+  const int p = (int)pb * lg_pixels(G) + warp / G * 32 + lane;
   const bool in = p < N1;
   const size_t base = (size_t)row * D * N1 + (in ? p : 0);
   constexpr int NV = V > 0 ? V : 1;
@@ -351,7 +398,7 @@ attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, 
   if constexpr (V > 0) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
-      const int d = grp + i * SM_GROUPS;
+      const int d = grp + i * G;
       const bool ok = in && d < D;
       gv[i] = ok ? g[base + (size_t)d * N1] : 0.f;
       av[i] = ok ? __ldg(a + base + (size_t)d * N1) : 0.f;
@@ -359,18 +406,20 @@ attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, 
 #pragma unroll
     for (int i = 0; i < V; ++i) s = fmaf(gv[i], av[i], s);
   } else if (in) {
-    for (int d = grp; d < D; d += SM_GROUPS) s = fmaf(g[base + (size_t)d * N1], __ldg(a + base + (size_t)d * N1), s);
+    for (int d = grp; d < D; d += G) s = fmaf(g[base + (size_t)d * N1], __ldg(a + base + (size_t)d * N1), s);
   }
-  red[grp][lane] = s;
-  __syncthreads();
-  s = 0.f;
+  if constexpr (G > 1) {
+    red[warp][lane] = s;
+    __syncthreads();
+    s = 0.f;
 #pragma unroll
-  for (int i = 0; i < SM_GROUPS; ++i) s += red[i][lane];
+    for (int i = 0; i < G; ++i) s += red[warp - grp + i][lane];
+  }
   float bsum = 0.f;
   if constexpr (V > 0) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
-      const int d = grp + i * SM_GROUPS;
+      const int d = grp + i * G;
       if (in && d < D) {
         const float gl = av[i] * (gv[i] - s);
         g[base + (size_t)d * N1] = gl;
@@ -378,7 +427,7 @@ attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, 
       }
     }
   } else if (in) {
-    for (int d = grp; d < D; d += SM_GROUPS) {
+    for (int d = grp; d < D; d += G) {
       const float gl = __ldg(a + base + (size_t)d * N1) * (g[base + (size_t)d * N1] - s);
       g[base + (size_t)d * N1] = gl;
       bsum += gl;
@@ -386,12 +435,12 @@ attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, 
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-  if (lane == 0) bred[grp] = bsum;
+  if (lane == 0) bred[warp] = bsum;
   __syncthreads();
   if (threadIdx.x == 0) {
     float t = 0.f;
 #pragma unroll
-    for (int i = 0; i < SM_GROUPS; ++i) t += bred[i];
+    for (int i = 0; i < WARPS; ++i) t += bred[i];
     const unsigned k = row % Kc, b = row / Kc, rows = gridDim.x / Kc;   // rows = B * pixel_blocks
     bias_partial[(size_t)k * rows + (size_t)b * pixel_blocks + pb] = t;
   }
@@ -881,7 +930,7 @@ static size_t walk_pieces_bound(size_t blocks, int D, int target, int min_walk) 
   return pieces < most ? pieces : most;
 }
 
-// Bias partials per 32-pixel block, weight partials per block / tile and piece of the walk.  An upper bound that does
+// Bias partials per block of at least 32 pixels, weight partials per block / tile and piece of the walk.  An upper bound that does
 // not fall when D grows: a level's two calls share one buffer sized for the larger D.
 size_t attention_partial_floats(const AttentionDims& d) {
   const size_t blocks = (size_t)pixel_grid(d).x * d.B, tiles = tile_count(d) * d.B;
@@ -899,20 +948,35 @@ static cudaError_t launch_softmax(float* a, size_t planes, int D, int N1, cudaSt
   if (v <= 4) attention_softmax_kernel<4><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
   else if (v <= 8) attention_softmax_kernel<8><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
   else if (v <= 16) attention_softmax_kernel<16><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  else if (v <= 20) attention_softmax_kernel<20><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+  else if (v <= 24) attention_softmax_kernel<24><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
   else if (v <= 32) attention_softmax_kernel<32><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
   else attention_softmax_kernel<0><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
   return cudaGetLastError();
 }
 
+// Displacements per block of the forward's walk, and whether the walk ends with the softmax of its columns.
+// A column short enough for that is not cut by launches that have two blocks per SM without it.
+static int forward_walk(const AttentionDims& d, bool tiled) {
+  const size_t blocks = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
+  return d.D <= AT_SOFT_MAX && blocks >= 2 * SM_COUNT ? d.D : walk_length(blocks, d.D);
+}
+static bool softmax_in_walk(const AttentionDims& d, bool tiled) { return d.D <= AT_SOFT_MAX && forward_walk(d, tiled) >= d.D; }
+
+int attention_forward_launches(const AttentionDims& d, const float* x, long long x_sb, const int* status) {
+  return (d.Kc + AT_KC - 1) / AT_KC + (softmax_in_walk(d, status != nullptr && tileable(d, x, x_sb)) ? 0 : 1);
+}
+
 cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
                                      const float* bias, float* a, cudaStream_t st, int* status) {
   const bool tiled = status != nullptr && tileable(d, x, x_sb);
+  const bool soft = softmax_in_walk(d, tiled);
   CUtensorMap tm_x;
   if (tiled) {
     cudaError_t err = tile_map(&tm_x, x, x_sb, 2, 2, d, true);
     if (err != cudaSuccess) return err;
   }
-  const int dc = walk_length((tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B, d.D);
+  const int dc = forward_walk(d, tiled);
   const unsigned pieces = (unsigned)((d.D + dc - 1) / dc);
   const dim3 grid(pixel_grid(d).x, d.B * pieces);
   const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * pieces);
@@ -923,18 +987,18 @@ cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, lon
       cudaError_t err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
       if (err != cudaSuccess) return err;
       if (tiled) {
-#define SFB_AT_FWD_T(KC) attention_logits_tiled_kernel<KC><<<tgrid, AT_THREADS + 32, 0, st>>>(tm_x, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1, status)
+#define SFB_AT_FWD_T(KC) (soft ? attention_logits_tiled_kernel<KC, true> : attention_logits_tiled_kernel<KC, false>)<<<tgrid, AT_THREADS + 32, 0, st>>>(tm_x, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1, status)
         if (kc == 1) SFB_AT_FWD_T(1); else if (kc == 2) SFB_AT_FWD_T(2); else if (kc == 3) SFB_AT_FWD_T(3); else SFB_AT_FWD_T(4);
 #undef SFB_AT_FWD_T
         continue;
       }
-#define SFB_AT_FWD(KC) attention_logits_kernel<KC><<<grid, AT_THREADS, 0, st>>>(x, x_sb, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1)
+#define SFB_AT_FWD(KC) (soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>)<<<grid, AT_THREADS, 0, st>>>(x, x_sb, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1)
       if (kc == 1) SFB_AT_FWD(1); else if (kc == 2) SFB_AT_FWD(2); else if (kc == 3) SFB_AT_FWD(3); else SFB_AT_FWD(4);
 #undef SFB_AT_FWD
     }
   }
   cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
+  if (err != cudaSuccess || soft) return err;
   return launch_softmax(a, (size_t)d.B * d.Kc, d.D, d.H1 * d.W1, st);
 }
 
@@ -956,17 +1020,25 @@ static cudaError_t launch_input_grad(const dim3 grid, const float* g, const floa
   return cudaGetLastError();
 }
 
-static cudaError_t launch_logit_grad(const AttentionDims& d, const float* a, float* g, float* bias_partial,
+// rows: bias partials per channel, B * pixel blocks
+static cudaError_t launch_logit_grad(const AttentionDims& d, const float* a, float* g, float* bias_partial, int* rows,
                                      cudaStream_t st) {
-  const int N1 = d.H1 * d.W1, v = (d.D + SM_GROUPS - 1) / SM_GROUPS;
-  const unsigned pb = (unsigned)((N1 + 31) / 32);
-  if ((unsigned long long)pb * d.B * d.Kc > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-  const unsigned blocks = pb * (unsigned)(d.B * d.Kc);
-#define SFB_AT_LG(V) attention_logit_grad_kernel<V><<<blocks, SM_THREADS, 0, st>>>(a, g, bias_partial, d.Kc, d.D, N1, pb)
-  if (v <= 4) SFB_AT_LG(4); else if (v <= 8) SFB_AT_LG(8); else if (v <= 16) SFB_AT_LG(16);
-  else if (v <= 32) SFB_AT_LG(32); else SFB_AT_LG(0);
-#undef SFB_AT_LG
-  return cudaGetLastError();
+  const int N1 = d.H1 * d.W1;
+  auto launch = [&](auto kern, int G) {
+    const unsigned pb = (unsigned)((N1 + lg_pixels(G) - 1) / lg_pixels(G));
+    if ((unsigned long long)pb * d.B * d.Kc > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+    *rows = (int)(pb * (unsigned)d.B);
+    kern<<<pb * (unsigned)(d.B * d.Kc), 32 * lg_warps(G), 0, st>>>(a, g, bias_partial, d.Kc, d.D, N1, pb);
+    return cudaGetLastError();
+  };
+  if (d.D <= 8) return launch(attention_logit_grad_kernel<1, 8, 5>, 1);
+  if (d.D <= 16) return launch(attention_logit_grad_kernel<2, 8, 6>, 2);
+  if (d.D <= 32) return launch(attention_logit_grad_kernel<4, 8, 6>, 4);
+  if (d.D <= 64) return launch(attention_logit_grad_kernel<8, 8, 6>, 8);
+  if (d.D <= 128) return launch(attention_logit_grad_kernel<8, 16, 3>, 8);
+  if (d.D <= 160) return launch(attention_logit_grad_kernel<16, 10, 2>, 16);
+  if (d.D <= 256) return launch(attention_logit_grad_kernel<16, 16, 2>, 16);
+  return launch(attention_logit_grad_kernel<8, 0, 6>, 8);
 }
 
 cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
@@ -974,12 +1046,12 @@ cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, lo
                                       float* gweight, float* gbias, float* partial, cudaStream_t st, int* status) {
   const int N1 = d.H1 * d.W1;
   const size_t blocks = (size_t)pixel_grid(d).x * d.B, tiles = tile_count(d) * d.B;
-  const int bias_rows = d.B * ((N1 + 31) / 32);
-  float* bias_partial = partial;                               // (Kc, bias_rows)
-  float* weight_partial = partial + (size_t)bias_rows * d.Kc;  // (Kc * 54, blocks or tiles times pieces)
+  int bias_rows = 0;
+  float* bias_partial = partial;                               // (Kc, bias_rows), bias_rows <= B * ceil(N1/32)
+  float* weight_partial = partial + (size_t)d.B * ((N1 + 31) / 32) * d.Kc;  // (Kc * 54, blocks or tiles times pieces)
   const long long g_sb = (long long)d.Kc * d.D * N1;
   const bool tiled = status != nullptr && tileable(d, x, x_sb) && tileable(d, g, g_sb);
-  cudaError_t err = launch_logit_grad(d, a, g, bias_partial, st);
+  cudaError_t err = launch_logit_grad(d, a, g, bias_partial, &bias_rows, st);
   if (err != cudaSuccess) return err;
   {
     const int dc = walk_length(tiled ? tiles : blocks, d.D);

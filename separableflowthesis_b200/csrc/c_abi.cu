@@ -139,7 +139,7 @@ const char* const kKernelNames[KID_COUNT] = {
     "grad_gemm_kernel<maxavg,image1-major>", "grad_gemm_kernel<maxavg,image2-major>",
     "grad_gemm_kernel<compress,image1-major>", "grad_gemm_kernel<compress,image2-major>",
     "grad_gemm_kernel<fused,image1-major>", "grad_gemm_kernel<fused,image2-major>",
-    "attention_forward_kernel", "attention backward (logit, input, weight grads)",
+    "attention forward (logits, softmax)", "attention backward (logit, input, weight grads)",
     "lookup kernels (pyramid, forward, backward)", "upsample_displacement kernels",
     "lookup4d kernels (forward, backward)"};
 struct TimingRec { cudaEvent_t e0, e1; int id; int launches; };
@@ -1166,7 +1166,7 @@ int sfb_attention_forward(const float* X, int64_t x_batch_stride, const float* w
   if (X == nullptr || weight == nullptr || bias == nullptr || A == nullptr)
     return fail(SFB_ERR_INVALID_ARGUMENT, "X, weight, bias and A must not be NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SFB_CUDA(timed(KID_ATTENTION_FWD, (Kc + 3) / 4 + 1, st,
+  SFB_CUDA(timed(KID_ATTENTION_FWD, attention_forward_launches(ad, X, x_batch_stride, nullptr), st,
                  [&] { return launch_attention_forward(ad, X, x_batch_stride, weight, bias, A, st); }));
   return SFB_OK;
 }
@@ -1261,11 +1261,12 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
-  SFB_CUDA(timed(KID_ATTENTION_FWD, 2 * ((K + 3) / 4 + 1), st, [&] {
-    SFB_LAUNCH(launch_attention_forward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + (size_t)c0 * d.W2 * N1, sb_u, weight_u,
-                                        bias_u, A_u, st, w.status));
-    return launch_attention_forward(AttentionDims{d.B, K, d.H2, d.H1, d.W1}, SEP_v + (size_t)c0 * d.H2 * N1, sb_v,
-                                    weight_v, bias_v, A_v, st, w.status);
+  const AttentionDims at_u{d.B, K, d.W2, d.H1, d.W1}, at_v{d.B, K, d.H2, d.H1, d.W1};
+  const float *const X_u = SEP_u + (size_t)c0 * d.W2 * N1, *const X_v = SEP_v + (size_t)c0 * d.H2 * N1;
+  const int at_launches = attention_forward_launches(at_u, X_u, sb_u, w.status) + attention_forward_launches(at_v, X_v, sb_v, w.status);
+  SFB_CUDA(timed(KID_ATTENTION_FWD, at_launches, st, [&] {
+    SFB_LAUNCH(launch_attention_forward(at_u, X_u, sb_u, weight_u, bias_u, A_u, st, w.status));
+    return launch_attention_forward(at_v, X_v, sb_v, weight_v, bias_v, A_v, st, w.status);
   }));
   // C_u (per u, weights A_u per v) -> SEP_v channels 2.., C_v -> SEP_u channels 2..
   return run_compress_sweeps(d, w, tm_f1, tm_f2, cf_view(A_v, K, d.H2, N1), cf_view(A_u, K, d.W2, N1), 0, 0, 1,

@@ -231,6 +231,7 @@ struct AttentionDims {
 // TMA; otherwise every thread gathers its own neighbourhood.
 [[nodiscard]] cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
                                      const float* bias, float* a, cudaStream_t stream, int* status = nullptr);
+int attention_forward_launches(const AttentionDims& d, const float* x, long long x_sb, const int* status);  // its kernels
 // Tiled fp32 tensor map without swizzle, zero fill out of bounds; dims / box innermost first, `strides_bytes` for
 // dimensions 1 .. rank-1.  Implemented next to the other tensor maps (c_abi.cu).
 [[nodiscard]] cudaError_t encode_plain_map(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,

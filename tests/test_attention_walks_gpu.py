@@ -53,3 +53,26 @@ def test_tiles(size, Kc, cuda_device):
     for sep, a, w, b in ((sep_u, a_u, params[0], params[1]), (sep_v, a_v, params[2], params[3])):
         ref = orc.attention_forward(sep[:, :2].double().cpu(), w.double(), b.double())
         assert relerr(a, ref) < TOL
+
+
+@pytest.mark.parametrize("D", [1, 3, 8, 9, 16, 17, 31, 160, 161, 192, 193])
+def test_a_sample_alone_and_in_a_batch(D, cuda_device):
+    """How the forward's walk is cut, and whether it ends with the softmax itself (short columns, launches of many blocks) or
+    leaves it to the kernel of its own, follows the number of blocks: the weights of a sample are the same bits either way.
+    Its gradients depend on D only as well."""
+    B, Kc, H1, W1 = 7, 3, 45, 131
+    g = torch.Generator().manual_seed(D)
+    x = torch.randn(B, 2, D, H1, W1, generator=g).to(cuda_device)
+    weight, bias = (torch.randn(Kc, 2, 3, 3, 3, generator=g) * 0.3).to(cuda_device), torch.randn(Kc, generator=g).to(cuda_device)
+    ga = torch.randn(B, Kc, D, H1, W1, generator=g).to(cuda_device)
+    a = ops.attention_forward(x, weight, bias)
+    gx = ops.attention_backward(x, weight, a, ga)[0]
+    for b in (0, B - 1):
+        ab = ops.attention_forward(x[b:b + 1].contiguous(), weight, bias)
+        assert torch.equal(a[b:b + 1], ab)
+        assert torch.equal(gx[b:b + 1], ops.attention_backward(x[b:b + 1].contiguous(), weight, ab, ga[b:b + 1].contiguous())[0])
+    ref = orc.attention_forward(x[:1].double().cpu(), weight.double().cpu(), bias.double().cpu())
+    assert relerr(a[:1], ref) < TOL
+    r_gx = orc.attention_backward(x[:1].double().cpu(), weight.double().cpu(), a[:1].double().cpu(), ga[:1].double().cpu(), None)[0]
+    if D > 1:
+        assert relerr(gx[:1], r_gx) < TOL
