@@ -277,9 +277,15 @@ __device__ __forceinline__ void l4_box_gradients(const L4Quad (&f1)[L4_PX][NCH],
   for (int q0 = 0; q0 < nq; q0 += J) {
     int r[J];
     L4Quad f2[J][NCH];
+    int all = -1;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       r[j] = rows[q0 + j];   // -1 past the box
+      all &= r[j];
+    }
+    if (NPX == 1 && all < 0) continue;   // nothing of the window here: beyond the image's edge, or no gradient
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
       const float* src = F2b + (size_t)(r[j] < 0 ? 0 : r[j]) * C + lane * 4;
 #pragma unroll
       for (int ch = 0; ch < NCH; ++ch) f2[j][ch] = l4_load(src + ch * 128, r[j] >= 0 && ch * 128 + lane * 4 < C);
@@ -316,36 +322,36 @@ __device__ __forceinline__ void l4_box_gradients(const L4Quad (&f1)[L4_PX][NCH],
   }
 }
 
-// Gradient of the integer positions of pixel px over one box: position (i, j) of a pixel's (2r+2)^2 grid takes from window
-// entries a in {i-1, i}, b in {j-1, j} with the weight that entry gives it.
-__device__ __forceinline__ void l4_position_gradients(float* gS, const L4Pixel& g, bool live, const L4Box& box,
-                                                      const float (*s_g)[L4_TILE + 1], int pp, int radius, int H2, int W2,
-                                                      float scale, int lane) {
-  const int win = 2 * radius + 1, side = 2 * radius + 2, nq = box.bw * box.bh;
-  for (int q = lane; q < nq; q += 32) {
-    const int row = q / box.bw, col = q - row * box.bw;
-    const int i = box.ox + col - (g.bx - radius), j = box.oy + row - (g.by - radius);
-    float acc = 0.f;
-    if (live && i >= 0 && i < side && j >= 0 && j < side) {
+// Gradient of one integer position of a pixel's window: position (i, j) of its (2r+2)^2 grid takes from window entries
+// a in {i-1, i}, b in {j-1, j} with the weight that entry gives it.  pp: the pixel's column of s_g.
+__device__ __forceinline__ float l4_position_gradient(const L4Pixel& g, int i, int j, const float (*s_g)[L4_TILE + 1], int pp,
+                                                      int radius, int H2, int W2) {
+  const int win = 2 * radius + 1, side = 2 * radius + 2;
+  float acc = 0.f;
+  if (i >= 0 && i < side && j >= 0 && j < side) {
 #pragma unroll
-      for (int da = 0; da < 2; ++da) {
-        const int a = i - da;
-        if (a < 0 || a >= win) continue;
-        const float fx = l4_fraction(g.cx, g.bx, a, radius, W2);
-        const float wx = da ? fx : 1.f - fx;
+    for (int da = 0; da < 2; ++da) {
+      const int a = i - da;
+      if (a < 0 || a >= win) continue;
+      const float fx = l4_fraction(g.cx, g.bx, a, radius, W2);
+      const float wx = da ? fx : 1.f - fx;
 #pragma unroll
-        for (int db = 0; db < 2; ++db) {
-          const int bb = j - db;
-          if (bb < 0 || bb >= win) continue;
-          const float fy = l4_fraction(g.cy, g.by, bb, radius, H2);
-          const float wy = db ? fy : 1.f - fy;
-          acc = fmaf(wx * wy, s_g[a * win + bb][pp], acc);
-        }
+      for (int db = 0; db < 2; ++db) {
+        const int bb = j - db;
+        if (bb < 0 || bb >= win) continue;
+        const float fy = l4_fraction(g.cy, g.by, bb, radius, H2);
+        const float wy = db ? fy : 1.f - fy;
+        acc = fmaf(wx * wy, s_g[a * win + bb][pp], acc);
       }
     }
-    gS[q] = acc * scale;
   }
+  return acc;
 }
+
+// In a walk for one pixel its table of rows lies behind its gradients, with room for the positions that the last step asks for
+// past the end.
+constexpr int L4_ALONE_ROWS = L4_BMAX / 2, L4_ALONE_PAD = 4;
+static_assert(L4_SIDE * L4_SIDE <= L4_ALONE_ROWS && L4_ALONE_ROWS + L4_SIDE * L4_SIDE + L4_ALONE_PAD <= L4_BMAX, "a pixel's positions and rows");
 
 // The forward's blocks of 8 x 4 and 2 x 2 pixels; every CTA walks all levels, so that gF1 is stored once.  Bound by
 // instruction issue like the forward.  A walk for 4 x 2 pixels with the channels split over two warps makes fewer
@@ -400,26 +406,43 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
     __syncthreads();
     if (mask == 0) continue;
 
-    L4Box box = l4_box(geo, mask, radius, lane);
+    const int pp0 = 2 * (w >> 2) * L4_TW + 2 * (w & 3);   // this warp's first pixel in s_g; pixel px: + px/2 rows, + px%2
+    const L4Box box = l4_box(geo, mask, radius, lane);
     if (l4_fits(box, L4_BMAX)) {
       l4_fill_rows(s_rows[w], box, H2, W2, lane);
-      for (int px = 0; px < L4_PX; ++px)
-        l4_position_gradients(s_gS[w][px], s_geo[w][px], (mask >> px) & 1u, box, s_g,
-                              (2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2, radius, H2, W2, scale, lane);
-      __syncwarp();
-      l4_box_gradients<NCH, L4_PX>(f1, gf1, F2b, G2b, C, s_rows[w], box.bw * box.bh, s_gS[w], 0, lane);
-    } else {  // motion boundaries: one pixel at a time
-#pragma unroll
+      const int nq = box.bw * box.bh;
       for (int px = 0; px < L4_PX; ++px) {
-        if (!((mask >> px) & 1u)) continue;
-        box = l4_box(geo, 1u << px, radius, lane);
-        __syncwarp();
-        l4_fill_rows(s_rows[w], box, H2, W2, lane);
-        l4_position_gradients(s_gS[w][px], s_geo[w][px], true, box, s_g,
-                              (2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2, radius, H2, W2, scale, lane);
-        __syncwarp();
-        l4_box_gradients<NCH, 1>(f1, gf1, F2b, G2b, C, s_rows[w], box.bw * box.bh, s_gS[w], px, lane);
+        const L4Pixel g = s_geo[w][px];
+        const bool live = (mask >> px) & 1u;
+        for (int q = lane; q < nq; q += 32) {
+          const int row = q / box.bw, i = box.ox + q - row * box.bw - (g.bx - radius), j = box.oy + row - (g.by - radius);
+          s_gS[w][px][q] = live ? l4_position_gradient(g, i, j, s_g, pp0 + px / 2 * L4_TW + px % 2, radius, H2, W2) * scale : 0.f;
+        }
       }
+      __syncwarp();
+      l4_box_gradients<NCH, L4_PX>(f1, gf1, F2b, G2b, C, s_rows[w], nq, s_gS[w], 0, lane);
+    } else {
+      // motion boundaries: one pixel at a time, each over its own window.  All four pixels' positions are prepared together (a
+      // pixel alone leaves lanes idle and waits on its own), a pixel's rows behind its gradients.  Windows scattered over
+      // 2 x 55 x 128 at C = 256, radius 4, four levels: 1121 us with a preparation per pixel, 857 now.
+      const int side = 2 * radius + 2, nq = side * side;
+      for (int idx = lane; idx < L4_PX * nq; idx += 32) {
+        const int px = idx / nq, q = idx - px * nq, j = q / side, i = q - j * side;
+        const L4Pixel g = s_geo[w][px];
+        const int x = g.bx - radius + i, y = g.by - radius + j;
+        const bool live = (mask >> px) & 1u;
+        const float v = live ? l4_position_gradient(g, i, j, s_g, pp0 + px / 2 * L4_TW + px % 2, radius, H2, W2) * scale : 0.f;
+        s_gS[w][px][q] = v;
+        s_gS[w][px][L4_ALONE_ROWS + q] = __int_as_float(x >= 0 && x < W2 && y >= 0 && y < H2 && v != 0.f ? y * W2 + x : -1);
+      }
+      if (lane < L4_PX * L4_ALONE_PAD)   // a walk asks for up to L4_ALONE_PAD positions past the last
+        s_gS[w][lane / L4_ALONE_PAD][L4_ALONE_ROWS + nq + lane % L4_ALONE_PAD] = __int_as_float(-1);
+      __syncwarp();
+#pragma unroll
+      for (int px = 0; px < L4_PX; ++px)
+        if ((mask >> px) & 1u)
+          l4_box_gradients<NCH, 1>(f1, gf1, F2b, G2b, C, reinterpret_cast<const int*>(&s_gS[w][px][L4_ALONE_ROWS]), nq, s_gS[w], px,
+                                   lane);
     }
     __syncwarp();
   }

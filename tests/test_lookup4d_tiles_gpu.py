@@ -47,3 +47,25 @@ def test_spread_windows(size, spread, C, cuda_device):
     assert len(gF2) == levels
     for a, b in zip(gF2, rF2):
         assert relerr(a, b) < TOL
+
+
+@pytest.mark.parametrize("radius", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("C", [20, 132, 512])
+def test_scattered_windows(radius, C, cuda_device):
+    """Windows all over the image and beyond its edges, so that every walk is for one pixel, for every window size."""
+    H, W, H2, W2, levels = 7, 19, 22, 37, 2
+    g = torch.Generator().manual_seed(radius + C)
+    coords = torch.rand(2, 2, H, W, generator=g) * torch.tensor([W2 + 30.0, H2 + 30.0]).view(1, 2, 1, 1) - 15
+    f1 = torch.randn(2, H, W, C, generator=g)
+    f2 = torch.randn(2, C, H2, W2, generator=g)
+    F2s = [t.permute(0, 2, 3, 1).contiguous() for t in (f2, F.avg_pool2d(f2, 2, stride=2))]
+    dev = cuda_device
+    out = ops.lookup4d_forward(f1.to(dev), [t.to(dev) for t in F2s], coords.to(dev), radius, C ** -0.5)
+    ref = orc.lookup4d_forward(f1.double(), [t.double() for t in F2s], coords.double(), radius, C ** -0.5)
+    assert relerr(out, ref) < TOL
+    gout = torch.randn(out.shape, generator=g)
+    gF1, gF2 = ops.lookup4d_backward(f1.to(dev), [t.to(dev) for t in F2s], coords.to(dev), gout.to(dev), radius, C ** -0.5)
+    rF1, rF2 = orc.lookup4d_backward(f1.double(), [t.double() for t in F2s], coords.double(), gout.double(), radius, C ** -0.5)
+    assert relerr(gF1, rF1) < TOL and len(gF2) == levels
+    for a, b in zip(gF2, rF2):
+        assert relerr(a, b) < TOL
