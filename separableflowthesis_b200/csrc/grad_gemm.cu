@@ -411,7 +411,9 @@ __device__ float* grad_row(const GradArgs& a, const GradSched& sc, int m, size_t
   cstride = (size_t)a.d.N2();
   return a.out + (size_t)sc.b * C * a.d.N2() + (size_t)u * a.d.W2 + v;
 }
-// Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][channel][128 rows]
+// Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][channel][128 rows] or [tail][piece - 1][128 rows][channel], as the
+// output has it, so that the fold reads both in runs (channel-major pieces under a pixel-major output, 16-byte accesses 1 KB
+// apart, made the launch for 1 x 55 x 128 against 27 x 64 take 58 us; 47 now, 48 with whole tiles).
 __device__ __forceinline__ float* grad_part(const GradArgs& a, int tail, int piece) {
   return a.part + ((size_t)tail * (a.pieces - 1) + piece - 1) * a.d.C * TILE_M;
 }
@@ -426,11 +428,11 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
   const int m = q * 32 + lane;
   size_t cstride;
   float* dst = grad_row<I2MAJOR>(a, sc, m, cstride);
-  bool channel_major = a.out_cf != 0, accumulate = a.accumulate != 0;
+  const bool channel_major = a.out_cf != 0;
+  bool accumulate = a.accumulate != 0;
   if (sc.piece > 0) {
-    if (dst != nullptr) dst = grad_part(a, sc.tail, sc.piece) + m;
+    if (dst != nullptr) dst = grad_part(a, sc.tail, sc.piece) + (channel_major ? m : m * C);
     cstride = TILE_M;
-    channel_major = true;
     accumulate = false;
   }
   const uint32_t tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -469,62 +471,69 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
 }
 
 // Pieces 1.. of a finished tail tile added to the output, in piece order (all threads of the CTA that finished last).  One
-// SM's loads move all of it, so a thread takes four rows x four channels at once and asks for several pieces' values
-// before it uses any.
+// SM's loads move all of it, so a thread takes sixteen values at once and asks for several pieces' values before it uses any.
+constexpr int FOLD_PIECES = 2;
+__device__ __forceinline__ void fold_add(const float* const (&part)[4], const bool (&in)[4], size_t step, int pieces, float4 (&sum)[4]) {
+  for (int s0 = 1; s0 < pieces; s0 += FOLD_PIECES) {
+    float4 o[FOLD_PIECES][4];
+#pragma unroll
+    for (int q = 0; q < FOLD_PIECES; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        o[q][j] = s0 + q < pieces && in[j] ? __ldcg(reinterpret_cast<const float4*>(part[j] + (s0 + q - 1) * step))
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < FOLD_PIECES; ++q) {
+      if (s0 + q >= pieces) break;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) add4(sum[j], o[q][j]);
+    }
+  }
+}
+
 template <int I2MAJOR>
 __device__ void grad_fold_pieces(const GradArgs& a, const GradSched& sc) {
-  constexpr int QUADS = TILE_M / 4, FOLD_PIECES = 2;
-  const int C = a.d.C;
-  for (int i = threadIdx.x; i < C / 4 * QUADS; i += GG_THREADS) {  // C is a multiple of 4
-    const int m = i % QUADS * 4, c0 = i / QUADS * 4;
-    size_t cstride, unused;
-    float* row[4];   // the four rows are neighbours in the image: the ones that exist come first
-    row[0] = grad_row<I2MAJOR>(a, sc, m, cstride);
-    if (row[0] == nullptr) continue;
-    int cnt = 1;
-#pragma unroll
-    for (int r = 1; r < 4; ++r) {
-      row[r] = grad_row<I2MAJOR>(a, sc, m + r, unused);
-      cnt += row[r] != nullptr;
-    }
-    float4 v[4];     // channel-major output: [channel] over the rows; pixel-major: [row] over the channels
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      v[j] = a.out_cf ? load4_cg(row[0] + (c0 + j) * cstride, cnt) : load4_cg(row[j] + c0, j < cnt ? 4 : 0);
-    float4 sum[4];   // [channel] over the rows
-#pragma unroll
-    for (int j = 0; j < 4; ++j) sum[j] = a.out_cf ? v[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!a.out_cf) {
+  const int C = a.d.C;   // a multiple of 4
+  const float* const part0 = grad_part(a, sc.tail, 1);
+  const size_t step = (size_t)C * TILE_M;
+  float4 sum[4];
+  const float* part[4];
+  bool in[4];
+  size_t cstride;
+  if (a.out_cf) {   // channel-major: four rows, neighbours in the image (the ones that exist come first), of four channels
+    constexpr int QUADS = TILE_M / 4;
+    for (int i = threadIdx.x; i < C / 4 * QUADS; i += GG_THREADS) {
+      const int m = i % QUADS * 4, c0 = i / QUADS * 4;
+      float* const row = grad_row<I2MAJOR>(a, sc, m, cstride);
+      if (row == nullptr) continue;
+      const int cnt = min(4, I2MAJOR ? a.d.W2 - (sc.v0 + m % GG_ROW_VT) : a.d.N1() - (sc.m0 + m));
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        (&sum[j].x)[0] = (&v[0].x)[j]; (&sum[j].x)[1] = (&v[1].x)[j];
-        (&sum[j].x)[2] = (&v[2].x)[j]; (&sum[j].x)[3] = (&v[3].x)[j];
+        sum[j] = load4_cg(row + (c0 + j) * cstride, cnt);
+        part[j] = part0 + (size_t)(c0 + j) * TILE_M + m;
+        in[j] = true;
       }
+      fold_add(part, in, step, a.pieces, sum);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) store4(row + (c0 + j) * cstride, sum[j], cnt);
     }
-    const float* part = grad_part(a, sc.tail, 1) + (size_t)c0 * TILE_M + m;
-    const size_t step = (size_t)C * TILE_M;
-    for (int s0 = 1; s0 < a.pieces; s0 += FOLD_PIECES) {
-      float4 o[FOLD_PIECES][4];
+  } else {          // pixel-major, as the pieces are: runs of four channels of a row, neighbouring runs to neighbouring threads
+    const int runs = C / 4, n = runs * TILE_M;
+    for (int i0 = threadIdx.x; i0 < n; i0 += 4 * GG_THREADS) {
+      float* row[4];
 #pragma unroll
-      for (int q = 0; q < FOLD_PIECES; ++q)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          o[q][j] = s0 + q < a.pieces ? __ldcg(reinterpret_cast<const float4*>(part + (s0 + q - 1) * step + j * TILE_M))
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int q = 0; q < FOLD_PIECES; ++q) {
-        if (s0 + q >= a.pieces) break;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) add4(sum[j], o[q][j]);
+      for (int j = 0; j < 4; ++j) {
+        const int i = i0 + j * GG_THREADS, m = i / runs;
+        row[j] = i < n ? grad_row<I2MAJOR>(a, sc, m, cstride) : nullptr;
+        in[j] = row[j] != nullptr;
+        if (in[j]) row[j] += (i - m * runs) * 4;
+        sum[j] = load4_cg(row[j], in[j] ? 4 : 0);
+        part[j] = part0 + (size_t)i * 4;
       }
-    }
-    if (a.out_cf) {
+      fold_add(part, in, step, a.pieces, sum);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) store4(row[0] + (c0 + j) * cstride, sum[j], cnt);
-    } else {
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (r < cnt) store4(row[r] + c0, make_float4((&sum[0].x)[r], (&sum[1].x)[r], (&sum[2].x)[r], (&sum[3].x)[r]), 4);
+      for (int j = 0; j < 4; ++j)
+        if (in[j]) store4(row[j], sum[j], 4);
     }
   }
 }
@@ -647,7 +656,12 @@ static int grad_tiles(const Dims& d, int image2_major) {
 
 // How the tail tiles are cut, in units of one K block's time (32 values, about 0.6 us): a CTA costs about eight blocks of
 // prologue and drain, a fold reads 128 KB per piece through one SM (about two blocks).  Pieces must save a quarter of the
-// tail (see sweep_split) and at least four blocks to be used.
+// tail (see sweep_split) and at least twelve blocks to be used: with predicted savings of seven and eleven, launches of 23
+// (2 x 33 x 70 against 16 x 35) and 33 us (3 x 55 x 128 against 13 x 32) got one or two us slower.  Whole and cut tiles
+// measured, image-1-major and image-2-major form (us per launch, C = 256, FP16): 1 x 48 x 64: 60 and
+// 37, 62 and 38; 1 x 55 x 128: 150 and 104, 148 and 107; 4 x 55 x 128: 300 and 246, 299 and 280; 8 x 47 x 156: 508 and
+// 438, 541 and 476; 1 x 55 x 128 against 27 x 64: 48 and 40, 147 and 49; 1 x 135 x 240 against 67 x 120: 350 whole, 634 and
+// 335.
 TileSplit grad_split(const Dims& d, int image2_major) {
   const int tiles = grad_tiles(d, image2_major), rest = tiles % SM_COUNT;
   const int blocks = image2_major ? (d.N1() + GG_KJ - 1) / GG_KJ
@@ -659,7 +673,7 @@ TileSplit grad_split(const Dims& d, int image2_major) {
     const double waves = (rest * n + SM_COUNT - 1) / SM_COUNT;
     const double cost = waves * ((blocks + n - 1) / n + 8) + (n > 1 ? 2.0 * n * d.C / MAX_C + 2 : 0.0);
     if (n == 1) best = whole = cost;
-    if (cost < best && cost < 0.75 * whole && cost < whole - 4) { best = cost; r.pieces = n; }
+    if (cost < best && cost < 0.75 * whole && cost < whole - 12) { best = cost; r.pieces = n; }
   }
   if (r.pieces > 1) {
     r.whole_tiles = tiles - rest;
