@@ -230,6 +230,10 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
   }
   const bool valid = e.valid;
 
+  // A NaN of a piece's first block must not stand in for a later piece (nothing compares greater than it, and the fold would
+  // drop the piece): read back, it counts as -inf there.  It stays in a whole tile and in piece 0, as it always has.
+  const float least = CUT && sc.piece > 0 ? -CUDART_INF_F : CUDART_NAN_F;   // fmaxf(x, NaN) is x
+
   float cm[SWEEP_VT];
   int ca[SWEEP_VT];
   int vb = sc.vb0, ub = 0;
@@ -245,6 +249,10 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
 #pragma unroll
     for (int ul = 0; ul < SW_RW; ++ul)
       rold[ul] = (valid && vb > sc.vb0 && ul < nu) ? pu[(ubase + ul) * usd] : -CUDART_INF_F;
+    if (CUT) {
+#pragma unroll
+      for (int ul = 0; ul < SW_RW; ++ul) rold[ul] = fmaxf(rold[ul], least);
+    }
 
     if (!epi_wait(sm, a, t)) return;
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * (SW_RW * SWEEP_VT);
@@ -281,8 +289,6 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
             for (int j = 0; j < SWEEP_VT; ++j) cm[j] = fmaxf(cm[j], r[j]);
           }
           m *= e.osc;  // memory holds scaled-back values; compare and store in that domain
-          // the first block of a later piece is compared too (with -inf): a NaN there must not stand in for its piece
-          if (CUT && sc.piece > 0 && vb == sc.vb0 && !(m > -CUDART_INF_F)) m = -CUDART_INF_F;
           if (valid && (vb == sc.vb0 || m > rold[ul])) {  // strict: the lowest column block wins ties
             pu[u * usd] = m;
             if (ARG) pua[u * uasd] = __int_as_float(v0 + arg);
@@ -622,10 +628,16 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     tmem_dealloc(sm.tmem_base, SW_TMEM_COLS);
   }
   if constexpr (CUT) {
-    // the schedule is worked out again: kept over the epilogue, its registers would be spilled there
-    int block;
-    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
-    const SweepSched tail_sc = sweep_sched<MODE, CUT>(a, block);
+    const SweepSched tail_sc = [&] {
+      if constexpr (MODE == SWEEP_COMPRESS) {
+        // worked out again: kept over the compression epilogue, its registers would be spilled there
+        int block;
+        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
+        return sweep_sched<MODE, CUT>(a, block);
+      } else {
+        return sc;
+      }
+    }();
     if (tail_sc.tail >= 0 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
       __threadfence();  // this thread's results before the count ...
       __syncthreads();
