@@ -77,9 +77,8 @@ int sfb_max_avg_forward(const float* F1, const float* F2, float* MA_u, float* MA
  * real-time or serving loop that must never enter the allocator, a host application that hands this library nothing
  * but input and output buffers.  Its scratch is a fixed array of sfb_static_scratch_bytes() bytes (32 MiB) that is
  * part of the library image: every GPU that loads the library holds it until the process exits.
- *   - Shapes whose scratch need (that of sfb_max_avg_forward without its 16-bit copies and without the optional scratch
- *     of its tail pieces) exceeds that size are rejected with SFB_ERR_UNSUPPORTED_SHAPE; 48x64 feature maps with C=256
- *     fit.
+ *   - Shapes whose scratch need (that of sfb_max_avg_forward without the optional scratch of its tail pieces) exceeds
+ *     that size are rejected with SFB_ERR_UNSUPPORTED_SHAPE; 48x64 feature maps with C=256 fit.
  *   - Set-up: the first call on each device looks up the array's device address (cudaGetSymbolAddress, with that
  *     device current) and caches it; the first call of a thread that has no CUDA context current binds the device's
  *     primary context (cudaFree(0)).  Make those first calls before any stream capture begins.  Apart from that

@@ -221,7 +221,7 @@ struct Workspace {
   float* F1r;
   float* F2r;
   float* aux;
-  uint16_t* F1h;  // 16-bit copies (FP16 or BF16) of the three arrays above: operands of the kind::f16 sweeps
+  uint16_t* F1h;  // the same three as 16-bit copies (FP16 or BF16), in the same memory: operands of the kind::f16 sweeps
   uint16_t* F2h;
   uint16_t* auxh;
   float* xu;   // packed inputs indexed by (u, slot, pixel): (B, H2, Rx, n1p)
@@ -256,8 +256,9 @@ PixView cf_view(const void* base, int slots, int D, int N1) {
   return PixView{static_cast<float*>(const_cast<void*>(base)), (long long)slots * D * N1, (uint32_t)N1, (uint32_t)(D * N1)};
 }
 
-// What an op keeps in the workspace: the mean rows of F2, Rx packed input slots, Ro packed output slots.
-struct WsPlan { bool aux; int Rx; int Ro; int Rg; bool level_bwd; bool bf16; };
+// What an op keeps in the workspace: the mean rows of F2, Rx packed input slots, Ro packed output slots, Rg interleaved ones;
+// whether it has correlation sweeps, whose operands may be 16-bit copies of the features.
+struct WsPlan { bool aux; int Rx; int Ro; int Rg; bool level_bwd; bool sweeps; };
 constexpr int MAXAVG_SLOTS = 3;  // max, mean, argmax bits
 constexpr int MAXAVG_PART_SLOTS = 2;  // of a tail piece: max, argmax bits
 int chunk_channels(int Kc) { return Kc < KC_MAX_PER_SWEEP ? Kc : KC_MAX_PER_SWEEP; }
@@ -295,12 +296,10 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   w.F1r = take((size_t)d.B * d.N1() * d.C);
   w.F2r = take((size_t)d.B * d.N2() * d.C);
   w.aux = plan.aux ? take((size_t)d.B * d.aux_rows() * d.C) : nullptr;
-  w.F1h = w.F2h = w.auxh = nullptr;
-  if (plan.bf16) {   // half the floats of the fp32 copies
-    w.F1h = reinterpret_cast<uint16_t*>(take(((size_t)d.B * d.N1() * d.C + 1) / 2));
-    w.F2h = reinterpret_cast<uint16_t*>(take(((size_t)d.B * d.N2() * d.C + 1) / 2));
-    w.auxh = reinterpret_cast<uint16_t*>(take(((size_t)d.B * d.aux_rows() * d.C + 1) / 2));
-  }
+  // A call makes the copies of one operand type (Features::op16), so the 16-bit ones lie where the FP32 ones would be.
+  w.F1h = plan.sweeps ? reinterpret_cast<uint16_t*>(w.F1r) : nullptr;
+  w.F2h = plan.sweeps ? reinterpret_cast<uint16_t*>(w.F2r) : nullptr;
+  w.auxh = reinterpret_cast<uint16_t*>(w.aux);
   w.xu = plan.Rx ? take((size_t)d.B * d.H2 * plan.Rx * w.n1p) : nullptr;
   w.xv = plan.Rx ? take((size_t)d.B * d.W2 * plan.Rx * w.n1p) : nullptr;
   w.ou = plan.Ro ? take((size_t)d.B * d.H2 * plan.Ro * w.n1p) : nullptr;
@@ -326,7 +325,7 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   w.tail_count = reinterpret_cast<int*>(p + WS_TAIL_OFFSET);
   size_t part = 0;
   if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS, false).part_floats);
-  if (d.Kc > 0 && plan.bf16) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
+  if (d.Kc > 0 && plan.sweeps) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
   if (plan.Rg) part = std::max(part, std::max(grad_split(d, 0).part_floats, grad_split(d, 1).part_floats));
   w.part = reinterpret_cast<float*>(p + off);
   w.part_bytes = part * sizeof(float);
@@ -783,8 +782,7 @@ int sfb_max_avg_forward_static(const float* F1, const float* F2, float* MA_u, fl
   Dims d;
   SFB_TRY(check_shape(shape, false, &d));
   SFB_CHECK_PTR(F1); SFB_CHECK_PTR(F2); SFB_CHECK_PTR(MA_u); SFB_CHECK_PTR(MA_v);
-  WsPlan plan = plan_for(SFB_OP_MAX_AVG_FORWARD, d);
-  plan.bf16 = false;  // this entry point always computes with TF32 operands: no room is set aside for 16-bit copies
+  const WsPlan plan = plan_for(SFB_OP_MAX_AVG_FORWARD, d);
   const size_t need = carve(d, nullptr, plan).bytes;
   if (need > STATIC_ARRAY_BYTES)
     return fail(SFB_ERR_UNSUPPORTED_SHAPE,

@@ -142,3 +142,13 @@ def test_missing_library_fails_loudly(tmp_path):
     out = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr
     assert out.stdout.strip().endswith("raised")
+
+
+def test_workspace_holds_the_copies_of_one_operand_type(lib):
+    """A call makes FP32 copies of the features or 16-bit ones, never both: the workspace has room for the larger kind, not
+    for their sum.  148 tiles are one full wave, so there is no scratch for pieces of tiles."""
+    B, H, W, C = 1, 148, 128, 64
+    s = _lib.SfbShape(B, H, W, H, W, C, 2)
+    copies = 4 * C * (2 * H * W + H + W)    # both images and the mean rows of image 2
+    assert lib.sfb_workspace_bytes(_lib.OP_MAX_AVG_FORWARD_CF, ctypes.byref(s)) == 1024 + copies
+    assert lib.sfb_workspace_bytes(_lib.OP_COMPRESSION_CF, ctypes.byref(s)) == 1024 + 4 * C * 2 * H * W
