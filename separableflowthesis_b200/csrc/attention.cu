@@ -2,10 +2,11 @@
 //   A = softmax_over_d( Conv3d(2 -> Kc, 3x3x3, padding 1)(X) )       core/corr.py:437-442, core/sepflow.py:59-60
 // on the channels-first tensors X (B, 2, D, H1, W1) -> A (B, Kc, D, H1, W1), and its backward.
 //
-// Every kernel gives one thread one image-1 pixel (h, w) and lets it walk the displacement axis d, so that a
-// warp reads 32 neighbouring pixels of a (channel, d) plane per load and the softmax over d stays inside the
-// thread.  The 3x3x3 stencil is applied in "scatter" form: the 3x3 neighbourhood of the plane that was just
-// loaded is added into the three outputs (d-1, d, d+1) it belongs to, which are kept in registers.
+// The stencil kernels give one thread one image-1 pixel (h, w) and let it walk the displacement axis d, or a piece of it, so
+// that a warp reads 32 neighbouring pixels of a (channel, d) plane per load.  The 3x3x3 stencil is applied in "scatter" form:
+// the 3x3 neighbourhood of the plane that was just loaded is added into the three outputs (d-1, d, d+1) it belongs to, which
+// are kept in registers.  The softmax over d and its backward are kernels of their own that share a pixel's column among
+// warps (short columns: the softmax ends the walk).
 //
 // Two things decide the speed of such a walk, and both are handled explicitly:
 //  * latency: a thread needs plane e+1 only after it is done with plane e, so on its own it has one plane of
@@ -15,7 +16,7 @@
 //    costs a 32-lane register write per weight, more than the FMA they feed; instead the weights of the (up to
 //    four) channels being processed are staged in __constant__ memory, where an FMA reads them as an operand.
 //
-//   forward     : logits -> A (a first kernel parks the raw logits in A, a second one normalises them in place)
+//   forward     : logits -> A (the stencil kernel parks the raw logits in A, where they are normalised in place)
 //   logit grads : gL = A * (gA - sum_d gA*A), in place over gA; per-block sums of gL for the bias gradient
 //   input grads : gX = transposed stencil of gL (+ an optional addend: the direct gradient of the max/avg channels)
 //   weight grads: gW[k,c,tap] = sum X(shifted by tap) * gL, per-block partial sums, reduced in a fixed order by

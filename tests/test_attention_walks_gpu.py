@@ -9,7 +9,11 @@ from separableflowthesis_b200 import ops
 
 pytestmark = pytest.mark.gpu
 
-# FP32 stencils of 54 products, softmax with __expf (2 ulp at |x| < 10) and sums of up to 300 weights: a few 1e-6
+# Weights relative to their norm.  A logit is an FP32 sum of 54 products of about 0.3: roundings of 2^-24 of a running sum of
+# a few units, sqrt(54) of them, up to 2e-6, which is the relative error it gives its weight.  __expf(x) is within
+# 2 + floor(abs(1.173 x)) ulp (its documented bound): 4 ulp = 5e-7 for the weights near a column's maximum, which carry the
+# norm, 13 ulp at x = -10, where a weight is 5e-5 of them.  The sum of up to 300 weights adds sqrt(300) 2^-24 = 1e-6.  About
+# 4e-6 in all; the gradients pass through two such sums more.
 TOL = 2e-5
 DS = [1, 2, 7, 8, 9, 17, 32, 33, 64, 65, 128, 129, 256, 257, 300]
 

@@ -1,5 +1,5 @@
-"""The 4D lookup's pixel blocks where neighbouring windows lie so far apart that a walk serves fewer pixels: two rows of
-four, single pixels, blocks cut by the image border, and a mix of all in one CTA, for one to four 128-channel chunks."""
+"""The 4D lookup's blocks of 2 x 2 pixels where the windows lie so far apart that a walk serves one pixel at a time, blocks cut
+by the image border, and blocks of both kinds in one CTA, for one to four 128-channel chunks."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -27,7 +27,7 @@ def test_spread_windows(size, spread, C, cuda_device):
     g = torch.Generator().manual_seed(C + W)
     ys, xs = torch.meshgrid(torch.arange(H).float(), torch.arange(W).float(), indexing="ij")
     coords = torch.stack((xs + 14, ys + 14)) + torch.rand(2, H, W, generator=g)
-    if spread in ("rows", "all"):       # every other row 18 below: the two rows of a block of 4 x 2 need a walk each
+    if spread in ("rows", "all"):       # every other row 18 below: the two rows of a block of 2 x 2 do not fit one walk
         coords[1] += 18 * (ys.long() % 2)
     if spread in ("columns", "all"):    # some columns far to the side: pixel by pixel there, together elsewhere
         coords[0] += 21 * (xs.long() % 5 == 3)
