@@ -332,6 +332,8 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   return w;
 }
 
+int sweep_launches(const SweepArgs& a) { return a.pieces > 1 ? 2 : 1; }   // pieces are folded by a kernel of their own
+
 // A sweep's cut into whole tiles and pieces, as far as the workspace has scratch for the pieces.
 void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
   const TileSplit s = sweep_split(a.d, slots, a.mode == SWEEP_COMPRESS);
@@ -341,7 +343,6 @@ void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
   a.parts = cut ? s.parts : 0;
   a.part_slots = slots;
   a.part = w.part;
-  a.tail_count = w.tail_count;
 }
 
 // The same for a gradient GEMM.
@@ -537,7 +538,7 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   a.pv_arg = packed_view(w.ov, d.W2, MAXAVG_SLOTS, w.n1p, 2);
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
-  SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
+  SFB_CUDA(timed(KID_SWEEP_MAXAVG, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   // packed (displacement, slot, pixel) -> the reference's (pixel, channel, displacement) tensors
   const int N1 = d.N1(), R = MAXAVG_SLOTS;
   SFB_CUDA(timed(KID_PACK, with_argmax ? 4 : 2, st, [&] {
@@ -572,7 +573,7 @@ int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm
     a.out_scale = out_scale;
     a.status = w.status;
     set_sweep_split(a, w, chunk_channels(d.Kc));
-    SFB_CUDA(timed(KID_SWEEP_COMPRESS, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_f2 /* unused */, st); }));
+    SFB_CUDA(timed(KID_SWEEP_COMPRESS, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_f2 /* unused */, st); }));
   }
   return SFB_OK;
 }
@@ -1044,7 +1045,7 @@ int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v
   a.pv_arg = cf_view(AM_v, 1, d.W2, N1);
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
-  SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
+  SFB_CUDA(timed(KID_SWEEP_MAXAVG, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   return SFB_OK;
 }
 
@@ -1257,7 +1258,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   a.out_scale = sweep_out_scale(w, op16);
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
-  SFB_CUDA(timed(KID_SWEEP_MAXAVG, 1, st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
+  SFB_CUDA(timed(KID_SWEEP_MAXAVG, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
   const AttentionDims at_u{d.B, K, d.W2, d.H1, d.W1}, at_v{d.B, K, d.H2, d.H1, d.W1};
   const float *const X_u = SEP_u + (size_t)c0 * d.W2 * N1, *const X_v = SEP_v + (size_t)c0 * d.H2 * N1;

@@ -42,8 +42,8 @@ constexpr int KBLK = 32;      // fp32 elements in one 128-byte swizzled row
 #endif
 constexpr int MAX_KB = SFB_MAX_KB;  // feature dimension C <= MAX_KB * KBLK
 constexpr int MAX_C = MAX_KB * KBLK;
-constexpr int SWEEP_UT = 16;  // image-2 rows per correlation tile (16 x 16 = 256 accumulator columns)
-constexpr int SWEEP_VT = 16;  // image-2 columns per correlation tile
+constexpr int SWEEP_UT = 8;   // image-2 rows per correlation tile (8 x 32 = 256 accumulator columns)
+constexpr int SWEEP_VT = 32;  // image-2 columns per correlation tile
 constexpr int GG_ROW_UT = 8;  // row tile of the image-2-major gradient GEMM: 8 x 16 image-2 pixels = 128 TMEM lanes
 constexpr int GG_ROW_VT = 16;
 constexpr int GG_UT = 2;      // image-2 rows per K-block of the gradient GEMM (image-1-major form)
@@ -93,10 +93,9 @@ struct SweepArgs {
   int* status;           // device status word
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
   int drop_last_load;    // test hook: the producer leaves out its last F2 block, so that one wait runs out
-  // Tiles past `whole_tiles` are done by `pieces` CTAs each (TileSplit); part / tail_count are unused when pieces is 1.
+  // Tiles past `whole_tiles` are done by `pieces` CTAs each (TileSplit); part is unused when pieces is 1.
   int whole_tiles, pieces, parts, part_slots;
   float* part;
-  int* tail_count;       // one zero per tail tile; every launch leaves them zero
 };
 
 // How a launch of equal tiles fills the SMs: whole_tiles CTAs do one tile each, every further tile is done by `pieces`
@@ -137,7 +136,7 @@ struct GradArgs {
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
   int whole_tiles, pieces;           // as in SweepArgs, here with pieces of the K sweep (TileSplit)
   float* part;
-  int* tail_count;
+  int* tail_count;       // one zero per tail tile; every launch leaves them zero
 };
 TileSplit grad_split(const Dims& d, int image2_major);
 
@@ -168,7 +167,7 @@ struct SlotSources {
 
 // Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, all cleared by
 // launch_prepare.  amax slots hold float bits (atomicMax), the others floats; every scale is a power of two.
-// From WS_TAIL_OFFSET on, SM_COUNT counters of the tail tiles (SweepArgs::tail_count).
+// From WS_TAIL_OFFSET on, SM_COUNT counters of the tail tiles (GradArgs::tail_count).
 constexpr size_t WS_HEADER_BYTES = 1024, WS_SCALES_OFFSET = 64, WS_TAIL_OFFSET = 256, WS_HEADER_CLEAR_BYTES = 1024;
 static_assert(WS_TAIL_OFFSET + SM_COUNT * sizeof(int) <= WS_HEADER_CLEAR_BYTES, "tail counters");
 enum : int {

@@ -70,7 +70,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Waits for the phase with the given parity.  Never spins forever: after the CTA's time limit, or as
 // soon as another role of this CTA has given up, it records `code` in *status (first error
 // wins), raises the CTA-wide abort flag and returns false.  Callers leave their loops on false.
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, WaitCtl* ctl, int* status,
+static __device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, WaitCtl* ctl, int* status,
                                                    int code) {
   const unsigned long long t0 = global_ns();
   const unsigned long long limit = *reinterpret_cast<volatile unsigned long long*>(&ctl->limit_ns);
@@ -287,6 +287,46 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
       : "memory");
 #pragma unroll
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The same 16 columns without the wait: the registers may be read after tmem_ld_wait16 on them, which waits for every load
+// this thread has issued (it names them so that no use of theirs is scheduled before it).
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+
+// Largest of three values, and 1 where two are equal, else 0: one instruction each.  NaNs are passed over / never equal.
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float is_equal(float a, float b) {
+  float r;
+  asm("set.eq.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// Registers a thread of this warpgroup may use from here on (every warp of the warpgroup calls it with the same N).
+template <int N, bool UP>
+__device__ __forceinline__ void set_max_registers() {
+  static_assert(N % 8 == 0 && N >= 24 && N <= 256, "register count");
+  if constexpr (UP) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+  else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
 // Named barriers (ids 1..15; id 0 is __syncthreads): one warpgroup signals, the other waits.

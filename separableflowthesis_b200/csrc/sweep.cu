@@ -2,71 +2,84 @@
 // accumulator in TMEM, reduced in the epilogue so that S never reaches HBM.
 //
 // One CTA owns 128 consecutive image-1 pixels of one sample (the rows / TMEM lanes of every
-// accumulator tile) and sweeps all image-2 pixels in tiles of SWEEP_UT x SWEEP_VT (16 rows x 16
+// accumulator tile) and sweeps all image-2 pixels in tiles of SWEEP_UT x SWEEP_VT (8 rows x 32
 // columns = 256 accumulator columns), column-blocks outermost.  Warp roles:
 //   warp 0      TMA producer: F1 tile once (stays resident), F2 tiles through a ring of stages
-//   warp 1      allocates TMEM, issues tcgen05.mma (TF32 in, FP32 accumulate), 2 accumulators in flight
-//   warps 2..   epilogue warpgroups (two, or four for the compression epilogue); in each, one thread per
-//               image-1 pixel reads its accumulator lane with tcgen05.ld.  All groups consume every tile and
-//               split its work.
+//   warp 1      allocates TMEM, issues tcgen05.mma (TF32 or 16-bit in, FP32 accumulate), 2 accumulators in flight
+//   warps 2, 3  idle: they make up a warpgroup, the unit in which registers are handed to the epilogues
+//   warps 4..11 two epilogue warpgroups; in each, one thread per image-1 pixel reads its accumulator lane with
+//               tcgen05.ld.  Both groups consume every tile and split its work.
 // Everything indexed by an image-1 pixel is read and written in the packed, pixel-fastest layout
 // (kernels.h), so a warp's 32 lanes touch one 128-byte line per access.
 // Epilogues
-//   max/avg      : group g takes tile rows 8g..8g+7.  Running column-direction max(+argmax) in
-//                  registers across the inner row-block loop (the two groups' partial results are merged
+//   max/avg      : group g takes tile rows 4g..4g+3.  Running column-direction max(+argmax) in
+//                  registers across the inner row-block loop (the two groups' partial results are put together
 //                  once per column block), row-direction max(+argmax) merged through the packed output
 //                  once per tile.  The two mean channels come from extra tiles whose "image-2 pixels"
 //                  are the row-mean and column-mean feature rows of F2 (mean_v S[u,v] = F1 . mean_v F2[u,v]).
+//   compression  : OU[k,u] = sum_v S*w_u[k,v] (reduced per tile, accumulated with red.add), OV[k,v] = sum_u S*w_v[k,u]
+//                  (register accumulators across the inner loop); two channels to a thread.
+// Code that runs once per CTA or column block is fetched cold and is kept short (loops, running pointers, no branch per
+// element): unrolled, the mean channels alone took as long as the tiles of a 55 x 128 launch.
 // Tail tiles: a grid that is not a multiple of 148 tiles leaves SMs idle in its last wave (and a single 55 x 128 pair has
 // 55 tiles in all), so the tiles past the last full wave are cut into `pieces` CTAs, each a range of column blocks.  Column
-// results are complete within a piece; row results of pieces 1.. go to scratch, and the CTA that finishes a tile last (a
-// counter per tile, nobody waits) folds them into piece 0's results in piece order, so the result does not depend on timing.
-//   compression  : group g takes channel g.  OU[k,u] = sum_v S*w_u[k,v] (reduced per tile, accumulated
-//                  with red.add), OV[k,v] = sum_u S*w_v[k,u] (register accumulators across the inner loop).
+// results are complete within a piece; row results of pieces 1.. go to scratch, and sweep_fold_kernel folds them into piece
+// 0's results in piece order, so the result does not depend on timing.
 // Replaces the reference kernels MemorySaver_kernel_forward.cu:128-313, :328-533, :550-753.
 #include <math_constants.h>
+
+#include <type_traits>
 
 #include "kernels.h"
 #include "sm100_primitives.cuh"
 
 namespace sfb {
 
-constexpr int SW_NSTAGE = 3;                    // 3 x 32 KB of F2 blocks next to the 128 KB resident F1 tile
 constexpr int SW_NACC = 2;                      // 2 x 256 TMEM columns
 constexpr int SW_TILE_N = SWEEP_UT * SWEEP_VT;  // 256 accumulator columns: tcgen05.mma issues at a fixed
                                                 // rate per instruction, so the widest N does the most work
-// Epilogue warps: two warpgroups for the max/avg and dump epilogues (each takes half of a tile's rows), four for
-// the compression epilogue (each takes one channel and reads the whole tile): its work per cell is 2 FMAs per
-// channel, and with 16 warps the FP32 pipes keep up with the tensor pipe.
-__host__ __device__ constexpr int sw_epi_warps(int mode) { return mode == SWEEP_COMPRESS ? 16 : 8; }
-__host__ __device__ constexpr int sw_threads(int mode) { return 64 + sw_epi_warps(mode) * 32; }
-constexpr int SW_RW = SWEEP_UT / 2;             // tile rows of one epilogue warpgroup
+constexpr int SW_EPI_WARPS = 8;                 // two epilogue warpgroups
+constexpr int SW_THREADS = 128 + SW_EPI_WARPS * 32;
+// Registers a thread (setmaxnreg): the launch has 168 for each of its 384 threads; the four warps of the first warpgroup
+// (TMA, MMA, two idle) need few, and the epilogues keep two channels' weights and sums of 32 columns (128 registers).
+constexpr int SW_REGS_LAUNCH = 168, SW_REGS_ISSUE = 40, SW_REGS_EPI = 232;
+static_assert(SW_REGS_ISSUE + 2 * SW_REGS_EPI <= 3 * SW_REGS_LAUNCH, "more registers than the launch has");
+constexpr int SW_RW = SWEEP_UT / 2;             // tile rows of one epilogue warpgroup when the two split a tile's rows
 constexpr int SW_NMERGE = 4;                    // ring of column-merge barriers (> SW_NACC tiles of run-ahead)
 constexpr uint32_t SW_STAGE_BYTES = SW_TILE_N * KBLK * 4;
 constexpr uint32_t SW_F1_BLOCK_BYTES = TILE_M * KBLK * 4;
 constexpr uint32_t SW_TMEM_COLS = 512;
+// Image-2 blocks (32 KB) in flight: what the resident image-1 tile leaves.  128 KB of it (TF32, 256 channels) leave three,
+// 64 KB (16-bit) five.
+constexpr int SW_MAX_STAGES = 6;
+constexpr uint32_t SW_RING_BYTES = MAX_KB * SW_F1_BLOCK_BYTES + 3 * SW_STAGE_BYTES;   // image-1 tile and ring together
+__device__ __forceinline__ uint32_t sw_stages(int nkb) {
+  const uint32_t n = (SW_RING_BYTES - nkb * SW_F1_BLOCK_BYTES) / SW_STAGE_BYTES;
+  return n < SW_MAX_STAGES ? n : SW_MAX_STAGES;
+}
 static_assert(SW_NACC * SW_TILE_N <= 512, "accumulators exceed TMEM");
 static_assert(SW_NMERGE > SW_NACC, "a warpgroup can run SW_NACC tiles ahead of the other");
-static_assert(SW_TILE_N == 256 && SW_RW * SWEEP_VT == 128, "epilogues read two 64-column halves per warpgroup");
+static_assert(SWEEP_UT == 8 && SWEEP_VT == 32, "the epilogues read a row as two 16-column halves, four rows per warpgroup");
 
 struct SweepSmem {
-  float f1[MAX_KB][TILE_M * KBLK];        // resident image-1 tile, one 128B-swizzled block per 32 channels
-  float f2[SW_NSTAGE][SW_TILE_N * KBLK];  // ring of image-2 tile blocks
+  uint8_t ring[SW_RING_BYTES];            // image-1 tile, one 128B-swizzled block per 128 bytes of channels; then the ring of
+                                          // image-2 tile blocks
   uint64_t f1_full;
-  uint64_t full[SW_NSTAGE];
-  uint64_t empty[SW_NSTAGE];
+  uint64_t full[SW_MAX_STAGES];
+  uint64_t empty[SW_MAX_STAGES];
   uint64_t acc_full[SW_NACC];
   uint64_t acc_empty[SW_NACC];
-  uint64_t merge[SW_NMERGE];              // group 1 -> group 0: partial column results are in memory
+  uint64_t merge[2][SW_NMERGE];           // to group g: the other group's part of g's columns is in memory
   uint32_t tmem_base;
-  int last_piece;                         // this CTA finished its tail tile last: it folds the pieces together
   WaitCtl ctl;
+  __device__ __forceinline__ uint8_t* f1(int kb) { return ring + kb * SW_F1_BLOCK_BYTES; }
+  __device__ __forceinline__ uint8_t* f2(int nkb, uint32_t stage) { return ring + nkb * SW_F1_BLOCK_BYTES + stage * SW_STAGE_BYTES; }
 };
 constexpr size_t SW_SMEM_BYTES = sizeof(SweepSmem) + 1024;  // + slack to align the base to 1024 B
 
 struct SweepSched {
   int b, m0, nkb, n_ub;
-  int vb0;              // first column block of this CTA
+  int vb0, vb1;         // column blocks vb0 .. vb1 - 1 of this CTA
   int t_main, t_total;  // tiles of its column blocks; the same plus the tiles of the mean rows
   int tail, piece;      // tail tile this CTA has a piece of (-1: a whole tile) and which piece
   int part_vb0;         // first column block of piece 1
@@ -105,7 +118,8 @@ __device__ __forceinline__ SweepSched sweep_sched(const SweepArgs& a, int block)
   const int n_pieces = CUT && sc.tail >= 0 ? a.pieces : 1;
   sc.vb0 = piece_start(n_vb, n_pieces, sc.piece);
   sc.part_vb0 = piece_start(n_vb, n_pieces, 1);
-  sc.t_main = sc.n_ub * (piece_start(n_vb, n_pieces, sc.piece + 1) - sc.vb0);
+  sc.vb1 = piece_start(n_vb, n_pieces, sc.piece + 1);
+  sc.t_main = sc.n_ub * (sc.vb1 - sc.vb0);
   const bool has_aux = (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG);
   const bool does_aux = has_aux && sc.piece == n_pieces - 1;       // the mean rows go to the last, smallest piece
   sc.t_total = sc.t_main + (does_aux ? (a.d.H2 + a.d.W2 + SW_TILE_N - 1) / SW_TILE_N : 0);
@@ -117,20 +131,21 @@ __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSch
                                const CUtensorMap* tm_f2, const CUtensorMap* tm_aux) {
   const int kel = a.op16 ? 2 * KBLK : KBLK;  // channels in one 128-byte row
   mbar_expect_tx(&sm.f1_full, sc.nkb * SW_F1_BLOCK_BYTES);
-  for (int kb = 0; kb < sc.nkb; ++kb) tma_load_3d(sm.f1[kb], tm_f1, &sm.f1_full, kb * kel, sc.m0, sc.b);
-  uint32_t it = 0;
+  for (int kb = 0; kb < sc.nkb; ++kb) tma_load_3d(sm.f1(kb), tm_f1, &sm.f1_full, kb * kel, sc.m0, sc.b);
+  const uint32_t n_stages = sw_stages(sc.nkb);
+  uint32_t s = 0, ph = 0;
   int vb = sc.vb0, ub = 0;
   for (int t = 0; t < sc.t_total; ++t) {
     const bool main_tile = t < sc.t_main;
-    for (int kb = 0; kb < sc.nkb; ++kb, ++it) {
-      const uint32_t s = it % SW_NSTAGE, ph = (it / SW_NSTAGE) & 1u;
+    for (int kb = 0; kb < sc.nkb; ++kb) {
       if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
       if (a.drop_last_load && t == sc.t_total - 1 && kb == sc.nkb - 1) return;  // test hook: this block never arrives
       mbar_expect_tx(&sm.full[s], SW_STAGE_BYTES);
       if (main_tile)
-        tma_load_4d(sm.f2[s], tm_f2, &sm.full[s], kb * kel, vb * SWEEP_VT, ub * SWEEP_UT, sc.b);
+        tma_load_4d(sm.f2(sc.nkb, s), tm_f2, &sm.full[s], kb * kel, vb * SWEEP_VT, ub * SWEEP_UT, sc.b);
       else
-        tma_load_3d(sm.f2[s], tm_aux, &sm.full[s], kb * kel, (t - sc.t_main) * SW_TILE_N, sc.b);
+        tma_load_3d(sm.f2(sc.nkb, s), tm_aux, &sm.full[s], kb * kel, (t - sc.t_main) * SW_TILE_N, sc.b);
+      if (++s == n_stages) { s = 0; ph ^= 1u; }
     }
     if (++ub == sc.n_ub) { ub = 0; ++vb; }
   }
@@ -143,18 +158,18 @@ __device__ void sweep_mma(SweepSmem& sm, const SweepArgs& a, const SweepSched& s
   const bool op16 = a.op16 != 0;
   if (!mbar_wait(&sm.f1_full, 0, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
   tc_fence_after();
-  uint32_t it = 0;
+  const uint32_t n_stages = sw_stages(sc.nkb);
+  uint32_t s = 0, ph = 0;
   for (int t = 0; t < sc.t_total; ++t) {
     const uint32_t acc = t % SW_NACC, aph = (t / SW_NACC) & 1u;
     if (!mbar_wait(&sm.acc_empty[acc], aph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
     tc_fence_after();
     const uint32_t d_tmem = sm.tmem_base + acc * SW_TILE_N;
-    for (int kb = 0; kb < sc.nkb; ++kb, ++it) {
-      const uint32_t s = it % SW_NSTAGE, ph = (it / SW_NSTAGE) & 1u;
+    for (int kb = 0; kb < sc.nkb; ++kb) {
       if (!mbar_wait(&sm.full[s], ph, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
       tc_fence_after();
-      const uint64_t adesc = make_smem_desc_sw128(smem_u32(sm.f1[kb]), 16, 1024);
-      const uint64_t bdesc = make_smem_desc_sw128(smem_u32(sm.f2[s]), 16, 1024);
+      const uint64_t adesc = make_smem_desc_sw128(smem_u32(sm.f1(kb)), 16, 1024);
+      const uint64_t bdesc = make_smem_desc_sw128(smem_u32(sm.f2(sc.nkb, s)), 16, 1024);
       if (op16) {
 #pragma unroll
         for (int k = 0; k < 4; ++k)  // one instruction consumes K = 16 16-bit values = 32 bytes of each row
@@ -165,6 +180,7 @@ __device__ void sweep_mma(SweepSmem& sm, const SweepArgs& a, const SweepSched& s
           umma_tf32(d_tmem, desc_advance(adesc, k * 32), desc_advance(bdesc, k * 32), idesc_tf32, (kb | k) != 0);
       }
       umma_commit(&sm.empty[s]);  // stage reusable once these MMAs have read it
+      if (++s == n_stages) { s = 0; ph ^= 1u; }
     }
     umma_commit(&sm.acc_full[acc]);
   }
@@ -196,22 +212,49 @@ __device__ __forceinline__ void epi_release(SweepSmem& sm, int t, int lane) {
   if (lane == 0) mbar_arrive(&sm.acc_empty[t % SW_NACC]);
 }
 
-// Maximum of 16 values and the LOWEST index holding it: pairwise tournament, the left (lower-index)
-// entry survives ties.  Same comparison count as a linear scan but only four dependent steps.
-__device__ __forceinline__ void max16_first(const float* r, float& m, int& arg) {
-  float v8[8], v4[4], v2[2];
-  int i8[8], i4[4], i2[2];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) { const bool g = r[2 * i + 1] > r[2 * i]; v8[i] = g ? r[2 * i + 1] : r[2 * i]; i8[i] = g ? 2 * i + 1 : 2 * i; }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { const bool g = v8[2 * i + 1] > v8[2 * i]; v4[i] = g ? v8[2 * i + 1] : v8[2 * i]; i4[i] = g ? i8[2 * i + 1] : i8[2 * i]; }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) { const bool g = v4[2 * i + 1] > v4[2 * i]; v2[i] = g ? v4[2 * i + 1] : v4[2 * i]; i2[i] = g ? i4[2 * i + 1] : i4[2 * i]; }
-  const bool g = v2[1] > v2[0];
-  m = g ? v2[1] : v2[0];
-  arg = g ? i2[1] : i2[0];
+// Column results of a block that the two groups hold parts of: each stores its part of the other's 16 columns to the output
+// and arrives, waits for the other, reads its own columns' other part back (all of it before it stores anything: a load that
+// follows a store waits for it, and one memory latency per column took longer than the block's tiles) and stores the two
+// together.
+__device__ __forceinline__ void merge_publish(SweepSmem& sm, const SweepSched& sc, int vb, const EpiCtx& e) {
+  __threadfence_block();
+  __syncwarp();
+  if (e.lane == 0) mbar_arrive(&sm.merge[1 - e.wg][(vb - sc.vb0) % SW_NMERGE]);
+}
+__device__ __forceinline__ bool merge_wait(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, int vb, const EpiCtx& e) {
+  const bool ok = mbar_wait(&sm.merge[e.wg][(vb - sc.vb0) % SW_NMERGE], ((vb - sc.vb0) / SW_NMERGE) & 1u, &sm.ctl, a.status,
+                            DEV_TIMEOUT_EPILOGUE);
+  return __all_sync(0xffffffffu, ok);
 }
 
+// Largest of 16 values; NaNs are passed over.
+__device__ __forceinline__ float max16(const uint32_t (&r)[16]) {
+  float m = fmax3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
+#pragma unroll
+  for (int i = 3; i + 1 < 16; i += 2) m = fmax3(m, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+  return fmaxf(m, __uint_as_float(r[15]));
+}
+// Which of the values equal m, as a sum of powers of two: value j of the first n - 1 counts 2^(n-1-j).  The lowest j is then the
+// leading bit, and the last value is the one when no bit is set.  One comparison on the ALU pipe and one multiply-add on the
+// FMA pipe per value, where carrying an index through a tournament takes a comparison and two selects, all on the ALU pipe
+// (half rate), which set the pace: 3 ALU operations per cell and direction.
+__device__ __forceinline__ float equal_bits16(const uint32_t (&r)[16], float m) {
+  float bits = 0.f;
+#pragma unroll
+  for (int j = 0; j < 15; ++j) bits = fmaf(is_equal(__uint_as_float(r[j]), m), static_cast<float>(1 << (15 - j)), bits);
+  return bits;
+}
+__device__ __forceinline__ int first_of16(float bits) {   // 2^15 .. 2^1: 0 .. 14; zero: 15
+  return min(142 - static_cast<int>(__float_as_uint(bits) >> 23), 15);
+}
+
+// Max / arg-max / mean.  Bound: the tensor core (some 2400 cycles per tile) without arg-max, and with it the ALU pipe (half
+// rate: about 480 of its instructions per warp and tile, 1900 cycles) beside what two warps per scheduler cannot hide.
+// 135 x 240, one pair, without / with arg-max: 590 -> 465 / 868 -> 630 us; 55 x 128: 81 -> 38 / 81 -> 50.
+// Group g takes tile rows 4g .. 4g+3, as two units of 4 rows x 16 columns, the second one being loaded
+// while the first is worked on.  State across the row blocks: the running maximum of each of the 32 columns and (ARG) where it
+// lies, as the float 8 * (row / 4) + (bits of the row inside its four rows), which is exact up to 2^24.
+// NaN entries are passed over; a row that holds nothing else has the maximum NaN at index 0, such a column -inf at index 0.
 template <bool ARG, bool CUT>
 __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
   const int H2 = a.d.H2, W2 = a.d.W2;
@@ -229,230 +272,353 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
     usd = uasd = TILE_M;
   }
   const bool valid = e.valid;
+  const bool all_valid = sc.m0 + TILE_M <= a.n_valid;
 
-  // A NaN of a piece's first block must not stand in for a later piece (nothing compares greater than it, and the fold would
-  // drop the piece): read back, it counts as -inf there.  It stays in a whole tile and in piece 0, as it always has.
-  const float least = CUT && sc.piece > 0 ? -CUDART_INF_F : CUDART_NAN_F;   // fmaxf(x, NaN) is x
-
-  float cm[SWEEP_VT];
-  int ca[SWEEP_VT];
-  int vb = sc.vb0, ub = 0;
-  for (int t = 0; t < sc.t_main; ++t) {
-    const int v0 = vb * SWEEP_VT, ubase = ub * SWEEP_UT + e.wg * SW_RW;
-    const int nu = min(SW_RW, H2 - ubase), nv = min(SWEEP_VT, W2 - v0);  // nu may be <= 0
-    if (ub == 0) {
+  float rnext[SW_RW];
+  auto load_rows = [&](int ub, bool none) {
+    const int u0 = ub * SWEEP_UT + e.wg * SW_RW;
 #pragma unroll
-      for (int j = 0; j < SWEEP_VT; ++j) { cm[j] = -CUDART_INF_F; ca[j] = 0; }
-    }
-    // row-direction state of earlier column blocks (issued before the wait to hide the latency)
+    for (int r = 0; r < SW_RW; ++r) rnext[r] = valid && !none && u0 + r < H2 ? pu[(u0 + r) * usd] : -CUDART_INF_F;
+  };
+#pragma unroll
+  for (int r = 0; r < SW_RW; ++r) rnext[r] = -CUDART_INF_F;
+  int main_tiles = 0;
+  for (int vb = sc.vb0; vb < sc.vb1; ++vb) {
+   const int v0 = vb * SWEEP_VT, nv = min(SWEEP_VT, W2 - v0);
+   const bool first = vb == sc.vb0;
+   float cm[SWEEP_VT], ca[SWEEP_VT];
+#pragma unroll
+   for (int j = 0; j < SWEEP_VT; ++j) { cm[j] = -CUDART_INF_F; ca[j] = 4.f; }
+   for (int ub = 0; ub < sc.n_ub; ++ub, ++main_tiles) {
+    const int t = main_tiles;
+    const int ubase = ub * SWEEP_UT + e.wg * SW_RW;
+    const int nu = min(SW_RW, H2 - ubase);  // may be <= 0
+    // row-direction state of earlier column blocks: asked for one tile ahead, unless that tile has the same rows
+    if (sc.n_ub == 1) load_rows(ub, first);
     float rold[SW_RW];
 #pragma unroll
-    for (int ul = 0; ul < SW_RW; ++ul)
-      rold[ul] = (valid && vb > sc.vb0 && ul < nu) ? pu[(ubase + ul) * usd] : -CUDART_INF_F;
-    if (CUT) {
-#pragma unroll
-      for (int ul = 0; ul < SW_RW; ++ul) rold[ul] = fmaxf(rold[ul], least);
-    }
+    for (int r = 0; r < SW_RW; ++r) rold[r] = rnext[r];
+    if (sc.n_ub > 1) load_rows(ub + 1 < sc.n_ub ? ub + 1 : 0, first && ub + 1 < sc.n_ub);
+    const float qbits = static_cast<float>(ubase / SW_RW * 8);
 
     if (!epi_wait(sm, a, t)) return;
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * (SW_RW * SWEEP_VT);
+    // two units of 4 rows x 16 columns; half of the second one is on its way while the first is worked on (all of it would
+    // cost the arg-max form registers that it does not have)
+    uint32_t s[2][SW_RW][16];
+    auto load = [&](int h, int r) { tmem_ld16_issue(tacc + r * SWEEP_VT + h * 16, s[h][r]); };
+    float rmax[SW_RW], rbits[SW_RW];
+    auto unit = [&](auto half, auto whole) {   // whole: every lane, row and column of this thread's part of the tile exists
+      constexpr int h = decltype(half)::value;
+      constexpr bool WHOLE = decltype(whole)::value;
+      uint32_t(&x)[SW_RW][16] = s[h];
+      if (!WHOLE) {  // cells outside the image are passed over
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      float s[64];
-      tmem_ld64(tacc + half * 64, s);
-      if (half == 1) epi_release(sm, t, e.lane);  // all values are in registers: hand the accumulator back
+        for (int r = 0; r < SW_RW; ++r)
 #pragma unroll
-      for (int hl = 0; hl < SW_RW / 2; ++hl) {
-        const int ul = half * (SW_RW / 2) + hl;
-        if (ul < nu) {  // warp-uniform
-          float* r = &s[hl * SWEEP_VT];
-          if (nv < SWEEP_VT) {
+          for (int j = 0; j < 16; ++j)
+            if (r >= nu || h * 16 + j >= nv) x[r][j] = 0x7FFFFFFFu;
+      }
+      // rows
 #pragma unroll
-            for (int j = 0; j < SWEEP_VT; ++j)
-              if (j >= nv) r[j] = -CUDART_INF_F;  // padded columns never win a max
-          }
-          const int u = ubase + ul;
-          float m;
-          int arg;
+      for (int r = 0; r < SW_RW; ++r) {
+        const float mh = max16(x[r]), bits = ARG ? equal_bits16(x[r], mh) : 0.f;
+        if (h == 0) {
+          rmax[r] = mh;
+          rbits[r] = bits;
+          continue;
+        }
+        const float m = fmaxf(rmax[r], mh);
+        int arg = 0;
+        if (ARG) {
+          const bool left = rmax[r] == m;
+          arg = first_of16(left ? rbits[r] : bits) + (left ? v0 : v0 + 16);
+          arg = m == m ? arg : 0;
+        }
+        const float ms = m * e.osc;  // memory holds scaled-back values; compare and store in that domain
+        float* const dst = pu + (ubase + r) * usd;
+        float* const dst_arg = ARG ? pua + (ubase + r) * uasd : nullptr;
+        const bool more = ms > fmaxf(rold[r], -CUDART_INF_F);  // strict: the lowest column block wins ties
+        if ((WHOLE || (valid && r < nu)) && (first || more)) {
+          *dst = ms;
+          if (ARG) *dst_arg = __int_as_float(arg);
+        }
+      }
+      // columns
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float x0 = __uint_as_float(x[0][j]), x1 = __uint_as_float(x[1][j]);
+        const float x2 = __uint_as_float(x[2][j]), x3 = __uint_as_float(x[3][j]);
+        float &c = cm[h * 16 + j], &where = ca[h * 16 + j];
+        if (ARG) {
+          const float m = fmaxf(fmax3(x0, x1, x2), x3);
+          const float bits = fmaf(is_equal(x0, m), 4.f, fmaf(is_equal(x1, m), 2.f, qbits + is_equal(x2, m)));
+          const bool more = m > c;  // strict: the lowest rows win ties
+          c = more ? m : c;
+          where = more ? bits : where;
+        } else {
+          c = fmax3(fmax3(c, x0, x1), x2, x3);
+        }
+      }
+    };
+    auto tile = [&](auto whole) {
+#pragma unroll
+      for (int r = 0; r < SW_RW; ++r) load(0, r);
+#pragma unroll
+      for (int r = 0; r < SW_RW; ++r) tmem_ld_wait16(s[0][r]);
+#pragma unroll
+      for (int r = 0; r < SW_RW / 2; ++r) load(1, r);
+      unit(std::integral_constant<int, 0>{}, whole);
+#pragma unroll
+      for (int r = SW_RW / 2; r < SW_RW; ++r) load(1, r);
+#pragma unroll
+      for (int r = 0; r < SW_RW; ++r) tmem_ld_wait16(s[1][r]);
+      epi_release(sm, t, e.lane);  // all values are in registers: hand the accumulator back
+      unit(std::integral_constant<int, 1>{}, whole);
+    };
+    if (all_valid && nu == SW_RW && nv == SWEEP_VT) tile(std::true_type{});
+    else tile(std::false_type{});
+   }
+    // end of a column block: group 0 puts columns 0 .. 15 together, group 1 the others
+    {
+      auto row = [&](int j) {
+        const int code = static_cast<int>(ca[j]);
+        return (code >> 3) * SW_RW + __clz(code & 7) - 29;   // 4, 2, 1, 0 stand for rows 0 .. 3 of the four
+      };
+      const int cols = valid ? nv : 0;   // columns this lane has
+      auto merge = [&](auto own_half) -> bool {
+        constexpr int OWN = decltype(own_half)::value * 16, OTHER = 16 - OWN;
+        float* q = pv + (v0 + OTHER) * vsd;
+        float* qa = ARG ? pva + (v0 + OTHER) * vasd : nullptr;
+#pragma unroll
+        for (int j = OTHER; j < OTHER + 16; ++j, q += vsd, qa += ARG ? vasd : 0) {
+          if (j < cols) *q = cm[j] * e.osc;
+          if (ARG && j < cols) *qa = __int_as_float(row(j));
+        }
+        merge_publish(sm, sc, vb, e);
+        if (!merge_wait(sm, a, sc, vb, e)) return false;
+        q = pv + (v0 + OWN) * vsd;
+        if (ARG) qa = pva + (v0 + OWN) * vasd;
+        float om[16], oa[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j, q += vsd, qa += ARG ? vasd : 0) {
+          om[j] = OWN + j < cols ? __ldcg(q) : 0.f;
+          if (ARG) oa[j] = OWN + j < cols ? __ldcg(qa) : 0.f;
+        }
+        q = pv + (v0 + OWN) * vsd;
+        if (ARG) qa = pva + (v0 + OWN) * vasd;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, q += vsd, qa += ARG ? vasd : 0) {
+          const float mine = cm[OWN + j] * e.osc;
           if (ARG) {
-            max16_first(r, m, arg);
-#pragma unroll
-            for (int j = 0; j < SWEEP_VT; ++j) {
-              if (r[j] > cm[j]) { cm[j] = r[j]; ca[j] = u; }  // strict: lowest u of this group wins ties
-            }
+            const int o = __float_as_int(oa[j]), own = row(OWN + j);
+            const bool other = om[j] > mine || (om[j] == mine && o < own);  // lowest u on ties
+            if (OWN + j < cols) *q = other ? om[j] : mine;
+            if (OWN + j < cols) *qa = __int_as_float(other ? o : own);
           } else {
-            m = r[0];
-            arg = 0;
-#pragma unroll
-            for (int j = 1; j < SWEEP_VT; ++j) m = fmaxf(m, r[j]);
-#pragma unroll
-            for (int j = 0; j < SWEEP_VT; ++j) cm[j] = fmaxf(cm[j], r[j]);
-          }
-          m *= e.osc;  // memory holds scaled-back values; compare and store in that domain
-          if (valid && (vb == sc.vb0 || m > rold[ul])) {  // strict: the lowest column block wins ties
-            pu[u * usd] = m;
-            if (ARG) pua[u * uasd] = __int_as_float(v0 + arg);
+            if (OWN + j < cols) *q = fmaxf(mine, om[j]);
           }
         }
-      }
+        return true;
+      };
+      if (!(e.wg == 0 ? merge(std::integral_constant<int, 0>{}) : merge(std::integral_constant<int, 1>{}))) return;
     }
-    if (ub == sc.n_ub - 1) {
-      // end of a column block: group 1 publishes its partial column maxima, group 0 merges and stores
-      uint64_t* bar = &sm.merge[(vb - sc.vb0) % SW_NMERGE];
-      if (e.wg == 1) {
-#pragma unroll
-        for (int j = 0; j < SWEEP_VT; ++j) {
-          if (valid && j < nv) {
-            pv[(v0 + j) * vsd] = cm[j] * e.osc;
-            if (ARG) pva[(v0 + j) * vasd] = __int_as_float(ca[j]);
-          }
-        }
-        __threadfence_block();
-        __syncwarp();
-        if (e.lane == 0) mbar_arrive(bar);
-      } else {
-        const bool ok = mbar_wait(bar, ((vb - sc.vb0) / SW_NMERGE) & 1u, &sm.ctl, a.status, DEV_TIMEOUT_EPILOGUE);
-        if (!__all_sync(0xffffffffu, ok)) return;
-#pragma unroll
-        for (int j = 0; j < SWEEP_VT; ++j) {
-          if (valid && j < nv) {
-            float* dst = pv + (v0 + j) * vsd;
-            const float om = __ldcg(dst);
-            float best = cm[j] * e.osc;
-            int besta = ca[j];
-            if (ARG) {
-              float* dsta = pva + (v0 + j) * vasd;
-              const int oa = __float_as_int(__ldcg(dsta));
-              if (om > best || (om == best && oa < besta)) { best = om; besta = oa; }  // lowest u on ties
-              *dsta = __int_as_float(besta);
-            } else {
-              best = fmaxf(best, om);
-            }
-            dst[0] = best;
-          }
-        }
-      }
-    }
-    if (++ub == sc.n_ub) { ub = 0; ++vb; }
   }
-  // mean channels: accumulator column r of an aux tile is F1[p] . (row-mean u=r | column-mean v=r-H2)
+  // mean channels: accumulator column r of an aux tile is F1[p] . (row-mean u=r | column-mean v=r-H2).  A loop over 16 columns
+  // at a time: this code runs once per CTA, so its instructions are fetched cold, and unrolled over 128 columns with a branch
+  // each it took 33,000 cycles, as long as the tiles of a 55 x 128 launch.
   const int naux = H2 + W2;
+  float* const pvm = pv + vss;
   for (int t = sc.t_main; t < sc.t_total; ++t) {
     if (!epi_wait(sm, a, t)) return;
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * 128;
+    const int r_end = min(naux, (t - sc.t_main) * SW_TILE_N + e.wg * 128 + 128);
+#pragma unroll 1
+    for (int r0 = (t - sc.t_main) * SW_TILE_N + e.wg * 128, c0 = 0; r0 < r_end; r0 += 16, c0 += 16) {
+      float s[16];
+      tmem_ld16(tacc + c0, s);
+      if (!valid) continue;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int r0 = (t - sc.t_main) * SW_TILE_N + e.wg * 128 + half * 64;
-      if (r0 < naux) {  // warp-uniform
-        float s[64];
-        tmem_ld64(tacc + half * 64, s);
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          const int r = r0 + j;
-          if (!valid) continue;
-          if (r < H2) pum[r * umsd] = s[j] * e.osc;
-          else if (r < naux) pv[(r - H2) * vsd + vss] = s[j] * e.osc;
-        }
+      for (int j = 0; j < 16; ++j) {
+        const int r = r0 + j;
+        float* const dst = r < H2 ? pum + r * umsd : pvm + (r - H2) * vsd;
+        if (r < r_end) *dst = s[j] * e.osc;
       }
     }
     epi_release(sm, t, e.lane);
   }
 }
 
-template <bool CUT>
+// acc += (lo, hi) * w on a packed pair; lo and hi are tcgen05.ld registers: volatile keeps the multiply-add behind the
+// tcgen05.wait::ld before it.
+__device__ __forceinline__ void fma2_tmem(uint64_t& acc, uint32_t lo, uint32_t hi, uint64_t w) {
+  asm volatile("{\n\t.reg .b64 s;\n\tmov.b64 s, {%1, %2};\n\tfma.rn.f32x2 %0, s, %3, %0;\n\t}" : "+l"(acc) : "r"(lo), "r"(hi), "l"(w));
+}
+
+// Compression sums.  A thread does CPT channels of its pixel.  With three or four channels the two groups take two each and read
+// whole tiles; with one or two (SPLIT) both do all of them and share a tile's rows, and the column sums of a block are put
+// together at its end.
+//   au2[c][j] = (w_u[v0+2j], w_u[v0+2j+1])         weights of this column block, per column pair
+//   cv2[c][j] = running (OV[v0+2j], OV[v0+2j+1])   over the rows of the column block
+// Cells outside the image hold S = 0 (TMA zero-fills the missing F2 rows) and get weight 0, so every tile is processed
+// whole and only the stores at the edges are predicated.
+// Bound: the FMA pipe and the register ports.  A cell takes a packed multiply-add (fma.rn.f32x2) per channel and direction;
+// with three different 64-bit operands that instruction takes 3 cycles of a scheduler (measured; 2.2 with one operand kept),
+// 3072 cycles per tile and scheduler at four channels, where the tensor core needs some 2600.  As scalar multiply-adds, twice
+// as many instructions at 1 cycle, the same loop was slower (780 .. 910 us): it is then issue that runs short.
+// What else mattered: one value per row of 32 columns and channel leaves a tile, instead of one per 16 (16 x 16 tiles); 16
+// columns are loaded while 16 others are worked on; loops nested by column block, so that the 128 registers of weights and
+// sums are not moved around at every tile (450 of 1860 instructions per warp and tile were moves); the row weights of the
+// next tile are asked for before the wait for this one.  135 x 240, one pair, four channels: 897 -> 717 us (8 pairs, two
+// sweeps: 14.2 -> 10.9 ms); 8 x 47 x 156, two channels: 337 -> 290 us.
+template <int CPT, bool SPLIT, bool CUT>
 __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
+  constexpr int NR = SPLIT ? SW_RW : SWEEP_UT;   // tile rows of this thread
   const int H2 = a.d.H2, W2 = a.d.W2;
-  const bool active = e.wg < a.kc;            // this warpgroup's channel exists (warp-uniform)
-  const bool valid = e.valid && active;
+  const int k_first = SPLIT ? 0 : e.wg * CPT;    // its first channel among those of this launch
+  const int n_ch = min(CPT, a.kc - k_first);     // how many of them exist
   const uint32_t xusd = a.xu.sd, xvsd = a.xv.sd, ovsd = a.ov.sd;
-  uint32_t ousd = a.ou.sd;
-  // this thread's pixel and channel in sample b of each view; displacement d at ptr[d*sd], 32-bit offsets
-  const int k = a.k0 + e.wg;
-  const float* wu = a.xv.base + sc.b * a.xv.sb + e.p + (a.wu_slot0 + k * a.w_stride) * a.xv.ss;  // w_u[k][v]
-  const float* wv = a.xu.base + sc.b * a.xu.sb + e.p + (a.wv_slot0 + k * a.w_stride) * a.xu.ss;  // w_v[k][u]
+  uint32_t ousd = a.ou.sd, ouss = a.ou.ss;
+  const uint32_t wuss = (uint32_t)a.w_stride * a.xv.ss, wvss = (uint32_t)a.w_stride * a.xu.ss, ovss = a.ov.ss;
+  // this thread's pixel and first channel in sample b of each view; displacement d at ptr[d*sd], 32-bit offsets.  Weights that
+  // do not exist (lanes past the image, a second channel past the last) are read from the nearest that do.
+  const int k = a.k0 + k_first, p_in = min(e.p, a.n_valid - 1);
+  const float* wu = a.xv.base + sc.b * a.xv.sb + p_in + (a.wu_slot0 + k * a.w_stride) * a.xv.ss;  // w_u[k][v]
+  const float* wv = a.xu.base + sc.b * a.xu.sb + p_in + (a.wv_slot0 + k * a.w_stride) * a.xu.ss;  // w_v[k][u]
   float* ou = a.ou.base + sc.b * a.ou.sb + e.p + k * a.ou.ss;
   float* ov = a.ov.base + sc.b * a.ov.sb + e.p + k * a.ov.ss;
-  // The first column block initialises the row sums, the others are added to them.  A later piece stores every block, into
-  // a part of its own (slot = channel of this launch).
+  // The first column block initialises the row sums, the others are added to them (same thread, same address in every block,
+  // hence ordered).  A later piece stores every block, into a part of its own (slot = channel of this launch).
   uint32_t part_step = 0;
   if (CUT && sc.piece > 0) {
-    ou = sweep_part(a, sc.tail, sc.vb0 - sc.part_vb0, e.wg) + (e.p - sc.m0);
+    ou = sweep_part(a, sc.tail, sc.vb0 - sc.part_vb0, k_first) + (e.p - sc.m0);
     ousd = TILE_M;
+    ouss = (uint32_t)H2 * TILE_M;
     part_step = (uint32_t)a.part_slots * H2 * TILE_M;
   }
-
-  // Both sums run on packed FP32 pairs (two neighbouring columns per fma.rn.f32x2), which halves the
-  // instructions per cell: the epilogue warps share their schedulers' issue slots, and with scalar FMAs
-  // those slots, not the tensor pipe, set the pace of this sweep.
-  //   au2[j] = (w_u[v0+2j], w_u[v0+2j+1])         weights of this column block, per column pair
-  //   cv2[j] = running (OV[v0+2j], OV[v0+2j+1])   over the rows of the column block
-  // Cells outside the image hold S = 0 (TMA zero-fills the missing F2 rows) and get weight 0, so every
-  // tile is processed whole and only the loads and stores at the edges are predicated.
-  uint64_t au2[SWEEP_VT / 2], cv2[SWEEP_VT / 2];
-  int vb = sc.vb0, ub = 0;
-  for (int t = 0; t < sc.t_main; ++t) {
-    const int v0 = vb * SWEEP_VT, u0 = ub * SWEEP_UT;
-    const int nu = min(SWEEP_UT, H2 - u0), nv = min(SWEEP_VT, W2 - v0);
-    if (ub == 0) {
-      const float* wu_t = wu + v0 * xvsd;
+  const int row0 = SPLIT ? e.wg * SW_RW : 0;
+  float av[CPT][NR];   // w_v of the coming tile's rows (past the image: the last row's)
+  auto load_av = [&](int u0) {
 #pragma unroll
-      for (int j = 0; j < SWEEP_VT / 2; ++j) {
-        const float lo = (valid && 2 * j < nv) ? __ldg(wu_t + (2 * j) * xvsd) : 0.f;
-        const float hi = (valid && 2 * j + 1 < nv) ? __ldg(wu_t + (2 * j + 1) * xvsd) : 0.f;
-        au2[j] = pack2(lo, hi);
-        cv2[j] = 0ull;
+    for (int c = 0; c < CPT; ++c)
+#pragma unroll
+      for (int ul = 0; ul < NR; ++ul) av[c][ul] = __ldg(wv + (c < n_ch ? c * wvss : 0u) + min(u0 + ul, H2 - 1) * xusd);
+  };
+  load_av(row0);
+  int t = 0;
+  for (int vb = sc.vb0; vb < sc.vb1; ++vb, ou += part_step) {
+    const int v0 = vb * SWEEP_VT, nv = min(SWEEP_VT, W2 - v0);
+    const bool first = vb == 0 || part_step != 0;
+    uint64_t au2[CPT][SWEEP_VT / 2], cv2[CPT][SWEEP_VT / 2];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+      const float* wu_t = wu + v0 * xvsd + (c < n_ch ? c * wuss : 0u);
+#pragma unroll
+      for (int j = 0; j < SWEEP_VT; j += 2) {
+        au2[c][j / 2] = pack2(j < nv ? __ldg(wu_t + j * xvsd) : 0.f, j + 1 < nv ? __ldg(wu_t + (j + 1) * xvsd) : 0.f);
+        cv2[c][j / 2] = 0ull;
       }
     }
-    float av[SWEEP_UT];
-    {
-      const float* wv_t = wv + u0 * xusd;
+    for (int ub = 0; ub < sc.n_ub; ++ub, ++t) {
+      const int u0 = ub * SWEEP_UT + row0, nu = min(NR, H2 - u0);   // nu may be <= 0
+      uint64_t a2[CPT][NR];
 #pragma unroll
-      for (int ul = 0; ul < SWEEP_UT; ++ul) av[ul] = (valid && ul < nu) ? __ldg(wv_t + ul * xusd) : 0.f;
-    }
-
-    if (!epi_wait(sm, a, t)) return;
-    const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N;
-    if (active) {
-      float* ou_t = ou + u0 * ousd;
-      const bool first = vb == 0 || part_step != 0;
+      for (int c = 0; c < CPT; ++c)
 #pragma unroll
-      for (int pr = 0; pr < SWEEP_UT / 2; ++pr) {
-        float s[2 * SWEEP_VT];
-        tmem_ld32(tacc + pr * 2 * SWEEP_VT, s);
-        if (pr == SWEEP_UT / 2 - 1) epi_release(sm, t, e.lane);  // last read of this tile
+        for (int ul = 0; ul < NR; ++ul) {
+          const float w = ul < nu ? av[c][ul] : 0.f;   // rows past the image hold S = 0; their weight must not be an infinity
+          a2[c][ul] = pack2(w, w);
+        }
+      load_av((ub + 1 == sc.n_ub ? 0 : ub + 1) * SWEEP_UT + row0);
+      int rows[CPT];   // rows of each channel that are stored
+      float* dst[CPT];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int ul = 2 * pr + h;
-          const uint64_t av2 = pack2(av[ul], av[ul]);
-          uint64_t r2 = 0ull;
+      for (int c = 0; c < CPT; ++c) {
+        rows[c] = e.valid && c < n_ch ? nu : 0;
+        dst[c] = ou + u0 * ousd + c * ouss;
+      }
+      if (!epi_wait(sm, a, t)) return;
+      const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + row0 * SWEEP_VT;
+      uint32_t s[2][16];
+      uint64_t r2[CPT];
+      tmem_ld16_issue(tacc, s[0]);
 #pragma unroll
-          for (int j = 0; j < SWEEP_VT / 2; ++j) {
-            const uint64_t s2 = pack2(s[h * SWEEP_VT + 2 * j], s[h * SWEEP_VT + 2 * j + 1]);
-            r2 = j == 0 ? mul2(s2, au2[0]) : fma2(s2, au2[j], r2);
-            cv2[j] = fma2(s2, av2, cv2[j]);
-          }
-          if (valid && ul < nu) {
-            float* dst = ou_t + ul * ousd;
-            const float r = sum2(r2) * e.osc;
-            if (first) *dst = r;
-            else atomicAdd(dst, r);  // same thread, same address in every column block: ordered
+      for (int i = 0; i < 2 * NR; ++i) {   // 16 columns of a row at a time, the next ones on their way
+        const int ul = i / 2, h = i % 2;
+        tmem_ld_wait();
+        if (i + 1 < 2 * NR) tmem_ld16_issue(tacc + (i + 1) * 16, s[(i + 1) % 2]);
+        else epi_release(sm, t, e.lane);   // last read of this tile
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          if (h == 0) r2[c] = 0ull;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) fma2_tmem(cv2[c][h * 8 + j], s[i % 2][2 * j], s[i % 2][2 * j + 1], a2[c][ul]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) fma2_tmem(r2[c], s[i % 2][2 * j], s[i % 2][2 * j + 1], au2[c][h * 8 + j]);
+        if (h == 1) {
+#pragma unroll
+          for (int c = 0; c < CPT; ++c, dst[c - 1] += ousd) {
+            if (rows[c] > ul) {
+              const float x = sum2(r2[c]) * e.osc;
+              if (first) *dst[c] = x;
+              else atomicAdd(dst[c], x);
+            }
           }
         }
       }
-    } else {
-      epi_release(sm, t, e.lane);
     }
-    if (ub == sc.n_ub - 1) {
-      float* ov_t = ov + v0 * ovsd;
+    float cv[CPT][SWEEP_VT];
 #pragma unroll
-      for (int j = 0; j < SWEEP_VT / 2; ++j) {
-        float lo, hi;
-        unpack2(cv2[j], lo, hi);
-        if (valid && 2 * j < nv) ov_t[(2 * j) * ovsd] = lo * e.osc;
-        if (valid && 2 * j + 1 < nv) ov_t[(2 * j + 1) * ovsd] = hi * e.osc;
+    for (int c = 0; c < CPT; ++c)
+#pragma unroll
+      for (int j = 0; j < SWEEP_VT / 2; ++j) unpack2(cv2[c][j], cv[c][2 * j], cv[c][2 * j + 1]);
+    auto column = [&](int c, int j) { return ov + (v0 + j) * ovsd + c * ovss; };
+    auto columns = [&](int c) { return e.valid && c < n_ch ? nv : 0; };   // how many of them this thread has
+    if constexpr (!SPLIT) {
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        float* q = column(c, 0);
+        const int n = columns(c);
+#pragma unroll
+        for (int j = 0; j < SWEEP_VT; ++j, q += ovsd)
+          if (j < n) *q = cv[c][j] * e.osc;
       }
+    } else {
+      auto merge = [&](auto own_half) -> bool {
+        constexpr int OWN = decltype(own_half)::value * 16, OTHER = 16 - OWN;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          float* q = column(c, OTHER);
+          const int n = columns(c);
+#pragma unroll
+          for (int j = OTHER; j < OTHER + 16; ++j, q += ovsd)
+            if (j < n) *q = cv[c][j] * e.osc;
+        }
+        merge_publish(sm, sc, vb, e);
+        if (!merge_wait(sm, a, sc, vb, e)) return false;
+        float o[CPT][16];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          const float* q = column(c, OWN);
+          const int n = columns(c);
+#pragma unroll
+          for (int j = 0; j < 16; ++j, q += ovsd) o[c][j] = OWN + j < n ? __ldcg(q) : 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          float* q = column(c, OWN);
+          const int n = columns(c);
+#pragma unroll
+          for (int j = 0; j < 16; ++j, q += ovsd)
+            if (OWN + j < n) *q = cv[c][OWN + j] * e.osc + o[c][j];
+        }
+        return true;
+      };
+      if (!(e.wg == 0 ? merge(std::integral_constant<int, 0>{}) : merge(std::integral_constant<int, 1>{}))) return;
     }
-    if (++ub == sc.n_ub) { ub = 0; ++vb; ou += part_step; }
   }
 }
 
@@ -486,84 +652,11 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
   }
 }
 
-// The parts of a finished tail tile folded into piece 0's row results, in order (all threads of the CTA that finished last).
-// Maxima: a later piece has the higher columns, so only a strictly larger value replaces.  Sums: block by block, the order
-// in which a whole tile adds them, so that a sample's sums do not depend on the cut, which follows the batch and the row
-// range.  One SM's loads are all that moves these bytes, so a thread takes four pixels of up to FOLD_ROWS rows at once and
-// asks for several parts' values before it uses any (with one 4-byte load at a time a fold of 135 rows x 4 channels took as
-// long as the sweep).
-__device__ __forceinline__ void max4_first(float& v, float& arg, float o, float oarg) {
-  if (o > v) { v = o; arg = oarg; }
-}
-template <int MODE>
-__device__ void sweep_fold_pieces(const SweepArgs& a, const SweepSched& sc) {
-  constexpr int NT = sw_threads(MODE), QUADS = TILE_M / 4, FOLD_ROWS = MODE == SWEEP_MAXAVG ? 4 : 2, FOLD_PARTS = MODE == SWEEP_COMPRESS ? 6 : 2;
-  const int H2 = a.d.H2, n = (MODE == SWEEP_COMPRESS ? a.kc : 1) * H2 * QUADS;
-  for (int i0 = threadIdx.x; i0 < n; i0 += FOLD_ROWS * NT) {
-    float* dst[FOLD_ROWS];
-    float* arg_dst[FOLD_ROWS];
-    const float* part[FOLD_ROWS];   // the first part's values; part s is s * part_slots slots further on
-    int cnt[FOLD_ROWS];
-    float4 v[FOLD_ROWS], va[FOLD_ROWS];
-#pragma unroll
-    for (int r = 0; r < FOLD_ROWS; ++r) {
-      const int i = i0 + r * NT, px = i % QUADS * 4, q = i / QUADS, k = q / H2, u = q - k * H2, p = sc.m0 + px;
-      cnt[r] = i < n ? min(4, a.n_valid - p) : 0;
-      if (cnt[r] <= 0) { cnt[r] = 0; dst[r] = arg_dst[r] = nullptr; part[r] = a.part; continue; }
-      if (MODE == SWEEP_COMPRESS) dst[r] = a.ou.base + sc.b * a.ou.sb + p + (a.k0 + k) * a.ou.ss + u * a.ou.sd;
-      else dst[r] = a.pu.base + sc.b * a.pu.sb + p + u * a.pu.sd;
-      arg_dst[r] = MODE == SWEEP_MAXARGAVG ? a.pu_arg.base + sc.b * a.pu_arg.sb + p + u * a.pu_arg.sd : nullptr;
-      part[r] = sweep_part(a, sc.tail, 0, k) + (size_t)u * TILE_M + px;
-      v[r] = load4_cg(dst[r], cnt[r]);
-      if (MODE == SWEEP_MAXARGAVG) va[r] = load4_cg(arg_dst[r], cnt[r]);
-    }
-    const size_t slot = (size_t)H2 * TILE_M, step = slot * a.part_slots;
-    for (int s0 = 0; s0 < a.parts; s0 += FOLD_PARTS) {
-      float4 o[FOLD_PARTS][FOLD_ROWS], oa[MODE == SWEEP_MAXARGAVG ? FOLD_PARTS : 1][FOLD_ROWS];
-#pragma unroll
-      for (int j = 0; j < FOLD_PARTS; ++j)
-#pragma unroll
-        for (int r = 0; r < FOLD_ROWS; ++r) {
-          const bool ok = s0 + j < a.parts && cnt[r] > 0;
-          const float* src = part[r] + (s0 + j) * step;
-          // lanes past the image were never written: their values are loaded and dropped
-          o[j][r] = ok ? __ldcg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (MODE == SWEEP_MAXARGAVG)
-            oa[j][r] = ok ? __ldcg(reinterpret_cast<const float4*>(src + slot)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-      for (int j = 0; j < FOLD_PARTS; ++j) {
-        if (s0 + j >= a.parts) break;
-#pragma unroll
-        for (int r = 0; r < FOLD_ROWS; ++r) {
-          if (MODE == SWEEP_COMPRESS) {
-            add4(v[r], o[j][r]);
-          } else if (MODE == SWEEP_MAXARGAVG) {
-            max4_first(v[r].x, va[r].x, o[j][r].x, oa[j][r].x);
-            max4_first(v[r].y, va[r].y, o[j][r].y, oa[j][r].y);
-            max4_first(v[r].z, va[r].z, o[j][r].z, oa[j][r].z);
-            max4_first(v[r].w, va[r].w, o[j][r].w, oa[j][r].w);
-          } else {
-            v[r] = make_float4(o[j][r].x > v[r].x ? o[j][r].x : v[r].x, o[j][r].y > v[r].y ? o[j][r].y : v[r].y,
-                               o[j][r].z > v[r].z ? o[j][r].z : v[r].z, o[j][r].w > v[r].w ? o[j][r].w : v[r].w);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < FOLD_ROWS; ++r) {
-      if (cnt[r] == 0) continue;
-      store4(dst[r], v[r], cnt[r]);
-      if (MODE == SWEEP_MAXARGAVG) store4(arg_dst[r], va[r], cnt[r]);
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------------- kernel
-// CUT: the launch has tail pieces.  A launch without any runs the kernel without their bookkeeping, whose registers cost
-// the compression epilogue 10 % (it is at its register limit: 897 -> 990 us at 135 x 240).
-template <int MODE, bool CUT>
-__global__ void __launch_bounds__(sw_threads(MODE), 1)
+// CUT: the launch has tail pieces.  A launch without any runs the kernel without their bookkeeping.
+// KC (compression): channels of the launch, 1, 2 or (three or four) 4.
+template <int MODE, bool CUT, int KC>
+__global__ void __launch_bounds__(SW_THREADS, 1)
 sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ CUtensorMap tm_f2,
              const __grid_constant__ CUtensorMap tm_aux, const SweepArgs a) {
   if (*reinterpret_cast<volatile int*>(a.status) != 0) return;  // an earlier CTA gave up: do not pile on
@@ -573,13 +666,12 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw + pad);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const SweepSched sc = sweep_sched<MODE, CUT>(a, blockIdx.x);
 
   if (threadIdx.x == 0) {
     mbar_init(&sm.f1_full, 1);
-    for (int s = 0; s < SW_NSTAGE; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
-    for (int i = 0; i < SW_NACC; ++i) { mbar_init(&sm.acc_full[i], 1); mbar_init(&sm.acc_empty[i], sw_epi_warps(MODE)); }
-    for (int i = 0; i < SW_NMERGE; ++i) mbar_init(&sm.merge[i], 4);  // the four warps of max/avg group 1
+    for (int s = 0; s < SW_MAX_STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
+    for (int i = 0; i < SW_NACC; ++i) { mbar_init(&sm.acc_full[i], 1); mbar_init(&sm.acc_empty[i], SW_EPI_WARPS); }
+    for (int i = 0; i < SW_NMERGE; ++i) { mbar_init(&sm.merge[0][i], 4); mbar_init(&sm.merge[1][i], 4); }  // four warps of a group
     wait_ctl_init(&sm.ctl, a.wait_limit_ns);
     fence_barrier_init();
     prefetch_tensormap(&tm_f1);
@@ -594,72 +686,110 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
 
-  if (warp == 0) {
-    if (lane == 0) sweep_producer(sm, a, sc, &tm_f1, &tm_f2, &tm_aux);
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) sweep_mma(sm, a, sc);
-    __syncwarp();
-  } else {
-    EpiCtx e;
-    const int q = warp & 3;  // tcgen05.ld lets a warp read TMEM lanes 32*(warp%4) .. +31 only
-    e.wg = (warp - 2) >> 2;
-    e.lane = lane;
-    e.p = sc.m0 + q * 32 + lane;
-    e.valid = e.p < a.n_valid;
-    e.tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
-    if (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT>(sm, a, sc, e);
-    else if (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT>(sm, a, sc, e);
-    else if (MODE == SWEEP_COMPRESS) epilogue_compress<CUT>(sm, a, sc, e);
-    else epilogue_dump(sm, a, sc, e);
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (wait_ctl_aborted(&sm.ctl)) {
-    // A wait ran out.  Give copies that are still in flight time to land before the CTA's shared
-    // memory is released (TMA latency is a few microseconds), then free TMEM as usual.
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  // Every role is through: its copies have landed (or, where a wait ran out, get time to; TMA latency is a few microseconds)
+  // before the CTA's shared memory is released.
+  auto meet = [&] {
+    tc_fence_before();
     __syncthreads();
-  }
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(sm.tmem_base, SW_TMEM_COLS);
-  }
-  if constexpr (CUT) {
-    const SweepSched tail_sc = [&] {
-      if constexpr (MODE == SWEEP_COMPRESS) {
-        // worked out again: kept over the compression epilogue, its registers would be spilled there
-        int block;
-        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
-        return sweep_sched<MODE, CUT>(a, block);
-      } else {
-        return sc;
-      }
-    }();
-    if (tail_sc.tail >= 0 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
-      __threadfence();  // this thread's results before the count ...
+    if (wait_ctl_aborted(&sm.ctl)) {
+      for (int i = 0; i < 64; ++i) __nanosleep(1000);
       __syncthreads();
-      if (threadIdx.x == 0) sm.last_piece = atomicAdd(a.tail_count + tail_sc.tail, 1) == a.pieces - 1;
-      __syncthreads();
-      if (sm.last_piece) {
-        __threadfence();  // ... and the count before the other pieces' results
-        sweep_fold_pieces<MODE>(a, tail_sc);
-        if (threadIdx.x == 0) a.tail_count[tail_sc.tail] = 0;  // as the next launch expects it
+    }
+  };
+  // The two kinds of warps do not meet in common code again: what follows here is compiled for SW_REGS_ISSUE registers, what
+  // follows there for SW_REGS_EPI.
+  if (warp < 4) {
+    set_max_registers<SW_REGS_ISSUE, false>();
+    const SweepSched sc = sweep_sched<MODE, CUT>(a, blockIdx.x);
+    if (warp == 0) {
+      if (lane == 0) sweep_producer(sm, a, sc, &tm_f1, &tm_f2, &tm_aux);
+    } else if (warp == 1) {
+      if (lane == 0) sweep_mma(sm, a, sc);
+    }
+    __syncwarp();
+    meet();
+    if (warp == 1) {
+      tc_fence_after();
+      tmem_dealloc(sm.tmem_base, SW_TMEM_COLS);
+    }
+    return;
+  }
+  set_max_registers<SW_REGS_EPI, true>();
+  const SweepSched sc = sweep_sched<MODE, CUT>(a, blockIdx.x);
+  EpiCtx e;
+  const int q = warp & 3;  // tcgen05.ld lets a warp read TMEM lanes 32*(warp%4) .. +31 only
+  e.wg = (warp >> 2) - 1;
+  e.lane = lane;
+  e.p = sc.m0 + q * 32 + lane;
+  e.valid = e.p < a.n_valid;
+  e.tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+  e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
+  if constexpr (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT>(sm, a, sc, e);
+  else if constexpr (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT>(sm, a, sc, e);
+  else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC == 1 ? 1 : 2, KC <= 2, CUT>(sm, a, sc, e);
+  else epilogue_dump(sm, a, sc, e);
+  __syncwarp();
+  meet();
+}
+
+// The parts of the cut tiles folded into their piece 0's row results, in order.  Maxima: a later piece has the higher columns,
+// so only a strictly larger value replaces (a NaN counts as -inf, as it does between the column blocks of a tile).  Sums:
+// block by block, the order in which a whole tile adds them, so that a sample's sums do not depend on the cut, which follows
+// the batch and the row range.  A kernel of its own, one thread per pixel and FOLD_ROWS rows: folded by the CTA that finished a
+// tile last, the 0.3 MB of a 55 x 128 tile with four channels took that one SM 16 us, most of it memory latency.
+constexpr int FOLD_ROWS = 4;
+template <int MODE>
+__global__ void __launch_bounds__(TILE_M) sweep_fold_kernel(const SweepArgs a) {
+  constexpr bool SUM = MODE == SWEEP_COMPRESS, ARG = MODE == SWEEP_MAXARGAVG;
+  if (*reinterpret_cast<volatile int*>(a.status) != 0) return;
+  const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M, H2 = a.d.H2;
+  const int tail = blockIdx.y, tile = a.whole_tiles + tail, b = tile / tiles_per_sample;
+  const int px = threadIdx.x, p = (tile - b * tiles_per_sample) * TILE_M + px;
+  if (p >= a.n_valid) return;
+  const PixView& out = SUM ? a.ou : a.pu;
+  const size_t slot = (size_t)H2 * TILE_M, step = slot * a.part_slots;
+  float *dst[FOLD_ROWS], *arg_dst[FOLD_ROWS], v[FOLD_ROWS], va[FOLD_ROWS];
+  const float* src[FOLD_ROWS];
+  bool in[FOLD_ROWS];
+#pragma unroll
+  for (int r = 0; r < FOLD_ROWS; ++r) {
+    const int q = blockIdx.x * FOLD_ROWS + r, k = q / H2, u = q - k * H2;   // slot (channel of the launch) and row
+    in[r] = k < (SUM ? a.kc : 1);
+    dst[r] = out.base + b * out.sb + p + (SUM ? (a.k0 + k) * out.ss : 0u) + u * out.sd;
+    arg_dst[r] = ARG ? a.pu_arg.base + b * a.pu_arg.sb + p + u * a.pu_arg.sd : nullptr;
+    src[r] = sweep_part(a, tail, 0, k) + (size_t)u * TILE_M + px;
+    v[r] = in[r] ? *dst[r] : 0.f;
+    va[r] = ARG && in[r] ? *arg_dst[r] : 0.f;
+  }
+#pragma unroll 4
+  for (int part = 0; part < a.parts; ++part) {
+#pragma unroll
+    for (int r = 0; r < FOLD_ROWS; ++r) {
+      if (!in[r]) continue;
+      const float o = src[r][part * step];
+      if (SUM) {
+        v[r] += o;
+      } else if (o > fmaxf(v[r], -CUDART_INF_F)) {
+        v[r] = o;
+        if (ARG) va[r] = src[r][part * step + slot];
       }
     }
   }
+#pragma unroll
+  for (int r = 0; r < FOLD_ROWS; ++r) {
+    if (!in[r]) continue;
+    *dst[r] = v[r];
+    if (ARG) *arg_dst[r] = va[r];
+  }
 }
 
-// How the tail tiles are cut, in units of one 256-column tile's time: a CTA costs about two tiles of prologue, a fold
-// reads (parts + 1) * slots * H2 rows of 128 values through one SM (about 677 rows per tile time).  Pieces must save a quarter
-// of the tail and a whole tile to be used: a wave with idle SMs runs its tiles faster than a full one, so little is left of
-// smaller predicted savings (106 tail tiles of 135 x 240 in four pieces, predicted 0.86: max/avg sweep 588 -> 551 us, but
-// the compression sweep no faster).  Whole and cut tiles measured (us per launch, C = 256, FP16, max/avg and compression):
-// 1 x 48 x 64: 65 and 44, 40 and 25; 1 x 55 x 128: 122 and 81, 113 and 83; 4 x 55 x 128: 240 and 199, 231 and 218;
-// 3 x 47 x 155: 246 and 171, 199 and 158; 8 x 47 x 156: 486 and 414, 349 and 339; 1 x 55 x 128 against 27 x 64: 54 and 46,
-// 37 and 31.  Adding the sums block by block costs a compression sweep 1 to 7 us against one sum per piece.
+// How the tail tiles are cut, in units of one 256-column tile's time: a CTA costs about two tiles of prologue.  Pieces must save
+// a quarter of the tail and a whole tile to be used: a wave with idle SMs runs its tiles faster than a full one, and the fold
+// is a launch of 4 to 10 us.
+// Whole and cut tiles measured (us per call with the fold, C = 256, FP16, max/arg-max/avg and compression; Kc = 4 but for two
+// channels at 8 x 47 x 156 and three at 3 x 47 x 155): 1 x 48 x 64: 37 and 27, 33 and 26; 1 x 55 x 128: 76 and 50, 72 and 53;
+// 4 x 55 x 128: 158 and 134, 155 and 145; 3 x 47 x 155: 179 and 130, 164 and 116; 8 x 47 x 156: 355 and 302, 277 and 244;
+// 1 x 55 x 128 against 27 x 64: 30 and 25, 25 and 21; 3 x 20 x 27 against 18 x 50: 25 and 19, 19 and 14.
 TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   const long long tiles = (long long)d.B * ((d.N1() + TILE_M - 1) / TILE_M);
   const int n_ub = (d.H2 + SWEEP_UT - 1) / SWEEP_UT, n_vb = (d.W2 + SWEEP_VT - 1) / SWEEP_VT;
@@ -670,7 +800,7 @@ TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   for (int n = 1; n <= n_vb && n <= MAX_PIECES; ++n) {
     const double waves = (rest * n + SM_COUNT - 1) / SM_COUNT;
     const int parts = sums ? n_vb - piece_start(n_vb, n, 1) : n - 1;
-    const double cost = waves * ((n_vb + n - 1) / n * n_ub + 2) + (n > 1 ? (parts + 1) * (double)slots * d.H2 / 677.0 + 0.5 : 0.0);
+    const double cost = waves * ((n_vb + n - 1) / n * n_ub + 2) + (n > 1 ? 0.5 : 0.0);
     if (n == 1) best = whole = cost;
     if (cost < best && cost < 0.75 * whole && cost < whole - 1) { best = cost; r.pieces = n; r.parts = parts; }
   }
@@ -681,10 +811,10 @@ TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   return r;
 }
 
-template <int MODE, bool CUT>
+template <int MODE, bool CUT, int KC>
 static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                               const CUtensorMap& tm_aux, cudaStream_t stream) {
-  auto kern = sweep_kernel<MODE, CUT>;
+  auto kern = sweep_kernel<MODE, CUT, KC>;
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM_BYTES);
@@ -693,26 +823,35 @@ static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, cons
   const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
   const int tiles = a.d.B * tiles_per_sample;
   const dim3 grid(a.whole_tiles + (tiles - a.whole_tiles) * a.pieces);
-  kern<<<grid, sw_threads(MODE), SW_SMEM_BYTES, stream>>>(tm_f1, tm_f2, tm_aux, a);
+  kern<<<grid, SW_THREADS, SW_SMEM_BYTES, stream>>>(tm_f1, tm_f2, tm_aux, a);
+  if constexpr (CUT) {
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    const int rows = (MODE == SWEEP_COMPRESS ? a.kc : 1) * a.d.H2;
+    sweep_fold_kernel<MODE><<<dim3((rows + FOLD_ROWS - 1) / FOLD_ROWS, tiles - a.whole_tiles), TILE_M, 0, stream>>>(a);
+  }
   return cudaGetLastError();
 }
 
-template <int MODE>
+template <int MODE, int KC>
 static cudaError_t launch_mode(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                                const CUtensorMap& tm_aux, cudaStream_t stream) {
-  return a.pieces > 1 ? launch_one<MODE, true>(a, tm_f1, tm_f2, tm_aux, stream)
-                      : launch_one<MODE, false>(a, tm_f1, tm_f2, tm_aux, stream);
+  return a.pieces > 1 ? launch_one<MODE, true, KC>(a, tm_f1, tm_f2, tm_aux, stream)
+                      : launch_one<MODE, false, KC>(a, tm_f1, tm_f2, tm_aux, stream);
 }
 
 cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                          const CUtensorMap& tm_aux, cudaStream_t stream) {
   switch (a.mode) {
-    case SWEEP_MAXAVG: return launch_mode<SWEEP_MAXAVG>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_MAXARGAVG: return launch_mode<SWEEP_MAXARGAVG>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_DUMP: return launch_one<SWEEP_DUMP, false>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_MAXAVG: return launch_mode<SWEEP_MAXAVG, 0>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_MAXARGAVG: return launch_mode<SWEEP_MAXARGAVG, 0>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_DUMP: return launch_one<SWEEP_DUMP, false, 0>(a, tm_f1, tm_f2, tm_aux, stream);
     case SWEEP_COMPRESS:
-      if (a.kc < 1 || a.kc > KC_MAX_PER_SWEEP) return cudaErrorInvalidValue;
-      return launch_mode<SWEEP_COMPRESS>(a, tm_f1, tm_f2, tm_aux, stream);
+      switch (a.kc) {
+        case 1: return launch_mode<SWEEP_COMPRESS, 1>(a, tm_f1, tm_f2, tm_aux, stream);
+        case 2: return launch_mode<SWEEP_COMPRESS, 2>(a, tm_f1, tm_f2, tm_aux, stream);
+        case 3: case 4: return launch_mode<SWEEP_COMPRESS, 4>(a, tm_f1, tm_f2, tm_aux, stream);
+        default: return cudaErrorInvalidValue;
+      }
     default: return cudaErrorInvalidValue;
   }
 }

@@ -1,0 +1,73 @@
+"""The correlation sweeps at the edges of their 8 x 32 tiles, of the two warpgroups that share one and of the column blocks, and
+with every number of channels a sweep takes.  Features are small whole numbers and weights multiples of 1/8, so every product
+and sum is exact in FP32 whatever its order: results are compared bit for bit, ties included (the lowest index wins)."""
+import pytest
+import torch
+
+from separableflowthesis_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+# (B, H1, W1, H2, W2, Kc)
+SHAPES = [(1, 3, 43, h2, w2, kc) for kc, (h2, w2) in enumerate([(4, 16), (5, 31), (8, 32), (9, 33)], 1)] + [
+    (2, 1, 128, 3, 17, 4),      # fewer rows than one warpgroup takes
+    (1, 8, 17, 12, 64, 1),      # rows of the second warpgroup only in the first tile
+    (1, 5, 26, 33, 97, 3),      # a channel without a neighbour, several blocks both ways
+    (1, 9, 31, 23, 48, 6),      # two sweeps, half a column block left over
+    (150, 1, 5, 9, 33, 2),      # more tiles than SMs
+]
+
+
+def features(shape, seed=3):
+    B, H1, W1, H2, W2, _ = shape
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randint(-2, 3, (B, H1, W1, 16), generator=g).float(), torch.randint(-2, 3, (B, H2, W2, 16), generator=g).float())
+
+
+def first_max(S, dim):
+    """Largest entries that are numbers and the lowest index of each."""
+    S = S.nan_to_num(nan=-float("inf"))
+    m = S.amax(dim)
+    n = S.shape[dim]
+    index = torch.arange(n).view([-1 if d == dim else 1 for d in range(S.dim())])
+    return m, torch.where(S == m.unsqueeze(dim), index, n).amin(dim)
+
+
+@pytest.mark.parametrize("operands", ["fp16", "tf32"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_exact(shape, operands, cuda_device):
+    F1, F2 = features(shape)
+    B, H1, W1, H2, W2, Kc = shape
+    g = torch.Generator().manual_seed(4)
+    A_u, A_v = (torch.randint(0, 8, (B, H1, W1, Kc, D), generator=g).float() / 8 for D in (W2, H2))
+    dev = [t.to(cuda_device) for t in (F1, F2, A_u, A_v)]
+    with ops.sweep_operands(operands):
+        MA_u, MA_v, AM_u, AM_v = [t.cpu() for t in ops.max_argmax_avg_forward(*dev[:2])]
+        M_u, M_v = [t.cpu() for t in ops.max_avg_forward(*dev[:2])]
+        C_u, C_v = [t.cpu() for t in ops.compression_forward(*dev)]
+    S = torch.einsum("bijc,buvc->bijuv", F1, F2)
+    for dim, value, plain, arg in ((4, MA_u, M_u, AM_u), (3, MA_v, M_v, AM_v)):
+        m, index = first_max(S, dim)
+        assert torch.equal(value[..., 0, :], m) and torch.equal(plain[..., 0, :], m)
+        assert torch.equal(arg[..., 0, :].long(), index)
+    assert torch.equal(C_u, torch.einsum("bijuv,bijkv->bijku", S, A_u))
+    assert torch.equal(C_v, torch.einsum("bijuv,bijku->bijkv", S, A_v))
+
+
+@pytest.mark.parametrize("shape", [SHAPES[3], SHAPES[6]])
+def test_entries_that_are_not_numbers_are_passed_over(shape, cuda_device):
+    """Also where they fill the rows of a column block; a pixel with no number has the maxima NaN over rows and -inf over
+    columns, both at index 0."""
+    F1, F2 = features(shape)
+    F2[0, 0, :32] = float("nan")
+    F2[0, 1, 3] = F2[0, 4, 0] = F2[0, -1, -1] = float("nan")
+    with ops.sweep_operands("tf32"):
+        F1[0, 0, 1] = float("nan")
+        MA_u, MA_v, AM_u, AM_v = [t.cpu() for t in ops.max_argmax_avg_forward(F1.to(cuda_device), F2.to(cuda_device))]
+    S = torch.einsum("bijc,buvc->bijuv", F1, F2)
+    for dim, value, arg, none in ((4, MA_u, AM_u, float("nan")), (3, MA_v, AM_v, -float("inf"))):
+        m, index = first_max(S, dim)
+        empty = S.isnan().all(dim)
+        m, index = torch.where(empty, none, m), torch.where(empty, 0, index)
+        assert torch.equal(value[..., 0, :].nan_to_num(nan=7e7), m.nan_to_num(nan=7e7))
+        assert torch.equal(arg[..., 0, :].long(), index)
