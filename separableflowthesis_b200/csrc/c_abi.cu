@@ -231,7 +231,7 @@ struct Workspace {
   float* gxu;  // interleaved gradient-GEMM operands, (B, H2, n1p, Rg)
   float* gxv;  // interleaved gradient-GEMM operands, (B, W2, n1p, Rg)
   float* F1t;  // channel-major copies of F1r / F2r for K-major B operands: (B, C, n1p) and, in column blocks of 16
-  float* F2t;  // with an even number of rows, (B, C, ceil(W2/16), h2p, 16)
+  float* F2t;  // with a multiple of GG_UT rows, (B, C, ceil(W2/16), h2p, 16)
   int h2p;     // H2 rounded up to a multiple of GG_UT
   float* ga_u;  // level backward: attention gradients (B, Kc, W2, N1) / (B, Kc, H2, N1) ...
   float* ga_v;
@@ -240,8 +240,7 @@ struct Workspace {
   float* at_partial;  // ... and the attention backward's per-block partial sums
   int n1p;
   size_t bytes;        // without the scratch of the tail pieces, which a caller's buffer may lack (the kernels then
-  int* tail_count;     // do whole tiles only)
-  float* part;
+  float* part;         // do whole tiles only)
   size_t part_bytes;
 };
 
@@ -322,7 +321,6 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
     w.at_partial = take(attention_partial_floats(AttentionDims{d.B, d.Kc, d.H2 > d.W2 ? d.H2 : d.W2, d.H1, d.W1}));
   }
   w.bytes = off;
-  w.tail_count = reinterpret_cast<int*>(p + WS_TAIL_OFFSET);
   size_t part = 0;
   if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS, false).part_floats);
   if (d.Kc > 0 && plan.sweeps) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
@@ -332,7 +330,7 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   return w;
 }
 
-int sweep_launches(const SweepArgs& a) { return a.pieces > 1 ? 2 : 1; }   // pieces are folded by a kernel of their own
+template <class Args> int contraction_launches(const Args& a) { return a.pieces > 1 ? 2 : 1; }   // pieces are folded by a kernel of their own
 
 // A sweep's cut into whole tiles and pieces, as far as the workspace has scratch for the pieces.
 void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
@@ -352,7 +350,6 @@ void set_grad_split(GradArgs& a, const Workspace& w) {
   a.whole_tiles = cut ? s.whole_tiles : s.tiles;
   a.pieces = cut ? s.pieces : 1;
   a.part = w.part;
-  a.tail_count = w.tail_count;
 }
 
 int check_shape(const sfb_shape* s, bool need_kc, Dims* d) {
@@ -538,7 +535,7 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   a.pv_arg = packed_view(w.ov, d.W2, MAXAVG_SLOTS, w.n1p, 2);
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
-  SFB_CUDA(timed(KID_SWEEP_MAXAVG, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
+  SFB_CUDA(timed(KID_SWEEP_MAXAVG, contraction_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   // packed (displacement, slot, pixel) -> the reference's (pixel, channel, displacement) tensors
   const int N1 = d.N1(), R = MAXAVG_SLOTS;
   SFB_CUDA(timed(KID_PACK, with_argmax ? 4 : 2, st, [&] {
@@ -573,7 +570,7 @@ int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm
     a.out_scale = out_scale;
     a.status = w.status;
     set_sweep_split(a, w, chunk_channels(d.Kc));
-    SFB_CUDA(timed(KID_SWEEP_COMPRESS, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_f2 /* unused */, st); }));
+    SFB_CUDA(timed(KID_SWEEP_COMPRESS, contraction_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_f2 /* unused */, st); }));
   }
   return SFB_OK;
 }
@@ -600,11 +597,11 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
   a.op16 = op16;
   const int Q = R4 / 4;
   const int kid = mode == GRAD_MAXAVG ? KID_GRAD_MAXAVG_IMG1 : (mode == GRAD_COMPRESS ? KID_GRAD_COMPRESS_IMG1 : KID_GRAD_FUSED_IMG1);
-  // K-major B operands: channel-major copies of the rounded features (image 2 in column blocks of 16 with an even
-  // number of rows, so that a 2 x 16 block of the image is 32 consecutive values).  Rows and columns of padding must
+  // K-major B operands: channel-major copies of the rounded features (image 2 in column blocks of 16 with a multiple of four
+  // rows, so that a 4 x 16 block of the image is 64 consecutive values).  Rows and columns of padding must
   // read as zero: they meet the G values of cells outside the image.
   const uint32_t crows = (uint32_t)((d.C + KBLK - 1) / KBLK * KBLK);  // channel rows of one feature block
-  // a row of 32 K-values is 128 bytes of FP32 or 64 bytes of a 16-bit type: the swizzle span follows
+  // image 1: a row of 32 K-values is 128 bytes of FP32 or 64 bytes of a 16-bit type: the swizzle span follows
   const CUtensorMapSwizzle fswz = op16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
   const size_t f2t_per_sample = (size_t)d.C * ((d.W2 + GG_VT - 1) / GG_VT) * w.h2p * GG_VT;
   if (!accumulate) {  // later passes over further channel chunks reuse the copies of the first
@@ -618,11 +615,11 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
       return launch_channel_major(op16 ? feat.F2 : w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
     }));
   }
-  // gF1 = G * F2 : rows are image-1 pixels, the K sweep streams 2 x 16 blocks of F2 and 2-row blocks of XU.
-  {  // (blocked pixels, C, B); box = 32 consecutive values (2 rows x 16 columns) x all channels
+  // gF1 = G * F2 : rows are image-1 pixels, the K sweep streams 4 x 16 blocks of F2 and 4-row blocks of XU.
+  {  // (blocked pixels, C, B); box = 128 bytes of consecutive values (4 rows x 16 columns of a 16-bit type) x all channels
     const uint64_t dims[3] = {(uint64_t)(f2t_per_sample / d.C), (uint64_t)d.C, (uint64_t)d.B};
-    const uint32_t box[3] = {GG_KJ, crows, 1};
-    SFB_TRY(make_map(&tm_y, w.F2t, 3, dims, box, fswz, op16 != 0));
+    const uint32_t box[3] = {op16 ? 64u : 32u, crows, 1};
+    SFB_TRY(make_map(&tm_y, w.F2t, 3, dims, box, CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0));
   }
   SFB_TRY(map_operands(&tm_xu, w.gxu, d.B, d.H2, Q, w.n1p, TILE_M / 2, GG_UT));  // two 64-pixel boxes per block
   a.out_cf = out_cf;
@@ -631,7 +628,7 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
   a.out_scale = scale1;
   a.dev_scale = op16 == OP16_FP16 ? w.scales + SCALE_INV_GF1 : nullptr;
   set_grad_split(a, w);
-  SFB_CUDA(timed(kid, 1, st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xu /* unused */, st); }));
+  SFB_CUDA(timed(kid, contraction_launches(a), st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xu /* unused */, st); }));
   // gF2 = G^T * F1 : rows are an 8 x 16 block of image-2 pixels, the K sweep streams 32 pixels of F1, XU and XV.
   {  // (N1, C, B) with rows padded to n1p; box = 32 pixels x all channels
     const uint64_t dims[3] = {(uint64_t)d.N1(), (uint64_t)d.C, (uint64_t)d.B};
@@ -645,7 +642,7 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
   a.out_scale = 1.f;
   a.dev_scale = op16 == OP16_FP16 ? w.scales + SCALE_INV_GF2 : nullptr;
   set_grad_split(a, w);
-  SFB_CUDA(timed(kid + 1, 1, st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xv, st); }));
+  SFB_CUDA(timed(kid + 1, contraction_launches(a), st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xv, st); }));
   return SFB_OK;
 }
 
@@ -1045,7 +1042,7 @@ int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v
   a.pv_arg = cf_view(AM_v, 1, d.W2, N1);
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
-  SFB_CUDA(timed(KID_SWEEP_MAXAVG, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
+  SFB_CUDA(timed(KID_SWEEP_MAXAVG, contraction_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   return SFB_OK;
 }
 
@@ -1258,7 +1255,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   a.out_scale = sweep_out_scale(w, op16);
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
-  SFB_CUDA(timed(KID_SWEEP_MAXAVG, sweep_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
+  SFB_CUDA(timed(KID_SWEEP_MAXAVG, contraction_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
   const AttentionDims at_u{d.B, K, d.W2, d.H1, d.W1}, at_v{d.B, K, d.H2, d.H1, d.W1};
   const float *const X_u = SEP_u + (size_t)c0 * d.W2 * N1, *const X_v = SEP_v + (size_t)c0 * d.H2 * N1;

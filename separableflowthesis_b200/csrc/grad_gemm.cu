@@ -6,16 +6,16 @@
 // (MemorySaver_kernel_max_avg_argmax_backward.cu:305-310, MemorySaver_kernel_compression_backward.cu:477-488).
 //
 //   image2_major = 0 : rows = 128 consecutive image-1 pixels, K = image-2 pixels in blocks of
-//                      2 rows x 16 columns (column blocks outermost), output gF1.  A generator thread owns one
+//                      4 rows x 16 columns (column blocks outermost), output gF1.  A generator thread owns one
 //                      row = one TMEM lane, so the generated blocks go to tensor memory (tcgen05.st) next to the
 //                      accumulator and the tensor core reads A from TMEM: no shared-memory stores, fences or
 //                      operand reads for A.
 //   image2_major = 1 : rows = an 8 x 16 block of image-2 pixels, K = 32 consecutive image-1 pixels,
 //                      output gF2.  A generator thread owns one K column (pixel), so the blocks are written to
-//                      shared memory in the swizzled K-major layout.
-// B operand, both forms: K-major, like the operands of the correlation sweeps: one TMA box of 32*ceil(C/32) channel
-// rows x 32 K-values from channel-major copies of the rounded features (image 1: (C, pixels); image 2: (C, column
-// blocks of 16, rows, 16), so that the 2 rows x 16 columns of a K block are 32 consecutive values).  The MN-major
+//                      shared memory, swizzled, K-major (TF32) or MN-major (16-bit).
+// B operand, both forms: K-major, like the operands of the correlation sweeps: TMA boxes of 32*ceil(C/32) channel
+// rows x the K-values of a block from channel-major copies of the rounded features (image 1: (C, pixels); image 2: (C, column
+// blocks of 16, rows, 16), so that the 4 rows x 16 columns of a K block are 64 consecutive values).  The MN-major
 // form (pixel-major features) issues about 1.4x slower per tcgen05.mma and was dropped.
 // G for the max/avg op (MemorySaver_kernel_max_avg_argmax_backward.cu:200-251):
 //   G[p,u,v] = gMax_u[p,u]*[v==AM_u[p,u]] + gAvg_u[p,u]/W2 + gMax_v[p,v]*[u==AM_v[p,v]] + gAvg_v[p,v]/H2
@@ -26,13 +26,13 @@
 // copied into shared memory by TMA a few steps ahead, so the generator's reads have shared-memory latency.
 //
 // 16-bit form (GradArgs::op16 = BF16 or FP16): the same kernels with tcgen05.mma kind::f16.  G is rounded to the 16-bit
-// type as it is generated (two values per 32-bit TMEM column / 64-byte shared-memory rows) and the feature copies are
-// 16-bit (64-byte rows, 64-byte swizzle), so a block is two instructions of K = 16 instead of four of K = 8.
+// type as it is generated (two values per 32-bit TMEM column) and the feature copies are 16-bit, so 32 K-values are two
+// instructions of K = 16 instead of four of K = 8.
 // Accumulation stays FP32.  With FP16 the operands carry power-of-two scales (kernels.h, SCALE_*) that the drain undoes.
 //
 // Tail tiles: like the correlation sweeps, the tiles past the last full wave of 148 CTAs are cut into `pieces` CTAs, each
-// a range of the K sweep.  Piece 0 drains to the output, the others to scratch, and the CTA that finishes a tile last
-// (a counter per tile, nobody waits) adds them to the output in piece order: deterministic.
+// a range of the K sweep.  Piece 0 drains to the output, the others to scratch, and grad_fold_kernel adds them to the output
+// in piece order: deterministic.
 //
 // Warp roles: warp 0 feature (B operand) producer, warp 1 TMEM allocation + MMA issue, warps 2..9 generate G
 // and, at the end, drain the accumulator (two warps per TMEM lane quarter, alternating 16-column chunks),
@@ -47,22 +47,25 @@ namespace sfb {
 constexpr int GG_GEN_WARPS = 8;
 constexpr int GG_THREADS = (3 + GG_GEN_WARPS) * 32;
 constexpr int GG_VH = GG_VT / (GG_GEN_WARPS / 4);          // columns of one image-1-major generator thread
-constexpr uint32_t GG_YBLOCK_BYTES = GG_KJ * KBLK * 4;     // 4 KB: 32 channel rows x 32 K-values
+constexpr uint32_t GG_YBLOCK_BYTES = KBLK * 128;           // 4 KB: 128 bytes of K-values of 32 channel rows
+constexpr uint32_t GG_A_MBLOCK = GG_KJ * 128;              // image-2-major 16-bit A block: 64 rows x 32 K-values
+constexpr int GG_KJ1 = GG_UT * GG_VT;                      // K extent of one image-1-major block
+static_assert(GG_KJ1 == 64, "one 128-byte row of 16-bit values, two of FP32");
 constexpr uint32_t GG_ACC_COLS = 256;                      // accumulator columns (the feature dimension)
 
 // Ring depths.  Every kind of block has its own ring, sized by how long a stage stays in use:
 //   NY   feature blocks (B operand, 32 KB at C = 256): freed when the MMAs of the block have completed
 //   NG   generated blocks (A operand): image-1-major in TMEM columns 256 + 32*stage .., image-2-major in shared memory
-//   NXU  (pixel, u) operand blocks: read row by row while the block is computed, freed after the computation
+//   NXU  (pixel, u) operand blocks: read row by row while the block is computed, freed when its values are stored
 //   NXV  (pixel, v) operand blocks (image-2-major only; the image-1-major form keeps those slots in registers): read
 //        into registers at the start of a block and freed at once, so that the next load has the whole computation
 //        of the block to arrive
 // The image-2-major form's two generator groups hold two operand blocks at a time and a TMA load takes about as long
 // as one block's computation: with fewer than four (pixel, u) stages the generators wait for their operands.
 template <int Q, int I2MAJOR> struct GradCfg;
-template <> struct GradCfg<1, 0> { static constexpr int NY = 6, NG = 6, NXU = 4, NXV = 1; };
-template <> struct GradCfg<2, 0> { static constexpr int NY = 5, NG = 5, NXU = 4, NXV = 1; };
-template <> struct GradCfg<3, 0> { static constexpr int NY = 5, NG = 5, NXU = 4, NXV = 1; };
+template <> struct GradCfg<1, 0> { static constexpr int NY = 6, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<2, 0> { static constexpr int NY = 5, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<3, 0> { static constexpr int NY = 4, NG = 4, NXU = 4, NXV = 1; };
 template <> struct GradCfg<1, 1> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
 template <> struct GradCfg<2, 1> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
 template <> struct GradCfg<3, 1> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
@@ -72,11 +75,11 @@ template <int Q, int I2MAJOR>
 struct GradSmem {
   using Cfg = GradCfg<Q, I2MAJOR>;
   static constexpr int AT = I2MAJOR ? 0 : 1;   // A blocks in tensor memory
-  static_assert(GG_ACC_COLS + (AT ? Cfg::NG * GG_KJ : 0) <= gg_tmem_cols<I2MAJOR>(), "A stages exceed TMEM");
-  // one operand block: [displacement][group of 4 slots][pixel][4]; image-1-major 2 x Q x 128, image-2-major 8 x Q x 32
+  static_assert(GG_ACC_COLS + (AT ? Cfg::NG * GG_KJ1 : 0) <= gg_tmem_cols<I2MAJOR>(), "A stages exceed TMEM");
+  // one operand block: [displacement][group of 4 slots][pixel][4]; image-1-major 4 x Q x 128, image-2-major 8 x Q x 32
   static constexpr int XU_FLOATS = (I2MAJOR ? GG_ROW_UT * GG_KJ : GG_UT * TILE_M) * Q * 4;
   static constexpr int XV_FLOATS = I2MAJOR ? GG_ROW_VT * GG_KJ * Q * 4 : 4;  // image-1-major keeps XV in registers
-  float y[Cfg::NY][MAX_KB * KBLK * GG_KJ];    // feature blocks [channel][32 K-values], K-major, 128B swizzle
+  float y[Cfg::NY][MAX_KB * GG_YBLOCK_BYTES / 4];  // feature stages [channel][K-values], K-major, swizzled
   float g[AT ? 1 : Cfg::NG][AT ? 32 : TILE_M * GG_KJ];  // generated A blocks (image-2-major form), K-major, 128B swizzle
   float xu[Cfg::NXU][XU_FLOATS];
   float xv[Cfg::NXV][XV_FLOATS];
@@ -90,7 +93,6 @@ struct GradSmem {
   uint64_t xv_empty[Cfg::NXV];
   uint64_t acc_full;
   uint32_t tmem_base;
-  int last_piece;                             // this CTA finished its tail tile last: it adds the pieces up
   WaitCtl ctl;
 };
 
@@ -100,31 +102,29 @@ struct GradSched {
   int tail, piece;   // tail tile this CTA has a piece of (-1: a whole tile) and which piece
   int m0;            // image-1-major: first pixel of the row tile
   int u0, v0;        // image-2-major: origin of the 8 x 16 row tile
-  int n_ub2;         // image-1-major: number of 2-row blocks along u
-  int h2p;           // image-1-major: rows of the column-blocked channel-major copy of image 2 (H2 rounded up to even)
+  int n_ub2;         // image-1-major: number of 4-row blocks along u
+  int h2p;           // image-1-major: rows of the column-blocked channel-major copy of image 2 (H2 rounded up to a multiple of 4)
 };
 
-// The 4*Q slots of one (pixel, displacement) pair as 2*Q packed float pairs.
+// The 4*Q slots of one (pixel, displacement) pair.
 template <int Q>
 struct Slots {
-  uint64_t v[2 * Q];
-  // global memory: group q of this pixel is `group_stride` floats after group q-1
+  float f[4 * Q];
+  // global memory: group q of this pixel is `group_stride` floats after group q-1.  Loads of one float each: a 16-byte load
+  // would put the four slots of a column into neighbouring registers, and then a slot of all columns into the same register
+  // bank as their sums, which costs every other multiply-add a cycle (9.5 against 8.5 ms at 8 x 135 x 240).
   __device__ __forceinline__ void load_global(const float* p, size_t group_stride, bool ok) {
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      ulonglong2 t = make_ulonglong2(0ull, 0ull);
-      if (ok) t = __ldg(reinterpret_cast<const ulonglong2*>(p + q * group_stride));
-      v[2 * q] = t.x;
-      v[2 * q + 1] = t.y;
-    }
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f[4 * q + k] = ok ? __ldg(p + q * group_stride + k) : 0.f;
   }
   // shared memory block [group][pixel][4]
   __device__ __forceinline__ void load_shared(const float* p, int group_stride) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p + q * group_stride);
-      v[2 * q] = t.x;
-      v[2 * q + 1] = t.y;
+      const float4 t = *reinterpret_cast<const float4*>(p + q * group_stride);
+      f[4 * q] = t.x; f[4 * q + 1] = t.y; f[4 * q + 2] = t.z; f[4 * q + 3] = t.w;
     }
   }
 };
@@ -143,22 +143,38 @@ __device__ __forceinline__ void add_if_equal(float& x, int a, int b, float add) 
       : "r"(a), "r"(b), "f"(add));
 }
 
-__device__ __forceinline__ float pair_lo(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
-__device__ __forceinline__ int pair_hi_bits(uint64_t v) { return static_cast<int>(static_cast<uint32_t>(v >> 32)); }
-
-// The part of a G value that is a sum of products of the two pixels' slots, as one packed multiply-add chain.
+// The part of the G values of one (pixel, u) and N (pixel, v) that is a sum of products of the two pixels' slots.
 // Max/avg group (slots 0..3 of XU: mean-gradient/W2, 1, max-gradient, argmax; of XV: 1, mean-gradient/H2,
-// max-gradient, argmax): pair 0 multiplies to (mean-gradient_u, mean-gradient_v), whose two halves the final
-// horizontal add sums; pair 1 takes no part in the chain.  Compression groups: every pair is a product.
-template <int MODE, int Q>
-__device__ __forceinline__ float g_products(const Slots<Q>& xu, const Slots<Q>& xv) {
-  uint64_t acc = mul2(xu.v[0], xv.v[0]);
+// max-gradient, argmax): the two mean-gradients are added.  Compression groups: every slot is a product.
+// Scalar multiply-adds, a slot of the (pixel, u) at a time: it stays in the operand's register port while the N columns take
+// theirs, and such a multiply-add issues every cycle.  A packed one (fma.rn.f32x2) with three different operands takes three.
+template <int MODE, int Q, int N>
+__device__ __forceinline__ void g_products(const Slots<Q>& xu, const Slots<Q> (&xv)[N], float (&x)[N]) {
 #pragma unroll
-  for (int q = (MODE == GRAD_COMPRESS ? 1 : 2); q < 2 * Q; ++q) acc = fma2(xu.v[q], xv.v[q], acc);
-  return sum2(acc);
+  for (int i = 0; i < N; ++i) x[i] = MODE == GRAD_COMPRESS ? xu.f[0] * xv[i].f[0] : xu.f[0] + xv[i].f[1];
+#pragma unroll
+  for (int k = MODE == GRAD_COMPRESS ? 1 : 4; k < 4 * Q; ++k)
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = fmaf(xu.f[k], xv[i].f[k], x[i]);
 }
 
-// rows = image-1 pixels.  Thread (pl, vh): row pl of the tile, columns vh*8 .. vh*8+7 of every 2 x 16 block.
+// A word of every 16 bytes of slots.  A stage of operands is handed back for the next TMA load only after something has used
+// what was read from it: an arrive that merely follows the reads in program order was seen to let the next load's data (whole
+// 32-byte sectors of it) into the values, in blocks of four rows, where many reads are under way.
+template <int Q, int N>
+__device__ __forceinline__ uint32_t loaded(const Slots<Q> (&x)[N]) {
+  uint32_t all = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int q = 0; q < Q; ++q) all |= __float_as_uint(x[i].f[4 * q]);
+  return all;
+}
+
+// rows = image-1 pixels.  Thread (pl, vh): row pl of the tile, columns vh*8 .. vh*8+7 of every 4 x 16 block.
+// Bound: issue.  A value takes 8 multiply-adds, 3 additions, 2 compares and half a conversion at four channels; blocks of four
+// rows instead of two halve what the barriers and waits of a block cost beside them (353 instead of 430 instructions per 16
+// values with the scalar multiply-adds; 8 x 135 x 240: 8.4 -> 7.3 ms, 8 x 47 x 156: 436 -> 346 us).
 // The (pixel, v) slots stay in registers across the inner sweep over u; the (pixel, u) slots of each block
 // arrive in shared memory by TMA.  The finished values go to this thread's TMEM lane (A operand in tensor memory).
 template <int MODE, int Q, int BF16>
@@ -173,6 +189,7 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
   // (BF16: two values per column, so the thread's 8 values of a row are 4 columns)
   const uint32_t ta0 = sm.tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + GG_ACC_COLS +
                        vh * (BF16 ? GG_VH / 2 : GG_VH);
+  constexpr uint32_t A_COLS = BF16 ? GG_KJ1 / 2 : GG_KJ1;   // tensor-memory columns of one stage
   int vb = sc.t0 / sc.n_ub2, ub2 = sc.t0 - vb * sc.n_ub2;
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t so = t % Cfg::NXU, pho = (t / Cfg::NXU) & 1u;
@@ -183,7 +200,7 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
       for (int i = 0; i < GG_VH; ++i)
         xv[i].load_global(xv_p + (size_t)(vbase + i) * row_stride, group_stride, vbase + i < W2);
     }
-    if (!mbar_wait(&sm.xu_full[so], pho, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+    if (!mbar_wait_warp(&sm.xu_full[so], pho, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     float g[GG_UT][GG_VH];
 #pragma unroll
     for (int ul = 0; ul < GG_UT; ++ul) {
@@ -191,21 +208,20 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
       xu.load_shared(sm.xu[so] + ((((pl >> 6) * GG_UT + ul) * Q) * 64 + (pl & 63)) * 4, 64 * 4);
       const int u = ub2 * GG_UT + ul;
       // the arg-max column of (pixel, u) relative to this thread's first column: equals i for at most one i
-      const int cu = MODE != GRAD_COMPRESS ? pair_hi_bits(xu.v[1]) - vbase : -1;
-      const float gu_max = MODE != GRAD_COMPRESS ? pair_lo(xu.v[1]) : 0.f;
+      const int cu = MODE != GRAD_COMPRESS ? __float_as_int(xu.f[3]) - vbase : -1;
+      const float gu_max = MODE != GRAD_COMPRESS ? xu.f[2] : 0.f;
+      float x[GG_VH];
+      g_products<MODE, Q>(xu, xv, x);
 #pragma unroll
       for (int i = 0; i < GG_VH; ++i) {
-        float x = g_products<MODE, Q>(xu, xv[i]);
         if (MODE != GRAD_COMPRESS) {
-          add_if_equal(x, cu, i, gu_max);
-          add_if_equal(x, pair_hi_bits(xv[i].v[1]), u, pair_lo(xv[i].v[1]));
+          add_if_equal(x[i], cu, i, gu_max);
+          add_if_equal(x[i], __float_as_int(xv[i].f[3]), u, xv[i].f[2]);
         }
-        g[ul][i] = BF16 ? x : round_for_mma(x);
+        g[ul][i] = BF16 ? x[i] : round_for_mma(x[i]);
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.xu_empty[so]);  // operands are in registers
-    if (!mbar_wait(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+    if (!mbar_wait_warp(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     tc_fence_after();  // the MMAs that read this stage's TMEM columns have completed
     if constexpr (BF16) {
 #pragma unroll
@@ -214,16 +230,19 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
 #pragma unroll
         for (int j = 0; j < GG_VH / 2; ++j)
           h[j] = BF16 == OP16_FP16 ? pack_fp16x2(g[ul][2 * j], g[ul][2 * j + 1]) : pack_bf16x2(g[ul][2 * j], g[ul][2 * j + 1]);
-        tmem_st4(ta0 + s * GG_KJ + ul * (GG_VT / 2), h);
+        tmem_st4(ta0 + s * A_COLS + ul * (GG_VT / 2), h);
       }
     } else {
 #pragma unroll
-      for (int ul = 0; ul < GG_UT; ++ul) tmem_st8(ta0 + s * GG_KJ + ul * GG_VT, g[ul]);
+      for (int ul = 0; ul < GG_UT; ++ul) tmem_st8(ta0 + s * A_COLS + ul * GG_VT, g[ul]);
     }
     tmem_st_wait();
     tc_fence_before();  // stores complete and ordered before the tensor core's reads, which follow the arrive
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.g_full[s]);
+    if (lane == 0) {
+      mbar_arrive(&sm.g_full[s]);
+      mbar_arrive(&sm.xu_empty[so]);   // not before the values are stored: see loaded()
+    }
     if (++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
   }
 }
@@ -241,15 +260,19 @@ __device__ void generator_image2(GradSmem<Q, 1>& sm, const GradArgs& a, const Gr
   const int pl = (sub >> 1) * 16 + (lane & 15);          // K column of this thread
   const int vloc = ((sub & 1) * 2 + (lane >> 4)) * VQ;   // first of its four columns inside the row tile
   const int vbase = sc.v0 + vloc;
-  // element (row, K column) of the swizzled block: row = ul*16 + vloc + i, so row % 8 == (vloc + i) % 8.
-  // FP32: 128-byte rows, 16-byte chunk index ^ (row % 8).  BF16: 64-byte rows, chunk index ^ ((row % 8) / 2).
+  // Element (row m, K column) of the block, m = ul*16 + vloc + i.  FP32: K-major, 128-byte rows m, 16-byte chunk index ^ (m % 8)
+  // (m % 8 == (vloc + i) % 8).  16-bit: MN-major, two blocks of 64 m, 128-byte rows K, chunk index ^ (K % 8), so that the four
+  // columns of a row are one 8-byte store; as 2-byte stores of a K-major block (a thread has one K column) the stores alone
+  // took as many shared-memory cycles as the operands' loads (445 -> 403 us at 8 x 47 x 156; at 8 x 135 x 240, which runs against
+  // the power cap, 8.7 ms with either).
   uint32_t coff[VQ];
 #pragma unroll
   for (int i = 0; i < VQ; ++i) {
     const uint32_t r = (uint32_t)(vloc + i), k = (uint32_t)pl;
-    coff[i] = BF16 ? r * 64u + ((((k >> 3) ^ ((r & 7u) >> 1)) & 3u) << 4) + ((k & 7u) << 1)
-                   : r * 128u + (((k >> 2) ^ (r & 7u)) << 4) + ((k & 3u) << 2);
+    coff[i] = r * 128u + (((k >> 2) ^ (r & 7u)) << 4) + ((k & 3u) << 2);
   }
+  const uint32_t row16 = (uint32_t)pl * 128u + (((uint32_t)vloc & 7u) << 1), chunk16 = (uint32_t)vloc >> 3, flip16 = (uint32_t)pl & 7u;
+  const uint32_t zero = *reinterpret_cast<volatile uint32_t*>(&sm.ctl.reserved);   // 0, which the compiler does not know
   // No more groups than ring stages: a group two fills ahead of a stage would see the parity of the fill before
   // last and pass its wait early.
   static_assert(GG_GEN_WARPS / 4 <= Cfg::NXU && GG_GEN_WARPS / 4 <= Cfg::NXV && GG_GEN_WARPS / 4 <= Cfg::NG,
@@ -258,72 +281,83 @@ __device__ void generator_image2(GradSmem<Q, 1>& sm, const GradArgs& a, const Gr
     const uint32_t su = t % Cfg::NXU, phu = (t / Cfg::NXU) & 1u;
     const uint32_t sv = t % Cfg::NXV, phv = (t / Cfg::NXV) & 1u;
     const uint32_t s = t % Cfg::NG, ph = (t / Cfg::NG) & 1u;
-    if (!mbar_wait(&sm.xv_full[sv], phv, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+    if (!mbar_wait_warp(&sm.xv_full[sv], phv, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     Slots<Q> xv[VQ];  // block layouts [displacement][group][pixel][4]
     int du[VQ];       // arg-max row of (pixel, v) relative to the tile's first row: equals ul for at most one ul
 #pragma unroll
     for (int i = 0; i < VQ; ++i) {
       xv[i].load_shared(sm.xv[sv] + ((vloc + i) * Q * GG_KJ + pl) * 4, GG_KJ * 4);
-      du[i] = MODE != GRAD_COMPRESS ? pair_hi_bits(xv[i].v[1]) - sc.u0 : -1;
+      du[i] = MODE != GRAD_COMPRESS ? __float_as_int(xv[i].f[3]) - sc.u0 : -1;
     }
+    const uint32_t none = loaded(xv) & zero;
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.xv_empty[sv]);  // the (pixel, v) slots are in registers: the next load may start
-    if (!mbar_wait(&sm.xu_full[su], phu, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+    if (lane == 0) mbar_arrive(&sm.xv_empty[sv + none]);  // the (pixel, v) slots are in registers: the next load may start
+    if (!mbar_wait_warp(&sm.xu_full[su], phu, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     float g[GG_ROW_UT][VQ];
 #pragma unroll
     for (int ul = 0; ul < GG_ROW_UT; ++ul) {
       Slots<Q> xu;
       xu.load_shared(sm.xu[su] + (ul * Q * GG_KJ + pl) * 4, GG_KJ * 4);
-      const int cu = MODE != GRAD_COMPRESS ? pair_hi_bits(xu.v[1]) - vbase : -1;
-      const float gu_max = MODE != GRAD_COMPRESS ? pair_lo(xu.v[1]) : 0.f;
+      const int cu = MODE != GRAD_COMPRESS ? __float_as_int(xu.f[3]) - vbase : -1;
+      const float gu_max = MODE != GRAD_COMPRESS ? xu.f[2] : 0.f;
+      float x[VQ];
+      g_products<MODE, Q>(xu, xv, x);
 #pragma unroll
       for (int i = 0; i < VQ; ++i) {
-        float x = g_products<MODE, Q>(xu, xv[i]);
         if (MODE != GRAD_COMPRESS) {
-          add_if_equal(x, cu, i, gu_max);
-          add_if_equal(x, du[i], ul, pair_lo(xv[i].v[1]));
+          add_if_equal(x[i], cu, i, gu_max);
+          add_if_equal(x[i], du[i], ul, xv[i].f[2]);
         }
-        g[ul][i] = BF16 ? x : round_for_mma(x);
+        g[ul][i] = BF16 ? x[i] : round_for_mma(x[i]);
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.xu_empty[su]);
-    if (!mbar_wait(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+    if (!mbar_wait_warp(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     uint8_t* base = reinterpret_cast<uint8_t*>(sm.g[s]);
 #pragma unroll
-    for (int ul = 0; ul < GG_ROW_UT; ++ul)
+    for (int ul = 0; ul < GG_ROW_UT; ++ul) {
+      if constexpr (BF16) {
+        const uint2 h = BF16 == OP16_FP16 ? make_uint2(pack_fp16x2(g[ul][0], g[ul][1]), pack_fp16x2(g[ul][2], g[ul][3]))
+                                          : make_uint2(pack_bf16x2(g[ul][0], g[ul][1]), pack_bf16x2(g[ul][2], g[ul][3]));
+        *reinterpret_cast<uint2*>(base + (ul >> 2) * GG_A_MBLOCK + row16 + (((((uint32_t)ul & 3u) * 2 + chunk16) ^ flip16) << 4)) = h;
+      } else {
 #pragma unroll
-      for (int i = 0; i < VQ; ++i) {
-        if constexpr (BF16)
-          *reinterpret_cast<uint16_t*>(base + ul * (GG_ROW_VT * 64) + coff[i]) = to_op16(g[ul][i], BF16);
-        else
-          *reinterpret_cast<float*>(base + ul * (GG_ROW_VT * 128) + coff[i]) = g[ul][i];
+        for (int i = 0; i < VQ; ++i) *reinterpret_cast<float*>(base + ul * (GG_ROW_VT * 128) + coff[i]) = g[ul][i];
       }
+    }
     fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core's async-proxy reads
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.g_full[s]);
+    if (lane == 0) {
+      mbar_arrive(&sm.g_full[s]);
+      mbar_arrive(&sm.xu_empty[su]);
+    }
   }
 }
 
-// B operand: one box of 32*nkb channel rows x 32 K-values of the other image's channel-major feature copy per block.
-// Image 2 is stored in column blocks of 16 with an even number of rows, so block (vb, ub2) of the image-1-major form
-// (2 rows x 16 columns) is 32 consecutive values.
+// B operand, a ring of 32 KB stages: one box of 32*nkb channel rows of the other image's channel-major feature copy each.
+// Image-1-major: 128 bytes of a row, i.e. the 64 K-values of a block (16-bit) or half of them; image 2 is stored in column
+// blocks of 16 with a multiple of four rows, so block (vb, ub2) (4 rows x 16 columns) is 64 consecutive values.
+// Image-2-major: the 32 pixels of a block (64 bytes of 16-bit values).
+template <int I2MAJOR, int BF16> __device__ constexpr int y_stages_per_block() { return !I2MAJOR && !BF16 ? 2 : 1; }
 template <int Q, int I2MAJOR, int BF16>
 __device__ void feature_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc,
                                  const CUtensorMap* tm_y) {
   using Cfg = GradCfg<Q, I2MAJOR>;
+  constexpr int PER = y_stages_per_block<I2MAJOR, BF16>();
   int vb = 0, ub2 = 0;
   if (I2MAJOR == 0) { vb = sc.t0 / sc.n_ub2; ub2 = sc.t0 - vb * sc.n_ub2; }
+  uint32_t s = 0, ph = 0;
   for (int t = 0; t < sc.n_blocks; ++t) {
-    const uint32_t s = t % Cfg::NY, ph = (t / Cfg::NY) & 1u;
-    if (!mbar_wait(&sm.y_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
-    mbar_expect_tx(&sm.y_full[s], sc.nkb * (BF16 ? GG_YBLOCK_BYTES / 2 : GG_YBLOCK_BYTES));
-    if (I2MAJOR == 0) {
-      tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (vb * sc.h2p + ub2 * GG_UT) * GG_VT, 0, sc.b);
-      if (++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
-    } else {
-      tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (sc.t0 + t) * GG_KJ, 0, sc.b);
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+      if (!mbar_wait(&sm.y_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
+      mbar_expect_tx(&sm.y_full[s], sc.nkb * (I2MAJOR && BF16 ? GG_YBLOCK_BYTES / 2 : GG_YBLOCK_BYTES));
+      if (I2MAJOR == 0)
+        tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (vb * sc.h2p + ub2 * GG_UT) * GG_VT + h * KBLK, 0, sc.b);
+      else
+        tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (sc.t0 + t) * GG_KJ, 0, sc.b);
+      if (++s == Cfg::NY) { s = 0; ph ^= 1u; }
     }
+    if (I2MAJOR == 0 && ++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
   }
 }
 
@@ -356,38 +390,43 @@ __device__ void operand_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, co
 template <int Q, int I2MAJOR, int BF16>
 __device__ void grad_mma(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc) {
   using Cfg = GradCfg<Q, I2MAJOR>;
-  // A: generated block, K-major: TMEM columns 256 + 32*stage .. (image-1-major) or shared memory (image-2-major).
-  // B: feature block [channels][32 K-values], K-major, 8-row groups 1024 B apart.  K = 8 per instruction: 8 TMEM
-  // columns / 32 bytes along a row of A, 32 bytes along a row of B.
-  // BF16: 64-byte rows with the 64-byte swizzle (8-row groups 512 B apart), K = 16 per instruction: 8 TMEM columns
-  // of two values / 32 bytes along a row.
-  const uint32_t idesc = BF16 ? make_idesc_op16(BF16, TILE_M, sc.nkb * KBLK) : make_idesc_tf32(TILE_M, sc.nkb * KBLK, false, false);
-  constexpr int NK = BF16 ? GG_KJ / 16 : GG_KJ / 8;  // instructions per block
+  // A: generated block, K-major: TMEM columns from 256 on (image-1-major; a 16-bit column holds two values) or shared memory
+  // (image-2-major).  B: feature block [channels][K-values], K-major.  Rows of 128 bytes have the 128-byte swizzle (8-row
+  // groups 1024 B apart); the 64-byte rows of 16-bit image-2-major blocks the 64-byte swizzle (512 B apart).  An instruction
+  // takes K = 8 TF32 or 16 16-bit values: 8 TMEM columns / 32 bytes along a row of A, 32 bytes along a row of B.  The 16-bit
+  // image-2-major A block is MN-major (generator_image2): 8-K groups 1024 B apart, two of them to an instruction.
+  const uint32_t idesc = BF16 ? make_idesc_op16(BF16, TILE_M, sc.nkb * KBLK, I2MAJOR != 0) : make_idesc_tf32(TILE_M, sc.nkb * KBLK, false, false);
+  constexpr int PER = y_stages_per_block<I2MAJOR, BF16>();
+  constexpr int NK = I2MAJOR && BF16 ? 2 : 4;   // instructions per feature stage
+  constexpr uint32_t A_COLS = BF16 ? GG_KJ1 / 2 : GG_KJ1;
+  uint32_t sy = 0, phy = 0;
   for (int t = 0; t < sc.n_blocks; ++t) {
-    const uint32_t sy = t % Cfg::NY, phy = (t / Cfg::NY) & 1u;
     const uint32_t sg = t % Cfg::NG, phg = (t / Cfg::NG) & 1u;
-    if (!mbar_wait(&sm.y_full[sy], phy, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
-    if (!mbar_wait(&sm.g_full[sg], phg, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
-    tc_fence_after();
-    const uint64_t bdesc = BF16 ? make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 512, 4)
-                                : make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 1024);
-    if constexpr (I2MAJOR == 0) {
-      const uint32_t a_tmem = sm.tmem_base + GG_ACC_COLS + sg * GG_KJ;
 #pragma unroll
-      for (int k = 0; k < NK; ++k) {
-        if constexpr (BF16) umma_bf16_ts(sm.tmem_base, a_tmem + k * 8, desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
-        else umma_tf32_ts(sm.tmem_base, a_tmem + k * 8, desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
-      }
-    } else {
-      const uint64_t adesc = BF16 ? make_smem_desc_sw128(smem_u32(sm.g[sg]), 16, 512, 4)
-                                  : make_smem_desc_sw128(smem_u32(sm.g[sg]), 16, 1024);
+    for (int h = 0; h < PER; ++h) {
+      if (!mbar_wait(&sm.y_full[sy], phy, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
+      if (h == 0 && !mbar_wait(&sm.g_full[sg], phg, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
+      tc_fence_after();
+      const uint64_t bdesc = I2MAJOR && BF16 ? make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 512, 4)
+                                             : make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 1024);
+      if constexpr (I2MAJOR == 0) {
+        const uint32_t a_tmem = sm.tmem_base + GG_ACC_COLS + sg * A_COLS + h * 32;
 #pragma unroll
-      for (int k = 0; k < NK; ++k) {
-        if constexpr (BF16) umma_bf16(sm.tmem_base, desc_advance(adesc, k * 32), desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
-        else umma_tf32(sm.tmem_base, desc_advance(adesc, k * 32), desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
+        for (int k = 0; k < NK; ++k) {
+          if constexpr (BF16) umma_bf16_ts(sm.tmem_base, a_tmem + k * 8, desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
+          else umma_tf32_ts(sm.tmem_base, a_tmem + k * 8, desc_advance(bdesc, k * 32), idesc, (t | h | k) != 0);
+        }
+      } else {
+        const uint64_t adesc = make_smem_desc_sw128(smem_u32(sm.g[sg]), BF16 ? GG_A_MBLOCK : 16, 1024);
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+          if constexpr (BF16) umma_bf16(sm.tmem_base, desc_advance(adesc, k * 2048), desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
+          else umma_tf32(sm.tmem_base, desc_advance(adesc, k * 32), desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
+        }
       }
+      umma_commit(&sm.y_empty[sy]);  // reusable once these MMAs have read it
+      if (++sy == Cfg::NY) { sy = 0; phy ^= 1u; }
     }
-    umma_commit(&sm.y_empty[sy]);  // both stages are reusable once these MMAs have read them
     umma_commit(&sm.g_empty[sg]);
   }
   umma_commit(&sm.acc_full);
@@ -470,72 +509,58 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
   }
 }
 
-// Pieces 1.. of a finished tail tile added to the output, in piece order (all threads of the CTA that finished last).  One
-// SM's loads move all of it, so a thread takes sixteen values at once and asks for several pieces' values before it uses any.
-constexpr int FOLD_PIECES = 2;
-__device__ __forceinline__ void fold_add(const float* const (&part)[4], const bool (&in)[4], size_t step, int pieces, float4 (&sum)[4]) {
-  for (int s0 = 1; s0 < pieces; s0 += FOLD_PIECES) {
-    float4 o[FOLD_PIECES][4];
-#pragma unroll
-    for (int q = 0; q < FOLD_PIECES; ++q)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        o[q][j] = s0 + q < pieces && in[j] ? __ldcg(reinterpret_cast<const float4*>(part[j] + (s0 + q - 1) * step))
-                                           : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < FOLD_PIECES; ++q) {
-      if (s0 + q >= pieces) break;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) add4(sum[j], o[q][j]);
-    }
+// Sample and origin of a row tile; returns the blocks of its K sweep.
+template <int I2MAJOR>
+__device__ __forceinline__ int grad_tile(const GradArgs& a, int tile, GradSched& sc) {
+  sc.m0 = sc.u0 = sc.v0 = sc.n_ub2 = sc.h2p = 0;
+  if (I2MAJOR == 0) {
+    const int tiles = (a.d.N1() + TILE_M - 1) / TILE_M;
+    sc.b = tile / tiles;
+    sc.m0 = (tile - sc.b * tiles) * TILE_M;
+    sc.n_ub2 = (a.d.H2 + GG_UT - 1) / GG_UT;
+    sc.h2p = sc.n_ub2 * GG_UT;
+    return sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT);
   }
+  const int n_ub = (a.d.H2 + GG_ROW_UT - 1) / GG_ROW_UT, n_vb = (a.d.W2 + GG_ROW_VT - 1) / GG_ROW_VT;
+  sc.b = tile / (n_ub * n_vb);
+  const int r = tile - sc.b * (n_ub * n_vb);
+  sc.u0 = (r / n_vb) * GG_ROW_UT;
+  sc.v0 = (r % n_vb) * GG_ROW_VT;
+  return (a.d.N1() + GG_KJ - 1) / GG_KJ;
 }
 
+// Pieces 1.. of the cut tiles added to the output, in piece order, four values to a thread.  A kernel of its own: added up by
+// the CTA that finished a tile last, the 128 KB of every piece came through that one SM.
+constexpr int GG_FOLD_THREADS = 256;
 template <int I2MAJOR>
-__device__ void grad_fold_pieces(const GradArgs& a, const GradSched& sc) {
-  const int C = a.d.C;   // a multiple of 4
-  const float* const part0 = grad_part(a, sc.tail, 1);
-  const size_t step = (size_t)C * TILE_M;
-  float4 sum[4];
-  const float* part[4];
-  bool in[4];
+__global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const GradArgs a) {
+  if (*reinterpret_cast<volatile int*>(a.status) != 0) return;
+  const int C = a.d.C, tail = blockIdx.y;   // C is a multiple of 4
+  const int i = blockIdx.x * GG_FOLD_THREADS + threadIdx.x;   // four neighbours of the pieces' layout (grad_part)
+  if (i >= C * (TILE_M / 4)) return;
+  GradSched sc;
+  grad_tile<I2MAJOR>(a, a.whole_tiles + tail, sc);
   size_t cstride;
-  if (a.out_cf) {   // channel-major: four rows, neighbours in the image (the ones that exist come first), of four channels
-    constexpr int QUADS = TILE_M / 4;
-    for (int i = threadIdx.x; i < C / 4 * QUADS; i += GG_THREADS) {
-      const int m = i % QUADS * 4, c0 = i / QUADS * 4;
-      float* const row = grad_row<I2MAJOR>(a, sc, m, cstride);
-      if (row == nullptr) continue;
-      const int cnt = min(4, I2MAJOR ? a.d.W2 - (sc.v0 + m % GG_ROW_VT) : a.d.N1() - (sc.m0 + m));
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        sum[j] = load4_cg(row + (c0 + j) * cstride, cnt);
-        part[j] = part0 + (size_t)(c0 + j) * TILE_M + m;
-        in[j] = true;
-      }
-      fold_add(part, in, step, a.pieces, sum);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) store4(row + (c0 + j) * cstride, sum[j], cnt);
-    }
-  } else {          // pixel-major, as the pieces are: runs of four channels of a row, neighbouring runs to neighbouring threads
-    const int runs = C / 4, n = runs * TILE_M;
-    for (int i0 = threadIdx.x; i0 < n; i0 += 4 * GG_THREADS) {
-      float* row[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = i0 + j * GG_THREADS, m = i / runs;
-        row[j] = i < n ? grad_row<I2MAJOR>(a, sc, m, cstride) : nullptr;
-        in[j] = row[j] != nullptr;
-        if (in[j]) row[j] += (i - m * runs) * 4;
-        sum[j] = load4_cg(row[j], in[j] ? 4 : 0);
-        part[j] = part0 + (size_t)i * 4;
-      }
-      fold_add(part, in, step, a.pieces, sum);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (in[j]) store4(row[j], sum[j], 4);
-    }
+  float* dst;
+  int cnt = 4;
+  if (a.out_cf) {   // channel-major: four rows, neighbours in the image (the ones that exist come first), of one channel
+    const int c = i / (TILE_M / 4), m = i % (TILE_M / 4) * 4;
+    dst = grad_row<I2MAJOR>(a, sc, m, cstride);
+    if (dst == nullptr) return;
+    dst += c * cstride;
+    cnt = min(4, I2MAJOR ? a.d.W2 - (sc.v0 + m % GG_ROW_VT) : a.d.N1() - (sc.m0 + m));
+  } else {          // pixel-major: four channels of a row
+    const int m = i / (C / 4);
+    dst = grad_row<I2MAJOR>(a, sc, m, cstride);
+    if (dst == nullptr) return;
+    dst += (i - m * (C / 4)) * 4;
   }
+  const float* part = grad_part(a, tail, 1) + (size_t)i * 4;
+  const size_t step = (size_t)C * TILE_M;
+  float4 sum = load4_cg(dst, cnt);
+#pragma unroll 4
+  for (int piece = 1; piece < a.pieces; ++piece, part += step) add4(sum, *reinterpret_cast<const float4*>(part));
+  store4(dst, sum, cnt);
 }
 
 template <int MODE, int Q, int I2MAJOR, int BF16>
@@ -562,26 +587,7 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
     sc.piece = r - sc.tail * a.pieces;
     tile = a.whole_tiles + sc.tail;
   }
-  int all_blocks;
-  if (I2MAJOR == 0) {
-    const int tiles = (a.d.N1() + TILE_M - 1) / TILE_M;
-    sc.b = tile / tiles;
-    sc.m0 = (tile - sc.b * tiles) * TILE_M;
-    sc.u0 = sc.v0 = 0;
-    sc.n_ub2 = (a.d.H2 + GG_UT - 1) / GG_UT;
-    sc.h2p = sc.n_ub2 * GG_UT;
-    all_blocks = sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT);
-  } else {
-    const int n_ub = (a.d.H2 + GG_ROW_UT - 1) / GG_ROW_UT, n_vb = (a.d.W2 + GG_ROW_VT - 1) / GG_ROW_VT;
-    sc.b = tile / (n_ub * n_vb);
-    const int r = tile - sc.b * (n_ub * n_vb);
-    sc.u0 = (r / n_vb) * GG_ROW_UT;
-    sc.v0 = (r % n_vb) * GG_ROW_VT;
-    sc.m0 = 0;
-    sc.n_ub2 = 0;
-    sc.h2p = 0;
-    all_blocks = (a.d.N1() + GG_KJ - 1) / GG_KJ;
-  }
+  const int all_blocks = grad_tile<I2MAJOR>(a, tile, sc);
   const int n_pieces = sc.tail >= 0 ? a.pieces : 1;
   {
     const int per = all_blocks / n_pieces, extra = all_blocks - per * n_pieces;  // the first `extra` pieces have one more
@@ -636,17 +642,6 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
     tc_fence_after();
     tmem_dealloc(sm.tmem_base, gg_tmem_cols<I2MAJOR>());
   }
-  if (n_pieces > 1 && !wait_ctl_aborted(&sm.ctl)) {  // uniform over the CTA after the barrier above
-    __threadfence();  // this thread's results before the count ...
-    __syncthreads();
-    if (threadIdx.x == 0) sm.last_piece = atomicAdd(a.tail_count + sc.tail, 1) == n_pieces - 1;
-    __syncthreads();
-    if (sm.last_piece) {
-      __threadfence();  // ... and the count before the other pieces' results
-      grad_fold_pieces<I2MAJOR>(a, sc);
-      if (threadIdx.x == 0) a.tail_count[sc.tail] = 0;  // as the next launch expects it
-    }
-  }
 }
 
 static int grad_tiles(const Dims& d, int image2_major) {
@@ -654,24 +649,23 @@ static int grad_tiles(const Dims& d, int image2_major) {
                       : d.B * ((d.N1() + TILE_M - 1) / TILE_M);
 }
 
-// How the tail tiles are cut, in units of one K block's time (32 values, about 0.6 us): a CTA costs about eight blocks of
-// prologue and drain, a fold reads 128 KB per piece through one SM (about two blocks).  Pieces must save a quarter of the
-// tail (see sweep_split) and at least twelve blocks to be used: with predicted savings of seven and eleven, launches of 23
-// (2 x 33 x 70 against 16 x 35) and 33 us (3 x 55 x 128 against 13 x 32) got one or two us slower.  Whole and cut tiles
-// measured, image-1-major and image-2-major form (us per launch, C = 256, FP16): 1 x 48 x 64: 60 and
-// 37, 62 and 38; 1 x 55 x 128: 150 and 104, 148 and 107; 4 x 55 x 128: 300 and 246, 299 and 280; 8 x 47 x 156: 508 and
-// 438, 541 and 476; 1 x 55 x 128 against 27 x 64: 48 and 40, 147 and 49; 1 x 135 x 240 against 67 x 120: 350 whole, 634 and
-// 335.
+// How the tail tiles are cut, in units of the time of 32 K-values (about 0.6 us): a CTA costs about eight of prologue and drain,
+// the fold is a launch of 4 to 11 us.  Pieces must save a quarter of the tail (see sweep_split) and at least twelve units to be
+// used.  Whole and cut tiles measured, the fold with the latter, image-1-major and image-2-major form (us, C = 256, FP16):
+// 1 x 48 x 64: 46 and 25, 50 and 24; 1 x 55 x 128: 122 and 79, 133 and 81; 4 x 55 x 128: 255 and 209, 268 and 249;
+// 3 x 47 x 155: 266 and 177, 273 and 189; 8 x 47 x 156: 418 and 350, 472 and 407; 1 x 55 x 128 against 27 x 64: 40 and 33,
+// 125 and 30; 1 x 135 x 240 against 67 x 120: 303 whole, 565 and 308; 2 x 33 x 70 against 16 x 35: 20 whole, 40 and 18.
 TileSplit grad_split(const Dims& d, int image2_major) {
   const int tiles = grad_tiles(d, image2_major), rest = tiles % SM_COUNT;
   const int blocks = image2_major ? (d.N1() + GG_KJ - 1) / GG_KJ
                                   : ((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT);
+  const int unit = image2_major ? 1 : GG_KJ1 / GG_KJ;   // of a block
   TileSplit r{tiles, tiles, 1, 0, 0};
   if (rest == 0) return r;
   double best = 0, whole = 0;
   for (int n = 1; n <= blocks && n <= MAX_PIECES; ++n) {
     const double waves = (rest * n + SM_COUNT - 1) / SM_COUNT;
-    const double cost = waves * ((blocks + n - 1) / n + 8) + (n > 1 ? 2.0 * n * d.C / MAX_C + 2 : 0.0);
+    const double cost = waves * ((blocks + n - 1) / n * unit + 8) + (n > 1 ? 6.0 : 0.0);
     if (n == 1) best = whole = cost;
     if (cost < best && cost < 0.75 * whole && cost < whole - 12) { best = cost; r.pieces = n; }
   }
@@ -694,8 +688,13 @@ static cudaError_t launch_one(const GradArgs& a, const CUtensorMap& tm_y, const 
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
   });
   if (err != cudaSuccess) return err;
-  const int ctas = a.whole_tiles + (grad_tiles(a.d, I2MAJOR) - a.whole_tiles) * a.pieces;
-  kern<<<dim3(ctas), GG_THREADS, smem_bytes, stream>>>(tm_y, tm_xu, tm_xv, a);
+  const int tails = grad_tiles(a.d, I2MAJOR) - a.whole_tiles;
+  kern<<<dim3(a.whole_tiles + tails * a.pieces), GG_THREADS, smem_bytes, stream>>>(tm_y, tm_xu, tm_xv, a);
+  if (a.pieces > 1) {
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    const int items = a.d.C * (TILE_M / 4);
+    grad_fold_kernel<I2MAJOR><<<dim3((items + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS, tails), GG_FOLD_THREADS, 0, stream>>>(a);
+  }
   return cudaGetLastError();
 }
 

@@ -46,9 +46,9 @@ constexpr int SWEEP_UT = 8;   // image-2 rows per correlation tile (8 x 32 = 256
 constexpr int SWEEP_VT = 32;  // image-2 columns per correlation tile
 constexpr int GG_ROW_UT = 8;  // row tile of the image-2-major gradient GEMM: 8 x 16 image-2 pixels = 128 TMEM lanes
 constexpr int GG_ROW_VT = 16;
-constexpr int GG_UT = 2;      // image-2 rows per K-block of the gradient GEMM (image-1-major form)
+constexpr int GG_UT = 4;      // a K block of the image-1-major gradient GEMM: 4 image-2 rows x 16 columns
 constexpr int GG_VT = 16;
-constexpr int GG_KJ = 32;     // K extent (pixels of the other image) of one gradient-GEMM block
+constexpr int GG_KJ = 32;     // and of the image-2-major one: 32 image-1 pixels
 constexpr int KC_MAX_PER_SWEEP = 4;  // attention channels handled by one compression sweep
 
 // 16-bit operand kinds of the contractions (0 = none: TF32 operands in FP32 storage).
@@ -136,7 +136,6 @@ struct GradArgs {
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
   int whole_tiles, pieces;           // as in SweepArgs, here with pieces of the K sweep (TileSplit)
   float* part;
-  int* tail_count;       // one zero per tail tile; every launch leaves them zero
 };
 TileSplit grad_split(const Dims& d, int image2_major);
 
@@ -167,9 +166,7 @@ struct SlotSources {
 
 // Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, all cleared by
 // launch_prepare.  amax slots hold float bits (atomicMax), the others floats; every scale is a power of two.
-// From WS_TAIL_OFFSET on, SM_COUNT counters of the tail tiles (GradArgs::tail_count).
-constexpr size_t WS_HEADER_BYTES = 1024, WS_SCALES_OFFSET = 64, WS_TAIL_OFFSET = 256, WS_HEADER_CLEAR_BYTES = 1024;
-static_assert(WS_TAIL_OFFSET + SM_COUNT * sizeof(int) <= WS_HEADER_CLEAR_BYTES, "tail counters");
+constexpr size_t WS_HEADER_BYTES = 1024, WS_SCALES_OFFSET = 64, WS_HEADER_CLEAR_BYTES = 256;
 enum : int {
   SCALE_AMAX_F1 = 0, SCALE_AMAX_F2 = 1, SCALE_AMAX_G = 2, SCALE_AMAX_A = 3,
   SCALE_F1 = 4, SCALE_F2 = 5, SCALE_INV_F1F2 = 6,   // F1h = fp16(s1 F1), F2h = fp16(s2 F2), sweep outputs * 1/(s1 s2)

@@ -501,8 +501,8 @@ cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int 
 
 // Channel-major copies of a pixel-major feature array (B, rows*width, C), the K-major B operands of the gradient GEMMs.
 //   blocked = 0: dst (B, C, pitch), pixel index = row*width + x (image 1: rows = 1, width = N1, pitch = n1p)
-//   blocked = 1: dst (B, C, ceil(width/16), pitch, 16): columns in blocks of 16, so that the 2 rows x 16 columns of one
-//                K block of the image-1-major GEMM are 32 consecutive values (image 2: pitch = H2 rounded up to even)
+//   blocked = 1: dst (B, C, ceil(width/16), pitch, 16): columns in blocks of 16, so that the 4 rows x 16 columns of one
+//                K block of the image-1-major GEMM are 64 consecutive values (image 2: pitch = H2 rounded up to 4)
 // Padding is not written (the caller clears the array).  32 x 32 tiles through shared memory; grid (ceil(width/32),
 // ceil(C/32), B*rows), block (32, 8).
 template <typename T>

@@ -91,6 +91,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, WaitCt
   return mbar_wait_slow(bar, parity, ctl, status, code);
 }
 
+// The same by all lanes of a warp, with one result for all of them: the lanes, which may leave the wait at different times, are
+// together again after it, as the .sync.aligned instructions that follow (tcgen05.ld / st) need them.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, WaitCtl* ctl, int* status, int code) {
+  const bool ok = mbar_wait(bar, parity, ctl, status, code);
+  return __all_sync(0xffffffffu, ok);
+}
+
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -378,8 +385,8 @@ __host__ __device__ constexpr uint32_t make_idesc_fp16(int M, int N) {
 #define SFB_OP16_KINDS
 enum : int { OP16_NONE = 0, OP16_BF16 = 1, OP16_FP16 = 2 };
 #endif
-__host__ __device__ constexpr uint32_t make_idesc_op16(int op16, int M, int N) {
-  return op16 == OP16_FP16 ? make_idesc_fp16(M, N) : make_idesc_bf16(M, N);
+__host__ __device__ constexpr uint32_t make_idesc_op16(int op16, int M, int N, bool a_mn_major = false) {
+  return (op16 == OP16_FP16 ? make_idesc_fp16(M, N) : make_idesc_bf16(M, N)) | ((a_mn_major ? 1u : 0u) << 15);
 }
 
 // Round-to-nearest (ties away from zero) to TF32's 10 mantissa bits.  Same result as cvt.rna.tf32.f32 for
