@@ -619,13 +619,18 @@ attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const 
   }
 }
 
-// out[i] = sum over rows of partial[i][row].  One block per column: thread t adds rows t, t + 256, ... in order, then
-// the 256 partial sums are combined in a fixed tree, so the result does not depend on scheduling (bit-reproducible).
+// out[i] = sum over rows of partial[i][row], for the weight gradients (blocks 0 .. weights.n - 1) and, in the same launch, the
+// bias gradients.  One block per column: thread t adds rows t, t + 256, ... in order, then the 256 partial sums are combined in
+// a fixed tree, so the result does not depend on scheduling (bit-reproducible).
 constexpr int RP_THREADS = 256;
+struct PartialSums { const float* partial; float* out; int rows, n; };
 __global__ void __launch_bounds__(RP_THREADS)
-attention_reduce_partials_kernel(const float* __restrict__ partial, int rows, float* __restrict__ out) {
+attention_reduce_partials_kernel(const PartialSums weights, const PartialSums biases) {
   __shared__ float red[RP_THREADS];
-  const int i = blockIdx.x;
+  const bool w = (int)blockIdx.x < weights.n;
+  const float* __restrict__ const partial = w ? weights.partial : biases.partial;
+  float* const out = w ? weights.out : biases.out;
+  const int rows = w ? weights.rows : biases.rows, i = w ? blockIdx.x : blockIdx.x - weights.n;
   float s = 0.f;
   for (int r = threadIdx.x; r < rows; r += RP_THREADS) s += __ldg(partial + (size_t)i * rows + r);
   red[threadIdx.x] = s;
@@ -873,6 +878,7 @@ struct WeightStage {
   cudaEvent_t done[AT_MAX_DEVICES] = {nullptr};
   cudaStream_t last[AT_MAX_DEVICES] = {nullptr};
   bool used[AT_MAX_DEVICES] = {false};
+  void* address[AT_MAX_DEVICES] = {nullptr};   // of c_att_weights
 } g_stage;
 
 class StagedWeights {
@@ -882,13 +888,14 @@ class StagedWeights {
     if (err_ == cudaSuccess && (dev_ < 0 || dev_ >= AT_MAX_DEVICES)) err_ = cudaErrorInvalidDevice;
     if (err_ != cudaSuccess) return;
     if (g_stage.done[dev_] == nullptr) err_ = cudaEventCreateWithFlags(&g_stage.done[dev_], cudaEventDisableTiming);
+    if (err_ == cudaSuccess && g_stage.address[dev_] == nullptr) err_ = cudaGetSymbolAddress(&g_stage.address[dev_], c_att_weights);
     if (err_ == cudaSuccess && g_stage.used[dev_] && g_stage.last[dev_] != st_)
       err_ = cudaStreamWaitEvent(st_, g_stage.done[dev_], 0);
   }
   cudaError_t put(const float* device_weights, int channels) {  // weights of `channels` <= AT_KC channels
     if (err_ != cudaSuccess) return err_;
-    err_ = cudaMemcpyToSymbolAsync(c_att_weights, device_weights, (size_t)channels * 2 * AT_TAPS * sizeof(float), 0,
-                                   cudaMemcpyDeviceToDevice, st_);
+    err_ = cudaMemcpyAsync(g_stage.address[dev_], device_weights, (size_t)channels * 2 * AT_TAPS * sizeof(float),
+                           cudaMemcpyDeviceToDevice, st_);
     return err_;
   }
   ~StagedWeights() {
@@ -1103,8 +1110,8 @@ cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, lo
     if (kw == 1) SFB_AT_WG(1); else if (kw == 2) SFB_AT_WG(2); else if (kw == 3) SFB_AT_WG(3); else SFB_AT_WG(4);
 #undef SFB_AT_WG
   }
-  attention_reduce_partials_kernel<<<d.Kc * 2 * AT_TAPS, RP_THREADS, 0, st>>>(weight_partial, wrows, gweight);
-  attention_reduce_partials_kernel<<<d.Kc, RP_THREADS, 0, st>>>(bias_partial, bias_rows, gbias);
+  const PartialSums weights{weight_partial, gweight, wrows, d.Kc * 2 * AT_TAPS}, biases{bias_partial, gbias, bias_rows, d.Kc};
+  attention_reduce_partials_kernel<<<weights.n + biases.n, RP_THREADS, 0, st>>>(weights, biases);
   return cudaGetLastError();
 }
 

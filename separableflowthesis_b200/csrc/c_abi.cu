@@ -1101,25 +1101,29 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const F
   const float* const gs = grad_slot_scales(w, op16);
   {
     const int kc = chunk_channels(K), Qc = grad_slots(kc) / 4, Q = 1 + Qc;
-    SFB_CUDA(timed(KID_PACK, 4, st, [&] {
+    SFB_CUDA(timed(KID_PACK, 1, st, [&] {
       SlotSources su, sv;
+      PackGroups groups{};
       // channel 0 = max gradient, channel 1 = mean gradient (same slots as the reference layout)
       maxavg_slot_sources(d, AM_u, AM_v, gM_v, gM_u, &su, &sv, gs);
-      SFB_LAUNCH(launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4, Q, 0, st));
-      SFB_LAUNCH(launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4, Q, 0, st));
+      groups.add(su, w.gxu, d.H2, 4, Q, 0);
+      groups.add(sv, w.gxv, d.W2, 4, Q, 0);
       compress_slot_sources(K, 0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs, gK, g0);
-      SFB_LAUNCH(launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st));
-      return launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4 * Qc, Q, 1, st);
+      groups.add(su, w.gxu, d.H2, 4 * Qc, Q, 1);
+      groups.add(sv, w.gxv, d.W2, 4 * Qc, Q, 1);
+      return launch_pack_interleaved_cf(groups, d.B, N1, w.n1p, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st, out_cf, scale1));
   }
   for (int k0 = KC_MAX_PER_SWEEP; k0 < K; k0 += KC_MAX_PER_SWEEP) {
     const int kc = chunk_channels(K - k0), R4 = grad_slots(kc);
-    SFB_CUDA(timed(KID_PACK, 2, st, [&] {
+    SFB_CUDA(timed(KID_PACK, 1, st, [&] {
       SlotSources su, sv;
+      PackGroups groups{};
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs, gK, g0);
-      SFB_LAUNCH(launch_pack_interleaved_cf(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st));
-      return launch_pack_interleaved_cf(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
+      groups.add(su, w.gxu, d.H2, R4, R4 / 4, 0);
+      groups.add(sv, w.gxv, d.W2, R4, R4 / 4, 0);
+      return launch_pack_interleaved_cf(groups, d.B, N1, w.n1p, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, 1, gF1, gF2, st, out_cf, scale1));
   }
@@ -1173,7 +1177,7 @@ size_t sfb_attention_backward_workspace_bytes(int32_t B, int32_t Kc, int32_t D, 
   return align_up(attention_partial_floats(ad) * sizeof(float), 256);
 }
 
-static int attention_backward_launches(int Kc) { return (Kc + 3) / 4 + 4; }
+static int attention_backward_launches(int Kc) { return (Kc + 3) / 4 + 3; }
 
 int sfb_attention_backward(const float* X, int64_t x_batch_stride, const float* weight, const float* A, float* gA,
                            const float* add, int64_t add_batch_stride, float* gX, float* gweight, float* gbias,

@@ -156,9 +156,29 @@ struct SlotSources {
   SlotSource s[MAX_SLOTS];
   const float* dev_scales;  // may be null when no slot has dev != 0
 };
-// Same, from channels-first sources: dst[b][d][q][p][j] = scale * src[b][k][d][p], src is (B, Ksrc, D, N1).
-[[nodiscard]] cudaError_t launch_pack_interleaved_cf(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
-                                       int Qtot, int q0, cudaStream_t stream);
+// Same, from channels-first sources: dst[b][d][q][p][j] = scale * src[b][k][d][p], src is (B, Ksrc, D, N1); the groups of four
+// slots of several operands in one launch.
+struct PackGroup {
+  SlotSource s[4];
+  float4* dst;    // the operand (B, D, Qtot, n1p, 4)
+  int D, Qtot, q; // q: this group
+};
+constexpr int MAX_PACK_GROUPS = 6;
+struct PackGroups {
+  PackGroup g[MAX_PACK_GROUPS];
+  int count;
+  const float* dev_scales;
+  void add(const SlotSources& src, float* dst, int D, int R4, int Qtot, int q0) {
+    for (int q = 0; q < R4 / 4; ++q) {
+      PackGroup& x = g[count++];
+      for (int j = 0; j < 4; ++j) x.s[j] = src.s[4 * q + j];
+      x.dst = reinterpret_cast<float4*>(dst);
+      x.D = D; x.Qtot = Qtot; x.q = q0 + q;
+    }
+    dev_scales = src.dev_scales;
+  }
+};
+[[nodiscard]] cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream);
 // Writes R4 (4 or 8) slots = R4/4 groups starting at group q0 of dst (B, D, Qtot, n1p, 4); pixels N1 <= p < n1p
 // and slots without a source are zero.
 [[nodiscard]] cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,

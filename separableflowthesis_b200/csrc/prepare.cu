@@ -361,61 +361,55 @@ cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, i
 
 // Channels-first sources are already pixel-fastest: one thread per pixel gathers the four slots of a group
 // and stores them as one 16-byte word, for PI_DB displacements at a time (all loads issued before the stores,
-// so that a thread keeps 4*Q*PI_DB loads in flight).  grid (n1p/256, ceil(D/PI_DB), B), block 256.
+// so that a thread keeps 4*PI_DB loads in flight).  One launch for all groups of a call's operands (a training step on small
+// crops is bound by the number of launches).  Four launches before: 8 x 135 x 240, four
+// channels 1720 -> 1360 us; 8 x 47 x 156, two 142 -> 115; the four levels of 2 x 48 x 64 60 -> 22.  grid (n1p/256, ceil(largest D/PI_DB), groups * B), block 256.
 constexpr int PI_DB = 4;
 
-template <int Q>
-__global__ void pack_interleaved_cf_kernel(const SlotSources src, float4* __restrict__ dst, int N1, int n1p, int D,
-                                           int Qtot, int q0) {
-  const int p = blockIdx.x * 256 + threadIdx.x, d0 = blockIdx.y * PI_DB, b = blockIdx.z;
-  if (p >= n1p) return;
-  // per slot: the factor its values are multiplied by (0 = raw 32-bit copy): host scale times device scale
-  float fac[Q][4];
+__global__ void __launch_bounds__(256)
+pack_interleaved_cf_kernel(const __grid_constant__ PackGroups groups, int B, int N1, int n1p) {
+  const int gi = blockIdx.z / B, b = blockIdx.z - gi * B;
+  const PackGroup& g = groups.g[gi];
+  const int p = blockIdx.x * 256 + threadIdx.x, d0 = blockIdx.y * PI_DB, D = g.D;
+  if (p >= n1p || d0 >= D) return;
+  const bool in = p < N1;
+  // per slot: where its values are (null: a constant), and the factor they are multiplied by (0 = raw 32-bit copy): host
+  // scale times device scale
+  const uint32_t* src[4];
+  float fac[4];
 #pragma unroll
-  for (int q = 0; q < Q; ++q)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const SlotSource& ss = src.s[4 * q + j];
-      fac[q][j] = ss.scale;
-      if (ss.dev != 0 && ss.src != nullptr) fac[q][j] = (ss.scale != 0.f ? ss.scale : 1.f) * __ldg(src.dev_scales + ss.dev - 1);
-    }
-  uint32_t w[PI_DB][Q][4];
+  for (int j = 0; j < 4; ++j) {
+    const SlotSource& ss = g.s[j];
+    src[j] = ss.src == nullptr ? nullptr : static_cast<const uint32_t*>(ss.src) + (((size_t)b * ss.Ksrc + ss.k) * D + d0) * N1 + p;
+    fac[j] = ss.scale;
+    if (ss.dev != 0 && ss.src != nullptr) fac[j] = (ss.scale != 0.f ? ss.scale : 1.f) * __ldg(groups.dev_scales + ss.dev - 1);
+  }
+  uint32_t w[PI_DB][4];
 #pragma unroll
   for (int i = 0; i < PI_DB; ++i)
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const SlotSource& ss = src.s[4 * q + j];
-        w[i][q][j] = 0;
-        if (ss.src != nullptr && p < N1 && d0 + i < D)
-          w[i][q][j] = __ldg(static_cast<const uint32_t*>(ss.src) + (((size_t)b * ss.Ksrc + ss.k) * D + d0 + i) * N1 + p);
-        else if (ss.src == nullptr && p < N1)
-          w[i][q][j] = __float_as_uint(ss.scale);  // constant slot
-      }
+    for (int j = 0; j < 4; ++j) {
+      w[i][j] = 0;
+      if (src[j] != nullptr && in && d0 + i < D) w[i][j] = __ldg(src[j] + (size_t)i * N1);
+      else if (src[j] == nullptr && in) w[i][j] = __float_as_uint(fac[j]);
+    }
+  float4* dst = g.dst + (((size_t)b * D + d0) * g.Qtot + g.q) * n1p + p;
 #pragma unroll
   for (int i = 0; i < PI_DB; ++i) {
     if (d0 + i >= D) break;
+    float v[4];
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      float v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const SlotSource& ss = src.s[4 * q + j];
-        v[j] = (fac[q][j] != 0.f && ss.src != nullptr) ? __uint_as_float(w[i][q][j]) * fac[q][j] : __uint_as_float(w[i][q][j]);
-      }
-      dst[(((size_t)b * D + d0 + i) * Qtot + q0 + q) * n1p + p] = make_float4(v[0], v[1], v[2], v[3]);
-    }
+    for (int j = 0; j < 4; ++j)
+      v[j] = (fac[j] != 0.f && src[j] != nullptr) ? __uint_as_float(w[i][j]) * fac[j] : __uint_as_float(w[i][j]);
+    dst[(size_t)i * g.Qtot * n1p] = make_float4(v[0], v[1], v[2], v[3]);
   }
 }
 
-cudaError_t launch_pack_interleaved_cf(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
-                                       int Qtot, int q0, cudaStream_t stream) {
-  const dim3 grid((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, B);
-  float4* out = reinterpret_cast<float4*>(dst);
-  if (R4 == 4) pack_interleaved_cf_kernel<1><<<grid, 256, 0, stream>>>(src, out, N1, n1p, D, Qtot, q0);
-  else if (R4 == 8) pack_interleaved_cf_kernel<2><<<grid, 256, 0, stream>>>(src, out, N1, n1p, D, Qtot, q0);
-  else return cudaErrorInvalidValue;
+cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream) {
+  int D = 1;
+  for (int i = 0; i < groups.count; ++i) D = groups.g[i].D > D ? groups.g[i].D : D;
+  const dim3 grid((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, groups.count * B);
+  pack_interleaved_cf_kernel<<<grid, 256, 0, stream>>>(groups, B, N1, n1p);
   return cudaGetLastError();
 }
 
