@@ -1,7 +1,7 @@
 """Contractions whose last wave of tiles is cut into pieces (column blocks of the sweeps, K ranges of the gradient GEMMs)
-and put together by the CTA that finishes last: one tile, a full wave of 148 tiles and one or two more, few column
+and put together by a kernel behind them: one tile, a full wave of 148 tiles and one or two more, few column
 blocks, ragged edges, several samples, more channels than one sweep takes.  Against the float64 oracle, and bit for bit
-against a second run: the pieces are added in a fixed order, whichever finishes last."""
+against a second run: the pieces are added in a fixed order."""
 import pytest
 import torch
 
