@@ -23,12 +23,10 @@ constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;  // 2 s per wait, th
 // role of the CTA then leaves its loops too) and the time limit of one wait.
 struct WaitCtl {
   int abort_flag;
-  int reserved;
   unsigned long long limit_ns;
 };
 __device__ __forceinline__ void wait_ctl_init(WaitCtl* ctl, unsigned long long limit_ns) {  // 0 = WAIT_LIMIT_NS
   ctl->abort_flag = 0;
-  ctl->reserved = 0;
   ctl->limit_ns = limit_ns != 0 ? limit_ns : WAIT_LIMIT_NS;
 }
 __device__ __forceinline__ bool wait_ctl_aborted(const WaitCtl* ctl) {
@@ -101,9 +99,18 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, W
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Makes generic-proxy shared-memory writes visible to the async proxy (tcgen05.mma operand reads).
+// Orders this thread's shared-memory accesses before those of the async proxy that follow: its writes become visible to
+// tcgen05.mma operand reads, its reads are over before a TMA load writes the same bytes.
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+// A warp hands a stage that it has read back to the TMA producer (one arrival).  The producer's next load is a write of the
+// async proxy, which an arrive that merely follows generic-proxy reads does not hold back: without the fence in every lane the
+// next load's data (whole 32-byte sectors of it) was seen among the values.
+__device__ __forceinline__ void hand_back_stage(uint64_t* empty, int lane) {
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(empty);
 }
 
 // ------------------------------------------------------------------ TMA (tiled loads, this CTA only)

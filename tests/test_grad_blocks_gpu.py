@@ -49,15 +49,24 @@ def test_exact(shape, operands, cuda_device):
         assert torch.equal(got[name][1].cpu(), torch.einsum("bijuv,bijc->buvc", G, F1)), name
 
 
+@pytest.mark.parametrize("operands", ["fp16", "bf16", "tf32"])
 @pytest.mark.parametrize("H,W", [(55, 128), (135, 240)])
-def test_repeated_calls_agree(H, W, cuda_device):
-    """Many K blocks through every ring of stages, four channels (whose values are made fastest): the same bits every time."""
+def test_repeated_calls_agree(H, W, operands, cuda_device):
+    """Many K blocks through every ring of stages, with the values of one op and of both: the same bits every time."""
     g = torch.Generator(device=cuda_device).manual_seed(5)
     randn = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
     F1, F2 = randn(1, H, W, 256) / 16, randn(1, H, W, 256)
     A_u, A_v = (randn(1, H, W, 4, D).softmax(-1) for D in (W, H))
-    gC_u, gC_v = (randn(1, H, W, 4, D) for D in (H, W))
-    first = ops.compression_backward(F1, F2, A_u, A_v, gC_u, gC_v)
-    for _ in range(8):
-        for x, y in zip(first, ops.compression_backward(F1, F2, A_u, A_v, gC_u, gC_v)):
-            assert torch.equal(x, y)
+    gC_u, gC_v, gM_u, gM_v = (randn(1, H, W, K, D) for K in (4, 2) for D in (H, W))
+    AM_u, AM_v = (torch.randint(0, n, (1, H, W, 1, D), generator=g, device=cuda_device, dtype=torch.int32) for n, D in ((W, H), (H, W)))
+
+    def run():
+        return (list(ops.compression_backward(F1, F2, A_u, A_v, gC_u, gC_v))
+                + list(ops.max_argmax_avg_backward(F1, F2, AM_u, AM_v, gM_u, gM_v))
+                + list(ops.separation_feature_backward(F1, F2, AM_u, AM_v, gM_u, gM_v, A_u, A_v, gC_u, gC_v)))
+
+    with ops.sweep_operands(operands):
+        first = run()
+        for _ in range(6):
+            for x, y in zip(first, run()):
+                assert torch.equal(x, y)
