@@ -267,8 +267,7 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int n = 0; n < 9; ++n) xv[c][n] = sm.x[s].v[c][ty + n / 3][tx + 3 + n % 3];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.empty[s]);  // the neighbourhoods are in registers
+    hand_back_stage(&sm.empty[s], lane);   // the neighbourhoods are in registers
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -705,8 +704,7 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
     for (int k = 0; k < KC; ++k)
 #pragma unroll
       for (int n = 0; n < 9; ++n) v[k][n] = sm.x[s].v[k][ty + n / 3][tx + 3 + n % 3];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.empty[s]);
+    hand_back_stage(&sm.empty[s], lane);
 #pragma unroll
     for (int k = 0; k < KC; ++k)
 #pragma unroll
@@ -807,8 +805,7 @@ attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, con
     for (int n = 0; n < 9; ++n) v[n] = sm.st[s].x[c][ty + n / 3][tx + 3 + n % 3];
 #pragma unroll
     for (int k = 0; k < KW; ++k) g_next[k] = sm.st[s].g[k][ty][tx];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.empty[s]);
+    hand_back_stage(&sm.empty[s], lane);
 #pragma unroll
     for (int q = 0; q < KP; ++q) {
       const uint64_t gn = pack2(g_next[2 * q], g_next[2 * q + 1]), gc = pack2(g_cur[2 * q], g_cur[2 * q + 1]),

@@ -80,3 +80,21 @@ def test_a_sample_alone_and_in_a_batch(D, cuda_device):
     r_gx = orc.attention_backward(x[:1].double().cpu(), weight.double().cpu(), a[:1].double().cpu(), ga[:1].double().cpu(), None)[0]
     if D > 1:
         assert relerr(gx[:1], r_gx) < TOL
+
+
+@pytest.mark.parametrize("H1,W1,D,Kc", [(55, 128, 128, 4), (55, 128, 55, 1), (135, 240, 135, 3), (135, 240, 240, 4)])
+def test_repeated_calls_agree(H1, W1, D, Kc, cuda_device):
+    """Many planes through the rings of the tiled forms, on many blocks at once: the same bits every time."""
+    g = torch.Generator(device=cuda_device).manual_seed(9)
+    randn = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
+    x, weight, bias = randn(2, 2, D, H1, W1), randn(Kc, 2, 3, 3, 3) * 0.3, randn(Kc)
+    ga, add = randn(2, Kc, D, H1, W1), randn(2, 2, D, H1, W1)
+
+    def run():
+        a = ops.attention_forward(x, weight, bias)
+        return [a, *ops.attention_backward(x, weight, a, ga.clone(), add)]
+
+    first = run()
+    for _ in range(6):
+        for p, q in zip(first, run()):
+            assert torch.equal(p, q)

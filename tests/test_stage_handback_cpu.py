@@ -9,7 +9,7 @@ import pytest
 
 from separableflowthesis_b200 import build
 
-SOURCES = ["grad_gemm.cu"]
+SOURCES = ["grad_gemm.cu", "attention.cu"]
 
 
 @pytest.mark.parametrize("name", SOURCES)
