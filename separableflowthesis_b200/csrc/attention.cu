@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(AT_THREADS + 32)
 attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const float* __restrict__ bias,
                               float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1,
                               int* status) {
-  if (*reinterpret_cast<volatile int*>(status) != 0) return;
+  if (!cta_has_work(status)) return;
   __shared__ __align__(128) AttentionTileSmem<2> sm;
   const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z % B, d0 = (blockIdx.z / B) * dc;
   const int d1 = min(d0 + dc, D);
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(AT_THREADS + 32)
 attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, const float* __restrict__ add,
                                   long long add_sb, float* __restrict__ gx, int accumulate, int k0, int B, int D,
                                   int dc, int H1, int W1, int* status) {
-  if (*reinterpret_cast<volatile int*>(status) != 0) return;
+  if (!cta_has_work(status)) return;
   __shared__ __align__(128) AttentionTileSmem<KC> sm;
   const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z % B, d0 = (blockIdx.z / B) * dc;
   const int d1 = min(d0 + dc, D);
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(WG_WARPS * 32 + 32, 1)
 attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_gl,
                                    const float* __restrict__ gl, float* __restrict__ partial, int Kc, int B, int D,
                                    int dc, int chunks, int H1, int W1, int* status) {
-  if (*reinterpret_cast<volatile int*>(status) != 0) return;
+  if (!cta_has_work(status)) return;
   __shared__ __align__(128) WeightGradTileSmem<KW> sm;
   constexpr int KP = KW / 2;   // packed channel pairs
   const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH;

@@ -551,7 +551,7 @@ template <int MODE, int Q, int I2MAJOR, int BF16>
 __global__ void __launch_bounds__(GG_THREADS, 1)
 grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_xu,
                  const __grid_constant__ CUtensorMap tm_xv, const GradArgs a) {
-  if (*reinterpret_cast<volatile int*>(a.status) != 0) return;
+  if (!cta_has_work(a.status)) return;
   using Smem = GradSmem<Q, I2MAJOR>;
   using Cfg = GradCfg<Q, I2MAJOR>;
 

@@ -29,6 +29,13 @@ __device__ __forceinline__ void wait_ctl_init(WaitCtl* ctl, unsigned long long l
   ctl->abort_flag = 0;
   ctl->limit_ns = limit_ns != 0 ? limit_ns : WAIT_LIMIT_NS;
 }
+// Whether a wait of the launch has run out already, in which case a CTA that starts now does nothing.  One read for the whole
+// CTA (every thread calls it, before any barrier or register split is set up): CTAs that give up write the word at any time,
+// and warps that read it for themselves could part ways, some of them gone and the others waiting for them.
+__device__ __forceinline__ bool cta_has_work(const int* status) {
+  const int gave_up = threadIdx.x == 0 ? *reinterpret_cast<const volatile int*>(status) : 0;
+  return __syncthreads_or(gave_up) == 0;
+}
 __device__ __forceinline__ bool wait_ctl_aborted(const WaitCtl* ctl) {
   return *reinterpret_cast<const volatile int*>(&ctl->abort_flag) != 0;
 }

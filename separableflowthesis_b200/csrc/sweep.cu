@@ -659,7 +659,7 @@ template <int MODE, bool CUT, int KC>
 __global__ void __launch_bounds__(SW_THREADS, 1)
 sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ CUtensorMap tm_f2,
              const __grid_constant__ CUtensorMap tm_aux, const SweepArgs a) {
-  if (*reinterpret_cast<volatile int*>(a.status) != 0) return;  // an earlier CTA gave up: do not pile on
+  if (!cta_has_work(a.status)) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;

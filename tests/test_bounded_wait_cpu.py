@@ -1,0 +1,31 @@
+"""CPU: what the kernels with bounded waits have to do so that every wait stays bounded, read from their source."""
+import os
+import re
+
+from separableflowthesis_b200 import build
+
+
+def kernels_with_barriers():
+    for name in build.SOURCES:
+        text = re.sub(r"//.*", "", open(os.path.join(build.CSRC, name)).read())
+        for part in re.split(r"(?m)^(?=__global__|template)", text):
+            if part.startswith("__global__") and "mbar_init(" in part:
+                # up to the end of the function: the first line that is a closing brace
+                yield re.search(r"(\w+)\(", part.split(")", 1)[1]).group(1), part[:part.index("\n}")]
+
+
+def test_the_kernels_are_found():
+    names = [name for name, _ in kernels_with_barriers()]
+    assert len(names) == 5 and "sweep_kernel" in names and "grad_gemm_kernel" in names, names
+
+
+def test_a_cta_leaves_early_as_a_whole():
+    """The status word can be written by another CTA between the reads of two warps.  A warp that left alone would be missing
+    from the barriers, from the barriers' initialisation or from the hand-over of registers, for which no limit exists."""
+    for name, body in kernels_with_barriers():
+        first = body[body.index("{") + 1:].strip()
+        assert re.match(r"if \(!cta_has_work\((a\.)?status\)\) return;", first), name
+        assert "volatile int*>(status)" not in body and "volatile int*>(a.status)" not in body, name
+    text = open(os.path.join(build.CSRC, "sm100_primitives.cuh")).read()
+    helper = text[text.index("bool cta_has_work("):]
+    assert "__syncthreads_or(" in helper[:helper.index("\n}")]
