@@ -43,7 +43,10 @@ constexpr int SW_THREADS = 128 + SW_EPI_WARPS * 32;
 // Registers a thread (setmaxnreg): the launch has 168 for each of its 384 threads; the four warps of the first warpgroup
 // (TMA, MMA, two idle) need few, and the epilogues keep two channels' weights and sums of 32 columns (128 registers).
 constexpr int SW_REGS_LAUNCH = 168, SW_REGS_ISSUE = 40, SW_REGS_EPI = 232;
-static_assert(SW_REGS_ISSUE + 2 * SW_REGS_EPI <= 3 * SW_REGS_LAUNCH, "more registers than the launch has");
+constexpr bool register_split_fits(int regs_per_thread) {   // at launch
+  return regs_per_thread * SW_THREADS >= 128 * SW_REGS_ISSUE + SW_EPI_WARPS * 32 * SW_REGS_EPI;
+}
+static_assert(register_split_fits(SW_REGS_LAUNCH) && !register_split_fits(SW_REGS_LAUNCH - 1), "more registers than the launch has");
 constexpr int SW_RW = SWEEP_UT / 2;             // tile rows of one epilogue warpgroup when the two split a tile's rows
 constexpr int SW_NMERGE = 4;                    // ring of column-merge barriers (> SW_NACC tiles of run-ahead)
 constexpr uint32_t SW_STAGE_BYTES = SW_TILE_N * KBLK * 4;
@@ -817,6 +820,10 @@ static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, cons
   auto kern = sweep_kernel<MODE, CUT, KC>;
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
+    // A kernel that was compiled for fewer registers than the split takes would wait in setmaxnreg.inc without a limit.
+    cudaFuncAttributes built;
+    if (cudaError_t e = cudaFuncGetAttributes(&built, kern); e != cudaSuccess) return e;
+    if (!register_split_fits(built.numRegs)) return cudaErrorInvalidKernelImage;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM_BYTES);
   });
   if (err != cudaSuccess) return err;

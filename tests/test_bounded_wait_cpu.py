@@ -29,3 +29,15 @@ def test_a_cta_leaves_early_as_a_whole():
     text = open(os.path.join(build.CSRC, "sm100_primitives.cuh")).read()
     helper = text[text.index("bool cta_has_work("):]
     assert "__syncthreads_or(" in helper[:helper.index("\n}")]
+
+
+def test_a_register_split_is_checked_against_the_compiled_kernel():
+    """setmaxnreg.inc waits for registers of the CTA's launch; a kernel compiled for fewer than the split adds up to must be
+    refused by the host."""
+    sources = [open(os.path.join(build.CSRC, name)).read() for name in build.SOURCES]
+    split = [text for text in sources if "set_max_registers<" in text]
+    assert len(split) == 1
+    host = split[0][split[0].index("static cudaError_t launch_one("):]
+    host = host[:host.index("\n}")]
+    order = [host.index(s) for s in ("cudaFuncGetAttributes(&built, kern)", "register_split_fits(built.numRegs)", "kern<<<")]
+    assert order == sorted(order)
