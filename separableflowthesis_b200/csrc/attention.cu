@@ -233,7 +233,7 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
     if (lane == 0) {
       for (int i = 0; i < n_planes; ++i) {
         const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) break;
+        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
         mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES);
         tma_load_5d(sm.x[s].v, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
       }
@@ -261,7 +261,7 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
     const int e = e0 + i;
     const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
     const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
-    if (!__all_sync(0xffffffffu, ok)) return;
+    if (!__all_sync(0xffffffffu, ok)) { let_copies_land(); return; }
     float xv[2][9];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -667,7 +667,7 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
     if (lane == 0) {
       for (int i = 0; i < n_planes; ++i) {
         const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) break;
+        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
         mbar_expect_tx(&sm.full[s], KC * AT_TILE_BYTES);
         tma_load_5d(sm.x[s].v, &tm_gl, &sm.full[s], w0 - 4, h0 - 1, e0 + i, k0, b);
       }
@@ -698,7 +698,7 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
     const int e = e0 + i;
     const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
     const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
-    if (!__all_sync(0xffffffffu, ok)) return;
+    if (!__all_sync(0xffffffffu, ok)) { let_copies_land(); return; }
     float v[KC][9];
 #pragma unroll
     for (int k = 0; k < KC; ++k)
@@ -767,7 +767,7 @@ attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, con
     if (lane == 0) {
       for (int i = 0; i < n_planes; ++i) {
         const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) break;
+        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
         mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES + KW * AT_TH * AT_TW * (uint32_t)sizeof(float));
         tma_load_5d(sm.st[s].x, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
         tma_load_5d(sm.st[s].g, &tm_gl, &sm.full[s], w0, h0, e0 + i + 1, k0, b);  // plane D, channels >= Kc read as zero
@@ -799,7 +799,7 @@ attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, con
   for (int i = 0; i < n_planes; ++i) {  // plane e of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2)
     const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
     const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
-    if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+    if (!__all_sync(0xffffffffu, ok)) { let_copies_land(); alive = false; break; }
     float v[9];
 #pragma unroll
     for (int n = 0; n < 9; ++n) v[n] = sm.st[s].x[c][ty + n / 3][tx + 3 + n % 3];

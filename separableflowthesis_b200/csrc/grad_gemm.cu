@@ -619,7 +619,7 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (wait_ctl_aborted(&sm.ctl)) {
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    let_copies_land();
     __syncthreads();
   }
   if (warp == 1) {

@@ -40,6 +40,12 @@ __device__ __forceinline__ bool wait_ctl_aborted(const WaitCtl* ctl) {
   return *reinterpret_cast<const volatile int*>(&ctl->abort_flag) != 0;
 }
 
+// After a wait that ran out: time for the CTA's own copies in flight (TMA latency is a few microseconds) before its shared
+// memory is released.
+__device__ __forceinline__ void let_copies_land() {
+  for (int i = 0; i < 64; ++i) __nanosleep(1000);
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

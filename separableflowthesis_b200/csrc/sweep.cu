@@ -689,13 +689,12 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
 
-  // Every role is through: its copies have landed (or, where a wait ran out, get time to; TMA latency is a few microseconds)
-  // before the CTA's shared memory is released.
+  // Every role is through: its copies have landed, or, where a wait ran out, get time to.
   auto meet = [&] {
     tc_fence_before();
     __syncthreads();
     if (wait_ctl_aborted(&sm.ctl)) {
-      for (int i = 0; i < 64; ++i) __nanosleep(1000);
+      let_copies_land();
       __syncthreads();
     }
   };

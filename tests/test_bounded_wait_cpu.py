@@ -41,3 +41,14 @@ def test_a_register_split_is_checked_against_the_compiled_kernel():
     host = host[:host.index("\n}")]
     order = [host.index(s) for s in ("cudaFuncGetAttributes(&built, kern)", "register_split_fits(built.numRegs)", "kern<<<")]
     assert order == sorted(order)
+
+
+def test_a_cta_that_gives_up_lets_its_copies_land():
+    """Shared memory may go to another CTA when the last warp leaves.  Either all roles meet at the end and wait there, or every
+    wait that fails is followed by the pause."""
+    for name, body in kernels_with_barriers():
+        waits = list(re.finditer(r"mbar_wait\([^;{]*;", body)) + list(re.finditer(r"if \(!mbar_wait\([^{]*", body))
+        if not waits:   # the roles are functions of their own: they meet
+            assert re.search(r"__syncthreads\(\);\s*if \(wait_ctl_aborted\(&sm\.ctl\)\) \{\s*let_copies_land\(\);", body), name
+        for m in waits:
+            assert "let_copies_land();" in body[m.start():m.start() + 400], name
