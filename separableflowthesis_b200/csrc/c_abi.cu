@@ -1101,7 +1101,7 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const F
   const float* const gs = grad_slot_scales(w, op16);
   {
     const int kc = chunk_channels(K), Qc = grad_slots(kc) / 4, Q = 1 + Qc;
-    SFB_CUDA(timed(KID_PACK, 1, st, [&] {
+    SFB_CUDA(timed(KID_PACK, pack_launches(2 * Q, d.B), st, [&] {
       SlotSources su, sv;
       PackGroups groups{};
       // channel 0 = max gradient, channel 1 = mean gradient (same slots as the reference layout)
@@ -1117,7 +1117,7 @@ static int run_fused_feature_grads_cf(const Dims& d, const Workspace& w, const F
   }
   for (int k0 = KC_MAX_PER_SWEEP; k0 < K; k0 += KC_MAX_PER_SWEEP) {
     const int kc = chunk_channels(K - k0), R4 = grad_slots(kc);
-    SFB_CUDA(timed(KID_PACK, 1, st, [&] {
+    SFB_CUDA(timed(KID_PACK, pack_launches(2 * (R4 / 4), d.B), st, [&] {
       SlotSources su, sv;
       PackGroups groups{};
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs, gK, g0);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
 namespace sfb {
@@ -157,7 +158,7 @@ struct SlotSources {
   const float* dev_scales;  // may be null when no slot has dev != 0
 };
 // Same, from channels-first sources: dst[b][d][q][p][j] = scale * src[b][k][d][p], src is (B, Ksrc, D, N1); the groups of four
-// slots of several operands in one launch.
+// slots of several operands in one launch (pack_launches, for very large batches).
 struct PackGroup {
   SlotSource s[4];
   float4* dst;    // the operand (B, D, Qtot, n1p, 4)
@@ -178,6 +179,8 @@ struct PackGroups {
     dev_scales = src.dev_scales;
   }
 };
+inline int pack_groups_per_launch(int B) { return std::max(1, std::min(MAX_PACK_GROUPS, 65535 / B)); }
+inline int pack_launches(int groups, int B) { return (groups + pack_groups_per_launch(B) - 1) / pack_groups_per_launch(B); }
 [[nodiscard]] cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream);
 // Writes R4 (4 or 8) slots = R4/4 groups starting at group q0 of dst (B, D, Qtot, n1p, 4); pixels N1 <= p < n1p
 // and slots without a source are zero.

@@ -362,8 +362,11 @@ cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, i
 // Channels-first sources are already pixel-fastest: one thread per pixel gathers the four slots of a group
 // and stores them as one 16-byte word, for PI_DB displacements at a time (all loads issued before the stores,
 // so that a thread keeps 4*PI_DB loads in flight).  One launch for all groups of a call's operands (a training step on small
-// crops is bound by the number of launches).  Four launches before: 8 x 135 x 240, four
-// channels 1720 -> 1360 us; 8 x 47 x 156, two 142 -> 115; the four levels of 2 x 48 x 64 60 -> 22.  grid (n1p/256, ceil(largest D/PI_DB), groups * B), block 256.
+// crops is bound by the number of launches): in place of four, 1720 -> 1400 us at 8 x 135 x 240 with four channels, 142 -> 111 at
+// 8 x 47 x 156 with two, 60 -> 21 for the four levels of 2 x 48 x 64.
+// grid (ceil(n1p/256), ceil(largest D/PI_DB), groups * B), block 256.  grid.z takes 65535 blocks: larger batches are packed by
+// several launches of fewer groups.  (The groups on grid.x, next to one another: 1500 us at 8 x 135 x 240; a loop over
+// (group, sample) pairs in the kernel: 1750.)
 constexpr int PI_DB = 4;
 
 __global__ void __launch_bounds__(256)
@@ -406,11 +409,20 @@ pack_interleaved_cf_kernel(const __grid_constant__ PackGroups groups, int B, int
 }
 
 cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream) {
-  int D = 1;
-  for (int i = 0; i < groups.count; ++i) D = groups.g[i].D > D ? groups.g[i].D : D;
-  const dim3 grid((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, groups.count * B);
-  pack_interleaved_cf_kernel<<<grid, 256, 0, stream>>>(groups, B, N1, n1p);
-  return cudaGetLastError();
+  const int per_launch = pack_groups_per_launch(B);
+  for (int first = 0; first < groups.count; first += per_launch) {
+    PackGroups some = groups;
+    some.count = std::min(per_launch, groups.count - first);
+    int D = 1;
+    for (int i = 0; i < some.count; ++i) {
+      some.g[i] = groups.g[first + i];
+      D = std::max(D, some.g[i].D);
+    }
+    const dim3 grid((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, some.count * B);
+    pack_interleaved_cf_kernel<<<grid, 256, 0, stream>>>(some, B, N1, n1p);
+    if (cudaError_t err = cudaGetLastError(); err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_pack(const void* src, float* dst, int B, int N1, int n1p, int Ksrc, int ksrc0, int K, int D,
