@@ -460,17 +460,23 @@ const float* sweep_out_scale(const Workspace& w, int op16) {
   return op16 == OP16_FP16 ? w.scales + SCALE_INV_F1F2 : nullptr;
 }
 
-// Tensor maps of the sweeps' operands in a workspace: the rounded FP32 copies or the 16-bit copies (aux may be null).
-int map_sweep_operands(const Dims& d, const Workspace& w, int op16, CUtensorMap* f1, CUtensorMap* f2, CUtensorMap* aux) {
-  if (op16) {
-    SFB_TRY(map_f1_rows(f1, d, w.F1h, TILE_M, CU_TENSOR_MAP_SWIZZLE_128B, true));
-    SFB_TRY(map_f2_tile(f2, d, w.F2h, SWEEP_UT, SWEEP_VT, CU_TENSOR_MAP_SWIZZLE_128B, true));
-    if (aux != nullptr) SFB_TRY(map_aux(aux, d, w.auxh, true));
-  } else {
-    SFB_TRY(map_f1_rows(f1, d, w.F1r, TILE_M));
-    SFB_TRY(map_f2_tile(f2, d, w.F2r, SWEEP_UT, SWEEP_VT));
-    if (aux != nullptr) SFB_TRY(map_aux(aux, d, w.aux));
+// Tensor maps of the sweeps' operands in a workspace: the rounded FP32 copies or the 16-bit copies.  Image 2 in the tiles of the
+// max/avg sweeps (f2) and of the compression (f2_sums); f2, f2_sums and aux may be null.
+int map_sweep_operands(const Dims& d, const Workspace& w, int op16, CUtensorMap* f1, CUtensorMap* f2, CUtensorMap* f2_sums,
+                       CUtensorMap* aux) {
+  SFB_TRY(map_f1_rows(f1, d, op16 ? static_cast<const void*>(w.F1h) : w.F1r, TILE_M, CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0));
+  for (const bool sums : {false, true}) {
+    CUtensorMap* const f = sums ? f2_sums : f2;
+    if (f == nullptr) continue;
+    const bool narrow = sweep_narrow(d, sums);
+    if (sums && f2 != nullptr && narrow == sweep_narrow(d, false)) {
+      *f2_sums = *f2;
+      continue;
+    }
+    SFB_TRY(map_f2_tile(f, d, op16 ? static_cast<const void*>(w.F2h) : w.F2r, narrow ? SWEEP_UT_NARROW : SWEEP_UT,
+                        narrow ? SWEEP_VT_NARROW : SWEEP_VT, CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0));
   }
+  if (aux != nullptr) SFB_TRY(map_aux(aux, d, op16 ? static_cast<const void*>(w.auxh) : w.aux, op16 != 0));
   return SFB_OK;
 }
 
@@ -519,7 +525,7 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   int op16;
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr, &tm_aux));
   const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, true);
   SweepArgs a;
@@ -712,7 +718,7 @@ const float* grad_slot_scales(const Workspace& w, int op16) { return op16 == OP1
 int run_attention_grads(const Dims& d, const Workspace& w, const float* gC_u, const float* gC_v, float* gA_u,
                         float* gA_v, cudaStream_t st, int op16) {
   CUtensorMap tm_f1, tm_f2;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, nullptr, &tm_f2, nullptr));
   const int N1 = d.N1(), K = d.Kc;
   SFB_CUDA(timed(KID_PACK, 2, st, [&] {
     SFB_LAUNCH(launch_pack(gC_v, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st));
@@ -792,9 +798,7 @@ int sfb_max_avg_forward_static(const float* F1, const float* F2, float* MA_u, fl
   if (need + w.part_bytes > STATIC_ARRAY_BYTES) w.part_bytes = 0;  // no room for the tail pieces: whole tiles only
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap tm_f1, tm_f2, tm_aux;
-  SFB_TRY(map_f1_rows(&tm_f1, d, w.F1r, TILE_M));
-  SFB_TRY(map_f2_tile(&tm_f2, d, w.F2r, SWEEP_UT, SWEEP_VT));
-  SFB_TRY(map_aux(&tm_aux, d, w.aux));
+  SFB_TRY(map_sweep_operands(d, w, OP16_NONE, &tm_f1, &tm_f2, nullptr, &tm_aux));
   // launch_prepare clears the status word; every other byte of the scratch that is read below is
   // written first by these launches, so nothing depends on what an earlier call left behind
   SFB_CUDA(launch_prepare(d, F1, F2, w.F1r, w.F2r, w.aux, w.status, st));
@@ -839,7 +843,7 @@ int sfb_compression_forward(const float* F1, const float* F2, const float* A_u, 
   int op16;
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, nullptr, &tm_f2, nullptr));
   const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
@@ -1025,7 +1029,7 @@ int sfb_max_argmax_avg_forward_cf(const float* F1, const float* F2, float* SEP_v
   int op16;
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2, tm_aux;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr, &tm_aux));
   const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, true);
   const int N1 = d.N1();
@@ -1059,7 +1063,7 @@ static int run_compress_cf(const float* F1, const float* F2, const float* W_u, c
   int op16;
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, nullptr, &tm_f2, nullptr));
   const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc;
@@ -1241,8 +1245,8 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d, &op16));
-  CUtensorMap tm_f1, tm_f2, tm_aux;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_aux));
+  CUtensorMap tm_f1, tm_f2, tm_f2_sums, tm_aux;
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, &tm_f2_sums, &tm_aux));
   const Features feat{F1, F2, fmaps != 0, scale1, op16};
   SFB_PREPARE(feat, true);
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
@@ -1269,7 +1273,7 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
     return launch_attention_forward(at_v, X_v, sb_v, weight_v, bias_v, A_v, st, w.status);
   }));
   // C_u (per u, weights A_u per v) -> SEP_v channels 2.., C_v -> SEP_u channels 2..
-  return run_compress_sweeps(d, w, tm_f1, tm_f2, cf_view(A_v, K, d.H2, N1), cf_view(A_u, K, d.W2, N1), 0, 0, 1,
+  return run_compress_sweeps(d, w, tm_f1, tm_f2_sums, cf_view(A_v, K, d.H2, N1), cf_view(A_u, K, d.W2, N1), 0, 0, 1,
                              cf_channels(SEP_v, Kt, c0 + 2, d.H2, N1), cf_channels(SEP_u, Kt, c0 + 2, d.W2, N1), N1, st,
                              op16, sweep_out_scale(w, op16));
 }
@@ -1313,7 +1317,7 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
   int op16;
   SFB_TRY(operand_mode(d, &op16));
   CUtensorMap tm_f1, tm_f2;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, nullptr, &tm_f2, nullptr));
   const Features feat{F1, F2, fmaps != 0, fmaps ? scale1 : 1.f, op16};
   SFB_PREPARE(feat, false);
   const int N1 = d.N1(), K = d.Kc, Kt = pl.Ktot, c0 = pl.c0;
@@ -1527,7 +1531,7 @@ int sfb_corr_volume(const float* F1, const float* F2, float* S, const sfb_shape*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int op16 = OP16_NONE;  // this test aid always computes with TF32 operands (its workspace has no 16-bit copies)
   CUtensorMap tm_f1, tm_f2;
-  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr));
+  SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, &tm_f2, nullptr, nullptr));
   const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
   SweepArgs a;

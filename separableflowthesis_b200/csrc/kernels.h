@@ -43,8 +43,10 @@ constexpr int KBLK = 32;      // fp32 elements in one 128-byte swizzled row
 #endif
 constexpr int MAX_KB = SFB_MAX_KB;  // feature dimension C <= MAX_KB * KBLK
 constexpr int MAX_C = MAX_KB * KBLK;
-constexpr int SWEEP_UT = 8;   // image-2 rows per correlation tile (8 x 32 = 256 accumulator columns)
-constexpr int SWEEP_VT = 32;  // image-2 columns per correlation tile
+// Image-2 rows and columns of a correlation tile (256 accumulator columns): wide, or narrow where that needs clearly fewer tiles
+// (sweep_narrow).
+constexpr int SWEEP_UT = 8, SWEEP_VT = 32;
+constexpr int SWEEP_UT_NARROW = 16, SWEEP_VT_NARROW = 16;
 constexpr int GG_ROW_UT = 8;  // row tile of the image-2-major gradient GEMM: 8 x 16 image-2 pixels = 128 TMEM lanes
 constexpr int GG_ROW_VT = 16;
 constexpr int GG_UT = 4;      // a K block of the image-1-major gradient GEMM: 4 image-2 rows x 16 columns
@@ -104,6 +106,18 @@ struct SweepArgs {
 constexpr int SM_COUNT = 148;
 constexpr int MAX_PIECES = 16;
 struct TileSplit { int tiles, whole_tiles, pieces, parts; size_t part_floats; };   // parts: results in scratch per tile and slot
+// Whether a sweep over this image 2 runs on narrow tiles; sums: the compression, whose row results are added up.  It follows the
+// shape of image 2 alone: the width of a tile is the order in which the compression adds up a row, and a sample's sums must not
+// depend on the batch or the row range.  A narrow tile takes as long as a wide one for max (/ arg-max) and 1.36 (two channels) to
+// 1.6 (four) times as long for the sums.  4 x 55 x 128 against 128 x 16, wide and narrow (us): maxima with arg-max 109 and 57,
+// sums of two and four channels 66 and 42, 83 and 61; against 128 x 48: 155 and 117, 112 and 115, 164 and 197.
+// What is left to the other side of the line: wide sums over 2 x 48 x 64 against 64 x 48, which narrow blocks would cut into three
+// pieces instead of two, 26 and 35 us where 24 and 33 are possible.
+__host__ __device__ inline bool sweep_narrow(const Dims& d, bool sums) {
+  const int wide = ((d.H2 + SWEEP_UT - 1) / SWEEP_UT) * ((d.W2 + SWEEP_VT - 1) / SWEEP_VT);
+  const int narrow = ((d.H2 + SWEEP_UT_NARROW - 1) / SWEEP_UT_NARROW) * ((d.W2 + SWEEP_VT_NARROW - 1) / SWEEP_VT_NARROW);
+  return sums ? 5 * narrow <= 3 * wide : 4 * narrow <= 3 * wide;
+}
 // slots: row results per pixel (max and argmax; channels of a launch); sums: they are added up, not compared
 TileSplit sweep_split(const Dims& d, int slots, bool sums);
 

@@ -2,8 +2,8 @@
 // accumulator in TMEM, reduced in the epilogue so that S never reaches HBM.
 //
 // One CTA owns 128 consecutive image-1 pixels of one sample (the rows / TMEM lanes of every
-// accumulator tile) and sweeps all image-2 pixels in tiles of SWEEP_UT x SWEEP_VT (8 rows x 32
-// columns = 256 accumulator columns), column-blocks outermost.  Warp roles:
+// accumulator tile) and sweeps all image-2 pixels in tiles of 8 rows x 32 columns (256 accumulator columns) or, over narrow
+// images, 16 x 16 (Tile), column-blocks outermost.  Warp roles:
 //   warp 0      TMA producer: F1 tile once (stays resident), F2 tiles through a ring of stages
 //   warp 1      allocates TMEM, issues tcgen05.mma (TF32 or 16-bit in, FP32 accumulate), 2 accumulators in flight
 //   warps 2, 3  idle: they make up a warpgroup, the unit in which registers are handed to the epilogues
@@ -12,7 +12,7 @@
 // Everything indexed by an image-1 pixel is read and written in the packed, pixel-fastest layout
 // (kernels.h), so a warp's 32 lanes touch one 128-byte line per access.
 // Epilogues
-//   max/avg      : group g takes tile rows 4g..4g+3.  Running column-direction max(+argmax) in
+//   max/avg      : group g takes one half of a tile's rows.  Running column-direction max(+argmax) in
 //                  registers across the inner row-block loop (the two groups' partial results are put together
 //                  once per column block), row-direction max(+argmax) merged through the packed output
 //                  once per tile.  The two mean channels come from extra tiles whose "image-2 pixels"
@@ -38,6 +38,17 @@ namespace sfb {
 constexpr int SW_NACC = 2;                      // 2 x 256 TMEM columns
 constexpr int SW_TILE_N = SWEEP_UT * SWEEP_VT;  // 256 accumulator columns: tcgen05.mma issues at a fixed
                                                 // rate per instruction, so the widest N does the most work
+// Rows and columns of a tile.  Half as many row results leave a wide tile per cell, but image 2 is padded to whole tiles, and a
+// narrow one (up to 16 columns, or one such block behind a few of 32) in half as many rows.  Both make 16 rows of 16 cells, the unit
+// that the epilogues read from tensor memory; HALVES of them lie side by side.
+template <bool NARROW>
+struct Tile {
+  static constexpr int UT = NARROW ? SWEEP_UT_NARROW : SWEEP_UT, VT = NARROW ? SWEEP_VT_NARROW : SWEEP_VT;
+  static constexpr int HALVES = VT / 16;
+  static constexpr int RW = UT / 2;   // rows of one epilogue warpgroup when the two split a tile's rows
+};
+static_assert(Tile<false>::UT * Tile<false>::VT == SW_TILE_N && Tile<true>::UT * Tile<true>::VT == SW_TILE_N, "accumulator columns");
+static_assert(Tile<false>::HALVES == 2 && Tile<true>::HALVES == 1 && Tile<false>::RW == 4 && Tile<true>::RW == 8, "see the epilogues");
 constexpr int SW_EPI_WARPS = 8;                 // two epilogue warpgroups
 constexpr int SW_THREADS = 128 + SW_EPI_WARPS * 32;
 // Registers a thread (setmaxnreg): the launch has 168 for each of its 384 threads; the four warps of the first warpgroup
@@ -47,7 +58,6 @@ constexpr bool register_split_fits(int regs_per_thread) {   // at launch
   return regs_per_thread * SW_THREADS >= 128 * SW_REGS_ISSUE + SW_EPI_WARPS * 32 * SW_REGS_EPI;
 }
 static_assert(register_split_fits(SW_REGS_LAUNCH) && !register_split_fits(SW_REGS_LAUNCH - 1), "more registers than the launch has");
-constexpr int SW_RW = SWEEP_UT / 2;             // tile rows of one epilogue warpgroup when the two split a tile's rows
 constexpr int SW_NMERGE = 4;                    // ring of column-merge barriers (> SW_NACC tiles of run-ahead)
 constexpr uint32_t SW_STAGE_BYTES = SW_TILE_N * KBLK * 4;
 constexpr uint32_t SW_F1_BLOCK_BYTES = TILE_M * KBLK * 4;
@@ -62,7 +72,6 @@ __device__ __forceinline__ uint32_t sw_stages(int nkb) {
 }
 static_assert(SW_NACC * SW_TILE_N <= 512, "accumulators exceed TMEM");
 static_assert(SW_NMERGE > SW_NACC, "a warpgroup can run SW_NACC tiles ahead of the other");
-static_assert(SWEEP_UT == 8 && SWEEP_VT == 32, "the epilogues read a row as two 16-column halves, four rows per warpgroup");
 
 struct SweepSmem {
   uint8_t ring[SW_RING_BYTES];            // image-1 tile, one 128B-swizzled block per 128 bytes of channels; then the ring of
@@ -100,7 +109,7 @@ __host__ __device__ __forceinline__ int piece_start(int n_vb, int pieces, int pi
 }
 
 // What the CTA of a block index does.
-template <int MODE, bool CUT>
+template <int MODE, bool CUT, bool NARROW>
 __device__ __forceinline__ SweepSched sweep_sched(const SweepArgs& a, int block) {
   const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
   SweepSched sc;
@@ -116,8 +125,9 @@ __device__ __forceinline__ SweepSched sweep_sched(const SweepArgs& a, int block)
   sc.b = tile / tiles_per_sample;
   sc.m0 = (tile - sc.b * tiles_per_sample) * TILE_M;
   sc.nkb = a.op16 ? (a.d.C + 2 * KBLK - 1) / (2 * KBLK) : (a.d.C + KBLK - 1) / KBLK;
-  sc.n_ub = (a.d.H2 + SWEEP_UT - 1) / SWEEP_UT;
-  const int n_vb = (a.d.W2 + SWEEP_VT - 1) / SWEEP_VT;
+  using T = Tile<NARROW>;
+  sc.n_ub = (a.d.H2 + T::UT - 1) / T::UT;
+  const int n_vb = (a.d.W2 + T::VT - 1) / T::VT;
   const int n_pieces = CUT && sc.tail >= 0 ? a.pieces : 1;
   sc.vb0 = piece_start(n_vb, n_pieces, sc.piece);
   sc.part_vb0 = piece_start(n_vb, n_pieces, 1);
@@ -130,6 +140,7 @@ __device__ __forceinline__ SweepSched sweep_sched(const SweepArgs& a, int block)
 }
 
 // ---------------------------------------------------------------------------------- producer
+template <bool NARROW>
 __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const CUtensorMap* tm_f1,
                                const CUtensorMap* tm_f2, const CUtensorMap* tm_aux) {
   const int kel = a.op16 ? 2 * KBLK : KBLK;  // channels in one 128-byte row
@@ -145,7 +156,7 @@ __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSch
       if (a.drop_last_load && t == sc.t_total - 1 && kb == sc.nkb - 1) return;  // test hook: this block never arrives
       mbar_expect_tx(&sm.full[s], SW_STAGE_BYTES);
       if (main_tile)
-        tma_load_4d(sm.f2(sc.nkb, s), tm_f2, &sm.full[s], kb * kel, vb * SWEEP_VT, ub * SWEEP_UT, sc.b);
+        tma_load_4d(sm.f2(sc.nkb, s), tm_f2, &sm.full[s], kb * kel, vb * Tile<NARROW>::VT, ub * Tile<NARROW>::UT, sc.b);
       else
         tma_load_3d(sm.f2(sc.nkb, s), tm_aux, &sm.full[s], kb * kel, (t - sc.t_main) * SW_TILE_N, sc.b);
       if (++s == n_stages) { s = 0; ph ^= 1u; }
@@ -254,12 +265,14 @@ __device__ __forceinline__ int first_of16(float bits) {   // 2^15 .. 2^1: 0 .. 1
 // Max / arg-max / mean.  Bound: the tensor core (some 2400 cycles per tile) without arg-max, and with it the ALU pipe (half
 // rate: about 480 of its instructions per warp and tile, 1900 cycles) beside what two warps per scheduler cannot hide.
 // 135 x 240, one pair, without / with arg-max: 590 -> 465 / 868 -> 630 us; 55 x 128: 81 -> 38 / 81 -> 50.
-// Group g takes tile rows 4g .. 4g+3, as two units of 4 rows x 16 columns, the second one being loaded
-// while the first is worked on.  State across the row blocks: the running maximum of each of the 32 columns and (ARG) where it
+// Group g takes half of a tile's rows, as two units of 4 rows x 16 columns (side by side, or in a narrow tile one above the
+// other), the second one being loaded while the first is worked on.  State across the row blocks: the running maximum of each column and (ARG) where it
 // lies, as the float 8 * (row / 4) + (bits of the row inside its four rows), which is exact up to 2^24.
 // NaN entries are passed over; a row that holds nothing else has the maximum NaN at index 0, such a column -inf at index 0.
-template <bool ARG, bool CUT>
+template <bool ARG, bool CUT, bool NARROW>
 __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
+  using T = Tile<NARROW>;
+  constexpr int RW = T::RW, VT = T::VT;
   const int H2 = a.d.H2, W2 = a.d.W2;
   // per-thread views: value of (displacement d, slot) at ptr[d*sd + slot*ss]
   float* pu = a.pu.base + sc.b * a.pu.sb + e.p;
@@ -277,82 +290,84 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
   const bool valid = e.valid;
   const bool all_valid = sc.m0 + TILE_M <= a.n_valid;
 
-  float rnext[SW_RW];
+  float rnext[RW];
   auto load_rows = [&](int ub, bool none) {
-    const int u0 = ub * SWEEP_UT + e.wg * SW_RW;
+    const int u0 = ub * T::UT + e.wg * RW;
 #pragma unroll
-    for (int r = 0; r < SW_RW; ++r) rnext[r] = valid && !none && u0 + r < H2 ? pu[(u0 + r) * usd] : -CUDART_INF_F;
+    for (int r = 0; r < RW; ++r) rnext[r] = valid && !none && u0 + r < H2 ? pu[(u0 + r) * usd] : -CUDART_INF_F;
   };
 #pragma unroll
-  for (int r = 0; r < SW_RW; ++r) rnext[r] = -CUDART_INF_F;
+  for (int r = 0; r < RW; ++r) rnext[r] = -CUDART_INF_F;
   int main_tiles = 0;
   for (int vb = sc.vb0; vb < sc.vb1; ++vb) {
-   const int v0 = vb * SWEEP_VT, nv = min(SWEEP_VT, W2 - v0);
+   const int v0 = vb * VT, nv = min(VT, W2 - v0);
    const bool first = vb == sc.vb0;
-   float cm[SWEEP_VT], ca[SWEEP_VT];
+   float cm[VT], ca[VT];
 #pragma unroll
-   for (int j = 0; j < SWEEP_VT; ++j) { cm[j] = -CUDART_INF_F; ca[j] = 4.f; }
+   for (int j = 0; j < VT; ++j) { cm[j] = -CUDART_INF_F; ca[j] = 4.f; }
    for (int ub = 0; ub < sc.n_ub; ++ub, ++main_tiles) {
     const int t = main_tiles;
-    const int ubase = ub * SWEEP_UT + e.wg * SW_RW;
-    const int nu = min(SW_RW, H2 - ubase);  // may be <= 0
+    const int ubase = ub * T::UT + e.wg * RW;
+    const int nu = min(RW, H2 - ubase);  // may be <= 0
     // row-direction state of earlier column blocks: asked for one tile ahead, unless that tile has the same rows
     if (sc.n_ub == 1) load_rows(ub, first);
-    float rold[SW_RW];
+    float rold[RW];
 #pragma unroll
-    for (int r = 0; r < SW_RW; ++r) rold[r] = rnext[r];
+    for (int r = 0; r < RW; ++r) rold[r] = rnext[r];
     if (sc.n_ub > 1) load_rows(ub + 1 < sc.n_ub ? ub + 1 : 0, first && ub + 1 < sc.n_ub);
-    const float qbits = static_cast<float>(ubase / SW_RW * 8);
+    const float qbase = static_cast<float>(ubase / 4 * 8);
 
     if (!epi_wait(sm, a, t)) return;
-    const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * (SW_RW * SWEEP_VT);
+    const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * (RW * VT);
     // two units of 4 rows x 16 columns; half of the second one is on its way while the first is worked on (all of it would
     // cost the arg-max form registers that it does not have)
-    uint32_t s[2][SW_RW][16];
-    auto load = [&](int h, int r) { tmem_ld16_issue(tacc + r * SWEEP_VT + h * 16, s[h][r]); };
-    float rmax[SW_RW], rbits[SW_RW];
+    uint32_t s[2][4][16];
+    auto load = [&](int h, int r) { tmem_ld16_issue(tacc + (NARROW ? (h * 4 + r) * VT : r * VT + h * 16), s[h][r]); };
+    float rmax[4], rbits[4];
     auto unit = [&](auto half, auto whole) {   // whole: every lane, row and column of this thread's part of the tile exists
       constexpr int h = decltype(half)::value;
       constexpr bool WHOLE = decltype(whole)::value;
-      uint32_t(&x)[SW_RW][16] = s[h];
+      constexpr int ROW = NARROW ? h * 4 : 0, COL = NARROW ? 0 : h * 16;   // of the unit in this thread's part
+      uint32_t(&x)[4][16] = s[h];
       if (!WHOLE) {  // cells outside the image are passed over
 #pragma unroll
-        for (int r = 0; r < SW_RW; ++r)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (r >= nu || h * 16 + j >= nv) x[r][j] = 0x7FFFFFFFu;
+            if (ROW + r >= nu || COL + j >= nv) x[r][j] = 0x7FFFFFFFu;
       }
       // rows
 #pragma unroll
-      for (int r = 0; r < SW_RW; ++r) {
+      for (int r = 0; r < 4; ++r) {
         const float mh = max16(x[r]), bits = ARG ? equal_bits16(x[r], mh) : 0.f;
-        if (h == 0) {
+        if (!NARROW && h == 0) {
           rmax[r] = mh;
           rbits[r] = bits;
           continue;
         }
-        const float m = fmaxf(rmax[r], mh);
+        const float m = NARROW ? mh : fmaxf(rmax[r], mh);
         int arg = 0;
         if (ARG) {
-          const bool left = rmax[r] == m;
-          arg = first_of16(left ? rbits[r] : bits) + (left ? v0 : v0 + 16);
+          const bool left = !NARROW && rmax[r] == m;
+          arg = first_of16(left ? rbits[r] : bits) + (NARROW || left ? v0 : v0 + 16);
           arg = m == m ? arg : 0;
         }
         const float ms = m * e.osc;  // memory holds scaled-back values; compare and store in that domain
-        float* const dst = pu + (ubase + r) * usd;
-        float* const dst_arg = ARG ? pua + (ubase + r) * uasd : nullptr;
-        const bool more = ms > fmaxf(rold[r], -CUDART_INF_F);  // strict: the lowest column block wins ties
-        if ((WHOLE || (valid && r < nu)) && (first || more)) {
+        float* const dst = pu + (ubase + ROW + r) * usd;
+        float* const dst_arg = ARG ? pua + (ubase + ROW + r) * uasd : nullptr;
+        const bool more = ms > fmaxf(rold[ROW + r], -CUDART_INF_F);  // strict: the lowest column block wins ties
+        if ((WHOLE || (valid && ROW + r < nu)) && (first || more)) {
           *dst = ms;
           if (ARG) *dst_arg = __int_as_float(arg);
         }
       }
       // columns
+      const float qbits = qbase + 2 * ROW;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const float x0 = __uint_as_float(x[0][j]), x1 = __uint_as_float(x[1][j]);
         const float x2 = __uint_as_float(x[2][j]), x3 = __uint_as_float(x[3][j]);
-        float &c = cm[h * 16 + j], &where = ca[h * 16 + j];
+        float &c = cm[COL + j], &where = ca[COL + j];
         if (ARG) {
           const float m = fmaxf(fmax3(x0, x1, x2), x3);
           const float bits = fmaf(is_equal(x0, m), 4.f, fmaf(is_equal(x1, m), 2.f, qbits + is_equal(x2, m)));
@@ -366,35 +381,35 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
     };
     auto tile = [&](auto whole) {
 #pragma unroll
-      for (int r = 0; r < SW_RW; ++r) load(0, r);
+      for (int r = 0; r < 4; ++r) load(0, r);
 #pragma unroll
-      for (int r = 0; r < SW_RW; ++r) tmem_ld_wait16(s[0][r]);
+      for (int r = 0; r < 4; ++r) tmem_ld_wait16(s[0][r]);
 #pragma unroll
-      for (int r = 0; r < SW_RW / 2; ++r) load(1, r);
+      for (int r = 0; r < 2; ++r) load(1, r);
       unit(std::integral_constant<int, 0>{}, whole);
 #pragma unroll
-      for (int r = SW_RW / 2; r < SW_RW; ++r) load(1, r);
+      for (int r = 2; r < 4; ++r) load(1, r);
 #pragma unroll
-      for (int r = 0; r < SW_RW; ++r) tmem_ld_wait16(s[1][r]);
+      for (int r = 0; r < 4; ++r) tmem_ld_wait16(s[1][r]);
       epi_release(sm, t, e.lane);  // all values are in registers: hand the accumulator back
       unit(std::integral_constant<int, 1>{}, whole);
     };
-    if (all_valid && nu == SW_RW && nv == SWEEP_VT) tile(std::true_type{});
+    if (all_valid && nu == RW && nv == VT) tile(std::true_type{});
     else tile(std::false_type{});
    }
-    // end of a column block: group 0 puts columns 0 .. 15 together, group 1 the others
+    // end of a column block: group 0 puts the first half of the columns together, group 1 the others
     {
       auto row = [&](int j) {
         const int code = static_cast<int>(ca[j]);
-        return (code >> 3) * SW_RW + __clz(code & 7) - 29;   // 4, 2, 1, 0 stand for rows 0 .. 3 of the four
+        return (code >> 3) * 4 + __clz(code & 7) - 29;   // 4, 2, 1, 0 stand for rows 0 .. 3 of the four
       };
       const int cols = valid ? nv : 0;   // columns this lane has
       auto merge = [&](auto own_half) -> bool {
-        constexpr int OWN = decltype(own_half)::value * 16, OTHER = 16 - OWN;
+        constexpr int HALF = VT / 2, OWN = decltype(own_half)::value * HALF, OTHER = HALF - OWN;
         float* q = pv + (v0 + OTHER) * vsd;
         float* qa = ARG ? pva + (v0 + OTHER) * vasd : nullptr;
 #pragma unroll
-        for (int j = OTHER; j < OTHER + 16; ++j, q += vsd, qa += ARG ? vasd : 0) {
+        for (int j = OTHER; j < OTHER + HALF; ++j, q += vsd, qa += ARG ? vasd : 0) {
           if (j < cols) *q = cm[j] * e.osc;
           if (ARG && j < cols) *qa = __int_as_float(row(j));
         }
@@ -402,16 +417,16 @@ __device__ void epilogue_maxavg(SweepSmem& sm, const SweepArgs& a, const SweepSc
         if (!merge_wait(sm, a, sc, vb, e)) return false;
         q = pv + (v0 + OWN) * vsd;
         if (ARG) qa = pva + (v0 + OWN) * vasd;
-        float om[16], oa[16];
+        float om[HALF], oa[HALF];
 #pragma unroll
-        for (int j = 0; j < 16; ++j, q += vsd, qa += ARG ? vasd : 0) {
+        for (int j = 0; j < HALF; ++j, q += vsd, qa += ARG ? vasd : 0) {
           om[j] = OWN + j < cols ? __ldcg(q) : 0.f;
           if (ARG) oa[j] = OWN + j < cols ? __ldcg(qa) : 0.f;
         }
         q = pv + (v0 + OWN) * vsd;
         if (ARG) qa = pva + (v0 + OWN) * vasd;
 #pragma unroll
-        for (int j = 0; j < 16; ++j, q += vsd, qa += ARG ? vasd : 0) {
+        for (int j = 0; j < HALF; ++j, q += vsd, qa += ARG ? vasd : 0) {
           const float mine = cm[OWN + j] * e.osc;
           if (ARG) {
             const int o = __float_as_int(oa[j]), own = row(OWN + j);
@@ -474,9 +489,11 @@ __device__ __forceinline__ void fma2_tmem(uint64_t& acc, uint32_t lo, uint32_t h
 // sums are not moved around at every tile (450 of 1860 instructions per warp and tile were moves); the row weights of the
 // next tile are asked for before the wait for this one.  135 x 240, one pair, four channels: 897 -> 717 us (8 pairs, two
 // sweeps: 14.2 -> 10.9 ms); 8 x 47 x 156, two channels: 337 -> 290 us.
-template <int CPT, bool SPLIT, bool CUT>
+template <int CPT, bool SPLIT, bool CUT, bool NARROW>
 __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
-  constexpr int NR = SPLIT ? SW_RW : SWEEP_UT;   // tile rows of this thread
+  using T = Tile<NARROW>;
+  constexpr int VT = T::VT, HALVES = T::HALVES;
+  constexpr int NR = SPLIT ? T::RW : T::UT;      // tile rows of this thread
   const int H2 = a.d.H2, W2 = a.d.W2;
   const int k_first = SPLIT ? 0 : e.wg * CPT;    // its first channel among those of this launch
   const int n_ch = min(CPT, a.kc - k_first);     // how many of them exist
@@ -499,7 +516,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
     ouss = (uint32_t)H2 * TILE_M;
     part_step = (uint32_t)a.part_slots * H2 * TILE_M;
   }
-  const int row0 = SPLIT ? e.wg * SW_RW : 0;
+  const int row0 = SPLIT ? e.wg * T::RW : 0;
   float av[CPT][NR];   // w_v of the coming tile's rows (past the image: the last row's)
   auto load_av = [&](int u0) {
 #pragma unroll
@@ -510,20 +527,20 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
   load_av(row0);
   int t = 0;
   for (int vb = sc.vb0; vb < sc.vb1; ++vb, ou += part_step) {
-    const int v0 = vb * SWEEP_VT, nv = min(SWEEP_VT, W2 - v0);
+    const int v0 = vb * VT, nv = min(VT, W2 - v0);
     const bool first = vb == 0 || part_step != 0;
-    uint64_t au2[CPT][SWEEP_VT / 2], cv2[CPT][SWEEP_VT / 2];
+    uint64_t au2[CPT][VT / 2], cv2[CPT][VT / 2];
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
       const float* wu_t = wu + v0 * xvsd + (c < n_ch ? c * wuss : 0u);
 #pragma unroll
-      for (int j = 0; j < SWEEP_VT; j += 2) {
+      for (int j = 0; j < VT; j += 2) {
         au2[c][j / 2] = pack2(j < nv ? __ldg(wu_t + j * xvsd) : 0.f, j + 1 < nv ? __ldg(wu_t + (j + 1) * xvsd) : 0.f);
         cv2[c][j / 2] = 0ull;
       }
     }
     for (int ub = 0; ub < sc.n_ub; ++ub, ++t) {
-      const int u0 = ub * SWEEP_UT + row0, nu = min(NR, H2 - u0);   // nu may be <= 0
+      const int u0 = ub * T::UT + row0, nu = min(NR, H2 - u0);   // nu may be <= 0
       uint64_t a2[CPT][NR];
 #pragma unroll
       for (int c = 0; c < CPT; ++c)
@@ -532,7 +549,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
           const float w = ul < nu ? av[c][ul] : 0.f;   // rows past the image hold S = 0; their weight must not be an infinity
           a2[c][ul] = pack2(w, w);
         }
-      load_av((ub + 1 == sc.n_ub ? 0 : ub + 1) * SWEEP_UT + row0);
+      load_av((ub + 1 == sc.n_ub ? 0 : ub + 1) * T::UT + row0);
       int rows[CPT];   // rows of each channel that are stored
       float* dst[CPT];
 #pragma unroll
@@ -541,15 +558,15 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         dst[c] = ou + u0 * ousd + c * ouss;
       }
       if (!epi_wait(sm, a, t)) return;
-      const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + row0 * SWEEP_VT;
+      const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + row0 * VT;
       uint32_t s[2][16];
       uint64_t r2[CPT];
       tmem_ld16_issue(tacc, s[0]);
 #pragma unroll
-      for (int i = 0; i < 2 * NR; ++i) {   // 16 columns of a row at a time, the next ones on their way
-        const int ul = i / 2, h = i % 2;
+      for (int i = 0; i < HALVES * NR; ++i) {   // 16 columns of a row at a time, the next ones on their way
+        const int ul = i / HALVES, h = i % HALVES;
         tmem_ld_wait();
-        if (i + 1 < 2 * NR) tmem_ld16_issue(tacc + (i + 1) * 16, s[(i + 1) % 2]);
+        if (i + 1 < HALVES * NR) tmem_ld16_issue(tacc + (i + 1) * 16, s[(i + 1) % 2]);
         else epi_release(sm, t, e.lane);   // last read of this tile
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
@@ -561,7 +578,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         for (int j = 0; j < 8; ++j)
 #pragma unroll
           for (int c = 0; c < CPT; ++c) fma2_tmem(r2[c], s[i % 2][2 * j], s[i % 2][2 * j + 1], au2[c][h * 8 + j]);
-        if (h == 1) {
+        if (h == HALVES - 1) {
 #pragma unroll
           for (int c = 0; c < CPT; ++c, dst[c - 1] += ousd) {
             if (rows[c] > ul) {
@@ -573,11 +590,11 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         }
       }
     }
-    float cv[CPT][SWEEP_VT];
+    float cv[CPT][VT];
 #pragma unroll
     for (int c = 0; c < CPT; ++c)
 #pragma unroll
-      for (int j = 0; j < SWEEP_VT / 2; ++j) unpack2(cv2[c][j], cv[c][2 * j], cv[c][2 * j + 1]);
+      for (int j = 0; j < VT / 2; ++j) unpack2(cv2[c][j], cv[c][2 * j], cv[c][2 * j + 1]);
     auto column = [&](int c, int j) { return ov + (v0 + j) * ovsd + c * ovss; };
     auto columns = [&](int c) { return e.valid && c < n_ch ? nv : 0; };   // how many of them this thread has
     if constexpr (!SPLIT) {
@@ -586,36 +603,36 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         float* q = column(c, 0);
         const int n = columns(c);
 #pragma unroll
-        for (int j = 0; j < SWEEP_VT; ++j, q += ovsd)
+        for (int j = 0; j < VT; ++j, q += ovsd)
           if (j < n) *q = cv[c][j] * e.osc;
       }
     } else {
       auto merge = [&](auto own_half) -> bool {
-        constexpr int OWN = decltype(own_half)::value * 16, OTHER = 16 - OWN;
+        constexpr int HALF = VT / 2, OWN = decltype(own_half)::value * HALF, OTHER = HALF - OWN;
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
           float* q = column(c, OTHER);
           const int n = columns(c);
 #pragma unroll
-          for (int j = OTHER; j < OTHER + 16; ++j, q += ovsd)
+          for (int j = OTHER; j < OTHER + HALF; ++j, q += ovsd)
             if (j < n) *q = cv[c][j] * e.osc;
         }
         merge_publish(sm, sc, vb, e);
         if (!merge_wait(sm, a, sc, vb, e)) return false;
-        float o[CPT][16];
+        float o[CPT][HALF];
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
           const float* q = column(c, OWN);
           const int n = columns(c);
 #pragma unroll
-          for (int j = 0; j < 16; ++j, q += ovsd) o[c][j] = OWN + j < n ? __ldcg(q) : 0.f;
+          for (int j = 0; j < HALF; ++j, q += ovsd) o[c][j] = OWN + j < n ? __ldcg(q) : 0.f;
         }
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
           float* q = column(c, OWN);
           const int n = columns(c);
 #pragma unroll
-          for (int j = 0; j < 16; ++j, q += ovsd)
+          for (int j = 0; j < HALF; ++j, q += ovsd)
             if (OWN + j < n) *q = cv[c][OWN + j] * e.osc + o[c][j];
         }
         return true;
@@ -626,14 +643,16 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
 }
 
 // Test aid: writes the dense volume of a (small) problem so the tensor-core plumbing can be checked alone.
+template <bool NARROW>
 __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
+  using T = Tile<NARROW>;
   const int H2 = a.d.H2, W2 = a.d.W2, N1 = a.d.N1();
   const bool valid = e.p < N1;
   float* out = a.dump + ((size_t)sc.b * N1 + (valid ? e.p : 0)) * H2 * W2;
   int vb = 0, ub = 0;
   for (int t = 0; t < sc.t_main; ++t) {
-    const int v0 = vb * SWEEP_VT, ubase = ub * SWEEP_UT + e.wg * SW_RW;
-    const int nu = min(SW_RW, H2 - ubase), nv = min(SWEEP_VT, W2 - v0);
+    const int v0 = vb * T::VT, ubase = ub * T::UT + e.wg * T::RW;
+    const int nu = min(T::RW, H2 - ubase), nv = min(T::VT, W2 - v0);
     if (!epi_wait(sm, a, t)) return;
     const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + e.wg * 128;
 #pragma unroll
@@ -643,11 +662,11 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
       if (half == 1) epi_release(sm, t, e.lane);
       if (valid) {
 #pragma unroll
-        for (int hl = 0; hl < SW_RW / 2; ++hl)
+        for (int hl = 0; hl < T::RW / 2; ++hl)
 #pragma unroll
-          for (int j = 0; j < SWEEP_VT; ++j) {
-            const int ul = half * (SW_RW / 2) + hl;
-            if (ul < nu && j < nv) out[(size_t)(ubase + ul) * W2 + v0 + j] = s[hl * SWEEP_VT + j] * e.osc;
+          for (int j = 0; j < T::VT; ++j) {
+            const int ul = half * (T::RW / 2) + hl;
+            if (ul < nu && j < nv) out[(size_t)(ubase + ul) * W2 + v0 + j] = s[hl * T::VT + j] * e.osc;
           }
       }
     }
@@ -658,7 +677,7 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
 // ---------------------------------------------------------------------------------- kernel
 // CUT: the launch has tail pieces.  A launch without any runs the kernel without their bookkeeping.
 // KC (compression): channels of the launch, 1, 2 or (three or four) 4.
-template <int MODE, bool CUT, int KC>
+template <int MODE, bool CUT, int KC, bool NARROW>
 __global__ void __launch_bounds__(SW_THREADS, 1)
 sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ CUtensorMap tm_f2,
              const __grid_constant__ CUtensorMap tm_aux, const SweepArgs a) {
@@ -702,9 +721,9 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   // follows there for SW_REGS_EPI.
   if (warp < 4) {
     set_max_registers<SW_REGS_ISSUE, false>();
-    const SweepSched sc = sweep_sched<MODE, CUT>(a, blockIdx.x);
+    const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, blockIdx.x);
     if (warp == 0) {
-      if (lane == 0) sweep_producer(sm, a, sc, &tm_f1, &tm_f2, &tm_aux);
+      if (lane == 0) sweep_producer<NARROW>(sm, a, sc, &tm_f1, &tm_f2, &tm_aux);
     } else if (warp == 1) {
       if (lane == 0) sweep_mma(sm, a, sc);
     }
@@ -717,7 +736,7 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     return;
   }
   set_max_registers<SW_REGS_EPI, true>();
-  const SweepSched sc = sweep_sched<MODE, CUT>(a, blockIdx.x);
+  const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, blockIdx.x);
   EpiCtx e;
   const int q = warp & 3;  // tcgen05.ld lets a warp read TMEM lanes 32*(warp%4) .. +31 only
   e.wg = (warp >> 2) - 1;
@@ -726,10 +745,10 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   e.valid = e.p < a.n_valid;
   e.tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
   e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
-  if constexpr (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT>(sm, a, sc, e);
-  else if constexpr (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT>(sm, a, sc, e);
-  else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC == 1 ? 1 : 2, KC <= 2, CUT>(sm, a, sc, e);
-  else epilogue_dump(sm, a, sc, e);
+  if constexpr (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT, NARROW>(sm, a, sc, e);
+  else if constexpr (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT, NARROW>(sm, a, sc, e);
+  else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC == 1 ? 1 : 2, KC <= 2, CUT, NARROW>(sm, a, sc, e);
+  else epilogue_dump<NARROW>(sm, a, sc, e);
   __syncwarp();
   meet();
 }
@@ -794,7 +813,9 @@ __global__ void __launch_bounds__(TILE_M) sweep_fold_kernel(const SweepArgs a) {
 // 1 x 55 x 128 against 27 x 64: 30 and 25, 25 and 21; 3 x 20 x 27 against 18 x 50: 25 and 19, 19 and 14.
 TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   const long long tiles = (long long)d.B * ((d.N1() + TILE_M - 1) / TILE_M);
-  const int n_ub = (d.H2 + SWEEP_UT - 1) / SWEEP_UT, n_vb = (d.W2 + SWEEP_VT - 1) / SWEEP_VT;
+  const bool narrow = sweep_narrow(d, sums);
+  const int ut = narrow ? SWEEP_UT_NARROW : SWEEP_UT, vt = narrow ? SWEEP_VT_NARROW : SWEEP_VT;
+  const int n_ub = (d.H2 + ut - 1) / ut, n_vb = (d.W2 + vt - 1) / vt;
   const int rest = (int)(tiles % SM_COUNT);
   TileSplit r{(int)tiles, (int)tiles, 1, 0, 0};
   if (rest == 0) return r;
@@ -813,10 +834,10 @@ TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   return r;
 }
 
-template <int MODE, bool CUT, int KC>
+template <int MODE, bool CUT, int KC, bool NARROW>
 static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                               const CUtensorMap& tm_aux, cudaStream_t stream) {
-  auto kern = sweep_kernel<MODE, CUT, KC>;
+  auto kern = sweep_kernel<MODE, CUT, KC, NARROW>;
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
     // A kernel that was compiled for fewer registers than the split takes would wait in setmaxnreg.inc without a limit.
@@ -838,11 +859,18 @@ static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, cons
   return cudaGetLastError();
 }
 
+template <int MODE, bool CUT, int KC>
+static cudaError_t launch_width(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
+                                const CUtensorMap& tm_aux, cudaStream_t stream) {
+  return sweep_narrow(a.d, MODE == SWEEP_COMPRESS) ? launch_one<MODE, CUT, KC, true>(a, tm_f1, tm_f2, tm_aux, stream)
+                           : launch_one<MODE, CUT, KC, false>(a, tm_f1, tm_f2, tm_aux, stream);
+}
+
 template <int MODE, int KC>
 static cudaError_t launch_mode(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                                const CUtensorMap& tm_aux, cudaStream_t stream) {
-  return a.pieces > 1 ? launch_one<MODE, true, KC>(a, tm_f1, tm_f2, tm_aux, stream)
-                      : launch_one<MODE, false, KC>(a, tm_f1, tm_f2, tm_aux, stream);
+  return a.pieces > 1 ? launch_width<MODE, true, KC>(a, tm_f1, tm_f2, tm_aux, stream)
+                      : launch_width<MODE, false, KC>(a, tm_f1, tm_f2, tm_aux, stream);
 }
 
 cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
@@ -850,7 +878,7 @@ cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUt
   switch (a.mode) {
     case SWEEP_MAXAVG: return launch_mode<SWEEP_MAXAVG, 0>(a, tm_f1, tm_f2, tm_aux, stream);
     case SWEEP_MAXARGAVG: return launch_mode<SWEEP_MAXARGAVG, 0>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_DUMP: return launch_one<SWEEP_DUMP, false, 0>(a, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_DUMP: return launch_width<SWEEP_DUMP, false, 0>(a, tm_f1, tm_f2, tm_aux, stream);
     case SWEEP_COMPRESS:
       switch (a.kc) {
         case 1: return launch_mode<SWEEP_COMPRESS, 1>(a, tm_f1, tm_f2, tm_aux, stream);
