@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 # (B, H1, W1, H2, W2, C, Kc), all of them cut
 SHAPES = [
-    (1, 1, 5, 5, 97, 16, 1),              # one tile of few pixels, seven column blocks
+    (1, 1, 5, 5, 97, 16, 1),              # one tile of few pixels, four column blocks
     (1, 9, 31, 33, 65, 40, 3),            # three tiles, ragged rows and columns
     (3, 20, 27, 18, 50, 64, 6),           # several samples, two compression sweeps
     (1, 1, 148 * 128 + 1, 17, 49, 8, 2),  # a wave of whole tiles and a tail of one pixel

@@ -4,7 +4,7 @@ and sum is exact in FP32 whatever its order: results are compared bit for bit, t
 import pytest
 import torch
 
-from separableflowthesis_b200 import ops
+from separableflowthesis_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -15,6 +15,8 @@ SHAPES = [(1, 3, 43, h2, w2, kc) for kc, (h2, w2) in enumerate([(4, 16), (5, 31)
     (1, 5, 26, 33, 97, 3),      # a channel without a neighbour, several blocks both ways
     (1, 9, 31, 23, 48, 6),      # two sweeps, half a column block left over
     (150, 1, 5, 9, 33, 2),      # more tiles than SMs
+    (149, 1, 5, 17, 97, 3),     # a tail of one tile behind a wave, in four pieces
+    (150, 1, 5, 33, 97, 6),     # of two tiles, of samples 148 and 149, two sweeps
 ]
 # image 2 so narrow, or so little wider than a block, that it is swept in tiles of 16 x 16
 NARROW = [
@@ -24,6 +26,7 @@ NARROW = [
     (1, 8, 17, 32, 48, 1),      # whole tiles in three blocks
     (1, 9, 31, 48, 47, 6),      # three blocks, two sweeps
     (150, 1, 5, 25, 8, 2),      # more tiles than SMs
+    (150, 1, 5, 48, 48, 2),     # a tail of two, in three pieces; the sums on wide tiles in two
 ]
 
 
@@ -97,3 +100,17 @@ def test_a_level_sweeps_its_maxima_and_its_sums_each_in_their_tiles(H2, W2, cuda
     S, a_u, a_v = S.double(), a_u.double(), a_v.double()
     assert (sep_v[:, 2:] - torch.einsum("buvij,bkvij->bkuij", S, a_u)).abs().max() <= bound
     assert (sep_u[:, 2:] - torch.einsum("buvij,bkuij->bkvij", S, a_v)).abs().max() <= bound
+
+
+@pytest.mark.parametrize("shape", [SHAPES[-2], SHAPES[-1], NARROW[-1]])
+def test_the_tails_behind_a_wave_are_cut(shape, cuda_device):
+    """What test_exact says of these shapes: the pieces are folded by a launch of their own."""
+    F1, F2 = [t.to(cuda_device) for t in features(shape)]
+    B, H1, W1, H2, W2, Kc = shape
+    A_u, A_v = (torch.ones(B, H1, W1, Kc, D, device=cuda_device) for D in (W2, H2))
+    _lib.kernel_timing(True)
+    ops.max_argmax_avg_forward(F1, F2)
+    ops.compression_forward(F1, F2, A_u, A_v)
+    report = {name: n for name, _, n in _lib.kernel_timing_report()}
+    _lib.kernel_timing(False)
+    assert report["sweep_kernel<maxavg>"] == 2 and report["sweep_kernel<compress>"] == 2 * ((Kc + 3) // 4)

@@ -15,7 +15,7 @@ TOL = 1e-3
 
 # (B, H1, W1, H2, W2, C, Kc)
 SHAPES = [
-    (1, 1, 5, 5, 97, 16, 1),        # one tile of few pixels, seven column blocks
+    (1, 1, 5, 5, 97, 16, 1),        # one tile of few pixels, four column blocks
     (1, 9, 31, 33, 65, 40, 3),      # three tiles, ragged rows and columns
     (3, 20, 27, 18, 50, 64, 6),     # several samples, two compression sweeps
     (1, 1, 148 * 128, 3, 17, 8, 2),        # exactly one wave: no tail
