@@ -14,6 +14,8 @@
  *       MA_u (B,H1,W1,2,H2)  [..,0,u] = max_v S   [..,1,u] = mean_v S
  *       MA_v (B,H1,W1,2,W2)  [..,0,v] = max_u S   [..,1,v] = mean_u S
  *       AM_u (B,H1,W1,1,H2), AM_v (B,H1,W1,1,W2)  int32 argmax, lowest index on ties
+ *     The maxima pass over entries of S that are not numbers; where a row or column has nothing else, MA_u is NaN,
+ *     MA_v is -inf, and the argmax is 0.
  *       A_u  (B,H1,W1,Kc,W2), A_v (B,H1,W1,Kc,H2) attention weights
  *       C_u  (B,H1,W1,Kc,H2) = sum_v S*A_u,  C_v (B,H1,W1,Kc,W2) = sum_u S*A_v
  *   - Outputs need no initialisation by the caller (the reference pre-fills with -inf / 0,

@@ -653,7 +653,7 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
 }
 
 // Interleaved slots of the max/avg backward (kernels.h): XU = (mean-gradient / W2, 1, max-gradient, argmax bits),
-// XV = (1, mean-gradient / H2, max-gradient, argmax bits); slots 0 and 1 of the two sides multiply to the mean terms.
+// XV = (1, mean-gradient / H2, max-gradient, argmax bits); the two mean-gradients are added, the constants are not read.
 // `scales` (FP16 operands, else null): the call's scale slots; the gradient values are then multiplied by sg * sa.
 void maxavg_slot_sources(const Dims& d, const int32_t* AM_u, const int32_t* AM_v, const float* gMA_u,
                          const float* gMA_v, SlotSources* su, SlotSources* sv, const float* scales) {
@@ -735,7 +735,7 @@ int run_attention_grads(const Dims& d, const Workspace& w, const float* gC_u, co
 
 // ---- scratch that lives in the library image, for callers that must not allocate ----
 constexpr size_t STATIC_SCRATCH_BYTES = 32u << 20;
-// The counters of the tail tiles, which the header holds beside its first 256 bytes, come on top.
+// The part of the header past its first 256 bytes comes on top: the shapes that fit stay the ones they were with a header of 256.
 constexpr size_t STATIC_ARRAY_BYTES = STATIC_SCRATCH_BYTES + WS_HEADER_BYTES - 256;
 static __device__ __align__(256) unsigned char g_static_scratch[STATIC_ARRAY_BYTES];
 

@@ -1,6 +1,6 @@
 // Gradient GEMMs of the backward ops:  gF1 = G * F2  and  gF2 = G^T * F1,  where
-// G = dLoss/dS (N1 x N2 per sample) is never stored: each 128 x 32 block of it is generated by CUDA
-// cores as the A operand of tcgen05.mma, while TMA streams the matching block of the other image's
+// G = dLoss/dS (N1 x N2 per sample) is never stored: each block of it, 128 rows x 64 (image-1-major) or 32 (image-2-major)
+// K-values, is generated by CUDA cores as the A operand of tcgen05.mma, while TMA streams the matching block of the other image's
 // features as the B operand.  The 128 x C output tile accumulates in TMEM over the whole K sweep and is
 // written once, so the result is deterministic (no atomics), unlike the reference's atomicAdd scatter
 // (MemorySaver_kernel_max_avg_argmax_backward.cu:305-310, MemorySaver_kernel_compression_backward.cu:477-488).
@@ -55,7 +55,8 @@ constexpr uint32_t GG_ACC_COLS = 256;                      // accumulator column
 
 // Ring depths.  Every kind of block has its own ring, sized by how long a stage stays in use:
 //   NY   feature blocks (B operand, 32 KB at C = 256): freed when the MMAs of the block have completed
-//   NG   generated blocks (A operand): image-1-major in TMEM columns 256 + 32*stage .., image-2-major in shared memory
+//   NG   generated blocks (A operand): image-1-major in TMEM columns 256 + 64*stage .. (32*stage with 16-bit values),
+//        image-2-major in shared memory
 //   NXU  (pixel, u) operand blocks: read row by row while the block is computed, freed when its values are stored
 //   NXV  (pixel, v) operand blocks (image-2-major only; the image-1-major form keeps those slots in registers): read
 //        into registers at the start of a block and freed at once, so that the next load has the whole computation
@@ -80,7 +81,8 @@ struct GradSmem {
   static constexpr int XU_FLOATS = (I2MAJOR ? GG_ROW_UT * GG_KJ : GG_UT * TILE_M) * Q * 4;
   static constexpr int XV_FLOATS = I2MAJOR ? GG_ROW_VT * GG_KJ * Q * 4 : 4;  // image-1-major keeps XV in registers
   float y[Cfg::NY][MAX_KB * GG_YBLOCK_BYTES / 4];  // feature stages [channel][K-values], K-major, swizzled
-  float g[AT ? 1 : Cfg::NG][AT ? 32 : TILE_M * GG_KJ];  // generated A blocks (image-2-major form), K-major, 128B swizzle
+  float g[AT ? 1 : Cfg::NG][AT ? 32 : TILE_M * GG_KJ];  // generated A blocks (image-2-major form), 128B swizzle, K-major (TF32)
+                                                        // or MN-major (16-bit)
   float xu[Cfg::NXU][XU_FLOATS];
   float xv[Cfg::NXV][XV_FLOATS];
   uint64_t y_full[Cfg::NY];
@@ -145,7 +147,8 @@ __device__ __forceinline__ void add_if_equal(float& x, int a, int b, float add) 
 
 // The part of the G values of one (pixel, u) and N (pixel, v) that is a sum of products of the two pixels' slots.
 // Max/avg group (slots 0..3 of XU: mean-gradient/W2, 1, max-gradient, argmax; of XV: 1, mean-gradient/H2,
-// max-gradient, argmax): the two mean-gradients are added.  Compression groups: every slot is a product.
+// max-gradient, argmax): the two mean-gradients are added (the constants beside them, which a product would need, are not read).
+// Columns past the image so hold the (pixel, u) mean-gradient, and meet the zero padding of the features.  Compression groups: every slot is a product.
 // Scalar multiply-adds, a slot of the (pixel, u) at a time: it stays in the operand's register port while the N columns take
 // theirs, and such a multiply-add issues every cycle.  A packed one (fma.rn.f32x2) with three different operands takes three.
 template <int MODE, int Q, int N>
@@ -435,8 +438,8 @@ __device__ float* grad_row(const GradArgs& a, const GradSched& sc, int m, size_t
   return a.out + (size_t)sc.b * C * a.d.N2() + (size_t)u * a.d.W2 + v;
 }
 // Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][channel][128 rows] or [tail][piece - 1][128 rows][channel], as the
-// output has it, so that the fold reads both in runs (channel-major pieces under a pixel-major output, 16-byte accesses 1 KB
-// apart, made the launch for 1 x 55 x 128 against 27 x 64 take 58 us; 47 now, 48 with whole tiles).
+// output has it, so that the fold reads both in runs (with channel-major pieces under a pixel-major output, 16-byte accesses 1 KB
+// apart, the form that folded in the tile's last CTA took 58 instead of 47 us for 1 x 55 x 128 against 27 x 64).
 __device__ __forceinline__ float* grad_part(const GradArgs& a, int tail, int piece) {
   return a.part + ((size_t)tail * (a.pieces - 1) + piece - 1) * a.d.C * TILE_M;
 }

@@ -129,8 +129,8 @@ TileSplit sweep_split(const Dims& d, int slots, bool sums);
 // TMA box row, and conflict-free 16-byte shared-memory reads after a TMA copy.
 //   GRAD_COMPRESS: G[p,u,v] = sum_r XU[u,p,r] * XV[v,p,r]            (2 slots per channel, zero padded)
 //   GRAD_MAXAVG  : XU slots (mean-gradient / W2, 1, max-gradient, argmax bits), XV slots (1, mean-gradient / H2,
-//                  max-gradient, argmax bits), so that slots 0 and 1 multiply to the two mean terms:
-//                  G[p,u,v] = XU[u,p,0]*XV[v,p,0] + XU[u,p,1]*XV[v,p,1]
+//                  max-gradient, argmax bits); the mean terms are added, the constants are not read:
+//                  G[p,u,v] = XU[u,p,0] + XV[v,p,1]
 //                             + (XU[u,p,3]==v ? XU[u,p,2] : 0) + (XV[v,p,3]==u ? XV[v,p,2] : 0)
 //   GRAD_FUSED   : group 0 as GRAD_MAXAVG, groups 1.. as GRAD_COMPRESS; G is the sum of both
 struct GradArgs {

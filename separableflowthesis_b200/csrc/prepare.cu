@@ -549,7 +549,7 @@ cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, i
   return cudaGetLastError();
 }
 
-// Clears the workspace header (status word, scale slots, counters) and, for FP16 operands, finds the two feature scales.
+// Clears the workspace header (status word, scale slots) and, for FP16 operands, finds the two feature scales.
 static cudaError_t begin_prepare(const Dims& d, const float* F1, const float* F2, float premul1, int* status, int op16,
                                  float* scales, cudaStream_t stream) {
   cudaError_t err = cudaMemsetAsync(status, 0, WS_HEADER_CLEAR_BYTES, stream);

@@ -275,24 +275,8 @@ __device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4])
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// 32 / 64 consecutive columns; the wait is part of the same asm statement so that no use of the
+// 64 consecutive columns; the wait is part of the same asm statement so that no use of the
 // destination registers can be scheduled between the load and its completion.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
 __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
   uint32_t r[64];
   asm volatile(
@@ -356,10 +340,7 @@ __device__ __forceinline__ void set_max_registers() {
   else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// Named barriers (ids 1..15; id 0 is __syncthreads): one warpgroup signals, the other waits.
-__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
+// Named barrier (ids 1..15; id 0 is __syncthreads).
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -442,7 +423,7 @@ __device__ __forceinline__ float sum2(uint64_t v) {
 }
 
 // Four consecutive floats of which the first n exist (n < 1: none), as one 16-byte access when all do and the address allows
-// it.  Loads bypass L1, so that they see what other SMs stored.
+// it.  Loads bypass L1: they are read once.
 __device__ __forceinline__ float4 load4_cg(const float* p, int n) {
   if (n >= 4 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) return __ldcg(reinterpret_cast<const float4*>(p));
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -463,12 +444,5 @@ __device__ __forceinline__ void store4(float* p, const float4& v, int n) {
   if (n > 3) p[3] = v.w;
 }
 __device__ __forceinline__ void add4(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
-
-// Byte offset of element (row, col) inside a [rows][32 fp32] tile stored with the 128-byte swizzle
-// (16-byte chunk index XOR row mod 8); the tile base must be 1024-byte aligned.
-__device__ __forceinline__ uint32_t sw128_offset(int row, int col) {
-  return static_cast<uint32_t>(row) * 128u + (((static_cast<uint32_t>(col) >> 2) ^ (static_cast<uint32_t>(row) & 7u)) << 4) +
-         ((static_cast<uint32_t>(col) & 3u) << 2);
-}
 
 }  // namespace sfb
