@@ -82,17 +82,19 @@ def test_a_sample_alone_and_in_a_batch(D, cuda_device):
         assert relerr(gx[:1], r_gx) < TOL
 
 
-@pytest.mark.parametrize("H1,W1,D,Kc", [(55, 128, 128, 4), (55, 128, 55, 1), (135, 240, 135, 3), (135, 240, 240, 4)])
-def test_repeated_calls_agree(H1, W1, D, Kc, cuda_device):
-    """Many planes through the rings of the tiled forms, on many blocks at once: the same bits every time."""
+@pytest.mark.parametrize("H1,W1,H2,W2,Kc", [(55, 128, 55, 128, 4), (55, 128, 20, 9, 1), (135, 240, 33, 135, 3), (135, 240, 135, 240, 2)])
+def test_tiles_agree_between_repeated_calls(H1, W1, H2, W2, Kc, cuda_device):
+    """Many planes through the rings of the tiled kernels (level calls on widths that are multiples of 4), on many blocks at once:
+    the same weights, and the same gradients that pass through them, every time."""
     g = torch.Generator(device=cuda_device).manual_seed(9)
     randn = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
-    x, weight, bias = randn(2, 2, D, H1, W1), randn(Kc, 2, 3, 3, 3) * 0.3, randn(Kc)
-    ga, add = randn(2, Kc, D, H1, W1), randn(2, 2, D, H1, W1)
+    F1, F2 = randn(2, H1, W1, 16) / 4, randn(2, H2, W2, 16)
+    w_u, b_u, w_v, b_v = randn(Kc, 2, 3, 3, 3) * 0.3, randn(Kc), randn(Kc, 2, 3, 3, 3) * 0.3, randn(Kc)
+    g_u, g_v = randn(2, 2 + Kc, W2, H1, W1), randn(2, 2 + Kc, H2, H1, W1)
 
     def run():
-        a = ops.attention_forward(x, weight, bias)
-        return [a, *ops.attention_backward(x, weight, a, ga.clone(), add)]
+        level = ops.separation_level_forward(F1, F2, w_u, b_u, w_v, b_v)
+        return level + ops.separation_level_backward(F1, F2, w_u, w_v, *level, g_u, g_v)
 
     first = run()
     for _ in range(6):
