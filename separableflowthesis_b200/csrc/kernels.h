@@ -111,8 +111,8 @@ struct TileSplit { int tiles, whole_tiles, pieces, parts; size_t part_floats; };
 // depend on the batch or the row range.  A narrow tile takes as long as a wide one for max (/ arg-max) and 1.36 (two channels) to
 // 1.6 (four) times as long for the sums.  4 x 55 x 128 against 128 x 16, wide and narrow (us): maxima with arg-max 109 and 57,
 // sums of two and four channels 66 and 42, 83 and 61; against 128 x 48: 155 and 117, 112 and 115, 164 and 197.
-// What is left to the other side of the line: wide sums over 2 x 48 x 64 against 64 x 48, which narrow blocks would cut into three
-// pieces instead of two, 26 and 35 us where 24 and 33 are possible.
+// What the line costs: sums over 2 x 48 x 64 against 64 x 48, where three narrow blocks cut the tail better than two wide ones, take
+// 26 and 35 us instead of 20 and 30.
 __host__ __device__ inline bool sweep_narrow(const Dims& d, bool sums) {
   const int wide = ((d.H2 + SWEEP_UT - 1) / SWEEP_UT) * ((d.W2 + SWEEP_VT - 1) / SWEEP_VT);
   const int narrow = ((d.H2 + SWEEP_UT_NARROW - 1) / SWEEP_UT_NARROW) * ((d.W2 + SWEEP_VT_NARROW - 1) / SWEEP_VT_NARROW);
