@@ -256,6 +256,27 @@ int sfb_lookup_backward(const float* gout, const float* coord, int64_t coord_bat
                         float* gpyramid, int32_t B, int32_t dim, int32_t D, int32_t H1, int32_t W1, int32_t levels,
                         int32_t radius, int32_t clamp_unit, void* stream);
 
+/* The same for both aggregated volumes of a model, which share B, dim, H1, W1, levels and radius: one launch for the two.
+ * corr1 (B,dim,D1,H1,W1) is read with component 0 of the coordinates (B,2,H1,W1) and clamped positions, corr2
+ * (B,dim,D2,H1,W1) with component 1, `coords_component_stride` elements further, and positions as they are. */
+int sfb_lookup_build_pyramid_pair(const float* corr1, float* pyramid1, const float* corr2, float* pyramid2, int32_t B,
+                                  int32_t dim, int32_t D1, int32_t D2, int32_t H1, int32_t W1, int32_t levels, void* stream);
+int sfb_lookup_forward_pair(const float* corr1, const float* pyramid1, const float* corr2, const float* pyramid2,
+                            const float* coords, int64_t coords_batch_stride, int64_t coords_component_stride, float* out1,
+                            float* out2, int32_t B, int32_t dim, int32_t D1, int32_t D2, int32_t H1, int32_t W1, int32_t levels,
+                            int32_t radius, void* stream);
+/* Gradients of several lookups on the same volumes: every lookup adds the gradients of its windows to an accumulator per
+ * volume (sfb_lookup_accumulator_bytes() bytes, zeroed by the caller before the first), sfb_lookup_fold_gradient then
+ * overwrites gcorr (B,dim,D,H1,W1) with the gradient of the volume.  gout1 / acc1 or gout2 / acc2 may be NULL, both of a
+ * pair: that volume is left out.  No atomics: the sum of the calls in their order. */
+size_t sfb_lookup_accumulator_bytes(int32_t B, int32_t dim, int32_t D, int32_t H1, int32_t W1, int32_t levels,
+                                    int32_t clamp_unit);
+int sfb_lookup_accumulate_pair(const float* gout1, const float* gout2, const float* coords, int64_t coords_batch_stride,
+                               int64_t coords_component_stride, float* acc1, float* acc2, int32_t B, int32_t dim, int32_t D1,
+                               int32_t D2, int32_t H1, int32_t W1, int32_t levels, int32_t radius, void* stream);
+int sfb_lookup_fold_gradient(const float* acc, float* gcorr, int32_t B, int32_t dim, int32_t D, int32_t H1, int32_t W1,
+                             int32_t levels, int32_t clamp_unit, void* stream);
+
 /* Lookup on the 4D correlation volume without storing it: the call the reference's memory-saving block leaves
  * unimplemented (core/corr.py:491-510 raises NotImplementedError, then sketches
  * alt_cuda_corr.forward(fmap1, fmap2_l, coords / 2^l, radius) per level; alt_cuda_corr is RAFT's extension and is not

@@ -44,7 +44,8 @@ EXPORTED_SYMBOLS = (
     "sfb_separation_level_forward_fmaps", "sfb_separation_level_backward_fmaps",
     "sfb_upsample_displacement", "sfb_upsample_displacement_backward", "sfb_lookup_pyramid_bytes",
     "sfb_set_sweep_operands", "sfb_get_sweep_operands", "sfb_lookup_build_pyramid", "sfb_lookup_forward", "sfb_lookup_backward",
-    "sfb_lookup4d_forward", "sfb_lookup4d_backward", "sfb_debug_wait_timeout",
+    "sfb_lookup4d_forward", "sfb_lookup4d_backward", "sfb_debug_wait_timeout", "sfb_lookup_build_pyramid_pair",
+    "sfb_lookup_forward_pair", "sfb_lookup_accumulator_bytes", "sfb_lookup_accumulate_pair", "sfb_lookup_fold_gradient",
 )
 
 
@@ -103,6 +104,16 @@ def load() -> ctypes.CDLL:
     lib.sfb_lookup_forward.argtypes = [P, P, P, I64, P] + [I32] * 8 + [P]
     lib.sfb_lookup_backward.restype = ctypes.c_int
     lib.sfb_lookup_backward.argtypes = [P, P, I64, P, P] + [I32] * 8 + [P]
+    lib.sfb_lookup_build_pyramid_pair.restype = ctypes.c_int
+    lib.sfb_lookup_build_pyramid_pair.argtypes = [P] * 4 + [I32] * 7 + [P]
+    lib.sfb_lookup_forward_pair.restype = ctypes.c_int
+    lib.sfb_lookup_forward_pair.argtypes = [P] * 5 + [I64, I64, P, P] + [I32] * 8 + [P]
+    lib.sfb_lookup_accumulator_bytes.restype = SZ
+    lib.sfb_lookup_accumulator_bytes.argtypes = [I32] * 7
+    lib.sfb_lookup_accumulate_pair.restype = ctypes.c_int
+    lib.sfb_lookup_accumulate_pair.argtypes = [P] * 3 + [I64, I64, P, P] + [I32] * 8 + [P]
+    lib.sfb_lookup_fold_gradient.restype = ctypes.c_int
+    lib.sfb_lookup_fold_gradient.argtypes = [P, P] + [I32] * 7 + [P]
     lib.sfb_lookup4d_forward.restype = ctypes.c_int
     lib.sfb_lookup4d_forward.argtypes = [P, P, P, P, I32, P, P] + [I32] * 5 + [ctypes.c_float, P]
     lib.sfb_lookup4d_backward.restype = ctypes.c_int

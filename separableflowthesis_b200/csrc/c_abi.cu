@@ -1408,6 +1408,8 @@ static int check_lookup_dims(int B, int dim, int D, int H1, int W1, int levels, 
   return SFB_OK;
 }
 
+static int lookup_pyramid_launches(int levels) { return (levels + 1) / 3; }   // three levels from one
+
 size_t sfb_lookup_pyramid_bytes(int32_t B, int32_t dim, int32_t D, int32_t H1, int32_t W1, int32_t levels) {
   LookupDims ld;
   if (check_lookup_dims(B, dim, D, H1, W1, levels, 0, &ld) != SFB_OK) return 0;
@@ -1421,7 +1423,7 @@ int sfb_lookup_build_pyramid(const float* corr, float* pyramid, int32_t B, int32
   if (corr == nullptr || (levels > 1 && pyramid == nullptr))
     return fail(SFB_ERR_INVALID_ARGUMENT, "corr and pyramid must not be NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SFB_CUDA(timed(KID_LOOKUP, levels - 1, st, [&] { return launch_lookup_pyramid(ld, corr, pyramid, st); }));
+  SFB_CUDA(timed(KID_LOOKUP, lookup_pyramid_launches(levels), st, [&] { return launch_lookup_pyramid(ld, corr, pyramid, st); }));
   return SFB_OK;
 }
 
@@ -1434,7 +1436,7 @@ int sfb_lookup_forward(const float* corr, const float* pyramid, const float* coo
     return fail(SFB_ERR_INVALID_ARGUMENT, "corr, pyramid, coord and out must not be NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SFB_CUDA(timed(KID_LOOKUP, 1, st, [&] {
-    return launch_lookup_forward(ld, corr, pyramid, coord, coord_batch_stride, out, clamp_unit, st);
+    return launch_lookup_forward(ld, LookupCall{corr, pyramid, coord, coord_batch_stride, out, clamp_unit}, st);
   }));
   return SFB_OK;
 }
@@ -1450,6 +1452,73 @@ int sfb_lookup_backward(const float* gout, const float* coord, int64_t coord_bat
   SFB_CUDA(timed(KID_LOOKUP, levels > 1 ? 2 : 1, st, [&] {
     return launch_lookup_backward(ld, gout, coord, coord_batch_stride, gcorr, gpyramid, clamp_unit, st);
   }));
+  return SFB_OK;
+}
+
+// ---- both aggregated volumes of a model at once ----
+static int check_lookup_pair(int B, int dim, int D1, int D2, int H1, int W1, int levels, int radius, LookupDims (&ld)[2]) {
+  SFB_TRY(check_lookup_dims(B, dim, D1, H1, W1, levels, radius, &ld[0]));
+  return check_lookup_dims(B, dim, D2, H1, W1, levels, radius, &ld[1]);
+}
+
+int sfb_lookup_build_pyramid_pair(const float* corr1, float* pyramid1, const float* corr2, float* pyramid2, int32_t B,
+                                  int32_t dim, int32_t D1, int32_t D2, int32_t H1, int32_t W1, int32_t levels, void* stream) {
+  LookupDims ld[2];
+  SFB_TRY(check_lookup_pair(B, dim, D1, D2, H1, W1, levels, 0, ld));
+  if (corr1 == nullptr || corr2 == nullptr || (levels > 1 && (pyramid1 == nullptr || pyramid2 == nullptr)))
+    return fail(SFB_ERR_INVALID_ARGUMENT, "corr1, corr2, pyramid1 and pyramid2 must not be NULL");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  SFB_CUDA(timed(KID_LOOKUP, lookup_pyramid_launches(levels), st,
+                 [&] { return launch_lookup_pyramid_pair(ld, {corr1, corr2}, {pyramid1, pyramid2}, st); }));
+  return SFB_OK;
+}
+
+int sfb_lookup_forward_pair(const float* corr1, const float* pyramid1, const float* corr2, const float* pyramid2,
+                            const float* coords, int64_t coords_batch_stride, int64_t coords_component_stride, float* out1,
+                            float* out2, int32_t B, int32_t dim, int32_t D1, int32_t D2, int32_t H1, int32_t W1, int32_t levels,
+                            int32_t radius, void* stream) {
+  LookupDims ld[2];
+  SFB_TRY(check_lookup_pair(B, dim, D1, D2, H1, W1, levels, radius, ld));
+  if (corr1 == nullptr || corr2 == nullptr || (levels > 1 && (pyramid1 == nullptr || pyramid2 == nullptr)) || coords == nullptr ||
+      out1 == nullptr || out2 == nullptr)
+    return fail(SFB_ERR_INVALID_ARGUMENT, "corr1, corr2, pyramid1, pyramid2, coords, out1 and out2 must not be NULL");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const LookupCall calls[2] = {{corr1, pyramid1, coords, coords_batch_stride, out1, 1},
+                               {corr2, pyramid2, coords + coords_component_stride, coords_batch_stride, out2, 0}};
+  SFB_CUDA(timed(KID_LOOKUP, 1, st, [&] { return launch_lookup_forward_pair(ld, calls, st); }));
+  return SFB_OK;
+}
+
+size_t sfb_lookup_accumulator_bytes(int32_t B, int32_t dim, int32_t D, int32_t H1, int32_t W1, int32_t levels,
+                                    int32_t clamp_unit) {
+  LookupDims ld;
+  if (check_lookup_dims(B, dim, D, H1, W1, levels, 0, &ld) != SFB_OK) return 0;
+  return lookup_accumulator_floats(ld, clamp_unit) * sizeof(float);
+}
+
+int sfb_lookup_accumulate_pair(const float* gout1, const float* gout2, const float* coords, int64_t coords_batch_stride,
+                               int64_t coords_component_stride, float* acc1, float* acc2, int32_t B, int32_t dim, int32_t D1,
+                               int32_t D2, int32_t H1, int32_t W1, int32_t levels, int32_t radius, void* stream) {
+  LookupDims ld[2];
+  SFB_TRY(check_lookup_pair(B, dim, D1, D2, H1, W1, levels, radius, ld));
+  if (coords == nullptr || (gout1 == nullptr) != (acc1 == nullptr) || (gout2 == nullptr) != (acc2 == nullptr) ||
+      (gout1 == nullptr && gout2 == nullptr))
+    return fail(SFB_ERR_INVALID_ARGUMENT, "coords and at least one volume's output gradient and accumulator are needed");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const LookupGradient g[2] = {{gout1, coords, coords_batch_stride, acc1, 1},
+                               {gout2, coords + coords_component_stride, coords_batch_stride, acc2, 0}};
+  const int first = gout1 != nullptr ? 0 : 1, volumes = gout1 != nullptr && gout2 != nullptr ? 2 : 1;
+  SFB_CUDA(timed(KID_LOOKUP, 1, st, [&] { return launch_lookup_accumulate(ld + first, g + first, volumes, st); }));
+  return SFB_OK;
+}
+
+int sfb_lookup_fold_gradient(const float* acc, float* gcorr, int32_t B, int32_t dim, int32_t D, int32_t H1, int32_t W1,
+                             int32_t levels, int32_t clamp_unit, void* stream) {
+  LookupDims ld;
+  SFB_TRY(check_lookup_dims(B, dim, D, H1, W1, levels, 0, &ld));
+  if (acc == nullptr || gcorr == nullptr) return fail(SFB_ERR_INVALID_ARGUMENT, "acc and gcorr must not be NULL");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  SFB_CUDA(timed(KID_LOOKUP, 1, st, [&] { return launch_lookup_gradient_fold(ld, acc, gcorr, clamp_unit, st); }));
   return SFB_OK;
 }
 

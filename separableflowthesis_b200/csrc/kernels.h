@@ -297,8 +297,28 @@ struct LookupDims {
 };
 size_t lookup_pyramid_floats(const LookupDims& d);
 [[nodiscard]] cudaError_t launch_lookup_pyramid(const LookupDims& d, const float* corr, float* pyramid, cudaStream_t stream);
-[[nodiscard]] cudaError_t launch_lookup_forward(const LookupDims& d, const float* corr, const float* pyramid, const float* coord,
-                                  long long coord_sb, float* out, int clamp_unit, cudaStream_t stream);
+struct LookupCall {
+  const float *corr, *pyramid, *coord;
+  long long coord_sb;
+  float* out;
+  int clamp_unit;
+};
+[[nodiscard]] cudaError_t launch_lookup_forward(const LookupDims& d, const LookupCall& c, cudaStream_t stream);
+// The same for two volumes that differ in D alone, in one launch.
+[[nodiscard]] cudaError_t launch_lookup_pyramid_pair(const LookupDims (&d)[2], const float* const (&corr)[2], float* const (&pyramid)[2],
+                                       cudaStream_t stream);
+[[nodiscard]] cudaError_t launch_lookup_forward_pair(const LookupDims (&d)[2], const LookupCall (&c)[2], cudaStream_t stream);
+// Gradients of several lookups: each adds the gradients of its windows to the accumulator of its volume (zero before the first),
+// for one or two volumes that differ in D alone; the accumulator is then folded into the gradient of the volume.
+struct LookupGradient {
+  const float *gout, *coord;
+  long long coord_sb;
+  float* acc;
+  int clamp_unit;
+};
+size_t lookup_accumulator_floats(const LookupDims& d, int clamp_unit);
+[[nodiscard]] cudaError_t launch_lookup_accumulate(const LookupDims* d, const LookupGradient* g, int volumes, cudaStream_t stream);
+[[nodiscard]] cudaError_t launch_lookup_gradient_fold(const LookupDims& d, const float* acc, float* gcorr, int clamp_unit, cudaStream_t stream);
 // gcorr and gpyramid (same sizes as corr / pyramid) are overwritten; gpyramid is scratch.
 [[nodiscard]] cudaError_t launch_lookup_backward(const LookupDims& d, const float* gout, const float* coord, long long coord_sb,
                                    float* gcorr, float* gpyramid, int clamp_unit, cudaStream_t stream);

@@ -340,6 +340,77 @@ class LookupFunction(Function):
         return gcorr, None, None, None, None, None
 
 
+# A refinement looks up a dozen times on the same two volumes.  Gradients of the volumes themselves, one per lookup, would each be
+# written whole and then added up by autograd.  Instead every lookup takes an edge to its volume (a tensor that stands for
+# the volume's accumulator and holds nothing) and hands it on to the next: in the backward the accumulator comes down that
+# chain, each lookup adds its windows to it, and the volume's node folds it into the gradient, once.
+class LookupVolumeFunction(Function):
+    """Start of a volume's chain: ``apply(corr, levels, clamp_unit)`` -> edge."""
+
+    @staticmethod
+    def forward(ctx, corr, levels, clamp_unit):
+        ctx.cfg = (tuple(corr.shape), levels, clamp_unit)
+        ctx.set_materialize_grads(False)
+        return torch.empty_strided((MemorySaver.lookup_accumulator_size(corr.shape, levels, clamp_unit),), (0,), dtype=corr.dtype,
+                                   device=corr.device)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, acc):
+        if acc is None:
+            return None, None, None
+        shape, levels, clamp_unit = ctx.cfg
+        with torch.cuda.device_of(acc):
+            return MemorySaver.lookup_fold_gradient(acc.contiguous(), shape, levels, clamp_unit), None, None
+
+
+class LookupPairFunction(Function):
+    """Lookup on both volumes: ``apply(corr1, corr2, pyramid1, pyramid2, coords, edge1, edge2, levels, radius)`` -> (out1, out2,
+    edge1, edge2).  An edge is None where the volume needs no gradient."""
+
+    @staticmethod
+    def forward(ctx, corr1, corr2, pyramid1, pyramid2, coords, edge1, edge2, levels, radius):
+        with torch.cuda.device_of(corr1):
+            out1, out2 = MemorySaver.lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels, radius)
+        if edge1 is not None or edge2 is not None:
+            ctx.save_for_backward(coords)
+            ctx.cfg = (tuple(corr1.shape), tuple(corr2.shape), levels, radius)
+            ctx.set_materialize_grads(False)
+            if edge1 is None:
+                ctx.mark_non_differentiable(out1)
+            elif edge2 is None:
+                ctx.mark_non_differentiable(out2)
+        return out1, out2, edge1, edge2
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g1, g2, acc1, acc2):
+        # An accumulator belongs to this chain alone (its edges go from lookup to lookup), so it is added to in place.  A lookup
+        # whose outputs are not part of the loss hands it on; its saved tensors may be gone by then.
+        shape1, shape2, levels, radius = ctx.cfg
+        if not ctx.needs_input_grad[5]:
+            g1 = None
+        if not ctx.needs_input_grad[6]:
+            g2 = None
+        if g1 is not None or g2 is not None:
+            (coords,) = ctx.saved_tensors
+            with torch.cuda.device_of(coords):
+                if g1 is not None:
+                    g1 = g1.contiguous()
+                    acc1 = _lookup_accumulator(acc1, shape1, levels, True, g1)
+                if g2 is not None:
+                    g2 = g2.contiguous()
+                    acc2 = _lookup_accumulator(acc2, shape2, levels, False, g2)
+                MemorySaver.lookup_accumulate_pair(shape1, shape2, coords, g1, g2, acc1, acc2, levels, radius)
+        return None, None, None, None, None, acc1, acc2, None, None
+
+
+def _lookup_accumulator(acc, shape, levels, clamp_unit, like):
+    if acc is not None:
+        return acc.contiguous()
+    return like.new_zeros(MemorySaver.lookup_accumulator_size(shape, levels, clamp_unit))
+
+
 class Lookup4dFunction(Function):
     """Lookup on the 4D correlation volume without storing it.  ``apply(coords, radius, scale, F1, *F2_levels)`` with
     channels-last features -> (B, levels*(2r+1)^2, H1, W1); gradients for the features only (the model detaches
