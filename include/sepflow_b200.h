@@ -222,6 +222,21 @@ int sfb_separation_level_backward_fmaps(const float* fmap1, const float* fmap2, 
                                         float* gbias_u, float* gweight_v, float* gbias_v, const sfb_shape* shape,
                                         void* workspace, size_t workspace_bytes, void* stream);
 
+/* All pyramid levels of the call site (core/corr.py:416-475), at most 4 of them and at most 4 attention channels: every kernel of
+ * the level calls above runs once for all levels.  fmap1 (B,C,H1,W1), fmap2[l] (B,C,H2[l],W2[l]) are the model's feature maps
+ * (host arrays of `levels` entries; no level larger than level 0), `shape` gives B, H1, W1, C and Kc; the other arguments as
+ * above.  SEP_u (B,(2+Kc)*levels,W2[0],H1,W1) and SEP_v (B,(2+Kc)*levels,H2[0],H1,W1) are the concatenated outputs, each level
+ * resampled to the displacement range of level 0.  `saved` (256-byte aligned) receives what a backward needs: the levels' own
+ * volumes, attention weights and, with_argmax != 0, arg-max indices. */
+size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
+                                          int32_t with_argmax);
+size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels);
+int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
+                                   int32_t levels, float scale1, const float* weight_u, const float* bias_u,
+                                   const float* weight_v, const float* bias_v, float* SEP_u, float* SEP_v, void* saved,
+                                   size_t saved_bytes, int32_t with_argmax, const sfb_shape* shape, void* workspace,
+                                   size_t workspace_bytes, void* stream);
+
 /* Placement of one pyramid level's volumes into the concatenated outputs of the call site (core/corr.py:459-475:
  * F.interpolate(..., [D0,H1,W1], mode='trilinear', align_corners=True), then torch.cat over levels).  H1, W1 do not
  * change, so this is linear interpolation along the displacement axis, with torch's arithmetic.

@@ -16,12 +16,17 @@
 //    costs a 32-lane register write per weight, more than the FMA they feed; instead the weights of the (up to
 //    four) channels being processed are staged in __constant__ memory, where an FMA reads them as an operand.
 //
+// A launch works through a list of jobs: the two modules of a level, or those of all levels of a pyramid.  A module is a compile-time
+// index into the constant memory, so every walk is there once per module.
+//
 //   forward     : logits -> A (the stencil kernel parks the raw logits in A, where they are normalised in place)
 //   logit grads : gL = A * (gA - sum_d gA*A), in place over gA; per-block sums of gL for the bias gradient
 //   input grads : gX = transposed stencil of gL (+ an optional addend: the direct gradient of the max/avg channels)
 //   weight grads: gW[k,c,tap] = sum X(shifted by tap) * gL, per-block partial sums, reduced in a fixed order by
 //                 a second kernel (bit-reproducible; no floating-point atomics)
+#include <climits>
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.h"
 #include "sm100_primitives.cuh"
@@ -32,8 +37,26 @@ constexpr int AT_THREADS = 128;
 constexpr int AT_TAPS = 27;
 constexpr int AT_KC = 4;  // channels per launch of the forward / logit-gradient kernels and per constant-memory stage
 
-// Filter weights (k, c, td, th, tw) of the channels the running kernel works on.
-__constant__ float c_att_weights[AT_KC * 2 * AT_TAPS];
+// Filter weights (k, c, td, th, tw) of the channels the running kernel works on, of both modules.
+constexpr int AT_WEIGHTS = AT_KC * 2 * AT_TAPS;
+__constant__ float c_att_weights[2 * AT_WEIGHTS];
+
+// Jobs of a launch: blocks first[j] .. first[j+1]-1 belong to job j.
+struct JobBlocks {
+  int first[MAX_ATTENTION_JOBS + 1];
+};
+__device__ __forceinline__ int job_of(const JobBlocks& jb, int block) {
+  int job = 0;
+#pragma unroll
+  for (int j = 1; j < MAX_ATTENTION_JOBS; ++j) job = block >= jb.first[j] ? j : job;
+  return job;
+}
+// f(integral constant) with the job's module
+template <class F>
+__device__ __forceinline__ void by_module(int module, F&& f) {
+  if (module == 0) f(std::integral_constant<int, 0>{});
+  else f(std::integral_constant<int, 1>{});
+}
 
 // Offsets of the 3x3 neighbourhood of pixel (h, w) inside a plane, and which of them exist.
 struct Neighbourhood {
@@ -81,7 +104,7 @@ struct PlaneRing {
 // AT_SOFT_MAX displacements walked in one piece is normalised at its end (SOFT, softmax_column): there the launch and the
 // idle warps of the other kernel cost more than the exponentials (8 x 47 x 156, four channels, D = 5, 8 and 16: 30, 36 and 44 us
 // with it, 21, 26 and 37 without).
-// Gather form: grid (ceil(N1/128), B * pieces), block 128.  Channels k0 .. k0+KC-1 of Kc, weights in c_att_weights.
+// Gather form: grid of ceil(N1/128) * B * pieces blocks per job, block 128.  Channels k0 .. k0+KC-1 of Kc, weights in c_att_weights.
 constexpr int FW_STAGES = 4;
 constexpr int AT_SOFT_MAX = 16;
 
@@ -113,23 +136,30 @@ __device__ __forceinline__ void softmax_column(float* col, int D, size_t plane) 
     if (d < D) col[d * plane] = v[d] * inv;
 }
 
-template <int KC, bool SOFT>
-__global__ void __launch_bounds__(AT_THREADS)
-attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float* __restrict__ bias,
-                        float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1) {
-  __shared__ float ring_mem[FW_STAGES * 18 * AT_THREADS];
-  const int N1 = H1 * W1;
-  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y % B, d0 = (blockIdx.y / B) * dc;
+struct LogitsJobs {
+  JobBlocks blocks;
+  struct Job {
+    const float* x;
+    long long x_sb;
+    const float* bias;
+    float* a;
+    int D, dc, module;
+  } j[MAX_ATTENTION_JOBS];
+};
+
+template <int KC, int MODULE>
+__device__ __forceinline__ void logits_walk_gather(const LogitsJobs::Job& job, float* ring_mem, int Kc, int k0, int b, int d0, int p,
+                                                   int H1, int W1) {
+  const int N1 = H1 * W1, D = job.D, dc = job.dc;
   const int d1 = min(d0 + dc, D);                              // this block's logits: d0 <= d < d1
   const int e0 = max(d0 - 1, 0), e1 = min(d1 + 1, D);          // the planes they need
-  if (p >= N1) return;
   const int h = p / W1, w = p - h * W1;
   const Neighbourhood nb(h, w, H1, W1);
   const PlaneRing<18, FW_STAGES> ring(ring_mem);
   const size_t plane = (size_t)N1;
-  const float* x0 = x + (size_t)b * x_sb + p;       // channel 0, plane 0
+  const float* x0 = job.x + (size_t)b * job.x_sb + p;       // channel 0, plane 0
   const float* x1 = x0 + (size_t)D * plane;         // channel 1
-  float* out = a + ((size_t)b * Kc + k0) * D * plane + p;
+  float* out = job.a + ((size_t)b * Kc + k0) * D * plane + p;
 
   auto issue = [&](int e) {  // neighbourhoods of plane e (both channels) -> stage e % FW_STAGES
     if (e < e1) {
@@ -148,7 +178,7 @@ attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float
   float bk[KC], acc[3][KC];
 #pragma unroll
   for (int k = 0; k < KC; ++k) {
-    bk[k] = __ldg(bias + k0 + k);
+    bk[k] = __ldg(job.bias + k0 + k);
     acc[0][k] = acc[1][k] = acc[2][k] = bk[k];
   }
   auto emit = [&](int d) {  // logit d is complete in acc[0]
@@ -168,9 +198,9 @@ attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float
         const float xv = *ring.slot(s, c * 9 + n);
 #pragma unroll
         for (int k = 0; k < KC; ++k) {
-          acc[2][k] = fmaf(xv, c_att_weights[(k * 2 + c) * AT_TAPS + n], acc[2][k]);
-          acc[1][k] = fmaf(xv, c_att_weights[(k * 2 + c) * AT_TAPS + 9 + n], acc[1][k]);
-          acc[0][k] = fmaf(xv, c_att_weights[(k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
+          acc[2][k] = fmaf(xv, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + n], acc[2][k]);
+          acc[1][k] = fmaf(xv, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 9 + n], acc[1][k]);
+          acc[0][k] = fmaf(xv, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
         }
       }
     if (e > d0) emit(e - 1);
@@ -178,10 +208,28 @@ attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float
     for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
   }
   if (d1 == D) emit(D - 1);
-  if constexpr (SOFT) {
+}
+
+// SOFT: the walks end with the softmax of their columns.
+template <int KC>
+__device__ __forceinline__ void softmax_columns(const LogitsJobs::Job& job, int Kc, int k0, int b, int p, size_t plane) {
+  float* const out = job.a + ((size_t)b * Kc + k0) * job.D * plane + p;
 #pragma unroll 1
-    for (int k = 0; k < KC; ++k) softmax_column(out + (size_t)k * D * plane, D, plane);
-  }
+  for (int k = 0; k < KC; ++k) softmax_column(out + (size_t)k * job.D * plane, job.D, plane);
+}
+
+template <int KC, bool SOFT>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_logits_kernel(const __grid_constant__ LogitsJobs jobs, int Kc, int k0, int B, int H1, int W1) {
+  __shared__ float ring_mem[FW_STAGES * 18 * AT_THREADS];
+  const int ji = job_of(jobs.blocks, blockIdx.x);
+  const LogitsJobs::Job& job = jobs.j[ji];
+  const int N1 = H1 * W1, pb = (N1 + AT_THREADS - 1) / AT_THREADS;
+  const int r = blockIdx.x - jobs.blocks.first[ji], z = r / pb;
+  const int p = (r - z * pb) * AT_THREADS + threadIdx.x, b = z % B, d0 = (z / B) * job.dc;
+  if (p >= N1) return;
+  by_module(job.module, [&](auto m) { logits_walk_gather<KC, decltype(m)::value>(job, ring_mem, Kc, k0, b, d0, p, H1, W1); });
+  if (SOFT) softmax_columns<KC>(job, Kc, k0, b, p, (size_t)N1);
 }
 
 // ---- logits, pixel tiles fetched by TMA -----------------------------------------------------------------
@@ -191,7 +239,7 @@ attention_logits_kernel(const float* __restrict__ x, long long x_sb, const float
 // convolution's zero padding), and the 128 pixel threads read their 18 neighbours from shared memory at constant
 // offsets.  Against the gather above this removes the 18 per-thread copies per plane and their address arithmetic,
 // which were a third of the instructions of an issue-bound kernel.  Needs W1 % 4 == 0 (TMA strides are multiples of
-// 16 bytes).  grid (ceil(W1/32), ceil(H1/4), B * pieces), block 128 + 32.
+// 16 bytes).  grid of ceil(W1/32) * ceil(H1/4) * B * pieces blocks per job, block 128 + 32.
 constexpr int AT_TW = 32, AT_TH = 4;
 constexpr int AT_BOX_W = AT_TW + 8, AT_BOX_H = AT_TH + 2;
 constexpr int AT_TSTAGES = 6;
@@ -211,45 +259,43 @@ struct AttentionTileSmem {
   WaitCtl ctl;
 };
 
-template <int KC, bool SOFT>
-__global__ void __launch_bounds__(AT_THREADS + 32)
-attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const float* __restrict__ bias,
-                              float* __restrict__ a, int Kc, int k0, int B, int D, int dc, int H1, int W1,
-                              int* status) {
-  if (!cta_has_work(status)) return;
-  __shared__ __align__(128) AttentionTileSmem<2> sm;
-  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z % B, d0 = (blockIdx.z / B) * dc;
-  const int d1 = min(d0 + dc, D);
-  const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, D) - e0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
-    wait_ctl_init(&sm.ctl, 0);
-    fence_barrier_init();
-    prefetch_tensormap(&tm_x);
+// A block of a job: its pixel tile, sample and piece of the walk.
+struct TileBlock {
+  int w0, h0, b, piece;
+};
+__device__ __forceinline__ TileBlock tile_block(int r, int B, int H1, int W1) {
+  const int tx = (W1 + AT_TW - 1) / AT_TW, tiles = tx * ((H1 + AT_TH - 1) / AT_TH);
+  const int z = r / tiles, t = r - z * tiles, ty = t / tx;
+  return TileBlock{(t - ty * tx) * AT_TW, ty * AT_TH, z % B, z / B};
+}
+struct TileMaps {
+  CUtensorMap m[MAX_ATTENTION_JOBS];
+};
+
+// The planes e0 .. e0 + n_planes - 1 of a tile, one box of `channel0` .. per plane.
+template <int NCH, class Smem>
+__device__ __forceinline__ void tile_producer(Smem& sm, const CUtensorMap* tm, const TileBlock& t, int e0, int n_planes, int channel0,
+                                              int* status) {
+  for (int i = 0; i < n_planes; ++i) {
+    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
+    if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) return;
+    mbar_expect_tx(&sm.full[s], NCH * AT_TILE_BYTES);
+    tma_load_5d(sm.x[s].v, tm, &sm.full[s], t.w0 - 4, t.h0 - 1, e0 + i, channel0, t.b);
   }
-  __syncthreads();
-  if (warp == AT_THREADS / 32) {  // producer
-    if (lane == 0) {
-      for (int i = 0; i < n_planes; ++i) {
-        const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
-        mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES);
-        tma_load_5d(sm.x[s].v, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
-      }
-    }
-    return;
-  }
-  const int tx = lane, ty = warp;
-  const int h = h0 + ty, w = w0 + tx;
+}
+
+template <int KC, int MODULE>   // false: a wait ran out
+__device__ __forceinline__ bool logits_walk_tiled(AttentionTileSmem<2>& sm, const LogitsJobs::Job& job, const TileBlock& t, int Kc, int k0,
+                                                  int d0, int d1, int e0, int n_planes, int ty, int tx, int H1, int W1, int* status) {
+  const int D = job.D, h = t.h0 + ty, w = t.w0 + tx;
   const bool valid = h < H1 && w < W1;
   const size_t plane = (size_t)H1 * W1;
-  float* out = a + ((size_t)b * Kc + k0) * D * plane + (size_t)(valid ? h * W1 + w : 0);
+  float* out = job.a + ((size_t)t.b * Kc + k0) * D * plane + (size_t)(valid ? h * W1 + w : 0);
 
   float bk[KC], acc[3][KC];
 #pragma unroll
   for (int k = 0; k < KC; ++k) {
-    bk[k] = __ldg(bias + k0 + k);
+    bk[k] = __ldg(job.bias + k0 + k);
     acc[0][k] = acc[1][k] = acc[2][k] = bk[k];
   }
   auto emit = [&](int d) {  // logit d is complete in acc[0]
@@ -260,23 +306,22 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
   for (int i = 0; i < n_planes; ++i) {  // plane e feeds logits e+1 (tap td=0), e (td=1), e-1 (td=2)
     const int e = e0 + i;
     const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-    const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
-    if (!__all_sync(0xffffffffu, ok)) { let_copies_land(); return; }
+    if (!mbar_wait_warp(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE)) return false;
     float xv[2][9];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int n = 0; n < 9; ++n) xv[c][n] = sm.x[s].v[c][ty + n / 3][tx + 3 + n % 3];
-    hand_back_stage(&sm.empty[s], lane);   // the neighbourhoods are in registers
+    hand_back_stage(&sm.empty[s], tx);   // the neighbourhoods are in registers
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int n = 0; n < 9; ++n) {
 #pragma unroll
         for (int k = 0; k < KC; ++k) {
-          acc[2][k] = fmaf(xv[c][n], c_att_weights[(k * 2 + c) * AT_TAPS + n], acc[2][k]);
-          acc[1][k] = fmaf(xv[c][n], c_att_weights[(k * 2 + c) * AT_TAPS + 9 + n], acc[1][k]);
-          acc[0][k] = fmaf(xv[c][n], c_att_weights[(k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
+          acc[2][k] = fmaf(xv[c][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + n], acc[2][k]);
+          acc[1][k] = fmaf(xv[c][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 9 + n], acc[1][k]);
+          acc[0][k] = fmaf(xv[c][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
         }
       }
     if (e > d0) emit(e - 1);
@@ -284,10 +329,42 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
     for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
   }
   if (d1 == D) emit(D - 1);
-  if constexpr (SOFT) {
-    if (!valid) return;
-#pragma unroll 1
-    for (int k = 0; k < KC; ++k) softmax_column(out + (size_t)k * D * plane, D, plane);
+  return true;
+}
+
+template <int KC, bool SOFT>
+__global__ void __launch_bounds__(AT_THREADS + 32)
+attention_logits_tiled_kernel(const __grid_constant__ TileMaps maps, const __grid_constant__ LogitsJobs jobs, int Kc, int k0, int B,
+                              int H1, int W1, int* status) {
+  if (!cta_has_work(status)) return;
+  __shared__ __align__(128) AttentionTileSmem<2> sm;
+  const int ji = job_of(jobs.blocks, blockIdx.x);
+  const LogitsJobs::Job& job = jobs.j[ji];
+  const TileBlock t = tile_block(blockIdx.x - jobs.blocks.first[ji], B, H1, W1);
+  const int d0 = t.piece * job.dc, d1 = min(d0 + job.dc, job.D);
+  const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, job.D) - e0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
+    wait_ctl_init(&sm.ctl, 0);
+    fence_barrier_init();
+    prefetch_tensormap(&maps.m[ji]);
+  }
+  __syncthreads();
+  if (warp == AT_THREADS / 32) {
+    if (lane == 0) tile_producer<2>(sm, &maps.m[ji], t, e0, n_planes, 0, status);
+    __syncwarp();
+  } else {
+    bool ok = true;
+    by_module(job.module, [&](auto m) {
+      ok = logits_walk_tiled<KC, decltype(m)::value>(sm, job, t, Kc, k0, d0, d1, e0, n_planes, warp, lane, H1, W1, status);
+    });
+    const int h = t.h0 + warp, w = t.w0 + lane;
+    if (SOFT && ok && h < H1 && w < W1) softmax_columns<KC>(job, Kc, k0, t.b, h * W1 + w, (size_t)H1 * W1);
+  }
+  __syncthreads();
+  if (wait_ctl_aborted(&sm.ctl)) {
+    let_copies_land();
   }
 }
 
@@ -295,18 +372,24 @@ attention_logits_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const fl
 // A block owns 32 consecutive pixels of one (sample, channel); warp g takes displacements g, g + 8, ... and keeps its
 // V = ceil(D / 8) values in registers, so that every logit is read once and every weight written once (HBM-bound, all
 // loads of a thread in flight together).  V = 0: any D, the values are read again in each of the three walks.  The
-// order of the sums depends on D only.  grid ceil(N1/32) * planes (= B * Kc), block 256.
+// order of the sums depends on D only.  grid of ceil(N1/32) * planes (= B * Kc) blocks per job, block 256.
 constexpr int SM_THREADS = SM_GROUPS * 32;
+struct SoftmaxJobs {
+  JobBlocks blocks;
+  float* a[MAX_ATTENTION_JOBS];
+  int D[MAX_ATTENTION_JOBS];
+};
 
 template <int V>
 __global__ void __launch_bounds__(SM_THREADS, V == 0 ? 8 : (V <= 8 ? 6 : (V <= 20 ? 3 : 2)))
-attention_softmax_kernel(float* __restrict__ a, int D, int N1, unsigned pixel_blocks) {
+attention_softmax_kernel(const __grid_constant__ SoftmaxJobs jobs, int N1, unsigned pixel_blocks) {
   __shared__ float red[2][SM_GROUPS][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const unsigned row = blockIdx.x / pixel_blocks;
-  const int p = (int)(blockIdx.x - row * pixel_blocks) * 32 + lane;
+  const int ji = job_of(jobs.blocks, blockIdx.x), D = jobs.D[ji];
+  const unsigned block = blockIdx.x - jobs.blocks.first[ji], row = block / pixel_blocks;
+  const int p = (int)(block - row * pixel_blocks) * 32 + lane;
   const bool in = p < N1;
-  float* base = a + (size_t)row * D * N1 + (in ? p : 0);
+  float* base = jobs.a[ji] + (size_t)row * D * N1 + (in ? p : 0);
   constexpr int NV = V > 0 ? V : 1;
   float v[NV];
   float m = -INFINITY;
@@ -889,10 +972,10 @@ class StagedWeights {
     if (err_ == cudaSuccess && g_stage.used[dev_] && g_stage.last[dev_] != st_)
       err_ = cudaStreamWaitEvent(st_, g_stage.done[dev_], 0);
   }
-  cudaError_t put(const float* device_weights, int channels) {  // weights of `channels` <= AT_KC channels
+  cudaError_t put(const float* device_weights, int channels, int module = 0) {  // weights of `channels` <= AT_KC channels
     if (err_ != cudaSuccess) return err_;
-    err_ = cudaMemcpyAsync(g_stage.address[dev_], device_weights, (size_t)channels * 2 * AT_TAPS * sizeof(float),
-                           cudaMemcpyDeviceToDevice, st_);
+    err_ = cudaMemcpyAsync(static_cast<float*>(g_stage.address[dev_]) + module * AT_WEIGHTS, device_weights,
+                           (size_t)channels * 2 * AT_TAPS * sizeof(float), cudaMemcpyDeviceToDevice, st_);
     return err_;
   }
   ~StagedWeights() {
@@ -945,66 +1028,119 @@ size_t attention_partial_floats(const AttentionDims& d) {
   return d.Kc * (bias + 2 * AT_TAPS * (gather > tiled ? gather : tiled));
 }
 
-static cudaError_t launch_softmax(float* a, size_t planes, int D, int N1, cudaStream_t st) {
-  const unsigned pb = (unsigned)((N1 + 31) / 32);
-  if ((unsigned long long)pb * planes > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-  const unsigned blocks = (unsigned)(pb * planes);
-  const int v = (D + SM_GROUPS - 1) / SM_GROUPS;
-  if (v <= 4) attention_softmax_kernel<4><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
-  else if (v <= 8) attention_softmax_kernel<8><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
-  else if (v <= 16) attention_softmax_kernel<16><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
-  else if (v <= 20) attention_softmax_kernel<20><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
-  else if (v <= 24) attention_softmax_kernel<24><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
-  else if (v <= 32) attention_softmax_kernel<32><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
-  else attention_softmax_kernel<0><<<blocks, SM_THREADS, 0, st>>>(a, D, N1, pb);
+// Columns of a class of lengths are done by one launch.
+template <int V>
+static cudaError_t launch_softmax_class(const AttentionJob* job, int count, int above, int upto, cudaStream_t st) {
+  SoftmaxJobs jobs{};
+  const AttentionDims& d = job[0].d;
+  const unsigned pb = (unsigned)((d.H1 * d.W1 + 31) / 32);
+  unsigned long long blocks = 0;
+  int n = 0;
+  for (int i = 0; i < count; ++i) {
+    const int v = (job[i].d.D + SM_GROUPS - 1) / SM_GROUPS;
+    if (v <= above || v > upto) continue;
+    jobs.a[n] = job[i].a;
+    jobs.D[n] = job[i].d.D;
+    jobs.blocks.first[n++] = (int)blocks;
+    blocks += (unsigned long long)pb * d.B * d.Kc;
+    if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+  }
+  if (n == 0) return cudaSuccess;
+  for (; n <= MAX_ATTENTION_JOBS; ++n) jobs.blocks.first[n] = (int)blocks;
+  attention_softmax_kernel<V><<<(unsigned)blocks, SM_THREADS, 0, st>>>(jobs, d.H1 * d.W1, pb);
   return cudaGetLastError();
 }
+static int softmax_class(int D) {   // largest values per warp of a class; 0: any
+  const int v = (D + SM_GROUPS - 1) / SM_GROUPS;
+  for (const int c : {4, 8, 16, 20, 24, 32})
+    if (v <= c) return c;
+  return 0;
+}
+static cudaError_t launch_softmax(const AttentionJob* job, int count, cudaStream_t st) {
+  cudaError_t err;
+  if ((err = launch_softmax_class<4>(job, count, 0, 4, st)) != cudaSuccess) return err;
+  if ((err = launch_softmax_class<8>(job, count, 4, 8, st)) != cudaSuccess) return err;
+  if ((err = launch_softmax_class<16>(job, count, 8, 16, st)) != cudaSuccess) return err;
+  if ((err = launch_softmax_class<20>(job, count, 16, 20, st)) != cudaSuccess) return err;
+  if ((err = launch_softmax_class<24>(job, count, 20, 24, st)) != cudaSuccess) return err;
+  if ((err = launch_softmax_class<32>(job, count, 24, 32, st)) != cudaSuccess) return err;
+  return launch_softmax_class<0>(job, count, 32, INT_MAX, st);
+}
 
-// Displacements per block of the forward's walk, and whether the walk ends with the softmax of its columns.
-// A column short enough for that is not cut by launches that have two blocks per SM without it.
-static int forward_walk(const AttentionDims& d, bool tiled) {
-  const size_t blocks = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
+// Displacements per block of the forward's walk, and whether the walks of a launch end with the softmax of their columns.  The jobs
+// of a launch fill the SMs together.  A column short enough for that is not cut by launches that have two blocks per SM without it.
+static int forward_walk(const AttentionDims& d, int jobs, bool tiled) {
+  const size_t blocks = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * jobs;
   return d.D <= AT_SOFT_MAX && blocks >= 2 * SM_COUNT ? d.D : walk_length(blocks, d.D);
 }
-static bool softmax_in_walk(const AttentionDims& d, bool tiled) { return d.D <= AT_SOFT_MAX && forward_walk(d, tiled) >= d.D; }
-
-int attention_forward_launches(const AttentionDims& d, const float* x, long long x_sb, const int* status) {
-  return (d.Kc + AT_KC - 1) / AT_KC + (softmax_in_walk(d, status != nullptr && tileable(d, x, x_sb)) ? 0 : 1);
+static bool softmax_in_walk(const AttentionJob* job, int count, bool tiled) {
+  for (int i = 0; i < count; ++i)
+    if (job[i].d.D > AT_SOFT_MAX || forward_walk(job[i].d, count, tiled) < job[i].d.D) return false;
+  return true;
+}
+static bool all_tileable(const AttentionJob* job, int count, const int* status) {
+  bool ok = status != nullptr;
+  for (int i = 0; i < count; ++i) ok = ok && tileable(job[i].d, job[i].x, job[i].x_sb);
+  return ok;
 }
 
-cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
-                                     const float* bias, float* a, cudaStream_t st, int* status) {
-  const bool tiled = status != nullptr && tileable(d, x, x_sb);
-  const bool soft = softmax_in_walk(d, tiled);
-  CUtensorMap tm_x;
-  if (tiled) {
-    cudaError_t err = tile_map(&tm_x, x, x_sb, 2, 2, d, true);
-    if (err != cudaSuccess) return err;
+int attention_forward_launches(const AttentionJob* job, int count, const int* status) {
+  const bool tiled = all_tileable(job, count, status);
+  int n = (job[0].d.Kc + AT_KC - 1) / AT_KC;
+  if (softmax_in_walk(job, count, tiled)) return n;
+  for (int i = 0; i < count; ++i) {
+    bool first = true;   // of its class of lengths
+    for (int k = 0; k < i; ++k) first = first && softmax_class(job[k].d.D) != softmax_class(job[i].d.D);
+    n += first ? 1 : 0;
   }
-  const int dc = forward_walk(d, tiled);
-  const unsigned pieces = (unsigned)((d.D + dc - 1) / dc);
-  const dim3 grid(pixel_grid(d).x, d.B * pieces);
-  const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * pieces);
+  return n;
+}
+
+cudaError_t launch_attention_forward(const AttentionJob* job, int count, const AttentionModules& modules, cudaStream_t st, int* status) {
+  if (count < 1 || count > MAX_ATTENTION_JOBS) return cudaErrorInvalidValue;
+  const AttentionDims& d = job[0].d;
+  const bool tiled = all_tileable(job, count, status);
+  const bool soft = softmax_in_walk(job, count, tiled);
+  TileMaps maps;
+  LogitsJobs jobs{};
+  unsigned long long blocks = 0;
+  for (int i = 0; i < MAX_ATTENTION_JOBS; ++i) {
+    jobs.blocks.first[i] = (int)blocks;
+    if (i >= count) continue;
+    const AttentionJob& j = job[i];
+    if (tiled) {
+      cudaError_t err = tile_map(&maps.m[i], j.x, j.x_sb, 2, 2, j.d, true);
+      if (err != cudaSuccess) return err;
+    }
+    const int dc = forward_walk(j.d, count, tiled);
+    jobs.j[i] = LogitsJobs::Job{j.x, j.x_sb, modules.bias[j.module], j.a, j.d.D, dc, j.module};
+    blocks += (unsigned long long)(tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * ((j.d.D + dc - 1) / dc);
+    if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+  }
+  jobs.blocks.first[MAX_ATTENTION_JOBS] = (int)blocks;
   {
     StagedWeights staged(st);
     for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
       const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
-      cudaError_t err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
-      if (err != cudaSuccess) return err;
+      for (int m = 0; m < 2; ++m) {
+        if (modules.weight[m] == nullptr) continue;
+        cudaError_t err = staged.put(modules.weight[m] + (size_t)k0 * 2 * AT_TAPS, kc, m);
+        if (err != cudaSuccess) return err;
+      }
       if (tiled) {
-#define SFB_AT_FWD_T(KC) (soft ? attention_logits_tiled_kernel<KC, true> : attention_logits_tiled_kernel<KC, false>)<<<tgrid, AT_THREADS + 32, 0, st>>>(tm_x, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1, status)
+#define SFB_AT_FWD_T(KC) (soft ? attention_logits_tiled_kernel<KC, true> : attention_logits_tiled_kernel<KC, false>)<<<(unsigned)blocks, AT_THREADS + 32, 0, st>>>(maps, jobs, d.Kc, k0, d.B, d.H1, d.W1, status)
         if (kc == 1) SFB_AT_FWD_T(1); else if (kc == 2) SFB_AT_FWD_T(2); else if (kc == 3) SFB_AT_FWD_T(3); else SFB_AT_FWD_T(4);
 #undef SFB_AT_FWD_T
         continue;
       }
-#define SFB_AT_FWD(KC) (soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>)<<<grid, AT_THREADS, 0, st>>>(x, x_sb, bias, a, d.Kc, k0, d.B, d.D, dc, d.H1, d.W1)
+#define SFB_AT_FWD(KC) (soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>)<<<(unsigned)blocks, AT_THREADS, 0, st>>>(jobs, d.Kc, k0, d.B, d.H1, d.W1)
       if (kc == 1) SFB_AT_FWD(1); else if (kc == 2) SFB_AT_FWD(2); else if (kc == 3) SFB_AT_FWD(3); else SFB_AT_FWD(4);
 #undef SFB_AT_FWD
     }
   }
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess || soft) return err;
-  return launch_softmax(a, (size_t)d.B * d.Kc, d.D, d.H1 * d.W1, st);
+  return launch_softmax(job, count, st);
 }
 
 template <int KC>

@@ -502,7 +502,8 @@ cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& 
   uint16_t* const F1h = op16 ? w.F1h : nullptr;
   uint16_t* const F2h = op16 ? w.F2h : nullptr;
   uint16_t* const auxh = op16 && with_aux ? w.auxh : nullptr;
-  return f.fmaps ? launch_prepare_cf(d, f.F1, f.F2, f.scale1, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales)
+  const LevelOperands out{F2r, aux, F2h, auxh};
+  return f.fmaps ? launch_prepare_cf(&d, 1, f.F1, &f.F2, f.scale1, &out, F1r, F1h, w.status, st, op16, w.scales)
                  : launch_prepare(d, f.F1, f.F2, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales);
 }
 // Launches of the above: FP16 operands add the search for the magnitudes.
@@ -705,9 +706,9 @@ int grad_operand_scales(const Workspace& w, int op16, std::initializer_list<Absm
   if (op16 != OP16_FP16) return SFB_OK;
   AbsmaxSource src[ABSMAX_MAX];
   int n = 0;
-  for (const AbsmaxSrc& g : grads) src[n++] = AbsmaxSource{g.p, g.n, 1.f, SCALE_AMAX_G};
-  for (const AbsmaxSrc& a : weights) src[n++] = AbsmaxSource{a.p, a.n, 1.f, SCALE_AMAX_A};
-  SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_absmax(src, n, w.scales, true, st); }));
+  for (const AbsmaxSrc& g : grads) src[n++] = absmax_array(g.p, g.n, 1.f, SCALE_AMAX_G);
+  for (const AbsmaxSrc& a : weights) src[n++] = absmax_array(a.p, a.n, 1.f, SCALE_AMAX_A);
+  SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_absmax(src, n, w.scales, 1, true, st); }));
   return SFB_OK;
 }
 const float* grad_slot_scales(const Workspace& w, int op16) { return op16 == OP16_FP16 ? w.scales : nullptr; }
@@ -1170,8 +1171,10 @@ int sfb_attention_forward(const float* X, int64_t x_batch_stride, const float* w
   if (X == nullptr || weight == nullptr || bias == nullptr || A == nullptr)
     return fail(SFB_ERR_INVALID_ARGUMENT, "X, weight, bias and A must not be NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SFB_CUDA(timed(KID_ATTENTION_FWD, attention_forward_launches(ad, X, x_batch_stride, nullptr), st,
-                 [&] { return launch_attention_forward(ad, X, x_batch_stride, weight, bias, A, st); }));
+  const AttentionJob job{ad, 0, X, x_batch_stride, A};
+  const AttentionModules modules{{weight, nullptr}, {bias, nullptr}};
+  SFB_CUDA(timed(KID_ATTENTION_FWD, attention_forward_launches(&job, 1, nullptr), st,
+                 [&] { return launch_attention_forward(&job, 1, modules, st); }));
   return SFB_OK;
 }
 
@@ -1267,11 +1270,10 @@ static int level_forward(Placement pl, const float* F1, const float* F2, int fma
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
   const AttentionDims at_u{d.B, K, d.W2, d.H1, d.W1}, at_v{d.B, K, d.H2, d.H1, d.W1};
   const float *const X_u = SEP_u + (size_t)c0 * d.W2 * N1, *const X_v = SEP_v + (size_t)c0 * d.H2 * N1;
-  const int at_launches = attention_forward_launches(at_u, X_u, sb_u, w.status) + attention_forward_launches(at_v, X_v, sb_v, w.status);
-  SFB_CUDA(timed(KID_ATTENTION_FWD, at_launches, st, [&] {
-    SFB_LAUNCH(launch_attention_forward(at_u, X_u, sb_u, weight_u, bias_u, A_u, st, w.status));
-    return launch_attention_forward(at_v, X_v, sb_v, weight_v, bias_v, A_v, st, w.status);
-  }));
+  const AttentionJob jobs[2] = {{at_u, 0, X_u, sb_u, A_u}, {at_v, 1, X_v, sb_v, A_v}};
+  const AttentionModules modules{{weight_u, weight_v}, {bias_u, bias_v}};
+  SFB_CUDA(timed(KID_ATTENTION_FWD, attention_forward_launches(jobs, 2, w.status), st,
+                 [&] { return launch_attention_forward(jobs, 2, modules, st, w.status); }));
   // C_u (per u, weights A_u per v) -> SEP_v channels 2.., C_v -> SEP_u channels 2..
   return run_compress_sweeps(d, w, tm_f1, tm_f2_sums, cf_view(A_v, K, d.H2, N1), cf_view(A_u, K, d.W2, N1), 0, 0, 1,
                              cf_channels(SEP_v, Kt, c0 + 2, d.H2, N1), cf_channels(SEP_u, Kt, c0 + 2, d.W2, N1), N1, st,
@@ -1378,7 +1380,8 @@ int sfb_upsample_displacement(const float* in, float* out, int64_t out_batch_str
   SFB_TRY(check_resample(in, out, B, K, Dl, D0, H1, W1));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SFB_CUDA(timed(KID_RESAMPLE, 1, st, [&] {
-    return launch_upsample_displacement(in, out, out_batch_stride, B, K, Dl, D0, H1 * W1, st);
+    const ResampleJob job{in, out, out_batch_stride, Dl, D0};
+    return launch_upsample_displacement(&job, 1, B, K, H1 * W1, st);
   }));
   return SFB_OK;
 }
@@ -1390,6 +1393,258 @@ int sfb_upsample_displacement_backward(const float* gout, int64_t gout_batch_str
   SFB_CUDA(timed(KID_RESAMPLE, 1, st, [&] {
     return launch_upsample_displacement_adjoint(gout, gout_batch_stride, gin, B, K, Dl, D0, H1 * W1, st);
   }));
+  return SFB_OK;
+}
+
+}  // extern "C"
+
+// ---- all pyramid levels of the call site ----
+namespace {
+// What the levels of a call share and what each has of its own.  Image 1, C and Kc are the same for all of them.
+struct Pyramid {
+  int levels;
+  Dims d[MAX_FUSED_LEVELS];
+  bool in_place[MAX_FUSED_LEVELS];   // the level has the displacement ranges of the outputs: its channels of them are its volumes
+};
+
+int check_pyramid(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int levels, Pyramid* py) {
+  if (shape == nullptr || H2 == nullptr || W2 == nullptr) return fail(SFB_ERR_INVALID_ARGUMENT, "shape, H2 and W2 must not be NULL");
+  if (levels < 1 || levels > MAX_FUSED_LEVELS)
+    return fail(SFB_ERR_UNSUPPORTED_SHAPE, "levels must be in [1, %d] (got %d)", MAX_FUSED_LEVELS, levels);
+  py->levels = levels;
+  for (int l = 0; l < levels; ++l) {
+    sfb_shape s = *shape;
+    s.H2 = H2[l];
+    s.W2 = W2[l];
+    SFB_TRY(check_shape(&s, true, &py->d[l]));
+    if (H2[l] > H2[0] || W2[l] > W2[0]) return fail(SFB_ERR_UNSUPPORTED_SHAPE, "level %d of image 2 is larger than level 0", l);
+    py->in_place[l] = H2[l] == H2[0] && W2[l] == W2[0];
+  }
+  const Dims& d = py->d[0];
+  if (d.Kc > KC_MAX_PER_SWEEP)
+    return fail(SFB_ERR_UNSUPPORTED_SHAPE, "the levels share a launch for at most %d attention channels (got %d)", KC_MAX_PER_SWEEP, d.Kc);
+  if ((long long)d.B * (2 + d.Kc) > 65535) return fail(SFB_ERR_UNSUPPORTED_SHAPE, "B * (2 + Kc) must be <= 65535");
+  Placement pl{levels * (2 + d.Kc), 0};
+  return check_placement(d, &pl);
+}
+
+// Tensors a forward leaves for its backward, in one buffer: the volumes of the levels that are not in place, arg-max indices (when
+// there is a backward), attention weights.
+struct PyramidSaved {
+  float *sep_u[MAX_FUSED_LEVELS], *sep_v[MAX_FUSED_LEVELS], *a_u[MAX_FUSED_LEVELS], *a_v[MAX_FUSED_LEVELS];
+  int32_t *am_u[MAX_FUSED_LEVELS], *am_v[MAX_FUSED_LEVELS];
+  size_t bytes;
+};
+PyramidSaved carve_saved(const Pyramid& py, void* base, bool with_argmax) {
+  PyramidSaved v;
+  size_t off = 0;
+  auto take = [&](size_t floats) {
+    float* r = reinterpret_cast<float*>(static_cast<char*>(base) + off);
+    off += align_up(floats * sizeof(float), 256);
+    return r;
+  };
+  for (int l = 0; l < py.levels; ++l) {
+    const Dims& d = py.d[l];
+    const size_t bn = (size_t)d.B * d.N1();
+    v.sep_u[l] = py.in_place[l] ? nullptr : take(bn * (2 + d.Kc) * d.W2);
+    v.sep_v[l] = py.in_place[l] ? nullptr : take(bn * (2 + d.Kc) * d.H2);
+    v.am_u[l] = with_argmax ? reinterpret_cast<int32_t*>(take(bn * d.H2)) : nullptr;
+    v.am_v[l] = with_argmax ? reinterpret_cast<int32_t*>(take(bn * d.W2)) : nullptr;
+    v.a_u[l] = take(bn * d.Kc * d.W2);
+    v.a_v[l] = take(bn * d.Kc * d.H2);
+  }
+  v.bytes = off;
+  return v;
+}
+
+// Workspaces of the levels: every level has what carve() gives it, image 1's copies and the header are level 0's, and the
+// scratch of cut tiles follows.
+struct PyramidWorkspace {
+  Workspace w[MAX_FUSED_LEVELS];
+  size_t bytes;
+};
+// A sweep over all levels is cut as a whole; the parts of its levels lie one behind the other.
+size_t pyramid_part_floats(const Pyramid& py, int slots, bool sums, TileSplit* split) {
+  sweep_split_levels(py.d, py.levels, slots, sums, split);
+  size_t floats = 0;
+  for (int l = 0; l < py.levels; ++l) floats += split[l].part_floats;
+  return floats;
+}
+PyramidWorkspace carve_pyramid_forward(const Pyramid& py, void* base) {
+  PyramidWorkspace p;
+  size_t off = 0;
+  auto take = [&](size_t floats) {
+    float* r = reinterpret_cast<float*>(static_cast<char*>(base) + off);
+    off += align_up(floats * sizeof(float), 256);
+    return r;
+  };
+  const Dims& d0 = py.d[0];
+  int* const status = reinterpret_cast<int*>(take(WS_HEADER_BYTES / sizeof(float)));
+  float* const F1 = take((size_t)d0.B * d0.N1() * d0.C);
+  for (int l = 0; l < py.levels; ++l) {
+    const Dims& d = py.d[l];
+    Workspace& w = p.w[l];
+    w = Workspace{};
+    w.status = status;
+    w.scales = reinterpret_cast<float*>(reinterpret_cast<char*>(status) + WS_SCALES_OFFSET) + l * SCALE_LEVEL;
+    w.n1p = padded_pixels(d);
+    w.F1r = F1;
+    w.F2r = take((size_t)d.B * d.N2() * d.C);
+    w.aux = take((size_t)d.B * d.aux_rows() * d.C);
+    w.F1h = reinterpret_cast<uint16_t*>(w.F1r);
+    w.F2h = reinterpret_cast<uint16_t*>(w.F2r);
+    w.auxh = reinterpret_cast<uint16_t*>(w.aux);
+  }
+  TileSplit split[MAX_FUSED_LEVELS];
+  const size_t part = std::max(pyramid_part_floats(py, MAXAVG_PART_SLOTS, false, split),
+                               pyramid_part_floats(py, chunk_channels(d0.Kc), true, split));
+  float* const parts = take(part);
+  for (int l = 0; l < py.levels; ++l) p.w[l].part = parts;
+  p.bytes = off;
+  return p;
+}
+
+// The sweeps of all levels: `fill(l, a)` sets a level's views, the rest is common.
+template <class Fill>
+int run_pyramid_sweeps(const Pyramid& py, const Workspace* w, int op16, int mode, cudaStream_t st, Fill&& fill) {
+  const bool sums = mode == SWEEP_COMPRESS;
+  const int slots = sums ? chunk_channels(py.d[0].Kc) : MAXAVG_PART_SLOTS;
+  CUtensorMap tm_f1, tm_f2[MAX_FUSED_LEVELS], tm_aux[MAX_FUSED_LEVELS];
+  SweepArgs a[MAX_FUSED_LEVELS];
+  TileSplit split[MAX_FUSED_LEVELS];
+  pyramid_part_floats(py, slots, sums, split);
+  float* part = w[0].part;
+  int launches = 1;
+  for (int l = 0; l < py.levels; ++l) {
+    SFB_TRY(map_sweep_operands(py.d[l], w[l], op16, &tm_f1, sums ? nullptr : &tm_f2[l], sums ? &tm_f2[l] : nullptr, sums ? nullptr : &tm_aux[l]));
+    if (sums) tm_aux[l] = tm_f2[l];   // unused
+    memset(&a[l], 0, sizeof(a[l]));
+    a[l].d = py.d[l];
+    a[l].mode = mode;
+    a[l].n_valid = py.d[l].N1();
+    a[l].kc = sums ? py.d[l].Kc : 0;
+    a[l].w_stride = 1;
+    a[l].op16 = op16;
+    a[l].out_scale = sweep_out_scale(w[l], op16);
+    a[l].status = w[l].status;
+    a[l].whole_tiles = split[l].whole_tiles;
+    a[l].pieces = split[l].pieces;
+    a[l].parts = split[l].parts;
+    a[l].part_slots = slots;
+    a[l].part = part;
+    part += split[l].part_floats;
+    if (split[l].pieces > 1) launches = 2;
+    fill(l, a[l]);
+    a[l] = with_wait_settings(a[l]);
+  }
+  SFB_CUDA(timed(sums ? KID_SWEEP_COMPRESS : KID_SWEEP_MAXAVG, launches, st,
+                 [&] { return launch_sweep_levels(a, py.levels, tm_f1, tm_f2, tm_aux, st); }));
+  return SFB_OK;
+}
+
+// Operand copies of all levels (and the mean rows of image 2 when with_aux).
+int prepare_pyramid(const Pyramid& py, const Workspace* w, const float* fmap1, const float* const* fmap2, float scale1, bool with_aux,
+                    int op16, cudaStream_t st) {
+  LevelOperands out[MAX_FUSED_LEVELS];
+  for (int l = 0; l < py.levels; ++l)
+    out[l] = op16 ? LevelOperands{nullptr, nullptr, w[l].F2h, with_aux ? w[l].auxh : nullptr}
+                  : LevelOperands{w[l].F2r, with_aux ? w[l].aux : nullptr, nullptr, nullptr};
+  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w[0], true, with_aux, op16), st, [&] {
+    return launch_prepare_cf(py.d, py.levels, fmap1, fmap2, scale1, out, op16 ? nullptr : w[0].F1r, op16 ? w[0].F1h : nullptr, w[0].status,
+                             st, op16, w[0].scales);
+  }));
+  return SFB_OK;
+}
+
+// Where the volumes of a level are: channels of the outputs, or tensors of their own.
+struct LevelVolumes {
+  float *u, *v;            // (B, 2 + Kc, W2, N1) / (B, 2 + Kc, H2, N1), first sample
+  long long sb_u, sb_v;    // elements between samples
+};
+LevelVolumes level_volumes(const Pyramid& py, int l, float* SEP_u, float* SEP_v, float* own_u, float* own_v) {
+  const Dims& d = py.d[l];
+  const int Kt = 2 + d.Kc, N1 = d.N1(), K = py.in_place[l] ? Kt * py.levels : Kt, c0 = py.in_place[l] ? l * Kt : 0;
+  return LevelVolumes{(py.in_place[l] ? SEP_u : own_u) + (size_t)c0 * d.W2 * N1, (py.in_place[l] ? SEP_v : own_v) + (size_t)c0 * d.H2 * N1,
+                      (long long)K * d.W2 * N1, (long long)K * d.H2 * N1};
+}
+PixView volume_view(float* base, long long sb, int channel, int D, int N1) {
+  return PixView{base + (size_t)channel * D * N1, sb, (uint32_t)N1, (uint32_t)(D * N1)};
+}
+}  // namespace
+
+extern "C" {
+
+size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
+                                          int32_t with_argmax) {
+  Pyramid py;
+  if (check_pyramid(shape, H2, W2, levels, &py) != SFB_OK) return 0;
+  return carve_saved(py, nullptr, with_argmax != 0).bytes;
+}
+
+size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels) {
+  Pyramid py;
+  if (check_pyramid(shape, H2, W2, levels, &py) != SFB_OK) return 0;
+  return carve_pyramid_forward(py, nullptr).bytes;
+}
+
+int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
+                                   int32_t levels, float scale1, const float* weight_u, const float* bias_u,
+                                   const float* weight_v, const float* bias_v, float* SEP_u, float* SEP_v, void* saved,
+                                   size_t saved_bytes, int32_t with_argmax, const sfb_shape* shape, void* workspace,
+                                   size_t workspace_bytes, void* stream) {
+  Pyramid py;
+  SFB_TRY(check_pyramid(shape, H2, W2, levels, &py));
+  SFB_CHECK_PTR(fmap1); SFB_CHECK_PTR(fmap2); SFB_CHECK_PTR(SEP_u); SFB_CHECK_PTR(SEP_v); SFB_CHECK_PTR(saved);
+  for (int l = 0; l < levels; ++l) SFB_CHECK_PTR(fmap2[l]);
+  if (weight_u == nullptr || bias_u == nullptr || weight_v == nullptr || bias_v == nullptr)
+    return fail(SFB_ERR_INVALID_ARGUMENT, "attention weights and biases must not be NULL");
+  const PyramidSaved sv = carve_saved(py, saved, with_argmax != 0);
+  if (saved_bytes < sv.bytes) return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "saved has %zu bytes, %zu needed", saved_bytes, sv.bytes);
+  if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+    return fail(SFB_ERR_INVALID_ARGUMENT, "workspace is NULL or not 256-byte aligned");
+  const PyramidWorkspace pw = carve_pyramid_forward(py, workspace);
+  if (workspace_bytes < pw.bytes)
+    return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", workspace_bytes, pw.bytes);
+  const Dims& d0 = py.d[0];
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int op16;
+  SFB_TRY(operand_mode(d0, &op16));
+  SFB_TRY(prepare_pyramid(py, pw.w, fmap1, fmap2, scale1, true, op16, st));
+  const int N1 = d0.N1(), K = d0.Kc, Kt = 2 + K;
+  LevelVolumes vol[MAX_FUSED_LEVELS];
+  for (int l = 0; l < levels; ++l) vol[l] = level_volumes(py, l, SEP_u, SEP_v, sv.sep_u[l], sv.sep_v[l]);
+  SFB_TRY(run_pyramid_sweeps(py, pw.w, op16, with_argmax != 0 ? SWEEP_MAXARGAVG : SWEEP_MAXAVG, st, [&](int l, SweepArgs& a) {
+    a.pu = volume_view(vol[l].v, vol[l].sb_v, 0, py.d[l].H2, N1);   // per-u channels live in the tensor the call site calls sep_v
+    a.pv = volume_view(vol[l].u, vol[l].sb_u, 0, py.d[l].W2, N1);
+    a.pu_arg = cf_view(sv.am_u[l], 1, py.d[l].H2, N1);
+    a.pv_arg = cf_view(sv.am_v[l], 1, py.d[l].W2, N1);
+  }));
+  AttentionJob jobs[MAX_ATTENTION_JOBS];
+  for (int l = 0; l < levels; ++l) {
+    const Dims& d = py.d[l];
+    jobs[2 * l] = AttentionJob{AttentionDims{d.B, K, d.W2, d.H1, d.W1}, 0, vol[l].u, vol[l].sb_u, sv.a_u[l]};
+    jobs[2 * l + 1] = AttentionJob{AttentionDims{d.B, K, d.H2, d.H1, d.W1}, 1, vol[l].v, vol[l].sb_v, sv.a_v[l]};
+  }
+  const AttentionModules modules{{weight_u, weight_v}, {bias_u, bias_v}};
+  int* const status = pw.w[0].status;
+  SFB_CUDA(timed(KID_ATTENTION_FWD, attention_forward_launches(jobs, 2 * levels, status), st,
+                 [&] { return launch_attention_forward(jobs, 2 * levels, modules, st, status); }));
+  // C_u (per u, weights A_u per v) -> the v volume's channels 2.., C_v -> the u volume's
+  SFB_TRY(run_pyramid_sweeps(py, pw.w, op16, SWEEP_COMPRESS, st, [&](int l, SweepArgs& a) {
+    a.xu = cf_view(sv.a_v[l], K, py.d[l].H2, N1);
+    a.xv = cf_view(sv.a_u[l], K, py.d[l].W2, N1);
+    a.ou = volume_view(vol[l].v, vol[l].sb_v, 2, py.d[l].H2, N1);
+    a.ov = volume_view(vol[l].u, vol[l].sb_u, 2, py.d[l].W2, N1);
+  }));
+  ResampleJob up[MAX_RESAMPLE_JOBS];
+  int n = 0;
+  for (int l = 0; l < levels; ++l) {
+    if (py.in_place[l]) continue;
+    const long long c0 = (long long)l * Kt;
+    up[n++] = ResampleJob{vol[l].u, SEP_u + c0 * d0.W2 * N1, (long long)Kt * levels * d0.W2 * N1, py.d[l].W2, d0.W2};
+    up[n++] = ResampleJob{vol[l].v, SEP_v + c0 * d0.H2 * N1, (long long)Kt * levels * d0.H2 * N1, py.d[l].H2, d0.H2};
+  }
+  if (n > 0) SFB_CUDA(timed(KID_RESAMPLE, 1, st, [&] { return launch_upsample_displacement(up, n, d0.B, Kt, N1, st); }));
   return SFB_OK;
 }
 

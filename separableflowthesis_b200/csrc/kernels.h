@@ -53,6 +53,7 @@ constexpr int GG_UT = 4;      // a K block of the image-1-major gradient GEMM: 4
 constexpr int GG_VT = 16;
 constexpr int GG_KJ = 32;     // and of the image-2-major one: 32 image-1 pixels
 constexpr int KC_MAX_PER_SWEEP = 4;  // attention channels handled by one compression sweep
+constexpr int MAX_FUSED_LEVELS = 4;  // levels of a pyramid that the kernels of a call take in one launch
 
 // 16-bit operand kinds of the contractions (0 = none: TF32 operands in FP32 storage).
 #ifndef SFB_OP16_KINDS
@@ -99,6 +100,7 @@ struct SweepArgs {
   // Tiles past `whole_tiles` are done by `pieces` CTAs each (TileSplit); part is unused when pieces is 1.
   int whole_tiles, pieces, parts, part_slots;
   float* part;
+  bool narrow;           // sweep_narrow of this shape and mode (set by the launcher)
 };
 
 // How a launch of equal tiles fills the SMs: whole_tiles CTAs do one tile each, every further tile is done by `pieces`
@@ -120,6 +122,43 @@ __host__ __device__ inline bool sweep_narrow(const Dims& d, bool sums) {
 }
 // slots: row results per pixel (max and argmax; channels of a launch); sums: they are added up, not compared
 TileSplit sweep_split(const Dims& d, int slots, bool sums);
+// The same for the levels of a pyramid that share a launch (same image 1).
+void sweep_split_levels(const Dims* d, int levels, int slots, bool sums, TileSplit* out);
+
+// Host side.  Makespan of a launch on SM_COUNT SMs with one block each at a time: groups of equal blocks, which start in the
+// order in which they are added wherever an SM is free.
+class BlockQueue {
+ public:
+  void add(int blocks, double length) {
+    while (blocks > 0) {
+      std::pop_heap(free_, free_ + n_, later);   // the SMs that are free first
+      Sms& first = free_[n_ - 1];
+      if (blocks >= first.count || n_ == MAX_GROUPS) {
+        blocks -= first.count;
+        first.at += length;
+      } else {
+        first.count -= blocks;
+        free_[n_] = Sms{first.at + length, blocks};
+        blocks = 0;
+        std::push_heap(free_, free_ + n_, later);
+        ++n_;
+      }
+      std::push_heap(free_, free_ + n_, later);
+    }
+  }
+  double makespan() const {
+    double most = 0;
+    for (int i = 0; i < n_; ++i) most = std::max(most, free_[i].at);
+    return most;
+  }
+
+ private:
+  struct Sms { double at; int count; };
+  static bool later(const Sms& x, const Sms& y) { return x.at > y.at; }
+  static constexpr int MAX_GROUPS = 32;   // SMs that become free together; past that many groups a remainder counts as a whole one
+  Sms free_[MAX_GROUPS] = {{0.0, SM_COUNT}};
+  int n_ = 1;
+};
 
 // Gradient GEMM.  G = dLoss/dS is generated from two "interleaved" operand sets: for every displacement
 // and image-1 pixel the R4 values (slots) that pixel contributes, in groups of four:
@@ -201,16 +240,18 @@ inline int pack_launches(int groups, int B) { return (groups + pack_groups_per_l
 [[nodiscard]] cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
                                     int Qtot, int q0, cudaStream_t stream);
 
-// Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, all cleared by
-// launch_prepare.  amax slots hold float bits (atomicMax), the others floats; every scale is a power of two.
-constexpr size_t WS_HEADER_BYTES = 1024, WS_SCALES_OFFSET = 64, WS_HEADER_CLEAR_BYTES = 256;
+// Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, SCALE_LEVEL for every level of the
+// call, all cleared by launch_prepare.  amax slots hold float bits (atomicMax), the others floats; every scale is a power of two.
+constexpr size_t WS_HEADER_BYTES = 1024, WS_SCALES_OFFSET = 64;
 enum : int {
   SCALE_AMAX_F1 = 0, SCALE_AMAX_F2 = 1, SCALE_AMAX_G = 2, SCALE_AMAX_A = 3,
   SCALE_F1 = 4, SCALE_F2 = 5, SCALE_INV_F1F2 = 6,   // F1h = fp16(s1 F1), F2h = fp16(s2 F2), sweep outputs * 1/(s1 s2)
   SCALE_GA = 7, SCALE_G = 8, SCALE_A = 9,           // gradient slots * sg (* sa when no weight multiplies them), weights * sa
   SCALE_INV_GF1 = 10, SCALE_INV_GF2 = 11,           // gF1 * 1/(sg sa s2), gF2 * 1/(sg sa s1)
-  SCALE_TICKET = 12                                 // blocks of a running magnitude search that are done
+  SCALE_TICKET = 12,                                // blocks of a running magnitude search that are done (the first level's)
+  SCALE_LEVEL = 16                                  // slots of a level
 };
+static_assert(WS_SCALES_OFFSET + MAX_FUSED_LEVELS * SCALE_LEVEL * sizeof(float) <= WS_HEADER_BYTES, "scale slots");
 // Makes the operand copies of a call's features and clears the workspace header.  TF32 operands (op16 = 0): F1r / F2r,
 // rounded to nearest, and the row/column mean rows of F2 in aux.  16-bit operands: F1h / F2h / auxh, from the unrounded
 // values (BF16, or FP16 after scaling by the powers of two this call derives from the arrays' largest magnitudes,
@@ -218,17 +259,19 @@ enum : int {
 [[nodiscard]] cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, float* F1r, float* F2r, float* aux,
                            int* status, cudaStream_t stream, uint16_t* F1h = nullptr, uint16_t* F2h = nullptr,
                            uint16_t* auxh = nullptr, int op16 = 0, float* scales = nullptr);
-// The same from the model's feature maps fmap1 (B, C, H1, W1), fmap2 (B, C, H2, W2): F1r = round(scale1 * fmap1)
-// transposed to (B, H1, W1, C), F2r = round(fmap2) transposed (core/corr.py:419-422 does this with
+// The same from the model's feature maps fmap1 (B, C, H1, W1) and, for every level of the call, fmap2[l] (B, C, H2, W2): F1r =
+// round(scale1 * fmap1) transposed to (B, H1, W1, C), F2r = round(fmap2) transposed (core/corr.py:419-422 does this with
 // permute().contiguous() and a division).
-[[nodiscard]] cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fmap2, float scale1, float* F1r,
-                              float* F2r, float* aux, int* status, cudaStream_t stream, uint16_t* F1h = nullptr,
-                              uint16_t* F2h = nullptr, uint16_t* auxh = nullptr, int op16 = 0, float* scales = nullptr);
-// Largest |x| * premul of each array, combined into its amax slot, and then the multipliers that follow from the slots:
-// those of the features or (gradients) those of the gradient operands.
-constexpr int ABSMAX_MAX = 6;
-struct AbsmaxSource { const float* p; size_t n; float premul; int slot; };
-[[nodiscard]] cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, bool gradients, cudaStream_t stream);
+struct LevelOperands { float *F2r, *aux; uint16_t *F2h, *auxh; };
+[[nodiscard]] cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, const float* const* fmap2, float scale1,
+                              const LevelOperands* out, float* F1r, uint16_t* F1h, int* status, cudaStream_t stream, int op16 = 0,
+                              float* scales = nullptr);
+// Largest |x| * premul of each array, `samples` runs of n values sb apart, combined into its amax slot (SCALE_* of a level), and then the
+// multipliers that follow from the slots of every level: those of the features or (gradients) those of the gradient operands.
+constexpr int ABSMAX_MAX = 4 * MAX_FUSED_LEVELS;
+struct AbsmaxSource { const float* p; size_t n; long long sb; int samples; float premul; int slot; };
+inline AbsmaxSource absmax_array(const float* p, size_t n, float premul, int slot) { return AbsmaxSource{p, n, (long long)n, 1, premul, slot}; }
+[[nodiscard]] cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int levels, bool gradients, cudaStream_t stream);
 // 16-bit channel-major copy from a (B, C, rows*width) feature map times `scale`, padding zeroed (layouts below).
 [[nodiscard]] cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
                                     int blocked, float scale, int op16, const float* scale16, cudaStream_t stream);
@@ -247,6 +290,9 @@ struct AbsmaxSource { const float* p; size_t n; float premul; int slot; };
                           int rstride, int Kdst, int kdst0, cudaStream_t stream);
 [[nodiscard]] cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                          const CUtensorMap& tm_aux, cudaStream_t stream);
+// The levels of a pyramid in one launch (same image 1, mode, channels and operand type).
+[[nodiscard]] cudaError_t launch_sweep_levels(const SweepArgs* a, int levels, const CUtensorMap& tm_f1, const CUtensorMap* tm_f2,
+                                const CUtensorMap* tm_aux, cudaStream_t stream);
 // tm_y: channel-major features of the other image (K-major B operand); tm_xu / tm_xv: interleaved operands (tm_xv is only read by the
 // image-2-major form; the image-1-major form keeps its (pixel, v) slots in registers).
 [[nodiscard]] cudaError_t launch_grad_gemm(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
@@ -259,12 +305,22 @@ struct AbsmaxSource { const float* p; size_t n; float premul; int slot; };
 struct AttentionDims {
   int B, Kc, D, H1, W1;
 };
-// `status` (optional): a device status word for bounded waits.  With it, and when W1 is a multiple of 4 and x is
+// One tensor that a module is applied to.  A launch takes several: those of a level or of a pyramid's levels, which differ in D alone.
+constexpr int MAX_ATTENTION_JOBS = 2 * MAX_FUSED_LEVELS;
+struct AttentionModules { const float *weight[2], *bias[2]; };   // null where no job uses the module
+struct AttentionJob {
+  AttentionDims d;
+  int module;
+  const float* x;
+  long long x_sb;
+  float* a;
+};
+// `status` (optional): a device status word for bounded waits.  With it, and when W1 is a multiple of 4 and every x is
 // 16-byte aligned, the kernels fetch their pixel tiles (with the stencil's halo, zero-filled outside the image) by
 // TMA; otherwise every thread gathers its own neighbourhood.
-[[nodiscard]] cudaError_t launch_attention_forward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
-                                     const float* bias, float* a, cudaStream_t stream, int* status = nullptr);
-int attention_forward_launches(const AttentionDims& d, const float* x, long long x_sb, const int* status);  // its kernels
+[[nodiscard]] cudaError_t launch_attention_forward(const AttentionJob* jobs, int count, const AttentionModules& modules,
+                                     cudaStream_t stream, int* status = nullptr);
+int attention_forward_launches(const AttentionJob* jobs, int count, const int* status);  // its kernels
 // Tiled fp32 tensor map without swizzle, zero fill out of bounds; dims / box innermost first, `strides_bytes` for
 // dimensions 1 .. rank-1.  Implemented next to the other tensor maps (c_abi.cu).
 [[nodiscard]] cudaError_t encode_plain_map(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,
@@ -280,9 +336,16 @@ size_t attention_partial_floats(const AttentionDims& d);
 
 
 // Linear resampling along the displacement axis (core/corr.py:459-467: trilinear interpolate with unchanged H1, W1):
-// in (B, K, Dl, N1) -> K channels of a larger tensor, out[b] at out + b*out_sb, each (K, D0, N1); Dl <= D0.
-[[nodiscard]] cudaError_t launch_upsample_displacement(const float* in, float* out, long long out_sb, int B, int K, int Dl, int D0,
-                                         int N1, cudaStream_t stream);
+// in (B, K, Dl, N1) -> K channels of a larger tensor, out[b] at out + b*out_sb, each (K, D0, N1); Dl <= D0.  A launch takes the
+// volumes of several levels.
+constexpr int MAX_RESAMPLE_JOBS = 2 * MAX_FUSED_LEVELS;
+struct ResampleJob {
+  const float* in;
+  float* out;
+  long long out_sb;
+  int Dl, D0;
+};
+[[nodiscard]] cudaError_t launch_upsample_displacement(const ResampleJob* jobs, int count, int B, int K, int N1, cudaStream_t stream);
 // Its adjoint: gin (B, K, Dl, N1) from the gradient of those K channels.
 [[nodiscard]] cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
                                                  int D0, int N1, cudaStream_t stream);

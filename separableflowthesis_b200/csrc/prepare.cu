@@ -12,6 +12,7 @@
 // The FP32 copies are made for TF32 operands only; with 16-bit operands every reader takes the 16-bit copies or the
 // caller's features themselves.
 #include <algorithm>
+#include <climits>
 
 #include <cuda_bf16.h>
 
@@ -32,9 +33,9 @@ __device__ __forceinline__ float pow2_scale(unsigned amax_bits, int target_log2)
   return __uint_as_float((unsigned)(127 + shift) << 23);
 }
 
-// scales[] (SCALE_* in kernels.h): feature scales from the two magnitudes found by absmax_kernel.
-__device__ void feature_scales(float* scales) {
-  const float s1 = pow2_scale(__float_as_uint(__ldcg(scales + SCALE_AMAX_F1)), 0);
+// scales[] (SCALE_* in kernels.h): feature scales from the two magnitudes found by absmax_kernel (image 1's: amax1).
+__device__ void feature_scales(float* scales, const float* amax1) {
+  const float s1 = pow2_scale(__float_as_uint(__ldcg(amax1)), 0);
   const float s2 = pow2_scale(__float_as_uint(__ldcg(scales + SCALE_AMAX_F2)), 0);
   scales[SCALE_F1] = s1;
   scales[SCALE_F2] = s2;
@@ -53,22 +54,26 @@ __device__ void grad_scales(float* scales) {
 
 // Largest |x| * premul of up to ABSMAX_MAX arrays, each as the bits of a non-negative float combined into its slot of
 // scales[] with atomicMax (integer order = float order for non-negative values; NaNs are ignored), one atomic per
-// block; the block that finishes last (SCALE_TICKET counts them, and is left at zero) turns the magnitudes into the
-// multipliers.  One launch in place of one per array and one for the multipliers.  grid (blocks, arrays), block 256.
+// block; the block that finishes last (SCALE_TICKET counts them, and is left at zero) turns the magnitudes of every level into the
+// multipliers.  One launch in place of one per array and one for the multipliers.  grid (blocks, rows: the samples of every array),
+// block 256.
 constexpr int AM_THREADS = 256, AM_UNROLL = 4;
 struct AbsmaxJobs {
-  const float* p[ABSMAX_MAX];
-  size_t n[ABSMAX_MAX];
-  float premul[ABSMAX_MAX];
-  int slot[ABSMAX_MAX];
+  AbsmaxSource src[ABSMAX_MAX];
+  int first_row[ABSMAX_MAX];   // of grid.y; sources that do not exist start past its end
 };
 __global__ void __launch_bounds__(AM_THREADS)
-absmax_kernel(const AbsmaxJobs jobs, float* scales, int gradients) {
+absmax_kernel(const __grid_constant__ AbsmaxJobs jobs, float* scales, int levels, int gradients) {
   __shared__ float red[AM_THREADS / 32];
-  const int job = blockIdx.y;
-  const float* x = jobs.p[job];
-  const size_t n = jobs.n[job], n4 = n / 4, stride = (size_t)gridDim.x * AM_THREADS;
-  const float4* x4 = reinterpret_cast<const float4*>(x);  // the arrays are 16-byte aligned
+  int job = 0;
+#pragma unroll
+  for (int j = 1; j < ABSMAX_MAX; ++j) job = (int)blockIdx.y >= jobs.first_row[j] ? j : job;
+  const AbsmaxSource& src = jobs.src[job];
+  const float* x = src.p + (size_t)(blockIdx.y - jobs.first_row[job]) * src.sb;
+  // a sample's channels may start off a 16-byte boundary: up to three values before the first vector, up to three behind the last
+  const size_t n = src.n, head = min((size_t)((16u - (reinterpret_cast<uintptr_t>(x) & 15u)) & 15u) / 4, n);
+  const size_t n4 = (n - head) / 4, stride = (size_t)gridDim.x * AM_THREADS;
+  const float4* x4 = reinterpret_cast<const float4*>(x + head);
   float m = 0.f;
   for (size_t i = (size_t)blockIdx.x * AM_THREADS + threadIdx.x; i < n4; i += AM_UNROLL * stride) {
     float4 v[AM_UNROLL];
@@ -78,7 +83,8 @@ absmax_kernel(const AbsmaxJobs jobs, float* scales, int gradients) {
     for (int j = 0; j < AM_UNROLL; ++j)
       m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
   }
-  if (blockIdx.x == 0 && threadIdx.x < n - 4 * n4) m = fmaxf(m, fabsf(__ldg(x + 4 * n4 + threadIdx.x)));
+  if (blockIdx.x == 0 && threadIdx.x < head) m = fmaxf(m, fabsf(__ldg(x + threadIdx.x)));
+  if (blockIdx.x == 0 && threadIdx.x < n - head - 4 * n4) m = fmaxf(m, fabsf(__ldg(x + head + 4 * n4 + threadIdx.x)));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
@@ -86,31 +92,38 @@ absmax_kernel(const AbsmaxJobs jobs, float* scales, int gradients) {
   if (threadIdx.x != 0) return;
 #pragma unroll
   for (int i = 1; i < AM_THREADS / 32; ++i) m = fmaxf(m, red[i]);
-  if (m > 0.f) atomicMax(reinterpret_cast<unsigned*>(scales) + jobs.slot[job], __float_as_uint(m * fabsf(jobs.premul[job])));
+  if (m > 0.f) atomicMax(reinterpret_cast<unsigned*>(scales) + src.slot, __float_as_uint(m * fabsf(src.premul)));
   __threadfence();
   unsigned* ticket = reinterpret_cast<unsigned*>(scales) + SCALE_TICKET;
   if (atomicAdd(ticket, 1u) != gridDim.x * gridDim.y - 1) return;
   __threadfence();
-  if (gradients) grad_scales(scales);
-  else feature_scales(scales);
+  for (int l = 0; l < levels; ++l) {
+    if (gradients) grad_scales(scales + l * SCALE_LEVEL);
+    else feature_scales(scales + l * SCALE_LEVEL, scales + SCALE_AMAX_F1);
+  }
   *ticket = 0;
 }
 
-cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, bool gradients, cudaStream_t stream) {
+cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int levels, bool gradients, cudaStream_t stream) {
   if (count < 1 || count > ABSMAX_MAX) return cudaErrorInvalidValue;
   AbsmaxJobs jobs;
   size_t most = 0;
+  long long rows = 0;
   for (int i = 0; i < ABSMAX_MAX; ++i) {
-    const AbsmaxSource& s = src[i < count ? i : 0];
-    jobs.p[i] = s.p;
-    jobs.n[i] = s.n;
-    jobs.premul[i] = s.premul;
-    jobs.slot[i] = s.slot;
-    most = std::max(most, s.n);
+    jobs.src[i] = src[i < count ? i : 0];
+    jobs.first_row[i] = i < count ? (int)rows : INT_MAX;
+    if (i >= count) continue;
+    if (src[i].sb == (long long)src[i].n) {   // samples that follow one another are one array
+      jobs.src[i].n *= src[i].samples;
+      jobs.src[i].samples = 1;
+    }
+    rows += jobs.src[i].samples;
+    most = std::max(most, jobs.src[i].n);
   }
+  if (rows > 65535) return cudaErrorInvalidConfiguration;
   const size_t per_block = (size_t)AM_THREADS * 4 * AM_UNROLL;
   const unsigned blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((most + per_block - 1) / per_block, 148 * 8));
-  absmax_kernel<<<dim3(blocks, count), AM_THREADS, 0, stream>>>(jobs, scales, gradients ? 1 : 0);
+  absmax_kernel<<<dim3(blocks, (unsigned)rows), AM_THREADS, 0, stream>>>(jobs, scales, levels, gradients ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -184,12 +197,26 @@ f2_means_kernel(const float* __restrict__ F2, float* __restrict__ aux, int H2, i
 // lane every 32nd column.  NV = ceil(W2 / 32) rounded up to a power of two: the column sums of a lane stay in registers, so
 // that the plane is read once, with FC_ROWS * NV loads of a lane in flight (HBM-bound; one walk for the rows and one for the
 // columns took 162 us at 8 x 135 x 240, C = 256).  NV = 0: any width, in the two walks.  Both add in the same order.
-// grid (C, B), block 256.
+// grid (C, B, levels), block 256.
 constexpr int FC_ROWS = 2;
+struct MeansJobs {
+  struct Job {
+    const float* fmap2;
+    float* aux;
+    uint16_t* auxh;
+    const float* scale16;
+    int H2, W2;
+  } j[MAX_FUSED_LEVELS];
+};
 template <int NV>
 __global__ void __launch_bounds__(256)
-f2_means_cf_kernel(const float* __restrict__ fmap2, float* __restrict__ aux, int H2, int W2, int C,
-                   uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
+f2_means_cf_kernel(const __grid_constant__ MeansJobs jobs, int C, int op16) {
+  const MeansJobs::Job& job = jobs.j[blockIdx.z];
+  const float* const fmap2 = job.fmap2;
+  float* const aux = job.aux;
+  uint16_t* const auxh = job.auxh;
+  const float* const scale16 = job.scale16;
+  const int H2 = job.H2, W2 = job.W2;
   __shared__ float red[8][NV > 0 ? NV : 1][33];
   const int c = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
@@ -441,18 +468,25 @@ cudaError_t launch_unpack(const float* src, void* dst, int B, int N1, int n1p, i
   return cudaGetLastError();
 }
 
-// (B, C, N) -> (B, N, C) for both images in one launch, scaled: as TF32 in `out` or as 16-bit operands in `outh` (the one
+// (B, C, N) -> (B, N, C) for all images of a call in one launch, scaled: as TF32 in `out` or as 16-bit operands in `outh` (the one
 // that is not wanted is null).  Tiles of 64 channels x 32 pixels through shared memory, so that a warp writes 64 channels
-// of a pixel, two per lane; the first t1 blocks of a row do image 1.  grid (t1 + t2, ceil(C/64), B), block (32, 8).
+// of a pixel, two per lane; image j has the blocks first[j] .. of a row.  grid (sum of the images' ceil(N/32), ceil(C/64), B), block
+// (32, 8).
 struct TransposeJob { const float* in; float* out; uint16_t* outh; const float* scale16; float scale; int N; };
+struct TransposeJobs {
+  TransposeJob j[1 + MAX_FUSED_LEVELS];
+  int first[1 + MAX_FUSED_LEVELS];   // images that do not exist start past the end of the grid
+};
 __global__ void __launch_bounds__(256)
-transpose_round_kernel(const TransposeJob j1, const TransposeJob j2, int t1, int C, int op16) {
+transpose_round_kernel(const __grid_constant__ TransposeJobs jobs, int C, int op16) {
   __shared__ float tile[64][33];
-  const bool first = (int)blockIdx.x < t1;
-  const TransposeJob& j = first ? j1 : j2;
+  int image = 0;
+#pragma unroll
+  for (int i = 1; i <= MAX_FUSED_LEVELS; ++i) image = (int)blockIdx.x >= jobs.first[i] ? i : image;
+  const TransposeJob& j = jobs.j[image];
   const int N = j.N;
   const float sc16 = (j.outh != nullptr && op16 == OP16_FP16 && j.scale16 != nullptr) ? __ldg(j.scale16) : 1.f;
-  const int b = blockIdx.z, p0 = ((int)blockIdx.x - (first ? 0 : t1)) * 32, c0 = blockIdx.y * 64;
+  const int b = blockIdx.z, p0 = ((int)blockIdx.x - jobs.first[image]) * 32, c0 = blockIdx.y * 64;
   const int tx = threadIdx.x, ty = threadIdx.y;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -549,35 +583,54 @@ cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, i
   return cudaGetLastError();
 }
 
-// Clears the workspace header (status word, scale slots) and, for FP16 operands, finds the two feature scales.
-static cudaError_t begin_prepare(const Dims& d, const float* F1, const float* F2, float premul1, int* status, int op16,
+// Clears the workspace header (status word, scale slots) and, for FP16 operands, finds the feature scales.
+static cudaError_t begin_prepare(const Dims* d, int levels, const float* F1, const float* const* F2, float premul1, int* status, int op16,
                                  float* scales, cudaStream_t stream) {
-  cudaError_t err = cudaMemsetAsync(status, 0, WS_HEADER_CLEAR_BYTES, stream);
+  cudaError_t err = cudaMemsetAsync(status, 0, WS_SCALES_OFFSET + (size_t)levels * SCALE_LEVEL * sizeof(float), stream);
   if (err != cudaSuccess || op16 != OP16_FP16 || scales == nullptr) return err;
-  const AbsmaxSource src[2] = {{F1, (size_t)d.B * d.N1() * d.C, premul1, SCALE_AMAX_F1},
-                               {F2, (size_t)d.B * d.N2() * d.C, 1.f, SCALE_AMAX_F2}};
-  return launch_absmax(src, 2, scales, false, stream);
+  AbsmaxSource src[1 + MAX_FUSED_LEVELS];
+  src[0] = absmax_array(F1, (size_t)d[0].B * d[0].N1() * d[0].C, premul1, SCALE_AMAX_F1);
+  for (int l = 0; l < levels; ++l)
+    src[1 + l] = absmax_array(F2[l], (size_t)d[l].B * d[l].N2() * d[l].C, 1.f, l * SCALE_LEVEL + SCALE_AMAX_F2);
+  return launch_absmax(src, 1 + levels, scales, levels, false, stream);
 }
 
-cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fmap2, float scale1, float* F1r,
-                              float* F2r, float* aux, int* status, cudaStream_t stream, uint16_t* F1h, uint16_t* F2h,
-                              uint16_t* auxh, int op16, float* scales) {
-  cudaError_t err = begin_prepare(d, fmap1, fmap2, scale1, status, op16, scales, stream);
+cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, const float* const* fmap2, float scale1,
+                              const LevelOperands* out, float* F1r, uint16_t* F1h, int* status, cudaStream_t stream, int op16, float* scales) {
+  if (levels < 1 || levels > MAX_FUSED_LEVELS) return cudaErrorInvalidValue;
+  cudaError_t err = begin_prepare(d, levels, fmap1, fmap2, scale1, status, op16, scales, stream);
   if (err != cudaSuccess) return err;
-  const float* s1 = (op16 == OP16_FP16 && scales != nullptr) ? scales + SCALE_F1 : nullptr;
-  const float* s2 = (op16 == OP16_FP16 && scales != nullptr) ? scales + SCALE_F2 : nullptr;
+  const bool scaled = op16 == OP16_FP16 && scales != nullptr;
+  const int B = d[0].B, C = d[0].C;
   if (F1r != nullptr || F1h != nullptr) {
-    const int t1 = (d.N1() + 31) / 32, t2 = (d.N2() + 31) / 32;
-    const TransposeJob j1{fmap1, F1r, F1h, s1, scale1, d.N1()}, j2{fmap2, F2r, F2h, s2, 1.f, d.N2()};
-    transpose_round_kernel<<<dim3(t1 + t2, (d.C + 63) / 64, d.B), dim3(32, 8), 0, stream>>>(j1, j2, t1, d.C, op16);
+    TransposeJobs jobs;
+    int blocks = (d[0].N1() + 31) / 32;
+    jobs.j[0] = TransposeJob{fmap1, F1r, F1h, scaled ? scales + SCALE_F1 : nullptr, scale1, d[0].N1()};
+    jobs.first[0] = 0;
+    for (int l = 0; l < MAX_FUSED_LEVELS; ++l) {
+      jobs.first[1 + l] = l < levels ? blocks : INT_MAX;
+      jobs.j[1 + l] = jobs.j[0];
+      if (l >= levels) continue;
+      jobs.j[1 + l] = TransposeJob{fmap2[l], out[l].F2r, out[l].F2h, scaled ? scales + l * SCALE_LEVEL + SCALE_F2 : nullptr, 1.f, d[l].N2()};
+      blocks += (d[l].N2() + 31) / 32;
+    }
+    transpose_round_kernel<<<dim3(blocks, (C + 63) / 64, B), dim3(32, 8), 0, stream>>>(jobs, C, op16);
   }
-  if (aux != nullptr || auxh != nullptr) {
-    auto kern = d.W2 <= 32    ? f2_means_cf_kernel<1>
-                : d.W2 <= 64  ? f2_means_cf_kernel<2>
-                : d.W2 <= 128 ? f2_means_cf_kernel<4>
-                : d.W2 <= 256 ? f2_means_cf_kernel<8>
-                              : f2_means_cf_kernel<0>;
-    kern<<<dim3(d.C, d.B), 256, 0, stream>>>(fmap2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
+  if (out[0].aux != nullptr || out[0].auxh != nullptr) {
+    MeansJobs jobs;
+    int W2 = 0;
+    for (int l = 0; l < MAX_FUSED_LEVELS; ++l) {
+      jobs.j[l] = jobs.j[0];
+      if (l >= levels) continue;
+      jobs.j[l] = MeansJobs::Job{fmap2[l], out[l].aux, out[l].auxh, scaled ? scales + l * SCALE_LEVEL + SCALE_F2 : nullptr, d[l].H2, d[l].W2};
+      W2 = std::max(W2, d[l].W2);
+    }
+    auto kern = W2 <= 32    ? f2_means_cf_kernel<1>
+                : W2 <= 64  ? f2_means_cf_kernel<2>
+                : W2 <= 128 ? f2_means_cf_kernel<4>
+                : W2 <= 256 ? f2_means_cf_kernel<8>
+                            : f2_means_cf_kernel<0>;
+    kern<<<dim3(C, B, levels), 256, 0, stream>>>(jobs, C, op16);
   }
   return cudaGetLastError();
 }
@@ -585,7 +638,7 @@ cudaError_t launch_prepare_cf(const Dims& d, const float* fmap1, const float* fm
 cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, float* F1r, float* F2r, float* aux,
                            int* status, cudaStream_t stream, uint16_t* F1h, uint16_t* F2h, uint16_t* auxh, int op16,
                            float* scales) {
-  cudaError_t err = begin_prepare(d, F1, F2, 1.f, status, op16, scales, stream);
+  cudaError_t err = begin_prepare(&d, 1, F1, &F2, 1.f, status, op16, scales, stream);
   if (err != cudaSuccess) return err;
   const float* s1 = (op16 == OP16_FP16 && scales != nullptr) ? scales + SCALE_F1 : nullptr;
   const float* s2 = (op16 == OP16_FP16 && scales != nullptr) ? scales + SCALE_F2 : nullptr;

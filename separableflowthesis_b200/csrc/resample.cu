@@ -5,6 +5,8 @@
 // float, lower neighbour by truncation, the upper neighbour clamped to the last row).  HBM-bound streaming kernels;
 // every output element is written once, the backward (the adjoint) has one thread per (sample, channel, pixel) walk
 // the displacement axis, so it needs no atomics.
+#include <climits>
+
 #include "kernels.h"
 
 namespace sfb {
@@ -22,8 +24,13 @@ __device__ __forceinline__ void resample_source(int d, float scale, int Dl, int&
 
 // A thread produces RS_DB output rows of its VEC neighbouring pixels, all loads first.  VEC = 4 (16-byte loads and stores)
 // when the planes allow it: a row is a coalesced store of two interpolated loads, and with 4-byte accesses the number of
-// instructions, not HBM, set the pace.  grid (ceil(N1/(128*VEC)), ceil(D0/RS_DB), B*K)
+// instructions, not HBM, set the pace.  grid (ceil(N1/(128*VEC)), sum over the volumes of ceil(D0/RS_DB), B*K)
 constexpr int RS_DB = 8;
+struct ResampleJobs {
+  ResampleJob j[MAX_RESAMPLE_JOBS];
+  float scale[MAX_RESAMPLE_JOBS];
+  int first[MAX_RESAMPLE_JOBS];   // of grid.y; volumes that do not exist start past its end
+};
 
 template <int VEC> struct RsVec;
 template <> struct RsVec<1> { typedef float type; };
@@ -35,13 +42,18 @@ __device__ __forceinline__ float4 rs_mix(const float4& a, const float4& b, float
 
 template <int VEC>
 __global__ void __launch_bounds__(RS_THREADS)
-upsample_displacement_kernel(const float* __restrict__ in, float* __restrict__ out, long long out_sb, int K, int Dl,
-                             int D0, int N1, float scale) {
+upsample_displacement_kernel(const __grid_constant__ ResampleJobs jobs, int K, int N1) {
   typedef typename RsVec<VEC>::type V;
-  const int p = (blockIdx.x * RS_THREADS + threadIdx.x) * VEC, d0 = blockIdx.y * RS_DB;
+  int ji = 0;
+#pragma unroll
+  for (int i = 1; i < MAX_RESAMPLE_JOBS; ++i) ji = (int)blockIdx.y >= jobs.first[i] ? i : ji;
+  const ResampleJob& job = jobs.j[ji];
+  const int Dl = job.Dl, D0 = job.D0;
+  const float scale = jobs.scale[ji];
+  const int p = (blockIdx.x * RS_THREADS + threadIdx.x) * VEC, d0 = (blockIdx.y - jobs.first[ji]) * RS_DB;
   if (p >= N1) return;
   const int b = blockIdx.z / K, k = blockIdx.z - b * K;
-  const float* src = in + ((size_t)blockIdx.z * Dl) * N1 + p;
+  const float* src = job.in + ((size_t)blockIdx.z * Dl) * N1 + p;
   V v0[RS_DB], v1[RS_DB];
   float l0[RS_DB], l1[RS_DB];
 #pragma unroll
@@ -51,7 +63,7 @@ upsample_displacement_kernel(const float* __restrict__ in, float* __restrict__ o
     v0[j] = __ldg(reinterpret_cast<const V*>(src + (size_t)i0 * N1));
     v1[j] = __ldg(reinterpret_cast<const V*>(src + (size_t)i1 * N1));
   }
-  float* dst = out + (size_t)b * out_sb + ((size_t)k * D0 + d0) * N1 + p;
+  float* dst = job.out + (size_t)b * job.out_sb + ((size_t)k * D0 + d0) * N1 + p;
 #pragma unroll
   for (int j = 0; j < RS_DB; ++j)
     if (d0 + j < D0) *reinterpret_cast<V*>(dst + (size_t)j * N1) = rs_mix(v0[j], v1[j], l0[j], l1[j]);
@@ -129,13 +141,23 @@ upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long g
 
 static float resample_scale(int Dl, int D0) { return D0 > 1 ? (float)(Dl - 1) / (float)(D0 - 1) : 0.f; }
 
-cudaError_t launch_upsample_displacement(const float* in, float* out, long long out_sb, int B, int K, int Dl, int D0,
-                                         int N1, cudaStream_t st) {
-  const bool vec = N1 % 4 == 0 && out_sb % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+cudaError_t launch_upsample_displacement(const ResampleJob* job, int count, int B, int K, int N1, cudaStream_t st) {
+  if (count < 1 || count > MAX_RESAMPLE_JOBS) return cudaErrorInvalidValue;
+  ResampleJobs jobs;
+  bool vec = N1 % 4 == 0;
+  int rows = 0;
+  for (int i = 0; i < MAX_RESAMPLE_JOBS; ++i) {
+    jobs.j[i] = job[i < count ? i : 0];
+    jobs.first[i] = i < count ? rows : INT_MAX;
+    jobs.scale[i] = resample_scale(jobs.j[i].Dl, jobs.j[i].D0);
+    if (i >= count) continue;
+    rows += (job[i].D0 + RS_DB - 1) / RS_DB;
+    vec = vec && job[i].out_sb % 4 == 0 && ((reinterpret_cast<uintptr_t>(job[i].in) | reinterpret_cast<uintptr_t>(job[i].out)) & 15u) == 0;
+  }
   const int px = RS_THREADS * (vec ? 4 : 1);
-  const dim3 grid((N1 + px - 1) / px, (D0 + RS_DB - 1) / RS_DB, B * K);
+  const dim3 grid((N1 + px - 1) / px, rows, B * K);
   auto kern = vec ? upsample_displacement_kernel<4> : upsample_displacement_kernel<1>;
-  kern<<<grid, RS_THREADS, 0, st>>>(in, out, out_sb, K, Dl, D0, N1, resample_scale(Dl, D0));
+  kern<<<grid, RS_THREADS, 0, st>>>(jobs, K, N1);
   return cudaGetLastError();
 }
 

@@ -675,19 +675,50 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
 }
 
 // ---------------------------------------------------------------------------------- kernel
+// What a launch works on: one pair of images, or the levels of a pyramid over the same image 1, whose tiles follow one another.
+template <int LEVELS>
+struct SweepLaunch {
+  CUtensorMap f1, f2[LEVELS], aux[LEVELS];
+  SweepArgs a[LEVELS];
+  int first_block[LEVELS + 1], first_tail[LEVELS + 1];   // of the sweep and of the fold; levels that do not exist have none
+};
+template <int LEVELS>
+__device__ __forceinline__ int level_of(const int (&first)[LEVELS + 1], int block) {
+  int level = 0;
+#pragma unroll
+  for (int l = 1; l < LEVELS; ++l) level = block >= first[l] ? l : level;
+  return level;
+}
+enum TileForm : int { TILES_WIDE = 0, TILES_NARROW = 1, TILES_BY_LEVEL = 2 };
+// f(std::true_type) for narrow tiles, f(std::false_type) for wide ones
+template <int FORM, class F>
+__device__ __forceinline__ void by_tile_form(const SweepArgs& a, F&& f) {
+  if constexpr (FORM == TILES_WIDE) f(std::false_type{});
+  else if constexpr (FORM == TILES_NARROW) f(std::true_type{});
+  else if (a.narrow) f(std::true_type{});
+  else f(std::false_type{});
+}
+
 // CUT: the launch has tail pieces.  A launch without any runs the kernel without their bookkeeping.
 // KC (compression): channels of the launch, 1, 2 or (three or four) 4.
-template <int MODE, bool CUT, int KC, bool NARROW>
+// LEVELS > 1: the levels of a pyramid in one launch.  The coarse ones have too few cells to fill the SMs (55 x 128: 8, 2 and 1 tiles per
+// pixel tile beside 28), and the finest leaves SMs idle in its last wave, which their tiles fill.  Both sweeps of four levels with their
+// folds, levels one after the other and together (us, four channels, FP16): 1 x 55 x 128 172 and 134, 4 x 55 x 128 422 and 360,
+// 1 x 135 x 240 1675 and 1558.
+template <int MODE, bool CUT, int KC, int FORM, int LEVELS>
 __global__ void __launch_bounds__(SW_THREADS, 1)
-sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ CUtensorMap tm_f2,
-             const __grid_constant__ CUtensorMap tm_aux, const SweepArgs a) {
-  if (!cta_has_work(a.status)) return;
+sweep_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch, int* status) {
+  if (!cta_has_work(status)) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw + pad);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int level = level_of<LEVELS>(launch.first_block, blockIdx.x);
+  const SweepArgs& a = launch.a[level];
+  const int block = LEVELS == 1 ? blockIdx.x : blockIdx.x - launch.first_block[level];
+  const CUtensorMap *const tm_f1 = &launch.f1, *const tm_f2 = &launch.f2[level], *const tm_aux = &launch.aux[level];
 
   if (threadIdx.x == 0) {
     mbar_init(&sm.f1_full, 1);
@@ -696,9 +727,9 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     for (int i = 0; i < SW_NMERGE; ++i) { mbar_init(&sm.merge[0][i], 4); mbar_init(&sm.merge[1][i], 4); }  // four warps of a group
     wait_ctl_init(&sm.ctl, a.wait_limit_ns);
     fence_barrier_init();
-    prefetch_tensormap(&tm_f1);
-    prefetch_tensormap(&tm_f2);
-    if (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG) prefetch_tensormap(&tm_aux);
+    prefetch_tensormap(tm_f1);
+    prefetch_tensormap(tm_f2);
+    if (MODE == SWEEP_MAXAVG || MODE == SWEEP_MAXARGAVG) prefetch_tensormap(tm_aux);
   }
   if (warp == 1) {
     tmem_alloc(&sm.tmem_base, SW_TMEM_COLS);
@@ -721,12 +752,15 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
   // follows there for SW_REGS_EPI.
   if (warp < 4) {
     set_max_registers<SW_REGS_ISSUE, false>();
-    const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, blockIdx.x);
-    if (warp == 0) {
-      if (lane == 0) sweep_producer<NARROW>(sm, a, sc, &tm_f1, &tm_f2, &tm_aux);
-    } else if (warp == 1) {
-      if (lane == 0) sweep_mma(sm, a, sc);
-    }
+    by_tile_form<FORM>(a, [&](auto narrow) {
+      constexpr bool NARROW = decltype(narrow)::value;
+      const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, block);
+      if (warp == 0) {
+        if (lane == 0) sweep_producer<NARROW>(sm, a, sc, tm_f1, tm_f2, tm_aux);
+      } else if (warp == 1) {
+        if (lane == 0) sweep_mma(sm, a, sc);
+      }
+    });
     __syncwarp();
     meet();
     if (warp == 1) {
@@ -736,19 +770,22 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
     return;
   }
   set_max_registers<SW_REGS_EPI, true>();
-  const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, blockIdx.x);
-  EpiCtx e;
-  const int q = warp & 3;  // tcgen05.ld lets a warp read TMEM lanes 32*(warp%4) .. +31 only
-  e.wg = (warp >> 2) - 1;
-  e.lane = lane;
-  e.p = sc.m0 + q * 32 + lane;
-  e.valid = e.p < a.n_valid;
-  e.tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-  e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
-  if constexpr (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT, NARROW>(sm, a, sc, e);
-  else if constexpr (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT, NARROW>(sm, a, sc, e);
-  else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC == 1 ? 1 : 2, KC <= 2, CUT, NARROW>(sm, a, sc, e);
-  else epilogue_dump<NARROW>(sm, a, sc, e);
+  by_tile_form<FORM>(a, [&](auto narrow) {
+    constexpr bool NARROW = decltype(narrow)::value;
+    const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, block);
+    EpiCtx e;
+    const int q = warp & 3;  // tcgen05.ld lets a warp read TMEM lanes 32*(warp%4) .. +31 only
+    e.wg = (warp >> 2) - 1;
+    e.lane = lane;
+    e.p = sc.m0 + q * 32 + lane;
+    e.valid = e.p < a.n_valid;
+    e.tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
+    if constexpr (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT, NARROW>(sm, a, sc, e);
+    else if constexpr (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT, NARROW>(sm, a, sc, e);
+    else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC == 1 ? 1 : 2, KC <= 2, CUT, NARROW>(sm, a, sc, e);
+    else epilogue_dump<NARROW>(sm, a, sc, e);
+  });
   __syncwarp();
   meet();
 }
@@ -759,12 +796,14 @@ sweep_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ 
 // the batch and the row range.  A kernel of its own, one thread per pixel and FOLD_ROWS rows: folded by the CTA that finished a
 // tile last, the 0.3 MB of a 55 x 128 tile with four channels took that one SM 16 us, most of it memory latency.
 constexpr int FOLD_ROWS = 4;
-template <int MODE>
-__global__ void __launch_bounds__(TILE_M) sweep_fold_kernel(const SweepArgs a) {
+template <int MODE, int LEVELS>
+__global__ void __launch_bounds__(TILE_M) sweep_fold_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch) {
   constexpr bool SUM = MODE == SWEEP_COMPRESS, ARG = MODE == SWEEP_MAXARGAVG;
+  const int level = level_of<LEVELS>(launch.first_tail, blockIdx.y);
+  const SweepArgs& a = launch.a[level];
   if (*reinterpret_cast<volatile int*>(a.status) != 0) return;
   const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M, H2 = a.d.H2;
-  const int tail = blockIdx.y, tile = a.whole_tiles + tail, b = tile / tiles_per_sample;
+  const int tail = LEVELS == 1 ? blockIdx.y : blockIdx.y - launch.first_tail[level], tile = a.whole_tiles + tail, b = tile / tiles_per_sample;
   const int px = threadIdx.x, p = (tile - b * tiles_per_sample) * TILE_M + px;
   if (p >= a.n_valid) return;
   const PixView& out = SUM ? a.ou : a.pu;
@@ -834,10 +873,45 @@ TileSplit sweep_split(const Dims& d, int slots, bool sums) {
   return r;
 }
 
-template <int MODE, bool CUT, int KC, bool NARROW>
-static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
-                              const CUtensorMap& tm_aux, cudaStream_t stream) {
-  auto kern = sweep_kernel<MODE, CUT, KC, NARROW>;
+// How the tiles of a pyramid's levels are cut when they share a launch, in the units of sweep_split.  The blocks start in the
+// order of the levels, so the short tiles of the coarse levels fill the gaps that the finest leaves: nothing is cut where its tiles
+// make more than a few waves.  Else the cut (the same for all tiles of a level) with the smallest makespan of that order.
+void sweep_split_levels(const Dims* d, int levels, int slots, bool sums, TileSplit* out) {
+  int n_ub[MAX_FUSED_LEVELS], n_vb[MAX_FUSED_LEVELS];
+  const int tiles = (int)((long long)d[0].B * ((d[0].N1() + TILE_M - 1) / TILE_M));
+  for (int l = 0; l < levels; ++l) {
+    const bool narrow = sweep_narrow(d[l], sums);
+    const int ut = narrow ? SWEEP_UT_NARROW : SWEEP_UT, vt = narrow ? SWEEP_VT_NARROW : SWEEP_VT;
+    n_ub[l] = (d[l].H2 + ut - 1) / ut;
+    n_vb[l] = (d[l].W2 + vt - 1) / vt;
+    out[l] = TileSplit{tiles, tiles, 1, 0, 0};
+  }
+  if (tiles > 4 * SM_COUNT) return;
+  int best_cut[2] = {1, 1};
+  double best = 0;
+  for (int n0 = 1; n0 <= std::min(n_vb[0], MAX_PIECES); ++n0) {
+    for (int n1 = 1; n1 <= (levels > 1 ? std::min(n_vb[1], n0) : 1); ++n1) {
+      BlockQueue queue;
+      for (int l = 0; l < levels; ++l) {
+        const int n = l == 0 ? n0 : (l == 1 ? n1 : 1), per = n_vb[l] / n, extra = n_vb[l] - per * n;
+        if (extra > 0) queue.add(tiles * extra, (per + 1) * n_ub[l] + 2);   // (the order inside a level does not matter much)
+        queue.add(tiles * (n - extra), per * n_ub[l] + 2);
+      }
+      const double cost = queue.makespan() + (n0 > 1 || n1 > 1 ? 2.0 : 0.0);
+      if (best == 0 || cost < 0.95 * best) { best = cost; best_cut[0] = n0; best_cut[1] = n1; }
+    }
+  }
+  for (int l = 0; l < std::min(levels, 2); ++l) {
+    const int n = best_cut[l];
+    if (n == 1) continue;
+    const int parts = sums ? n_vb[l] - piece_start(n_vb[l], n, 1) : n - 1;
+    out[l] = TileSplit{tiles, 0, n, parts, (size_t)tiles * parts * slots * d[l].H2 * TILE_M};
+  }
+}
+
+template <int MODE, bool CUT, int KC, int FORM, int LEVELS>
+static cudaError_t launch_one(SweepLaunch<LEVELS>& launch, int levels, cudaStream_t stream) {
+  auto kern = sweep_kernel<MODE, CUT, KC, FORM, LEVELS>;
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
     // A kernel that was compiled for fewer registers than the split takes would wait in setmaxnreg.inc without a limit.
@@ -847,47 +921,80 @@ static cudaError_t launch_one(const SweepArgs& a, const CUtensorMap& tm_f1, cons
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM_BYTES);
   });
   if (err != cudaSuccess) return err;
-  const int tiles_per_sample = (a.d.N1() + TILE_M - 1) / TILE_M;
-  const int tiles = a.d.B * tiles_per_sample;
-  const dim3 grid(a.whole_tiles + (tiles - a.whole_tiles) * a.pieces);
-  kern<<<grid, SW_THREADS, SW_SMEM_BYTES, stream>>>(tm_f1, tm_f2, tm_aux, a);
+  int blocks = 0, tails = 0, rows = 0;
+  for (int l = 0; l < LEVELS; ++l) {
+    launch.first_block[l] = blocks;
+    launch.first_tail[l] = tails;
+    if (l >= levels) continue;
+    const SweepArgs& a = launch.a[l];
+    const int cut = a.d.B * ((a.d.N1() + TILE_M - 1) / TILE_M) - a.whole_tiles;
+    blocks += a.whole_tiles + cut * a.pieces;
+    if (a.pieces > 1) {
+      tails += cut;
+      rows = std::max(rows, (MODE == SWEEP_COMPRESS ? a.kc : 1) * a.d.H2);
+    }
+  }
+  launch.first_block[LEVELS] = blocks;
+  launch.first_tail[LEVELS] = tails;
+  kern<<<blocks, SW_THREADS, SW_SMEM_BYTES, stream>>>(launch, launch.a[0].status);
   if constexpr (CUT) {
+    if (tails == 0) return cudaGetLastError();
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    const int rows = (MODE == SWEEP_COMPRESS ? a.kc : 1) * a.d.H2;
-    sweep_fold_kernel<MODE><<<dim3((rows + FOLD_ROWS - 1) / FOLD_ROWS, tiles - a.whole_tiles), TILE_M, 0, stream>>>(a);
+    sweep_fold_kernel<MODE, LEVELS><<<dim3((rows + FOLD_ROWS - 1) / FOLD_ROWS, tails), TILE_M, 0, stream>>>(launch);
   }
   return cudaGetLastError();
 }
 
-template <int MODE, bool CUT, int KC>
-static cudaError_t launch_width(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
-                                const CUtensorMap& tm_aux, cudaStream_t stream) {
-  return sweep_narrow(a.d, MODE == SWEEP_COMPRESS) ? launch_one<MODE, CUT, KC, true>(a, tm_f1, tm_f2, tm_aux, stream)
-                           : launch_one<MODE, CUT, KC, false>(a, tm_f1, tm_f2, tm_aux, stream);
-}
-
 template <int MODE, int KC>
-static cudaError_t launch_mode(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
-                               const CUtensorMap& tm_aux, cudaStream_t stream) {
-  return a.pieces > 1 ? launch_width<MODE, true, KC>(a, tm_f1, tm_f2, tm_aux, stream)
-                      : launch_width<MODE, false, KC>(a, tm_f1, tm_f2, tm_aux, stream);
+static cudaError_t launch_mode(const SweepArgs* a, int levels, const CUtensorMap& tm_f1, const CUtensorMap* tm_f2,
+                               const CUtensorMap* tm_aux, cudaStream_t stream) {
+  auto fill = [&](auto& launch) {
+    launch.f1 = tm_f1;
+    for (int l = 0; l < levels; ++l) {
+      launch.f2[l] = tm_f2[l];
+      launch.aux[l] = tm_aux[l];
+      launch.a[l] = a[l];
+      launch.a[l].narrow = sweep_narrow(a[l].d, MODE == SWEEP_COMPRESS);
+    }
+  };
+  if constexpr (MODE != SWEEP_DUMP) {
+    if (levels > 1) {
+      SweepLaunch<MAX_FUSED_LEVELS> launch{};
+      fill(launch);
+      return launch_one<MODE, true, KC, TILES_BY_LEVEL>(launch, levels, stream);
+    }
+  }
+  SweepLaunch<1> launch{};
+  fill(launch);
+  const bool narrow = launch.a[0].narrow;
+  if constexpr (MODE != SWEEP_DUMP) {
+    if (a->pieces > 1)
+      return narrow ? launch_one<MODE, true, KC, TILES_NARROW>(launch, 1, stream) : launch_one<MODE, true, KC, TILES_WIDE>(launch, 1, stream);
+  }
+  return narrow ? launch_one<MODE, false, KC, TILES_NARROW>(launch, 1, stream) : launch_one<MODE, false, KC, TILES_WIDE>(launch, 1, stream);
 }
 
-cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
-                         const CUtensorMap& tm_aux, cudaStream_t stream) {
-  switch (a.mode) {
-    case SWEEP_MAXAVG: return launch_mode<SWEEP_MAXAVG, 0>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_MAXARGAVG: return launch_mode<SWEEP_MAXARGAVG, 0>(a, tm_f1, tm_f2, tm_aux, stream);
-    case SWEEP_DUMP: return launch_width<SWEEP_DUMP, false, 0>(a, tm_f1, tm_f2, tm_aux, stream);
+cudaError_t launch_sweep_levels(const SweepArgs* a, int levels, const CUtensorMap& tm_f1, const CUtensorMap* tm_f2,
+                                const CUtensorMap* tm_aux, cudaStream_t stream) {
+  if (levels < 1 || levels > MAX_FUSED_LEVELS) return cudaErrorInvalidValue;
+  switch (a->mode) {
+    case SWEEP_MAXAVG: return launch_mode<SWEEP_MAXAVG, 0>(a, levels, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_MAXARGAVG: return launch_mode<SWEEP_MAXARGAVG, 0>(a, levels, tm_f1, tm_f2, tm_aux, stream);
+    case SWEEP_DUMP: return levels == 1 ? launch_mode<SWEEP_DUMP, 0>(a, 1, tm_f1, tm_f2, tm_aux, stream) : cudaErrorInvalidValue;
     case SWEEP_COMPRESS:
-      switch (a.kc) {
-        case 1: return launch_mode<SWEEP_COMPRESS, 1>(a, tm_f1, tm_f2, tm_aux, stream);
-        case 2: return launch_mode<SWEEP_COMPRESS, 2>(a, tm_f1, tm_f2, tm_aux, stream);
-        case 3: case 4: return launch_mode<SWEEP_COMPRESS, 4>(a, tm_f1, tm_f2, tm_aux, stream);
+      switch (a->kc) {
+        case 1: return launch_mode<SWEEP_COMPRESS, 1>(a, levels, tm_f1, tm_f2, tm_aux, stream);
+        case 2: return launch_mode<SWEEP_COMPRESS, 2>(a, levels, tm_f1, tm_f2, tm_aux, stream);
+        case 3: case 4: return launch_mode<SWEEP_COMPRESS, 4>(a, levels, tm_f1, tm_f2, tm_aux, stream);
         default: return cudaErrorInvalidValue;
       }
     default: return cudaErrorInvalidValue;
   }
+}
+
+cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
+                         const CUtensorMap& tm_aux, cudaStream_t stream) {
+  return launch_sweep_levels(&a, 1, tm_f1, &tm_f2, &tm_aux, stream);
 }
 
 }  // namespace sfb

@@ -248,9 +248,16 @@ class SeparationLevelFunction(Function):
 
 
 # --------------------------------------------------------------------------------------------------
-# All pyramid levels as one autograd node (core/corr.py:416-475): per level the one-call forward from the feature
-# maps, then its volumes are resampled along the displacement axis and written straight into their channel slice of
-# the concatenated outputs (the reference runs F.interpolate per level and torch.cat over levels).
+# All pyramid levels as one autograd node (core/corr.py:416-475): the maps of up to four levels go to the library in one call, which
+# runs every kernel once for all of them.  Else, per level, the one-call forward from the feature maps, whose volumes are
+# resampled along the displacement axis and written straight into their channel slice of the concatenated outputs (the reference runs
+# F.interpolate per level and torch.cat over levels).
+def _levels_together(fmap1, fmap2_levels, Kc):
+    H2, W2 = fmap2_levels[0].shape[2:]
+    return (fmap1.is_cuda and len(fmap2_levels) <= MemorySaver.PYRAMID_MAX_LEVELS and Kc <= MemorySaver.PYRAMID_MAX_CHANNELS
+            and all(f.shape[2] <= H2 and f.shape[3] <= W2 for f in fmap2_levels) and fmap1.shape[0] * (2 + Kc) <= 65535)
+
+
 class SeparationPyramidFunction(Function):
     @staticmethod
     def forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, *fmap2_levels):
@@ -260,6 +267,16 @@ class SeparationPyramidFunction(Function):
         H2, W2 = fmap2_levels[0].shape[2:]     # displacement ranges of the outputs (= H1, W1 unless image-1 rows are sharded)
         L, Kt = len(fmap2_levels), 2 + weight_u.shape[0]
         saved = []
+        ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, L
+        if _levels_together(fmap1, fmap2_levels, weight_u.shape[0]):
+            with torch.cuda.device_of(fmap1):
+                sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
+            if with_argmax:
+                saved = MemorySaver.separation_pyramid_saved(buffer, fmap1, fmap2_levels, weight_u.shape[0], True)
+                ctx.in_place = [t[0] is None for t in saved]
+                flat = [x for t in saved for x in t if x is not None]
+                ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, *flat)
+            return sep_u, sep_v
         with torch.cuda.device_of(fmap1):
             sep_u = torch.empty(B, Kt * L, W2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
             sep_v = torch.empty(B, Kt * L, H2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
@@ -273,7 +290,6 @@ class SeparationPyramidFunction(Function):
                     MemorySaver.upsample_displacement_into(su, sep_u, l * Kt)
                     MemorySaver.upsample_displacement_into(sv, sep_v, l * Kt)
                 saved.append((su, sv, am_u, am_v, a_u, a_v))
-        ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, L
         if with_argmax:
             # volumes written in place are saved as the outputs themselves
             ctx.in_place = [t[0] is None for t in saved]

@@ -7,6 +7,7 @@ allocates the outputs and calls the C ABI of ``libsepflow_b200.so`` on the curre
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 import threading
 from typing import Dict, List, Tuple
@@ -86,6 +87,14 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr() if t is not None else None)
 
 
+def _check_device_status(lib, name, ws, stream):
+    if os.environ.get("SFB_CHECK_DEVICE_STATUS", "0") == "1":
+        dev_status = ctypes.c_int32(0)
+        rc = lib.sfb_device_status(ctypes.c_void_p(ws.data_ptr()), ctypes.c_void_p(stream), ctypes.byref(dev_status))
+        if rc != _lib.SFB_OK:
+            raise RuntimeError(f"{name}: {lib.sfb_last_error().decode()}")
+
+
 def _call(name: str, op: int, shape: _lib.SfbShape, device: torch.device, tensors) -> None:
     lib = _lib.load()
     with torch.cuda.device(device):
@@ -100,12 +109,7 @@ def _call(name: str, op: int, shape: _lib.SfbShape, device: torch.device, tensor
                                 ctypes.c_void_p(stream))
         if rc != _lib.SFB_OK:
             raise RuntimeError(f"{name}: {lib.sfb_status_string(rc).decode()}: {lib.sfb_last_error().decode()}")
-        if os.environ.get("SFB_CHECK_DEVICE_STATUS", "0") == "1":
-            dev_status = ctypes.c_int32(0)
-            rc = lib.sfb_device_status(ctypes.c_void_p(ws.data_ptr()), ctypes.c_void_p(stream),
-                                       ctypes.byref(dev_status))
-            if rc != _lib.SFB_OK:
-                raise RuntimeError(f"{name}: {lib.sfb_last_error().decode()}")
+        _check_device_status(lib, name, ws, stream)
 
 
 def max_avg_forward(img1_features_l0: torch.Tensor, img2_features_lk: torch.Tensor) -> List[torch.Tensor]:
@@ -485,6 +489,70 @@ def separation_level_backward(img1_features_l0, img2_features_lk, weight_u, weig
           head + (weight_u, weight_v, sep_u, sep_v) + place + (am_u, am_v, a_u, a_v, g_sep_u, g_sep_v, gF1, gF2, gw_u,
                                                                gb_u, gw_v, gb_v))
     return [gF1, gF2, gw_u, gb_u, gw_v, gb_v]
+
+
+# ------------------------------------------------------------------------------------------------------
+# All levels of the call site's pyramid in one call (core/corr.py:416-475).
+PYRAMID_MAX_LEVELS, PYRAMID_MAX_CHANNELS = 4, 4
+
+
+def _pyramid_arrays(fmap2_levels):
+    n = len(fmap2_levels)
+    ptrs = (ctypes.c_void_p * n)(*[t.data_ptr() for t in fmap2_levels])
+    sizes = (ctypes.c_int32 * (2 * n))(*[t.shape[2] for t in fmap2_levels], *[t.shape[3] for t in fmap2_levels])
+    return ptrs, ctypes.addressof(sizes), ctypes.addressof(sizes) + 4 * n, sizes
+
+
+def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, bias_v, with_argmax, scale1):
+    """(sep_u, sep_v, saved): separation_level_forward of every level on the model's feature maps, resampled to the displacement range
+    of level 0 and concatenated; `saved` is what the backward needs beside the inputs and outputs (one flat buffer)."""
+    s = None
+    for f2 in fmap2_levels:
+        level = _check_fmaps(fmap1, f2)
+        s = s or level
+    dev = fmap1.device
+    s.Kc = _check_attention_params(weight_u, bias_u, "attention1", dev)
+    if _check_attention_params(weight_v, bias_v, "attention2", dev) != s.Kc:
+        raise RuntimeError("attention1 and attention2 must have the same number of output channels")
+    L = len(fmap2_levels)
+    Kt = (2 + s.Kc) * L
+    sep_u = torch.empty(s.B, Kt, s.W2, s.H1, s.W1, dtype=torch.float32, device=dev)
+    sep_v = torch.empty(s.B, Kt, s.H2, s.H1, s.W1, dtype=torch.float32, device=dev)
+    lib = _lib.load()
+    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels)
+    shape = ctypes.byref(s)
+    saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax)), 256), dtype=torch.uint8, device=dev)
+    with torch.cuda.device(dev):
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L), 256), dev, stream)
+        _raise_on(lib.sfb_separation_pyramid_forward(
+            fmap1.data_ptr(), ptrs, H2, W2, L, scale1, weight_u.data_ptr(), bias_u.data_ptr(), weight_v.data_ptr(), bias_v.data_ptr(),
+            sep_u.data_ptr(), sep_v.data_ptr(), saved.data_ptr(), saved.numel(), int(with_argmax), shape, ws.data_ptr(), ws.numel(),
+            stream), "sfb_separation_pyramid_forward")
+        _check_device_status(lib, "sfb_separation_pyramid_forward", ws, stream)
+    return sep_u, sep_v, saved
+
+
+def separation_pyramid_saved(saved, fmap1, fmap2_levels, Kc, with_argmax):
+    """Per level (sep_u, sep_v, argmax_u, argmax_v, a_u, a_v) as views of the buffer; the volumes of a level that lies in the outputs are
+    None, and so are the arg-max indices of a forward without them."""
+    B, _, H1, W1 = fmap1.shape
+    off, out = 0, []
+
+    def take(*size, dtype=torch.float32):
+        nonlocal off
+        n = 4 * math.prod(size)
+        view = saved[off:off + n].view(dtype).view(size)
+        off += (n + 255) // 256 * 256
+        return view
+
+    for f2 in fmap2_levels:
+        H2, W2 = f2.shape[2:]
+        in_place = f2.shape[2:] == fmap2_levels[0].shape[2:]
+        vols = (None, None) if in_place else (take(B, 2 + Kc, W2, H1, W1), take(B, 2 + Kc, H2, H1, W1))
+        am = (take(B, H2, H1, W1, dtype=torch.int32), take(B, W2, H1, W1, dtype=torch.int32)) if with_argmax else (None, None)
+        out.append((*vols, *am, take(B, Kc, W2, H1, W1), take(B, Kc, H2, H1, W1)))
+    return out
 
 
 # ------------------------------------------------------------------------------------------------------
