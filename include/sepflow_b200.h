@@ -230,12 +230,22 @@ int sfb_separation_level_backward_fmaps(const float* fmap1, const float* fmap2, 
  * volumes, attention weights and, with_argmax != 0, arg-max indices. */
 size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
                                           int32_t with_argmax);
-size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels);
+size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
+                                              int32_t backward);
 int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
                                    int32_t levels, float scale1, const float* weight_u, const float* bias_u,
                                    const float* weight_v, const float* bias_v, float* SEP_u, float* SEP_v, void* saved,
                                    size_t saved_bytes, int32_t with_argmax, const sfb_shape* shape, void* workspace,
                                    size_t workspace_bytes, void* stream);
+
+/* Gradients for upstream gradients gSEP_u / gSEP_v of the concatenated outputs, from what a forward with arg-max left in `saved`:
+ * gfmap1 (B,C,H1,W1) and gfmap2[l] (B,C,H2[l],W2[l]) (gfmap1 times scale1) and the attention parameters', all overwritten. */
+int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
+                                    int32_t levels, float scale1, const float* weight_u, const float* weight_v,
+                                    const float* SEP_u, const float* SEP_v, const void* saved, size_t saved_bytes,
+                                    const float* gSEP_u, const float* gSEP_v, float* gfmap1, float* const* gfmap2,
+                                    float* gweight_u, float* gbias_u, float* gweight_v, float* gbias_v,
+                                    const sfb_shape* shape, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Placement of one pyramid level's volumes into the concatenated outputs of the call site (core/corr.py:459-475:
  * F.interpolate(..., [D0,H1,W1], mode='trilinear', align_corners=True), then torch.cat over levels).  H1, W1 do not

@@ -459,19 +459,34 @@ static bool tileable(const AttentionDims& d, const void* x, long long sb) {
 // channel).  V = 0: any D, both arrays read twice.  The order of the sums depends on D only.  Eight warps for every D
 // took 66 us for the attention backward of 2 x 135 x 240 and four channels at D = 5 and, spilling at V = 32, 635 us at
 // D = 135; 55 and 554 now.
-// bias_partial: (Kc, B * pixel_blocks), the block's sum of gL.  grid pixel_blocks * B * Kc, block 32 * max(G, 8).
+// A block's sum of gL goes to its module's bias partials (Kc, rows).  grid of pixel_blocks * B * Kc blocks per job, block
+// 32 * max(G, 8).
+struct LogitGradJobs {
+  JobBlocks blocks;
+  struct Job {
+    const float* a;
+    float* g;
+    float* partial;   // of the module
+    int D, row0, rows;
+  } j[MAX_ATTENTION_JOBS];
+};
 __host__ __device__ constexpr int lg_warps(int G) { return G > 8 ? G : 8; }
 __host__ __device__ constexpr int lg_pixels(int G) { return lg_warps(G) / G * 32; }
 template <int G, int V, int MIN_BLOCKS>
 __global__ void __launch_bounds__(32 * lg_warps(G), MIN_BLOCKS)
-attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, float* __restrict__ bias_partial,
-                            int Kc, int D, int N1, unsigned pixel_blocks) {
+attention_logit_grad_kernel(const __grid_constant__ LogitGradJobs jobs, int Kc, int N1, unsigned pixel_blocks) {
+  const int ji = job_of(jobs.blocks, blockIdx.x);
+  const LogitGradJobs::Job& job = jobs.j[ji];
+  const float* __restrict__ const a = job.a;
+  float* __restrict__ const g = job.g;
+  const int D = job.D;
+  const unsigned block = blockIdx.x - jobs.blocks.first[ji];
   constexpr int WARPS = lg_warps(G);
   __shared__ float red[WARPS][32];
   __shared__ float bred[WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = warp % G;
-  const unsigned row = blockIdx.x / pixel_blocks;   // sample * Kc + channel
-  const unsigned pb = blockIdx.x - row * pixel_blocks;
+  const unsigned row = block / pixel_blocks;   // sample * Kc + channel
+  const unsigned pb = block - row * pixel_blocks;
   const int p = (int)pb * lg_pixels(G) + warp / G * 32 + lane;
   const bool in = p < N1;
   const size_t base = (size_t)row * D * N1 + (in ? p : 0);
@@ -524,8 +539,8 @@ attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, 
     float t = 0.f;
 #pragma unroll
     for (int i = 0; i < WARPS; ++i) t += bred[i];
-    const unsigned k = row % Kc, b = row / Kc, rows = gridDim.x / Kc;   // rows = B * pixel_blocks
-    bias_partial[(size_t)k * rows + (size_t)b * pixel_blocks + pb] = t;
+    const unsigned k = row % Kc, b = row / Kc;
+    job.partial[(size_t)k * job.rows + job.row0 + (size_t)b * pixel_blocks + pb] = t;
   }
 }
 
@@ -533,18 +548,27 @@ attention_logit_grad_kernel(const float* __restrict__ a, float* __restrict__ g, 
 // gX[c, d, h, w] = add[c, d, h, w] + sum_{k, td, th, tw} W[k, c, td, th, tw] * gL[k, d - td + 1, h - th + 1, w - tw + 1]
 // Channels k0 .. k0+KC-1 (weights in c_att_weights); a later chunk adds to what the earlier ones stored.
 // The walk is cut into pieces of `dc` displacements like the forward's.
-// grid (ceil(N1/128), B * pieces), block 128, dynamic shared memory PlaneRing<9*KC, IG_STAGES>::bytes().
+// grid of ceil(N1/128) * B * pieces blocks per job, block 128, dynamic shared memory PlaneRing<9*KC, IG_STAGES>::bytes().
 constexpr int IG_STAGES = 3;
+struct InputGradJobs {
+  JobBlocks blocks;
+  struct Job {
+    const float *gl, *add;
+    long long add_sb;
+    float* gx;
+    int D, dc, module;
+  } j[MAX_ATTENTION_JOBS];
+};
 
-template <int KC>
-__global__ void __launch_bounds__(AT_THREADS)
-attention_input_grad_kernel(const float* __restrict__ gl, const float* __restrict__ add, long long add_sb,
-                            float* __restrict__ gx, int accumulate, int Kc, int k0, int B, int D, int dc, int H1, int W1) {
-  extern __shared__ float ring_dyn[];
-  const int N1 = H1 * W1;
-  const int p = blockIdx.x * AT_THREADS + threadIdx.x, b = blockIdx.y % B, d0 = (blockIdx.y / B) * dc;
+template <int KC, int MODULE>
+__device__ __forceinline__ void input_grad_walk_gather(const InputGradJobs::Job& job, float* ring_dyn, int accumulate, int Kc, int k0, int b,
+                                                       int d0, int p, int H1, int W1) {
+  const float* __restrict__ const gl = job.gl;
+  const float* __restrict__ const add = k0 == 0 ? job.add : nullptr;
+  const long long add_sb = job.add_sb;
+  float* __restrict__ const gx = job.gx;
+  const int N1 = H1 * W1, D = job.D, dc = job.dc;
   const int d1 = min(d0 + dc, D), e0 = max(d0 - 1, 0), e1 = min(d1 + 1, D);
-  if (p >= N1) return;
   const int h = p / W1, w = p - h * W1;
   const Neighbourhood nb(h, w, H1, W1);
   const PlaneRing<9 * KC, IG_STAGES> ring(ring_dyn);
@@ -595,7 +619,7 @@ attention_input_grad_kernel(const float* __restrict__ gl, const float* __restric
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int td = 0; td < 3; ++td)
-            acc[c][td] = fmaf(v, c_att_weights[(k * 2 + c) * AT_TAPS + td * 9 + t], acc[c][td]);
+            acc[c][td] = fmaf(v, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + td * 9 + t], acc[c][td]);
       }
     if (e > d0) emit(e - 1);
 #pragma unroll
@@ -604,25 +628,54 @@ attention_input_grad_kernel(const float* __restrict__ gl, const float* __restric
   if (d1 == D) emit(D - 1);
 }
 
+template <int KC>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_input_grad_kernel(const __grid_constant__ InputGradJobs jobs, int accumulate, int Kc, int k0, int B, int H1, int W1) {
+  extern __shared__ float ring_dyn[];
+  const int ji = job_of(jobs.blocks, blockIdx.x);
+  const InputGradJobs::Job& job = jobs.j[ji];
+  const int N1 = H1 * W1, pb = (N1 + AT_THREADS - 1) / AT_THREADS;
+  const int r = blockIdx.x - jobs.blocks.first[ji], z = r / pb;
+  const int p = (r - z * pb) * AT_THREADS + threadIdx.x, b = z % B, d0 = (z / B) * job.dc;
+  if (p >= N1) return;
+  by_module(job.module, [&](auto m) { input_grad_walk_gather<KC, decltype(m)::value>(job, ring_dyn, accumulate, Kc, k0, b, d0, p, H1, W1); });
+}
+
 // ---- weight gradients ----------------------------------------------------------------------------------
 // gW[k, c, td, th, tw] = sum_{b, d, h, w} gL[k, d, h, w] * X[c, d + td - 1, h + th - 1, w + tw - 1]
-// grid (ceil(N1/128), B * pieces, 2 * ceil(Kc/KW)), block 128: a thread owns input channel c and KW output channels;
+// grid (ceil(N1/128) * B * pieces blocks per job, 2 * ceil(Kc/KW)), block 128: a thread owns input channel c and KW output channels;
 // its KW*27 sums live in registers, every X value it reads feeds 3*KW of them.  A piece is `dc` planes of X.
-// partial: (Kc * 2 * 27, gridDim.x * gridDim.y), one column per block, so that the reduction reads consecutive values.
+// partial: of the module, (Kc * 2 * 27, rows), one column per block, so that the reduction reads consecutive values.
 constexpr int WG_STAGES = 4;
+struct WeightGradJobs {
+  JobBlocks blocks;
+  struct Job {
+    const float* x;
+    long long x_sb;
+    const float* gl;
+    float* partial;
+    int D, dc, row0, rows;
+  } j[MAX_ATTENTION_JOBS];
+};
 
 template <int KW>
 __global__ void __launch_bounds__(AT_THREADS)
-attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const float* __restrict__ gl,
-                             float* __restrict__ partial, int Kc, int B, int D, int dc, int H1, int W1) {
+attention_weight_grad_kernel(const __grid_constant__ WeightGradJobs jobs, int Kc, int B, int H1, int W1) {
+  const int ji = job_of(jobs.blocks, blockIdx.x);
+  const WeightGradJobs::Job& job = jobs.j[ji];
+  const float* __restrict__ const x = job.x;
+  const float* __restrict__ const gl = job.gl;
+  const long long x_sb = job.x_sb;
+  const int D = job.D, dc = job.dc;
   constexpr int NV = 9 + KW;
   __shared__ float ring_mem[WG_STAGES * NV * AT_THREADS];
   __shared__ float red[(AT_THREADS / 32) * KW * AT_TAPS];
-  const int N1 = H1 * W1;
-  const int b = blockIdx.y % B, c = blockIdx.z & 1, k0 = (blockIdx.z >> 1) * KW;
-  const int e0 = (blockIdx.y / B) * dc, e1 = min(e0 + dc, D);
+  const int N1 = H1 * W1, pb = (N1 + AT_THREADS - 1) / AT_THREADS;
+  const int r = blockIdx.x - jobs.blocks.first[ji], z = r / pb;
+  const int b = z % B, c = blockIdx.y & 1, k0 = (blockIdx.y >> 1) * KW;
+  const int e0 = (z / B) * dc, e1 = min(e0 + dc, D);
   const size_t plane = (size_t)N1;
-  const int p = blockIdx.x * AT_THREADS + threadIdx.x;
+  const int p = (r - z * pb) * AT_THREADS + threadIdx.x;
   float acc[KW * AT_TAPS];  // [k][td][neighbour]
 #pragma unroll
   for (int i = 0; i < KW * AT_TAPS; ++i) acc[i] = 0.f;
@@ -689,8 +742,8 @@ attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const 
     for (int i = 0; i < KW * AT_TAPS; ++i) red[warp * KW * AT_TAPS + i] = acc[i];
   }
   __syncthreads();
-  const size_t rows = (size_t)gridDim.x * gridDim.y;
-  float* dst = partial + (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+  const size_t rows = job.rows;
+  float* dst = job.partial + job.row0 + r;
   for (int i = threadIdx.x; i < KW * AT_TAPS; i += AT_THREADS) {
     const int k = i / AT_TAPS, t = i - k * AT_TAPS;
     if (k0 + k >= Kc) continue;
@@ -701,18 +754,23 @@ attention_weight_grad_kernel(const float* __restrict__ x, long long x_sb, const 
   }
 }
 
-// out[i] = sum over rows of partial[i][row], for the weight gradients (blocks 0 .. weights.n - 1) and, in the same launch, the
-// bias gradients.  One block per column: thread t adds rows t, t + 256, ... in order, then the 256 partial sums are combined in
-// a fixed tree, so the result does not depend on scheduling (bit-reproducible).
-constexpr int RP_THREADS = 256;
-struct PartialSums { const float* partial; float* out; int rows, n; };
+// out[i] = sum over rows of partial[i][row], for the weight and bias gradients of both modules in one launch.  One block per column:
+// thread t adds rows t, t + 256, ... in order, then the 256 partial sums are combined in a fixed tree, so the result does not depend on
+// scheduling (bit-reproducible).
+constexpr int RP_THREADS = 256, RP_SUMS = 4;
+struct PartialSums {
+  const float* partial[RP_SUMS];
+  float* out[RP_SUMS];
+  int rows[RP_SUMS], first[RP_SUMS + 1];   // blocks first[i] .. first[i+1]-1
+};
 __global__ void __launch_bounds__(RP_THREADS)
-attention_reduce_partials_kernel(const PartialSums weights, const PartialSums biases) {
+attention_reduce_partials_kernel(const __grid_constant__ PartialSums sums) {
   __shared__ float red[RP_THREADS];
-  const bool w = (int)blockIdx.x < weights.n;
-  const float* __restrict__ const partial = w ? weights.partial : biases.partial;
-  float* const out = w ? weights.out : biases.out;
-  const int rows = w ? weights.rows : biases.rows, i = w ? blockIdx.x : blockIdx.x - weights.n;
+  int j = 0;
+#pragma unroll
+  for (int i = 1; i < RP_SUMS; ++i) j = (int)blockIdx.x >= sums.first[i] ? i : j;
+  const int rows = sums.rows[j], i = blockIdx.x - sums.first[j];
+  const float* __restrict__ const partial = sums.partial[j];
   float s = 0.f;
   for (int r = threadIdx.x; r < rows; r += RP_THREADS) s += __ldg(partial + (size_t)i * rows + r);
   red[threadIdx.x] = s;
@@ -722,47 +780,21 @@ attention_reduce_partials_kernel(const PartialSums weights, const PartialSums bi
     if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[i] = red[0];
+  if (threadIdx.x == 0) sums.out[j][i] = red[0];
 }
 
 // ---- input and weight gradients, pixel tiles fetched by TMA -------------------------------------------------
 // Same arithmetic as the two gather kernels above with the tile scheme of attention_logits_tiled_kernel.
 // Input gradients: the stage holds the tile (with halo) of the KC logit-gradient channels of one plane.
-template <int KC>
-__global__ void __launch_bounds__(AT_THREADS + 32)
-attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, const float* __restrict__ add,
-                                  long long add_sb, float* __restrict__ gx, int accumulate, int k0, int B, int D,
-                                  int dc, int H1, int W1, int* status) {
-  if (!cta_has_work(status)) return;
-  __shared__ __align__(128) AttentionTileSmem<KC> sm;
-  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH, b = blockIdx.z % B, d0 = (blockIdx.z / B) * dc;
-  const int d1 = min(d0 + dc, D);
-  const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, D) - e0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
-    wait_ctl_init(&sm.ctl, 0);
-    fence_barrier_init();
-    prefetch_tensormap(&tm_gl);
-  }
-  __syncthreads();
-  if (warp == AT_THREADS / 32) {  // producer
-    if (lane == 0) {
-      for (int i = 0; i < n_planes; ++i) {
-        const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
-        mbar_expect_tx(&sm.full[s], KC * AT_TILE_BYTES);
-        tma_load_5d(sm.x[s].v, &tm_gl, &sm.full[s], w0 - 4, h0 - 1, e0 + i, k0, b);
-      }
-    }
-    return;
-  }
-  const int tx = lane, ty = warp;
-  const int h = h0 + ty, w = w0 + tx;
+template <int KC, int MODULE>
+__device__ __forceinline__ void input_grad_walk_tiled(AttentionTileSmem<KC>& sm, const InputGradJobs::Job& job, const TileBlock& t,
+                                                      int accumulate, int k0, int d0, int d1, int e0, int n_planes, int ty, int tx, int H1,
+                                                      int W1, int* status) {
+  const int D = job.D, h = t.h0 + ty, w = t.w0 + tx;
   const bool valid = h < H1 && w < W1;
   const size_t plane = (size_t)H1 * W1, p = valid ? (size_t)h * W1 + w : 0;
-  float* o0 = gx + (size_t)b * 2 * D * plane + p;
-  const float* ad = add != nullptr ? add + (size_t)b * add_sb + p : nullptr;
+  float* o0 = job.gx + (size_t)t.b * 2 * D * plane + p;
+  const float* ad = job.add != nullptr && k0 == 0 ? job.add + (size_t)t.b * job.add_sb + p : nullptr;
   float acc[2][3];  // [c][output d = e-1, e, e+1]
 #pragma unroll
   for (int c = 0; c < 2; ++c) acc[c][0] = acc[c][1] = acc[c][2] = 0.f;
@@ -780,25 +812,24 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
   for (int i = 0; i < n_planes; ++i) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
     const int e = e0 + i;
     const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-    const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
-    if (!__all_sync(0xffffffffu, ok)) { let_copies_land(); return; }
+    if (!mbar_wait_warp(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE)) return;
     float v[KC][9];
 #pragma unroll
     for (int k = 0; k < KC; ++k)
 #pragma unroll
       for (int n = 0; n < 9; ++n) v[k][n] = sm.x[s].v[k][ty + n / 3][tx + 3 + n % 3];
-    hand_back_stage(&sm.empty[s], lane);
+    hand_back_stage(&sm.empty[s], tx);
 #pragma unroll
     for (int k = 0; k < KC; ++k)
 #pragma unroll
       for (int n = 0; n < 9; ++n) {
         // neighbour n = (nh, nw) holds gL at (h + nh - 1, w + nw - 1), which meets tap th = 2 - nh, tw = 2 - nw
-        const int t = (2 - n / 3) * 3 + (2 - n % 3);
+        const int tap = (2 - n / 3) * 3 + (2 - n % 3);
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int td = 0; td < 3; ++td)
-            acc[c][td] = fmaf(v[k][n], c_att_weights[(k * 2 + c) * AT_TAPS + td * 9 + t], acc[c][td]);
+            acc[c][td] = fmaf(v[k][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + td * 9 + tap], acc[c][td]);
       }
     if (e > d0) emit(e - 1);
 #pragma unroll
@@ -807,12 +838,45 @@ attention_input_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_gl, con
   if (d1 == D) emit(D - 1);
 }
 
+template <int KC>
+__global__ void __launch_bounds__(AT_THREADS + 32)
+attention_input_grad_tiled_kernel(const __grid_constant__ TileMaps maps, const __grid_constant__ InputGradJobs jobs, int accumulate, int k0,
+                                  int B, int H1, int W1, int* status) {
+  if (!cta_has_work(status)) return;
+  __shared__ __align__(128) AttentionTileSmem<KC> sm;
+  const int ji = job_of(jobs.blocks, blockIdx.x);
+  const InputGradJobs::Job& job = jobs.j[ji];
+  const TileBlock t = tile_block(blockIdx.x - jobs.blocks.first[ji], B, H1, W1);
+  const int d0 = t.piece * job.dc, d1 = min(d0 + job.dc, job.D);
+  const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, job.D) - e0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
+    wait_ctl_init(&sm.ctl, 0);
+    fence_barrier_init();
+    prefetch_tensormap(&maps.m[ji]);
+  }
+  __syncthreads();
+  if (warp == AT_THREADS / 32) {
+    if (lane == 0) tile_producer<KC>(sm, &maps.m[ji], t, e0, n_planes, k0, status);
+    __syncwarp();
+  } else {
+    by_module(job.module, [&](auto m) {
+      input_grad_walk_tiled<KC, decltype(m)::value>(sm, job, t, accumulate, k0, d0, d1, e0, n_planes, warp, lane, H1, W1, status);
+    });
+  }
+  __syncthreads();
+  if (wait_ctl_aborted(&sm.ctl)) {
+    let_copies_land();
+  }
+}
+
 // Weight gradients: warps 0-3 own input channel 0, warps 4-7 input channel 1, each thread KW output channels of its
 // pixel; the stage holds the tile (with halo) of plane e of both X channels and the tile (without halo) of plane e+1 of
 // the KW logit-gradient channels, which the two halves share.  The sums of two output channels are one packed pair
 // (fma.rn.f32x2 with the X value in both halves), which halves the multiply-add instructions; KW odd leaves one
 // channel on scalar ones.  A piece is `dc` planes of X.
-// grid (ceil(W1/32), ceil(H1/4), B * chunks * pieces); partial: (Kc * 2 * 27, tiles * B * pieces).
+// grid (ceil(W1/32) * ceil(H1/4) * B * pieces blocks per job, chunks of KW channels); partial: of the module, (Kc * 2 * 27, rows).
 constexpr int WG_WARPS = 8;
 template <int KW>
 struct WeightGradTileSmem {
@@ -828,22 +892,25 @@ struct WeightGradTileSmem {
 
 template <int KW>
 __global__ void __launch_bounds__(WG_WARPS * 32 + 32, 1)
-attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_gl,
-                                   const float* __restrict__ gl, float* __restrict__ partial, int Kc, int B, int D,
-                                   int dc, int chunks, int H1, int W1, int* status) {
+attention_weight_grad_tiled_kernel(const __grid_constant__ TileMaps maps_x, const __grid_constant__ TileMaps maps_gl,
+                                   const __grid_constant__ WeightGradJobs jobs, int Kc, int B, int H1, int W1, int* status) {
   if (!cta_has_work(status)) return;
   __shared__ __align__(128) WeightGradTileSmem<KW> sm;
   constexpr int KP = KW / 2;   // packed channel pairs
-  const int w0 = blockIdx.x * AT_TW, h0 = blockIdx.y * AT_TH;
-  const int b = blockIdx.z % B, zr = blockIdx.z / B, k0 = (zr % chunks) * KW, piece = zr / chunks;
-  const int e0 = piece * dc, n_planes = min(dc, D - e0);
+  const int ji = job_of(jobs.blocks, blockIdx.x), r = blockIdx.x - jobs.blocks.first[ji];
+  const WeightGradJobs::Job& job = jobs.j[ji];
+  const TileBlock tb = tile_block(r, B, H1, W1);
+  const int w0 = tb.w0, h0 = tb.h0, b = tb.b, k0 = blockIdx.y * KW, D = job.D;
+  const float* __restrict__ const gl = job.gl;
+  const CUtensorMap *const tm_x = &maps_x.m[ji], *const tm_gl = &maps_gl.m[ji];
+  const int e0 = tb.piece * job.dc, n_planes = min(job.dc, D - e0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], WG_WARPS); }
     wait_ctl_init(&sm.ctl, 0);
     fence_barrier_init();
-    prefetch_tensormap(&tm_x);
-    prefetch_tensormap(&tm_gl);
+    prefetch_tensormap(tm_x);
+    prefetch_tensormap(tm_gl);
   }
   __syncthreads();
   if (warp == WG_WARPS) {  // producer
@@ -852,8 +919,8 @@ attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, con
         const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
         if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
         mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES + KW * AT_TH * AT_TW * (uint32_t)sizeof(float));
-        tma_load_5d(sm.st[s].x, &tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
-        tma_load_5d(sm.st[s].g, &tm_gl, &sm.full[s], w0, h0, e0 + i + 1, k0, b);  // plane D, channels >= Kc read as zero
+        tma_load_5d(sm.st[s].x, tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
+        tma_load_5d(sm.st[s].g, tm_gl, &sm.full[s], w0, h0, e0 + i + 1, k0, b);  // plane D, channels >= Kc read as zero
       }
     }
     return;
@@ -934,9 +1001,8 @@ attention_weight_grad_tiled_kernel(const __grid_constant__ CUtensorMap tm_x, con
     for (int t = 0; t < AT_TAPS; ++t) put((KW - 1) * AT_TAPS + t, acc1[t]);
   }
   named_bar_sync(1, WG_WARPS * 32);
-  const int tiles = gridDim.x * gridDim.y;
-  const size_t rows = (size_t)tiles * (gridDim.z / chunks);
-  float* dst = partial + ((size_t)piece * B + b) * tiles + blockIdx.y * gridDim.x + blockIdx.x;
+  const size_t rows = job.rows;
+  float* dst = job.partial + job.row0 + r;
   for (int i = threadIdx.x; i < 2 * KW * AT_TAPS; i += WG_WARPS * 32) {
     const int cc = i / (KW * AT_TAPS), j = i - cc * KW * AT_TAPS, k = j / AT_TAPS, t = j - k * AT_TAPS;
     if (k0 + k >= Kc) continue;
@@ -1012,20 +1078,25 @@ static int walk_length(size_t blocks, int D, int target = AT_BLOCKS_TARGET, int 
   const int least = D < min_walk ? D : min_walk;
   return dc > least ? dc : least;
 }
-// No walk of at most D displacements over these blocks has more pieces than this.
-static size_t walk_pieces_bound(size_t blocks, int D, int target, int min_walk) {
-  const size_t pieces = (target + blocks - 1) / blocks, most = (size_t)(D + min_walk - 1) / min_walk;
-  return pieces < most ? pieces : most;
+// Displacements per block of the weight gradients' walk, and the blocks of a job (partial sums of a weight).  The jobs of a launch fill the
+// SMs together.
+static int weight_walk(const AttentionDims& d, int jobs, bool tiled) {
+  return walk_length((tiled ? tile_count(d) : 2 * (size_t)pixel_grid(d).x) * d.B * jobs, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
 }
+static size_t weight_rows(const AttentionDims& d, int jobs, bool tiled) {
+  const int dc = weight_walk(d, jobs, tiled);
+  return (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * ((d.D + dc - 1) / dc);
+}
+// The softmax backward: pixels of a block by the length of the column (attention_logit_grad_kernel).
+static int logit_grad_pixels(int D) { return D <= 8 ? lg_pixels(1) : D <= 16 ? lg_pixels(2) : D <= 32 ? lg_pixels(4) : 32; }
+static size_t bias_rows(const AttentionDims& d) { return (size_t)d.B * ((d.H1 * d.W1 + logit_grad_pixels(d.D) - 1) / logit_grad_pixels(d.D)); }
 
-// Bias partials per block of at least 32 pixels, weight partials per block / tile and piece of the walk.  An upper bound that does
-// not fall when D grows: a level's two calls share one buffer sized for the larger D.
-size_t attention_partial_floats(const AttentionDims& d) {
-  const size_t blocks = (size_t)pixel_grid(d).x * d.B, tiles = tile_count(d) * d.B;
-  const size_t gather = blocks * walk_pieces_bound(2 * blocks, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
-  const size_t tiled = tiles * walk_pieces_bound(tiles, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
-  const size_t bias = (size_t)d.B * (((size_t)d.H1 * d.W1 + 31) / 32);
-  return d.Kc * (bias + 2 * AT_TAPS * (gather > tiled ? gather : tiled));
+// Bias partials per block of the softmax backward, weight partials per block of the weight gradients, whichever form they take.
+size_t attention_partial_floats(const AttentionDims* d, int count) {
+  size_t floats = 0;
+  for (int i = 0; i < count; ++i)
+    floats += d[i].Kc * (bias_rows(d[i]) + 2 * AT_TAPS * std::max(weight_rows(d[i], count, true), weight_rows(d[i], count, false)));
+  return floats;
 }
 
 // Columns of a class of lengths are done by one launch.
@@ -1144,107 +1215,180 @@ cudaError_t launch_attention_forward(const AttentionJob* job, int count, const A
 }
 
 template <int KC>
-static cudaError_t launch_input_grad(const dim3 grid, const float* g, const float* add, long long add_sb, float* gx,
-                                     int accumulate, const AttentionDims& d, int dc, int k0, cudaStream_t st) {
+static cudaError_t launch_input_grad(unsigned blocks, const InputGradJobs& jobs, int accumulate, const AttentionDims& d, int k0,
+                                     cudaStream_t st) {
   constexpr size_t smem = PlaneRing<9 * KC, IG_STAGES>::bytes();
-  static bool configured[AT_MAX_DEVICES] = {false};  // benign race: setting the attribute twice is harmless
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return err;
-  if (smem > 48 * 1024 && dev >= 0 && dev < AT_MAX_DEVICES && !configured[dev]) {
-    err = cudaFuncSetAttribute(attention_input_grad_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static DeviceOnce configured;
+  if (smem > 48 * 1024) {
+    cudaError_t err = configured.run(
+        [&] { return cudaFuncSetAttribute(attention_input_grad_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
     if (err != cudaSuccess) return err;
-    configured[dev] = true;
   }
-  attention_input_grad_kernel<KC><<<grid, AT_THREADS, smem, st>>>(g, add, add_sb, gx, accumulate, d.Kc, k0, d.B, d.D, dc,
-                                                                  d.H1, d.W1);
+  attention_input_grad_kernel<KC><<<blocks, AT_THREADS, smem, st>>>(jobs, accumulate, d.Kc, k0, d.B, d.H1, d.W1);
   return cudaGetLastError();
 }
 
-// rows: bias partials per channel, B * pixel blocks
-static cudaError_t launch_logit_grad(const AttentionDims& d, const float* a, float* g, float* bias_partial, int* rows,
-                                     cudaStream_t st) {
-  const int N1 = d.H1 * d.W1;
-  auto launch = [&](auto kern, int G) {
-    const unsigned pb = (unsigned)((N1 + lg_pixels(G) - 1) / lg_pixels(G));
-    if ((unsigned long long)pb * d.B * d.Kc > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-    *rows = (int)(pb * (unsigned)d.B);
-    kern<<<pb * (unsigned)(d.B * d.Kc), 32 * lg_warps(G), 0, st>>>(a, g, bias_partial, d.Kc, d.D, N1, pb);
-    return cudaGetLastError();
-  };
-  if (d.D <= 8) return launch(attention_logit_grad_kernel<1, 8, 5>, 1);
-  if (d.D <= 16) return launch(attention_logit_grad_kernel<2, 8, 6>, 2);
-  if (d.D <= 32) return launch(attention_logit_grad_kernel<4, 8, 6>, 4);
-  if (d.D <= 64) return launch(attention_logit_grad_kernel<8, 8, 6>, 8);
-  if (d.D <= 128) return launch(attention_logit_grad_kernel<8, 16, 3>, 8);
-  if (d.D <= 160) return launch(attention_logit_grad_kernel<16, 10, 2>, 16);
-  if (d.D <= 256) return launch(attention_logit_grad_kernel<16, 16, 2>, 16);
-  return launch(attention_logit_grad_kernel<8, 0, 6>, 8);
+// A job's place among the partial sums of its module.
+struct PartialPlace {
+  float *bias, *weight;   // of the module
+  int bias_row0, bias_rows, weight_row0, weight_rows;
+};
+
+// Softmax backward of the jobs with above < D <= upto, by one launch.
+template <int G, int V, int MIN_BLOCKS>
+static cudaError_t launch_logit_grad_class(const AttentionGradJob* job, const PartialPlace* place, int count, int above, int upto,
+                                           cudaStream_t st) {
+  LogitGradJobs jobs{};
+  const AttentionDims& d = job[0].d;
+  const unsigned pb = (unsigned)((d.H1 * d.W1 + lg_pixels(G) - 1) / lg_pixels(G));
+  unsigned long long blocks = 0;
+  int n = 0;
+  for (int i = 0; i < count; ++i) {
+    if (job[i].d.D <= above || job[i].d.D > upto) continue;
+    jobs.j[n] = LogitGradJobs::Job{job[i].a, job[i].g, place[i].bias, job[i].d.D, place[i].bias_row0, place[i].bias_rows};
+    jobs.blocks.first[n++] = (int)blocks;
+    blocks += (unsigned long long)pb * d.B * d.Kc;
+    if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+  }
+  if (n == 0) return cudaSuccess;
+  for (; n <= MAX_ATTENTION_JOBS; ++n) jobs.blocks.first[n] = (int)blocks;
+  attention_logit_grad_kernel<G, V, MIN_BLOCKS><<<(unsigned)blocks, 32 * lg_warps(G), 0, st>>>(jobs, d.Kc, d.H1 * d.W1, pb);
+  return cudaGetLastError();
+}
+static int logit_grad_class(int D) {
+  for (const int c : {8, 16, 32, 64, 128, 160, 256})
+    if (D <= c) return c;
+  return 0;
+}
+static cudaError_t launch_logit_grad(const AttentionGradJob* job, const PartialPlace* place, int count, cudaStream_t st) {
+  cudaError_t err;
+  if ((err = launch_logit_grad_class<1, 8, 5>(job, place, count, 0, 8, st)) != cudaSuccess) return err;
+  if ((err = launch_logit_grad_class<2, 8, 6>(job, place, count, 8, 16, st)) != cudaSuccess) return err;
+  if ((err = launch_logit_grad_class<4, 8, 6>(job, place, count, 16, 32, st)) != cudaSuccess) return err;
+  if ((err = launch_logit_grad_class<8, 8, 6>(job, place, count, 32, 64, st)) != cudaSuccess) return err;
+  if ((err = launch_logit_grad_class<8, 16, 3>(job, place, count, 64, 128, st)) != cudaSuccess) return err;
+  if ((err = launch_logit_grad_class<16, 10, 2>(job, place, count, 128, 160, st)) != cudaSuccess) return err;
+  if ((err = launch_logit_grad_class<16, 16, 2>(job, place, count, 160, 256, st)) != cudaSuccess) return err;
+  return launch_logit_grad_class<8, 0, 6>(job, place, count, 256, INT_MAX, st);
 }
 
-cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
-                                      const float* a, float* g, const float* add, long long add_sb, float* gx,
-                                      float* gweight, float* gbias, float* partial, cudaStream_t st, int* status) {
+int attention_backward_launches(const AttentionGradJob* job, int count) {
+  int n = (job[0].d.Kc + AT_KC - 1) / AT_KC + 2;   // input gradients per chunk of channels, weight gradients, the reduction
+  for (int i = 0; i < count; ++i) {
+    bool first = true;   // of its class of lengths
+    for (int k = 0; k < i; ++k) first = first && logit_grad_class(job[k].d.D) != logit_grad_class(job[i].d.D);
+    n += first ? 1 : 0;
+  }
+  return n;
+}
+
+cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, const AttentionModules& modules,
+                                      const AttentionGradients& grads, float* partial, cudaStream_t st, int* status) {
+  if (count < 1 || count > MAX_ATTENTION_JOBS) return cudaErrorInvalidValue;
+  const AttentionDims& d = job[0].d;
   const int N1 = d.H1 * d.W1;
-  const size_t blocks = (size_t)pixel_grid(d).x * d.B, tiles = tile_count(d) * d.B;
-  int bias_rows = 0;
-  float* bias_partial = partial;                               // (Kc, bias_rows), bias_rows <= B * ceil(N1/32)
-  float* weight_partial = partial + (size_t)d.B * ((N1 + 31) / 32) * d.Kc;  // (Kc * 54, blocks or tiles times pieces)
-  const long long g_sb = (long long)d.Kc * d.D * N1;
-  const bool tiled = status != nullptr && tileable(d, x, x_sb) && tileable(d, g, g_sb);
-  cudaError_t err = launch_logit_grad(d, a, g, bias_partial, &bias_rows, st);
+  auto g_sb = [&](const AttentionGradJob& j) { return (long long)d.Kc * j.d.D * N1; };
+  bool tiled = status != nullptr;
+  for (int i = 0; i < count; ++i) tiled = tiled && tileable(job[i].d, job[i].x, job[i].x_sb) && tileable(job[i].d, job[i].g, g_sb(job[i]));
+
+  // partial sums: per module the bias partials (Kc, rows), then the weight partials (Kc * 54, rows)
+  PartialPlace place[MAX_ATTENTION_JOBS];
+  PartialSums sums{};
+  int columns = 0;
+  for (int m = 0; m < 2; ++m) {
+    int brows = 0, wrows = 0;
+    for (int i = 0; i < count; ++i) {
+      if (job[i].module != m) continue;
+      place[i].bias_row0 = brows;
+      place[i].weight_row0 = wrows;
+      brows += (int)bias_rows(job[i].d);
+      wrows += (int)weight_rows(job[i].d, count, tiled);
+    }
+    float *const bias = partial, *const weight = bias + (size_t)brows * d.Kc;
+    partial = weight + (size_t)wrows * d.Kc * 2 * AT_TAPS;
+    for (int i = 0; i < count; ++i) {
+      if (job[i].module != m) continue;
+      place[i].bias = bias;
+      place[i].weight = weight;
+      place[i].bias_rows = brows;
+      place[i].weight_rows = wrows;
+    }
+    const bool used = brows > 0;
+    sums.partial[2 * m] = weight; sums.out[2 * m] = grads.weight[m]; sums.rows[2 * m] = wrows; sums.first[2 * m] = columns;
+    columns += used ? d.Kc * 2 * AT_TAPS : 0;
+    sums.partial[2 * m + 1] = bias; sums.out[2 * m + 1] = grads.bias[m]; sums.rows[2 * m + 1] = brows; sums.first[2 * m + 1] = columns;
+    columns += used ? d.Kc : 0;
+  }
+  sums.first[RP_SUMS] = columns;
+
+  cudaError_t err = launch_logit_grad(job, place, count, st);
   if (err != cudaSuccess) return err;
   {
-    const int dc = walk_length(tiled ? tiles : blocks, d.D);
-    const unsigned pieces = (unsigned)((d.D + dc - 1) / dc);
-    const dim3 grid(pixel_grid(d).x, d.B * pieces);
-    const dim3 tgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * pieces);
+    InputGradJobs jobs{};
+    unsigned long long blocks = 0;
+    for (int i = 0; i <= MAX_ATTENTION_JOBS; ++i) {
+      jobs.blocks.first[i] = (int)blocks;
+      if (i >= count) continue;
+      const size_t tiles = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
+      const int dc = walk_length(tiles * count, job[i].d.D);
+      jobs.j[i] = InputGradJobs::Job{job[i].g, job[i].add, job[i].add_sb, job[i].gx, job[i].d.D, dc, job[i].module};
+      blocks += (unsigned long long)tiles * ((job[i].d.D + dc - 1) / dc);
+      if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+    }
     StagedWeights staged(st);
     for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
-      const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
-      err = staged.put(weight + (size_t)k0 * 2 * AT_TAPS, kc);
-      if (err != cudaSuccess) return err;
-      const float* ad = k0 == 0 ? add : nullptr;
-      const int accumulate = k0 == 0 ? 0 : 1;
-      if (tiled) {
-        CUtensorMap tm_gl;
-        err = tile_map(&tm_gl, g, g_sb, d.Kc, kc, d, true);
+      const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC, accumulate = k0 == 0 ? 0 : 1;
+      for (int m = 0; m < 2; ++m) {
+        if (modules.weight[m] == nullptr) continue;
+        err = staged.put(modules.weight[m] + (size_t)k0 * 2 * AT_TAPS, kc, m);
         if (err != cudaSuccess) return err;
-#define SFB_AT_IG_T(KC) attention_input_grad_tiled_kernel<KC><<<tgrid, AT_THREADS + 32, 0, st>>>(tm_gl, ad, add_sb, gx, accumulate, k0, d.B, d.D, dc, d.H1, d.W1, status)
+      }
+      if (tiled) {
+        TileMaps maps;
+        for (int i = 0; i < count; ++i) {
+          err = tile_map(&maps.m[i], job[i].g, g_sb(job[i]), d.Kc, kc, job[i].d, true);
+          if (err != cudaSuccess) return err;
+        }
+#define SFB_AT_IG_T(KC) attention_input_grad_tiled_kernel<KC><<<(unsigned)blocks, AT_THREADS + 32, 0, st>>>(maps, jobs, accumulate, k0, d.B, d.H1, d.W1, status)
         if (kc == 1) SFB_AT_IG_T(1); else if (kc == 2) SFB_AT_IG_T(2); else if (kc == 3) SFB_AT_IG_T(3); else SFB_AT_IG_T(4);
 #undef SFB_AT_IG_T
         continue;
       }
-      if (kc == 1) err = launch_input_grad<1>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
-      else if (kc == 2) err = launch_input_grad<2>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
-      else if (kc == 3) err = launch_input_grad<3>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
-      else err = launch_input_grad<4>(grid, g, ad, add_sb, gx, accumulate, d, dc, k0, st);
+      if (kc == 1) err = launch_input_grad<1>((unsigned)blocks, jobs, accumulate, d, k0, st);
+      else if (kc == 2) err = launch_input_grad<2>((unsigned)blocks, jobs, accumulate, d, k0, st);
+      else if (kc == 3) err = launch_input_grad<3>((unsigned)blocks, jobs, accumulate, d, k0, st);
+      else err = launch_input_grad<4>((unsigned)blocks, jobs, accumulate, d, k0, st);
       if (err != cudaSuccess) return err;
     }
   }
   const int kw = d.Kc >= 4 ? 4 : d.Kc, chunks = (d.Kc + kw - 1) / kw;
-  const int dc = walk_length(tiled ? tiles : 2 * blocks, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
-  const int pieces = (d.D + dc - 1) / dc;
-  int wrows;
+  WeightGradJobs jobs{};
+  unsigned long long blocks = 0;
+  TileMaps maps_x, maps_gl;
+  for (int i = 0; i <= MAX_ATTENTION_JOBS; ++i) {
+    jobs.blocks.first[i] = (int)blocks;
+    if (i >= count) continue;
+    jobs.j[i] = WeightGradJobs::Job{job[i].x, job[i].x_sb, job[i].g, place[i].weight, job[i].d.D, weight_walk(job[i].d, count, tiled),
+                                    place[i].weight_row0, place[i].weight_rows};
+    blocks += weight_rows(job[i].d, count, tiled);
+    if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+    if (tiled) {
+      err = tile_map(&maps_x.m[i], job[i].x, job[i].x_sb, 2, 2, job[i].d, true);
+      if (err == cudaSuccess) err = tile_map(&maps_gl.m[i], job[i].g, g_sb(job[i]), d.Kc, kw, job[i].d, false);
+      if (err != cudaSuccess) return err;
+    }
+  }
   if (tiled) {
-    CUtensorMap tm_x, tm_gl;
-    err = tile_map(&tm_x, x, x_sb, 2, 2, d, true);
-    if (err == cudaSuccess) err = tile_map(&tm_gl, g, g_sb, d.Kc, kw, d, false);
-    if (err != cudaSuccess) return err;
-    const dim3 wgrid((d.W1 + AT_TW - 1) / AT_TW, (d.H1 + AT_TH - 1) / AT_TH, d.B * chunks * pieces);
-    wrows = (int)(tiles * pieces);
-#define SFB_AT_WG_T(KW) attention_weight_grad_tiled_kernel<KW><<<wgrid, WG_WARPS * 32 + 32, 0, st>>>(tm_x, tm_gl, g, weight_partial, d.Kc, d.B, d.D, dc, chunks, d.H1, d.W1, status)
+#define SFB_AT_WG_T(KW) attention_weight_grad_tiled_kernel<KW><<<dim3((unsigned)blocks, chunks), WG_WARPS * 32 + 32, 0, st>>>(maps_x, maps_gl, jobs, d.Kc, d.B, d.H1, d.W1, status)
     if (kw == 1) SFB_AT_WG_T(1); else if (kw == 2) SFB_AT_WG_T(2); else if (kw == 3) SFB_AT_WG_T(3); else SFB_AT_WG_T(4);
 #undef SFB_AT_WG_T
   } else {
-    const dim3 wgrid(pixel_grid(d).x, d.B * pieces, 2 * chunks);
-    wrows = (int)(blocks * pieces);
-#define SFB_AT_WG(KW) attention_weight_grad_kernel<KW><<<wgrid, AT_THREADS, 0, st>>>(x, x_sb, g, weight_partial, d.Kc, d.B, d.D, dc, d.H1, d.W1)
+#define SFB_AT_WG(KW) attention_weight_grad_kernel<KW><<<dim3((unsigned)blocks, 2 * chunks), AT_THREADS, 0, st>>>(jobs, d.Kc, d.B, d.H1, d.W1)
     if (kw == 1) SFB_AT_WG(1); else if (kw == 2) SFB_AT_WG(2); else if (kw == 3) SFB_AT_WG(3); else SFB_AT_WG(4);
 #undef SFB_AT_WG
   }
-  const PartialSums weights{weight_partial, gweight, wrows, d.Kc * 2 * AT_TAPS}, biases{bias_partial, gbias, bias_rows, d.Kc};
-  attention_reduce_partials_kernel<<<weights.n + biases.n, RP_THREADS, 0, st>>>(weights, biases);
+  if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  attention_reduce_partials_kernel<<<columns, RP_THREADS, 0, st>>>(sums);
   return cudaGetLastError();
 }
 

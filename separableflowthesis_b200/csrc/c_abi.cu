@@ -318,7 +318,8 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
     w.ga_v = take((size_t)d.B * d.Kc * d.H2 * n1);
     w.gm_u = take((size_t)d.B * 2 * d.W2 * n1);
     w.gm_v = take((size_t)d.B * 2 * d.H2 * n1);
-    w.at_partial = take(attention_partial_floats(AttentionDims{d.B, d.Kc, d.H2 > d.W2 ? d.H2 : d.W2, d.H1, d.W1}));
+    const AttentionDims at[2] = {{d.B, d.Kc, d.W2, d.H1, d.W1}, {d.B, d.Kc, d.H2, d.H1, d.W1}};
+    w.at_partial = take(attention_partial_floats(at, 2));
   }
   w.bytes = off;
   size_t part = 0;
@@ -330,7 +331,7 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   return w;
 }
 
-template <class Args> int contraction_launches(const Args& a) { return a.pieces > 1 ? 2 : 1; }   // pieces are folded by a kernel of their own
+template <class Args> int contraction_launches(const Args& a) { return a.parts > 0 ? 2 : 1; }   // pieces are folded by a kernel of their own
 
 // A sweep's cut into whole tiles and pieces, as far as the workspace has scratch for the pieces.
 void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
@@ -349,6 +350,8 @@ void set_grad_split(GradArgs& a, const Workspace& w) {
   const bool cut = s.pieces > 1 && s.part_floats * sizeof(float) <= w.part_bytes;
   a.whole_tiles = cut ? s.whole_tiles : s.tiles;
   a.pieces = cut ? s.pieces : 1;
+  a.parts = a.pieces - 1;
+  a.part0 = -1;
   a.part = w.part;
 }
 
@@ -582,6 +585,55 @@ int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm
   return SFB_OK;
 }
 
+// Arguments and tensor maps of one level's gradient GEMM, image-1-major or image-2-major, but for its cut.
+// gF1 = G * F2 : rows are image-1 pixels, the K sweep streams 4 x 16 blocks of F2 and 4-row blocks of XU.
+// gF2 = G^T * F1 : rows are an 8 x 16 block of image-2 pixels, the K sweep streams 32 pixels of F1, XU and XV.
+// K-major B operands: channel-major copies of the rounded features (image 2 in column blocks of 16 with a multiple of four
+// rows, so that a 4 x 16 block of the image is 64 consecutive values).  Rows and columns of padding must
+// read as zero: they meet the G values of cells outside the image.
+size_t f2t_per_sample(const Dims& d, const Workspace& w) { return (size_t)d.C * ((d.W2 + GG_VT - 1) / GG_VT) * w.h2p * GG_VT; }
+int grad_arguments(const Dims& d, const Workspace& w, int op16, int mode, int R4, int image2_major, float* out, int out_cf, float scale1,
+                   GradArgs* a, CUtensorMap* tm_y, CUtensorMap* tm_xu, CUtensorMap* tm_xv) {
+  memset(a, 0, sizeof(*a));
+  a->d = d;
+  a->mode = mode;
+  a->R4 = R4;
+  a->n1p = w.n1p;
+  a->xu = w.gxu;
+  a->xv = w.gxv;
+  a->status = w.status;
+  a->op16 = op16;
+  a->out_cf = out_cf;
+  a->image2_major = image2_major;
+  a->out = out;
+  a->out_scale = image2_major ? 1.f : scale1;
+  a->dev_scale = op16 == OP16_FP16 ? w.scales + (image2_major ? SCALE_INV_GF2 : SCALE_INV_GF1) : nullptr;
+  const int Q = R4 / 4;
+  const uint32_t crows = (uint32_t)((d.C + KBLK - 1) / KBLK * KBLK);  // channel rows of one feature block
+  if (!image2_major) {  // (blocked pixels, C, B); box = 128 bytes of consecutive values (4 rows x 16 columns of a 16-bit type) x all channels
+    const uint64_t dims[3] = {(uint64_t)(f2t_per_sample(d, w) / d.C), (uint64_t)d.C, (uint64_t)d.B};
+    const uint32_t box[3] = {op16 ? 64u : 32u, crows, 1};
+    SFB_TRY(make_map(tm_y, w.F2t, 3, dims, box, CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0));
+    SFB_TRY(map_operands(tm_xu, w.gxu, d.B, d.H2, Q, w.n1p, TILE_M / 2, GG_UT));  // two 64-pixel boxes per block
+    *tm_xv = *tm_xu;  // unused
+    return SFB_OK;
+  }
+  // (N1, C, B) with rows padded to n1p; box = 32 pixels x all channels: a row of 32 K-values is 128 bytes of FP32 or 64 bytes of a
+  // 16-bit type, the swizzle span follows
+  const uint64_t dims[3] = {(uint64_t)d.N1(), (uint64_t)d.C, (uint64_t)d.B};
+  const uint32_t box[3] = {GG_KJ, crows, 1};
+  SFB_TRY(make_map(tm_y, w.F1t, 3, dims, box, op16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0, (uint64_t)w.n1p));
+  SFB_TRY(map_operands(tm_xu, w.gxu, d.B, d.H2, Q, w.n1p, GG_KJ, GG_ROW_UT));
+  return map_operands(tm_xv, w.gxv, d.B, d.W2, Q, w.n1p, GG_KJ, GG_ROW_VT);
+}
+
+MapCopy f1_copy(const Dims& d, const Workspace& w, const Features& f) {
+  return MapCopy{f.F1, w.F1t, 1, d.N1(), w.n1p, 0, f.scale1, f.op16 == OP16_FP16 ? w.scales + SCALE_F1 : nullptr};
+}
+MapCopy f2_copy(const Dims& d, const Workspace& w, const float* F2, int op16) {
+  return MapCopy{F2, w.F2t, d.H2, d.W2, w.h2p, 1, 1.f, op16 == OP16_FP16 ? w.scales + SCALE_F2 : nullptr};
+}
+
 // out_cf: the gradients are written channel-major, (B, C, pixels), gF1 multiplied by scale1.
 int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int mode, int R4, int accumulate, float* gF1, float* gF2,
                   cudaStream_t st, int out_cf = 0, float scale1 = 1.f) {
@@ -590,66 +642,27 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
   const int op16 = feat.op16;
   const float* const s1 = op16 == OP16_FP16 ? w.scales + SCALE_F1 : nullptr;
   const float* const s2 = op16 == OP16_FP16 ? w.scales + SCALE_F2 : nullptr;
-  CUtensorMap tm_y, tm_xu, tm_xv;
-  GradArgs a;
-  memset(&a, 0, sizeof(a));
-  a.d = d;
-  a.mode = mode;
-  a.R4 = R4;
-  a.n1p = w.n1p;
-  a.accumulate = accumulate;
-  a.xu = w.gxu;
-  a.xv = w.gxv;
-  a.status = w.status;
-  a.op16 = op16;
-  const int Q = R4 / 4;
   const int kid = mode == GRAD_MAXAVG ? KID_GRAD_MAXAVG_IMG1 : (mode == GRAD_COMPRESS ? KID_GRAD_COMPRESS_IMG1 : KID_GRAD_FUSED_IMG1);
-  // K-major B operands: channel-major copies of the rounded features (image 2 in column blocks of 16 with a multiple of four
-  // rows, so that a 4 x 16 block of the image is 64 consecutive values).  Rows and columns of padding must
-  // read as zero: they meet the G values of cells outside the image.
-  const uint32_t crows = (uint32_t)((d.C + KBLK - 1) / KBLK * KBLK);  // channel rows of one feature block
-  // image 1: a row of 32 K-values is 128 bytes of FP32 or 64 bytes of a 16-bit type: the swizzle span follows
-  const CUtensorMapSwizzle fswz = op16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-  const size_t f2t_per_sample = (size_t)d.C * ((d.W2 + GG_VT - 1) / GG_VT) * w.h2p * GG_VT;
   if (!accumulate) {  // later passes over further channel chunks reuse the copies of the first
-    SFB_CUDA(timed(KID_PREPARE, 2, st, [&] {
-      if (op16 && feat.fmaps) {  // already channel-major
-        SFB_LAUNCH(launch_channel_major_cf(feat.F1, reinterpret_cast<uint16_t*>(w.F1t), d.B, 1, d.N1(), w.n1p, d.C, 0, feat.scale1, op16, s1, st));
-        return launch_channel_major_cf(feat.F2, reinterpret_cast<uint16_t*>(w.F2t), d.B, d.H2, d.W2, w.h2p, d.C, 1, 1.f, op16, s2, st);
+    SFB_CUDA(timed(KID_PREPARE, feat.fmaps ? 1 : 2, st, [&] {
+      if (feat.fmaps) {  // already channel-major
+        const MapCopy copies[2] = {f1_copy(d, w, feat), f2_copy(d, w, feat.F2, op16)};
+        return launch_channel_major_cf(copies, 2, d.B, d.C, op16, st);
       }
-      SFB_LAUNCH(cudaMemsetAsync(w.F2t, 0, (size_t)d.B * f2t_per_sample * (op16 ? 2 : sizeof(float)), st));
+      SFB_LAUNCH(cudaMemsetAsync(w.F2t, 0, (size_t)d.B * f2t_per_sample(d, w) * (op16 ? 2 : sizeof(float)), st));
       SFB_LAUNCH(launch_channel_major(op16 ? feat.F1 : w.F1r, w.F1t, d.B, 1, d.N1(), w.n1p, d.C, 0, op16, s1, st));
       return launch_channel_major(op16 ? feat.F2 : w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
     }));
   }
-  // gF1 = G * F2 : rows are image-1 pixels, the K sweep streams 4 x 16 blocks of F2 and 4-row blocks of XU.
-  {  // (blocked pixels, C, B); box = 128 bytes of consecutive values (4 rows x 16 columns of a 16-bit type) x all channels
-    const uint64_t dims[3] = {(uint64_t)(f2t_per_sample / d.C), (uint64_t)d.C, (uint64_t)d.B};
-    const uint32_t box[3] = {op16 ? 64u : 32u, crows, 1};
-    SFB_TRY(make_map(&tm_y, w.F2t, 3, dims, box, CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0));
+  for (const int image2_major : {0, 1}) {
+    GradArgs a;
+    GradMaps maps;
+    SFB_TRY(grad_arguments(d, w, op16, mode, R4, image2_major, image2_major ? gF2 : gF1, out_cf, scale1, &a, maps.y, maps.xu, maps.xv));
+    a.accumulate = accumulate;
+    set_grad_split(a, w);
+    a = with_wait_settings(a);
+    SFB_CUDA(timed(kid + image2_major, contraction_launches(a), st, [&] { return launch_grad_gemm(&a, 1, maps, st); }));
   }
-  SFB_TRY(map_operands(&tm_xu, w.gxu, d.B, d.H2, Q, w.n1p, TILE_M / 2, GG_UT));  // two 64-pixel boxes per block
-  a.out_cf = out_cf;
-  a.image2_major = 0;
-  a.out = gF1;
-  a.out_scale = scale1;
-  a.dev_scale = op16 == OP16_FP16 ? w.scales + SCALE_INV_GF1 : nullptr;
-  set_grad_split(a, w);
-  SFB_CUDA(timed(kid, contraction_launches(a), st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xu /* unused */, st); }));
-  // gF2 = G^T * F1 : rows are an 8 x 16 block of image-2 pixels, the K sweep streams 32 pixels of F1, XU and XV.
-  {  // (N1, C, B) with rows padded to n1p; box = 32 pixels x all channels
-    const uint64_t dims[3] = {(uint64_t)d.N1(), (uint64_t)d.C, (uint64_t)d.B};
-    const uint32_t box[3] = {GG_KJ, crows, 1};
-    SFB_TRY(make_map(&tm_y, w.F1t, 3, dims, box, fswz, op16 != 0, (uint64_t)w.n1p));
-  }
-  SFB_TRY(map_operands(&tm_xu, w.gxu, d.B, d.H2, Q, w.n1p, GG_KJ, GG_ROW_UT));
-  SFB_TRY(map_operands(&tm_xv, w.gxv, d.B, d.W2, Q, w.n1p, GG_KJ, GG_ROW_VT));
-  a.image2_major = 1;
-  a.out = gF2;
-  a.out_scale = 1.f;
-  a.dev_scale = op16 == OP16_FP16 ? w.scales + SCALE_INV_GF2 : nullptr;
-  set_grad_split(a, w);
-  SFB_CUDA(timed(kid + 1, contraction_launches(a), st, [&] { return launch_grad_gemm(with_wait_settings(a), tm_y, tm_xu, tm_xv, st); }));
   return SFB_OK;
 }
 
@@ -1181,10 +1194,8 @@ int sfb_attention_forward(const float* X, int64_t x_batch_stride, const float* w
 size_t sfb_attention_backward_workspace_bytes(int32_t B, int32_t Kc, int32_t D, int32_t H1, int32_t W1) {
   AttentionDims ad;
   if (check_attention_dims(B, Kc, D, H1, W1, &ad) != SFB_OK) return 0;
-  return align_up(attention_partial_floats(ad) * sizeof(float), 256);
+  return align_up(attention_partial_floats(&ad, 1) * sizeof(float), 256);
 }
-
-static int attention_backward_launches(int Kc) { return (Kc + 3) / 4 + 3; }
 
 int sfb_attention_backward(const float* X, int64_t x_batch_stride, const float* weight, const float* A, float* gA,
                            const float* add, int64_t add_batch_stride, float* gX, float* gweight, float* gbias,
@@ -1200,10 +1211,11 @@ int sfb_attention_backward(const float* X, int64_t x_batch_stride, const float* 
   if (workspace_bytes < need)
     return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", workspace_bytes, need);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SFB_CUDA(timed(KID_ATTENTION_BWD, attention_backward_launches(Kc), st, [&] {
-    return launch_attention_backward(ad, X, x_batch_stride, weight, A, gA, add, add_batch_stride, gX, gweight, gbias,
-                                     static_cast<float*>(workspace), st);
-  }));
+  const AttentionGradJob job{ad, 0, X, x_batch_stride, A, gA, add, add_batch_stride, gX};
+  const AttentionModules modules{{weight, nullptr}, {nullptr, nullptr}};
+  const AttentionGradients grads{{gweight, nullptr}, {gbias, nullptr}};
+  SFB_CUDA(timed(KID_ATTENTION_BWD, attention_backward_launches(&job, 1), st,
+                 [&] { return launch_attention_backward(&job, 1, modules, grads, static_cast<float*>(workspace), st); }));
   return SFB_OK;
 }
 
@@ -1330,13 +1342,14 @@ static int level_backward(Placement pl, const float* F1, const float* F2, int fm
                               cf_view(w.ga_u, K, d.W2, N1), N1, st, op16, sweep_out_scale(w, op16)));
   // through softmax and Conv3d: parameter gradients, and the total gradients of the max/avg channels
   const long long sb_u = (long long)Kt * d.W2 * N1, sb_v = (long long)Kt * d.H2 * N1;
-  SFB_CUDA(timed(KID_ATTENTION_BWD, 2 * attention_backward_launches(K), st, [&] {
-    const size_t ou = (size_t)c0 * d.W2 * N1, ov = (size_t)c0 * d.H2 * N1;  // first channel of this level
-    SFB_LAUNCH(launch_attention_backward(AttentionDims{d.B, K, d.W2, d.H1, d.W1}, SEP_u + ou, sb_u, weight_u, A_u, w.ga_u,
-                                         gSEP_u + ou, sb_u, w.gm_u, gweight_u, gbias_u, w.at_partial, st, w.status));
-    return launch_attention_backward(AttentionDims{d.B, K, d.H2, d.H1, d.W1}, SEP_v + ov, sb_v, weight_v, A_v, w.ga_v,
-                                     gSEP_v + ov, sb_v, w.gm_v, gweight_v, gbias_v, w.at_partial, st, w.status);
-  }));
+  const size_t ou = (size_t)c0 * d.W2 * N1, ov = (size_t)c0 * d.H2 * N1;  // first channel of this level
+  const AttentionGradJob jobs[2] = {
+      {AttentionDims{d.B, K, d.W2, d.H1, d.W1}, 0, SEP_u + ou, sb_u, A_u, w.ga_u, gSEP_u + ou, sb_u, w.gm_u},
+      {AttentionDims{d.B, K, d.H2, d.H1, d.W1}, 1, SEP_v + ov, sb_v, A_v, w.ga_v, gSEP_v + ov, sb_v, w.gm_v}};
+  const AttentionModules modules{{weight_u, weight_v}, {nullptr, nullptr}};
+  const AttentionGradients grads{{gweight_u, gweight_v}, {gbias_u, gbias_v}};
+  SFB_CUDA(timed(KID_ATTENTION_BWD, attention_backward_launches(jobs, 2), st,
+                 [&] { return launch_attention_backward(jobs, 2, modules, grads, w.at_partial, st, w.status); }));
   return run_fused_feature_grads_cf(d, w, feat, AM_u, AM_v, w.gm_v, w.gm_u, A_u, A_v, gSEP_v, gSEP_u, Kt, c0 + 2, gF1, gF2, st,
                                     fmaps, fmaps ? scale1 : 1.f, /*unit_weights=*/true);
 }
@@ -1391,7 +1404,8 @@ int sfb_upsample_displacement_backward(const float* gout, int64_t gout_batch_str
   SFB_TRY(check_resample(gout, gin, B, K, Dl, D0, H1, W1));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   SFB_CUDA(timed(KID_RESAMPLE, 1, st, [&] {
-    return launch_upsample_displacement_adjoint(gout, gout_batch_stride, gin, B, K, Dl, D0, H1 * W1, st);
+    const ResampleAdjointJob job{gout, gout_batch_stride, gin, Dl, D0};
+    return launch_upsample_displacement_adjoint(&job, 1, B, K, H1 * W1, st);
   }));
   return SFB_OK;
 }
@@ -1504,6 +1518,68 @@ PyramidWorkspace carve_pyramid_forward(const Pyramid& py, void* base) {
   return p;
 }
 
+// The backward's: attention gradients, gradients of the max/avg channels, GEMM operands and image 2's copies per level, image 1's shared;
+// the gradients of the level's own volumes (gs_u, gs_v) where it is not in place.
+struct PyramidBackward {
+  Workspace w[MAX_FUSED_LEVELS];
+  float *gs_u[MAX_FUSED_LEVELS], *gs_v[MAX_FUSED_LEVELS];
+  size_t bytes;
+};
+PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
+  PyramidBackward p;
+  size_t off = 0;
+  auto take = [&](size_t floats) {
+    float* r = reinterpret_cast<float*>(static_cast<char*>(base) + off);
+    off += align_up(floats * sizeof(float), 256);
+    return r;
+  };
+  const Dims& d0 = py.d[0];
+  const size_t bn = (size_t)d0.B * d0.N1();
+  const int n1p = padded_pixels(d0), Kt = 2 + d0.Kc, Rg = 4 + grad_slots(d0.Kc);
+  int* const status = reinterpret_cast<int*>(take(WS_HEADER_BYTES / sizeof(float)));
+  float* const F1 = take(bn * d0.C);
+  float* const F1t = take((size_t)d0.B * d0.C * n1p);
+  AttentionDims at[MAX_ATTENTION_JOBS];
+  for (int l = 0; l < py.levels; ++l) {
+    const Dims& d = py.d[l];
+    Workspace& w = p.w[l];
+    w = Workspace{};
+    w.status = status;
+    w.scales = reinterpret_cast<float*>(reinterpret_cast<char*>(status) + WS_SCALES_OFFSET) + l * SCALE_LEVEL;
+    w.n1p = n1p;
+    w.F1r = F1;
+    w.F2r = take((size_t)d.B * d.N2() * d.C);
+    w.F1h = reinterpret_cast<uint16_t*>(w.F1r);
+    w.F2h = reinterpret_cast<uint16_t*>(w.F2r);
+    w.F1t = F1t;
+    w.h2p = (d.H2 + GG_UT - 1) / GG_UT * GG_UT;
+    w.F2t = take((size_t)d.B * f2t_per_sample(d, w));
+    w.gxu = take((size_t)d.B * d.H2 * Rg * n1p);
+    w.gxv = take((size_t)d.B * d.W2 * Rg * n1p);
+    w.ga_u = take(bn * d.Kc * d.W2);
+    w.ga_v = take(bn * d.Kc * d.H2);
+    w.gm_u = take(bn * 2 * d.W2);
+    w.gm_v = take(bn * 2 * d.H2);
+    p.gs_u[l] = py.in_place[l] ? nullptr : take(bn * Kt * d.W2);
+    p.gs_v[l] = py.in_place[l] ? nullptr : take(bn * Kt * d.H2);
+    at[2 * l] = AttentionDims{d.B, d.Kc, d.W2, d.H1, d.W1};
+    at[2 * l + 1] = AttentionDims{d.B, d.Kc, d.H2, d.H1, d.W1};
+  }
+  p.w[0].at_partial = take(attention_partial_floats(at, 2 * py.levels));
+  TileSplit split[MAX_FUSED_LEVELS];
+  size_t part = pyramid_part_floats(py, chunk_channels(d0.Kc), true, split);
+  for (const int image2_major : {0, 1}) {
+    grad_split_levels(py.d, py.levels, image2_major, split);
+    size_t floats = 0;
+    for (int l = 0; l < py.levels; ++l) floats += split[l].part_floats;
+    part = std::max(part, floats);
+  }
+  float* const parts = take(part);
+  for (int l = 0; l < py.levels; ++l) p.w[l].part = parts;
+  p.bytes = off;
+  return p;
+}
+
 // The sweeps of all levels: `fill(l, a)` sets a level's views, the rest is common.
 template <class Fill>
 int run_pyramid_sweeps(const Pyramid& py, const Workspace* w, int op16, int mode, cudaStream_t st, Fill&& fill) {
@@ -1581,10 +1657,11 @@ size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t*
   return carve_saved(py, nullptr, with_argmax != 0).bytes;
 }
 
-size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels) {
+size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
+                                              int32_t backward) {
   Pyramid py;
   if (check_pyramid(shape, H2, W2, levels, &py) != SFB_OK) return 0;
-  return carve_pyramid_forward(py, nullptr).bytes;
+  return backward != 0 ? carve_pyramid_backward(py, nullptr).bytes : carve_pyramid_forward(py, nullptr).bytes;
 }
 
 int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
@@ -1645,6 +1722,136 @@ int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2
     up[n++] = ResampleJob{vol[l].v, SEP_v + c0 * d0.H2 * N1, (long long)Kt * levels * d0.H2 * N1, py.d[l].H2, d0.H2};
   }
   if (n > 0) SFB_CUDA(timed(KID_RESAMPLE, 1, st, [&] { return launch_upsample_displacement(up, n, d0.B, Kt, N1, st); }));
+  return SFB_OK;
+}
+
+int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
+                                    int32_t levels, float scale1, const float* weight_u, const float* weight_v,
+                                    const float* SEP_u, const float* SEP_v, const void* saved, size_t saved_bytes,
+                                    const float* gSEP_u, const float* gSEP_v, float* gfmap1, float* const* gfmap2,
+                                    float* gweight_u, float* gbias_u, float* gweight_v, float* gbias_v,
+                                    const sfb_shape* shape, void* workspace, size_t workspace_bytes, void* stream) {
+  Pyramid py;
+  SFB_TRY(check_pyramid(shape, H2, W2, levels, &py));
+  SFB_CHECK_PTR(fmap1); SFB_CHECK_PTR(fmap2); SFB_CHECK_PTR(SEP_u); SFB_CHECK_PTR(SEP_v); SFB_CHECK_PTR(saved);
+  SFB_CHECK_PTR(gSEP_u); SFB_CHECK_PTR(gSEP_v); SFB_CHECK_PTR(gfmap1); SFB_CHECK_PTR(gfmap2);
+  for (int l = 0; l < levels; ++l) { SFB_CHECK_PTR(fmap2[l]); SFB_CHECK_PTR(gfmap2[l]); }
+  if (weight_u == nullptr || weight_v == nullptr || gweight_u == nullptr || gbias_u == nullptr || gweight_v == nullptr ||
+      gbias_v == nullptr)
+    return fail(SFB_ERR_INVALID_ARGUMENT, "attention weights and their gradient buffers must not be NULL");
+  const PyramidSaved sv = carve_saved(py, const_cast<void*>(saved), true);
+  if (saved_bytes < sv.bytes) return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "saved has %zu bytes, %zu needed", saved_bytes, sv.bytes);
+  if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+    return fail(SFB_ERR_INVALID_ARGUMENT, "workspace is NULL or not 256-byte aligned");
+  const PyramidBackward pb = carve_pyramid_backward(py, workspace);
+  if (workspace_bytes < pb.bytes)
+    return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", workspace_bytes, pb.bytes);
+  const Dims& d0 = py.d[0];
+  const Workspace* const w = pb.w;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int op16;
+  SFB_TRY(operand_mode(d0, &op16));
+  SFB_TRY(prepare_pyramid(py, w, fmap1, fmap2, scale1, false, op16, st));
+  const int N1 = d0.N1(), K = d0.Kc, Kt = 2 + K;
+  const size_t bn = (size_t)d0.B * N1;
+  float *const SU = const_cast<float*>(SEP_u), *const SV = const_cast<float*>(SEP_v);
+  float *const GU = const_cast<float*>(gSEP_u), *const GV = const_cast<float*>(gSEP_v);
+  LevelVolumes vol[MAX_FUSED_LEVELS], grad[MAX_FUSED_LEVELS];
+  ResampleAdjointJob down[MAX_RESAMPLE_JOBS];
+  int n = 0;
+  for (int l = 0; l < levels; ++l) {
+    vol[l] = level_volumes(py, l, SU, SV, sv.sep_u[l], sv.sep_v[l]);
+    grad[l] = level_volumes(py, l, GU, GV, pb.gs_u[l], pb.gs_v[l]);
+    if (py.in_place[l]) continue;
+    const long long c0 = (long long)l * Kt;
+    down[n++] = ResampleAdjointJob{gSEP_u + c0 * d0.W2 * N1, (long long)Kt * levels * d0.W2 * N1, pb.gs_u[l], py.d[l].W2, d0.W2};
+    down[n++] = ResampleAdjointJob{gSEP_v + c0 * d0.H2 * N1, (long long)Kt * levels * d0.H2 * N1, pb.gs_v[l], py.d[l].H2, d0.H2};
+  }
+  if (n > 0) SFB_CUDA(timed(KID_RESAMPLE, 1, st, [&] { return launch_upsample_displacement_adjoint(down, n, d0.B, Kt, N1, st); }));
+  // attention gradients: the compression sweep with the upstream gradients in the role of the weights (level_backward)
+  SFB_TRY(run_pyramid_sweeps(py, w, op16, SWEEP_COMPRESS, st, [&](int l, SweepArgs& a) {
+    a.xu = volume_view(grad[l].v, grad[l].sb_v, 2, py.d[l].H2, N1);
+    a.xv = volume_view(grad[l].u, grad[l].sb_u, 2, py.d[l].W2, N1);
+    a.ou = cf_view(w[l].ga_v, K, py.d[l].H2, N1);
+    a.ov = cf_view(w[l].ga_u, K, py.d[l].W2, N1);
+  }));
+  AttentionGradJob jobs[MAX_ATTENTION_JOBS];
+  for (int l = 0; l < levels; ++l) {
+    const Dims& d = py.d[l];
+    jobs[2 * l] = AttentionGradJob{AttentionDims{d.B, K, d.W2, d.H1, d.W1}, 0, vol[l].u, vol[l].sb_u, sv.a_u[l], w[l].ga_u,
+                                   grad[l].u, grad[l].sb_u, w[l].gm_u};
+    jobs[2 * l + 1] = AttentionGradJob{AttentionDims{d.B, K, d.H2, d.H1, d.W1}, 1, vol[l].v, vol[l].sb_v, sv.a_v[l], w[l].ga_v,
+                                       grad[l].v, grad[l].sb_v, w[l].gm_v};
+  }
+  const AttentionModules modules{{weight_u, weight_v}, {nullptr, nullptr}};
+  const AttentionGradients grads{{gweight_u, gweight_v}, {gbias_u, gbias_v}};
+  SFB_CUDA(timed(KID_ATTENTION_BWD, attention_backward_launches(jobs, 2 * levels), st, [&] {
+    return launch_attention_backward(jobs, 2 * levels, modules, grads, w[0].at_partial, st, w[0].status);
+  }));
+  if (op16 == OP16_FP16) {   // scales of the gradient operands, from the level's channels alone; the weights are softmax outputs
+    AbsmaxSource src[ABSMAX_MAX];
+    int m = 0;
+    for (int l = 0; l < levels; ++l) {
+      const Dims& d = py.d[l];
+      const int slot = l * SCALE_LEVEL + SCALE_AMAX_G;
+      auto channels = [&](const float* vols, long long sb, int D) {
+        const size_t len = (size_t)K * D * N1;
+        // very large batches: the samples with the channels between them, as one array
+        return d.B <= 1024 ? AbsmaxSource{vols + (size_t)2 * D * N1, len, sb, d.B, 1.f, slot}
+                           : absmax_array(vols + (size_t)2 * D * N1, (size_t)sb * (d.B - 1) + len, 1.f, slot);
+      };
+      src[m++] = absmax_array(w[l].gm_v, bn * 2 * d.H2, 1.f, slot);
+      src[m++] = absmax_array(w[l].gm_u, bn * 2 * d.W2, 1.f, slot);
+      src[m++] = channels(grad[l].v, grad[l].sb_v, d.H2);
+      src[m++] = channels(grad[l].u, grad[l].sb_u, d.W2);
+    }
+    SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_absmax(src, m, w[0].scales, levels, true, st); }));
+  }
+  // G = max/avg terms + compression terms, as in run_fused_feature_grads_cf
+  const int Qc = grad_slots(K) / 4, Q = 1 + Qc;
+  PackGroups groups{};
+  MapCopy copies[MAX_MAP_COPIES];
+  const Features feat{fmap1, nullptr, true, scale1, op16};
+  copies[0] = f1_copy(d0, w[0], feat);
+  for (int l = 0; l < levels; ++l) {
+    const Dims& d = py.d[l];
+    const float* const gs = grad_slot_scales(w[l], op16);
+    SlotSources su, sv2;
+    maxavg_slot_sources(d, sv.am_u[l], sv.am_v[l], w[l].gm_v, w[l].gm_u, &su, &sv2, gs);
+    groups.add(su, w[l].gxu, d.H2, 4, Q, 0);
+    groups.add(sv2, w[l].gxv, d.W2, 4, Q, 0);
+    // (a level that is not in place has its channels in tensors of 2 + Kc)
+    const int gK = py.in_place[l] ? Kt * levels : Kt, g0 = py.in_place[l] ? l * Kt + 2 : 2;
+    compress_slot_sources(K, 0, K, sv.a_u[l], sv.a_v[l], py.in_place[l] ? gSEP_v : pb.gs_v[l], py.in_place[l] ? gSEP_u : pb.gs_u[l], &su, &sv2,
+                          gs, gK, g0);
+    groups.add(su, w[l].gxu, d.H2, 4 * Qc, Q, 1);
+    groups.add(sv2, w[l].gxv, d.W2, 4 * Qc, Q, 1);
+    copies[1 + l] = f2_copy(d, w[l], fmap2[l], op16);
+  }
+  SFB_CUDA(timed(KID_PACK, pack_launches(groups.count, d0.B), st, [&] { return launch_pack_interleaved_cf(groups, d0.B, N1, w[0].n1p, st); }));
+  SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_channel_major_cf(copies, 1 + levels, d0.B, d0.C, op16, st); }));
+  for (const int image2_major : {0, 1}) {
+    GradArgs a[MAX_FUSED_LEVELS];
+    GradMaps maps;
+    TileSplit split[MAX_FUSED_LEVELS];
+    grad_split_levels(py.d, levels, image2_major, split);
+    float* part = w[0].part;
+    int part0 = -1, launches = 1;
+    for (int l = 0; l < levels; ++l) {
+      SFB_TRY(grad_arguments(py.d[l], w[l], op16, GRAD_FUSED, 4 * Q, image2_major, image2_major ? gfmap2[l] : gfmap1, 1, scale1, &a[l],
+                             &maps.y[l], &maps.xu[l], &maps.xv[l]));
+      a[l].whole_tiles = split[l].whole_tiles;
+      a[l].pieces = split[l].pieces;
+      a[l].parts = split[l].parts;
+      a[l].part0 = part0;
+      a[l].part = part;
+      if (image2_major) part += split[l].part_floats;
+      else part0 += split[l].pieces;
+      if (a[l].parts > 0) launches = 2;
+      a[l] = with_wait_settings(a[l]);
+    }
+    SFB_CUDA(timed(KID_GRAD_FUSED_IMG1 + image2_major, launches, st, [&] { return launch_grad_gemm(a, levels, maps, st); }));
+  }
   return SFB_OK;
 }
 

@@ -34,6 +34,9 @@
 // a range of the K sweep.  Piece 0 drains to the output, the others to scratch, and grad_fold_kernel adds them to the output
 // in piece order: deterministic.
 //
+// The levels of a pyramid share a launch: the tiles of a level follow those of the one before, with maps and arguments of their own.
+// gF1 is the sum over the levels, whose tiles beyond the first level's go to scratch like pieces.
+//
 // Warp roles: warp 0 feature (B operand) producer, warp 1 TMEM allocation + MMA issue, warps 2..9 generate G
 // and, at the end, drain the accumulator (two warps per TMEM lane quarter, alternating 16-column chunks),
 // warp 10 producer of the XU / XV blocks.
@@ -437,11 +440,12 @@ __device__ float* grad_row(const GradArgs& a, const GradSched& sc, int m, size_t
   cstride = (size_t)a.d.N2();
   return a.out + (size_t)sc.b * C * a.d.N2() + (size_t)u * a.d.W2 + v;
 }
-// Scratch of pieces 1.. of the tail tiles: [tail][piece - 1][channel][128 rows] or [tail][piece - 1][128 rows][channel], as the
+// Scratch of the parts of a tile that do not go straight to the output (a cut tile's pieces 1.., the other levels' pieces):
+// [tail][part][channel][128 rows] or [tail][part][128 rows][channel], as the
 // output has it, so that the fold reads both in runs (with channel-major pieces under a pixel-major output, 16-byte accesses 1 KB
 // apart, the form that folded in the tile's last CTA took 58 instead of 47 us for 1 x 55 x 128 against 27 x 64).
-__device__ __forceinline__ float* grad_part(const GradArgs& a, int tail, int piece) {
-  return a.part + ((size_t)tail * (a.pieces - 1) + piece - 1) * a.d.C * TILE_M;
+__device__ __forceinline__ float* grad_part(const GradArgs& a, int tail, int part) {
+  return a.part + ((size_t)tail * a.parts + part) * a.d.C * TILE_M;
 }
 
 template <int Q, int I2MAJOR>
@@ -456,8 +460,8 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
   float* dst = grad_row<I2MAJOR>(a, sc, m, cstride);
   const bool channel_major = a.out_cf != 0;
   bool accumulate = a.accumulate != 0;
-  if (sc.piece > 0) {
-    if (dst != nullptr) dst = grad_part(a, sc.tail, sc.piece) + (channel_major ? m : m * C);
+  if (a.part0 + sc.piece >= 0) {
+    if (dst != nullptr) dst = grad_part(a, sc.tail, a.part0 + sc.piece) + (channel_major ? m : m * C);
     cstride = TILE_M;
     accumulate = false;
   }
@@ -516,14 +520,31 @@ __device__ __forceinline__ int grad_tile(const GradArgs& a, int tile, GradSched&
   return (a.d.N1() + GG_KJ - 1) / GG_KJ;
 }
 
-// Pieces 1.. of the cut tiles added to the output, in piece order, four values to a thread.  A kernel of its own: added up by
+// What a launch works on: one pair of images, or the levels of a pyramid over the same image 1.
+template <int LEVELS>
+struct GradLaunch {
+  CUtensorMap y[LEVELS], xu[LEVELS], xv[LEVELS];
+  GradArgs a[LEVELS];
+  int first_block[LEVELS + 1], first_tail[LEVELS + 1];   // of the GEMM and of the fold; levels that do not exist have none
+};
+template <int LEVELS>
+__device__ __forceinline__ int grad_level(const int (&first)[LEVELS + 1], int block) {
+  int level = 0;
+#pragma unroll
+  for (int l = 1; l < LEVELS; ++l) level = block >= first[l] ? l : level;
+  return level;
+}
+
+// The parts of a tile in scratch added to the output, in their order, four values to a thread.  A kernel of its own: added up by
 // the CTA that finished a tile last, the 128 KB of every piece came through that one SM.
 constexpr int GG_FOLD_THREADS = 256;
-template <int I2MAJOR>
-__global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const GradArgs a) {
+template <int I2MAJOR, int LEVELS>
+__global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const __grid_constant__ GradLaunch<LEVELS> launch) {
+  const int level = grad_level<LEVELS>(launch.first_tail, blockIdx.y);
+  const GradArgs& a = launch.a[level];
   if (*reinterpret_cast<volatile int*>(a.status) != 0) return;
-  const int C = a.d.C, tail = blockIdx.y;   // C is a multiple of 4
-  const int i = blockIdx.x * GG_FOLD_THREADS + threadIdx.x;   // four neighbours of the pieces' layout (grad_part)
+  const int C = a.d.C, tail = LEVELS == 1 ? blockIdx.y : blockIdx.y - launch.first_tail[level];   // C is a multiple of 4
+  const int i = blockIdx.x * GG_FOLD_THREADS + threadIdx.x;   // four neighbours of the parts' layout (grad_part)
   if (i >= C * (TILE_M / 4)) return;
   GradSched sc;
   grad_tile<I2MAJOR>(a, a.whole_tiles + tail, sc);
@@ -542,19 +563,21 @@ __global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const GradAr
     if (dst == nullptr) return;
     dst += (i - m * (C / 4)) * 4;
   }
-  const float* part = grad_part(a, tail, 1) + (size_t)i * 4;
+  const float* part = grad_part(a, tail, 0) + (size_t)i * 4;
   const size_t step = (size_t)C * TILE_M;
   float4 sum = load4_cg(dst, cnt);
 #pragma unroll 4
-  for (int piece = 1; piece < a.pieces; ++piece, part += step) add4(sum, *reinterpret_cast<const float4*>(part));
+  for (int k = 0; k < a.parts; ++k, part += step) add4(sum, *reinterpret_cast<const float4*>(part));
   store4(dst, sum, cnt);
 }
 
-template <int MODE, int Q, int I2MAJOR, int BF16>
+template <int MODE, int Q, int I2MAJOR, int BF16, int LEVELS>
 __global__ void __launch_bounds__(GG_THREADS, 1)
-grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_xu,
-                 const __grid_constant__ CUtensorMap tm_xv, const GradArgs a) {
-  if (!cta_has_work(a.status)) return;
+grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status) {
+  if (!cta_has_work(status)) return;
+  const int level = grad_level<LEVELS>(launch.first_block, blockIdx.x);
+  const GradArgs& a = launch.a[level];
+  const CUtensorMap *const tm_y = &launch.y[level], *const tm_xu = &launch.xu[level], *const tm_xv = &launch.xv[level];
   using Smem = GradSmem<Q, I2MAJOR>;
   using Cfg = GradCfg<Q, I2MAJOR>;
 
@@ -565,7 +588,7 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
 
   GradSched sc;
   sc.nkb = (a.d.C + KBLK - 1) / KBLK;
-  int tile = blockIdx.x;
+  int tile = LEVELS == 1 ? blockIdx.x : blockIdx.x - launch.first_block[level];
   sc.tail = -1;
   sc.piece = 0;
   if (tile >= a.whole_tiles) {  // pieces of the tail tiles follow the whole tiles
@@ -591,9 +614,9 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
     mbar_init(&sm.acc_full, 1);
     wait_ctl_init(&sm.ctl, a.wait_limit_ns);
     fence_barrier_init();
-    prefetch_tensormap(&tm_y);
-    prefetch_tensormap(&tm_xu);
-    if (I2MAJOR) prefetch_tensormap(&tm_xv);
+    prefetch_tensormap(tm_y);
+    prefetch_tensormap(tm_xu);
+    if (I2MAJOR) prefetch_tensormap(tm_xv);
   }
   if (warp == 1) {
     tmem_alloc(&sm.tmem_base, gg_tmem_cols<I2MAJOR>());
@@ -604,13 +627,13 @@ grad_gemm_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_constant
   tc_fence_after();
 
   if (warp == 0) {
-    if (lane == 0) feature_producer<Q, I2MAJOR, BF16>(sm, a, sc, &tm_y);
+    if (lane == 0) feature_producer<Q, I2MAJOR, BF16>(sm, a, sc, tm_y);
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) grad_mma<Q, I2MAJOR, BF16>(sm, a, sc);
     __syncwarp();
   } else if (warp == 2 + GG_GEN_WARPS) {
-    if (lane == 0) operand_producer<Q, I2MAJOR>(sm, a, sc, &tm_xu, &tm_xv);
+    if (lane == 0) operand_producer<Q, I2MAJOR>(sm, a, sc, tm_xu, tm_xv);
     __syncwarp();
   } else {
     const int gw = warp - 2;
@@ -664,10 +687,51 @@ TileSplit grad_split(const Dims& d, int image2_major) {
   return r;
 }
 
-template <int MODE, int Q, int I2MAJOR, int BF16>
-static cudaError_t launch_one(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
-                              const CUtensorMap& tm_xv, cudaStream_t stream) {
-  auto kern = grad_gemm_kernel<MODE, Q, I2MAJOR, BF16>;
+// How the tiles of a pyramid's levels are cut when they share a launch, in the same units: all tiles of a level alike, the first two
+// levels of the image-1-major form into pieces of their own, all levels of the image-2-major form, whose K sweeps are equally
+// long, into the same number.  The cut with the smallest makespan; nothing is cut where the tiles make more than a few waves.
+void grad_split_levels(const Dims* d, int levels, int image2_major, TileSplit* out) {
+  int tiles[MAX_FUSED_LEVELS], blocks[MAX_FUSED_LEVELS], all = 0;
+  for (int l = 0; l < levels; ++l) {
+    tiles[l] = grad_tiles(d[l], image2_major);
+    blocks[l] = image2_major ? (d[l].N1() + GG_KJ - 1) / GG_KJ : ((d[l].H2 + GG_UT - 1) / GG_UT) * ((d[l].W2 + GG_VT - 1) / GG_VT);
+    all += tiles[l];
+    out[l] = TileSplit{tiles[l], tiles[l], 1, 0, 0};
+  }
+  const int unit = image2_major ? 1 : GG_KJ1 / GG_KJ;   // of a block
+  int cut[MAX_FUSED_LEVELS] = {1, 1, 1, 1};
+  static_assert(MAX_FUSED_LEVELS == 4, "cut");
+  if (all <= 4 * SM_COUNT) {
+    double best = 0;
+    for (int n0 = 1; n0 <= std::min(blocks[0], MAX_PIECES); ++n0) {
+      for (int n1 = 1; n1 <= (image2_major || levels < 2 ? 1 : std::min(n0, blocks[1])); ++n1) {
+        BlockQueue queue;
+        for (int l = 0; l < levels; ++l) {
+          const int n = l == 0 || image2_major ? n0 : (l == 1 ? n1 : 1);
+          queue.add(tiles[l] * n, (double)blocks[l] / n * unit + 8);
+        }
+        const double cost = queue.makespan() + (image2_major && n0 > 1 ? 6.0 : 0.0);
+        if (best == 0 || cost < 0.95 * best) {
+          best = cost;
+          for (int l = 0; l < levels; ++l) cut[l] = l == 0 || image2_major ? n0 : (l == 1 ? n1 : 1);
+        }
+      }
+    }
+  }
+  int parts = -1;   // the image-1-major form: of all levels, less the one that goes to the output
+  for (int l = 0; l < levels; ++l) parts += cut[l];
+  for (int l = 0; l < levels; ++l) {
+    if (image2_major && cut[l] == 1) continue;
+    out[l].whole_tiles = 0;
+    out[l].pieces = cut[l];
+    out[l].parts = image2_major ? cut[l] - 1 : parts;
+    out[l].part_floats = image2_major || l == 0 ? (size_t)tiles[l] * out[l].parts * d[l].C * TILE_M : 0;   // image 1: one array for all
+  }
+}
+
+template <int MODE, int Q, int I2MAJOR, int BF16, int LEVELS>
+static cudaError_t launch_one(GradLaunch<LEVELS>& launch, int levels, cudaStream_t stream) {
+  auto kern = grad_gemm_kernel<MODE, Q, I2MAJOR, BF16, LEVELS>;
   constexpr size_t smem_bytes = sizeof(GradSmem<Q, I2MAJOR>) + 1024;
   static_assert(smem_bytes <= 232448, "shared memory of one CTA");
   static DeviceOnce configured;  // the attribute is per device and stays set
@@ -675,37 +739,67 @@ static cudaError_t launch_one(const GradArgs& a, const CUtensorMap& tm_y, const 
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
   });
   if (err != cudaSuccess) return err;
-  const int tails = grad_tiles(a.d, I2MAJOR) - a.whole_tiles;
-  kern<<<dim3(a.whole_tiles + tails * a.pieces), GG_THREADS, smem_bytes, stream>>>(tm_y, tm_xu, tm_xv, a);
-  if (a.pieces > 1) {
+  int blocks = 0, tails = 0;
+  for (int l = 0; l < LEVELS; ++l) {
+    launch.first_block[l] = blocks;
+    launch.first_tail[l] = tails;
+    if (l >= levels) continue;
+    const GradArgs& a = launch.a[l];
+    const int cut = grad_tiles(a.d, I2MAJOR) - a.whole_tiles;
+    blocks += a.whole_tiles + cut * a.pieces;
+    if (a.parts > 0 && a.part0 < 0) tails += cut;   // the level whose piece 0 is in the output adds up the parts
+  }
+  launch.first_block[LEVELS] = blocks;
+  launch.first_tail[LEVELS] = tails;
+  kern<<<blocks, GG_THREADS, smem_bytes, stream>>>(launch, launch.a[0].status);
+  if (tails > 0) {
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    const int items = a.d.C * (TILE_M / 4);
-    grad_fold_kernel<I2MAJOR><<<dim3((items + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS, tails), GG_FOLD_THREADS, 0, stream>>>(a);
+    const int items = launch.a[0].d.C * (TILE_M / 4);
+    grad_fold_kernel<I2MAJOR, LEVELS><<<dim3((items + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS, tails), GG_FOLD_THREADS, 0, stream>>>(launch);
   }
   return cudaGetLastError();
 }
 
-template <int MODE, int Q>
-static cudaError_t launch_major(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
-                                const CUtensorMap& tm_xv, cudaStream_t stream) {
-  if (a.op16 == OP16_FP16)
-    return a.image2_major ? launch_one<MODE, Q, 1, OP16_FP16>(a, tm_y, tm_xu, tm_xv, stream)
-                          : launch_one<MODE, Q, 0, OP16_FP16>(a, tm_y, tm_xu, tm_xv, stream);
-  if (a.op16 == OP16_BF16)
-    return a.image2_major ? launch_one<MODE, Q, 1, OP16_BF16>(a, tm_y, tm_xu, tm_xv, stream)
-                          : launch_one<MODE, Q, 0, OP16_BF16>(a, tm_y, tm_xu, tm_xv, stream);
-  return a.image2_major ? launch_one<MODE, Q, 1, 0>(a, tm_y, tm_xu, tm_xv, stream)
-                        : launch_one<MODE, Q, 0, 0>(a, tm_y, tm_xu, tm_xv, stream);
+template <int MODE, int Q, int I2MAJOR, int BF16>
+static cudaError_t launch_levels(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {
+  auto fill = [&](auto& launch) {
+    for (int l = 0; l < levels; ++l) {
+      launch.y[l] = maps.y[l];
+      launch.xu[l] = maps.xu[l];
+      launch.xv[l] = maps.xv[l];
+      launch.a[l] = a[l];
+    }
+  };
+  if constexpr (MODE == GRAD_FUSED) {
+    if (levels > 1) {
+      GradLaunch<MAX_FUSED_LEVELS> launch{};
+      fill(launch);
+      return launch_one<MODE, Q, I2MAJOR, BF16>(launch, levels, stream);
+    }
+  }
+  if (levels != 1) return cudaErrorInvalidValue;
+  GradLaunch<1> launch{};
+  fill(launch);
+  return launch_one<MODE, Q, I2MAJOR, BF16>(launch, 1, stream);
 }
 
-cudaError_t launch_grad_gemm(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
-                             const CUtensorMap& tm_xv, cudaStream_t stream) {
-  const int Q = a.R4 / 4;
-  if (a.mode == GRAD_MAXAVG && Q == 1) return launch_major<GRAD_MAXAVG, 1>(a, tm_y, tm_xu, tm_xv, stream);
-  if (a.mode == GRAD_COMPRESS && Q == 1) return launch_major<GRAD_COMPRESS, 1>(a, tm_y, tm_xu, tm_xv, stream);
-  if (a.mode == GRAD_COMPRESS && Q == 2) return launch_major<GRAD_COMPRESS, 2>(a, tm_y, tm_xu, tm_xv, stream);
-  if (a.mode == GRAD_FUSED && Q == 2) return launch_major<GRAD_FUSED, 2>(a, tm_y, tm_xu, tm_xv, stream);
-  if (a.mode == GRAD_FUSED && Q == 3) return launch_major<GRAD_FUSED, 3>(a, tm_y, tm_xu, tm_xv, stream);
+template <int MODE, int Q>
+static cudaError_t launch_major(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {
+  if (a->op16 == OP16_FP16)
+    return a->image2_major ? launch_levels<MODE, Q, 1, OP16_FP16>(a, levels, maps, stream) : launch_levels<MODE, Q, 0, OP16_FP16>(a, levels, maps, stream);
+  if (a->op16 == OP16_BF16)
+    return a->image2_major ? launch_levels<MODE, Q, 1, OP16_BF16>(a, levels, maps, stream) : launch_levels<MODE, Q, 0, OP16_BF16>(a, levels, maps, stream);
+  return a->image2_major ? launch_levels<MODE, Q, 1, 0>(a, levels, maps, stream) : launch_levels<MODE, Q, 0, 0>(a, levels, maps, stream);
+}
+
+cudaError_t launch_grad_gemm(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {
+  if (levels < 1 || levels > MAX_FUSED_LEVELS) return cudaErrorInvalidValue;
+  const int Q = a->R4 / 4;
+  if (a->mode == GRAD_MAXAVG && Q == 1) return launch_major<GRAD_MAXAVG, 1>(a, levels, maps, stream);
+  if (a->mode == GRAD_COMPRESS && Q == 1) return launch_major<GRAD_COMPRESS, 1>(a, levels, maps, stream);
+  if (a->mode == GRAD_COMPRESS && Q == 2) return launch_major<GRAD_COMPRESS, 2>(a, levels, maps, stream);
+  if (a->mode == GRAD_FUSED && Q == 2) return launch_major<GRAD_FUSED, 2>(a, levels, maps, stream);
+  if (a->mode == GRAD_FUSED && Q == 3) return launch_major<GRAD_FUSED, 3>(a, levels, maps, stream);
   return cudaErrorInvalidValue;
 }
 

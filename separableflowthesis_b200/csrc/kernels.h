@@ -189,9 +189,13 @@ struct GradArgs {
   int* status;
   unsigned long long wait_limit_ns;  // time limit of one device-side wait; 0 = the default (2 s)
   int whole_tiles, pieces;           // as in SweepArgs, here with pieces of the K sweep (TileSplit)
+  int parts, part0;                  // parts of a cut tile in scratch; piece i is part0 + i of them (-1: the output)
   float* part;
 };
 TileSplit grad_split(const Dims& d, int image2_major);
+// The same for the levels of a pyramid that share a launch (same image 1).  Image-1-major: the tiles of all levels but the first go to
+// scratch as a whole, to be added up.
+void grad_split_levels(const Dims* d, int levels, int image2_major, TileSplit* out);
 
 // Launchers, here and below: the returned error is taken off the runtime, so a caller must pass it on; dropping it does not
 // compile (unused results are errors in this build).
@@ -216,20 +220,20 @@ struct PackGroup {
   SlotSource s[4];
   float4* dst;    // the operand (B, D, Qtot, n1p, 4)
   int D, Qtot, q; // q: this group
+  const float* dev_scales;
 };
-constexpr int MAX_PACK_GROUPS = 6;
+constexpr int MAX_PACK_GROUPS = 6 * MAX_FUSED_LEVELS;
 struct PackGroups {
   PackGroup g[MAX_PACK_GROUPS];
   int count;
-  const float* dev_scales;
   void add(const SlotSources& src, float* dst, int D, int R4, int Qtot, int q0) {
     for (int q = 0; q < R4 / 4; ++q) {
       PackGroup& x = g[count++];
       for (int j = 0; j < 4; ++j) x.s[j] = src.s[4 * q + j];
       x.dst = reinterpret_cast<float4*>(dst);
       x.D = D; x.Qtot = Qtot; x.q = q0 + q;
+      x.dev_scales = src.dev_scales;
     }
-    dev_scales = src.dev_scales;
   }
 };
 inline int pack_groups_per_launch(int B) { return std::max(1, std::min(MAX_PACK_GROUPS, 65535 / B)); }
@@ -272,9 +276,17 @@ constexpr int ABSMAX_MAX = 4 * MAX_FUSED_LEVELS;
 struct AbsmaxSource { const float* p; size_t n; long long sb; int samples; float premul; int slot; };
 inline AbsmaxSource absmax_array(const float* p, size_t n, float premul, int slot) { return AbsmaxSource{p, n, (long long)n, 1, premul, slot}; }
 [[nodiscard]] cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int levels, bool gradients, cudaStream_t stream);
-// 16-bit channel-major copy from a (B, C, rows*width) feature map times `scale`, padding zeroed (layouts below).
-[[nodiscard]] cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
-                                    int blocked, float scale, int op16, const float* scale16, cudaStream_t stream);
+// Channel-major copies from the model's feature maps (B, C, rows*width) times `scale`, as 16-bit operands or (op16 = 0) TF32, padding
+// zeroed (layouts below); image 1 and the levels of image 2 in one launch.
+constexpr int MAX_MAP_COPIES = 1 + MAX_FUSED_LEVELS;
+struct MapCopy {
+  const float* src;
+  void* dst;
+  int rows, width, pitch, blocked;
+  float scale;
+  const float* scale16;
+};
+[[nodiscard]] cudaError_t launch_channel_major_cf(const MapCopy* copies, int count, int B, int C, int op16, cudaStream_t stream);
 // Channel-major copy of a pixel-major feature array (B, rows*width, C), as FP32 (of rounded values) or (op16 != 0) as 16-bit
 // operands (FP16: times the device scalar *scale16); padding is not written.
 //   blocked = 0: dst (B, C, pitch) with pixel index row*width + x (rows = 1)
@@ -293,10 +305,10 @@ inline AbsmaxSource absmax_array(const float* p, size_t n, float premul, int slo
 // The levels of a pyramid in one launch (same image 1, mode, channels and operand type).
 [[nodiscard]] cudaError_t launch_sweep_levels(const SweepArgs* a, int levels, const CUtensorMap& tm_f1, const CUtensorMap* tm_f2,
                                 const CUtensorMap* tm_aux, cudaStream_t stream);
-// tm_y: channel-major features of the other image (K-major B operand); tm_xu / tm_xv: interleaved operands (tm_xv is only read by the
-// image-2-major form; the image-1-major form keeps its (pixel, v) slots in registers).
-[[nodiscard]] cudaError_t launch_grad_gemm(const GradArgs& a, const CUtensorMap& tm_y, const CUtensorMap& tm_xu,
-                             const CUtensorMap& tm_xv, cudaStream_t stream);
+// Per level: y, channel-major features of the other image (K-major B operand); xu / xv, interleaved operands (xv is only read by the
+// image-2-major form; the image-1-major form keeps its (pixel, v) slots in registers).  Several levels: GRAD_FUSED only.
+struct GradMaps { CUtensorMap y[MAX_FUSED_LEVELS], xu[MAX_FUSED_LEVELS], xv[MAX_FUSED_LEVELS]; };
+[[nodiscard]] cudaError_t launch_grad_gemm(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream);
 
 
 // Attention weights A = softmax over d of Conv3d(2 -> Kc, 3x3x3, padding 1)(X) on channels-first tensors
@@ -325,14 +337,26 @@ int attention_forward_launches(const AttentionJob* jobs, int count, const int* s
 // dimensions 1 .. rank-1.  Implemented next to the other tensor maps (c_abi.cu).
 [[nodiscard]] cudaError_t encode_plain_map(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,
                              const uint64_t* strides_bytes, const uint32_t* box);
-// Floats of scratch the backward needs for its per-block partial sums.
-size_t attention_partial_floats(const AttentionDims& d);
+// Floats of scratch the backward of these jobs needs for its per-block partial sums.
+size_t attention_partial_floats(const AttentionDims* d, int count);
 // Backward: `g` holds dLoss/dA on entry and the logit gradients on return; gx (B, 2, D, H1, W1) = add + dLoss/dX
-// where `add` (same shape, `add_sb` elements between samples) may be null; gweight (Kc, 2, 3, 3, 3), gbias (Kc).
-[[nodiscard]] cudaError_t launch_attention_backward(const AttentionDims& d, const float* x, long long x_sb, const float* weight,
-                                      const float* a, float* g, const float* add, long long add_sb, float* gx,
-                                      float* gweight, float* gbias, float* partial, cudaStream_t stream,
-                                      int* status = nullptr);
+// where `add` (same shape, `add_sb` elements between samples) may be null.  The gradients of a module, weight (Kc, 2, 3, 3, 3) and bias
+// (Kc), are summed over the jobs that use it.
+struct AttentionGradients { float *weight[2], *bias[2]; };
+struct AttentionGradJob {
+  AttentionDims d;
+  int module;
+  const float* x;
+  long long x_sb;
+  const float* a;
+  float* g;
+  const float* add;
+  long long add_sb;
+  float* gx;
+};
+[[nodiscard]] cudaError_t launch_attention_backward(const AttentionGradJob* jobs, int count, const AttentionModules& modules,
+                                      const AttentionGradients& grads, float* partial, cudaStream_t stream, int* status = nullptr);
+int attention_backward_launches(const AttentionGradJob* jobs, int count);
 
 
 // Linear resampling along the displacement axis (core/corr.py:459-467: trilinear interpolate with unchanged H1, W1):
@@ -346,9 +370,15 @@ struct ResampleJob {
   int Dl, D0;
 };
 [[nodiscard]] cudaError_t launch_upsample_displacement(const ResampleJob* jobs, int count, int B, int K, int N1, cudaStream_t stream);
-// Its adjoint: gin (B, K, Dl, N1) from the gradient of those K channels.
-[[nodiscard]] cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
-                                                 int D0, int N1, cudaStream_t stream);
+// Its adjoint: in (B, K, Dl, N1) is written, from the gradient of those K channels (out is read).
+struct ResampleAdjointJob {
+  const float* gout;
+  long long gout_sb;
+  float* gin;
+  int Dl, D0;
+};
+[[nodiscard]] cudaError_t launch_upsample_displacement_adjoint(const ResampleAdjointJob* jobs, int count, int B, int K, int N1,
+                                                 cudaStream_t stream);
 
 // Lookup on an aggregated 3D cost volume (the reference's CorrBlock1D, core/corr.py:513-624).
 // corr (B, dim, D, H1, W1); pyramid = levels 1 .. levels-1 back to back, level l being (B, dim, D >> l, H1, W1);

@@ -412,7 +412,7 @@ pack_interleaved_cf_kernel(const __grid_constant__ PackGroups groups, int B, int
     const SlotSource& ss = g.s[j];
     src[j] = ss.src == nullptr ? nullptr : static_cast<const uint32_t*>(ss.src) + (((size_t)b * ss.Ksrc + ss.k) * D + d0) * N1 + p;
     fac[j] = ss.scale;
-    if (ss.dev != 0 && ss.src != nullptr) fac[j] = (ss.scale != 0.f ? ss.scale : 1.f) * __ldg(groups.dev_scales + ss.dev - 1);
+    if (ss.dev != 0 && ss.src != nullptr) fac[j] = (ss.scale != 0.f ? ss.scale : 1.f) * __ldg(g.dev_scales + ss.dev - 1);
   }
   uint32_t w[PI_DB][4];
 #pragma unroll
@@ -507,35 +507,49 @@ transpose_round_kernel(const __grid_constant__ TransposeJobs jobs, int C, int op
   }
 }
 
-// 16-bit channel-major copies straight from the model's feature maps (B, C, rows*width), times `scale` and, for FP16, the
-// device scalar: the layouts of channel_major_kernel, padding included (zeros), two values per store.  One grid row per
-// channel of a sample: grid (ceil(pairs per channel / 256), C, B).
+// Channel-major copies straight from the model's feature maps (B, C, rows*width), times `scale`: as 16-bit operands (FP16: times the device
+// scalar as well) or TF32.  The layouts of channel_major_kernel, padding included (zeros), two values per store.  One grid row per
+// channel of a sample: grid (sum over the copies of ceil(pairs per channel / 256), C, B).
+struct MapCopies {
+  MapCopy c[MAX_MAP_COPIES];
+  int first[MAX_MAP_COPIES];   // of grid.x; copies that do not exist start past its end
+};
+__host__ __device__ inline int map_copy_channel(const MapCopy& c) { return c.blocked ? (c.width + 15) / 16 * c.pitch * 16 : c.pitch; }
 __global__ void __launch_bounds__(256)
-channel_major_cf_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, int rows, int width, int pitch, int C,
-                        int blocked, float scale, int op16, const float* __restrict__ scale16) {
-  const int per_channel = blocked ? (width + 15) / 16 * pitch * 16 : pitch;
-  const int i = (blockIdx.x * 256 + threadIdx.x) * 2;
+channel_major_cf_kernel(const __grid_constant__ MapCopies copies, int C, int op16) {
+  int ci = 0;
+#pragma unroll
+  for (int i = 1; i < MAX_MAP_COPIES; ++i) ci = (int)blockIdx.x >= copies.first[i] ? i : ci;
+  const MapCopy& copy = copies.c[ci];
+  const int per_channel = map_copy_channel(copy), width = copy.width;
+  const int i = ((blockIdx.x - copies.first[ci]) * 256 + threadIdx.x) * 2;
   if (i >= per_channel) return;
-  const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
+  const float sc16 = (op16 == OP16_FP16 && copy.scale16 != nullptr) ? __ldg(copy.scale16) : 1.f;
   int row = 0, x = i;
-  if (blocked) {
-    const int xb = i / (pitch * 16), r = i - xb * pitch * 16;
+  if (copy.blocked) {
+    const int xb = i / (copy.pitch * 16), r = i - xb * copy.pitch * 16;
     row = r / 16;
     x = xb * 16 + (r & 15);
   }
   const size_t chan = (size_t)blockIdx.z * C + blockIdx.y;
-  const float* src = in + (chan * rows + row) * width + x;
-  const bool ok = row < rows;
-  const float lo = ok && x < width ? __ldg(src) * scale : 0.f, hi = ok && x + 1 < width ? __ldg(src + 1) * scale : 0.f;
-  out[(chan * per_channel + i) / 2] = op16 == OP16_FP16 ? pack_fp16x2(lo * sc16, hi * sc16) : pack_bf16x2(lo, hi);
+  const float* src = copy.src + (chan * copy.rows + row) * width + x;
+  const bool ok = row < copy.rows;
+  const float lo = ok && x < width ? __ldg(src) * copy.scale : 0.f, hi = ok && x + 1 < width ? __ldg(src + 1) * copy.scale : 0.f;
+  const size_t at = (chan * per_channel + i) / 2;
+  if (op16 == 0) static_cast<float2*>(copy.dst)[at] = make_float2(round_tf32(lo), round_tf32(hi));
+  else static_cast<uint32_t*>(copy.dst)[at] = op16 == OP16_FP16 ? pack_fp16x2(lo * sc16, hi * sc16) : pack_bf16x2(lo, hi);
 }
 
-cudaError_t launch_channel_major_cf(const float* src, uint16_t* dst, int B, int rows, int width, int pitch, int C,
-                                    int blocked, float scale, int op16, const float* scale16, cudaStream_t stream) {
-  const int per_channel = blocked ? (width + 15) / 16 * pitch * 16 : pitch;
-  const dim3 grid((per_channel / 2 + 255) / 256, C, B);
-  channel_major_cf_kernel<<<grid, 256, 0, stream>>>(src, reinterpret_cast<uint32_t*>(dst), rows, width, pitch, C, blocked,
-                                                    scale, op16, scale16);
+cudaError_t launch_channel_major_cf(const MapCopy* copy, int count, int B, int C, int op16, cudaStream_t stream) {
+  if (count < 1 || count > MAX_MAP_COPIES) return cudaErrorInvalidValue;
+  MapCopies copies;
+  int blocks = 0;
+  for (int i = 0; i < MAX_MAP_COPIES; ++i) {
+    copies.c[i] = copy[i < count ? i : 0];
+    copies.first[i] = i < count ? blocks : INT_MAX;
+    if (i < count) blocks += (map_copy_channel(copy[i]) / 2 + 255) / 256;
+  }
+  channel_major_cf_kernel<<<dim3(blocks, C, B), 256, 0, stream>>>(copies, C, op16);
   return cudaGetLastError();
 }
 

@@ -18,7 +18,7 @@ __device__ __forceinline__ void resample_source(int d, float scale, int Dl, int&
   i0 = (int)src;
   if (i0 > Dl - 1) i0 = Dl - 1;
   i1 = i0 + (i0 < Dl - 1 ? 1 : 0);
-  l1 = src - (float)i0;
+  l1 = fmaf(scale, (float)d, -(float)i0);   // in every kernel alike, so that what they add up is the same
   l0 = 1.f - l1;
 }
 
@@ -75,19 +75,30 @@ upsample_displacement_kernel(const __grid_constant__ ResampleJobs jobs, int K, i
 // so only launches of fewer than RS_CUT_BELOW blocks are cut, which on their own leave HBM idle.  Whole and cut, us:
 // 55 blocks (1 x 55 x 128, 128 -> 128 rows) 35 and 10, 464 (8 x 47 x 156, 156 rows) 50 and 39, 1016 (4 x 135 x 240, 240 rows)
 // 100 and 115, 2784 (six channels of 8 x 47 x 156) 153 and 197, 6096 (six of 4 x 135 x 240) 472 and 647.
-// grid (ceil(N1/128), B*K, CUT ? ceil(Dl/RS_IB) : 1)
+// The volumes of a launch are cut together or not at all.
+// grid (ceil(N1/128), B*K, sum over the volumes of CUT ? ceil(Dl/RS_IB) : 1)
 constexpr int RS_IB = 8, RS_CUT_BELOW = 6 * SM_COUNT;
+struct ResampleAdjointJobs {
+  ResampleAdjointJob j[MAX_RESAMPLE_JOBS];
+  float scale[MAX_RESAMPLE_JOBS];
+  int first[MAX_RESAMPLE_JOBS];   // of grid.z; volumes that do not exist start past its end
+};
 
 template <bool CUT>
 __global__ void __launch_bounds__(RS_THREADS)
-upsample_displacement_adjoint_kernel(const float* __restrict__ gout, long long gout_sb, float* __restrict__ gin, int K,
-                                     int Dl, int D0, int N1, float scale) {
+upsample_displacement_adjoint_kernel(const __grid_constant__ ResampleAdjointJobs jobs, int K, int N1) {
+  int ji = 0;
+#pragma unroll
+  for (int i = 1; i < MAX_RESAMPLE_JOBS; ++i) ji = (int)blockIdx.z >= jobs.first[i] ? i : ji;
+  const ResampleAdjointJob& job = jobs.j[ji];
+  const int Dl = job.Dl, D0 = job.D0;
+  const float scale = jobs.scale[ji];
   const int p = blockIdx.x * RS_THREADS + threadIdx.x;
   if (p >= N1) return;
   const int b = blockIdx.y / K, k = blockIdx.y - b * K;
-  const int r0 = CUT ? blockIdx.z * RS_IB : 0, r1 = CUT ? min(r0 + RS_IB, Dl) : Dl;
-  const float* g = gout + (size_t)b * gout_sb + ((size_t)k * D0) * N1 + p;
-  float* dst = gin + ((size_t)blockIdx.y * Dl) * N1 + p;
+  const int r0 = CUT ? (blockIdx.z - jobs.first[ji]) * RS_IB : 0, r1 = CUT ? min(r0 + RS_IB, Dl) : Dl;
+  const float* g = job.gout + (size_t)b * job.gout_sb + ((size_t)k * D0) * N1 + p;
+  float* dst = job.gin + ((size_t)blockIdx.y * Dl) * N1 + p;
   // first output row with lower neighbour >= r0 - 1: an estimate, corrected with the exact rule (neighbours never fall
   // as d grows)
   int first = 0;
@@ -161,13 +172,22 @@ cudaError_t launch_upsample_displacement(const ResampleJob* job, int count, int 
   return cudaGetLastError();
 }
 
-cudaError_t launch_upsample_displacement_adjoint(const float* gout, long long gout_sb, float* gin, int B, int K, int Dl,
-                                                 int D0, int N1, cudaStream_t st) {
+cudaError_t launch_upsample_displacement_adjoint(const ResampleAdjointJob* job, int count, int B, int K, int N1, cudaStream_t st) {
+  if (count < 1 || count > MAX_RESAMPLE_JOBS) return cudaErrorInvalidValue;
   const int blocks = (N1 + RS_THREADS - 1) / RS_THREADS;
-  const bool cut = Dl > RS_IB && (long long)blocks * B * K < RS_CUT_BELOW;
-  const dim3 grid(blocks, B * K, cut ? (Dl + RS_IB - 1) / RS_IB : 1);
+  bool cut = false;
+  for (int i = 0; i < count; ++i) cut = cut || job[i].Dl > RS_IB;
+  cut = cut && (long long)blocks * B * K * count < RS_CUT_BELOW;
+  ResampleAdjointJobs jobs;
+  int pieces = 0;
+  for (int i = 0; i < MAX_RESAMPLE_JOBS; ++i) {
+    jobs.j[i] = job[i < count ? i : 0];
+    jobs.first[i] = i < count ? pieces : INT_MAX;
+    jobs.scale[i] = resample_scale(jobs.j[i].Dl, jobs.j[i].D0);
+    if (i < count) pieces += cut ? (job[i].Dl + RS_IB - 1) / RS_IB : 1;
+  }
   auto kern = cut ? upsample_displacement_adjoint_kernel<true> : upsample_displacement_adjoint_kernel<false>;
-  kern<<<grid, RS_THREADS, 0, st>>>(gout, gout_sb, gin, K, Dl, D0, N1, resample_scale(Dl, D0));
+  kern<<<dim3(blocks, B * K, pieces), RS_THREADS, 0, st>>>(jobs, K, N1);
   return cudaGetLastError();
 }
 

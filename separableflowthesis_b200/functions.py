@@ -268,14 +268,12 @@ class SeparationPyramidFunction(Function):
         L, Kt = len(fmap2_levels), 2 + weight_u.shape[0]
         saved = []
         ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, L
-        if _levels_together(fmap1, fmap2_levels, weight_u.shape[0]):
+        ctx.together = _levels_together(fmap1, fmap2_levels, weight_u.shape[0])
+        if ctx.together:
             with torch.cuda.device_of(fmap1):
                 sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
             if with_argmax:
-                saved = MemorySaver.separation_pyramid_saved(buffer, fmap1, fmap2_levels, weight_u.shape[0], True)
-                ctx.in_place = [t[0] is None for t in saved]
-                flat = [x for t in saved for x in t if x is not None]
-                ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, *flat)
+                ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, buffer)
             return sep_u, sep_v
         with torch.cuda.device_of(fmap1):
             sep_u = torch.empty(B, Kt * L, W2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
@@ -308,6 +306,11 @@ class SeparationPyramidFunction(Function):
         flat = list(ctx.saved_tensors[5 + L:])
         wu, wv = weight_u.contiguous(), weight_v.contiguous()
         gu, gv = grad_sep_u.contiguous(), grad_sep_v.contiguous()
+        if ctx.together:
+            with torch.cuda.device_of(gu):
+                g1, g2, gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(fmap1, fmap2_levels, wu, wv, sep_u, sep_v, flat[0],
+                                                                                         gu, gv, ctx.scale1)
+            return (None, None, gw_u, gb_u, gw_v, gb_v, g1, *g2)
         Kt = 2 + weight_u.shape[0]
         g1 = gw_u = gb_u = gw_v = gb_v = None
         g2 = []

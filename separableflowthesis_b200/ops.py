@@ -524,13 +524,50 @@ def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, 
     saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax)), 256), dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
-        ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L), 256), dev, stream)
+        ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, 0), 256), dev, stream)
         _raise_on(lib.sfb_separation_pyramid_forward(
             fmap1.data_ptr(), ptrs, H2, W2, L, scale1, weight_u.data_ptr(), bias_u.data_ptr(), weight_v.data_ptr(), bias_v.data_ptr(),
             sep_u.data_ptr(), sep_v.data_ptr(), saved.data_ptr(), saved.numel(), int(with_argmax), shape, ws.data_ptr(), ws.numel(),
             stream), "sfb_separation_pyramid_forward")
         _check_device_status(lib, "sfb_separation_pyramid_forward", ws, stream)
     return sep_u, sep_v, saved
+
+
+def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, g_sep_u, g_sep_v, scale1):
+    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max."""
+    s = None
+    for f2 in fmap2_levels:
+        level = _check_fmaps(fmap1, f2)
+        s = s or level
+    dev = fmap1.device
+    _check(weight_u, "attention1.weight", torch.float32, 5)
+    s.Kc = weight_u.shape[0]
+    _check_like(weight_u, "attention1.weight", (s.Kc, 2, 3, 3, 3), torch.float32, dev)
+    _check_like(weight_v, "attention2.weight", (s.Kc, 2, 3, 3, 3), torch.float32, dev)
+    L = len(fmap2_levels)
+    Kt = (2 + s.Kc) * L
+    for t, name, D in ((sep_u, "sep_u", s.W2), (sep_v, "sep_v", s.H2), (g_sep_u, "grad_sep_u", s.W2), (g_sep_v, "grad_sep_v", s.H2)):
+        _check_like(t, name, (s.B, Kt, D, s.H1, s.W1), torch.float32, dev)
+    _check(saved, "saved", torch.uint8, 1)
+    gF1 = torch.empty_like(fmap1)
+    gF2 = [torch.empty_like(f2) for f2 in fmap2_levels]
+    gw_u, gw_v = torch.empty_like(weight_u), torch.empty_like(weight_v)
+    gb_u = torch.empty(s.Kc, dtype=torch.float32, device=dev)
+    gb_v = torch.empty(s.Kc, dtype=torch.float32, device=dev)
+    lib = _lib.load()
+    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels)
+    gptrs = (ctypes.c_void_p * L)(*[t.data_ptr() for t in gF2])
+    shape = ctypes.byref(s)
+    with torch.cuda.device(dev):
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, 1), 256), dev, stream)
+        _raise_on(lib.sfb_separation_pyramid_backward(
+            fmap1.data_ptr(), ptrs, H2, W2, L, scale1, weight_u.data_ptr(), weight_v.data_ptr(), sep_u.data_ptr(), sep_v.data_ptr(),
+            saved.data_ptr(), saved.numel(), g_sep_u.data_ptr(), g_sep_v.data_ptr(), gF1.data_ptr(), gptrs, gw_u.data_ptr(),
+            gb_u.data_ptr(), gw_v.data_ptr(), gb_v.data_ptr(), shape, ws.data_ptr(), ws.numel(), stream),
+            "sfb_separation_pyramid_backward")
+        _check_device_status(lib, "sfb_separation_pyramid_backward", ws, stream)
+    return gF1, gF2, gw_u, gb_u, gw_v, gb_v
 
 
 def separation_pyramid_saved(saved, fmap1, fmap2_levels, Kc, with_argmax):

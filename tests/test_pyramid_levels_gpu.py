@@ -57,3 +57,48 @@ def test_forward(shape, with_argmax, operands, cuda_device):
     for got, want in zip(ops.separation_pyramid_saved(buffer, f1, pyr, Kc, with_argmax), ref):
         for x, y in zip(got, want):
             assert (x is None) == (y is None) and (x is None or torch.equal(x, y))
+
+
+# The feature gradients are sums over up to H*W pixels that the tensor core forms 8 (TF32) or 16 products at a time, each addition to the
+# FP32 accumulator cut off at 2^-23 of it: other pieces of the sum, other errors, up to H*W / 8 * 2^-23 of the result.  Beside that
+# (and for the parameters alone): sums over levels and blocks in another order, 2^-24 of a few hundred terms each; and FP16 operands may take
+# another power of two where a level's gradients are searched without its neighbours', for values in FP16's subnormal range (2^-25 of
+# the largest).
+TOL = 2e-5
+
+
+def relerr(x, ref):
+    return ((x.double() - ref.double()).norm() / ref.double().norm().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("operands", ["fp16", "tf32", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_backward(shape, operands, cuda_device):
+    B, C, H, W, Kc, levels = shape
+    if operands == "bf16" and C % 8:
+        pytest.skip("needs C % 8 == 0")
+    f1, pyr, params = inputs(B, C, H, W, Kc, levels, H * W + Kc, cuda_device)
+    scale1, Kt, tol = 1 / math.sqrt(C), 2 + Kc, H * W / 8 * 2 ** -23 + TOL
+    gen = torch.Generator().manual_seed(3)
+    gu = torch.randn(B, Kt * levels, W, H, W, generator=gen).to(cuda_device)
+    gv = torch.randn(B, Kt * levels, H, H, W, generator=gen).to(cuda_device)
+    with ops.sweep_operands(operands):
+        sep_u, sep_v, buffer = ops.separation_pyramid_forward(f1, pyr, *params, True, scale1)
+        g1, g2, *gp = ops.separation_pyramid_backward(f1, pyr, params[0], params[2], sep_u, sep_v, buffer, gu, gv, scale1)
+        _, _, saved = one_by_one(f1, pyr, params, True)
+        ref1, refp = 0, [0, 0, 0, 0]
+        for l, (f2, (su, sv, am_u, am_v, a_u, a_v)) in enumerate(zip(pyr, saved)):
+            if l == 0:
+                out = ops.separation_level_backward(f1, f2, params[0], params[2], sep_u, sep_v, am_u, am_v, a_u, a_v, gu, gv, True, scale1, 0)
+            else:
+                gsu = ops.upsample_displacement_backward(gu, l * Kt, Kt, su.shape[2])
+                gsv = ops.upsample_displacement_backward(gv, l * Kt, Kt, sv.shape[2])
+                out = ops.separation_level_backward(f1, f2, params[0], params[2], su, sv, am_u, am_v, a_u, a_v, gsu, gsv, True, scale1)
+            assert relerr(g2[l], out[1]) < tol
+            ref1 = ref1 + out[0].double()
+            refp = [r + p.double() for r, p in zip(refp, out[2:])]
+        again = ops.separation_pyramid_backward(f1, pyr, params[0], params[2], sep_u, sep_v, buffer, gu, gv, scale1)
+    assert relerr(g1, ref1) < tol
+    # a softmax does not see its bias: those gradients are rounding
+    assert relerr(gp[0], refp[0]) < TOL and relerr(gp[2], refp[2]) < TOL
+    assert torch.equal(again[0], g1) and all(torch.equal(x, y) for x, y in zip(again[1], g2)) and all(torch.equal(x, y) for x, y in zip(again[2:], gp))
