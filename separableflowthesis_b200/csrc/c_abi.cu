@@ -242,6 +242,8 @@ struct Workspace {
   size_t bytes;        // without the scratch of the tail pieces, which a caller's buffer may lack (the kernels then
   float* part;         // do whole tiles only)
   size_t part_bytes;
+  uint8_t* stored;     // G between the gradient GEMMs, behind the scratch; a buffer may lack it as well (G is then generated twice)
+  size_t stored_bytes;  // the samples that the buffer has room for
 };
 
 int padded_pixels(const Dims& d) { return (d.N1() + TILE_M - 1) / TILE_M * TILE_M; }
@@ -277,6 +279,19 @@ WsPlan plan_for(int op, const Dims& d) {
     case SFB_OP_SEPARATION_LEVEL_BACKWARD: return {false, 0, 0, 4 + grad_slots(chunk_channels(d.Kc)), true, true};
     default: return {false, 0, 0, 0, false, false};
   }
+}
+
+// Whether a pair of gradient GEMMs over one or several levels of an image 2 hands G over through memory, or generates it twice.  The storing
+// GEMM has one tile per 128 image-1 pixels whose generator waits for its own stores, the reading one tiles of 256 image-2 pixels: less than a
+// wave of short tiles gains nothing.  Pairs of one level, C = 256, generated twice / stored (us): 2 x 48 x 64 on itself 70 / 74, 6 x 48 x 64 (144
+// tiles) 103 / 114, 4 x 55 x 128 on 13 x 32 64 / 68, 1 x 40 x 100 69 / 72; 8 x 48 x 64 (192 tiles) 161 / 138, 32 x 24 x 32 (192) 81 / 68,
+// 4 x 55 x 128 on 27 x 64 136 / 122, 1 x 55 x 128 (55 tiles of 7040 values each) 134 / 121, 1 x 135 x 240 1578 / 1166.
+bool grad_hands_over(const Dims& d, int levels) {
+  return d.N2() > 4096 || (d.N2() >= 512 && (long long)d.B * ((d.N1() + TILE_M - 1) / TILE_M) * levels > SM_COUNT);
+}
+// Samples whose G (`bytes` each) is stored at a time: all, as many as fit, or (0) none.
+int grad_chunk(const Dims& d, int levels, size_t bytes) {
+  return grad_hands_over(d, levels) ? (int)std::min<size_t>(d.B, GRAD_STORED_LIMIT / bytes) : 0;
 }
 
 Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
@@ -325,9 +340,20 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   size_t part = 0;
   if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS, false).part_floats);
   if (d.Kc > 0 && plan.sweeps) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
-  if (plan.Rg) part = std::max(part, std::max(grad_split(d, 0).part_floats, grad_split(d, 1).part_floats));
+  const int samples = plan.Rg ? grad_chunk(d, 1, grad_stored_bytes(d, w.n1p)) : 0;
+  if (plan.Rg) {
+    for (const int form : {GRAD_IMAGE1, GRAD_IMAGE2}) part = std::max(part, grad_split(d, form).part_floats);
+    for (const int n : {samples, samples > 0 ? d.B % samples : 0}) {   // full chunks and what is left
+      if (n == 0) continue;
+      Dims some = d;
+      some.B = n;
+      for (const int form : {GRAD_IMAGE1_STORING, GRAD_IMAGE2_STORED}) part = std::max(part, grad_split(some, form).part_floats);
+    }
+  }
   w.part = reinterpret_cast<float*>(p + off);
-  w.part_bytes = part * sizeof(float);
+  w.part_bytes = align_up(part * sizeof(float), 256);
+  w.stored = reinterpret_cast<uint8_t*>(p + off + w.part_bytes);
+  w.stored_bytes = samples * grad_stored_bytes(d, w.n1p);
   return w;
 }
 
@@ -346,7 +372,7 @@ void set_sweep_split(SweepArgs& a, const Workspace& w, int slots) {
 
 // The same for a gradient GEMM.
 void set_grad_split(GradArgs& a, const Workspace& w) {
-  const TileSplit s = grad_split(a.d, a.image2_major);
+  const TileSplit s = grad_split(a.d, a.form);
   const bool cut = s.pieces > 1 && s.part_floats * sizeof(float) <= w.part_bytes;
   a.whole_tiles = cut ? s.whole_tiles : s.tiles;
   a.pieces = cut ? s.pieces : 1;
@@ -414,7 +440,9 @@ int check_workspace(const Dims& d, void* ws, size_t ws_bytes, int op, Workspace*
   *out = carve(d, ws, plan_for(op, d));
   if (ws_bytes < out->bytes)
     return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", ws_bytes, out->bytes);
-  if (ws_bytes < out->bytes + out->part_bytes) out->part_bytes = 0;
+  const size_t room = ws_bytes - out->bytes;
+  out->stored_bytes = room > out->part_bytes ? std::min(out->stored_bytes, room - out->part_bytes) : 0;
+  if (room < out->part_bytes) out->part_bytes = 0;
   return SFB_OK;
 }
 
@@ -592,8 +620,9 @@ int run_compress_sweeps(const Dims& d, const Workspace& w, const CUtensorMap& tm
 // rows, so that a 4 x 16 block of the image is 64 consecutive values).  Rows and columns of padding must
 // read as zero: they meet the G values of cells outside the image.
 size_t f2t_per_sample(const Dims& d, const Workspace& w) { return (size_t)d.C * ((d.W2 + GG_VT - 1) / GG_VT) * w.h2p * GG_VT; }
-int grad_arguments(const Dims& d, const Workspace& w, int op16, int mode, int R4, int image2_major, float* out, int out_cf, float scale1,
+int grad_arguments(const Dims& d, const Workspace& w, int op16, int mode, int R4, int form, float* out, int out_cf, float scale1,
                    GradArgs* a, CUtensorMap* tm_y, CUtensorMap* tm_xu, CUtensorMap* tm_xv) {
+  const bool image2_major = grad_is_image2(form);
   memset(a, 0, sizeof(*a));
   a->d = d;
   a->mode = mode;
@@ -604,8 +633,9 @@ int grad_arguments(const Dims& d, const Workspace& w, int op16, int mode, int R4
   a->status = w.status;
   a->op16 = op16;
   a->out_cf = out_cf;
-  a->image2_major = image2_major;
+  a->form = form;
   a->out = out;
+  a->stored = w.stored;
   a->out_scale = image2_major ? 1.f : scale1;
   a->dev_scale = op16 == OP16_FP16 ? w.scales + (image2_major ? SCALE_INV_GF2 : SCALE_INV_GF1) : nullptr;
   const int Q = R4 / 4;
@@ -618,11 +648,16 @@ int grad_arguments(const Dims& d, const Workspace& w, int op16, int mode, int R4
     *tm_xv = *tm_xu;  // unused
     return SFB_OK;
   }
-  // (N1, C, B) with rows padded to n1p; box = 32 pixels x all channels: a row of 32 K-values is 128 bytes of FP32 or 64 bytes of a
-  // 16-bit type, the swizzle span follows
+  // (N1, C, B) with rows padded to n1p; box = the pixels of a block x all channels: a row of 32 K-values is 128 bytes of FP32 or 64 bytes of
+  // a 16-bit type, one of 64 16-bit values 128 bytes; the swizzle span follows
+  const bool stored = form == GRAD_IMAGE2_STORED;
   const uint64_t dims[3] = {(uint64_t)d.N1(), (uint64_t)d.C, (uint64_t)d.B};
-  const uint32_t box[3] = {GG_KJ, crows, 1};
-  SFB_TRY(make_map(tm_y, w.F1t, 3, dims, box, op16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0, (uint64_t)w.n1p));
+  const uint32_t box[3] = {stored ? (uint32_t)GG_SJ : (uint32_t)GG_KJ, crows, 1};
+  SFB_TRY(make_map(tm_y, w.F1t, 3, dims, box, op16 && !stored ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, op16 != 0, (uint64_t)w.n1p));
+  if (stored) {
+    *tm_xu = *tm_xv = *tm_y;  // unused
+    return SFB_OK;
+  }
   SFB_TRY(map_operands(tm_xu, w.gxu, d.B, d.H2, Q, w.n1p, GG_KJ, GG_ROW_UT));
   return map_operands(tm_xv, w.gxv, d.B, d.W2, Q, w.n1p, GG_KJ, GG_ROW_VT);
 }
@@ -654,14 +689,21 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
       return launch_channel_major(op16 ? feat.F2 : w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
     }));
   }
-  for (const int image2_major : {0, 1}) {
-    GradArgs a;
-    GradMaps maps;
-    SFB_TRY(grad_arguments(d, w, op16, mode, R4, image2_major, image2_major ? gF2 : gF1, out_cf, scale1, &a, maps.y, maps.xu, maps.xv));
-    a.accumulate = accumulate;
-    set_grad_split(a, w);
-    a = with_wait_settings(a);
-    SFB_CUDA(timed(kid + image2_major, contraction_launches(a), st, [&] { return launch_grad_gemm(&a, 1, maps, st); }));
+  // 16-bit operands: G of as many samples as the workspace takes is generated and stored by one GEMM and read back by the other
+  const int samples = op16 != 0 ? (int)(w.stored_bytes / grad_stored_bytes(d, w.n1p)) : 0;
+  for (int b0 = 0; b0 < d.B; b0 += samples > 0 ? samples : d.B) {
+    for (const int form : {samples > 0 ? GRAD_IMAGE1_STORING : GRAD_IMAGE1, samples > 0 ? GRAD_IMAGE2_STORED : GRAD_IMAGE2}) {
+      const bool image2_major = grad_is_image2(form);
+      GradArgs a;
+      GradMaps maps;
+      SFB_TRY(grad_arguments(d, w, op16, mode, R4, form, image2_major ? gF2 : gF1, out_cf, scale1, &a, maps.y, maps.xu, maps.xv));
+      a.accumulate = accumulate;
+      a.b0 = b0;
+      if (samples > 0) a.d.B = std::min(samples, d.B - b0);
+      set_grad_split(a, w);
+      a = with_wait_settings(a);
+      SFB_CUDA(timed(kid + (image2_major ? 1 : 0), contraction_launches(a), st, [&] { return launch_grad_gemm(&a, 1, maps, st); }));
+    }
   }
   return SFB_OK;
 }
@@ -787,7 +829,7 @@ size_t sfb_workspace_bytes(int op, const sfb_shape* shape) {
                        op == SFB_OP_SEPARATION_LEVEL_BACKWARD;
   if (check_shape(shape, need_kc, &d) != SFB_OK) return 0;
   const Workspace w = carve(d, nullptr, plan_for(op, d));
-  return w.bytes + w.part_bytes;
+  return w.bytes + w.part_bytes + w.stored_bytes;
 }
 
 int sfb_max_avg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, const sfb_shape* shape,
@@ -1523,7 +1565,9 @@ PyramidWorkspace carve_pyramid_forward(const Pyramid& py, void* base) {
 struct PyramidBackward {
   Workspace w[MAX_FUSED_LEVELS];
   float *gs_u[MAX_FUSED_LEVELS], *gs_v[MAX_FUSED_LEVELS];
-  size_t bytes;
+  int samples;             // whose G of all levels is stored at a time (0: none)
+  size_t bytes;            // without the stored G, which a caller's buffer may lack
+  size_t stored_bytes;
 };
 PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
   PyramidBackward p;
@@ -1567,16 +1611,29 @@ PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
   }
   p.w[0].at_partial = take(attention_partial_floats(at, 2 * py.levels));
   TileSplit split[MAX_FUSED_LEVELS];
-  size_t part = pyramid_part_floats(py, chunk_channels(d0.Kc), true, split);
-  for (const int image2_major : {0, 1}) {
-    grad_split_levels(py.d, py.levels, image2_major, split);
+  size_t part = pyramid_part_floats(py, chunk_channels(d0.Kc), true, split), stored = 0;
+  for (int l = 0; l < py.levels; ++l) stored += grad_stored_bytes(py.d[l], n1p);
+  p.samples = grad_chunk(d0, py.levels, stored);
+  auto grad_parts = [&](int form, int samples) {
+    Dims d[MAX_FUSED_LEVELS];
+    for (int l = 0; l < py.levels; ++l) {
+      d[l] = py.d[l];
+      d[l].B = samples;
+    }
+    grad_split_levels(d, py.levels, form, split);
     size_t floats = 0;
     for (int l = 0; l < py.levels; ++l) floats += split[l].part_floats;
     part = std::max(part, floats);
-  }
+  };
+  for (const int form : {GRAD_IMAGE1, GRAD_IMAGE2}) grad_parts(form, d0.B);
+  for (const int n : {p.samples, p.samples > 0 ? d0.B % p.samples : 0})   // full chunks and what is left
+    for (const int form : {GRAD_IMAGE1_STORING, GRAD_IMAGE2_STORED})
+      if (n > 0) grad_parts(form, n);
   float* const parts = take(part);
   for (int l = 0; l < py.levels; ++l) p.w[l].part = parts;
   p.bytes = off;
+  for (int l = 0; l < py.levels; ++l) p.w[l].stored = reinterpret_cast<uint8_t*>(take(p.samples * grad_stored_bytes(py.d[l], n1p) / sizeof(float)));
+  p.stored_bytes = off - p.bytes;
   return p;
 }
 
@@ -1661,7 +1718,9 @@ size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int3
                                               int32_t backward) {
   Pyramid py;
   if (check_pyramid(shape, H2, W2, levels, &py) != SFB_OK) return 0;
-  return backward != 0 ? carve_pyramid_backward(py, nullptr).bytes : carve_pyramid_forward(py, nullptr).bytes;
+  if (backward == 0) return carve_pyramid_forward(py, nullptr).bytes;
+  const PyramidBackward pb = carve_pyramid_backward(py, nullptr);
+  return pb.bytes + pb.stored_bytes;
 }
 
 int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
@@ -1830,27 +1889,38 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
   }
   SFB_CUDA(timed(KID_PACK, pack_launches(groups.count, d0.B), st, [&] { return launch_pack_interleaved_cf(groups, d0.B, N1, w[0].n1p, st); }));
   SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_channel_major_cf(copies, 1 + levels, d0.B, d0.C, op16, st); }));
-  for (const int image2_major : {0, 1}) {
-    GradArgs a[MAX_FUSED_LEVELS];
-    GradMaps maps;
-    TileSplit split[MAX_FUSED_LEVELS];
-    grad_split_levels(py.d, levels, image2_major, split);
-    float* part = w[0].part;
-    int part0 = -1, launches = 1;
-    for (int l = 0; l < levels; ++l) {
-      SFB_TRY(grad_arguments(py.d[l], w[l], op16, GRAD_FUSED, 4 * Q, image2_major, image2_major ? gfmap2[l] : gfmap1, 1, scale1, &a[l],
-                             &maps.y[l], &maps.xu[l], &maps.xv[l]));
-      a[l].whole_tiles = split[l].whole_tiles;
-      a[l].pieces = split[l].pieces;
-      a[l].parts = split[l].parts;
-      a[l].part0 = part0;
-      a[l].part = part;
-      if (image2_major) part += split[l].part_floats;
-      else part0 += split[l].pieces;
-      if (a[l].parts > 0) launches = 2;
-      a[l] = with_wait_settings(a[l]);
+  const int samples = op16 != 0 && workspace_bytes >= pb.bytes + pb.stored_bytes ? pb.samples : 0;   // as in run_grad_pair
+  for (int b0 = 0; b0 < d0.B; b0 += samples > 0 ? samples : d0.B) {
+    for (const int form : {samples > 0 ? GRAD_IMAGE1_STORING : GRAD_IMAGE1, samples > 0 ? GRAD_IMAGE2_STORED : GRAD_IMAGE2}) {
+      const bool image2_major = grad_is_image2(form);
+      GradArgs a[MAX_FUSED_LEVELS];
+      GradMaps maps;
+      TileSplit split[MAX_FUSED_LEVELS];
+      Dims d[MAX_FUSED_LEVELS];
+      for (int l = 0; l < levels; ++l) {
+        d[l] = py.d[l];
+        if (samples > 0) d[l].B = std::min(samples, d0.B - b0);
+      }
+      grad_split_levels(d, levels, form, split);
+      float* part = w[0].part;
+      int part0 = -1, launches = 1;
+      for (int l = 0; l < levels; ++l) {
+        SFB_TRY(grad_arguments(py.d[l], w[l], op16, GRAD_FUSED, 4 * Q, form, image2_major ? gfmap2[l] : gfmap1, 1, scale1, &a[l], &maps.y[l],
+                               &maps.xu[l], &maps.xv[l]));
+        a[l].d = d[l];
+        a[l].b0 = b0;
+        a[l].whole_tiles = split[l].whole_tiles;
+        a[l].pieces = split[l].pieces;
+        a[l].parts = split[l].parts;
+        a[l].part0 = part0;
+        a[l].part = part;
+        if (image2_major) part += split[l].part_floats;
+        else part0 += split[l].pieces;
+        if (a[l].parts > 0) launches = 2;
+        a[l] = with_wait_settings(a[l]);
+      }
+      SFB_CUDA(timed(KID_GRAD_FUSED_IMG1 + (image2_major ? 1 : 0), launches, st, [&] { return launch_grad_gemm(a, levels, maps, st); }));
     }
-    SFB_CUDA(timed(KID_GRAD_FUSED_IMG1 + image2_major, launches, st, [&] { return launch_grad_gemm(a, levels, maps, st); }));
   }
   return SFB_OK;
 }

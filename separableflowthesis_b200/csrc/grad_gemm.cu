@@ -1,5 +1,5 @@
 // Gradient GEMMs of the backward ops:  gF1 = G * F2  and  gF2 = G^T * F1,  where
-// G = dLoss/dS (N1 x N2 per sample) is never stored: each block of it, 128 rows x 64 (image-1-major) or 32 (image-2-major)
+// G = dLoss/dS (N1 x N2 per sample) is made block by block: each, 128 rows x 64 (image-1-major) or 32 (image-2-major)
 // K-values, is generated by CUDA cores as the A operand of tcgen05.mma, while TMA streams the matching block of the other image's
 // features as the B operand.  The 128 x C output tile accumulates in TMEM over the whole K sweep and is
 // written once, so the result is deterministic (no atomics), unlike the reference's atomicAdd scatter
@@ -13,7 +13,17 @@
 //   image2_major = 1 : rows = an 8 x 16 block of image-2 pixels, K = 32 consecutive image-1 pixels,
 //                      output gF2.  A generator thread owns one K column (pixel), so the blocks are written to
 //                      shared memory, swizzled, K-major (TF32) or MN-major (16-bit).
-// B operand, both forms: K-major, like the operands of the correlation sweeps: TMA boxes of 32*ceil(C/32) channel
+//   With 16-bit operands G is generated once.  It costs the CUDA cores several times what its multiply-adds cost the tensor core, and the
+//   image-2-major generator, which shares no operand across a block, is the dearer one:
+//   storing          : image-1-major as above; the blocks also go to shared memory, from where one bulk copy per block takes them
+//                      to memory (16 KB per 128 x 64 values, beside some 1900 cycles of generating them).
+//   stored           : rows = 256 image-2 pixels (four blocks of 4 x 16, two accumulators), K = 64 image-1 pixels.  A block is 128-byte
+//                      rows of 64 image-2 pixels, MN-major, and is loaded as it lies in memory.  A plain GEMM: bound by the HBM
+//                      that G comes from, next to the tensor core.  With tiles of 128 rows it would read 1.5 times as much of image 1
+//                      through L2 per multiply-add as it gives the tensor core time for.
+//   G generated twice and once (the pair, us): 8 x 135 x 240 with four channels 17.6 ms and 12.9, 8 x 47 x 156 with two 782 and
+//   630 (BF16); the rule is grad_hands_over in c_abi.cu.
+// B operand, all forms: K-major, like the operands of the correlation sweeps: TMA boxes of 32*ceil(C/32) channel
 // rows x the K-values of a block from channel-major copies of the rounded features (image 1: (C, pixels); image 2: (C, column
 // blocks of 16, rows, 16), so that the 4 rows x 16 columns of a K block are 64 consecutive values).  The MN-major
 // form (pixel-major features) issues about 1.4x slower per tcgen05.mma and was dropped.
@@ -39,7 +49,7 @@
 //
 // Warp roles: warp 0 feature (B operand) producer, warp 1 TMEM allocation + MMA issue, warps 2..9 generate G
 // and, at the end, drain the accumulator (two warps per TMEM lane quarter, alternating 16-column chunks),
-// warp 10 producer of the XU / XV blocks.
+// warp 10 producer of the XU / XV blocks; storing: warp 11 copies the blocks to memory.
 #include <cuda_bf16.h>
 
 #include "kernels.h"
@@ -48,7 +58,7 @@
 namespace sfb {
 
 constexpr int GG_GEN_WARPS = 8;
-constexpr int GG_THREADS = (3 + GG_GEN_WARPS) * 32;
+template <int FORM> __host__ __device__ constexpr int gg_threads() { return (3 + GG_GEN_WARPS + (FORM == GRAD_IMAGE1_STORING ? 1 : 0)) * 32; }
 constexpr int GG_VH = GG_VT / (GG_GEN_WARPS / 4);          // columns of one image-1-major generator thread
 constexpr uint32_t GG_YBLOCK_BYTES = KBLK * 128;           // 4 KB: 128 bytes of K-values of 32 channel rows
 constexpr uint32_t GG_A_MBLOCK = GG_KJ * 128;              // image-2-major 16-bit A block: 64 rows x 32 K-values
@@ -66,26 +76,34 @@ constexpr uint32_t GG_ACC_COLS = 256;                      // accumulator column
 //        of the block to arrive
 // The image-2-major form's two generator groups hold two operand blocks at a time and a TMA load takes about as long
 // as one block's computation: with fewer than four (pixel, u) stages the generators wait for their operands.
-template <int Q, int I2MAJOR> struct GradCfg;
-template <> struct GradCfg<1, 0> { static constexpr int NY = 6, NG = 4, NXU = 4, NXV = 1; };
-template <> struct GradCfg<2, 0> { static constexpr int NY = 5, NG = 4, NXU = 4, NXV = 1; };
-template <> struct GradCfg<3, 0> { static constexpr int NY = 4, NG = 4, NXU = 4, NXV = 1; };
-template <> struct GradCfg<1, 1> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
-template <> struct GradCfg<2, 1> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
-template <> struct GradCfg<3, 1> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
-template <int I2MAJOR> __host__ __device__ constexpr uint32_t gg_tmem_cols() { return I2MAJOR ? 256u : 512u; }
+// The storing form gives a ring of three blocks on their way to memory what it takes from the others; the stored form has one ring,
+// a feature block and the four blocks of G that go with it to a stage.
+template <int Q, int FORM> struct GradCfg;
+template <> struct GradCfg<1, GRAD_IMAGE1> { static constexpr int NY = 6, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<2, GRAD_IMAGE1> { static constexpr int NY = 5, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<3, GRAD_IMAGE1> { static constexpr int NY = 4, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<1, GRAD_IMAGE1_STORING> { static constexpr int NY = 4, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<2, GRAD_IMAGE1_STORING> { static constexpr int NY = 3, NG = 4, NXU = 4, NXV = 1; };
+template <> struct GradCfg<3, GRAD_IMAGE1_STORING> { static constexpr int NY = 3, NG = 4, NXU = 3, NXV = 1; };
+template <int Q> struct GradCfg<Q, GRAD_IMAGE2> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
+template <int Q> struct GradCfg<Q, GRAD_IMAGE2_STORED> { static constexpr int NY = 3, NG = 3, NXU = 1, NXV = 1; };
+constexpr int GG_NST = 3;                                  // blocks on their way to memory
+constexpr uint32_t GG_SBLOCK_BYTES = GG_SJ * 128;          // stored form: 64 pixels of one block of G
+template <int FORM> __host__ __device__ constexpr uint32_t gg_tmem_cols() { return FORM == GRAD_IMAGE2 ? 256u : 512u; }
 
-template <int Q, int I2MAJOR>
+template <int Q, int FORM>
 struct GradSmem {
-  using Cfg = GradCfg<Q, I2MAJOR>;
-  static constexpr int AT = I2MAJOR ? 0 : 1;   // A blocks in tensor memory
-  static_assert(GG_ACC_COLS + (AT ? Cfg::NG * GG_KJ1 : 0) <= gg_tmem_cols<I2MAJOR>(), "A stages exceed TMEM");
+  using Cfg = GradCfg<Q, FORM>;
+  static constexpr bool STORING = FORM == GRAD_IMAGE1_STORING, STORED = FORM == GRAD_IMAGE2_STORED;
+  static constexpr bool AT = FORM == GRAD_IMAGE1 || STORING;   // A blocks in tensor memory
+  static_assert(GG_ACC_COLS + (AT ? Cfg::NG * GG_KJ1 : 0) <= gg_tmem_cols<FORM>(), "A stages exceed TMEM");
   // one operand block: [displacement][group of 4 slots][pixel][4]; image-1-major 4 x Q x 128, image-2-major 8 x Q x 32
-  static constexpr int XU_FLOATS = (I2MAJOR ? GG_ROW_UT * GG_KJ : GG_UT * TILE_M) * Q * 4;
-  static constexpr int XV_FLOATS = I2MAJOR ? GG_ROW_VT * GG_KJ * Q * 4 : 4;  // image-1-major keeps XV in registers
+  static constexpr int XU_FLOATS = STORED ? 4 : (AT ? GG_UT * TILE_M : GG_ROW_UT * GG_KJ) * Q * 4;
+  static constexpr int XV_FLOATS = FORM == GRAD_IMAGE2 ? GG_ROW_VT * GG_KJ * Q * 4 : 4;  // image-1-major keeps XV in registers
   float y[Cfg::NY][MAX_KB * GG_YBLOCK_BYTES / 4];  // feature stages [channel][K-values], K-major, swizzled
-  float g[AT ? 1 : Cfg::NG][AT ? 32 : TILE_M * GG_KJ];  // generated A blocks (image-2-major form), 128B swizzle, K-major (TF32)
-                                                        // or MN-major (16-bit)
+  // A blocks in shared memory, 128B swizzle: generated ones, K-major (TF32) or MN-major (16-bit); stored ones, MN-major
+  float g[AT ? 1 : Cfg::NG][AT ? 32 : (STORED ? GG_SM * GG_SBLOCK_BYTES / 4 : TILE_M * GG_KJ)];
+  uint8_t st[STORING ? GG_NST : 1][STORING ? TILE_M * 128 : 128];   // blocks on their way to memory
   float xu[Cfg::NXU][XU_FLOATS];
   float xv[Cfg::NXV][XV_FLOATS];
   uint64_t y_full[Cfg::NY];
@@ -96,6 +114,8 @@ struct GradSmem {
   uint64_t xu_empty[Cfg::NXU];
   uint64_t xv_full[Cfg::NXV];
   uint64_t xv_empty[Cfg::NXV];
+  uint64_t st_full[GG_NST];
+  uint64_t st_empty[GG_NST];
   uint64_t acc_full;
   uint32_t tmem_base;
   WaitCtl ctl;
@@ -107,7 +127,8 @@ struct GradSched {
   int tail, piece;   // tail tile this CTA has a piece of (-1: a whole tile) and which piece
   int m0;            // image-1-major: first pixel of the row tile
   int u0, v0;        // image-2-major: origin of the 8 x 16 row tile
-  int n_ub2;         // image-1-major: number of 4-row blocks along u
+  int kb;            // over a stored G: the first of the tile's blocks of 4 x 16 (of 128 rows, once they are drained)
+  int n_ub2;         // number of 4-row blocks along u
   int h2p;           // image-1-major: rows of the column-blocked channel-major copy of image 2 (H2 rounded up to a multiple of 4)
 };
 
@@ -170,9 +191,10 @@ __device__ __forceinline__ void g_products(const Slots<Q>& xu, const Slots<Q> (&
 // values with the scalar multiply-adds; 8 x 135 x 240: 8.4 -> 7.3 ms, 8 x 47 x 156: 436 -> 346 us).
 // The (pixel, v) slots stay in registers across the inner sweep over u; the (pixel, u) slots of each block
 // arrive in shared memory by TMA.  The finished values go to this thread's TMEM lane (A operand in tensor memory).
-template <int MODE, int Q, int BF16>
-__device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const GradSched& sc, int warp, int gw, int lane) {
-  using Cfg = GradCfg<Q, 0>;
+template <int MODE, int Q, int BF16, int FORM>
+__device__ void generator_image1(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSched& sc, int warp, int gw, int lane) {
+  using Cfg = GradCfg<Q, FORM>;
+  constexpr bool STORING = FORM == GRAD_IMAGE1_STORING;
   const int W2 = a.d.W2;
   const size_t group_stride = (size_t)a.n1p * 4, row_stride = group_stride * Q;
   const int pl = (warp & 3) * 32 + lane, vh = gw >> 2;
@@ -216,6 +238,9 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
     }
     if (!mbar_wait_warp(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     tc_fence_after();  // the MMAs that read this stage's TMEM columns have completed
+    if constexpr (STORING) {
+      if (!mbar_wait_warp(&sm.st_empty[t % GG_NST], ((t / GG_NST) & 1u) ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+    }
     if constexpr (BF16) {
 #pragma unroll
       for (int ul = 0; ul < GG_UT; ++ul) {
@@ -224,6 +249,10 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
         for (int j = 0; j < GG_VH / 2; ++j)
           h[j] = BF16 == OP16_FP16 ? pack_fp16x2(g[ul][2 * j], g[ul][2 * j + 1]) : pack_bf16x2(g[ul][2 * j], g[ul][2 * j + 1]);
         tmem_st4(ta0 + s * A_COLS + ul * (GG_VT / 2), h);
+        // eight values = chunk 2 * ul + vh of the pixel's row; eight lanes' chunks lie in different banks
+        if constexpr (STORING)
+          *reinterpret_cast<uint4*>(sm.st[t % GG_NST] + pl * 128 + ((((uint32_t)ul * 2 + vh) ^ ((uint32_t)pl & 7u)) << 4)) =
+              make_uint4(h[0], h[1], h[2], h[3]);
       }
     } else {
 #pragma unroll
@@ -231,9 +260,15 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
     }
     tmem_st_wait();
     tc_fence_before();  // stores complete and ordered before the tensor core's reads, which follow the arrive
+    if constexpr (STORING) fence_proxy_async_smem();   // ... and before the bulk copy's; the operand stage has been read, too
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.g_full[s]);
-    hand_back_stage(&sm.xu_empty[so], lane);
+    if constexpr (STORING) {
+      if (lane == 0) mbar_arrive(&sm.st_full[t % GG_NST]);
+      if (lane == 0) mbar_arrive(&sm.xu_empty[so]);
+    } else {
+      hand_back_stage(&sm.xu_empty[so], lane);
+    }
     if (++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
   }
 }
@@ -244,8 +279,8 @@ __device__ void generator_image1(GradSmem<Q, 0>& sm, const GradArgs& a, const Gr
 // which shared memory serves as one broadcast, so a warp's loads of those slots touch half as many bytes as with
 // one pixel per lane.
 template <int MODE, int Q, int BF16>
-__device__ void generator_image2(GradSmem<Q, 1>& sm, const GradArgs& a, const GradSched& sc, int gw, int lane) {
-  using Cfg = GradCfg<Q, 1>;
+__device__ void generator_image2(GradSmem<Q, GRAD_IMAGE2>& sm, const GradArgs& a, const GradSched& sc, int gw, int lane) {
+  using Cfg = GradCfg<Q, GRAD_IMAGE2>;
   constexpr int VQ = GG_ROW_VT / 4;  // columns per thread
   const int group = gw >> 2, sub = gw & 3;
   const int pl = (sub >> 1) * 16 + (lane & 15);          // K column of this thread
@@ -327,37 +362,51 @@ __device__ void generator_image2(GradSmem<Q, 1>& sm, const GradArgs& a, const Gr
 // Image-1-major: 128 bytes of a row, i.e. the 64 K-values of a block (16-bit) or half of them; image 2 is stored in column
 // blocks of 16 with a multiple of four rows, so block (vb, ub2) (4 rows x 16 columns) is 64 consecutive values.
 // Image-2-major: the 32 pixels of a block (64 bytes of 16-bit values).
-template <int I2MAJOR, int BF16> __device__ constexpr int y_stages_per_block() { return !I2MAJOR && !BF16 ? 2 : 1; }
-template <int Q, int I2MAJOR, int BF16>
-__device__ void feature_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc,
+// Over a stored G: the 64 pixels of a block and, with them, four blocks of G.
+template <int FORM, int BF16> __device__ constexpr int y_stages_per_block() { return !grad_is_image2(FORM) && !BF16 ? 2 : 1; }
+template <int Q, int FORM, int BF16>
+__device__ void feature_producer(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSched& sc,
                                  const CUtensorMap* tm_y) {
-  using Cfg = GradCfg<Q, I2MAJOR>;
-  constexpr int PER = y_stages_per_block<I2MAJOR, BF16>();
+  using Cfg = GradCfg<Q, FORM>;
+  constexpr int PER = y_stages_per_block<FORM, BF16>();
   int vb = 0, ub2 = 0;
-  if (I2MAJOR == 0) { vb = sc.t0 / sc.n_ub2; ub2 = sc.t0 - vb * sc.n_ub2; }
+  if (!grad_is_image2(FORM)) { vb = sc.t0 / sc.n_ub2; ub2 = sc.t0 - vb * sc.n_ub2; }
+  const int n_kb = sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT);
   uint32_t s = 0, ph = 0;
   for (int t = 0; t < sc.n_blocks; ++t) {
 #pragma unroll
     for (int h = 0; h < PER; ++h) {
       if (!mbar_wait(&sm.y_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
-      mbar_expect_tx(&sm.y_full[s], sc.nkb * (I2MAJOR && BF16 ? GG_YBLOCK_BYTES / 2 : GG_YBLOCK_BYTES));
-      if (I2MAJOR == 0)
-        tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (vb * sc.h2p + ub2 * GG_UT) * GG_VT + h * KBLK, 0, sc.b);
-      else
-        tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (sc.t0 + t) * GG_KJ, 0, sc.b);
+      if constexpr (FORM == GRAD_IMAGE2_STORED) {
+        mbar_expect_tx(&sm.y_full[s], sc.nkb * GG_YBLOCK_BYTES + GG_SM * GG_SBLOCK_BYTES);
+        tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (sc.t0 + t) * GG_SJ, 0, sc.b);
+#pragma unroll
+        for (int i = 0; i < GG_SM; ++i) {   // (rows past the last block are not stored: they may hold any)
+          const size_t kb = (size_t)(sc.b - a.b0) * n_kb + min(sc.kb + i, n_kb - 1);
+          bulk_load(reinterpret_cast<uint8_t*>(sm.g[s]) + i * GG_SBLOCK_BYTES, a.stored + (kb * a.n1p + (sc.t0 + t) * GG_SJ) * 128, GG_SBLOCK_BYTES,
+                    &sm.y_full[s]);
+        }
+      } else {
+        mbar_expect_tx(&sm.y_full[s], sc.nkb * (FORM == GRAD_IMAGE2 && BF16 ? GG_YBLOCK_BYTES / 2 : GG_YBLOCK_BYTES));
+        if (!grad_is_image2(FORM))
+          tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (vb * sc.h2p + ub2 * GG_UT) * GG_VT + h * KBLK, 0, sc.b);
+        else
+          tma_load_3d(sm.y[s], tm_y, &sm.y_full[s], (sc.t0 + t) * GG_KJ, 0, sc.b);
+      }
       if (++s == Cfg::NY) { s = 0; ph ^= 1u; }
     }
-    if (I2MAJOR == 0 && ++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
+    if (!grad_is_image2(FORM) && ++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
   }
 }
 
 // Interleaved operand blocks.  Tensor maps are 4-D (4*n1p, Q, D, B); a box is (4*pixels, Q, displacements, 1)
 // with at most 64 pixels (256 floats) per box, so the image-1-major form copies its 128 pixels as two boxes.
-template <int Q, int I2MAJOR>
-__device__ void operand_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc,
+template <int Q, int FORM>
+__device__ void operand_producer(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSched& sc,
                                  const CUtensorMap* tm_xu, const CUtensorMap* tm_xv) {
-  using Cfg = GradCfg<Q, I2MAJOR>;
-  using Smem = GradSmem<Q, I2MAJOR>;
+  using Cfg = GradCfg<Q, FORM>;
+  using Smem = GradSmem<Q, FORM>;
+  constexpr int I2MAJOR = grad_is_image2(FORM) ? 1 : 0;
   int ub2 = I2MAJOR == 0 ? sc.t0 % sc.n_ub2 : 0;
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t su = t % Cfg::NXU, phu = (t / Cfg::NXU) & 1u;
@@ -377,17 +426,18 @@ __device__ void operand_producer(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, co
   }
 }
 
-template <int Q, int I2MAJOR, int BF16>
-__device__ void grad_mma(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc) {
-  using Cfg = GradCfg<Q, I2MAJOR>;
+template <int Q, int FORM, int BF16>
+__device__ void grad_mma(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSched& sc) {
+  using Cfg = GradCfg<Q, FORM>;
   // A: generated block, K-major: TMEM columns from 256 on (image-1-major; a 16-bit column holds two values) or shared memory
   // (image-2-major).  B: feature block [channels][K-values], K-major.  Rows of 128 bytes have the 128-byte swizzle (8-row
   // groups 1024 B apart); the 64-byte rows of 16-bit image-2-major blocks the 64-byte swizzle (512 B apart).  An instruction
   // takes K = 8 TF32 or 16 16-bit values: 8 TMEM columns / 32 bytes along a row of A, 32 bytes along a row of B.  The 16-bit
   // image-2-major A block is MN-major (generator_image2): 8-K groups 1024 B apart, two of them to an instruction.
-  const uint32_t idesc = BF16 ? make_idesc_op16(BF16, TILE_M, sc.nkb * KBLK, I2MAJOR != 0) : make_idesc_tf32(TILE_M, sc.nkb * KBLK, false, false);
-  constexpr int PER = y_stages_per_block<I2MAJOR, BF16>();
-  constexpr int NK = I2MAJOR && BF16 ? 2 : 4;   // instructions per feature stage
+  constexpr bool I2MAJOR = grad_is_image2(FORM);
+  const uint32_t idesc = BF16 ? make_idesc_op16(BF16, TILE_M, sc.nkb * KBLK, I2MAJOR) : make_idesc_tf32(TILE_M, sc.nkb * KBLK, false, false);
+  constexpr int PER = y_stages_per_block<FORM, BF16>();
+  constexpr int NK = FORM == GRAD_IMAGE2 && BF16 ? 2 : 4;   // instructions per feature stage
   constexpr uint32_t A_COLS = BF16 ? GG_KJ1 / 2 : GG_KJ1;
   uint32_t sy = 0, phy = 0;
   for (int t = 0; t < sc.n_blocks; ++t) {
@@ -395,16 +445,24 @@ __device__ void grad_mma(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Grad
 #pragma unroll
     for (int h = 0; h < PER; ++h) {
       if (!mbar_wait(&sm.y_full[sy], phy, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
-      if (h == 0 && !mbar_wait(&sm.g_full[sg], phg, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
+      if (FORM != GRAD_IMAGE2_STORED && h == 0 && !mbar_wait(&sm.g_full[sg], phg, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
       tc_fence_after();
-      const uint64_t bdesc = I2MAJOR && BF16 ? make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 512, 4)
-                                             : make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 1024);
-      if constexpr (I2MAJOR == 0) {
+      const uint64_t bdesc = FORM == GRAD_IMAGE2 && BF16 ? make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 512, 4)
+                                                         : make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 1024);
+      if constexpr (!I2MAJOR) {
         const uint32_t a_tmem = sm.tmem_base + GG_ACC_COLS + sg * A_COLS + h * 32;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
           if constexpr (BF16) umma_bf16_ts(sm.tmem_base, a_tmem + k * 8, desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
           else umma_tf32_ts(sm.tmem_base, a_tmem + k * 8, desc_advance(bdesc, k * 32), idesc, (t | h | k) != 0);
+        }
+      } else if constexpr (FORM == GRAD_IMAGE2_STORED) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {   // 128 rows = two blocks each
+          const uint64_t adesc = make_smem_desc_sw128(smem_u32(sm.g[sy]) + half * 2 * GG_SBLOCK_BYTES, GG_SBLOCK_BYTES, 1024);
+#pragma unroll
+          for (int k = 0; k < NK; ++k)
+            umma_bf16(sm.tmem_base + half * GG_ACC_COLS, desc_advance(adesc, k * 2048), desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
         }
       } else {
         const uint64_t adesc = make_smem_desc_sw128(smem_u32(sm.g[sg]), BF16 ? GG_A_MBLOCK : 16, 1024);
@@ -417,24 +475,47 @@ __device__ void grad_mma(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Grad
       umma_commit(&sm.y_empty[sy]);  // reusable once these MMAs have read it
       if (++sy == Cfg::NY) { sy = 0; phy ^= 1u; }
     }
-    umma_commit(&sm.g_empty[sg]);
+    if constexpr (FORM != GRAD_IMAGE2_STORED) umma_commit(&sm.g_empty[sg]);
   }
   umma_commit(&sm.acc_full);
 }
 
+// The storing form's blocks, from shared memory to their place in memory.  A thread of its own: as a duty of the MMA thread, which then
+// waits for a copy to have read its block before it issues the next block's multiply-adds, the copies cost a third of the launch.
+template <int Q>
+__device__ void block_storer(GradSmem<Q, GRAD_IMAGE1_STORING>& sm, const GradArgs& a, const GradSched& sc) {
+  // the tile's pixels in the first of its blocks, and bytes from one block to the next
+  const size_t step = (size_t)a.n1p * 128;
+  uint8_t* dst = a.stored + ((size_t)(sc.b - a.b0) * sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT) + sc.t0) * step + (size_t)sc.m0 * 128;
+  for (int t = 0; t < sc.n_blocks; ++t, dst += step) {
+    const uint32_t s = t % GG_NST, ph = (t / GG_NST) & 1u;
+    if (!mbar_wait(&sm.st_full[s], ph, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
+    bulk_store(dst, sm.st[s], TILE_M * 128);
+    bulk_wait_read<1>();   // the block before this one has been read
+    if (t > 0) mbar_arrive(&sm.st_empty[(t - 1) % GG_NST]);
+  }
+  bulk_wait_all();
+}
+
+
 // Where output row m of this CTA's tile lives (null: past the image); consecutive channels are cstride floats apart.
-template <int I2MAJOR>
+template <int FORM>
 __device__ float* grad_row(const GradArgs& a, const GradSched& sc, int m, size_t& cstride) {
   const int C = a.d.C;
   cstride = 1;
-  if (I2MAJOR == 0) {
+  if (!grad_is_image2(FORM)) {
     const int p = sc.m0 + m;
     if (p >= a.d.N1()) return nullptr;
     if (!a.out_cf) return a.out + ((size_t)sc.b * a.d.N1() + p) * C;
     cstride = (size_t)a.d.N1();
     return a.out + (size_t)sc.b * C * a.d.N1() + p;
   }
-  const int u = sc.u0 + m / GG_ROW_VT, v = sc.v0 + m % GG_ROW_VT;
+  int u = sc.u0 + m / GG_ROW_VT, v = sc.v0 + m % GG_ROW_VT;
+  if constexpr (FORM == GRAD_IMAGE2_STORED) {
+    const int kb = sc.kb + m / GG_KJ1, vb = kb / sc.n_ub2, r = m % GG_KJ1;
+    u = (kb - vb * sc.n_ub2) * GG_UT + r / GG_VT;
+    v = vb * GG_VT + r % GG_VT;   // a block past the last lies past the last column
+  }
   if (u >= a.d.H2 || v >= a.d.W2) return nullptr;
   if (!a.out_cf) return a.out + (((size_t)sc.b * a.d.H2 + u) * a.d.W2 + v) * C;
   cstride = (size_t)a.d.N2();
@@ -448,8 +529,9 @@ __device__ __forceinline__ float* grad_part(const GradArgs& a, int tail, int par
   return a.part + ((size_t)tail * a.parts + part) * a.d.C * TILE_M;
 }
 
-template <int Q, int I2MAJOR>
-__device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const GradSched& sc, int warp, int gw, int lane) {
+template <int Q, int FORM>
+__device__ void grad_drain(GradSmem<Q, FORM>& sm, const GradArgs& a, GradSched sc, int warp, int gw, int lane) {
+  constexpr bool STORED = FORM == GRAD_IMAGE2_STORED;
   const bool ok = mbar_wait(&sm.acc_full, 0, &sm.ctl, a.status, DEV_TIMEOUT_EPILOGUE);
   if (!__all_sync(0xffffffffu, ok)) return;
   tc_fence_after();
@@ -457,19 +539,21 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
   const int q = warp & 3;  // TMEM lane quarter this warp may read
   const int m = q * 32 + lane;
   size_t cstride;
-  float* dst = grad_row<I2MAJOR>(a, sc, m, cstride);
+  const int half = STORED ? gw >> 2 : 0;   // of the 256 rows: an accumulator each, drained by four warps
+  if (STORED) sc.kb += half * (TILE_M / GG_KJ1);
+  float* dst = grad_row<FORM>(a, sc, m, cstride);
   const bool channel_major = a.out_cf != 0;
   bool accumulate = a.accumulate != 0;
   if (a.part0 + sc.piece >= 0) {
-    if (dst != nullptr) dst = grad_part(a, sc.tail, a.part0 + sc.piece) + (channel_major ? m : m * C);
+    if (dst != nullptr) dst = grad_part(a, STORED ? sc.tail * 2 + half : sc.tail, a.part0 + sc.piece) + (channel_major ? m : m * C);
     cstride = TILE_M;
     accumulate = false;
   }
-  const uint32_t tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+  const uint32_t tbase = sm.tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * GG_ACC_COLS;
   const float osc = a.out_scale * (a.dev_scale != nullptr ? __ldg(a.dev_scale) : 1.f);
   // the two warps of a quarter take alternate 16-column chunks; C is a multiple of 4 and the
   // accumulator has 32*nkb >= C columns
-  for (int c0 = (gw >> 2) * 16; c0 < C; c0 += 16 * (GG_GEN_WARPS / 4)) {
+  for (int c0 = STORED ? 0 : (gw >> 2) * 16; c0 < C; c0 += STORED ? 16 : 16 * (GG_GEN_WARPS / 4)) {
     float s[16];
     tmem_ld16(tbase + c0, s);
     if (dst == nullptr) continue;
@@ -501,22 +585,31 @@ __device__ void grad_drain(GradSmem<Q, I2MAJOR>& sm, const GradArgs& a, const Gr
 }
 
 // Sample and origin of a row tile; returns the blocks of its K sweep.
-template <int I2MAJOR>
+template <int FORM>
 __device__ __forceinline__ int grad_tile(const GradArgs& a, int tile, GradSched& sc) {
-  sc.m0 = sc.u0 = sc.v0 = sc.n_ub2 = sc.h2p = 0;
-  if (I2MAJOR == 0) {
+  sc.m0 = sc.u0 = sc.v0 = sc.kb = 0;
+  sc.n_ub2 = (a.d.H2 + GG_UT - 1) / GG_UT;
+  sc.h2p = sc.n_ub2 * GG_UT;
+  if (!grad_is_image2(FORM)) {
     const int tiles = (a.d.N1() + TILE_M - 1) / TILE_M;
     sc.b = tile / tiles;
     sc.m0 = (tile - sc.b * tiles) * TILE_M;
-    sc.n_ub2 = (a.d.H2 + GG_UT - 1) / GG_UT;
-    sc.h2p = sc.n_ub2 * GG_UT;
+    sc.b += a.b0;
     return sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT);
+  }
+  if constexpr (FORM == GRAD_IMAGE2_STORED) {
+    const int tiles = (sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT) + GG_SM - 1) / GG_SM;
+    sc.b = tile / tiles;
+    sc.kb = (tile - sc.b * tiles) * GG_SM;
+    sc.b += a.b0;
+    return (a.d.N1() + GG_SJ - 1) / GG_SJ;
   }
   const int n_ub = (a.d.H2 + GG_ROW_UT - 1) / GG_ROW_UT, n_vb = (a.d.W2 + GG_ROW_VT - 1) / GG_ROW_VT;
   sc.b = tile / (n_ub * n_vb);
   const int r = tile - sc.b * (n_ub * n_vb);
   sc.u0 = (r / n_vb) * GG_ROW_UT;
   sc.v0 = (r % n_vb) * GG_ROW_VT;
+  sc.b += a.b0;
   return (a.d.N1() + GG_KJ - 1) / GG_KJ;
 }
 
@@ -538,7 +631,7 @@ __device__ __forceinline__ int grad_level(const int (&first)[LEVELS + 1], int bl
 // The parts of a tile in scratch added to the output, in their order, four values to a thread.  A kernel of its own: added up by
 // the CTA that finished a tile last, the 128 KB of every piece came through that one SM.
 constexpr int GG_FOLD_THREADS = 256;
-template <int I2MAJOR, int LEVELS>
+template <int FORM, int LEVELS>
 __global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const __grid_constant__ GradLaunch<LEVELS> launch) {
   const int level = grad_level<LEVELS>(launch.first_tail, blockIdx.y);
   const GradArgs& a = launch.a[level];
@@ -547,19 +640,22 @@ __global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const __grid
   const int i = blockIdx.x * GG_FOLD_THREADS + threadIdx.x;   // four neighbours of the parts' layout (grad_part)
   if (i >= C * (TILE_M / 4)) return;
   GradSched sc;
-  grad_tile<I2MAJOR>(a, a.whole_tiles + tail, sc);
+  constexpr bool STORED = FORM == GRAD_IMAGE2_STORED;   // tails are halves of a tile
+  grad_tile<FORM>(a, a.whole_tiles + (STORED ? tail / 2 : tail), sc);
+  if (STORED) sc.kb += tail % 2 * (TILE_M / GG_KJ1);
   size_t cstride;
   float* dst;
   int cnt = 4;
   if (a.out_cf) {   // channel-major: four rows, neighbours in the image (the ones that exist come first), of one channel
     const int c = i / (TILE_M / 4), m = i % (TILE_M / 4) * 4;
-    dst = grad_row<I2MAJOR>(a, sc, m, cstride);
+    dst = grad_row<FORM>(a, sc, m, cstride);
     if (dst == nullptr) return;
     dst += c * cstride;
-    cnt = min(4, I2MAJOR ? a.d.W2 - (sc.v0 + m % GG_ROW_VT) : a.d.N1() - (sc.m0 + m));
+    const int v0 = STORED ? (sc.kb + m / GG_KJ1) / sc.n_ub2 * GG_VT : sc.v0;   // (16 columns a row in either)
+    cnt = min(4, grad_is_image2(FORM) ? a.d.W2 - (v0 + m % GG_ROW_VT) : a.d.N1() - (sc.m0 + m));
   } else {          // pixel-major: four channels of a row
     const int m = i / (C / 4);
-    dst = grad_row<I2MAJOR>(a, sc, m, cstride);
+    dst = grad_row<FORM>(a, sc, m, cstride);
     if (dst == nullptr) return;
     dst += (i - m * (C / 4)) * 4;
   }
@@ -571,15 +667,15 @@ __global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const __grid
   store4(dst, sum, cnt);
 }
 
-template <int MODE, int Q, int I2MAJOR, int BF16, int LEVELS>
-__global__ void __launch_bounds__(GG_THREADS, 1)
+template <int MODE, int Q, int FORM, int BF16, int LEVELS>
+__global__ void __launch_bounds__(gg_threads<FORM>(), 1)
 grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status) {
   if (!cta_has_work(status)) return;
   const int level = grad_level<LEVELS>(launch.first_block, blockIdx.x);
   const GradArgs& a = launch.a[level];
   const CUtensorMap *const tm_y = &launch.y[level], *const tm_xu = &launch.xu[level], *const tm_xv = &launch.xv[level];
-  using Smem = GradSmem<Q, I2MAJOR>;
-  using Cfg = GradCfg<Q, I2MAJOR>;
+  using Smem = GradSmem<Q, FORM>;
+  using Cfg = GradCfg<Q, FORM>;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
@@ -597,7 +693,7 @@ grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status)
     sc.piece = r - sc.tail * a.pieces;
     tile = a.whole_tiles + sc.tail;
   }
-  const int all_blocks = grad_tile<I2MAJOR>(a, tile, sc);
+  const int all_blocks = grad_tile<FORM>(a, tile, sc);
   const int n_pieces = sc.tail >= 0 ? a.pieces : 1;
   {
     const int per = all_blocks / n_pieces, extra = all_blocks - per * n_pieces;  // the first `extra` pieces have one more
@@ -606,20 +702,21 @@ grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status)
   }
 
   if (threadIdx.x == 0) {
-    constexpr int gen_arrivals = I2MAJOR ? 4 : GG_GEN_WARPS;  // one arrival per warp that writes / reads a block
+    constexpr int gen_arrivals = FORM == GRAD_IMAGE2 ? 4 : GG_GEN_WARPS;  // one arrival per warp that writes / reads a block
     for (int s = 0; s < Cfg::NY; ++s) { mbar_init(&sm.y_full[s], 1); mbar_init(&sm.y_empty[s], 1); }
     for (int s = 0; s < Cfg::NG; ++s) { mbar_init(&sm.g_full[s], gen_arrivals); mbar_init(&sm.g_empty[s], 1); }
     for (int s = 0; s < Cfg::NXU; ++s) { mbar_init(&sm.xu_full[s], 1); mbar_init(&sm.xu_empty[s], gen_arrivals); }
     for (int s = 0; s < Cfg::NXV; ++s) { mbar_init(&sm.xv_full[s], 1); mbar_init(&sm.xv_empty[s], gen_arrivals); }
+    for (int s = 0; s < GG_NST; ++s) { mbar_init(&sm.st_full[s], gen_arrivals); mbar_init(&sm.st_empty[s], 1); }
     mbar_init(&sm.acc_full, 1);
     wait_ctl_init(&sm.ctl, a.wait_limit_ns);
     fence_barrier_init();
     prefetch_tensormap(tm_y);
-    prefetch_tensormap(tm_xu);
-    if (I2MAJOR) prefetch_tensormap(tm_xv);
+    if (FORM != GRAD_IMAGE2_STORED) prefetch_tensormap(tm_xu);
+    if (FORM == GRAD_IMAGE2) prefetch_tensormap(tm_xv);
   }
   if (warp == 1) {
-    tmem_alloc(&sm.tmem_base, gg_tmem_cols<I2MAJOR>());
+    tmem_alloc(&sm.tmem_base, gg_tmem_cols<FORM>());
     tmem_relinquish();
   }
   tc_fence_before();
@@ -627,19 +724,26 @@ grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status)
   tc_fence_after();
 
   if (warp == 0) {
-    if (lane == 0) feature_producer<Q, I2MAJOR, BF16>(sm, a, sc, tm_y);
+    if (lane == 0) feature_producer<Q, FORM, BF16>(sm, a, sc, tm_y);
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) grad_mma<Q, I2MAJOR, BF16>(sm, a, sc);
+    if (lane == 0) grad_mma<Q, FORM, BF16>(sm, a, sc);
     __syncwarp();
   } else if (warp == 2 + GG_GEN_WARPS) {
-    if (lane == 0) operand_producer<Q, I2MAJOR>(sm, a, sc, tm_xu, tm_xv);
+    if constexpr (FORM != GRAD_IMAGE2_STORED) {
+      if (lane == 0) operand_producer<Q, FORM>(sm, a, sc, tm_xu, tm_xv);
+    }
+    __syncwarp();
+  } else if (FORM == GRAD_IMAGE1_STORING && warp == 3 + GG_GEN_WARPS) {
+    if constexpr (FORM == GRAD_IMAGE1_STORING) {
+      if (lane == 0) block_storer<Q>(sm, a, sc);
+    }
     __syncwarp();
   } else {
     const int gw = warp - 2;
-    if constexpr (I2MAJOR == 0) generator_image1<MODE, Q, BF16>(sm, a, sc, warp, gw, lane);
-    else generator_image2<MODE, Q, BF16>(sm, a, sc, gw, lane);
-    grad_drain<Q, I2MAJOR>(sm, a, sc, warp, gw, lane);
+    if constexpr (!grad_is_image2(FORM)) generator_image1<MODE, Q, BF16, FORM>(sm, a, sc, warp, gw, lane);
+    else if constexpr (FORM == GRAD_IMAGE2) generator_image2<MODE, Q, BF16>(sm, a, sc, gw, lane);
+    grad_drain<Q, FORM>(sm, a, sc, warp, gw, lane);
   }
 
   tc_fence_before();
@@ -650,14 +754,28 @@ grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status)
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(sm.tmem_base, gg_tmem_cols<I2MAJOR>());
+    tmem_dealloc(sm.tmem_base, gg_tmem_cols<FORM>());
   }
 }
 
-static int grad_tiles(const Dims& d, int image2_major) {
-  return image2_major ? d.B * ((d.H2 + GG_ROW_UT - 1) / GG_ROW_UT) * ((d.W2 + GG_ROW_VT - 1) / GG_ROW_VT)
-                      : d.B * ((d.N1() + TILE_M - 1) / TILE_M);
+// Row tiles of a launch, and blocks of a tile's K sweep with the time of one in units of 32 generated K-values (a block of the stored
+// form's 256 rows takes about as long).
+static int grad_tiles(const Dims& d, int form) {
+  switch (form) {
+    case GRAD_IMAGE2: return d.B * ((d.H2 + GG_ROW_UT - 1) / GG_ROW_UT) * ((d.W2 + GG_ROW_VT - 1) / GG_ROW_VT);
+    case GRAD_IMAGE2_STORED: return d.B * ((((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT) + GG_SM - 1) / GG_SM);
+    default: return d.B * ((d.N1() + TILE_M - 1) / TILE_M);
+  }
 }
+static int grad_blocks(const Dims& d, int form, int* unit) {
+  *unit = grad_is_image2(form) ? 1 : GG_KJ1 / GG_KJ;
+  switch (form) {
+    case GRAD_IMAGE2: return (d.N1() + GG_KJ - 1) / GG_KJ;
+    case GRAD_IMAGE2_STORED: return (d.N1() + GG_SJ - 1) / GG_SJ;
+    default: return ((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT);
+  }
+}
+static int grad_tail_rows(int form) { return form == GRAD_IMAGE2_STORED ? 2 * TILE_M : TILE_M; }
 
 // How the tail tiles are cut, in units of the time of 32 K-values (about 0.6 us): a CTA costs about eight of prologue and drain,
 // the fold is a launch of 4 to 11 us.  Pieces must save a quarter of the tail (see sweep_split) and at least twelve units to be
@@ -665,11 +783,10 @@ static int grad_tiles(const Dims& d, int image2_major) {
 // 1 x 48 x 64: 46 and 25, 50 and 24; 1 x 55 x 128: 122 and 79, 133 and 81; 4 x 55 x 128: 255 and 209, 268 and 249;
 // 3 x 47 x 155: 266 and 177, 273 and 189; 8 x 47 x 156: 418 and 350, 472 and 407; 1 x 55 x 128 against 27 x 64: 40 and 33,
 // 125 and 30; 1 x 135 x 240 against 67 x 120: 303 whole, 565 and 308; 2 x 33 x 70 against 16 x 35: 20 whole, 40 and 18.
-TileSplit grad_split(const Dims& d, int image2_major) {
-  const int tiles = grad_tiles(d, image2_major), rest = tiles % SM_COUNT;
-  const int blocks = image2_major ? (d.N1() + GG_KJ - 1) / GG_KJ
-                                  : ((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT);
-  const int unit = image2_major ? 1 : GG_KJ1 / GG_KJ;   // of a block
+TileSplit grad_split(const Dims& d, int form) {
+  const int tiles = grad_tiles(d, form), rest = tiles % SM_COUNT;
+  int unit;
+  const int blocks = grad_blocks(d, form, &unit);
   TileSplit r{tiles, tiles, 1, 0, 0};
   if (rest == 0) return r;
   double best = 0, whole = 0;
@@ -682,7 +799,7 @@ TileSplit grad_split(const Dims& d, int image2_major) {
   if (r.pieces > 1) {
     r.whole_tiles = tiles - rest;
     r.parts = r.pieces - 1;
-    r.part_floats = (size_t)rest * (r.pieces - 1) * d.C * TILE_M;
+    r.part_floats = (size_t)rest * (r.pieces - 1) * d.C * grad_tail_rows(form);
   }
   return r;
 }
@@ -690,15 +807,15 @@ TileSplit grad_split(const Dims& d, int image2_major) {
 // How the tiles of a pyramid's levels are cut when they share a launch, in the same units: all tiles of a level alike, the first two
 // levels of the image-1-major form into pieces of their own, all levels of the image-2-major form, whose K sweeps are equally
 // long, into the same number.  The cut with the smallest makespan; nothing is cut where the tiles make more than a few waves.
-void grad_split_levels(const Dims* d, int levels, int image2_major, TileSplit* out) {
-  int tiles[MAX_FUSED_LEVELS], blocks[MAX_FUSED_LEVELS], all = 0;
+void grad_split_levels(const Dims* d, int levels, int form, TileSplit* out) {
+  const bool image2_major = grad_is_image2(form);
+  int tiles[MAX_FUSED_LEVELS], blocks[MAX_FUSED_LEVELS], all = 0, unit = 1;
   for (int l = 0; l < levels; ++l) {
-    tiles[l] = grad_tiles(d[l], image2_major);
-    blocks[l] = image2_major ? (d[l].N1() + GG_KJ - 1) / GG_KJ : ((d[l].H2 + GG_UT - 1) / GG_UT) * ((d[l].W2 + GG_VT - 1) / GG_VT);
+    tiles[l] = grad_tiles(d[l], form);
+    blocks[l] = grad_blocks(d[l], form, &unit);
     all += tiles[l];
     out[l] = TileSplit{tiles[l], tiles[l], 1, 0, 0};
   }
-  const int unit = image2_major ? 1 : GG_KJ1 / GG_KJ;   // of a block
   int cut[MAX_FUSED_LEVELS] = {1, 1, 1, 1};
   static_assert(MAX_FUSED_LEVELS == 4, "cut");
   if (all <= 4 * SM_COUNT) {
@@ -725,14 +842,14 @@ void grad_split_levels(const Dims* d, int levels, int image2_major, TileSplit* o
     out[l].whole_tiles = 0;
     out[l].pieces = cut[l];
     out[l].parts = image2_major ? cut[l] - 1 : parts;
-    out[l].part_floats = image2_major || l == 0 ? (size_t)tiles[l] * out[l].parts * d[l].C * TILE_M : 0;   // image 1: one array for all
+    out[l].part_floats = image2_major || l == 0 ? (size_t)tiles[l] * out[l].parts * d[l].C * grad_tail_rows(form) : 0;   // image 1: one array for all
   }
 }
 
-template <int MODE, int Q, int I2MAJOR, int BF16, int LEVELS>
+template <int MODE, int Q, int FORM, int BF16, int LEVELS>
 static cudaError_t launch_one(GradLaunch<LEVELS>& launch, int levels, cudaStream_t stream) {
-  auto kern = grad_gemm_kernel<MODE, Q, I2MAJOR, BF16, LEVELS>;
-  constexpr size_t smem_bytes = sizeof(GradSmem<Q, I2MAJOR>) + 1024;
+  auto kern = grad_gemm_kernel<MODE, Q, FORM, BF16, LEVELS>;
+  constexpr size_t smem_bytes = sizeof(GradSmem<Q, FORM>) + 1024;
   static_assert(smem_bytes <= 232448, "shared memory of one CTA");
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
@@ -745,22 +862,22 @@ static cudaError_t launch_one(GradLaunch<LEVELS>& launch, int levels, cudaStream
     launch.first_tail[l] = tails;
     if (l >= levels) continue;
     const GradArgs& a = launch.a[l];
-    const int cut = grad_tiles(a.d, I2MAJOR) - a.whole_tiles;
+    const int cut = grad_tiles(a.d, FORM) - a.whole_tiles;
     blocks += a.whole_tiles + cut * a.pieces;
-    if (a.parts > 0 && a.part0 < 0) tails += cut;   // the level whose piece 0 is in the output adds up the parts
+    if (a.parts > 0 && a.part0 < 0) tails += cut * grad_tail_rows(FORM) / TILE_M;   // the level whose piece 0 is in the output adds up the parts
   }
   launch.first_block[LEVELS] = blocks;
   launch.first_tail[LEVELS] = tails;
-  kern<<<blocks, GG_THREADS, smem_bytes, stream>>>(launch, launch.a[0].status);
+  kern<<<blocks, gg_threads<FORM>(), smem_bytes, stream>>>(launch, launch.a[0].status);
   if (tails > 0) {
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     const int items = launch.a[0].d.C * (TILE_M / 4);
-    grad_fold_kernel<I2MAJOR, LEVELS><<<dim3((items + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS, tails), GG_FOLD_THREADS, 0, stream>>>(launch);
+    grad_fold_kernel<FORM, LEVELS><<<dim3((items + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS, tails), GG_FOLD_THREADS, 0, stream>>>(launch);
   }
   return cudaGetLastError();
 }
 
-template <int MODE, int Q, int I2MAJOR, int BF16>
+template <int MODE, int Q, int FORM, int BF16>
 static cudaError_t launch_levels(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {
   auto fill = [&](auto& launch) {
     for (int l = 0; l < levels; ++l) {
@@ -774,22 +891,35 @@ static cudaError_t launch_levels(const GradArgs* a, int levels, const GradMaps& 
     if (levels > 1) {
       GradLaunch<MAX_FUSED_LEVELS> launch{};
       fill(launch);
-      return launch_one<MODE, Q, I2MAJOR, BF16>(launch, levels, stream);
+      return launch_one<MODE, Q, FORM, BF16>(launch, levels, stream);
     }
   }
   if (levels != 1) return cudaErrorInvalidValue;
   GradLaunch<1> launch{};
   fill(launch);
-  return launch_one<MODE, Q, I2MAJOR, BF16>(launch, 1, stream);
+  return launch_one<MODE, Q, FORM, BF16>(launch, 1, stream);
+}
+
+template <int MODE, int Q, int BF16>
+static cudaError_t launch_form(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {
+  switch (a->form) {
+    case GRAD_IMAGE1: return launch_levels<MODE, Q, GRAD_IMAGE1, BF16>(a, levels, maps, stream);
+    case GRAD_IMAGE2: return launch_levels<MODE, Q, GRAD_IMAGE2, BF16>(a, levels, maps, stream);
+    case GRAD_IMAGE1_STORING:
+      if constexpr (BF16 != 0) return launch_levels<MODE, Q, GRAD_IMAGE1_STORING, BF16>(a, levels, maps, stream);
+      break;
+    case GRAD_IMAGE2_STORED:   // whatever G is a sum of
+      if constexpr (BF16 != 0) return launch_levels<GRAD_FUSED, 1, GRAD_IMAGE2_STORED, BF16>(a, levels, maps, stream);
+      break;
+  }
+  return cudaErrorInvalidValue;
 }
 
 template <int MODE, int Q>
 static cudaError_t launch_major(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {
-  if (a->op16 == OP16_FP16)
-    return a->image2_major ? launch_levels<MODE, Q, 1, OP16_FP16>(a, levels, maps, stream) : launch_levels<MODE, Q, 0, OP16_FP16>(a, levels, maps, stream);
-  if (a->op16 == OP16_BF16)
-    return a->image2_major ? launch_levels<MODE, Q, 1, OP16_BF16>(a, levels, maps, stream) : launch_levels<MODE, Q, 0, OP16_BF16>(a, levels, maps, stream);
-  return a->image2_major ? launch_levels<MODE, Q, 1, 0>(a, levels, maps, stream) : launch_levels<MODE, Q, 0, 0>(a, levels, maps, stream);
+  if (a->op16 == OP16_FP16) return launch_form<MODE, Q, OP16_FP16>(a, levels, maps, stream);
+  if (a->op16 == OP16_BF16) return launch_form<MODE, Q, OP16_BF16>(a, levels, maps, stream);
+  return launch_form<MODE, Q, 0>(a, levels, maps, stream);
 }
 
 cudaError_t launch_grad_gemm(const GradArgs* a, int levels, const GradMaps& maps, cudaStream_t stream) {

@@ -52,6 +52,7 @@ constexpr int GG_ROW_VT = 16;
 constexpr int GG_UT = 4;      // a K block of the image-1-major gradient GEMM: 4 image-2 rows x 16 columns
 constexpr int GG_VT = 16;
 constexpr int GG_KJ = 32;     // and of the image-2-major one: 32 image-1 pixels
+constexpr int GG_SJ = 64, GG_SM = 4;  // over a stored G: 64 pixels, tiles of 4 blocks of 4 x 16 image-2 pixels
 constexpr int KC_MAX_PER_SWEEP = 4;  // attention channels handled by one compression sweep
 constexpr int MAX_FUSED_LEVELS = 4;  // levels of a pyramid that the kernels of a call take in one launch
 
@@ -62,6 +63,10 @@ enum : int { OP16_NONE = 0, OP16_BF16 = 1, OP16_FP16 = 2 };
 #endif
 enum SweepMode : int { SWEEP_MAXAVG = 0, SWEEP_MAXARGAVG = 1, SWEEP_COMPRESS = 2, SWEEP_DUMP = 3 };
 enum GradMode : int { GRAD_MAXAVG = 0, GRAD_COMPRESS = 1, GRAD_FUSED = 2 };
+// Forms of the gradient GEMM.  Rows are image-1 pixels (output gF1) or image-2 pixels (gF2); G is generated, or, with 16-bit operands,
+// generated once: the image-1-major form stores its blocks and the image-2-major form reads them back.
+enum GradForm : int { GRAD_IMAGE1 = 0, GRAD_IMAGE2 = 1, GRAD_IMAGE1_STORING = 2, GRAD_IMAGE2_STORED = 3 };
+__host__ __device__ constexpr bool grad_is_image2(int form) { return form == GRAD_IMAGE2 || form == GRAD_IMAGE2_STORED; }
 
 // A tensor indexed by (sample b, displacement d, slot, image-1 pixel p) with the pixel fastest:
 // element at base + b*sb + d*sd + slot*ss + p.  Two instances of this are used:
@@ -175,7 +180,7 @@ class BlockQueue {
 struct GradArgs {
   Dims d;
   int mode;
-  int image2_major;      // 0: rows = image-1 pixels, output gF1; 1: rows = image-2 pixels, output gF2
+  int form;              // GradForm
   int R4;                // slots per pixel in the interleaved operands: 4 or 8
   int n1p;               // padded pixel count of the interleaved operands
   int accumulate;        // 0: out = result, 1: out += result (later channel chunks of the compression op)
@@ -191,11 +196,22 @@ struct GradArgs {
   int whole_tiles, pieces;           // as in SweepArgs, here with pieces of the K sweep (TileSplit)
   int parts, part0;                  // parts of a cut tile in scratch; piece i is part0 + i of them (-1: the output)
   float* part;
+  int b0;                            // first sample of the launch, which does d.B of them
+  uint8_t* stored;                   // G of those samples (the storing and the stored form), grad_stored_bytes each
 };
-TileSplit grad_split(const Dims& d, int image2_major);
+// Stored G of a sample: [block of 4 image-2 rows x 16 columns, column blocks outermost][n1p image-1 pixels][64 16-bit values], the 16-byte
+// chunks of a pixel's 128 bytes in the order of the 128-byte swizzle (chunk index ^ pixel % 8), so that a run of pixels is an operand
+// as it lies there.
+inline size_t grad_stored_bytes(const Dims& d, int n1p) {
+  return (size_t)((d.H2 + GG_UT - 1) / GG_UT) * ((d.W2 + GG_VT - 1) / GG_VT) * n1p * (GG_UT * GG_VT * 2);
+}
+// Stored G of a launch at most: 4 GiB, a fortieth of the device's memory and enough for launches of several waves (two samples of
+// 135 x 240 on itself).  Larger batches take several launches; a sample beyond it generates G twice.
+constexpr size_t GRAD_STORED_LIMIT = (size_t)1 << 32;
+TileSplit grad_split(const Dims& d, int form);
 // The same for the levels of a pyramid that share a launch (same image 1).  Image-1-major: the tiles of all levels but the first go to
 // scratch as a whole, to be added up.
-void grad_split_levels(const Dims* d, int levels, int image2_major, TileSplit* out);
+void grad_split_levels(const Dims* d, int levels, int form, TileSplit* out);
 
 // Launchers, here and below: the returned error is taken off the runtime, so a caller must pass it on; dropping it does not
 // compile (unused results are errors in this build).
