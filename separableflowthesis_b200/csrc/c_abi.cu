@@ -538,12 +538,12 @@ cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& 
                  : launch_prepare(d, f.F1, f.F2, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales);
 }
 // Launches of the above: FP16 operands add the search for the magnitudes.
-int prepare_launches(const Workspace& w, bool fmaps, bool with_aux, int op16) {
+int prepare_launches(const Workspace& w, bool with_aux, int op16) {
   const bool copies = !op16 || w.F1h != nullptr;
-  return (copies ? (fmaps ? 1 : 2) : 0) + (with_aux ? 1 : 0) + (op16 == OP16_FP16 ? 1 : 0);
+  return (copies ? 1 : 0) + (with_aux ? 1 : 0) + (op16 == OP16_FP16 ? 1 : 0);
 }
 #define SFB_PREPARE(f, with_aux) \
-  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, (f).fmaps, with_aux, (f).op16), st, [&] { return prepare_operands(d, w, f, with_aux, st); }))
+  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, with_aux, (f).op16), st, [&] { return prepare_operands(d, w, f, with_aux, st); }))
 
 int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, int32_t* AM_u, int32_t* AM_v,
                        bool with_argmax, const sfb_shape* shape, void* ws, size_t ws_bytes, void* stream) {
@@ -575,16 +575,9 @@ int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(timed(KID_SWEEP_MAXAVG, contraction_launches(a), st, [&] { return launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st); }));
   // packed (displacement, slot, pixel) -> the reference's (pixel, channel, displacement) tensors
-  const int N1 = d.N1(), R = MAXAVG_SLOTS;
-  SFB_CUDA(timed(KID_PACK, with_argmax ? 4 : 2, st, [&] {
-    SFB_LAUNCH(launch_unpack(w.ou, MA_u, d.B, N1, w.n1p, 2, d.H2, R, 0, 1, 2, 0, st));
-    cudaError_t e = launch_unpack(w.ov, MA_v, d.B, N1, w.n1p, 2, d.W2, R, 0, 1, 2, 0, st);
-    if (with_argmax) {
-      SFB_LAUNCH(launch_unpack(w.ou, AM_u, d.B, N1, w.n1p, 1, d.H2, R, 2, 1, 1, 0, st));
-      e = launch_unpack(w.ov, AM_v, d.B, N1, w.n1p, 1, d.W2, R, 2, 1, 1, 0, st);
-    }
-    return e;
-  }));
+  const PatchJob out[4] = {{MA_u, w.ou, 2, d.H2, 2, 0, MAXAVG_SLOTS, 0}, {MA_v, w.ov, 2, d.W2, 2, 0, MAXAVG_SLOTS, 0},
+                           {AM_u, w.ou, 1, d.H2, 1, 0, MAXAVG_SLOTS, 2}, {AM_v, w.ov, 1, d.W2, 1, 0, MAXAVG_SLOTS, 2}};
+  SFB_CUDA(timed(KID_PACK, 1, st, [&] { return launch_unpack(out, with_argmax ? 4 : 2, d.B, d.N1(), w.n1p, st); }));
   return SFB_OK;
 }
 
@@ -675,18 +668,16 @@ int run_grad_pair(const Dims& d, const Workspace& w, const Features& feat, int m
   // 16-bit form when the call has 16-bit operands; with FP16 the callers have run grad_operand_scales and packed the
   // operands with those scales
   const int op16 = feat.op16;
-  const float* const s1 = op16 == OP16_FP16 ? w.scales + SCALE_F1 : nullptr;
-  const float* const s2 = op16 == OP16_FP16 ? w.scales + SCALE_F2 : nullptr;
   const int kid = mode == GRAD_MAXAVG ? KID_GRAD_MAXAVG_IMG1 : (mode == GRAD_COMPRESS ? KID_GRAD_COMPRESS_IMG1 : KID_GRAD_FUSED_IMG1);
   if (!accumulate) {  // later passes over further channel chunks reuse the copies of the first
-    SFB_CUDA(timed(KID_PREPARE, feat.fmaps ? 1 : 2, st, [&] {
-      if (feat.fmaps) {  // already channel-major
-        const MapCopy copies[2] = {f1_copy(d, w, feat), f2_copy(d, w, feat.F2, op16)};
-        return launch_channel_major_cf(copies, 2, d.B, d.C, op16, st);
+    SFB_CUDA(timed(KID_PREPARE, 1, st, [&] {
+      MapCopy copies[2] = {f1_copy(d, w, feat), f2_copy(d, w, feat.F2, op16)};
+      if (feat.fmaps) return launch_channel_major_cf(copies, 2, d.B, d.C, op16, st);   // already channel-major
+      if (!op16) {   // pixel-major features are rounded already
+        copies[0].src = w.F1r;
+        copies[1].src = w.F2r;
       }
-      SFB_LAUNCH(cudaMemsetAsync(w.F2t, 0, (size_t)d.B * f2t_per_sample(d, w) * (op16 ? 2 : sizeof(float)), st));
-      SFB_LAUNCH(launch_channel_major(op16 ? feat.F1 : w.F1r, w.F1t, d.B, 1, d.N1(), w.n1p, d.C, 0, op16, s1, st));
-      return launch_channel_major(op16 ? feat.F2 : w.F2r, w.F2t, d.B, d.H2, d.W2, w.h2p, d.C, 1, op16, s2, st);
+      return launch_channel_major(copies[0], copies[1], d.B, d.C, op16, st);
     }));
   }
   // 16-bit operands: G of as many samples as the workspace takes is generated and stored by one GEMM and read back by the other
@@ -768,6 +759,20 @@ int grad_operand_scales(const Workspace& w, int op16, std::initializer_list<Absm
 }
 const float* grad_slot_scales(const Workspace& w, int op16) { return op16 == OP16_FP16 ? w.scales : nullptr; }
 
+// Weights w_u (B,N1,K,W2) / w_v (B,N1,K,H2) into the packed inputs, and the packed sums into C_u (B,N1,K,H2) / C_v (B,N1,K,W2).
+int pack_weights(const Dims& d, const Workspace& w, const float* w_u, const float* w_v, cudaStream_t st) {
+  const int K = d.Kc;
+  const PatchJob in[2] = {{w_u, w.xv, K, d.W2, K, 0, K, 0}, {w_v, w.xu, K, d.H2, K, 0, K, 0}};
+  SFB_CUDA(timed(KID_PACK, 1, st, [&] { return launch_pack(in, 2, d.B, d.N1(), w.n1p, st); }));
+  return SFB_OK;
+}
+int unpack_sums(const Dims& d, const Workspace& w, float* C_u, float* C_v, cudaStream_t st) {
+  const int K = d.Kc;
+  const PatchJob out[2] = {{C_u, w.ou, K, d.H2, K, 0, K, 0}, {C_v, w.ov, K, d.W2, K, 0, K, 0}};
+  SFB_CUDA(timed(KID_PACK, 1, st, [&] { return launch_unpack(out, 2, d.B, d.N1(), w.n1p, st); }));
+  return SFB_OK;
+}
+
 // Attention gradients of the compression backward: gA_v[p,k,u] = sum_v S * gC_v[p,k,v] and
 // gA_u[p,k,v] = sum_u S * gC_u[p,k,u] -- the forward compression sweep with the upstream gradients in the
 // role of the weights (w_u = gC_v, w_v = gC_u).
@@ -775,18 +780,11 @@ int run_attention_grads(const Dims& d, const Workspace& w, const float* gC_u, co
                         float* gA_v, cudaStream_t st, int op16) {
   CUtensorMap tm_f1, tm_f2;
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, nullptr, &tm_f2, nullptr));
-  const int N1 = d.N1(), K = d.Kc;
-  SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    SFB_LAUNCH(launch_pack(gC_v, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st));
-    return launch_pack(gC_u, w.xu, d.B, N1, w.n1p, K, 0, K, d.H2, K, 0, 1, 0.f, st);
-  }));
+  const int K = d.Kc;
+  SFB_TRY(pack_weights(d, w, gC_v, gC_u, st));
   SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
                               0, 0, 1, packed_view(w.ou, d.H2, K, w.n1p), packed_view(w.ov, d.W2, K, w.n1p), w.n1p, st, op16, sweep_out_scale(w, op16)));
-  SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    SFB_LAUNCH(launch_unpack(w.ou, gA_v, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st));
-    return launch_unpack(w.ov, gA_u, d.B, N1, w.n1p, K, d.W2, K, 0, 1, K, 0, st);
-  }));
-  return SFB_OK;
+  return unpack_sums(d, w, gA_v, gA_u, st);
 }
 
 // ---- scratch that lives in the library image, for callers that must not allocate ----
@@ -868,8 +866,8 @@ int sfb_max_avg_forward_static(const float* F1, const float* F2, float* MA_u, fl
   a.status = w.status;
   set_sweep_split(a, w, MAXAVG_PART_SLOTS);
   SFB_CUDA(launch_sweep(with_wait_settings(a), tm_f1, tm_f2, tm_aux, st));
-  SFB_CUDA(launch_unpack(w.ou, MA_u, d.B, d.N1(), w.n1p, 2, d.H2, MAXAVG_SLOTS, 0, 1, 2, 0, st));
-  SFB_CUDA(launch_unpack(w.ov, MA_v, d.B, d.N1(), w.n1p, 2, d.W2, MAXAVG_SLOTS, 0, 1, 2, 0, st));
+  const PatchJob out[2] = {{MA_u, w.ou, 2, d.H2, 2, 0, MAXAVG_SLOTS, 0}, {MA_v, w.ov, 2, d.W2, 2, 0, MAXAVG_SLOTS, 0}};
+  SFB_CUDA(launch_unpack(out, 2, d.B, d.N1(), w.n1p, st));
   return SFB_OK;
 }
 
@@ -902,18 +900,11 @@ int sfb_compression_forward(const float* F1, const float* F2, const float* A_u, 
   SFB_TRY(map_sweep_operands(d, w, op16, &tm_f1, nullptr, &tm_f2, nullptr));
   const Features feat{F1, F2, false, 1.f, op16};
   SFB_PREPARE(feat, false);
-  const int N1 = d.N1(), K = d.Kc;
-  SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    SFB_LAUNCH(launch_pack(A_u, w.xv, d.B, N1, w.n1p, K, 0, K, d.W2, K, 0, 1, 0.f, st));  // w_u[k][v] = XV slot k
-    return launch_pack(A_v, w.xu, d.B, N1, w.n1p, K, 0, K, d.H2, K, 0, 1, 0.f, st);  // w_v[k][u] = XU slot k
-  }));
+  const int K = d.Kc;
+  SFB_TRY(pack_weights(d, w, A_u, A_v, st));   // w_u[k][v] = XV slot k, w_v[k][u] = XU slot k
   SFB_TRY(run_compress_sweeps(d, w, tm_f1, tm_f2, packed_view(w.xu, d.H2, K, w.n1p), packed_view(w.xv, d.W2, K, w.n1p),
                               0, 0, 1, packed_view(w.ou, d.H2, K, w.n1p), packed_view(w.ov, d.W2, K, w.n1p), w.n1p, st, op16, sweep_out_scale(w, op16)));
-  SFB_CUDA(timed(KID_PACK, 2, st, [&] {
-    SFB_LAUNCH(launch_unpack(w.ou, C_u, d.B, N1, w.n1p, K, d.H2, K, 0, 1, K, 0, st));
-    return launch_unpack(w.ov, C_v, d.B, N1, w.n1p, K, d.W2, K, 0, 1, K, 0, st);
-  }));
-  return SFB_OK;
+  return unpack_sums(d, w, C_u, C_v, st);
 }
 
 int sfb_max_argmax_avg_backward(const float* F1, const float* F2, const int32_t* AM_u, const int32_t* AM_v,
@@ -932,11 +923,13 @@ int sfb_max_argmax_avg_backward(const float* F1, const float* F2, const int32_t*
   SFB_PREPARE(feat, false);
   const size_t pix = (size_t)d.B * d.N1();
   SFB_TRY(grad_operand_scales(w, op16, {{gMA_u, pix * 2 * d.H2}, {gMA_v, pix * 2 * d.W2}}, {}, st));
-  SFB_CUDA(timed(KID_PACK, 2, st, [&] {
+  SFB_CUDA(timed(KID_PACK, pack_launches(2, d.B), st, [&] {
     SlotSources su, sv;
+    PackGroups groups{};
     maxavg_slot_sources(d, AM_u, AM_v, gMA_u, gMA_v, &su, &sv, grad_slot_scales(w, op16));
-    SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, d.N1(), w.n1p, d.H2, 4, 1, 0, st));
-    return launch_pack_interleaved(sv, w.gxv, d.B, d.N1(), w.n1p, d.W2, 4, 1, 0, st);
+    groups.add(su, w.gxu, d.H2, 4, 1, 0);
+    groups.add(sv, w.gxv, d.W2, 4, 1, 0);
+    return launch_pack_interleaved(groups, d.B, d.N1(), w.n1p, st);
   }));
   return run_grad_pair(d, w, feat, GRAD_MAXAVG, 4, 0, gF1, gF2, st);
 }
@@ -965,11 +958,13 @@ int sfb_compression_backward(const float* F1, const float* F2, const float* A_u,
   // gradient GEMMs, at most KC_MAX_PER_SWEEP channels per pass; later passes add to gF1 / gF2.
   for (int k0 = 0; k0 < K; k0 += KC_MAX_PER_SWEEP) {
     const int kc = chunk_channels(K - k0), R4 = grad_slots(kc);
-    SFB_CUDA(timed(KID_PACK, 2, st, [&] {
+    SFB_CUDA(timed(KID_PACK, pack_launches(R4 / 2, d.B), st, [&] {
       SlotSources su, sv;
+      PackGroups groups{};
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, grad_slot_scales(w, op16));
-      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st));
-      return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
+      groups.add(su, w.gxu, d.H2, R4, R4 / 4, 0);
+      groups.add(sv, w.gxv, d.W2, R4, R4 / 4, 0);
+      return launch_pack_interleaved(groups, d.B, N1, w.n1p, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, k0 > 0 ? 1 : 0, gF1, gF2, st));
   }
@@ -1008,24 +1003,28 @@ static int run_fused_feature_grads(const Dims& d, const Workspace& w, const Feat
   const float* const gs = grad_slot_scales(w, op16);
   {  // group 0 = max/avg slots, groups 1.. = the first (up to 4) compression channels; G is their sum
     const int kc = chunk_channels(K), Qc = grad_slots(kc) / 4, Q = 1 + Qc;
-    SFB_CUDA(timed(KID_PACK, 4, st, [&] {
+    SFB_CUDA(timed(KID_PACK, pack_launches(2 * Q, d.B), st, [&] {
       SlotSources su, sv;
+      PackGroups groups{};
       maxavg_slot_sources(d, AM_u, AM_v, gMA_u, gMA_v, &su, &sv, gs);
-      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4, Q, 0, st));
-      SFB_LAUNCH(launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4, Q, 0, st));
+      groups.add(su, w.gxu, d.H2, 4, Q, 0);
+      groups.add(sv, w.gxv, d.W2, 4, Q, 0);
       compress_slot_sources(K, 0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs);
-      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, 4 * Qc, Q, 1, st));
-      return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, 4 * Qc, Q, 1, st);
+      groups.add(su, w.gxu, d.H2, 4 * Qc, Q, 1);
+      groups.add(sv, w.gxv, d.W2, 4 * Qc, Q, 1);
+      return launch_pack_interleaved(groups, d.B, N1, w.n1p, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_FUSED, 4 * Q, 0, gF1, gF2, st));
   }
   for (int k0 = KC_MAX_PER_SWEEP; k0 < K; k0 += KC_MAX_PER_SWEEP) {  // remaining channels: compression form, accumulated
     const int kc = chunk_channels(K - k0), R4 = grad_slots(kc);
-    SFB_CUDA(timed(KID_PACK, 2, st, [&] {
+    SFB_CUDA(timed(KID_PACK, pack_launches(R4 / 2, d.B), st, [&] {
       SlotSources su, sv;
+      PackGroups groups{};
       compress_slot_sources(K, k0, kc, A_u, A_v, gC_u, gC_v, &su, &sv, gs);
-      SFB_LAUNCH(launch_pack_interleaved(su, w.gxu, d.B, N1, w.n1p, d.H2, R4, R4 / 4, 0, st));
-      return launch_pack_interleaved(sv, w.gxv, d.B, N1, w.n1p, d.W2, R4, R4 / 4, 0, st);
+      groups.add(su, w.gxu, d.H2, R4, R4 / 4, 0);
+      groups.add(sv, w.gxv, d.W2, R4, R4 / 4, 0);
+      return launch_pack_interleaved(groups, d.B, N1, w.n1p, st);
     }));
     SFB_TRY(run_grad_pair(d, w, feat, GRAD_COMPRESS, R4, 1, gF1, gF2, st));
   }
@@ -1682,7 +1681,7 @@ int prepare_pyramid(const Pyramid& py, const Workspace* w, const float* fmap1, c
   for (int l = 0; l < py.levels; ++l)
     out[l] = op16 ? LevelOperands{nullptr, nullptr, w[l].F2h, with_aux ? w[l].auxh : nullptr}
                   : LevelOperands{w[l].F2r, with_aux ? w[l].aux : nullptr, nullptr, nullptr};
-  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w[0], true, with_aux, op16), st, [&] {
+  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w[0], with_aux, op16), st, [&] {
     return launch_prepare_cf(py.d, py.levels, fmap1, fmap2, scale1, out, op16 ? nullptr : w[0].F1r, op16 ? w[0].F1h : nullptr, w[0].status,
                              st, op16, w[0].scales);
   }));

@@ -255,10 +255,8 @@ struct PackGroups {
 inline int pack_groups_per_launch(int B) { return std::max(1, std::min(MAX_PACK_GROUPS, 65535 / B)); }
 inline int pack_launches(int groups, int B) { return (groups + pack_groups_per_launch(B) - 1) / pack_groups_per_launch(B); }
 [[nodiscard]] cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream);
-// Writes R4 (4 or 8) slots = R4/4 groups starting at group q0 of dst (B, D, Qtot, n1p, 4); pixels N1 <= p < n1p
-// and slots without a source are zero.
-[[nodiscard]] cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
-                                    int Qtot, int q0, cudaStream_t stream);
+// The same from sources (B, N1, Ksrc, D).
+[[nodiscard]] cudaError_t launch_pack_interleaved(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream);
 
 // Workspace header: the status word, then (64 bytes in) the scale slots of the FP16 operand kind, SCALE_LEVEL for every level of the
 // call, all cleared by launch_prepare.  amax slots hold float bits (atomicMax), the others floats; every scale is a power of two.
@@ -303,19 +301,22 @@ struct MapCopy {
   const float* scale16;
 };
 [[nodiscard]] cudaError_t launch_channel_major_cf(const MapCopy* copies, int count, int B, int C, int op16, cudaStream_t stream);
-// Channel-major copy of a pixel-major feature array (B, rows*width, C), as FP32 (of rounded values) or (op16 != 0) as 16-bit
-// operands (FP16: times the device scalar *scale16); padding is not written.
+// Channel-major copies of pixel-major feature arrays (B, rows*width, C), as FP32 (of rounded values) or (op16 != 0) as 16-bit operands;
+// `scale` is not read.  Padding is zeroed.
 //   blocked = 0: dst (B, C, pitch) with pixel index row*width + x (rows = 1)
 //   blocked = 1: dst (B, C, ceil(width/16), pitch, 16), element (row, x) at ((x/16)*pitch + row)*16 + x%16
-[[nodiscard]] cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, int width, int pitch, int C,
-                                 int blocked, int op16, const float* scale16, cudaStream_t stream);
-// Pack: dst[b][d][r0 + k*rstride][p] = scale * src[b][p][ksrc0 + k][d] for k < K (raw 32-bit copy when
-// scale == 0), zero for N1 <= p < n1p.  src is (B, N1, Ksrc, D), dst is (B, D, R, n1p).
-[[nodiscard]] cudaError_t launch_pack(const void* src, float* dst, int B, int N1, int n1p, int Ksrc, int ksrc0, int K, int D,
-                        int R, int r0, int rstride, float scale, cudaStream_t stream);
-// Unpack: dst[b][p][kdst0 + k][d] = src[b][d][r0 + k*rstride][p] for k < K; dst is (B, N1, Kdst, D).
-[[nodiscard]] cudaError_t launch_unpack(const float* src, void* dst, int B, int N1, int n1p, int K, int D, int R, int r0,
-                          int rstride, int Kdst, int kdst0, cudaStream_t stream);
+[[nodiscard]] cudaError_t launch_channel_major(const MapCopy& c1, const MapCopy& c2, int B, int C, int op16, cudaStream_t stream);
+// Transposes between a tensor of the reference's layout, pixels (B, N1, Kpix, D), of which channels k0 .. k0 + K - 1, and a packed array
+// (B, D, R, n1p), of which slots r0 .. (32-bit values as they are).  Pack writes the packed array, zero for N1 <= p < n1p; unpack the
+// other.  All tensors of a call in one launch.
+constexpr int MAX_PATCH_JOBS = 4;
+struct PatchJob {
+  const void* pixels;
+  float* packed;
+  int K, D, Kpix, k0, R, r0;
+};
+[[nodiscard]] cudaError_t launch_pack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream);
+[[nodiscard]] cudaError_t launch_unpack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream);
 [[nodiscard]] cudaError_t launch_sweep(const SweepArgs& a, const CUtensorMap& tm_f1, const CUtensorMap& tm_f2,
                          const CUtensorMap& tm_aux, cudaStream_t stream);
 // The levels of a pyramid in one launch (same image 1, mode, channels and operand type).

@@ -127,21 +127,28 @@ cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int
   return cudaGetLastError();
 }
 
-// `outh` (optional): the same values as 16-bit operands of kind `op16` instead (BF16, or FP16 of the value times the
-// device scalar *scale16).
-__global__ void round_copy_kernel(const float4* __restrict__ in, float4* __restrict__ out, size_t n4,
-                                  uint2* __restrict__ outh, int op16, const float* __restrict__ scale16) {
+// Both images of a call: rounded to TF32 in `out`, or in `outh` as 16-bit operands of kind `op16` (BF16, or FP16 of the value times the
+// device scalar *scale16); the one that is not wanted is null.  grid (blocks, 2), block 256.
+struct RoundJob {
+  const float4* in;
+  float4* out;
+  uint2* outh;
+  const float* scale16;
+  size_t n4;
+};
+__global__ void round_copy_kernel(const RoundJob j1, const RoundJob j2, int op16) {
+  const RoundJob& j = blockIdx.y == 0 ? j1 : j2;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const float sc = (outh != nullptr && scale16 != nullptr) ? __ldg(scale16) : 1.f;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    float4 v = __ldg(in + i);
-    if (outh != nullptr) {
-      if (op16 == OP16_FP16) outh[i] = make_uint2(pack_fp16x2(v.x * sc, v.y * sc), pack_fp16x2(v.z * sc, v.w * sc));
-      else outh[i] = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+  const float sc = (j.outh != nullptr && j.scale16 != nullptr) ? __ldg(j.scale16) : 1.f;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < j.n4; i += stride) {
+    float4 v = __ldg(j.in + i);
+    if (j.outh != nullptr) {
+      if (op16 == OP16_FP16) j.outh[i] = make_uint2(pack_fp16x2(v.x * sc, v.y * sc), pack_fp16x2(v.z * sc, v.w * sc));
+      else j.outh[i] = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
     }
-    if (out != nullptr) {
+    if (j.out != nullptr) {
       v.x = round_tf32(v.x); v.y = round_tf32(v.y); v.z = round_tf32(v.z); v.w = round_tf32(v.w);
-      out[i] = v;
+      j.out[i] = v;
     }
   }
 }
@@ -288,102 +295,155 @@ f2_means_cf_kernel(const __grid_constant__ MeansJobs jobs, int C, int op16) {
 // Tiled transposes between the reference's per-pixel layout (B, N1, K, D) (displacement d fastest) and the
 // packed layout (B, D, R, n1p) (pixel fastest) the kernels use.  A block moves a patch of 128 pixels x 32
 // displacements through shared memory so that both sides are coalesced; every thread keeps 16 loads in flight,
-// and the displacement tiles are the fastest grid dimension so that blocks running together read neighbouring
-// 128-byte pieces of the same rows.  grid (ceil(D/32), n1p/128, B*K), block (32, 8).
+// and the displacement tiles are the fastest so that blocks running together read neighbouring
+// 128-byte pieces of the same rows.  One launch for all tensors of a call (a launch of a small one is mostly latency: the four outputs of
+// 2 x 48 x 64 took 31 us in four launches, 10 in one).
+// grid: ceil(D/32) * n1p/128 * B*K blocks per tensor, block (32, 8).
 constexpr int PACK_PX = 128;
-
-__global__ void pack_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int N1, int n1p, int Ksrc,
-                            int ksrc0, int K, int D, int R, int r0, int rstride, float scale) {
-  __shared__ uint32_t tile[PACK_PX][33];
-  const int b = blockIdx.z / K, k = blockIdx.z - b * K, d0 = blockIdx.x * 32, p0 = blockIdx.y * PACK_PX;
-  const int tx = threadIdx.x, ty = threadIdx.y;
+struct PatchJobs {
+  PatchJob j[MAX_PATCH_JOBS];
+  int first[MAX_PATCH_JOBS];   // blocks; tensors that do not exist start past the end of the grid
+};
+struct Patch {
+  int b, k, d0, p0;
+};
+__device__ __forceinline__ Patch patch_of(const PatchJobs& jobs, int n1p, int& job) {
+  job = 0;
 #pragma unroll
-  for (int j = ty; j < PACK_PX; j += 8) {
-    const int p = p0 + j, d = d0 + tx;
+  for (int i = 1; i < MAX_PATCH_JOBS; ++i) job = (int)blockIdx.x >= jobs.first[i] ? i : job;
+  const PatchJob& j = jobs.j[job];
+  const int r = blockIdx.x - jobs.first[job], nd = (j.D + 31) / 32, np = n1p / PACK_PX;
+  const int q = r / nd, z = q / np, b = z / j.K;
+  return Patch{b, z - b * j.K, (r - q * nd) * 32, (q - z * np) * PACK_PX};
+}
+
+__global__ void pack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
+  __shared__ uint32_t tile[PACK_PX][33];
+  int ji;
+  const Patch t = patch_of(jobs, n1p, ji);
+  const PatchJob& j = jobs.j[ji];
+  const int tx = threadIdx.x, ty = threadIdx.y, D = j.D;
+  const uint32_t* src = static_cast<const uint32_t*>(j.pixels) + (((size_t)t.b * N1 + t.p0) * j.Kpix + j.k0 + t.k) * D + t.d0 + tx;
+#pragma unroll
+  for (int i = ty; i < PACK_PX; i += 8) {
     uint32_t v = 0;
-    if (p < N1 && d < D) v = __ldg(src + (((size_t)b * N1 + p) * Ksrc + ksrc0 + k) * D + d);
-    tile[j][tx] = v;
+    if (t.p0 + i < N1 && t.d0 + tx < D) v = __ldg(src + (size_t)i * j.Kpix * D);
+    tile[i][tx] = v;
   }
   __syncthreads();
-  const int r = r0 + k * rstride;
+  uint32_t* dst = reinterpret_cast<uint32_t*>(j.packed) + (((size_t)t.b * D + t.d0) * j.R + j.r0 + t.k) * n1p + t.p0;
 #pragma unroll
   for (int i = ty; i < 32 * (PACK_PX / 32); i += 8) {
-    const int d = d0 + i / (PACK_PX / 32), p = (i % (PACK_PX / 32)) * 32 + tx;
-    if (d < D) {
-      uint32_t v = tile[p][i / (PACK_PX / 32)];
-      if (scale != 0.f) v = __float_as_uint(__uint_as_float(v) * scale);
-      dst[(((size_t)b * D + d) * R + r) * n1p + p0 + p] = v;
-    }
+    const int d = i / (PACK_PX / 32), p = (i % (PACK_PX / 32)) * 32 + tx;
+    if (t.d0 + d < D) dst[(size_t)d * j.R * n1p + p] = tile[p][d];
   }
 }
 
-__global__ void unpack_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int N1, int n1p, int K,
-                              int D, int R, int r0, int rstride, int Kdst, int kdst0) {
+__global__ void unpack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
   __shared__ uint32_t tile[PACK_PX][33];
-  const int b = blockIdx.z / K, k = blockIdx.z - b * K, d0 = blockIdx.x * 32, p0 = blockIdx.y * PACK_PX;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int r = r0 + k * rstride;
+  int ji;
+  const Patch t = patch_of(jobs, n1p, ji);
+  const PatchJob& j = jobs.j[ji];
+  const int tx = threadIdx.x, ty = threadIdx.y, D = j.D;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(j.packed) + (((size_t)t.b * D + t.d0) * j.R + j.r0 + t.k) * n1p + t.p0;
 #pragma unroll
   for (int i = ty; i < 32 * (PACK_PX / 32); i += 8) {
-    const int dl = i / (PACK_PX / 32), p = (i % (PACK_PX / 32)) * 32 + tx;
-    tile[p][dl] = (d0 + dl < D) ? __ldg(src + (((size_t)b * D + d0 + dl) * R + r) * n1p + p0 + p) : 0u;
+    const int d = i / (PACK_PX / 32), p = (i % (PACK_PX / 32)) * 32 + tx;
+    tile[p][d] = t.d0 + d < D ? __ldg(src + (size_t)d * j.R * n1p + p) : 0u;
   }
   __syncthreads();
+  uint32_t* dst = static_cast<uint32_t*>(const_cast<void*>(j.pixels)) + (((size_t)t.b * N1 + t.p0) * j.Kpix + j.k0 + t.k) * D + t.d0 + tx;
 #pragma unroll
-  for (int j = ty; j < PACK_PX; j += 8) {
-    const int p = p0 + j, d = d0 + tx;
-    if (p < N1 && d < D) dst[(((size_t)b * N1 + p) * Kdst + kdst0 + k) * D + d] = tile[j][tx];
-  }
+  for (int i = ty; i < PACK_PX; i += 8)
+    if (t.p0 + i < N1 && t.d0 + tx < D) dst[(size_t)i * j.Kpix * D] = tile[i][tx];
 }
 
-// Interleaved pack: every block transposes a 32-pixel x 32-displacement patch of each source through
-// shared memory, then writes, per displacement, the R4 slots of its 32 pixels as one contiguous run.
-template <int R4>
-__global__ void pack_interleaved_kernel(const SlotSources src, uint32_t* __restrict__ dst, int N1, int n1p, int D,
-                                        int Qtot, int q0) {
-  constexpr int RS = 32 * 33 + 32 / R4;  // slot stride chosen so that the interleaved read below is conflict-free
-  __shared__ uint32_t tile[R4 * RS];
-  const int b = blockIdx.z, d0 = blockIdx.x * 32, p0 = blockIdx.y * 32;  // displacement tiles fastest
+template <class Kernel>
+static cudaError_t launch_patches(Kernel kern, const PatchJob* job, int count, int B, int N1, int n1p, cudaStream_t stream) {
+  if (count < 1 || count > MAX_PATCH_JOBS) return cudaErrorInvalidValue;
+  PatchJobs jobs;
+  long long blocks = 0;
+  for (int i = 0; i < MAX_PATCH_JOBS; ++i) {
+    jobs.j[i] = job[i < count ? i : 0];
+    jobs.first[i] = i < count ? (int)blocks : INT_MAX;
+    if (i < count) blocks += (long long)((job[i].D + 31) / 32) * (n1p / PACK_PX) * B * job[i].K;
+    if (blocks > INT_MAX) return cudaErrorInvalidConfiguration;
+  }
+  kern<<<(unsigned)blocks, dim3(32, 8), 0, stream>>>(jobs, N1, n1p);
+  return cudaGetLastError();
+}
+cudaError_t launch_pack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream) {
+  return launch_patches(pack_kernel, jobs, count, B, N1, n1p, stream);
+}
+cudaError_t launch_unpack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream) {
+  return launch_patches(unpack_kernel, jobs, count, B, N1, n1p, stream);
+}
+
+// Interleaved pack of groups of four slots: every block transposes a 32-pixel x 32-displacement patch of each of a group's sources through
+// shared memory, then writes, per displacement, the four slots of its 32 pixels as one contiguous run.  All groups of a call in one
+// launch.  grid (ceil(largest D/32), n1p/32, groups * B), block (32, 8).
+__global__ void __launch_bounds__(256)
+pack_interleaved_kernel(const __grid_constant__ PackGroups groups, int B, int N1, int n1p) {
+  constexpr int RS = 32 * 33 + 32 / 4;  // slot stride chosen so that the interleaved read below is conflict-free
+  __shared__ uint32_t tile[4 * RS];
+  const int gi = blockIdx.z / B, b = blockIdx.z - gi * B;
+  const PackGroup& g = groups.g[gi];
+  const int D = g.D, d0 = blockIdx.x * 32, p0 = blockIdx.y * 32;  // displacement tiles fastest
+  if (d0 >= D) return;
   const int tx = threadIdx.x, ty = threadIdx.y;
 #pragma unroll
-  for (int r = 0; r < R4; ++r) {
-    const uint32_t* s = static_cast<const uint32_t*>(src.s[r].src);
+  for (int r = 0; r < 4; ++r) {
+    const SlotSource& ss = g.s[r];
+    const uint32_t* s = ss.src == nullptr ? nullptr : static_cast<const uint32_t*>(ss.src) + (((size_t)b * N1 + p0) * ss.Ksrc + ss.k) * D + d0 + tx;
+    const float dev = ss.dev != 0 ? __ldg(g.dev_scales + ss.dev - 1) : 1.f;
+#pragma unroll
     for (int j = ty; j < 32; j += 8) {
-      const int p = p0 + j, d = d0 + tx;
       uint32_t v = 0;
-      if (p < N1 && d < D) {
+      if (p0 + j < N1 && d0 + tx < D) {
         if (s == nullptr) {
-          v = __float_as_uint(src.s[r].scale);  // constant slot
+          v = __float_as_uint(ss.scale);  // constant slot
         } else {
-          v = __ldg(s + (((size_t)b * N1 + p) * src.s[r].Ksrc + src.s[r].k) * D + d);
-          if (src.s[r].scale != 0.f) v = __float_as_uint(__uint_as_float(v) * src.s[r].scale);
-          if (src.s[r].dev != 0) v = __float_as_uint(__uint_as_float(v) * __ldg(src.dev_scales + src.s[r].dev - 1));
+          v = __ldg(s + (size_t)j * ss.Ksrc * D);
+          if (ss.scale != 0.f) v = __float_as_uint(__uint_as_float(v) * ss.scale);
+          if (ss.dev != 0) v = __float_as_uint(__uint_as_float(v) * dev);
         }
       }
       tile[r * RS + j * 33 + tx] = v;
     }
   }
   __syncthreads();
-  // per displacement and group of four slots: 32 pixels x 4 slots = 128 consecutive words
-  const int t = ty * 32 + tx;
-  for (int j = 0; j < 32; ++j) {
-    const int d = d0 + j;
-    if (d >= D) break;
-    for (int i = t; i < 32 * R4; i += 256) {
-      const int q = i / 128, w = i % 128;  // group, word inside the group's 32-pixel run
-      dst[((((size_t)b * D + d) * Qtot + q0 + q) * n1p + p0) * 4 + w] = tile[(q * 4 + (w & 3)) * RS + (w >> 2) * 33 + j];
-    }
+  // per displacement: 32 pixels x 4 slots = 128 consecutive words, half a block each
+  const int t = ty * 32 + tx, w = t % 128;
+  uint32_t* dst = reinterpret_cast<uint32_t*>(g.dst) + ((((size_t)b * D + d0) * g.Qtot + g.q) * n1p + p0) * 4 + w;
+#pragma unroll 4
+  for (int j = t / 128; j < 32; j += 2) {
+    if (d0 + j >= D) break;
+    dst[(size_t)j * g.Qtot * n1p * 4] = tile[(w & 3) * RS + (w >> 2) * 33 + j];
   }
 }
 
-cudaError_t launch_pack_interleaved(const SlotSources& src, float* dst, int B, int N1, int n1p, int D, int R4,
-                                    int Qtot, int q0, cudaStream_t stream) {
-  const dim3 grid((D + 31) / 32, n1p / 32, B), block(32, 8);
-  uint32_t* out = reinterpret_cast<uint32_t*>(dst);
-  if (R4 == 4) pack_interleaved_kernel<4><<<grid, block, 0, stream>>>(src, out, N1, n1p, D, Qtot, q0);
-  else if (R4 == 8) pack_interleaved_kernel<8><<<grid, block, 0, stream>>>(src, out, N1, n1p, D, Qtot, q0);
-  else return cudaErrorInvalidValue;
-  return cudaGetLastError();
+// Launches of at most as many groups as grid.z takes.
+template <class Launch>
+static cudaError_t launch_groups(const PackGroups& groups, int B, Launch&& launch) {
+  const int per_launch = pack_groups_per_launch(B);
+  for (int first = 0; first < groups.count; first += per_launch) {
+    PackGroups some = groups;
+    some.count = std::min(per_launch, groups.count - first);
+    int D = 1;
+    for (int i = 0; i < some.count; ++i) {
+      some.g[i] = groups.g[first + i];
+      D = std::max(D, some.g[i].D);
+    }
+    launch(some, D);
+    if (cudaError_t err = cudaGetLastError(); err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_pack_interleaved(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream) {
+  return launch_groups(groups, B, [&](const PackGroups& some, int D) {
+    pack_interleaved_kernel<<<dim3((D + 31) / 32, n1p / 32, some.count * B), dim3(32, 8), 0, stream>>>(some, B, N1, n1p);
+  });
 }
 
 // Channels-first sources are already pixel-fastest: one thread per pixel gathers the four slots of a group
@@ -436,36 +496,9 @@ pack_interleaved_cf_kernel(const __grid_constant__ PackGroups groups, int B, int
 }
 
 cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream) {
-  const int per_launch = pack_groups_per_launch(B);
-  for (int first = 0; first < groups.count; first += per_launch) {
-    PackGroups some = groups;
-    some.count = std::min(per_launch, groups.count - first);
-    int D = 1;
-    for (int i = 0; i < some.count; ++i) {
-      some.g[i] = groups.g[first + i];
-      D = std::max(D, some.g[i].D);
-    }
-    const dim3 grid((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, some.count * B);
-    pack_interleaved_cf_kernel<<<grid, 256, 0, stream>>>(some, B, N1, n1p);
-    if (cudaError_t err = cudaGetLastError(); err != cudaSuccess) return err;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t launch_pack(const void* src, float* dst, int B, int N1, int n1p, int Ksrc, int ksrc0, int K, int D,
-                        int R, int r0, int rstride, float scale, cudaStream_t stream) {
-  const dim3 grid((D + 31) / 32, n1p / PACK_PX, B * K), block(32, 8);
-  pack_kernel<<<grid, block, 0, stream>>>(static_cast<const uint32_t*>(src), reinterpret_cast<uint32_t*>(dst), N1,
-                                          n1p, Ksrc, ksrc0, K, D, R, r0, rstride, scale);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_unpack(const float* src, void* dst, int B, int N1, int n1p, int K, int D, int R, int r0,
-                          int rstride, int Kdst, int kdst0, cudaStream_t stream) {
-  const dim3 grid((D + 31) / 32, n1p / PACK_PX, B * K), block(32, 8);
-  unpack_kernel<<<grid, block, 0, stream>>>(reinterpret_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), N1,
-                                            n1p, K, D, R, r0, rstride, Kdst, kdst0);
-  return cudaGetLastError();
+  return launch_groups(groups, B, [&](const PackGroups& some, int D) {
+    pack_interleaved_cf_kernel<<<dim3((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, some.count * B), 256, 0, stream>>>(some, B, N1, n1p);
+  });
 }
 
 // (B, C, N) -> (B, N, C) for all images of a call in one launch, scaled: as TF32 in `out` or as 16-bit operands in `outh` (the one
@@ -553,47 +586,45 @@ cudaError_t launch_channel_major_cf(const MapCopy* copy, int count, int B, int C
   return cudaGetLastError();
 }
 
-// Channel-major copies of a pixel-major feature array (B, rows*width, C), the K-major B operands of the gradient GEMMs.
+// Channel-major copies of pixel-major feature arrays (B, rows*width, C), the K-major B operands of the gradient GEMMs.
 //   blocked = 0: dst (B, C, pitch), pixel index = row*width + x (image 1: rows = 1, width = N1, pitch = n1p)
 //   blocked = 1: dst (B, C, ceil(width/16), pitch, 16): columns in blocks of 16, so that the 4 rows x 16 columns of one
 //                K block of the image-1-major GEMM are 64 consecutive values (image 2: pitch = H2 rounded up to 4)
-// Padding is not written (the caller clears the array).  32 x 32 tiles through shared memory; grid (ceil(width/32),
-// ceil(C/32), B*rows), block (32, 8).
+// Padding is zero.  32 x 32 tiles through shared memory, both images in one launch; grid (sum over the images of tiles of their padded
+// rows, ceil(C/32), B), block (32, 8).
+__host__ __device__ inline int map_copy_columns(const MapCopy& c) { return c.blocked ? (c.width + 15) / 16 * 16 : c.pitch; }   // of a padded row
+__host__ __device__ inline int map_copy_rows(const MapCopy& c) { return c.blocked ? c.pitch : 1; }
 template <typename T>
-__global__ void channel_major_kernel(const float* __restrict__ in, T* __restrict__ out, int rows, int width,
-                                     int pitch, int C, int blocked, int op16, const float* __restrict__ scale16) {
+__global__ void channel_major_kernel(const MapCopy c1, const MapCopy c2, int blocks1, int C, int op16) {
   __shared__ float tile[32][33];
-  const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
-  const int b = blockIdx.z / rows, row = blockIdx.z - b * rows, x0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  const bool first = (int)blockIdx.x < blocks1;
+  const MapCopy& c = first ? c1 : c2;
+  const float sc16 = (op16 == OP16_FP16 && c.scale16 != nullptr) ? __ldg(c.scale16) : 1.f;
+  const int columns = map_copy_columns(c), per_row = (columns + 31) / 32, r = blockIdx.x - (first ? 0 : blocks1);
+  const int row = r / per_row, x0 = (r - row * per_row) * 32, c0 = blockIdx.y * 32, b = blockIdx.z;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const float* src = in + ((size_t)b * rows + row) * width * C;
+  const float* src = c.src + (((size_t)b * c.rows + row) * c.width + x0) * C + c0 + tx;
 #pragma unroll
-  for (int j = ty; j < 32; j += 8) {
-    const int x = x0 + j, c = c0 + tx;
-    tile[j][tx] = (x < width && c < C) ? __ldg(src + (size_t)x * C + c) : 0.f;
-  }
+  for (int j = ty; j < 32; j += 8) tile[j][tx] = (row < c.rows && x0 + j < c.width && c0 + tx < C) ? __ldg(src + (size_t)j * C) : 0.f;
   __syncthreads();
-  const size_t per_channel = blocked ? (size_t)((width + 15) / 16) * pitch * 16 : (size_t)pitch;
+  const size_t per_channel = (size_t)map_copy_rows(c) * columns;
+  const int x = x0 + tx;
+  const size_t off = c.blocked ? ((size_t)(x >> 4) * c.pitch + row) * 16 + (x & 15) : (size_t)x;
+  T* dst = static_cast<T*>(c.dst) + ((size_t)b * C + c0) * per_channel + off;
 #pragma unroll
   for (int j = ty; j < 32; j += 8) {
-    const int c = c0 + j, x = x0 + tx;
-    if (c < C && x < width) {
-      const size_t off = blocked ? ((size_t)(x >> 4) * pitch + row) * 16 + (x & 15) : (size_t)x;
-      if constexpr (sizeof(T) == 2) out[((size_t)b * C + c) * per_channel + off] = to_op16(tile[tx][j] * sc16, op16);
-      else out[((size_t)b * C + c) * per_channel + off] = tile[tx][j];
+    if (c0 + j < C && x < columns) {
+      if constexpr (sizeof(T) == 2) dst[(size_t)j * per_channel] = to_op16(tile[tx][j] * sc16, op16);
+      else dst[(size_t)j * per_channel] = tile[tx][j];
     }
   }
 }
 
-cudaError_t launch_channel_major(const float* src, void* dst, int B, int rows, int width, int pitch, int C,
-                                 int blocked, int op16, const float* scale16, cudaStream_t stream) {
-  const dim3 grid((width + 31) / 32, (C + 31) / 32, B * rows), block(32, 8);
-  if (op16)
-    channel_major_kernel<<<grid, block, 0, stream>>>(src, static_cast<uint16_t*>(dst), rows, width, pitch, C, blocked,
-                                                     op16, scale16);
-  else
-    channel_major_kernel<<<grid, block, 0, stream>>>(src, static_cast<float*>(dst), rows, width, pitch, C, blocked, 0,
-                                                     nullptr);
+cudaError_t launch_channel_major(const MapCopy& c1, const MapCopy& c2, int B, int C, int op16, cudaStream_t stream) {
+  auto blocks = [](const MapCopy& c) { return (map_copy_columns(c) + 31) / 32 * map_copy_rows(c); };
+  const dim3 grid(blocks(c1) + blocks(c2), (C + 31) / 32, B), block(32, 8);
+  if (op16) channel_major_kernel<uint16_t><<<grid, block, 0, stream>>>(c1, c2, blocks(c1), C, op16);
+  else channel_major_kernel<float><<<grid, block, 0, stream>>>(c1, c2, blocks(c1), C, 0);
   return cudaGetLastError();
 }
 
@@ -660,12 +691,9 @@ cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, floa
   const int threads = 256;
   auto blocks = [&](size_t n) { return (unsigned)std::min<size_t>((n + threads - 1) / threads, 148 * 16); };
   if (F1r != nullptr || F1h != nullptr) {
-    round_copy_kernel<<<blocks(n1), threads, 0, stream>>>(reinterpret_cast<const float4*>(F1),
-                                                          reinterpret_cast<float4*>(F1r), n1,
-                                                          reinterpret_cast<uint2*>(F1h), op16, s1);
-    round_copy_kernel<<<blocks(n2), threads, 0, stream>>>(reinterpret_cast<const float4*>(F2),
-                                                          reinterpret_cast<float4*>(F2r), n2,
-                                                          reinterpret_cast<uint2*>(F2h), op16, s2);
+    const RoundJob j1{reinterpret_cast<const float4*>(F1), reinterpret_cast<float4*>(F1r), reinterpret_cast<uint2*>(F1h), s1, n1};
+    const RoundJob j2{reinterpret_cast<const float4*>(F2), reinterpret_cast<float4*>(F2r), reinterpret_cast<uint2*>(F2h), s2, n2};
+    round_copy_kernel<<<dim3(blocks(std::max(n1, n2)), 2), threads, 0, stream>>>(j1, j2, op16);
   }
   if (aux != nullptr || auxh != nullptr)
     f2_means_kernel<<<dim3(d.H2 + d.W2, d.B), FM_GROUPS * FM_QUADS, 0, stream>>>(F2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
