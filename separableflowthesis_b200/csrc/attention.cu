@@ -1072,19 +1072,20 @@ static size_t tile_count(const AttentionDims& d) {
 // SM, hence fewer and longer pieces.
 constexpr int AT_BLOCKS_TARGET = 148 * 8, AT_MIN_WALK = 8;
 constexpr int WG_BLOCKS_TARGET = 148 * 3, WG_MIN_WALK = 16;
-static int walk_length(size_t blocks, int D, int target = AT_BLOCKS_TARGET, int min_walk = AT_MIN_WALK) {
-  const int pieces = (int)((target + blocks - 1) / blocks);
-  const int dc = (D + pieces - 1) / pieces;
-  const int least = D < min_walk ? D : min_walk;
-  return dc > least ? dc : least;
+// The jobs of a launch fill the SMs together, with walks of about the same length: `total` is the sum of their D.  (Every job with as
+// many pieces as if it were the only one of its size, 1 x 55 x 128 with four levels and channels spent the last half of its logits on a few
+// long walks: 56 us, 50 now.)
+static int walk_length(size_t blocks, int D, int total, int target = AT_BLOCKS_TARGET, int min_walk = AT_MIN_WALK) {
+  const int pieces = (int)((target + blocks - 1) / blocks);   // of all jobs
+  const int dc = std::max((total + pieces - 1) / pieces, min_walk), own = (D + dc - 1) / dc;
+  return (D + own - 1) / own;
 }
-// Displacements per block of the weight gradients' walk, and the blocks of a job (partial sums of a weight).  The jobs of a launch fill the
-// SMs together.
-static int weight_walk(const AttentionDims& d, int jobs, bool tiled) {
-  return walk_length((tiled ? tile_count(d) : 2 * (size_t)pixel_grid(d).x) * d.B * jobs, d.D, WG_BLOCKS_TARGET, WG_MIN_WALK);
+// Displacements per block of the weight gradients' walk, and the blocks of a job (partial sums of a weight).
+static int weight_walk(const AttentionDims& d, int total, bool tiled) {
+  return walk_length((tiled ? tile_count(d) : 2 * (size_t)pixel_grid(d).x) * d.B, d.D, total, WG_BLOCKS_TARGET, WG_MIN_WALK);
 }
-static size_t weight_rows(const AttentionDims& d, int jobs, bool tiled) {
-  const int dc = weight_walk(d, jobs, tiled);
+static size_t weight_rows(const AttentionDims& d, int total, bool tiled) {
+  const int dc = weight_walk(d, total, tiled);
   return (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * ((d.D + dc - 1) / dc);
 }
 // The softmax backward: pixels of a block by the length of the column (attention_logit_grad_kernel).
@@ -1094,8 +1095,10 @@ static size_t bias_rows(const AttentionDims& d) { return (size_t)d.B * ((d.H1 * 
 // Bias partials per block of the softmax backward, weight partials per block of the weight gradients, whichever form they take.
 size_t attention_partial_floats(const AttentionDims* d, int count) {
   size_t floats = 0;
+  int total = 0;
+  for (int i = 0; i < count; ++i) total += d[i].D;
   for (int i = 0; i < count; ++i)
-    floats += d[i].Kc * (bias_rows(d[i]) + 2 * AT_TAPS * std::max(weight_rows(d[i], count, true), weight_rows(d[i], count, false)));
+    floats += d[i].Kc * (bias_rows(d[i]) + 2 * AT_TAPS * std::max(weight_rows(d[i], total, true), weight_rows(d[i], total, false)));
   return floats;
 }
 
@@ -1138,15 +1141,22 @@ static cudaError_t launch_softmax(const AttentionJob* job, int count, cudaStream
   return launch_softmax_class<0>(job, count, 32, INT_MAX, st);
 }
 
-// Displacements per block of the forward's walk, and whether the walks of a launch end with the softmax of their columns.  The jobs
-// of a launch fill the SMs together.  A column short enough for that is not cut by launches that have two blocks per SM without it.
-static int forward_walk(const AttentionDims& d, int jobs, bool tiled) {
-  const size_t blocks = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * jobs;
-  return d.D <= AT_SOFT_MAX && blocks >= 2 * SM_COUNT ? d.D : walk_length(blocks, d.D);
+template <class Job>
+static int total_D(const Job* job, int count) {
+  int total = 0;
+  for (int i = 0; i < count; ++i) total += job[i].d.D;
+  return total;
+}
+// Displacements per block of the forward's walk, and whether the walks of a launch end with the softmax of their columns.  A column
+// short enough for that is not cut by launches that have two blocks per SM without it.
+static int forward_walk(const AttentionDims& d, int jobs, int total, bool tiled) {
+  const size_t blocks = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
+  return d.D <= AT_SOFT_MAX && blocks * jobs >= 2 * SM_COUNT ? d.D : walk_length(blocks, d.D, total);
 }
 static bool softmax_in_walk(const AttentionJob* job, int count, bool tiled) {
+  const int total = total_D(job, count);
   for (int i = 0; i < count; ++i)
-    if (job[i].d.D > AT_SOFT_MAX || forward_walk(job[i].d, count, tiled) < job[i].d.D) return false;
+    if (job[i].d.D > AT_SOFT_MAX || forward_walk(job[i].d, count, total, tiled) < job[i].d.D) return false;
   return true;
 }
 static bool all_tileable(const AttentionJob* job, int count, const int* status) {
@@ -1183,7 +1193,7 @@ cudaError_t launch_attention_forward(const AttentionJob* job, int count, const A
       cudaError_t err = tile_map(&maps.m[i], j.x, j.x_sb, 2, 2, j.d, true);
       if (err != cudaSuccess) return err;
     }
-    const int dc = forward_walk(j.d, count, tiled);
+    const int dc = forward_walk(j.d, count, total_D(job, count), tiled);
     jobs.j[i] = LogitsJobs::Job{j.x, j.x_sb, modules.bias[j.module], j.a, j.d.D, dc, j.module};
     blocks += (unsigned long long)(tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * ((j.d.D + dc - 1) / dc);
     if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
@@ -1286,7 +1296,7 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
                                       const AttentionGradients& grads, float* partial, cudaStream_t st, int* status) {
   if (count < 1 || count > MAX_ATTENTION_JOBS) return cudaErrorInvalidValue;
   const AttentionDims& d = job[0].d;
-  const int N1 = d.H1 * d.W1;
+  const int N1 = d.H1 * d.W1, total = total_D(job, count);
   auto g_sb = [&](const AttentionGradJob& j) { return (long long)d.Kc * j.d.D * N1; };
   bool tiled = status != nullptr;
   for (int i = 0; i < count; ++i) tiled = tiled && tileable(job[i].d, job[i].x, job[i].x_sb) && tileable(job[i].d, job[i].g, g_sb(job[i]));
@@ -1302,7 +1312,7 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
       place[i].bias_row0 = brows;
       place[i].weight_row0 = wrows;
       brows += (int)bias_rows(job[i].d);
-      wrows += (int)weight_rows(job[i].d, count, tiled);
+      wrows += (int)weight_rows(job[i].d, total, tiled);
     }
     float *const bias = partial, *const weight = bias + (size_t)brows * d.Kc;
     partial = weight + (size_t)wrows * d.Kc * 2 * AT_TAPS;
@@ -1330,7 +1340,7 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
       jobs.blocks.first[i] = (int)blocks;
       if (i >= count) continue;
       const size_t tiles = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
-      const int dc = walk_length(tiles * count, job[i].d.D);
+      const int dc = walk_length(tiles, job[i].d.D, total);
       jobs.j[i] = InputGradJobs::Job{job[i].g, job[i].add, job[i].add_sb, job[i].gx, job[i].d.D, dc, job[i].module};
       blocks += (unsigned long long)tiles * ((job[i].d.D + dc - 1) / dc);
       if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
@@ -1368,9 +1378,9 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
   for (int i = 0; i <= MAX_ATTENTION_JOBS; ++i) {
     jobs.blocks.first[i] = (int)blocks;
     if (i >= count) continue;
-    jobs.j[i] = WeightGradJobs::Job{job[i].x, job[i].x_sb, job[i].g, place[i].weight, job[i].d.D, weight_walk(job[i].d, count, tiled),
+    jobs.j[i] = WeightGradJobs::Job{job[i].x, job[i].x_sb, job[i].g, place[i].weight, job[i].d.D, weight_walk(job[i].d, total, tiled),
                                     place[i].weight_row0, place[i].weight_rows};
-    blocks += weight_rows(job[i].d, count, tiled);
+    blocks += weight_rows(job[i].d, total, tiled);
     if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
     if (tiled) {
       err = tile_map(&maps_x.m[i], job[i].x, job[i].x_sb, 2, 2, job[i].d, true);
