@@ -78,16 +78,16 @@ __device__ __forceinline__ L4Quad l4_load(const float* p, bool ok) {
   return q;
 }
 
-// v[i] of all lanes summed; lane i keeps the total of v[i].  31 shuffles for 32 values.
-__device__ __forceinline__ float warp_transpose_reduce(float (&v)[32], int lane) {
+// v[i] summed over each group of N neighbouring lanes; lane i of a group keeps the total of v[i].  N - 1 shuffles for N values.
+template <int N>
+__device__ __forceinline__ float group_transpose_reduce(float (&v)[N], int lane) {
 #pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const int off = 16 >> s, n = 32 >> s;
+  for (int off = N / 2; off > 0; off /= 2) {
     const bool up = (lane & off) != 0;
 #pragma unroll
-    for (int i = 0; i < n / 2; ++i) {
-      const float send = up ? v[i] : v[i + n / 2];
-      const float keep = up ? v[i + n / 2] : v[i];
+    for (int i = 0; i < off; ++i) {
+      const float send = up ? v[i] : v[i + off];
+      const float keep = up ? v[i + off] : v[i];
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
     }
   }
@@ -145,45 +145,58 @@ constexpr int L4_BMAX = 224;                   // largest box a four-pixel walk 
 static_assert(L4_SIDE * L4_SIDE <= L4_BMAX && L4_BMAX % 32 == 0, "one pixel's positions must fit the table");
 
 // Dot products of NPX pixels' feature rows with the image-2 rows of a box, scaled, into S[px0 + px][position]; zero
-// outside the image.
-template <int NCH, int NPX>
-__device__ __forceinline__ void l4_box_products(const L4Quad (&f1)[NPX][NCH], const float* __restrict__ F2b, int C,
+// outside the image.  LP lanes split the channels, so the warp does 32 / LP positions at a time: up to 256 channels 16 lanes, which
+// halves the work of the reductions and keeps the additions of a lane as many as with 32 lanes (two chains).
+// FULL: C = NQ * 4 * LP, no lane without channels.
+template <int NQ, int NPX, int LP, bool FULL>
+__device__ __forceinline__ void l4_box_products(const L4Quad (&f1)[NPX][NQ], const float* __restrict__ F2b, int C,
                                                 const int* rows, int nq, float scale, float (*S)[L4_BMAX], int px0,
                                                 int lane) {
-  constexpr int QB = 32 / NPX;
-  for (int q0 = 0; q0 < nq; q0 += QB) {
-    float v[32];
+  constexpr int PB = 32 / LP, STEPS = LP / NPX, HALF = LP == 16 ? (NQ + 1) / 2 : NQ;   // chunks of the first chain
+  const int group = lane / LP, at = lane % LP;
+  const uint32_t row_bytes = 4 * C;   // (32-bit factors: the product and the sum are one multiply-add)
+  const char* const src = reinterpret_cast<const char*>(F2b + at * 4);
+  for (int q0 = 0; q0 < nq; q0 += PB * STEPS) {
+    float v[LP];
 #pragma unroll
-    for (int qi = 0; qi < QB; ++qi) {
-      const int r = rows[q0 + qi];
-      const float* src = F2b + (size_t)(r < 0 ? 0 : r) * C + lane * 4;
-      L4Quad f2[NCH];
+    for (int step = 0; step < STEPS; ++step) {
+      const int r = rows[q0 + step * PB + group];   // (beyond the image row 0 is read, and not used)
+      const float* const row = reinterpret_cast<const float*>(src + (uint64_t)row_bytes * (uint32_t)max(r, 0));
+      L4Quad f2[NQ];
 #pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) f2[ch] = l4_load(src + ch * 128, r >= 0 && ch * 128 + lane * 4 < C);
+      for (int ch = 0; ch < NQ; ++ch) f2[ch] = l4_load(row + ch * 4 * LP, FULL || (r >= 0 && (ch * LP + at) * 4 < C));
 #pragma unroll
       for (int px = 0; px < NPX; ++px) {
-        uint64_t acc = mul2(f1[px][0].lo, f2[0].lo);
-        acc = fma2(f1[px][0].hi, f2[0].hi, acc);
+        uint64_t acc = fma2(f1[px][0].hi, f2[0].hi, mul2(f1[px][0].lo, f2[0].lo));
 #pragma unroll
-        for (int ch = 1; ch < NCH; ++ch) acc = fma2(f1[px][ch].hi, f2[ch].hi, fma2(f1[px][ch].lo, f2[ch].lo, acc));
-        v[qi * NPX + px] = sum2(acc);
+        for (int ch = 1; ch < HALF; ++ch) acc = fma2(f1[px][ch].hi, f2[ch].hi, fma2(f1[px][ch].lo, f2[ch].lo, acc));
+        if (HALF < NQ) {
+          uint64_t acc2 = fma2(f1[px][HALF].hi, f2[HALF].hi, mul2(f1[px][HALF].lo, f2[HALF].lo));
+#pragma unroll
+          for (int ch = HALF + 1; ch < NQ; ++ch) acc2 = fma2(f1[px][ch].hi, f2[ch].hi, fma2(f1[px][ch].lo, f2[ch].lo, acc2));
+          acc = add2(acc, acc2);
+        }
+        v[step * NPX + px] = sum2(acc);
       }
     }
-    const float total = warp_transpose_reduce(v, lane);
-    const int q = q0 + lane / NPX;
-    if (q < nq) S[px0 + lane % NPX][q] = total * scale;
+    const float total = group_transpose_reduce<LP>(v, lane);
+    const int q = q0 + at / NPX * PB + group;
+    if (q < nq) S[px0 + at % NPX][q] = rows[q] >= 0 ? total * scale : 0.f;
   }
 }
 
+// Two packed multiply-adds per 4 channels, pixel and position, and the reductions, bound the forward: 2 x 55 x 128 at C = 256, four
+// levels, radius 4 takes 172 us with 32 lanes a position, 148 with 16.
 // grid (ceil(W1/8) * ceil(H1/4), levels, B)
-template <int NCH>
+template <int NQ, int LP, bool FULL>
 __global__ void __launch_bounds__(L4_THREADS, 2)
 lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                         float* __restrict__ out, int H1, int W1, int C, int radius, int levels, float scale) {
   __shared__ float s_S[L4_WARPS][L4_PX][L4_BMAX];
   __shared__ float s_out[L4_WIN * L4_WIN][L4_TILE + 1];
   __shared__ int s_rows[L4_WARPS][L4_BMAX];
-  __shared__ L4Pixel s_geo[L4_WARPS][L4_PX];
+  __shared__ int2 s_base[L4_WARPS][L4_PX];               // integer positions under the window centres
+  __shared__ float s_frac[L4_WARPS][2][L4_PX][L4_WIN];   // l4_fraction of the window entries along x, y
 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int level = blockIdx.y, b = blockIdx.z, N1 = H1 * W1;
@@ -199,16 +212,22 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
   const int mh = ph + ((lane >> 1) & 1), mw = pw + (lane & 1);
   const bool mine = lane < L4_PX && mh < H1 && mw < W1;
   if (mine) geo = l4_pixel_geometry(coords, b, mh * W1 + mw, N1, level, H2, W2);
-  if (lane < L4_PX) s_geo[w][lane] = geo;
+  if (lane < L4_PX) s_base[w][lane] = make_int2(geo.bx, geo.by);
   const unsigned mask = __ballot_sync(0xffffffffu, mine);
+  for (int i = lane; i - lane < 2 * L4_PX * win; i += 32) {
+    const int axis = i & 1, px = (i >> 1) % L4_PX, t = i / (2 * L4_PX);
+    const float cx = __shfl_sync(0xffffffffu, geo.cx, px), cy = __shfl_sync(0xffffffffu, geo.cy, px);
+    const int bx = __shfl_sync(0xffffffffu, geo.bx, px), by = __shfl_sync(0xffffffffu, geo.by, px);
+    if (t < win) s_frac[w][axis][px][t] = l4_fraction(axis ? cy : cx, axis ? by : bx, t, radius, axis ? H2 : W2);
+  }
 
   if (mask != 0) {
-    L4Quad f1[L4_PX][NCH];
+    L4Quad f1[L4_PX][NQ];
 #pragma unroll
     for (int px = 0; px < L4_PX; ++px)
 #pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        const int c = ch * 128 + lane * 4;
+      for (int ch = 0; ch < NQ; ++ch) {
+        const int c = (ch * LP + lane % LP) * 4;
         const size_t p = (size_t)b * N1 + (size_t)(ph + px / 2) * W1 + pw + px % 2;
         const bool ok = ((mask >> px) & 1u) && c < C;
         f1[px][ch] = l4_load(F1 + (ok ? p * C + c : 0), ok);
@@ -219,19 +238,19 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
     if (together) {
       l4_fill_rows(s_rows[w], box, H2, W2, lane);
       __syncwarp();
-      l4_box_products<NCH, L4_PX>(f1, F2b, C, s_rows[w], box.bw * box.bh, scale, s_S[w], 0, lane);
+      l4_box_products<NQ, L4_PX, LP, FULL>(f1, F2b, C, s_rows[w], box.bw * box.bh, scale, s_S[w], 0, lane);
     } else {  // motion boundaries: one pixel at a time
 #pragma unroll
       for (int px = 0; px < L4_PX; ++px) {
         if (!((mask >> px) & 1u)) continue;
-        L4Quad one[1][NCH];
+        L4Quad one[1][NQ];
 #pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) one[0][ch] = f1[px][ch];
+        for (int ch = 0; ch < NQ; ++ch) one[0][ch] = f1[px][ch];
         box = l4_box(geo, 1u << px, radius, lane);
         __syncwarp();
         l4_fill_rows(s_rows[w], box, H2, W2, lane);
         __syncwarp();
-        l4_box_products<NCH, 1>(one, F2b, C, s_rows[w], box.bw * box.bh, scale, s_S[w], px, lane);
+        l4_box_products<NQ, 1, LP, FULL>(one, F2b, C, s_rows[w], box.bw * box.bh, scale, s_S[w], px, lane);
       }
     }
     __syncwarp();
@@ -241,13 +260,12 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
       const int px = idx / (win * win), o = idx - px * win * win;
       if (!((mask >> px) & 1u)) continue;
       const int a = o / win, bb = o - a * win;
-      const L4Pixel g = s_geo[w][px];
-      const int ox = together ? box.ox : g.bx - radius;
-      const int oy = together ? box.oy : g.by - radius;
+      const int2 g = s_base[w][px];
+      const int ox = together ? box.ox : g.x - radius;
+      const int oy = together ? box.oy : g.y - radius;
       const int sbw = together ? box.bw : 2 * radius + 2;
-      const float fx = l4_fraction(g.cx, g.bx, a, radius, W2);
-      const float fy = l4_fraction(g.cy, g.by, bb, radius, H2);
-      const float* S = s_S[w][px] + (g.by + bb - radius - oy) * sbw + (g.bx + a - radius - ox);
+      const float fx = s_frac[w][0][px][a], fy = s_frac[w][1][px][bb];
+      const float* S = s_S[w][px] + (g.y + bb - radius - oy) * sbw + (g.x + a - radius - ox);
       const float top = S[0] + fx * (S[1] - S[0]);
       const float bot = S[sbw] + fx * (S[sbw + 1] - S[sbw]);
       s_out[o][(2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2] = top + fy * (bot - top);
@@ -478,12 +496,16 @@ cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, cons
                                     const float* coords, float* out, float scale, cudaStream_t stream) {
   const Lookup4dLevels lv = make_levels(d, F2, nullptr);
   const dim3 grid(l4_tiles(d), d.levels, d.B);
-#define SFB_L4_FWD(NCH) lookup4d_forward_kernel<NCH><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, out, d.H1, d.W1, d.C, d.radius, d.levels, scale)
-  switch ((d.C + 127) / 128) {
-    case 1: SFB_L4_FWD(1); break;
-    case 2: SFB_L4_FWD(2); break;
-    case 3: SFB_L4_FWD(3); break;
-    case 4: SFB_L4_FWD(4); break;
+#define SFB_L4_FWD(NQ, LP)                                                                                                             \
+  (d.C == NQ * 4 * LP ? lookup4d_forward_kernel<NQ, LP, true> : lookup4d_forward_kernel<NQ, LP, false>)<<<grid, L4_THREADS, 0, stream>>>( \
+      F1, lv, coords, out, d.H1, d.W1, d.C, d.radius, d.levels, scale)
+  switch ((d.C + 63) / 64) {
+    case 1: SFB_L4_FWD(1, 16); break;
+    case 2: SFB_L4_FWD(2, 16); break;
+    case 3: SFB_L4_FWD(3, 16); break;
+    case 4: SFB_L4_FWD(4, 16); break;
+    case 5: case 6: SFB_L4_FWD(3, 32); break;
+    case 7: case 8: SFB_L4_FWD(4, 32); break;
     default: return cudaErrorInvalidValue;
   }
 #undef SFB_L4_FWD

@@ -413,6 +413,11 @@ __device__ __forceinline__ float round_tf32(float x) {
 
 // Packed FP32 pairs (sm_100): two floats in one 64-bit register, multiplied / fused-multiply-added in
 // one instruction.
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
