@@ -2109,7 +2109,7 @@ int sfb_lookup4d_backward(const float* F1, const float* const* F2_levels, const 
   if (reinterpret_cast<uintptr_t>(gF1) % 16 != 0)
     return fail(SFB_ERR_INVALID_ARGUMENT, "gF1 must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SFB_CUDA(timed(KID_LOOKUP4D, 1, st, [&] {
+  SFB_CUDA(timed(KID_LOOKUP4D, lookup4d_backward_launches(ld), st, [&] {
     return launch_lookup4d_backward(ld, F1, F2_levels, coords, gout, gF1, gF2_levels, scale, st);
   }));
   return SFB_OK;

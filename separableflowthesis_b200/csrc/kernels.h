@@ -444,6 +444,7 @@ struct Lookup4dDims {
 [[nodiscard]] cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                     const float* coords, float* out, float scale, cudaStream_t stream);
 // gF1 (shape of F1) is overwritten; gF2[l] (shape of F2[l]) is zeroed and then accumulated with float reductions.
+int lookup4d_backward_launches(const Lookup4dDims& d);
 [[nodiscard]] cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                      const float* coords, const float* gout, float* gF1, float* const* gF2,
                                      float scale, cudaStream_t stream);

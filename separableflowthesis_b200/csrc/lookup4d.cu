@@ -16,10 +16,13 @@
 // boundary) the walk is done for fewer pixels at a time.  A CTA covers 8 x 4 pixels and stages its outputs in shared
 // memory, so that the (B, levels*(2r+1)^2, H1, W1) result is written in runs of eight pixels (a 32-byte sector).
 //
-// Backward (features only: the model detaches the coordinates, core/sepflow.py:193): the same walk with the roles
-// swapped.  The gradient of a pixel's window is spread back onto the integer positions (each takes from at most four
-// window entries), gF1 accumulates in registers over all positions and levels and is stored once, and the
-// image-2 feature gradient of every position receives one 16-byte vector reduction per lane (red.global.add.v4.f32).
+// Backward (features only: the model detaches the coordinates, core/sepflow.py:193): the gradient of a pixel's window is
+// spread back onto the integer positions (each takes from at most four window entries); gF1 is the sum over positions of
+// that times the image-2 row, gF2 of a position the sum over pixels of the same times the pixel's row.  The channel is a
+// free index of both, so a lane owns one channel for all pixels of a 4 x 4 tile, and the box of all their windows is
+// walked once: an image-2 row is read, and reduced into L2, once per tile.  Tiles whose windows lie too far apart take
+// the forward's walks, with one 16-byte vector reduction per lane (red.global.add.v4.f32) and position.
+#include <algorithm>
 #include <climits>
 
 #include "kernels.h"
@@ -279,6 +282,17 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
 }
 
 // ---- backward ---------------------------------------------------------------------------------------------
+constexpr int L4_BT = 4;                        // tile of 4 x 4 pixels
+constexpr int L4_BPX = L4_BT * L4_BT;
+constexpr int L4_BBOX = 384;                    // positions of the largest box walked for the whole tile
+constexpr int L4_BTHREADS = 256, L4_BWARPS = L4_BTHREADS / 32;
+// Largest box of a tile for windows of a radius.  A level of a whole tile takes 1.2 us per position plus 35, where four walks of 2 x 2 pixels take
+// 0.85 (2 x 55 x 128, C = 256); those have (2r + 3)^2 positions each in a smooth field and (2r + 4)^2 or more where the tile's box is near the
+// limit: radius 4 382, 3 256, 2 153.  With (2r + 3)^2 a field with noise of half a pixel took 337 us at radius 3, 2 x 2 pixels alone 299, 220 with
+// this.  Radius 1 and 0 walk 2 x 2 pixels only.
+inline int l4_tile_limit(int radius) { return radius < 2 ? 0 : std::min(L4_BBOX, (4 * (2 * radius + 4) * (2 * radius + 4) - 41) * 5 / 7); }
+static_assert(L4_BTHREADS <= L4_BBOX && L4_BBOX % 4 == 0, "partial sums of warps that share channels; steps of four positions");
+
 __device__ __forceinline__ void red_add_v4(float* addr, uint64_t lo, uint64_t hi) {
   float x, y, z, w;
   unpack2(lo, x, y);
@@ -342,7 +356,7 @@ __device__ __forceinline__ void l4_box_gradients(const L4Quad (&f1)[L4_PX][NCH],
 
 // Gradient of one integer position of a pixel's window: position (i, j) of its (2r+2)^2 grid takes from window entries
 // a in {i-1, i}, b in {j-1, j} with the weight that entry gives it.  pp: the pixel's column of s_g.
-__device__ __forceinline__ float l4_position_gradient(const L4Pixel& g, int i, int j, const float (*s_g)[L4_TILE + 1], int pp,
+__device__ __forceinline__ float l4_position_gradient(const L4Pixel& g, int i, int j, const float (*s_g)[L4_BPX + 1], int pp,
                                                       int radius, int H2, int W2) {
   const int win = 2 * radius + 1, side = 2 * radius + 2;
   float acc = 0.f;
@@ -371,28 +385,267 @@ __device__ __forceinline__ float l4_position_gradient(const L4Pixel& g, int i, i
 constexpr int L4_ALONE_ROWS = L4_BMAX / 2, L4_ALONE_PAD = 4;
 static_assert(L4_SIDE * L4_SIDE <= L4_ALONE_ROWS && L4_ALONE_ROWS + L4_SIDE * L4_SIDE + L4_ALONE_PAD <= L4_BMAX, "a pixel's positions and rows");
 
-// The forward's blocks of 8 x 4 and 2 x 2 pixels; every CTA walks all levels, so that gF1 is stored once.  Bound by
-// instruction issue like the forward.  A walk for 4 x 2 pixels with the channels split over two warps makes fewer
-// reductions into L2, but it reads every position's gradients twice and was slower (474 us, against 444 us for the scalar
-// kernel that took four pixels of a row).  grid (ceil(W1/8) * ceil(H1/4), 1, B)
-template <int NCH>
-__global__ void __launch_bounds__(L4_THREADS, 2)
+// Geometry of a tile's pixels and the boxes of their windows at all levels, a warp per level; whether every box has at most `limit`
+// positions.  All threads; ends with a barrier.
+struct L4Tile {
+  L4Pixel geo[LOOKUP_MAX_LEVELS][L4_BPX];
+  L4Box box[LOOKUP_MAX_LEVELS];
+};
+__device__ __forceinline__ bool l4_tile(L4Tile& t, const float* __restrict__ coords, const Lookup4dLevels& lv, int levels, int b, int h0, int w0,
+                                        int H1, int W1, int radius, int limit) {
+  const int lane = threadIdx.x & 31, h = h0 + lane / L4_BT, x = w0 + lane % L4_BT;
+  const bool in = lane < L4_BPX && h < H1 && x < W1;
+  for (int level = threadIdx.x >> 5; level < levels; level += blockDim.x >> 5) {
+    L4Pixel geo{0.f, 0.f, 0, 0};
+    if (in) geo = l4_pixel_geometry(coords, b, h * W1 + x, H1 * W1, level, lv.H2[level], lv.W2[level]);
+    const L4Box box = l4_box(geo, __ballot_sync(0xffffffffu, in), radius, lane);
+    if (lane < L4_BPX) t.geo[level][lane] = geo;
+    if (lane == 0) t.box[level] = box;
+  }
+  __syncthreads();
+  bool fits = true;
+  for (int level = 0; level < levels; ++level) fits &= l4_fits(t.box[level], limit);
+  return fits;
+}
+
+constexpr int L4_TROW = L4_WIN + 2;             // window rows with a zero before and behind
+
+// A step of four positions where a feature is infinite or NaN: it reaches only what has it under its window.
+template <class Load, class Add>
+__device__ __forceinline__ void l4_nonfinite(const float (*gS)[L4_BPX], const int* rows, int q0, const float (&f1)[L4_BPX], float (&gf1)[L4_BPX],
+                                             Load&& f2_at, Add&& add_at) {
+#pragma unroll 1
+  for (int q = q0; q < q0 + 4; ++q) {
+    const float f = f2_at(rows[q]);
+    float total = 0.f;
+#pragma unroll
+    for (int px = 0; px < L4_BPX; ++px) {
+      const float g = gS[q][px];
+      if (g != 0.f) {
+        gf1[px] = fmaf(g, f, gf1[px]);
+        total = fmaf(g, f1[px], total);
+      }
+    }
+    add_at(rows[q], total);
+  }
+}
+
+// Every CTA walks all levels of its tile, so that gF1 is stored once.  Warp w owns channels 32 (w % groups) .. of the CTA's 256; warps
+// beyond the channels share out the positions.  Bound by FP32 issue: 32 multiply-adds of some 45 instructions per warp and position (packed
+// pairs with three different operands take 3 cycles, no gain over two scalar ones).  With a walk per 2 x 2 pixels, lanes splitting
+// the channels, each walk reduced its own 140 positions of 1 KB into L2: 2 x 55 x 128 pixels at C = 256, four levels, radius 4 took 416 us;
+// 278 now.
+// grid (ceil(W1/4) * ceil(H1/4), ceil(C/256), B)
+__global__ void __launch_bounds__(L4_BTHREADS, 2)
 lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                          const float* __restrict__ gout, float* __restrict__ gF1, int H1, int W1, int C, int radius,
-                         int levels, float scale) {
-  __shared__ float s_gS[L4_WARPS][L4_PX][L4_BMAX];
-  __shared__ float s_g[L4_WIN * L4_WIN][L4_TILE + 1];
-  __shared__ int s_rows[L4_WARPS][L4_BMAX];
-  __shared__ L4Pixel s_geo[L4_WARPS][L4_PX];
+                         int levels, int limit, float scale) {
+  __shared__ L4Tile s_tile;
+  __shared__ __align__(16) float s_gS[L4_BBOX + 4][L4_BPX];     // gradient of (position, pixel), scaled; positions without any are left out
+  __shared__ __align__(16) int s_rows[L4_BBOX + 4];             // their image-2 rows
+  __shared__ float s_t[L4_BPX][L4_SIDE][L4_TROW];               // gradients of a pixel's window, spread along x
+  __shared__ float s_fx[L4_BPX][L4_WIN];                        // l4_fraction of a pixel's window entries
+  __shared__ float s_wy[L4_BPX][L4_SIDE][2];                    // what a position takes along y from the window row above it and its own
+  __shared__ __align__(16) int s_bx[L4_BPX], s_by[L4_BPX];      // of this level, next to one another: four a load
+  __shared__ int s_count[L4_BWARPS];
+  float(*const s_g)[L4_BPX + 1] = reinterpret_cast<float(*)[L4_BPX + 1]>(s_gS);   // output gradients; dead before s_gS is written
+  static_assert(L4_WIN * L4_WIN * (L4_BPX + 1) <= L4_BBOX * L4_BPX, "both uses of s_gS");
+
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.z, N1 = H1 * W1, win = 2 * radius + 1, side = 2 * radius + 2;
+  const int tiles_x = (W1 + L4_BT - 1) / L4_BT;
+  const int h0 = (int)(blockIdx.x / tiles_x) * L4_BT, w0 = (int)(blockIdx.x % tiles_x) * L4_BT;
+  const bool in = lane < L4_BPX && h0 + lane / L4_BT < H1 && w0 + lane % L4_BT < W1;
+  const unsigned mask = __ballot_sync(0xffffffffu, in);
+  const size_t tile = ((size_t)b * N1 + (size_t)h0 * W1 + w0) * C;
+  const int c0 = (int)blockIdx.y * L4_BTHREADS, groups = min(L4_BWARPS, (C - c0 + 31) / 32), sharers = L4_BWARPS / groups;
+  const int c = c0 + w % groups * 32 + lane, share = w / groups;
+  const bool mine = c < C && share < sharers;
+  float f1[L4_BPX], gf1[L4_BPX];
+  bool finite1 = true;
+#pragma unroll
+  for (int px = 0; px < L4_BPX; ++px) {
+    const bool ok = mine && h0 + px / L4_BT < H1 && w0 + px % L4_BT < W1;
+    f1[px] = ok ? __ldg(F1 + tile + ((size_t)(px / L4_BT) * W1 + px % L4_BT) * C + c) : 0.f;
+    finite1 &= isfinite(f1[px]);
+    gf1[px] = 0.f;
+  }
+  if (!l4_tile(s_tile, coords, lv, levels, b, h0, w0, H1, W1, radius, limit)) return;   // lookup4d_backward_apart_kernel does it
+  for (int level = 0; level < levels; ++level) {
+    const int H2 = lv.H2[level], W2 = lv.W2[level];
+    const L4Box box = s_tile.box[level];
+    const int nq = box.bw * box.bh;
+
+    constexpr int PER = (L4_WIN * L4_WIN * L4_BPX + L4_BTHREADS - 1) / L4_BTHREADS;
+    float g[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int i = k * L4_BTHREADS + threadIdx.x, o = i / L4_BPX, h = h0 + i % L4_BPX / L4_BT, x = w0 + i % L4_BT;
+      const bool ok = o < win * win && h < H1 && x < W1;
+      g[k] = ok ? __ldg(gout + (((size_t)b * levels + level) * win * win + o) * N1 + (size_t)h * W1 + x) * scale : 0.f;
+    }
+    __syncthreads();   // the previous level's tables are no longer read
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int i = k * L4_BTHREADS + threadIdx.x;
+      if (i < win * win * L4_BPX) s_g[i / L4_BPX][i % L4_BPX] = g[k];
+    }
+    if (lane < L4_BPX) {   // warp w: window entries w, w + 8, ...
+      const L4Pixel geo = s_tile.geo[level][lane];
+      for (int t = w; t < win; t += L4_BWARPS) {
+        s_fx[lane][t] = l4_fraction(geo.cx, geo.bx, t, radius, W2);
+        const float fy = l4_fraction(geo.cy, geo.by, t, radius, H2);
+        s_wy[lane][t][1] = 1.f - fy;
+        s_wy[lane][t + 1][0] = fy;
+      }
+      if (w == 0) {
+        s_bx[lane] = geo.bx;
+        s_by[lane] = geo.by;
+        s_wy[lane][0][0] = s_wy[lane][win][1] = 0.f;
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < L4_BPX * side * (win + 2); i += L4_BTHREADS) {
+      const int px = i % L4_BPX, r = i / L4_BPX, bb = r % (win + 2) - 1, at = r / (win + 2);   // window row, column of positions
+      float t = 0.f;
+      if (bb >= 0 && bb < win) {
+        if (at < win) t = (1.f - s_fx[px][at]) * s_g[at * win + bb][px];
+        if (at > 0) t = fmaf(s_fx[px][at - 1], s_g[(at - 1) * win + bb][px], t);
+      }
+      s_t[px][at][bb + 1] = t;
+    }
+    __syncthreads();
+    int count = 0;   // positions with a gradient
+    for (int q0 = 0; q0 < nq; q0 += L4_BTHREADS) {
+      const int q = q0 + threadIdx.x, row = q / box.bw, x = box.ox + q - row * box.bw, y = box.oy + row;
+      float v[L4_BPX];
+      bool any = false;
+      if (q < nq && x >= 0 && x < W2 && y >= 0 && y < H2) {
+#pragma unroll
+        for (int px = 0; px < L4_BPX; ++px) {
+          const int i = x - (s_bx[px] - radius), j = y - (s_by[px] - radius);
+          v[px] = 0.f;
+          if (((mask >> px) & 1u) && (unsigned)i < (unsigned)side && (unsigned)j < (unsigned)side)
+            v[px] = fmaf(s_wy[px][j][0], s_t[px][i][j], s_wy[px][j][1] * s_t[px][i][j + 1]);
+          any |= v[px] != 0.f;
+        }
+      }
+      const unsigned with = __ballot_sync(0xffffffffu, any);
+      if (lane == 0) s_count[w] = __popc(with);
+      __syncthreads();
+      int at = count + __popc(with & ((1u << lane) - 1));
+#pragma unroll
+      for (int k = 0; k < L4_BWARPS; ++k) {
+        at += k < w ? s_count[k] : 0;
+        count += s_count[k];
+      }
+      if (any) {
+        s_rows[at] = y * W2 + x;
+#pragma unroll
+        for (int p4 = 0; p4 < L4_BPX; p4 += 4) *reinterpret_cast<float4*>(&s_gS[at][p4]) = make_float4(v[p4], v[p4 + 1], v[p4 + 2], v[p4 + 3]);
+      }
+      __syncthreads();
+    }
+    if (count == 0) continue;
+    // up to a multiple of four: the last position again, with no gradient
+    const int padded = (count + 3) & ~3;
+    if (threadIdx.x < (padded - count) * L4_BPX) s_gS[count + threadIdx.x / L4_BPX][threadIdx.x % L4_BPX] = 0.f;
+    if (threadIdx.x < padded - count) s_rows[count + threadIdx.x] = s_rows[count - 1];
+    __syncthreads();
+    if (!mine) continue;
+
+    // (32-bit factors: the product and the sum are one multiply-add)
+    const char* const F2c = reinterpret_cast<const char*>(lv.f2[level] + (size_t)b * H2 * W2 * C + c);
+    char* const G2c = reinterpret_cast<char*>(lv.g2[level] + (size_t)b * H2 * W2 * C + c);
+    const uint32_t row_bytes = 4 * C;
+    const auto f2_at = [&](int r) { return __ldg(reinterpret_cast<const float*>(F2c + (uint64_t)row_bytes * (uint32_t)r)); };
+    const auto add_at = [&](int r, float v) { atomicAdd(reinterpret_cast<float*>(G2c + (uint64_t)row_bytes * (uint32_t)r), v); };
+    // four positions a step; the next step's rows are requested before this one's are used
+    int next_r[4];
+    float next_f[4];
+    const auto fetch = [&](int q0) {
+      if (q0 >= padded) return;
+      *reinterpret_cast<int4*>(next_r) = *reinterpret_cast<const int4*>(&s_rows[q0]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) next_f[k] = f2_at(next_r[k]);
+    };
+    fetch(share * 4);
+#pragma unroll 2
+    for (int q0 = share * 4; q0 < padded; q0 += sharers * 4) {
+      int r[4];
+      float f[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        r[k] = next_r[k];
+        f[k] = next_f[k];
+      }
+      fetch(q0 + sharers * 4);
+      if (!finite1 || !isfinite((fabsf(f[0]) + fabsf(f[1])) + (fabsf(f[2]) + fabsf(f[3])))) {
+        l4_nonfinite(s_gS, s_rows, q0, f1, gf1, f2_at, add_at);
+        continue;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float g2[4];
+#pragma unroll
+        for (int p4 = 0; p4 < L4_BPX; p4 += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(&s_gS[q0 + k][p4]);
+          const float g[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            gf1[p4 + i] = fmaf(g[i], f[k], gf1[p4 + i]);
+            g2[i] = p4 == 0 ? g[i] * f1[i] : fmaf(g[i], f1[p4 + i], g2[i]);
+          }
+        }
+        add_at(r[k], (g2[0] + g2[1]) + (g2[2] + g2[3]));
+      }
+    }
+  }
+  if (sharers > 1) {   // sum over the warps of the same channels, in their order
+    __syncthreads();
+    if (mine && share > 0) {
+#pragma unroll
+      for (int px = 0; px < L4_BPX; ++px) s_gS[threadIdx.x][px] = gf1[px];
+    }
+    __syncthreads();
+    if (mine && share == 0) {
+      for (int k = 1; k < sharers; ++k)
+#pragma unroll
+        for (int px = 0; px < L4_BPX; ++px) gf1[px] += s_gS[threadIdx.x + k * groups * 32][px];
+    }
+  }
+  if (mine && share == 0) {
+#pragma unroll
+    for (int px = 0; px < L4_BPX; ++px)
+      if (h0 + px / L4_BT < H1 && w0 + px % L4_BT < W1) gF1[tile + ((size_t)(px / L4_BT) * W1 + px % L4_BT) * C + c] = gf1[px];
+  }
+}
+
+// The tiles that the kernel above leaves out: four warps with 2 x 2 pixels each, together at the levels where the box of their windows has at
+// most L4_BMAX positions, else one pixel at a time.  Same grid.
+constexpr int L4_APART = 128, L4_APART_WARPS = L4_APART / 32;
+static_assert(L4_APART_WARPS * L4_PX == L4_BPX, "2 x 2 pixels a warp");
+
+template <int NCH>
+__global__ void __launch_bounds__(L4_APART, 4)
+lookup4d_backward_apart_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
+                               const float* __restrict__ gout, float* __restrict__ gF1, int H1, int W1, int C, int radius,
+                               int levels, int limit, float scale) {
+  __shared__ L4Tile s_tile;
+  __shared__ float s_gS[L4_APART_WARPS][L4_PX][L4_BMAX];
+  __shared__ float s_g[L4_WIN * L4_WIN][L4_BPX + 1];
+  __shared__ int s_rows[L4_APART_WARPS][L4_BMAX];
 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int b = blockIdx.z, N1 = H1 * W1, win = 2 * radius + 1;
-  const int tiles_x = (W1 + L4_TW - 1) / L4_TW;
-  const int h0 = (int)(blockIdx.x / tiles_x) * L4_TH, w0 = (int)(blockIdx.x % tiles_x) * L4_TW;
-  const int ph = h0 + 2 * (w >> 2), pw = w0 + 2 * (w & 3);
+  const int tiles_x = (W1 + L4_BT - 1) / L4_BT;
+  const int h0 = (int)(blockIdx.x / tiles_x) * L4_BT, w0 = (int)(blockIdx.x % tiles_x) * L4_BT;
+  if (l4_tile(s_tile, coords, lv, levels, b, h0, w0, H1, W1, radius, limit)) return;
+  const int ph = h0 + 2 * (w >> 1), pw = w0 + 2 * (w & 1);
   const int mh = ph + ((lane >> 1) & 1), mw = pw + (lane & 1);
   const bool mine = lane < L4_PX && mh < H1 && mw < W1;
   const unsigned mask = __ballot_sync(0xffffffffu, mine);
+  const int px0 = 2 * (w >> 1) * L4_BT + 2 * (w & 1);   // this warp's first pixel of the tile; pixel px: + px/2 rows, + px%2
 
   L4Quad f1[L4_PX][NCH], gf1[L4_PX][NCH];
 #pragma unroll
@@ -412,29 +665,26 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
     float* G2b = lv.g2[level] + (size_t)b * H2 * W2 * C;
 
     __syncthreads();   // the previous level's s_g is no longer read
-    for (int i = threadIdx.x; i < win * win * L4_TILE; i += L4_THREADS) {
-      const int o = i / L4_TILE, pp = i % L4_TILE, h = h0 + pp / L4_TW, x = w0 + pp % L4_TW;
+    for (int i = threadIdx.x; i < win * win * L4_BPX; i += L4_APART) {
+      const int o = i / L4_BPX, pp = i % L4_BPX, h = h0 + pp / L4_BT, x = w0 + pp % L4_BT;
       s_g[o][pp] = (h < H1 && x < W1)
                        ? __ldg(gout + (((size_t)b * levels + level) * win * win + o) * N1 + (size_t)h * W1 + x)
                        : 0.f;
     }
-    L4Pixel geo{0.f, 0.f, 0, 0};
-    if (mine) geo = l4_pixel_geometry(coords, b, mh * W1 + mw, N1, level, H2, W2);
-    if (lane < L4_PX) s_geo[w][lane] = geo;
+    const L4Pixel geo = s_tile.geo[level][px0 + lane / 2 % 2 * L4_BT + lane % 2];
     __syncthreads();
     if (mask == 0) continue;
 
-    const int pp0 = 2 * (w >> 2) * L4_TW + 2 * (w & 3);   // this warp's first pixel in s_g; pixel px: + px/2 rows, + px%2
     const L4Box box = l4_box(geo, mask, radius, lane);
     if (l4_fits(box, L4_BMAX)) {
       l4_fill_rows(s_rows[w], box, H2, W2, lane);
       const int nq = box.bw * box.bh;
       for (int px = 0; px < L4_PX; ++px) {
-        const L4Pixel g = s_geo[w][px];
+        const L4Pixel g = s_tile.geo[level][px0 + px / 2 * L4_BT + px % 2];
         const bool live = (mask >> px) & 1u;
         for (int q = lane; q < nq; q += 32) {
           const int row = q / box.bw, i = box.ox + q - row * box.bw - (g.bx - radius), j = box.oy + row - (g.by - radius);
-          s_gS[w][px][q] = live ? l4_position_gradient(g, i, j, s_g, pp0 + px / 2 * L4_TW + px % 2, radius, H2, W2) * scale : 0.f;
+          s_gS[w][px][q] = live ? l4_position_gradient(g, i, j, s_g, px0 + px / 2 * L4_BT + px % 2, radius, H2, W2) * scale : 0.f;
         }
       }
       __syncwarp();
@@ -442,14 +692,15 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
     } else {
       // motion boundaries: one pixel at a time, each over its own window.  All four pixels' positions are prepared together (a
       // pixel alone leaves lanes idle and waits on its own), a pixel's rows behind its gradients.  Windows scattered over
-      // 2 x 55 x 128 at C = 256, radius 4, four levels: 1121 us with a preparation per pixel, 857 now.
+      // 2 x 55 x 128 at C = 256, radius 4, four levels: 1121 us with a preparation per pixel, 857 with this
+      // one, 1058 against 1117 at uniformly scattered windows with tiles sorted out first.
       const int side = 2 * radius + 2, nq = side * side;
       for (int idx = lane; idx < L4_PX * nq; idx += 32) {
         const int px = idx / nq, q = idx - px * nq, j = q / side, i = q - j * side;
-        const L4Pixel g = s_geo[w][px];
+        const L4Pixel g = s_tile.geo[level][px0 + px / 2 * L4_BT + px % 2];
         const int x = g.bx - radius + i, y = g.by - radius + j;
         const bool live = (mask >> px) & 1u;
-        const float v = live ? l4_position_gradient(g, i, j, s_g, pp0 + px / 2 * L4_TW + px % 2, radius, H2, W2) * scale : 0.f;
+        const float v = live ? l4_position_gradient(g, i, j, s_g, px0 + px / 2 * L4_BT + px % 2, radius, H2, W2) * scale : 0.f;
         s_gS[w][px][q] = v;
         s_gS[w][px][L4_ALONE_ROWS + q] = __int_as_float(x >= 0 && x < W2 && y >= 0 && y < H2 && v != 0.f ? y * W2 + x : -1);
       }
@@ -475,6 +726,13 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
         *reinterpret_cast<ulonglong2*>(gF1 + p * C + c) = make_ulonglong2(gf1[px][ch].lo, gf1[px][ch].hi);
       }
     }
+}
+
+// Zeros for the reductions, all levels in one launch (C is a multiple of 4 and the pointers are 16-byte aligned).
+__global__ void __launch_bounds__(256) lookup4d_clear_kernel(Lookup4dLevels lv, int B, int C) {
+  float4* const p = reinterpret_cast<float4*>(lv.g2[blockIdx.y]);
+  const size_t n = (size_t)B * lv.H2[blockIdx.y] * lv.W2[blockIdx.y] * (C / 4);
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 static Lookup4dLevels make_levels(const Lookup4dDims& d, const float* const* F2, float* const* gF2) {
@@ -512,17 +770,26 @@ cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, cons
   return cudaGetLastError();
 }
 
+int lookup4d_backward_launches(const Lookup4dDims& d) { return l4_tile_limit(d.radius) > 0 ? 3 : 2; }
+
 cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, const float* const* F2,
                                      const float* coords, const float* gout, float* gF1, float* const* gF2,
                                      float scale, cudaStream_t stream) {
-  for (int l = 0; l < d.levels; ++l) {
-    const cudaError_t err =
-        cudaMemsetAsync(gF2[l], 0, (size_t)d.B * d.H2[l] * d.W2[l] * d.C * sizeof(float), stream);
+  const Lookup4dLevels lv = make_levels(d, F2, gF2);
+  size_t largest = 0;
+  for (int l = 0; l < d.levels; ++l) largest = std::max(largest, (size_t)d.B * d.H2[l] * d.W2[l] * (d.C / 4));
+  lookup4d_clear_kernel<<<dim3((unsigned)std::min<size_t>((largest + 1023) / 1024, 148 * 8), d.levels), 256, 0, stream>>>(lv, d.B, d.C);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  const dim3 grid((unsigned)((d.W1 + L4_BT - 1) / L4_BT) * (unsigned)((d.H1 + L4_BT - 1) / L4_BT), 1, d.B);   // per tile
+  const int limit = l4_tile_limit(d.radius);
+  if (limit > 0) {
+    const dim3 whole(grid.x, (unsigned)((d.C + L4_BTHREADS - 1) / L4_BTHREADS), d.B);
+    lookup4d_backward_kernel<<<whole, L4_BTHREADS, 0, stream>>>(F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale);
+    err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
-  const Lookup4dLevels lv = make_levels(d, F2, gF2);
-  const dim3 grid(l4_tiles(d), 1, d.B);
-#define SFB_L4_BWD(NCH) lookup4d_backward_kernel<NCH><<<grid, L4_THREADS, 0, stream>>>(F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, scale)
+#define SFB_L4_BWD(NCH) lookup4d_backward_apart_kernel<NCH><<<grid, L4_APART, 0, stream>>>(F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale)
   switch ((d.C + 127) / 128) {
     case 1: SFB_L4_BWD(1); break;
     case 2: SFB_L4_BWD(2); break;
