@@ -227,9 +227,12 @@ int sfb_separation_level_backward_fmaps(const float* fmap1, const float* fmap2, 
  * (host arrays of `levels` entries; no level larger than level 0), `shape` gives B, H1, W1, C and Kc; the other arguments as
  * above.  SEP_u (B,(2+Kc)*levels,W2[0],H1,W1) and SEP_v (B,(2+Kc)*levels,H2[0],H1,W1) are the concatenated outputs, each level
  * resampled to the displacement range of level 0.  `saved` (256-byte aligned) receives what a backward needs: the levels' own
- * volumes, attention weights and, with_argmax != 0, arg-max indices. */
+ * volumes, attention weights and, with_argmax != 0, arg-max indices.
+ * Image 2's levels may be made here: with fmap2[1..] NULL they are the 2 x 2 averages of one another (core/corr.py:377-382),
+ * `saved` then holds them too (pooled != 0), and a backward with gfmap2[1..] NULL returns the gradient of fmap2[0] alone, with
+ * what its averages contribute. */
 size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
-                                          int32_t with_argmax);
+                                          int32_t with_argmax, int32_t pooled);
 size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
                                               int32_t backward);
 int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,

@@ -125,7 +125,7 @@ def load() -> ctypes.CDLL:
     lib.sfb_separation_level_backward_fmaps.restype = ctypes.c_int
     lib.sfb_separation_level_backward_fmaps.argtypes = [P, P, ctypes.c_float] + [P] * 4 + [I32, I32] + [P] * 12 + tail
     lib.sfb_separation_pyramid_saved_bytes.restype = SZ
-    lib.sfb_separation_pyramid_saved_bytes.argtypes = [SH, P, P, I32, I32]
+    lib.sfb_separation_pyramid_saved_bytes.argtypes = [SH, P, P, I32, I32, I32]
     lib.sfb_separation_pyramid_workspace_bytes.restype = SZ
     lib.sfb_separation_pyramid_workspace_bytes.argtypes = [SH, P, P, I32, I32]
     lib.sfb_separation_pyramid_forward.restype = ctypes.c_int

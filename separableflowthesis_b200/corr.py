@@ -25,7 +25,8 @@ import torch.nn.functional as F
 from .functions import (ComputeMaxArgmaxAvgFunction, ComputeMaxAvgFunction, ComputeSelfCompressionFunction,
                         FusedMaxArgmaxAvgFunction, FusedSelfCompressionFunction, SeparationCompressionCF,
                         Lookup4dFunction, LookupFunction, LookupPairFunction, LookupVolumeFunction,
-                        SeparationLevelFunction, SeparationMaxAvgCF, SeparationPyramidFunction,
+                        SeparationLevelFunction, SeparationMaxAvgCF,
+                        SeparationPooledPyramidFunction, SeparationPyramidFunction,
                         SeparationState)
 from . import ops as _ops
 
@@ -54,11 +55,32 @@ class AlternateCorrBlockSepflow:
         self.num_levels = num_levels
         self.radius = radius
         self.fmap1_l0 = fmap1
-        self.pyramid = [fmap2]
-        for _ in range(num_levels - 1):
-            fmap2 = F.avg_pool2d(fmap2, 2, stride=2)
-            self.pyramid.append(fmap2)
+        self._fmap2, self._pyramid, self._grad_mode = fmap2, None, torch.is_grad_enabled()
+        # the call for all levels makes the pyramid itself; whoever reads it gets the tensors
+        if not (2 <= num_levels <= _ops.PYRAMID_MAX_LEVELS and fmap2.is_cuda and fmap2.dtype == torch.float32 and fmap2.dim() == 4
+                and min(fmap2.shape[2:]) >> (num_levels - 1) >= 1):
+            self._build_pyramid()
         self._channels_last = None
+
+    def _build_pyramid(self):
+        level = self._fmap2
+        levels = [level]
+        with torch.set_grad_enabled(self._grad_mode):   # as the constructor was called
+            for _ in range(self.num_levels - 1):
+                level = F.avg_pool2d(level, 2, stride=2)
+                levels.append(level)
+        self._pyramid = levels
+
+    @property
+    def pyramid(self):
+        """Image 2's feature maps per level, average-pooled (core/corr.py:377-382)."""
+        if self._pyramid is None:
+            self._build_pyramid()
+        return self._pyramid
+
+    @pyramid.setter
+    def pyramid(self, levels):
+        self._pyramid = levels
 
     def _one_node_per_level(self, attention_weights) -> bool:
         return (self.channels_first and self.fuse_backward and self.fuse_attention and attention_weights is not None
@@ -108,6 +130,13 @@ class AlternateCorrBlockSepflow:
         """All levels, each trilinearly resampled to the level-0 displacement range and concatenated
         over channels: sep_u (B, K*levels, W, H, W), sep_v (B, K*levels, H, H, W) (core/corr.py:384-477)."""
         batch, fdim, h1, w1 = self.fmap1_l0.shape
+        if (self._pyramid is None and (self._grad_mode or not torch.is_grad_enabled()) and self.fmap1_l0.is_cuda
+                and self._one_node_per_level(attention_weights)
+                and attention_weights[0].out_channels <= _ops.PYRAMID_MAX_CHANNELS and batch * (2 + attention_weights[0].out_channels) <= 65535):
+            attention1, attention2 = attention_weights
+            return SeparationPooledPyramidFunction.apply(self.support_backward, 1.0 / math.sqrt(fdim), self.num_levels, attention1.weight,
+                                                         attention1.bias, attention2.weight, attention2.bias,
+                                                         self.fmap1_l0.contiguous(), self._fmap2.contiguous())
         h2, w2 = self.pyramid[0].shape[2:]
         if self._one_node_per_level(attention_weights) and self.num_levels > 1:
             # one node for the whole pyramid: levels are resampled along the displacement axis and written into

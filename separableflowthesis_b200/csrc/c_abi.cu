@@ -1488,9 +1488,10 @@ int check_pyramid(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, 
 struct PyramidSaved {
   float *sep_u[MAX_FUSED_LEVELS], *sep_v[MAX_FUSED_LEVELS], *a_u[MAX_FUSED_LEVELS], *a_v[MAX_FUSED_LEVELS];
   int32_t *am_u[MAX_FUSED_LEVELS], *am_v[MAX_FUSED_LEVELS];
+  float* fmap2[MAX_FUSED_LEVELS];   // pooled levels
   size_t bytes;
 };
-PyramidSaved carve_saved(const Pyramid& py, void* base, bool with_argmax) {
+PyramidSaved carve_saved(const Pyramid& py, void* base, bool with_argmax, bool pooled) {
   PyramidSaved v;
   size_t off = 0;
   auto take = [&](size_t floats) {
@@ -1508,6 +1509,7 @@ PyramidSaved carve_saved(const Pyramid& py, void* base, bool with_argmax) {
     v.a_u[l] = take(bn * d.Kc * d.W2);
     v.a_v[l] = take(bn * d.Kc * d.H2);
   }
+  for (int l = 0; l < py.levels; ++l) v.fmap2[l] = pooled && l > 0 ? take((size_t)py.d[l].B * py.d[l].C * py.d[l].N2()) : nullptr;
   v.bytes = off;
   return v;
 }
@@ -1560,10 +1562,10 @@ PyramidWorkspace carve_pyramid_forward(const Pyramid& py, void* base) {
 }
 
 // The backward's: attention gradients, gradients of the max/avg channels, GEMM operands and image 2's copies per level, image 1's shared;
-// the gradients of the level's own volumes (gs_u, gs_v) where it is not in place.
+// the gradients of the level's own volumes (gs_u, gs_v) where it is not in place; those of pooled levels of image 2 (gf2).
 struct PyramidBackward {
   Workspace w[MAX_FUSED_LEVELS];
-  float *gs_u[MAX_FUSED_LEVELS], *gs_v[MAX_FUSED_LEVELS];
+  float *gs_u[MAX_FUSED_LEVELS], *gs_v[MAX_FUSED_LEVELS], *gf2[MAX_FUSED_LEVELS];
   int samples;             // whose G of all levels is stored at a time (0: none)
   size_t bytes;            // without the stored G, which a caller's buffer may lack
   size_t stored_bytes;
@@ -1605,6 +1607,7 @@ PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
     w.gm_v = take(bn * 2 * d.H2);
     p.gs_u[l] = py.in_place[l] ? nullptr : take(bn * Kt * d.W2);
     p.gs_v[l] = py.in_place[l] ? nullptr : take(bn * Kt * d.H2);
+    p.gf2[l] = l == 0 ? nullptr : take((size_t)d.B * d.C * d.N2());
     at[2 * l] = AttentionDims{d.B, d.Kc, d.W2, d.H1, d.W1};
     at[2 * l + 1] = AttentionDims{d.B, d.Kc, d.H2, d.H1, d.W1};
   }
@@ -1675,16 +1678,32 @@ int run_pyramid_sweeps(const Pyramid& py, const Workspace* w, int op16, int mode
 }
 
 // Operand copies of all levels (and the mean rows of image 2 when with_aux).
-int prepare_pyramid(const Pyramid& py, const Workspace* w, const float* fmap1, const float* const* fmap2, float scale1, bool with_aux,
-                    int op16, cudaStream_t st) {
+int prepare_pyramid(const Pyramid& py, const Workspace* w, const float* fmap1, const float* const* fmap2, float* const* pooled, float scale1,
+                    bool with_aux, int op16, cudaStream_t st) {
   LevelOperands out[MAX_FUSED_LEVELS];
   for (int l = 0; l < py.levels; ++l)
     out[l] = op16 ? LevelOperands{nullptr, nullptr, w[l].F2h, with_aux ? w[l].auxh : nullptr}
                   : LevelOperands{w[l].F2r, with_aux ? w[l].aux : nullptr, nullptr, nullptr};
-  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w[0], with_aux, op16), st, [&] {
+  const int launches = prepare_launches(w[0], with_aux, op16) + (pooled != nullptr && op16 != OP16_FP16 ? 1 : 0);
+  SFB_CUDA(timed(KID_PREPARE, launches, st, [&] {
     return launch_prepare_cf(py.d, py.levels, fmap1, fmap2, scale1, out, op16 ? nullptr : w[0].F1r, op16 ? w[0].F1h : nullptr, w[0].status,
-                             st, op16, w[0].scales);
+                             st, op16, w[0].scales, pooled);
   }));
+  return SFB_OK;
+}
+
+// Image 2's levels as the caller gives them: all, or the first alone (the others NULL), which are then its 2 x 2 averages.
+int check_levels(const Pyramid& py, const void* const* fmap2, const char* name, bool* pooled) {
+  *pooled = py.levels > 1 && fmap2[1] == nullptr;
+  for (int l = 0; l < py.levels; ++l) {
+    if (*pooled && l > 0) {
+      if (fmap2[l] != nullptr) return fail(SFB_ERR_INVALID_ARGUMENT, "%s: all levels from the second on must be NULL or none", name);
+      if (py.d[l].H2 != py.d[l - 1].H2 / 2 || py.d[l].W2 != py.d[l - 1].W2 / 2)
+        return fail(SFB_ERR_INVALID_ARGUMENT, "%s: level %d is not half of the level before", name, l);
+      continue;
+    }
+    SFB_TRY(check_ptr(fmap2[l], name));
+  }
   return SFB_OK;
 }
 
@@ -1707,10 +1726,10 @@ PixView volume_view(float* base, long long sb, int channel, int D, int N1) {
 extern "C" {
 
 size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
-                                          int32_t with_argmax) {
+                                          int32_t with_argmax, int32_t pooled) {
   Pyramid py;
   if (check_pyramid(shape, H2, W2, levels, &py) != SFB_OK) return 0;
-  return carve_saved(py, nullptr, with_argmax != 0).bytes;
+  return carve_saved(py, nullptr, with_argmax != 0, pooled != 0).bytes;
 }
 
 size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
@@ -1729,11 +1748,13 @@ int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2
                                    size_t workspace_bytes, void* stream) {
   Pyramid py;
   SFB_TRY(check_pyramid(shape, H2, W2, levels, &py));
-  SFB_CHECK_PTR(fmap1); SFB_CHECK_PTR(fmap2); SFB_CHECK_PTR(SEP_u); SFB_CHECK_PTR(SEP_v); SFB_CHECK_PTR(saved);
-  for (int l = 0; l < levels; ++l) SFB_CHECK_PTR(fmap2[l]);
+  SFB_CHECK_PTR(fmap1); SFB_CHECK_PTR(SEP_u); SFB_CHECK_PTR(SEP_v); SFB_CHECK_PTR(saved);
+  if (fmap2 == nullptr) return fail(SFB_ERR_INVALID_ARGUMENT, "fmap2 is NULL");
+  bool pooled;
+  SFB_TRY(check_levels(py, reinterpret_cast<const void* const*>(fmap2), "fmap2", &pooled));
   if (weight_u == nullptr || bias_u == nullptr || weight_v == nullptr || bias_v == nullptr)
     return fail(SFB_ERR_INVALID_ARGUMENT, "attention weights and biases must not be NULL");
-  const PyramidSaved sv = carve_saved(py, saved, with_argmax != 0);
+  const PyramidSaved sv = carve_saved(py, saved, with_argmax != 0, pooled);
   if (saved_bytes < sv.bytes) return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "saved has %zu bytes, %zu needed", saved_bytes, sv.bytes);
   if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return fail(SFB_ERR_INVALID_ARGUMENT, "workspace is NULL or not 256-byte aligned");
@@ -1744,7 +1765,9 @@ int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d0, &op16));
-  SFB_TRY(prepare_pyramid(py, pw.w, fmap1, fmap2, scale1, true, op16, st));
+  const float* maps2[MAX_FUSED_LEVELS];
+  for (int l = 0; l < levels; ++l) maps2[l] = pooled && l > 0 ? sv.fmap2[l] : fmap2[l];
+  SFB_TRY(prepare_pyramid(py, pw.w, fmap1, maps2, pooled ? sv.fmap2 : nullptr, scale1, true, op16, st));
   const int N1 = d0.N1(), K = d0.Kc, Kt = 2 + K;
   LevelVolumes vol[MAX_FUSED_LEVELS];
   for (int l = 0; l < levels; ++l) vol[l] = level_volumes(py, l, SEP_u, SEP_v, sv.sep_u[l], sv.sep_v[l]);
@@ -1791,13 +1814,17 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
                                     const sfb_shape* shape, void* workspace, size_t workspace_bytes, void* stream) {
   Pyramid py;
   SFB_TRY(check_pyramid(shape, H2, W2, levels, &py));
-  SFB_CHECK_PTR(fmap1); SFB_CHECK_PTR(fmap2); SFB_CHECK_PTR(SEP_u); SFB_CHECK_PTR(SEP_v); SFB_CHECK_PTR(saved);
-  SFB_CHECK_PTR(gSEP_u); SFB_CHECK_PTR(gSEP_v); SFB_CHECK_PTR(gfmap1); SFB_CHECK_PTR(gfmap2);
-  for (int l = 0; l < levels; ++l) { SFB_CHECK_PTR(fmap2[l]); SFB_CHECK_PTR(gfmap2[l]); }
+  SFB_CHECK_PTR(fmap1); SFB_CHECK_PTR(SEP_u); SFB_CHECK_PTR(SEP_v); SFB_CHECK_PTR(saved);
+  SFB_CHECK_PTR(gSEP_u); SFB_CHECK_PTR(gSEP_v); SFB_CHECK_PTR(gfmap1);
+  if (fmap2 == nullptr || gfmap2 == nullptr) return fail(SFB_ERR_INVALID_ARGUMENT, "fmap2 and gfmap2 must not be NULL");
+  bool pooled, grads_pooled;
+  SFB_TRY(check_levels(py, reinterpret_cast<const void* const*>(fmap2), "fmap2", &pooled));
+  SFB_TRY(check_levels(py, reinterpret_cast<const void* const*>(gfmap2), "gfmap2", &grads_pooled));
+  if (pooled != grads_pooled) return fail(SFB_ERR_INVALID_ARGUMENT, "fmap2 and gfmap2 must both have all levels or both the first alone");
   if (weight_u == nullptr || weight_v == nullptr || gweight_u == nullptr || gbias_u == nullptr || gweight_v == nullptr ||
       gbias_v == nullptr)
     return fail(SFB_ERR_INVALID_ARGUMENT, "attention weights and their gradient buffers must not be NULL");
-  const PyramidSaved sv = carve_saved(py, const_cast<void*>(saved), true);
+  const PyramidSaved sv = carve_saved(py, const_cast<void*>(saved), true, pooled);
   if (saved_bytes < sv.bytes) return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "saved has %zu bytes, %zu needed", saved_bytes, sv.bytes);
   if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return fail(SFB_ERR_INVALID_ARGUMENT, "workspace is NULL or not 256-byte aligned");
@@ -1809,7 +1836,13 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int op16;
   SFB_TRY(operand_mode(d0, &op16));
-  SFB_TRY(prepare_pyramid(py, w, fmap1, fmap2, scale1, false, op16, st));
+  const float* maps2[MAX_FUSED_LEVELS];
+  float* grads2[MAX_FUSED_LEVELS];
+  for (int l = 0; l < levels; ++l) {
+    maps2[l] = pooled && l > 0 ? sv.fmap2[l] : fmap2[l];
+    grads2[l] = pooled && l > 0 ? pb.gf2[l] : gfmap2[l];
+  }
+  SFB_TRY(prepare_pyramid(py, w, fmap1, maps2, nullptr, scale1, false, op16, st));
   const int N1 = d0.N1(), K = d0.Kc, Kt = 2 + K;
   const size_t bn = (size_t)d0.B * N1;
   float *const SU = const_cast<float*>(SEP_u), *const SV = const_cast<float*>(SEP_v);
@@ -1884,7 +1917,7 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
                           gs, gK, g0);
     groups.add(su, w[l].gxu, d.H2, 4 * Qc, Q, 1);
     groups.add(sv2, w[l].gxv, d.W2, 4 * Qc, Q, 1);
-    copies[1 + l] = f2_copy(d, w[l], fmap2[l], op16);
+    copies[1 + l] = f2_copy(d, w[l], maps2[l], op16);
   }
   SFB_CUDA(timed(KID_PACK, pack_launches(groups.count, d0.B), st, [&] { return launch_pack_interleaved_cf(groups, d0.B, N1, w[0].n1p, st); }));
   SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_channel_major_cf(copies, 1 + levels, d0.B, d0.C, op16, st); }));
@@ -1904,7 +1937,7 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
       float* part = w[0].part;
       int part0 = -1, launches = 1;
       for (int l = 0; l < levels; ++l) {
-        SFB_TRY(grad_arguments(py.d[l], w[l], op16, GRAD_FUSED, 4 * Q, form, image2_major ? gfmap2[l] : gfmap1, 1, scale1, &a[l], &maps.y[l],
+        SFB_TRY(grad_arguments(py.d[l], w[l], op16, GRAD_FUSED, 4 * Q, form, image2_major ? grads2[l] : gfmap1, 1, scale1, &a[l], &maps.y[l],
                                &maps.xu[l], &maps.xv[l]));
         a[l].d = d[l];
         a[l].b0 = b0;
@@ -1921,6 +1954,8 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
       SFB_CUDA(timed(KID_GRAD_FUSED_IMG1 + (image2_major ? 1 : 0), launches, st, [&] { return launch_grad_gemm(a, levels, maps, st); }));
     }
   }
+  if (pooled)
+    SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_unpool_levels(py.d, levels, gfmap2[0], grads2, st); }));
   return SFB_OK;
 }
 

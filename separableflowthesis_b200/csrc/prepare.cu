@@ -104,6 +104,194 @@ absmax_kernel(const __grid_constant__ AbsmaxJobs jobs, float* scales, int levels
   *ticket = 0;
 }
 
+// The coarser levels of image 2, each the 2 x 2 average of the one before (core/corr.py:377-382, in avg_pool2d's order of additions), and
+// with FP16 operands the magnitudes of all levels and of image 1 and the multipliers that follow, in one launch: one walk over both images
+// in place of a launch per level and one over all of them.  A thread makes what 8 x 8 pixels of a plane contribute, so that no level
+// is read back.  HBM-bound.  1 x 55 x 128, C = 256, three levels from one: 23 us in four launches (averages and magnitudes), 9 now.
+// grid: blocks of 256 of the planes' 8 x 8 regions, then those of image 1; block 256.
+struct PoolJob {
+  const float* in;              // (planes, H, W)
+  float* out[MAX_FUSED_LEVELS - 1];
+  int planes, H, W, levels;     // levels made here
+  const float* image1;
+  size_t n1;
+  float premul1;
+  int blocks2;                  // blocks of image 2
+};
+static_assert(MAX_FUSED_LEVELS == 4, "8 x 8 pixels are one of the coarsest level");
+template <bool VEC, bool MAGNITUDES>
+__global__ void __launch_bounds__(AM_THREADS)
+pool_levels_kernel(const __grid_constant__ PoolJob job, float* scales) {
+  constexpr int SLOTS = MAX_FUSED_LEVELS + 1;   // magnitudes of the levels of image 2, of image 1
+  float m[SLOTS];
+#pragma unroll
+  for (int i = 0; i < SLOTS; ++i) m[i] = 0.f;
+  if ((int)blockIdx.x < job.blocks2) {
+    const int H = job.H, W = job.W, rw = (W + 7) / 8, rh = (H + 7) / 8;
+    const long long i = (long long)blockIdx.x * AM_THREADS + threadIdx.x;
+    const int plane = (int)(i / (rw * rh)), r = (int)(i - (long long)plane * (rw * rh)), ry = r / rw, rx = r - ry * rw;
+    if (plane < job.planes) {
+      const float* in = job.in + (size_t)plane * H * W + rx * 8;
+      float fine[2][8], mid[2][4], top[2][2];   // rows of level 0, 1 and 2 that make a row of the next
+      // one row of a level from two of the one before; stored where it exists
+      auto next = [&](int l, int y, const float* upper, const float* lower, float* out, int n, float& most) {
+        const int h = H >> l, w = W >> l, x0 = rx * n;
+        float* dst = l <= job.levels ? job.out[l - 1] + ((size_t)plane * h + y) * w + x0 : nullptr;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (j >= n) break;
+          out[j] = (((upper[2 * j] + upper[2 * j + 1]) + lower[2 * j]) + lower[2 * j + 1]) * 0.25f;
+          if (dst != nullptr && y < h && x0 + j < w) {
+            dst[j] = out[j];
+            if (MAGNITUDES) most = fmaxf(most, fabsf(out[j]));
+          }
+        }
+      };
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int y = ry * 8 + 2 * q + k;
+          const float* row = in + (size_t)y * W;
+          if constexpr (VEC) {
+#pragma unroll
+            for (int c = 0; c < 8; c += 4) {
+              const float4 v = y < H && rx * 8 + c < W ? __ldg(reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              fine[k][c] = v.x; fine[k][c + 1] = v.y; fine[k][c + 2] = v.z; fine[k][c + 3] = v.w;
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) fine[k][c] = y < H && rx * 8 + c < W ? __ldg(row + c) : 0.f;
+          }
+          if (MAGNITUDES) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) m[0] = fmaxf(m[0], fabsf(fine[k][c]));
+          }
+        }
+        next(1, ry * 4 + q, fine[0], fine[1], mid[q & 1], 4, m[1]);
+        if (q & 1) next(2, ry * 2 + q / 2, mid[0], mid[1], top[q / 2], 2, m[2]);
+      }
+      float last[1];
+      next(3, ry, top[0], top[1], last, 1, m[3]);
+    }
+  } else if (MAGNITUDES) {
+    const float4* x4 = reinterpret_cast<const float4*>(job.image1);   // 16-byte aligned
+    const size_t n4 = job.n1 / 4, stride = (size_t)(gridDim.x - job.blocks2) * AM_THREADS;
+    const size_t at = (size_t)(blockIdx.x - job.blocks2) * AM_THREADS + threadIdx.x;
+    for (size_t i = at; i < n4; i += AM_UNROLL * stride) {
+      float4 v[AM_UNROLL];
+#pragma unroll
+      for (int j = 0; j < AM_UNROLL; ++j) v[j] = i + j * stride < n4 ? __ldg(x4 + i + j * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < AM_UNROLL; ++j)
+        m[SLOTS - 1] = fmaxf(m[SLOTS - 1], fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+    }
+    if (at < job.n1 - 4 * n4) m[SLOTS - 1] = fmaxf(m[SLOTS - 1], fabsf(__ldg(job.image1 + 4 * n4 + at)));
+  }
+  if constexpr (MAGNITUDES) {
+    __shared__ float red[AM_THREADS / 32][SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m[s] = fmaxf(m[s], __shfl_xor_sync(0xffffffffu, m[s], o));
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][s] = m[s];
+    }
+    __syncthreads();
+    if (threadIdx.x < SLOTS) {
+      const int s = threadIdx.x;
+      float most = red[0][s];
+#pragma unroll
+      for (int i = 1; i < AM_THREADS / 32; ++i) most = fmaxf(most, red[i][s]);
+      if (s == SLOTS - 1) most *= fabsf(job.premul1);
+      const int slot = s == SLOTS - 1 ? SCALE_AMAX_F1 : s * SCALE_LEVEL + SCALE_AMAX_F2;
+      if (most > 0.f) atomicMax(reinterpret_cast<unsigned*>(scales) + slot, __float_as_uint(most));
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    unsigned* ticket = reinterpret_cast<unsigned*>(scales) + SCALE_TICKET;
+    if (atomicAdd(ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    for (int l = 0; l <= job.levels; ++l) feature_scales(scales + l * SCALE_LEVEL, scales + SCALE_AMAX_F1);
+    *ticket = 0;
+  }
+}
+
+static cudaError_t launch_pool_levels(const Dims* d, int levels, const float* fmap1, const float* fmap2, float* const* pooled,
+                                      float premul1, bool magnitudes, float* scales, cudaStream_t stream) {
+  PoolJob job{};
+  job.in = fmap2;
+  for (int l = 1; l < levels; ++l) job.out[l - 1] = pooled[l];
+  job.planes = d[0].B * d[0].C;
+  job.H = d[0].H2;
+  job.W = d[0].W2;
+  job.levels = levels - 1;
+  job.image1 = fmap1;
+  job.n1 = (size_t)d[0].B * d[0].N1() * d[0].C;
+  job.premul1 = premul1;
+  const long long regions = (long long)job.planes * ((job.H + 7) / 8) * ((job.W + 7) / 8);
+  const long long blocks2 = (regions + AM_THREADS - 1) / AM_THREADS;
+  const size_t per_block = (size_t)AM_THREADS * 4 * AM_UNROLL;
+  const long long blocks1 = magnitudes ? (long long)std::max<size_t>(1, std::min<size_t>((job.n1 + per_block - 1) / per_block, 148 * 8)) : 0;
+  if (blocks1 + blocks2 > INT_MAX) return cudaErrorInvalidConfiguration;
+  job.blocks2 = (int)blocks2;
+  const bool vec = job.W % 4 == 0;
+  auto kern = magnitudes ? (vec ? pool_levels_kernel<true, true> : pool_levels_kernel<false, true>)
+                         : (vec ? pool_levels_kernel<true, false> : pool_levels_kernel<false, false>);
+  kern<<<(unsigned)(blocks1 + blocks2), AM_THREADS, 0, stream>>>(job, scales);
+  return cudaGetLastError();
+}
+
+// Gradient of image 2 from those of its pooled levels, in place on level 0's: every level's gradient spreads evenly over the 2 x 2 entries
+// it averaged, the coarsest first, as the chain of avg_pool2d's adjoints adds them up.  Four neighbouring columns a thread.
+// grid (ceil(ceil(W/4) * H / 256), planes), block 256.
+struct UnpoolJob {
+  float* g0;
+  const float* g[MAX_FUSED_LEVELS - 1];
+  int H, W, levels;
+};
+__global__ void __launch_bounds__(256)
+unpool_levels_kernel(const __grid_constant__ UnpoolJob job) {
+  const int H = job.H, W = job.W, quads = (W + 3) / 4;
+  const int i = blockIdx.x * 256 + threadIdx.x, y = i / quads, x0 = (i - y * quads) * 4;
+  if (y >= H) return;
+  const size_t plane = blockIdx.y;
+  float add[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int l = job.levels; l >= 1; --l) {
+    const int h = H >> l, w = W >> l;
+    const float* g = job.g[l - 1] + (plane * h + (y >> l)) * w;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int x = (x0 + j) >> l;
+      // (an entry that the floor of an odd size drops has no parent at this level, and what it would have had of a coarser one
+      // does not exist either)
+      add[j] = (y >> l) < h && x < w ? (__ldg(g + x) + add[j]) * 0.25f : 0.f;
+    }
+  }
+  float* dst = job.g0 + (plane * H + y) * W + x0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (x0 + j < W) dst[j] += add[j];
+}
+cudaError_t launch_unpool_levels(const Dims* d, int levels, float* g0, const float* const* g, cudaStream_t stream) {
+  UnpoolJob job{};
+  job.g0 = g0;
+  for (int l = 1; l < levels; ++l) job.g[l - 1] = g[l];
+  job.H = d[0].H2;
+  job.W = d[0].W2;
+  job.levels = levels - 1;
+  const int quads = (job.W + 3) / 4;
+  const long long planes = (long long)d[0].B * d[0].C;
+  for (long long p0 = 0; p0 < planes; p0 += 65535) {
+    const unsigned n = (unsigned)std::min<long long>(planes - p0, 65535);
+    unpool_levels_kernel<<<dim3((unsigned)(((long long)quads * job.H + 255) / 256), n), 256, 0, stream>>>(job);
+    if (cudaError_t err = cudaGetLastError(); err != cudaSuccess) return err;
+    job.g0 += (size_t)n * d[0].N2();
+    for (int l = 1; l < levels; ++l) job.g[l - 1] += (size_t)n * d[l].N2();
+  }
+  return cudaSuccess;
+}
+
 cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int levels, bool gradients, cudaStream_t stream) {
   if (count < 1 || count > ABSMAX_MAX) return cudaErrorInvalidValue;
   AbsmaxJobs jobs;
@@ -628,10 +816,13 @@ cudaError_t launch_channel_major(const MapCopy& c1, const MapCopy& c2, int B, in
   return cudaGetLastError();
 }
 
+static cudaError_t clear_header(int levels, int* status, cudaStream_t stream) {
+  return cudaMemsetAsync(status, 0, WS_SCALES_OFFSET + (size_t)levels * SCALE_LEVEL * sizeof(float), stream);
+}
 // Clears the workspace header (status word, scale slots) and, for FP16 operands, finds the feature scales.
 static cudaError_t begin_prepare(const Dims* d, int levels, const float* F1, const float* const* F2, float premul1, int* status, int op16,
                                  float* scales, cudaStream_t stream) {
-  cudaError_t err = cudaMemsetAsync(status, 0, WS_SCALES_OFFSET + (size_t)levels * SCALE_LEVEL * sizeof(float), stream);
+  cudaError_t err = clear_header(levels, status, stream);
   if (err != cudaSuccess || op16 != OP16_FP16 || scales == nullptr) return err;
   AbsmaxSource src[1 + MAX_FUSED_LEVELS];
   src[0] = absmax_array(F1, (size_t)d[0].B * d[0].N1() * d[0].C, premul1, SCALE_AMAX_F1);
@@ -641,9 +832,16 @@ static cudaError_t begin_prepare(const Dims* d, int levels, const float* F1, con
 }
 
 cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, const float* const* fmap2, float scale1,
-                              const LevelOperands* out, float* F1r, uint16_t* F1h, int* status, cudaStream_t stream, int op16, float* scales) {
+                              const LevelOperands* out, float* F1r, uint16_t* F1h, int* status, cudaStream_t stream, int op16, float* scales,
+                              float* const* pooled) {
   if (levels < 1 || levels > MAX_FUSED_LEVELS) return cudaErrorInvalidValue;
-  cudaError_t err = begin_prepare(d, levels, fmap1, fmap2, scale1, status, op16, scales, stream);
+  cudaError_t err;
+  if (pooled != nullptr) {
+    err = clear_header(levels, status, stream);
+    if (err == cudaSuccess) err = launch_pool_levels(d, levels, fmap1, fmap2[0], pooled, scale1, op16 == OP16_FP16 && scales != nullptr, scales, stream);
+  } else {
+    err = begin_prepare(d, levels, fmap1, fmap2, scale1, status, op16, scales, stream);
+  }
   if (err != cudaSuccess) return err;
   const bool scaled = op16 == OP16_FP16 && scales != nullptr;
   const int B = d[0].B, C = d[0].C;

@@ -336,6 +336,33 @@ class SeparationPyramidFunction(Function):
         return (None, None, gw_u, gb_u, gw_v, gb_v, g1, *g2)
 
 
+class SeparationPooledPyramidFunction(Function):
+    """The same with the pyramid of image 2 made by the library from its first level: ``apply(with_argmax, scale1, levels, weight_u,
+    bias_u, weight_v, bias_v, fmap1, fmap2)`` on CUDA maps, 2 to 4 levels."""
+
+    @staticmethod
+    def forward(ctx, with_argmax, scale1, levels, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2):
+        params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
+        ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, levels
+        with torch.cuda.device_of(fmap1):
+            sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, [fmap2], *params, with_argmax, scale1, levels)
+        if with_argmax:
+            ctx.save_for_backward(fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, buffer)
+        return sep_u, sep_v
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, grad_sep_u, grad_sep_v):
+        if not ctx.with_argmax:
+            raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
+        fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, buffer = ctx.saved_tensors
+        with torch.cuda.device_of(grad_sep_u):
+            g1, (g2,), gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(
+                fmap1, [fmap2], weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, buffer, grad_sep_u.contiguous(),
+                grad_sep_v.contiguous(), ctx.scale1, ctx.levels)
+        return None, None, None, gw_u, gb_u, gw_v, gb_v, g1, g2
+
+
 # --------------------------------------------------------------------------------------------------
 # Lookup on one aggregated 3D volume (CorrBlock1D, core/corr.py:576-594).  The volume's pyramid is passed in so that
 # it is built once per volume, not once per refinement iteration.  No gradient for the coordinates: the model

@@ -496,32 +496,44 @@ def separation_level_backward(img1_features_l0, img2_features_lk, weight_u, weig
 PYRAMID_MAX_LEVELS, PYRAMID_MAX_CHANNELS = 4, 4
 
 
-def _pyramid_arrays(fmap2_levels):
-    n = len(fmap2_levels)
-    ptrs = (ctypes.c_void_p * n)(*[t.data_ptr() for t in fmap2_levels])
-    sizes = (ctypes.c_int32 * (2 * n))(*[t.shape[2] for t in fmap2_levels], *[t.shape[3] for t in fmap2_levels])
-    return ptrs, ctypes.addressof(sizes), ctypes.addressof(sizes) + 4 * n, sizes
+def _pyramid_arrays(maps, levels):
+    """Host arrays of an entry point: pointers (NULL for the levels that the library pools itself), heights, widths."""
+    H, W = maps[0].shape[2:]
+    sizes = [t.shape[2:] for t in maps] + [(H >> l, W >> l) for l in range(len(maps), levels)]
+    ptrs = (ctypes.c_void_p * levels)(*[t.data_ptr() for t in maps])
+    sizes = (ctypes.c_int32 * (2 * levels))(*[h for h, _ in sizes], *[w for _, w in sizes])
+    return ptrs, ctypes.addressof(sizes), ctypes.addressof(sizes) + 4 * levels, sizes
 
 
-def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, bias_v, with_argmax, scale1):
-    """(sep_u, sep_v, saved): separation_level_forward of every level on the model's feature maps, resampled to the displacement range
-    of level 0 and concatenated; `saved` is what the backward needs beside the inputs and outputs (one flat buffer)."""
+def _check_pyramid(fmap1, fmap2_levels, levels):
+    """Shape of a pyramid call.  fmap2_levels: all levels of image 2, or the first alone with the number of `levels`."""
     s = None
     for f2 in fmap2_levels:
         level = _check_fmaps(fmap1, f2)
         s = s or level
+    if levels != len(fmap2_levels) and (len(fmap2_levels) != 1 or min(s.H2, s.W2) >> (levels - 1) < 1):
+        raise RuntimeError(f"{len(fmap2_levels)} maps given for {levels} levels of at least one pixel")
+    return s
+
+
+def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, bias_v, with_argmax, scale1, levels=None):
+    """(sep_u, sep_v, saved): separation_level_forward of every level on the model's feature maps, resampled to the displacement range
+    of level 0 and concatenated; `saved` is what the backward needs beside the inputs and outputs (one flat buffer).  With one map and the
+    number of `levels`, the others are its 2 x 2 averages, made by the library."""
+    L = levels or len(fmap2_levels)
+    s = _check_pyramid(fmap1, fmap2_levels, L)
     dev = fmap1.device
     s.Kc = _check_attention_params(weight_u, bias_u, "attention1", dev)
     if _check_attention_params(weight_v, bias_v, "attention2", dev) != s.Kc:
         raise RuntimeError("attention1 and attention2 must have the same number of output channels")
-    L = len(fmap2_levels)
     Kt = (2 + s.Kc) * L
     sep_u = torch.empty(s.B, Kt, s.W2, s.H1, s.W1, dtype=torch.float32, device=dev)
     sep_v = torch.empty(s.B, Kt, s.H2, s.H1, s.W1, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels)
-    shape = ctypes.byref(s)
-    saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax)), 256), dtype=torch.uint8, device=dev)
+    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L)
+    shape, pooled = ctypes.byref(s), int(L != len(fmap2_levels))
+    saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax), pooled), 256), dtype=torch.uint8,
+                        device=dev)
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
         ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, 0), 256), dev, stream)
@@ -533,18 +545,16 @@ def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, 
     return sep_u, sep_v, saved
 
 
-def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, g_sep_u, g_sep_v, scale1):
-    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max."""
-    s = None
-    for f2 in fmap2_levels:
-        level = _check_fmaps(fmap1, f2)
-        s = s or level
+def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, g_sep_u, g_sep_v, scale1, levels=None):
+    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max; with pooled levels
+    the gradient of the one map."""
+    L = levels or len(fmap2_levels)
+    s = _check_pyramid(fmap1, fmap2_levels, L)
     dev = fmap1.device
     _check(weight_u, "attention1.weight", torch.float32, 5)
     s.Kc = weight_u.shape[0]
     _check_like(weight_u, "attention1.weight", (s.Kc, 2, 3, 3, 3), torch.float32, dev)
     _check_like(weight_v, "attention2.weight", (s.Kc, 2, 3, 3, 3), torch.float32, dev)
-    L = len(fmap2_levels)
     Kt = (2 + s.Kc) * L
     for t, name, D in ((sep_u, "sep_u", s.W2), (sep_v, "sep_v", s.H2), (g_sep_u, "grad_sep_u", s.W2), (g_sep_v, "grad_sep_v", s.H2)):
         _check_like(t, name, (s.B, Kt, D, s.H1, s.W1), torch.float32, dev)
@@ -555,7 +565,7 @@ def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, 
     gb_u = torch.empty(s.Kc, dtype=torch.float32, device=dev)
     gb_v = torch.empty(s.Kc, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels)
+    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L)
     gptrs = (ctypes.c_void_p * L)(*[t.data_ptr() for t in gF2])
     shape = ctypes.byref(s)
     with torch.cuda.device(dev):

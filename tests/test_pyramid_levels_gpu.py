@@ -102,3 +102,45 @@ def test_backward(shape, operands, cuda_device):
     # a softmax does not see its bias: those gradients are rounding
     assert relerr(gp[0], refp[0]) < TOL and relerr(gp[2], refp[2]) < TOL
     assert torch.equal(again[0], g1) and all(torch.equal(x, y) for x, y in zip(again[1], g2)) and all(torch.equal(x, y) for x, y in zip(again[2:], gp))
+
+
+# One batch with an odd side at every level, one whose planes are not read 16 bytes at a time, one that ends inside an 8 x 8 region
+@pytest.mark.parametrize("operands", ["fp16", "tf32"])
+@pytest.mark.parametrize("shape", SHAPES + [(1, 32, 15, 23, 1, 4), (2, 32, 9, 13, 2, 3), (1, 64, 31, 60, 2, 4)])
+def test_pooled_levels(shape, operands, cuda_device):
+    """The pyramid made by the library is avg_pool2d's, bit for bit, and its gradient that of the chain of avg_pool2d."""
+    B, C, H, W, Kc, levels = shape
+    f1, pyr, params = inputs(B, C, H, W, Kc, levels, H + W, cuda_device)
+    scale1, Kt = 1 / math.sqrt(C), 2 + Kc
+    gen = torch.Generator().manual_seed(4)
+    gu = torch.randn(B, Kt * levels, W, H, W, generator=gen).to(cuda_device)
+    gv = torch.randn(B, Kt * levels, H, H, W, generator=gen).to(cuda_device)
+    with ops.sweep_operands(operands):
+        sep_u, sep_v, buffer = ops.separation_pyramid_forward(f1, pyr[:1], *params, True, scale1, levels)
+        ref_u, ref_v, ref_buffer = ops.separation_pyramid_forward(f1, pyr, *params, True, scale1)
+        assert torch.equal(sep_u, ref_u) and torch.equal(sep_v, ref_v)
+        g1, (g2,), *gp = ops.separation_pyramid_backward(f1, pyr[:1], params[0], params[2], sep_u, sep_v, buffer, gu, gv, scale1, levels)
+        r1, r2, *rp = ops.separation_pyramid_backward(f1, pyr, params[0], params[2], ref_u, ref_v, ref_buffer, gu, gv, scale1)
+    assert torch.equal(g1, r1) and all(torch.equal(x, y) for x, y in zip(gp, rp))
+    f2 = pyr[0].clone().requires_grad_(True)
+    chain = [f2]
+    for _ in range(levels - 1):
+        chain.append(F.avg_pool2d(chain[-1], 2, stride=2))
+    (ref2,) = torch.autograd.grad(chain, f2, r2)
+    assert relerr(g2, ref2) < 1e-6   # the same additions, in an order of autograd's choice
+
+
+def test_block_pyramid_on_demand(cuda_device):
+    """A block makes its pyramid when it is read, with the grad mode it was made in."""
+    import separableflowthesis_b200 as sfb
+    f1, pyr, _ = inputs(1, 32, 16, 24, 2, 3, 1, cuda_device)
+    f2 = pyr[0].requires_grad_(True)
+    block = sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=3)
+    with torch.no_grad():
+        levels = block.pyramid
+    assert all(torch.equal(x, y) for x, y in zip(levels, pyr)) and levels[2].requires_grad and block.pyramid is levels
+    with torch.no_grad():
+        block = sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=3)
+    assert not block.pyramid[1].requires_grad
+    with pytest.raises(RuntimeError):
+        sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=6)
