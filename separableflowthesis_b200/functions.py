@@ -1,5 +1,5 @@
 """The three autograd Functions of libs/MemorySaver/functions/MemorySaver.py, same names, argument
-order, outputs and error behaviour, on top of the B200 ops."""
+order, outputs and error behaviour, on top of the B200 ops, which make the tensors' device current themselves."""
 from __future__ import annotations
 
 import torch
@@ -15,8 +15,7 @@ class ComputeMaxAvgFunction(Function):
     @staticmethod
     def forward(ctx, img1_features_l0, img2_features_lk):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            max_avg_output_u, max_avg_output_v = MemorySaver.max_avg_forward(img1_features_l0, img2_features_lk)
+        max_avg_output_u, max_avg_output_v = MemorySaver.max_avg_forward(img1_features_l0, img2_features_lk)
         return max_avg_output_u, max_avg_output_v
 
     @staticmethod
@@ -30,8 +29,7 @@ class ComputeMaxArgmaxAvgFunction(Function):
     @staticmethod
     def forward(ctx, img1_features_l0, img2_features_lk):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            ma_u, ma_v, am_u, am_v = MemorySaver.max_argmax_avg_forward(img1_features_l0, img2_features_lk)
+        ma_u, ma_v, am_u, am_v = MemorySaver.max_argmax_avg_forward(img1_features_l0, img2_features_lk)
         ctx.save_for_backward(img1_features_l0, img2_features_lk, am_u, am_v)
         return ma_u, ma_v
 
@@ -40,9 +38,8 @@ class ComputeMaxArgmaxAvgFunction(Function):
         img1_features_l0, img2_features_lk, am_u, am_v = ctx.saved_tensors
         grad_MaxAvg_u = grad_MaxAvg_u.contiguous()
         grad_MaxAvg_v = grad_MaxAvg_v.contiguous()
-        with torch.cuda.device_of(grad_MaxAvg_u):
-            g1, g2 = MemorySaver.max_argmax_avg_backward(img1_features_l0, img2_features_lk, am_u, am_v,
-                                                         grad_MaxAvg_u, grad_MaxAvg_v)
+        g1, g2 = MemorySaver.max_argmax_avg_backward(img1_features_l0, img2_features_lk, am_u, am_v,
+                                                     grad_MaxAvg_u, grad_MaxAvg_v)
         return g1, g2
 
 
@@ -53,9 +50,8 @@ class ComputeSelfCompressionFunction(Function):
     def forward(ctx, img1_features_l0, img2_features_lk, attention_weights_u, attention_weights_v):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
         assert attention_weights_u.is_contiguous() and attention_weights_v.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            c_u, c_v = MemorySaver.compression_forward(img1_features_l0, img2_features_lk,
-                                                       attention_weights_u, attention_weights_v)
+        c_u, c_v = MemorySaver.compression_forward(img1_features_l0, img2_features_lk,
+                                                   attention_weights_u, attention_weights_v)
         ctx.save_for_backward(img1_features_l0, img2_features_lk, attention_weights_u, attention_weights_v)
         return c_u, c_v
 
@@ -64,9 +60,8 @@ class ComputeSelfCompressionFunction(Function):
         f1, f2, a_u, a_v = ctx.saved_tensors
         grad_compressed_output_u = grad_compressed_output_u.contiguous()
         grad_compressed_output_v = grad_compressed_output_v.contiguous()
-        with torch.cuda.device_of(grad_compressed_output_u):
-            g1, g2, ga_u, ga_v = MemorySaver.compression_backward(f1, f2, a_u, a_v, grad_compressed_output_u,
-                                                                  grad_compressed_output_v)
+        g1, g2, ga_u, ga_v = MemorySaver.compression_backward(f1, f2, a_u, a_v, grad_compressed_output_u,
+                                                              grad_compressed_output_v)
         return g1, g2, ga_u, ga_v
 
 
@@ -104,8 +99,7 @@ class FusedMaxArgmaxAvgFunction(Function):
     @staticmethod
     def forward(ctx, img1_features_l0, img2_features_lk, state):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            ma_u, ma_v, am_u, am_v = MemorySaver.max_argmax_avg_forward(img1_features_l0, img2_features_lk)
+        ma_u, ma_v, am_u, am_v = MemorySaver.max_argmax_avg_forward(img1_features_l0, img2_features_lk)
         ctx.save_for_backward(img1_features_l0, img2_features_lk, am_u, am_v)
         ctx.state = state
         return ma_u, ma_v
@@ -116,13 +110,12 @@ class FusedMaxArgmaxAvgFunction(Function):
         grad_MaxAvg_u = grad_MaxAvg_u.contiguous()
         grad_MaxAvg_v = grad_MaxAvg_v.contiguous()
         pending, ctx.state.pending = ctx.state.pending, None
-        with torch.cuda.device_of(grad_MaxAvg_u):
-            if pending is None:
-                g1, g2 = MemorySaver.max_argmax_avg_backward(f1, f2, am_u, am_v, grad_MaxAvg_u, grad_MaxAvg_v)
-            else:
-                a_u, a_v, gc_u, gc_v = pending
-                g1, g2 = MemorySaver.separation_feature_backward(f1, f2, am_u, am_v, grad_MaxAvg_u, grad_MaxAvg_v,
-                                                                 a_u, a_v, gc_u, gc_v)
+        if pending is None:
+            g1, g2 = MemorySaver.max_argmax_avg_backward(f1, f2, am_u, am_v, grad_MaxAvg_u, grad_MaxAvg_v)
+        else:
+            a_u, a_v, gc_u, gc_v = pending
+            g1, g2 = MemorySaver.separation_feature_backward(f1, f2, am_u, am_v, grad_MaxAvg_u, grad_MaxAvg_v,
+                                                             a_u, a_v, gc_u, gc_v)
         return g1, g2, None
 
 
@@ -131,9 +124,8 @@ class FusedSelfCompressionFunction(Function):
     def forward(ctx, img1_features_l0, img2_features_lk, attention_weights_u, attention_weights_v, state):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
         assert attention_weights_u.is_contiguous() and attention_weights_v.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            c_u, c_v = MemorySaver.compression_forward(img1_features_l0, img2_features_lk,
-                                                       attention_weights_u, attention_weights_v)
+        c_u, c_v = MemorySaver.compression_forward(img1_features_l0, img2_features_lk,
+                                                   attention_weights_u, attention_weights_v)
         ctx.save_for_backward(img1_features_l0, img2_features_lk, attention_weights_u, attention_weights_v)
         ctx.state = state
         return c_u, c_v
@@ -143,18 +135,17 @@ class FusedSelfCompressionFunction(Function):
         f1, f2, a_u, a_v = ctx.saved_tensors
         gc_u = grad_compressed_output_u.contiguous()
         gc_v = grad_compressed_output_v.contiguous()
-        with torch.cuda.device_of(gc_u):
-            if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[1]):
-                ga_u, ga_v = MemorySaver.compression_attention_backward(f1, f2, gc_u, gc_v)
-                return None, None, ga_u, ga_v, None
-            if not (ctx.needs_input_grad[2] or ctx.needs_input_grad[3]):
-                # the attention weights do not depend on the max/avg node: nothing guarantees that node's
-                # backward runs after this one, so do not defer
-                g1, g2, ga_u, ga_v = MemorySaver.compression_backward(f1, f2, a_u, a_v, gc_u, gc_v)
-                return g1, g2, ga_u, ga_v, None
+        if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[1]):
             ga_u, ga_v = MemorySaver.compression_attention_backward(f1, f2, gc_u, gc_v)
-            ctx.state.pending = (a_u, a_v, gc_u, gc_v)
-            torch.autograd.Variable._execution_engine.queue_callback(_guard_pending(ctx.state))
+            return None, None, ga_u, ga_v, None
+        if not (ctx.needs_input_grad[2] or ctx.needs_input_grad[3]):
+            # the attention weights do not depend on the max/avg node: nothing guarantees that node's
+            # backward runs after this one, so do not defer
+            g1, g2, ga_u, ga_v = MemorySaver.compression_backward(f1, f2, a_u, a_v, gc_u, gc_v)
+            return g1, g2, ga_u, ga_v, None
+        ga_u, ga_v = MemorySaver.compression_attention_backward(f1, f2, gc_u, gc_v)
+        ctx.state.pending = (a_u, a_v, gc_u, gc_v)
+        torch.autograd.Variable._execution_engine.queue_callback(_guard_pending(ctx.state))
         return None, None, ga_u, ga_v, None
 
 
@@ -165,9 +156,8 @@ class SeparationMaxAvgCF(Function):
     @staticmethod
     def forward(ctx, img1_features_l0, img2_features_lk, state, with_argmax):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            sep_v, sep_u, am_u, am_v = MemorySaver.max_argmax_avg_forward_cf(img1_features_l0, img2_features_lk,
-                                                                             with_argmax)
+        sep_v, sep_u, am_u, am_v = MemorySaver.max_argmax_avg_forward_cf(img1_features_l0, img2_features_lk,
+                                                                         with_argmax)
         if with_argmax:
             ctx.save_for_backward(img1_features_l0, img2_features_lk, am_u, am_v)
         ctx.state = state
@@ -184,9 +174,8 @@ class SeparationMaxAvgCF(Function):
             raise RuntimeError("channels-first separation backward needs the compression node's backward first "
                                "(use AlternateCorrBlockSepflow(..., channels_first=False) for max/avg alone)")
         a_u, a_v, gc_u, gc_v = pending
-        with torch.cuda.device_of(grad_sep_v):
-            g1, g2 = MemorySaver.separation_feature_backward_cf(f1, f2, am_u, am_v, grad_sep_v.contiguous(),
-                                                                grad_sep_u.contiguous(), a_u, a_v, gc_u, gc_v)
+        g1, g2 = MemorySaver.separation_feature_backward_cf(f1, f2, am_u, am_v, grad_sep_v.contiguous(),
+                                                            grad_sep_u.contiguous(), a_u, a_v, gc_u, gc_v)
         return g1, g2, None, None
 
 
@@ -195,8 +184,7 @@ class SeparationCompressionCF(Function):
     def forward(ctx, img1_features_l0, img2_features_lk, a_u, a_v, state):
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
         assert a_u.is_contiguous() and a_v.is_contiguous()
-        with torch.cuda.device_of(img1_features_l0):
-            c_u, c_v = MemorySaver.compression_forward_cf(img1_features_l0, img2_features_lk, a_u, a_v)
+        c_u, c_v = MemorySaver.compression_forward_cf(img1_features_l0, img2_features_lk, a_u, a_v)
         ctx.save_for_backward(img1_features_l0, img2_features_lk, a_u, a_v)
         ctx.state = state
         return c_u, c_v
@@ -205,8 +193,7 @@ class SeparationCompressionCF(Function):
     def backward(ctx, grad_c_u, grad_c_v):
         f1, f2, a_u, a_v = ctx.saved_tensors
         gc_u, gc_v = grad_c_u.contiguous(), grad_c_v.contiguous()
-        with torch.cuda.device_of(gc_u):
-            ga_u, ga_v = MemorySaver.compression_attention_backward_cf(f1, f2, gc_u, gc_v)
+        ga_u, ga_v = MemorySaver.compression_attention_backward_cf(f1, f2, gc_u, gc_v)
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
             ctx.state.pending = (a_u, a_v, gc_u, gc_v)
             torch.autograd.Variable._execution_engine.queue_callback(_guard_pending(ctx.state))
@@ -224,10 +211,9 @@ class SeparationLevelFunction(Function):
         """With ``fmaps`` the features are the model's maps (B,C,H,W) and ``scale1`` multiplies image 1's."""
         assert img1_features_l0.is_contiguous() and img2_features_lk.is_contiguous()
         ctx.fmaps, ctx.scale1 = fmaps, scale1
-        with torch.cuda.device_of(img1_features_l0):
-            sep_u, sep_v, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(
-                img1_features_l0, img2_features_lk, weight_u.contiguous(), bias_u.contiguous(),
-                weight_v.contiguous(), bias_v.contiguous(), with_argmax, fmaps, scale1)
+        sep_u, sep_v, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(
+            img1_features_l0, img2_features_lk, weight_u.contiguous(), bias_u.contiguous(),
+            weight_v.contiguous(), bias_v.contiguous(), with_argmax, fmaps, scale1)
         if with_argmax:
             ctx.save_for_backward(img1_features_l0, img2_features_lk, weight_u, weight_v, sep_u, sep_v, am_u, am_v,
                                   a_u, a_v)
@@ -240,10 +226,9 @@ class SeparationLevelFunction(Function):
         if not ctx.with_argmax:
             raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
         f1, f2, weight_u, weight_v, sep_u, sep_v, am_u, am_v, a_u, a_v = ctx.saved_tensors
-        with torch.cuda.device_of(grad_sep_u):
-            g1, g2, gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_level_backward(
-                f1, f2, weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, am_u, am_v, a_u, a_v,
-                grad_sep_u.contiguous(), grad_sep_v.contiguous(), ctx.fmaps, ctx.scale1)
+        g1, g2, gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_level_backward(
+            f1, f2, weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, am_u, am_v, a_u, a_v,
+            grad_sep_u.contiguous(), grad_sep_v.contiguous(), ctx.fmaps, ctx.scale1)
         return g1, g2, gw_u, gb_u, gw_v, gb_v, None, None, None
 
 
@@ -270,24 +255,22 @@ class SeparationPyramidFunction(Function):
         ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, L
         ctx.together = _levels_together(fmap1, fmap2_levels, weight_u.shape[0])
         if ctx.together:
-            with torch.cuda.device_of(fmap1):
-                sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
+            sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
             if with_argmax:
                 ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, buffer)
             return sep_u, sep_v
-        with torch.cuda.device_of(fmap1):
-            sep_u = torch.empty(B, Kt * L, W2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
-            sep_v = torch.empty(B, Kt * L, H2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
-            for l, fmap2 in enumerate(fmap2_levels):
-                if tuple(fmap2.shape[2:]) == (H2, W2):   # displacement range of the output: written in place
-                    su, sv, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(
-                        fmap1, fmap2, *params, with_argmax, True, scale1, (sep_u, sep_v, l * Kt))
-                else:
-                    su, sv, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(fmap1, fmap2, *params,
-                                                                                        with_argmax, True, scale1)
-                    MemorySaver.upsample_displacement_into(su, sep_u, l * Kt)
-                    MemorySaver.upsample_displacement_into(sv, sep_v, l * Kt)
-                saved.append((su, sv, am_u, am_v, a_u, a_v))
+        sep_u = torch.empty(B, Kt * L, W2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
+        sep_v = torch.empty(B, Kt * L, H2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
+        for l, fmap2 in enumerate(fmap2_levels):
+            if tuple(fmap2.shape[2:]) == (H2, W2):   # displacement range of the output: written in place
+                su, sv, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(
+                    fmap1, fmap2, *params, with_argmax, True, scale1, (sep_u, sep_v, l * Kt))
+            else:
+                su, sv, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(fmap1, fmap2, *params,
+                                                                                    with_argmax, True, scale1)
+                MemorySaver.upsample_displacement_into(su, sep_u, l * Kt)
+                MemorySaver.upsample_displacement_into(sv, sep_v, l * Kt)
+            saved.append((su, sv, am_u, am_v, a_u, a_v))
         if with_argmax:
             # volumes written in place are saved as the outputs themselves
             ctx.in_place = [t[0] is None for t in saved]
@@ -307,32 +290,30 @@ class SeparationPyramidFunction(Function):
         wu, wv = weight_u.contiguous(), weight_v.contiguous()
         gu, gv = grad_sep_u.contiguous(), grad_sep_v.contiguous()
         if ctx.together:
-            with torch.cuda.device_of(gu):
-                g1, g2, gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(fmap1, fmap2_levels, wu, wv, sep_u, sep_v, flat[0],
-                                                                                         gu, gv, ctx.scale1)
+            g1, g2, gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(fmap1, fmap2_levels, wu, wv, sep_u, sep_v, flat[0],
+                                                                                     gu, gv, ctx.scale1)
             return (None, None, gw_u, gb_u, gw_v, gb_v, g1, *g2)
         Kt = 2 + weight_u.shape[0]
         g1 = gw_u = gb_u = gw_v = gb_v = None
         g2 = []
-        with torch.cuda.device_of(gu):
-            for l in range(L):
-                if ctx.in_place[l]:
-                    am_u, am_v, a_u, a_v = flat[:4]
-                    del flat[:4]
-                    out = MemorySaver.separation_level_backward(fmap1, fmap2_levels[l], wu, wv, sep_u, sep_v, am_u, am_v,
-                                                                a_u, a_v, gu, gv, True, ctx.scale1, l * Kt)
-                else:
-                    su, sv, am_u, am_v, a_u, a_v = flat[:6]
-                    del flat[:6]
-                    gsu = MemorySaver.upsample_displacement_backward(gu, l * Kt, Kt, su.shape[2])
-                    gsv = MemorySaver.upsample_displacement_backward(gv, l * Kt, Kt, sv.shape[2])
-                    out = MemorySaver.separation_level_backward(fmap1, fmap2_levels[l], wu, wv, su, sv, am_u, am_v, a_u,
-                                                                a_v, gsu, gsv, True, ctx.scale1)
-                g2.append(out[1])
-                if l == 0:
-                    g1, gw_u, gb_u, gw_v, gb_v = out[0], out[2], out[3], out[4], out[5]
-                else:
-                    g1 += out[0]; gw_u += out[2]; gb_u += out[3]; gw_v += out[4]; gb_v += out[5]
+        for l in range(L):
+            if ctx.in_place[l]:
+                am_u, am_v, a_u, a_v = flat[:4]
+                del flat[:4]
+                out = MemorySaver.separation_level_backward(fmap1, fmap2_levels[l], wu, wv, sep_u, sep_v, am_u, am_v,
+                                                            a_u, a_v, gu, gv, True, ctx.scale1, l * Kt)
+            else:
+                su, sv, am_u, am_v, a_u, a_v = flat[:6]
+                del flat[:6]
+                gsu = MemorySaver.upsample_displacement_backward(gu, l * Kt, Kt, su.shape[2])
+                gsv = MemorySaver.upsample_displacement_backward(gv, l * Kt, Kt, sv.shape[2])
+                out = MemorySaver.separation_level_backward(fmap1, fmap2_levels[l], wu, wv, su, sv, am_u, am_v, a_u,
+                                                            a_v, gsu, gsv, True, ctx.scale1)
+            g2.append(out[1])
+            if l == 0:
+                g1, gw_u, gb_u, gw_v, gb_v = out[0], out[2], out[3], out[4], out[5]
+            else:
+                g1 += out[0]; gw_u += out[2]; gb_u += out[3]; gw_v += out[4]; gb_v += out[5]
         return (None, None, gw_u, gb_u, gw_v, gb_v, g1, *g2)
 
 
@@ -344,8 +325,7 @@ class SeparationPooledPyramidFunction(Function):
     def forward(ctx, with_argmax, scale1, levels, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2):
         params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
         ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, levels
-        with torch.cuda.device_of(fmap1):
-            sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, [fmap2], *params, with_argmax, scale1, levels)
+        sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, [fmap2], *params, with_argmax, scale1, levels)
         if with_argmax:
             ctx.save_for_backward(fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, buffer)
         return sep_u, sep_v
@@ -356,10 +336,9 @@ class SeparationPooledPyramidFunction(Function):
         if not ctx.with_argmax:
             raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
         fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, buffer = ctx.saved_tensors
-        with torch.cuda.device_of(grad_sep_u):
-            g1, (g2,), gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(
-                fmap1, [fmap2], weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, buffer, grad_sep_u.contiguous(),
-                grad_sep_v.contiguous(), ctx.scale1, ctx.levels)
+        g1, (g2,), gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(
+            fmap1, [fmap2], weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, buffer, grad_sep_u.contiguous(),
+            grad_sep_v.contiguous(), ctx.scale1, ctx.levels)
         return None, None, None, gw_u, gb_u, gw_v, gb_v, g1, g2
 
 
@@ -370,8 +349,7 @@ class SeparationPooledPyramidFunction(Function):
 class LookupFunction(Function):
     @staticmethod
     def forward(ctx, corr, pyramid, coord, levels, radius, clamp_unit):
-        with torch.cuda.device_of(corr):
-            out = MemorySaver.lookup_forward(corr, pyramid, coord, levels, radius, clamp_unit)
+        out = MemorySaver.lookup_forward(corr, pyramid, coord, levels, radius, clamp_unit)
         ctx.save_for_backward(coord)
         ctx.cfg = (tuple(corr.shape), levels, radius, clamp_unit)
         return out
@@ -381,8 +359,7 @@ class LookupFunction(Function):
     def backward(ctx, grad_out):
         (coord,) = ctx.saved_tensors
         shape, levels, radius, clamp_unit = ctx.cfg
-        with torch.cuda.device_of(grad_out):
-            gcorr = MemorySaver.lookup_backward(shape, coord, grad_out.contiguous(), levels, radius, clamp_unit)
+        gcorr = MemorySaver.lookup_backward(shape, coord, grad_out.contiguous(), levels, radius, clamp_unit)
         return gcorr, None, None, None, None, None
 
 
@@ -406,8 +383,7 @@ class LookupVolumeFunction(Function):
         if acc is None:
             return None, None, None
         shape, levels, clamp_unit = ctx.cfg
-        with torch.cuda.device_of(acc):
-            return MemorySaver.lookup_fold_gradient(acc.contiguous(), shape, levels, clamp_unit), None, None
+        return MemorySaver.lookup_fold_gradient(acc.contiguous(), shape, levels, clamp_unit), None, None
 
 
 class LookupPairFunction(Function):
@@ -416,8 +392,7 @@ class LookupPairFunction(Function):
 
     @staticmethod
     def forward(ctx, corr1, corr2, pyramid1, pyramid2, coords, edge1, edge2, levels, radius):
-        with torch.cuda.device_of(corr1):
-            out1, out2 = MemorySaver.lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels, radius)
+        out1, out2 = MemorySaver.lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels, radius)
         if edge1 is not None or edge2 is not None:
             ctx.save_for_backward(coords)
             ctx.cfg = (tuple(corr1.shape), tuple(corr2.shape), levels, radius)
@@ -440,14 +415,13 @@ class LookupPairFunction(Function):
             g2 = None
         if g1 is not None or g2 is not None:
             (coords,) = ctx.saved_tensors
-            with torch.cuda.device_of(coords):
-                if g1 is not None:
-                    g1 = g1.contiguous()
-                    acc1 = _lookup_accumulator(acc1, shape1, levels, True, g1)
-                if g2 is not None:
-                    g2 = g2.contiguous()
-                    acc2 = _lookup_accumulator(acc2, shape2, levels, False, g2)
-                MemorySaver.lookup_accumulate_pair(shape1, shape2, coords, g1, g2, acc1, acc2, levels, radius)
+            if g1 is not None:
+                g1 = g1.contiguous()
+                acc1 = _lookup_accumulator(acc1, shape1, levels, True, g1)
+            if g2 is not None:
+                g2 = g2.contiguous()
+                acc2 = _lookup_accumulator(acc2, shape2, levels, False, g2)
+            MemorySaver.lookup_accumulate_pair(shape1, shape2, coords, g1, g2, acc1, acc2, levels, radius)
         return None, None, None, None, None, acc1, acc2, None, None
 
 
@@ -464,8 +438,7 @@ class Lookup4dFunction(Function):
 
     @staticmethod
     def forward(ctx, coords, radius, scale, F1, *F2_levels):
-        with torch.cuda.device_of(F1):
-            out = MemorySaver.lookup4d_forward(F1, list(F2_levels), coords, radius, scale)
+        out = MemorySaver.lookup4d_forward(F1, list(F2_levels), coords, radius, scale)
         ctx.save_for_backward(coords, F1, *F2_levels)
         ctx.cfg = (radius, scale)
         return out
@@ -475,6 +448,5 @@ class Lookup4dFunction(Function):
     def backward(ctx, grad_out):
         coords, F1, *F2_levels = ctx.saved_tensors
         radius, scale = ctx.cfg
-        with torch.cuda.device_of(grad_out):
-            gF1, gF2 = MemorySaver.lookup4d_backward(F1, F2_levels, coords, grad_out.contiguous(), radius, scale)
+        gF1, gF2 = MemorySaver.lookup4d_backward(F1, F2_levels, coords, grad_out.contiguous(), radius, scale)
         return (None, None, None, gF1, *gF2)

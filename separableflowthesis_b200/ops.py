@@ -6,6 +6,7 @@ allocates the outputs and calls the C ABI of ``libsepflow_b200.so`` on the curre
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import os
@@ -22,6 +23,20 @@ from . import _lib
 # from several threads.
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 _workspaces_lock = threading.Lock()
+
+
+# What a call costs on the host decides the small ones, so the device is switched only when another one is current, its stream is
+# asked for by number, and pointers go to the library as plain integers (ctypes converts them by the declared types).
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """Context in which `device` (of a CUDA tensor) is current."""
+    return _HERE if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
+
+
+def _stream(device: torch.device) -> int:
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def _check(t: torch.Tensor, name: str, dtype: torch.dtype, ndim: int) -> None:
@@ -80,33 +95,28 @@ def release_workspaces(device=None) -> int:
 
 
 def _ptr(t):
-    if isinstance(t, float):
-        return ctypes.c_float(t)
-    if isinstance(t, int):
-        return ctypes.c_int32(t)
-    return ctypes.c_void_p(t.data_ptr() if t is not None else None)
+    """An argument of the library: the address of a tensor, None, or a number as it is."""
+    return t.data_ptr() if isinstance(t, torch.Tensor) else t
 
 
 def _check_device_status(lib, name, ws, stream):
     if os.environ.get("SFB_CHECK_DEVICE_STATUS", "0") == "1":
         dev_status = ctypes.c_int32(0)
-        rc = lib.sfb_device_status(ctypes.c_void_p(ws.data_ptr()), ctypes.c_void_p(stream), ctypes.byref(dev_status))
+        rc = lib.sfb_device_status(ws.data_ptr(), stream, ctypes.byref(dev_status))
         if rc != _lib.SFB_OK:
             raise RuntimeError(f"{name}: {lib.sfb_last_error().decode()}")
 
 
 def _call(name: str, op: int, shape: _lib.SfbShape, device: torch.device, tensors) -> None:
     lib = _lib.load()
-    with torch.cuda.device(device):
-        stream = torch.cuda.current_stream(device).cuda_stream
+    with _on(device):
+        stream = _stream(device)
         nbytes = lib.sfb_workspace_bytes(op, ctypes.byref(shape))
         if nbytes == 0:
             # run the entry point anyway so that the library reports the precise reason
             nbytes = 256
         ws = _workspace(nbytes, device, stream)
-        rc = getattr(lib, name)(*[_ptr(t) for t in tensors], ctypes.byref(shape),
-                                ctypes.c_void_p(ws.data_ptr()), ctypes.c_size_t(ws.numel()),
-                                ctypes.c_void_p(stream))
+        rc = getattr(lib, name)(*[_ptr(t) for t in tensors], ctypes.byref(shape), ws.data_ptr(), ws.numel(), stream)
         if rc != _lib.SFB_OK:
             raise RuntimeError(f"{name}: {lib.sfb_status_string(rc).decode()}: {lib.sfb_last_error().decode()}")
         _check_device_status(lib, name, ws, stream)
@@ -355,10 +365,10 @@ def attention_forward(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor)
     Kc = _check_attention_params(weight, bias, "attention", x.device)
     a = torch.empty(B, Kc, D, H1, W1, dtype=torch.float32, device=x.device)
     lib = _lib.load()
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+    with _on(x.device):
+        stream = _stream(x.device)
         _raise_on(lib.sfb_attention_forward(_ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(a), B, Kc, D, H1, W1,
-                                            ctypes.c_void_p(stream)), "sfb_attention_forward")
+                                            stream), "sfb_attention_forward")
     return a
 
 
@@ -376,14 +386,14 @@ def attention_backward(x, weight, a, grad_a, add=None) -> List[torch.Tensor]:
     gw = torch.empty_like(weight)
     gb = torch.empty(Kc, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _on(dev):
+        stream = _stream(dev)
         nbytes = lib.sfb_attention_backward_workspace_bytes(B, Kc, D, H1, W1)
         ws = _workspace(max(nbytes, 256), dev, stream)
         _raise_on(lib.sfb_attention_backward(_ptr(x), x.stride(0), _ptr(weight), _ptr(a), _ptr(g), _ptr(add),
                                              add.stride(0) if add is not None else 0, _ptr(gx), _ptr(gw), _ptr(gb),
-                                             B, Kc, D, H1, W1, ctypes.c_void_p(ws.data_ptr()),
-                                             ctypes.c_size_t(ws.numel()), ctypes.c_void_p(stream)),
+                                             B, Kc, D, H1, W1, ws.data_ptr(),
+                                             ws.numel(), stream),
                   "sfb_attention_backward")
     return [gx, gw, gb]
 
@@ -534,8 +544,8 @@ def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, 
     shape, pooled = ctypes.byref(s), int(L != len(fmap2_levels))
     saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax), pooled), 256), dtype=torch.uint8,
                         device=dev)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _on(dev):
+        stream = _stream(dev)
         ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, 0), 256), dev, stream)
         _raise_on(lib.sfb_separation_pyramid_forward(
             fmap1.data_ptr(), ptrs, H2, W2, L, scale1, weight_u.data_ptr(), bias_u.data_ptr(), weight_v.data_ptr(), bias_v.data_ptr(),
@@ -568,8 +578,8 @@ def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, 
     ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L)
     gptrs = (ctypes.c_void_p * L)(*[t.data_ptr() for t in gF2])
     shape = ctypes.byref(s)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _on(dev):
+        stream = _stream(dev)
         ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, 1), 256), dev, stream)
         _raise_on(lib.sfb_separation_pyramid_backward(
             fmap1.data_ptr(), ptrs, H2, W2, L, scale1, weight_u.data_ptr(), weight_v.data_ptr(), sep_u.data_ptr(), sep_v.data_ptr(),
@@ -614,11 +624,11 @@ def upsample_displacement_into(src: torch.Tensor, dst: torch.Tensor, c0: int) ->
         raise RuntimeError(f"cannot place {tuple(src.shape)} at channel {c0} of {tuple(dst.shape)}")
     D0 = dst.shape[2]
     lib = _lib.load()
-    with torch.cuda.device(src.device):
-        stream = torch.cuda.current_stream(src.device).cuda_stream
-        out = ctypes.c_void_p(dst.data_ptr() + 4 * c0 * D0 * H1 * W1)
+    with _on(src.device):
+        stream = _stream(src.device)
+        out = dst.data_ptr() + 4 * c0 * D0 * H1 * W1
         _raise_on(lib.sfb_upsample_displacement(_ptr(src), out, dst.stride(0), B, K, Dl, D0, H1, W1,
-                                                ctypes.c_void_p(stream)), "sfb_upsample_displacement")
+                                                stream), "sfb_upsample_displacement")
 
 
 def upsample_displacement_backward(grad_dst: torch.Tensor, c0: int, K: int, Dl: int) -> torch.Tensor:
@@ -629,11 +639,11 @@ def upsample_displacement_backward(grad_dst: torch.Tensor, c0: int, K: int, Dl: 
         raise RuntimeError(f"channels {c0}..{c0 + K} outside {Ktot}")
     gsrc = torch.empty(B, K, Dl, H1, W1, dtype=torch.float32, device=grad_dst.device)
     lib = _lib.load()
-    with torch.cuda.device(grad_dst.device):
-        stream = torch.cuda.current_stream(grad_dst.device).cuda_stream
-        g = ctypes.c_void_p(grad_dst.data_ptr() + 4 * c0 * D0 * H1 * W1)
+    with _on(grad_dst.device):
+        stream = _stream(grad_dst.device)
+        g = grad_dst.data_ptr() + 4 * c0 * D0 * H1 * W1
         _raise_on(lib.sfb_upsample_displacement_backward(g, grad_dst.stride(0), _ptr(gsrc), B, K, Dl, D0, H1, W1,
-                                                         ctypes.c_void_p(stream)), "sfb_upsample_displacement_backward")
+                                                         stream), "sfb_upsample_displacement_backward")
     return gsrc
 
 
@@ -658,10 +668,10 @@ def lookup_build_pyramid(corr: torch.Tensor, levels: int) -> torch.Tensor:
     lib = _lib.load()
     nbytes = lib.sfb_lookup_pyramid_bytes(B, dim, D, H1, W1, levels)
     pyr = torch.empty(max(nbytes // 4, 1), dtype=torch.float32, device=corr.device)
-    with torch.cuda.device(corr.device):
-        stream = torch.cuda.current_stream(corr.device).cuda_stream
+    with _on(corr.device):
+        stream = _stream(corr.device)
         _raise_on(lib.sfb_lookup_build_pyramid(_ptr(corr), _ptr(pyr), B, dim, D, H1, W1, levels,
-                                               ctypes.c_void_p(stream)), "sfb_lookup_build_pyramid")
+                                               stream), "sfb_lookup_build_pyramid")
     return pyr
 
 
@@ -672,10 +682,10 @@ def lookup_forward(corr, pyramid, coord, levels=4, radius=4, clamp_unit=False) -
     _check_coord(coord, B, H1, W1, corr.device)
     out = torch.empty(B, levels * dim * (2 * radius + 1), H1, W1, dtype=torch.float32, device=corr.device)
     lib = _lib.load()
-    with torch.cuda.device(corr.device):
-        stream = torch.cuda.current_stream(corr.device).cuda_stream
+    with _on(corr.device):
+        stream = _stream(corr.device)
         _raise_on(lib.sfb_lookup_forward(_ptr(corr), _ptr(pyramid), _ptr(coord), coord.stride(0), _ptr(out), B, dim, D,
-                                         H1, W1, levels, radius, int(bool(clamp_unit)), ctypes.c_void_p(stream)),
+                                         H1, W1, levels, radius, int(bool(clamp_unit)), stream),
                   "sfb_lookup_forward")
     return out
 
@@ -689,12 +699,12 @@ def lookup_backward(corr_shape, coord, grad_out, levels=4, radius=4, clamp_unit=
     gcorr = torch.empty(B, dim, D, H1, W1, dtype=torch.float32, device=dev)
     lib = _lib.load()
     nbytes = lib.sfb_lookup_pyramid_bytes(B, dim, D, H1, W1, levels)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _on(dev):
+        stream = _stream(dev)
         ws = _workspace(max(nbytes, 256), dev, stream)
         _raise_on(lib.sfb_lookup_backward(_ptr(grad_out), _ptr(coord), coord.stride(0), _ptr(gcorr),
-                                          ctypes.c_void_p(ws.data_ptr()), B, dim, D, H1, W1, levels, radius,
-                                          int(bool(clamp_unit)), ctypes.c_void_p(stream)), "sfb_lookup_backward")
+                                          ws.data_ptr(), B, dim, D, H1, W1, levels, radius,
+                                          int(bool(clamp_unit)), stream), "sfb_lookup_backward")
     return gcorr
 
 
@@ -732,8 +742,8 @@ def lookup_build_pyramid_pair(corr1, corr2, levels: int):
     lib = _lib.load()
     pyr = [torch.empty(max(lib.sfb_lookup_pyramid_bytes(B, dim, D, H1, W1, levels) // 4, 1), dtype=torch.float32, device=corr1.device)
            for D in (D1, D2)]
-    with torch.cuda.device(corr1.device):
-        stream = torch.cuda.current_stream(corr1.device).cuda_stream
+    with _on(corr1.device):
+        stream = _stream(corr1.device)
         _raise_on(lib.sfb_lookup_build_pyramid_pair(corr1.data_ptr(), pyr[0].data_ptr(), corr2.data_ptr(), pyr[1].data_ptr(), B, dim,
                                                     D1, D2, H1, W1, levels, stream), "sfb_lookup_build_pyramid_pair")
     return pyr
@@ -748,8 +758,8 @@ def lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels=4, radi
     out1 = torch.empty(size, dtype=torch.float32, device=dev)
     out2 = torch.empty(size, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _on(dev):
+        stream = _stream(dev)
         _raise_on(lib.sfb_lookup_forward_pair(corr1.data_ptr(), pyramid1.data_ptr(), corr2.data_ptr(), pyramid2.data_ptr(),
                                               coords.data_ptr(), sb, sc, out1.data_ptr(), out2.data_ptr(), B, dim, D1, D2, H1, W1,
                                               levels, radius, stream), "sfb_lookup_forward_pair")
@@ -772,8 +782,8 @@ def lookup_accumulate_pair(shape1, shape2, coords, gout1, gout2, acc1, acc2, lev
             _check_like(gout, "grad_out", (B, levels * dim * (2 * radius + 1), H1, W1), torch.float32, dev)
             _check_like(acc, "accumulator", (lookup_accumulator_size(shape, levels, clamp),), torch.float32, dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _on(dev):
+        stream = _stream(dev)
         _raise_on(lib.sfb_lookup_accumulate_pair(
             gout1.data_ptr() if gout1 is not None else None, gout2.data_ptr() if gout2 is not None else None, coords.data_ptr(), sb,
             sc, acc1.data_ptr() if gout1 is not None else None, acc2.data_ptr() if gout2 is not None else None, B, dim, D1, D2, H1,
@@ -786,8 +796,8 @@ def lookup_fold_gradient(acc, corr_shape, levels=4, clamp_unit=False) -> torch.T
     _check_like(acc, "accumulator", (lookup_accumulator_size(corr_shape, levels, clamp_unit),), torch.float32, acc.device)
     gcorr = torch.empty(corr_shape, dtype=torch.float32, device=acc.device)
     lib = _lib.load()
-    with torch.cuda.device(acc.device):
-        stream = torch.cuda.current_stream(acc.device).cuda_stream
+    with _on(acc.device):
+        stream = _stream(acc.device)
         _raise_on(lib.sfb_lookup_fold_gradient(acc.data_ptr(), gcorr.data_ptr(), B, dim, D, H1, W1, levels, int(bool(clamp_unit)),
                                                stream), "sfb_lookup_fold_gradient")
     return gcorr
@@ -862,10 +872,10 @@ def lookup4d_forward(F1, F2_levels, coords, radius=4, scale=1.0) -> torch.Tensor
     out = torch.empty(B, n * (2 * radius + 1) ** 2, H1, W1, dtype=torch.float32, device=F1.device)
     ptrs, H2, W2 = _level_arrays(F2_levels)
     lib = _lib.load()
-    with torch.cuda.device(F1.device):
-        stream = torch.cuda.current_stream(F1.device).cuda_stream
+    with _on(F1.device):
+        stream = _stream(F1.device)
         _raise_on(lib.sfb_lookup4d_forward(_ptr(F1), ptrs, H2, W2, n, _ptr(coords), _ptr(out), B, H1, W1, C, radius,
-                                           float(scale), ctypes.c_void_p(stream)), "sfb_lookup4d_forward")
+                                           float(scale), stream), "sfb_lookup4d_forward")
     return out
 
 
@@ -881,9 +891,9 @@ def lookup4d_backward(F1, F2_levels, coords, grad_out, radius=4, scale=1.0):
     ptrs, H2, W2 = _level_arrays(F2_levels)
     gptrs, _, _ = _level_arrays(gF2)
     lib = _lib.load()
-    with torch.cuda.device(F1.device):
-        stream = torch.cuda.current_stream(F1.device).cuda_stream
+    with _on(F1.device):
+        stream = _stream(F1.device)
         _raise_on(lib.sfb_lookup4d_backward(_ptr(F1), ptrs, H2, W2, n, _ptr(coords), _ptr(grad_out), _ptr(gF1), gptrs,
-                                            B, H1, W1, C, radius, float(scale), ctypes.c_void_p(stream)),
+                                            B, H1, W1, C, radius, float(scale), stream),
                   "sfb_lookup4d_backward")
     return gF1, gF2
