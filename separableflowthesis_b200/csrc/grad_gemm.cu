@@ -15,14 +15,15 @@
 //                      shared memory, swizzled, K-major (TF32) or MN-major (16-bit).
 //   With 16-bit operands G is generated once.  It costs the CUDA cores several times what its multiply-adds cost the tensor core, and the
 //   image-2-major generator, which shares no operand across a block, is the dearer one:
-//   storing          : image-1-major as above; the blocks also go to shared memory, from where one bulk copy per block takes them
-//                      to memory (16 KB per 128 x 64 values, beside some 1900 cycles of generating them).
+//   storing          : image-1-major, but the blocks go to shared memory, where the tensor core reads them as they are and from where
+//                      one bulk copy per block takes them to memory (16 KB per 128 x 64 values, beside some 1900 cycles of generating
+//                      them).  Written to tensor memory as well, they took 418 instead of 404 us at 8 x 47 x 156.
 //   stored           : rows = 256 image-2 pixels (four blocks of 4 x 16, two accumulators), K = 64 image-1 pixels.  A block is 128-byte
 //                      rows of 64 image-2 pixels, MN-major, and is loaded as it lies in memory.  A plain GEMM: bound by the HBM
 //                      that G comes from, next to the tensor core.  With tiles of 128 rows it would read 1.5 times as much of image 1
 //                      through L2 per multiply-add as it gives the tensor core time for.
-//   G generated twice and once (the pair, us): 8 x 135 x 240 with four channels 17.6 ms and 12.9, 8 x 47 x 156 with two 782 and
-//   630 (BF16); the rule is grad_hands_over in c_abi.cu.
+//   G generated twice and once (the pair, us): 8 x 135 x 240 with four channels 17.6 ms and 13.1, 8 x 47 x 156 with two 782 and
+//   614 (BF16); the rule is grad_hands_over in c_abi.cu.
 // B operand, all forms: K-major, like the operands of the correlation sweeps: TMA boxes of 32*ceil(C/32) channel
 // rows x the K-values of a block from channel-major copies of the rounded features (image 1: (C, pixels); image 2: (C, column
 // blocks of 16, rows, 16), so that the 4 rows x 16 columns of a K block are 64 consecutive values).  The MN-major
@@ -76,34 +77,36 @@ constexpr uint32_t GG_ACC_COLS = 256;                      // accumulator column
 //        of the block to arrive
 // The image-2-major form's two generator groups hold two operand blocks at a time and a TMA load takes about as long
 // as one block's computation: with fewer than four (pixel, u) stages the generators wait for their operands.
-// The storing form gives a ring of three blocks on their way to memory what it takes from the others; the stored form has one ring,
-// a feature block and the four blocks of G that go with it to a stage.
+// The storing form has a ring (NST) of blocks that the multiply-adds and the copy to memory both read, and gives it what it takes from the
+// others (three (pixel, u) stages and four of these: 412 us instead of 404 at 8 x 47 x 156, 10.99 ms instead of 9.5 at 8 x 135 x 240); the
+// stored form has one ring, a feature block and the four blocks of G that go with it to a stage.
 template <int Q, int FORM> struct GradCfg;
 template <> struct GradCfg<1, GRAD_IMAGE1> { static constexpr int NY = 6, NG = 4, NXU = 4, NXV = 1; };
 template <> struct GradCfg<2, GRAD_IMAGE1> { static constexpr int NY = 5, NG = 4, NXU = 4, NXV = 1; };
 template <> struct GradCfg<3, GRAD_IMAGE1> { static constexpr int NY = 4, NG = 4, NXU = 4, NXV = 1; };
-template <> struct GradCfg<1, GRAD_IMAGE1_STORING> { static constexpr int NY = 4, NG = 4, NXU = 4, NXV = 1; };
-template <> struct GradCfg<2, GRAD_IMAGE1_STORING> { static constexpr int NY = 3, NG = 4, NXU = 4, NXV = 1; };
-template <> struct GradCfg<3, GRAD_IMAGE1_STORING> { static constexpr int NY = 3, NG = 4, NXU = 3, NXV = 1; };
+template <> struct GradCfg<1, GRAD_IMAGE1_STORING> { static constexpr int NY = 4, NG = 1, NXU = 4, NXV = 1; };
+template <> struct GradCfg<2, GRAD_IMAGE1_STORING> { static constexpr int NY = 3, NG = 1, NXU = 4, NXV = 1; };
+template <> struct GradCfg<3, GRAD_IMAGE1_STORING> { static constexpr int NY = 3, NG = 1, NXU = 3, NXV = 1; };
 template <int Q> struct GradCfg<Q, GRAD_IMAGE2> { static constexpr int NY = 3, NG = 2, NXU = 4, NXV = 2; };
 template <int Q> struct GradCfg<Q, GRAD_IMAGE2_STORED> { static constexpr int NY = 3, NG = 3, NXU = 1, NXV = 1; };
-constexpr int GG_NST = 3;                                  // blocks on their way to memory
 constexpr uint32_t GG_SBLOCK_BYTES = GG_SJ * 128;          // stored form: 64 pixels of one block of G
-template <int FORM> __host__ __device__ constexpr uint32_t gg_tmem_cols() { return FORM == GRAD_IMAGE2 ? 256u : 512u; }
+template <int FORM> __host__ __device__ constexpr uint32_t gg_tmem_cols() { return FORM == GRAD_IMAGE2 || FORM == GRAD_IMAGE1_STORING ? 256u : 512u; }
 
 template <int Q, int FORM>
 struct GradSmem {
   using Cfg = GradCfg<Q, FORM>;
   static constexpr bool STORING = FORM == GRAD_IMAGE1_STORING, STORED = FORM == GRAD_IMAGE2_STORED;
-  static constexpr bool AT = FORM == GRAD_IMAGE1 || STORING;   // A blocks in tensor memory
+  static constexpr bool AT = FORM == GRAD_IMAGE1;   // A blocks in tensor memory
+  static constexpr bool I1 = !grad_is_image2(FORM);
+  static constexpr int NST = STORING ? (Q == 1 ? 4 : 3) : 1;
   static_assert(GG_ACC_COLS + (AT ? Cfg::NG * GG_KJ1 : 0) <= gg_tmem_cols<FORM>(), "A stages exceed TMEM");
   // one operand block: [displacement][group of 4 slots][pixel][4]; image-1-major 4 x Q x 128, image-2-major 8 x Q x 32
-  static constexpr int XU_FLOATS = STORED ? 4 : (AT ? GG_UT * TILE_M : GG_ROW_UT * GG_KJ) * Q * 4;
+  static constexpr int XU_FLOATS = STORED ? 4 : (I1 ? GG_UT * TILE_M : GG_ROW_UT * GG_KJ) * Q * 4;
   static constexpr int XV_FLOATS = FORM == GRAD_IMAGE2 ? GG_ROW_VT * GG_KJ * Q * 4 : 4;  // image-1-major keeps XV in registers
   float y[Cfg::NY][MAX_KB * GG_YBLOCK_BYTES / 4];  // feature stages [channel][K-values], K-major, swizzled
   // A blocks in shared memory, 128B swizzle: generated ones, K-major (TF32) or MN-major (16-bit); stored ones, MN-major
-  float g[AT ? 1 : Cfg::NG][AT ? 32 : (STORED ? GG_SM * GG_SBLOCK_BYTES / 4 : TILE_M * GG_KJ)];
-  uint8_t st[STORING ? GG_NST : 1][STORING ? TILE_M * 128 : 128];   // blocks on their way to memory
+  float g[I1 ? 1 : Cfg::NG][I1 ? (STORING ? 256 : 32) : (STORED ? GG_SM * GG_SBLOCK_BYTES / 4 : TILE_M * GG_KJ)];
+  uint8_t st[NST][STORING ? TILE_M * 128 : 128];   // the storing form's A blocks, K-major, 128B swizzle, as they go to memory
   float xu[Cfg::NXU][XU_FLOATS];
   float xv[Cfg::NXV][XV_FLOATS];
   uint64_t y_full[Cfg::NY];
@@ -114,8 +117,8 @@ struct GradSmem {
   uint64_t xu_empty[Cfg::NXU];
   uint64_t xv_full[Cfg::NXV];
   uint64_t xv_empty[Cfg::NXV];
-  uint64_t st_full[GG_NST];
-  uint64_t st_empty[GG_NST];
+  uint64_t st_full[NST];
+  uint64_t st_empty[NST];
   uint64_t acc_full;
   uint32_t tmem_base;
   WaitCtl ctl;
@@ -185,6 +188,13 @@ __device__ __forceinline__ void g_products(const Slots<Q>& xu, const Slots<Q> (&
     for (int i = 0; i < N; ++i) x[i] = fmaf(xu.f[k], xv[i].f[k], x[i]);
 }
 
+// Eight values as pairs of the 16-bit type.
+template <int OP>
+__device__ __forceinline__ void pack_row(const float (&g)[GG_VH], uint32_t (&h)[GG_VH / 2]) {
+#pragma unroll
+  for (int j = 0; j < GG_VH / 2; ++j) h[j] = OP == OP16_FP16 ? pack_fp16x2(g[2 * j], g[2 * j + 1]) : pack_bf16x2(g[2 * j], g[2 * j + 1]);
+}
+
 // rows = image-1 pixels.  Thread (pl, vh): row pl of the tile, columns vh*8 .. vh*8+7 of every 4 x 16 block.
 // Bound: issue.  A value takes 8 multiply-adds, 3 additions, 2 compares and half a conversion at four channels; blocks of four
 // rows instead of two halve what the barriers and waits of a block cost beside them (353 instead of 430 instructions per 16
@@ -208,7 +218,6 @@ __device__ void generator_image1(GradSmem<Q, FORM>& sm, const GradArgs& a, const
   int vb = sc.t0 / sc.n_ub2, ub2 = sc.t0 - vb * sc.n_ub2;
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t so = t % Cfg::NXU, pho = (t / Cfg::NXU) & 1u;
-    const uint32_t s = t % Cfg::NG, ph = (t / Cfg::NG) & 1u;
     const int vbase = vb * GG_VT + vh * GG_VH;
     if (ub2 == 0 || t == 0) {
 #pragma unroll
@@ -236,37 +245,41 @@ __device__ void generator_image1(GradSmem<Q, FORM>& sm, const GradArgs& a, const
         g[ul][i] = BF16 ? x[i] : round_for_mma(x[i]);
       }
     }
-    if (!mbar_wait_warp(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
-    tc_fence_after();  // the MMAs that read this stage's TMEM columns have completed
     if constexpr (STORING) {
-      if (!mbar_wait_warp(&sm.st_empty[t % GG_NST], ((t / GG_NST) & 1u) ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
-    }
-    if constexpr (BF16) {
+      // the multiply-adds and the copy that read this stage have completed
+      const uint32_t d = t % GradSmem<Q, FORM>::NST;
+      if (!mbar_wait_warp(&sm.st_empty[d], ((t / GradSmem<Q, FORM>::NST) & 1u) ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
 #pragma unroll
       for (int ul = 0; ul < GG_UT; ++ul) {
         uint32_t h[GG_VH / 2];
-#pragma unroll
-        for (int j = 0; j < GG_VH / 2; ++j)
-          h[j] = BF16 == OP16_FP16 ? pack_fp16x2(g[ul][2 * j], g[ul][2 * j + 1]) : pack_bf16x2(g[ul][2 * j], g[ul][2 * j + 1]);
-        tmem_st4(ta0 + s * A_COLS + ul * (GG_VT / 2), h);
+        pack_row<BF16>(g[ul], h);
         // eight values = chunk 2 * ul + vh of the pixel's row; eight lanes' chunks lie in different banks
-        if constexpr (STORING)
-          *reinterpret_cast<uint4*>(sm.st[t % GG_NST] + pl * 128 + ((((uint32_t)ul * 2 + vh) ^ ((uint32_t)pl & 7u)) << 4)) =
-              make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4*>(sm.st[d] + pl * 128 + ((((uint32_t)ul * 2 + vh) ^ ((uint32_t)pl & 7u)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+      }
+      fence_proxy_async_smem();   // before the tensor core's and the bulk copy's reads; the operand stage has been read, too
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&sm.st_full[d]);
+        mbar_arrive(&sm.xu_empty[so]);
       }
     } else {
+      const uint32_t s = t % Cfg::NG, ph = (t / Cfg::NG) & 1u;
+      if (!mbar_wait_warp(&sm.g_empty[s], ph ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
+      tc_fence_after();  // the MMAs that read this stage's TMEM columns have completed
 #pragma unroll
-      for (int ul = 0; ul < GG_UT; ++ul) tmem_st8(ta0 + s * A_COLS + ul * GG_VT, g[ul]);
-    }
-    tmem_st_wait();
-    tc_fence_before();  // stores complete and ordered before the tensor core's reads, which follow the arrive
-    if constexpr (STORING) fence_proxy_async_smem();   // ... and before the bulk copy's; the operand stage has been read, too
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.g_full[s]);
-    if constexpr (STORING) {
-      if (lane == 0) mbar_arrive(&sm.st_full[t % GG_NST]);
-      if (lane == 0) mbar_arrive(&sm.xu_empty[so]);
-    } else {
+      for (int ul = 0; ul < GG_UT; ++ul) {
+        if constexpr (BF16) {
+          uint32_t h[GG_VH / 2];
+          pack_row<BF16>(g[ul], h);
+          tmem_st4(ta0 + s * A_COLS + ul * (GG_VT / 2), h);
+        } else {
+          tmem_st8(ta0 + s * A_COLS + ul * GG_VT, g[ul]);
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();  // stores complete and ordered before the tensor core's reads, which follow the arrive
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.g_full[s]);
       hand_back_stage(&sm.xu_empty[so], lane);
     }
     if (++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
@@ -440,16 +453,24 @@ __device__ void grad_mma(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSch
   constexpr int NK = FORM == GRAD_IMAGE2 && BF16 ? 2 : 4;   // instructions per feature stage
   constexpr uint32_t A_COLS = BF16 ? GG_KJ1 / 2 : GG_KJ1;
   uint32_t sy = 0, phy = 0;
+  constexpr bool STORING = FORM == GRAD_IMAGE1_STORING;
+  constexpr int N_A = STORING ? GradSmem<Q, FORM>::NST : Cfg::NG;
+  uint64_t *const a_full = STORING ? sm.st_full : sm.g_full, *const a_empty = STORING ? sm.st_empty : sm.g_empty;
   for (int t = 0; t < sc.n_blocks; ++t) {
-    const uint32_t sg = t % Cfg::NG, phg = (t / Cfg::NG) & 1u;
+    const uint32_t sg = t % N_A, phg = (t / N_A) & 1u;
 #pragma unroll
     for (int h = 0; h < PER; ++h) {
       if (!mbar_wait(&sm.y_full[sy], phy, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
-      if (FORM != GRAD_IMAGE2_STORED && h == 0 && !mbar_wait(&sm.g_full[sg], phg, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
+      if (FORM != GRAD_IMAGE2_STORED && h == 0 && !mbar_wait(&a_full[sg], phg, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
       tc_fence_after();
       const uint64_t bdesc = FORM == GRAD_IMAGE2 && BF16 ? make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 512, 4)
                                                          : make_smem_desc_sw128(smem_u32(sm.y[sy]), 16, 1024);
-      if constexpr (!I2MAJOR) {
+      if constexpr (STORING) {
+        const uint64_t adesc = make_smem_desc_sw128(smem_u32(sm.st[sg]), 16, 1024);
+#pragma unroll
+        for (int k = 0; k < NK; ++k)
+          umma_bf16(sm.tmem_base, desc_advance(adesc, k * 32), desc_advance(bdesc, k * 32), idesc, (t | k) != 0);
+      } else if constexpr (!I2MAJOR) {
         const uint32_t a_tmem = sm.tmem_base + GG_ACC_COLS + sg * A_COLS + h * 32;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
@@ -475,7 +496,7 @@ __device__ void grad_mma(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSch
       umma_commit(&sm.y_empty[sy]);  // reusable once these MMAs have read it
       if (++sy == Cfg::NY) { sy = 0; phy ^= 1u; }
     }
-    if constexpr (FORM != GRAD_IMAGE2_STORED) umma_commit(&sm.g_empty[sg]);
+    if constexpr (FORM != GRAD_IMAGE2_STORED) umma_commit(&a_empty[sg]);
   }
   umma_commit(&sm.acc_full);
 }
@@ -484,15 +505,16 @@ __device__ void grad_mma(GradSmem<Q, FORM>& sm, const GradArgs& a, const GradSch
 // waits for a copy to have read its block before it issues the next block's multiply-adds, the copies cost a third of the launch.
 template <int Q>
 __device__ void block_storer(GradSmem<Q, GRAD_IMAGE1_STORING>& sm, const GradArgs& a, const GradSched& sc) {
+  constexpr uint32_t NST = GradSmem<Q, GRAD_IMAGE1_STORING>::NST;
   // the tile's pixels in the first of its blocks, and bytes from one block to the next
   const size_t step = (size_t)a.n1p * 128;
   uint8_t* dst = a.stored + ((size_t)(sc.b - a.b0) * sc.n_ub2 * ((a.d.W2 + GG_VT - 1) / GG_VT) + sc.t0) * step + (size_t)sc.m0 * 128;
   for (int t = 0; t < sc.n_blocks; ++t, dst += step) {
-    const uint32_t s = t % GG_NST, ph = (t / GG_NST) & 1u;
+    const uint32_t s = t % NST, ph = (t / NST) & 1u;
     if (!mbar_wait(&sm.st_full[s], ph, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
     bulk_store(dst, sm.st[s], TILE_M * 128);
     bulk_wait_read<1>();   // the block before this one has been read
-    if (t > 0) mbar_arrive(&sm.st_empty[(t - 1) % GG_NST]);
+    if (t > 0) mbar_arrive(&sm.st_empty[(t - 1) % NST]);
   }
   bulk_wait_all();
 }
@@ -707,7 +729,7 @@ grad_gemm_kernel(const __grid_constant__ GradLaunch<LEVELS> launch, int* status)
     for (int s = 0; s < Cfg::NG; ++s) { mbar_init(&sm.g_full[s], gen_arrivals); mbar_init(&sm.g_empty[s], 1); }
     for (int s = 0; s < Cfg::NXU; ++s) { mbar_init(&sm.xu_full[s], 1); mbar_init(&sm.xu_empty[s], gen_arrivals); }
     for (int s = 0; s < Cfg::NXV; ++s) { mbar_init(&sm.xv_full[s], 1); mbar_init(&sm.xv_empty[s], gen_arrivals); }
-    for (int s = 0; s < GG_NST; ++s) { mbar_init(&sm.st_full[s], gen_arrivals); mbar_init(&sm.st_empty[s], 1); }
+    for (int s = 0; s < Smem::NST; ++s) { mbar_init(&sm.st_full[s], gen_arrivals); mbar_init(&sm.st_empty[s], 2); }   // read by two
     mbar_init(&sm.acc_full, 1);
     wait_ctl_init(&sm.ctl, a.wait_limit_ns);
     fence_barrier_init();
