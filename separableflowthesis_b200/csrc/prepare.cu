@@ -388,12 +388,13 @@ f2_means_kernel(const float* __restrict__ F2, float* __restrict__ aux, int H2, i
   }
 }
 
-// From channel-major feature maps: a block owns one channel plane; its warps take every eighth row, FC_ROWS rows at a time, a
+// From channel-major feature maps: a block owns one channel plane; its warps take every eighth row, ROWS rows at a time, a
 // lane every 32nd column.  NV = ceil(W2 / 32) rounded up to a power of two: the column sums of a lane stay in registers, so
-// that the plane is read once, with FC_ROWS * NV loads of a lane in flight (HBM-bound; one walk for the rows and one for the
-// columns took 162 us at 8 x 135 x 240, C = 256).  NV = 0: any width, in the two walks.  Both add in the same order.
+// that the plane is read once, with ROWS * NV loads of a lane in flight (one walk for the rows and one for the
+// columns took 162 us at 8 x 135 x 240, C = 256; 62 now).  Bound by the latency of a block's few steps: at four columns a lane four rows a step
+// take 6.6 us for the levels of 1 x 55 x 128 where two take 9.8; at two columns (2 x 48 x 64) four take 10.7 and two 8.3, the coarse
+// levels having few rows; at eight (8 x 135 x 240) one takes 66 and four 73.  NV = 0: any width, in the two walks.  Both add in the same order.
 // grid (C, B, levels), block 256.
-constexpr int FC_ROWS = 2;
 struct MeansJobs {
   struct Job {
     const float* fmap2;
@@ -417,33 +418,34 @@ f2_means_cf_kernel(const __grid_constant__ MeansJobs jobs, int C, int op16) {
   const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
   const float* plane = fmap2 + ((size_t)b * C + c) * H2 * W2;
   const size_t out0 = (size_t)b * (H2 + W2) * C + c;
-  auto store_row = [&](int u, float acc) {   // acc: this lane's share of row u
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) store_mean(acc / (float)W2, out0 + (size_t)u * C, aux, auxh, op16, sc16);
-  };
   if constexpr (NV > 0) {
     float col[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) col[i] = 0.f;
-    for (int u0 = warp; u0 < H2; u0 += 8 * FC_ROWS) {
-      float v[FC_ROWS][NV];
+    constexpr int ROWS = NV == 4 ? 4 : 2;
+    for (int u0 = warp; u0 < H2; u0 += 8 * ROWS) {
+      float v[ROWS][NV], acc[ROWS];
 #pragma unroll
-      for (int r = 0; r < FC_ROWS; ++r)
+      for (int r = 0; r < ROWS; ++r)
 #pragma unroll
         for (int i = 0; i < NV; ++i)
           v[r][i] = u0 + 8 * r < H2 && lane + 32 * i < W2 ? __ldg(plane + (size_t)(u0 + 8 * r) * W2 + lane + 32 * i) : 0.f;
 #pragma unroll
-      for (int r = 0; r < FC_ROWS; ++r) {
-        if (u0 + 8 * r >= H2) break;
-        float acc = 0.f;
+      for (int r = 0; r < ROWS; ++r) {
+        acc[r] = 0.f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-          acc += v[r][i];
-          col[i] += v[r][i];
+          acc[r] += v[r][i];
+          if (u0 + 8 * r < H2) col[i] += v[r][i];
         }
-        store_row(u0 + 8 * r, acc);
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r)
+        if (lane == 0 && u0 + 8 * r < H2) store_mean(acc[r] / (float)W2, out0 + (size_t)(u0 + 8 * r) * C, aux, auxh, op16, sc16);
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i) red[warp][i][lane] = col[i];
@@ -455,6 +457,11 @@ f2_means_cf_kernel(const __grid_constant__ MeansJobs jobs, int C, int op16) {
       store_mean(acc / (float)H2, out0 + (size_t)(H2 + v) * C, aux, auxh, op16, sc16);
     }
   } else {
+    auto store_row = [&](int u, float acc) {   // acc: this lane's share of row u
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) store_mean(acc / (float)W2, out0 + (size_t)u * C, aux, auxh, op16, sc16);
+    };
     for (int u = warp; u < H2; u += 8) {
       float acc = 0.f;
 #pragma unroll 4
@@ -730,10 +737,9 @@ transpose_round_kernel(const __grid_constant__ TransposeJobs jobs, int C, int op
 
 // Channel-major copies straight from the model's feature maps (B, C, rows*width), times `scale`: as 16-bit operands (FP16: times the device
 // scalar as well) or TF32.  The layouts of channel_major_kernel, padding included (zeros), two values per store.  A thread makes CM_PAIRS
-// pairs, 512 values apart, with all loads first: with one pair a thread HBM waited for them (8 x 47 x 156, C = 256: 81 us, 39 now; with eight pairs 33, but 10.6 instead of
-// 9.4 for the levels of 2 x 48 x 64).  The two
-// values of a pair are one load where every pair of a copy lies on 8 bytes.  One grid row per
-// channel of a sample: grid (sum over the copies of ceil(pairs per channel / (256 * CM_PAIRS)), C, B).
+// pairs, 512 values apart, with all loads first: with one pair a thread HBM waited for them (8 x 47 x 156, C = 256: 81 us, 39 now; with eight
+// pairs 33, but 10.6 instead of 9.4 for the levels of 2 x 48 x 64).  The two values of a pair are one load where every pair of a copy lies on
+// 8 bytes.  One grid row per channel of a sample: grid (sum over the copies of ceil(pairs per channel / (256 * CM_PAIRS)), C, B).
 constexpr int CM_PAIRS = 4;
 struct MapCopies {
   MapCopy c[MAX_MAP_COPIES];
