@@ -537,13 +537,13 @@ cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& 
   return f.fmaps ? launch_prepare_cf(&d, 1, f.F1, &f.F2, f.scale1, &out, F1r, F1h, w.status, st, op16, w.scales)
                  : launch_prepare(d, f.F1, f.F2, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales);
 }
-// Launches of the above: FP16 operands add the search for the magnitudes.
-int prepare_launches(const Workspace& w, bool with_aux, int op16) {
+// Launches of the above: FP16 operands add the search for the magnitudes; pixel-major features have copies and mean rows in one.
+int prepare_launches(const Workspace& w, bool fmaps, bool with_aux, int op16) {
   const bool copies = !op16 || w.F1h != nullptr;
-  return (copies ? 1 : 0) + (with_aux ? 1 : 0) + (op16 == OP16_FP16 ? 1 : 0);
+  return (fmaps ? (copies ? 1 : 0) + (with_aux ? 1 : 0) : (copies || with_aux ? 1 : 0)) + (op16 == OP16_FP16 ? 1 : 0);
 }
 #define SFB_PREPARE(f, with_aux) \
-  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, with_aux, (f).op16), st, [&] { return prepare_operands(d, w, f, with_aux, st); }))
+  SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, (f).fmaps, with_aux, (f).op16), st, [&] { return prepare_operands(d, w, f, with_aux, st); }))
 
 int run_maxavg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, int32_t* AM_u, int32_t* AM_v,
                        bool with_argmax, const sfb_shape* shape, void* ws, size_t ws_bytes, void* stream) {
@@ -1684,7 +1684,7 @@ int prepare_pyramid(const Pyramid& py, const Workspace* w, const float* fmap1, c
   for (int l = 0; l < py.levels; ++l)
     out[l] = op16 ? LevelOperands{nullptr, nullptr, w[l].F2h, with_aux ? w[l].auxh : nullptr}
                   : LevelOperands{w[l].F2r, with_aux ? w[l].aux : nullptr, nullptr, nullptr};
-  const int launches = prepare_launches(w[0], with_aux, op16) + (pooled != nullptr && op16 != OP16_FP16 ? 1 : 0);
+  const int launches = prepare_launches(w[0], true, with_aux, op16) + (pooled != nullptr && op16 != OP16_FP16 ? 1 : 0);
   SFB_CUDA(timed(KID_PREPARE, launches, st, [&] {
     return launch_prepare_cf(py.d, py.levels, fmap1, fmap2, scale1, out, op16 ? nullptr : w[0].F1r, op16 ? w[0].F1h : nullptr, w[0].status,
                              st, op16, w[0].scales, pooled);

@@ -316,7 +316,7 @@ cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int
 }
 
 // Both images of a call: rounded to TF32 in `out`, or in `outh` as 16-bit operands of kind `op16` (BF16, or FP16 of the value times the
-// device scalar *scale16); the one that is not wanted is null.  grid (blocks, 2), block 256.
+// device scalar *scale16); the one that is not wanted is null.
 struct RoundJob {
   const float4* in;
   float4* out;
@@ -324,11 +324,10 @@ struct RoundJob {
   const float* scale16;
   size_t n4;
 };
-__global__ void round_copy_kernel(const RoundJob j1, const RoundJob j2, int op16) {
-  const RoundJob& j = blockIdx.y == 0 ? j1 : j2;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
+__device__ __forceinline__ void round_copy(const RoundJob& j, int op16, int block, int blocks) {
+  const size_t stride = (size_t)blocks * blockDim.x;
   const float sc = (j.outh != nullptr && j.scale16 != nullptr) ? __ldg(j.scale16) : 1.f;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < j.n4; i += stride) {
+  for (size_t i = (size_t)block * blockDim.x + threadIdx.x; i < j.n4; i += stride) {
     float4 v = __ldg(j.in + i);
     if (j.outh != nullptr) {
       if (op16 == OP16_FP16) j.outh[i] = make_uint2(pack_fp16x2(v.x * sc, v.y * sc), pack_fp16x2(v.z * sc, v.w * sc));
@@ -347,14 +346,22 @@ __device__ __forceinline__ void store_mean(float mean, size_t at, float* aux, ui
   if (auxh != nullptr) auxh[at] = to_op16(mean * sc16, op16);
 }
 
-// From pixel-major features.  A block owns one mean row; four groups of 64 threads take every fourth pixel of it, a
-// thread four channels at a time, so that the pixels' loads are in flight side by side.  grid (H2 + W2, B), block 256.
+// From pixel-major features, in one launch with the copies (1 x 48 x 64, C = 256: 4 + 4.5 us apart, 3.6 together).  A block owns one mean
+// row; four groups of 64 threads take every fourth pixel of it, a
+// thread four channels at a time, so that the pixels' loads are in flight side by side.  The blocks of the mean rows come first.
+// grid (mean_rows * B + copies1 + copies2), block 256.
 constexpr int FM_GROUPS = 4, FM_QUADS = 64;
 __global__ void __launch_bounds__(FM_GROUPS * FM_QUADS)
-f2_means_kernel(const float* __restrict__ F2, float* __restrict__ aux, int H2, int W2, int C,
-                uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
+round_means_kernel(const RoundJob j1, const RoundJob j2, int copies1, int copies2, const float* __restrict__ F2, float* __restrict__ aux, int mean_rows,
+                   int B, int H2, int W2, int C, uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
   __shared__ float4 red[FM_GROUPS][FM_QUADS];
-  const int r = blockIdx.x, b = blockIdx.y, g = threadIdx.x / FM_QUADS, q = threadIdx.x % FM_QUADS;
+  const int block = (int)blockIdx.x - mean_rows * B;
+  if (block >= 0) {
+    if (block < copies1) round_copy(j1, op16, block, copies1);
+    else round_copy(j2, op16, block - copies1, copies2);
+    return;
+  }
+  const int b = blockIdx.x / mean_rows, r = blockIdx.x - b * mean_rows, g = threadIdx.x / FM_QUADS, q = threadIdx.x % FM_QUADS;
   const float sc16 = (op16 == OP16_FP16 && scale16 != nullptr) ? __ldg(scale16) : 1.f;
   const int count = r < H2 ? W2 : H2;
   const size_t step = r < H2 ? (size_t)C : (size_t)W2 * C;   // between the pixels of the row / column
@@ -914,13 +921,15 @@ cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, floa
   const size_t n1 = (size_t)d.B * d.N1() * d.C / 4, n2 = (size_t)d.B * d.N2() * d.C / 4;  // C % 4 == 0
   const int threads = 256;
   auto blocks = [&](size_t n) { return (unsigned)std::min<size_t>((n + threads - 1) / threads, 148 * 16); };
-  if (F1r != nullptr || F1h != nullptr) {
-    const RoundJob j1{reinterpret_cast<const float4*>(F1), reinterpret_cast<float4*>(F1r), reinterpret_cast<uint2*>(F1h), s1, n1};
-    const RoundJob j2{reinterpret_cast<const float4*>(F2), reinterpret_cast<float4*>(F2r), reinterpret_cast<uint2*>(F2h), s2, n2};
-    round_copy_kernel<<<dim3(blocks(std::max(n1, n2)), 2), threads, 0, stream>>>(j1, j2, op16);
-  }
-  if (aux != nullptr || auxh != nullptr)
-    f2_means_kernel<<<dim3(d.H2 + d.W2, d.B), FM_GROUPS * FM_QUADS, 0, stream>>>(F2, aux, d.H2, d.W2, d.C, auxh, op16, s2);
+  const bool copies = F1r != nullptr || F1h != nullptr, means = aux != nullptr || auxh != nullptr;
+  if (!copies && !means) return cudaSuccess;
+  const RoundJob j1{reinterpret_cast<const float4*>(F1), reinterpret_cast<float4*>(F1r), reinterpret_cast<uint2*>(F1h), s1, n1};
+  const RoundJob j2{reinterpret_cast<const float4*>(F2), reinterpret_cast<float4*>(F2r), reinterpret_cast<uint2*>(F2h), s2, n2};
+  const unsigned c1 = copies ? blocks(n1) : 0, c2 = copies ? blocks(n2) : 0;
+  const int mean_rows = means ? d.H2 + d.W2 : 0;
+  const long long grid = (long long)mean_rows * d.B + c1 + c2;
+  if (grid > INT_MAX) return cudaErrorInvalidConfiguration;
+  round_means_kernel<<<(unsigned)grid, threads, 0, stream>>>(j1, j2, (int)c1, (int)c2, F2, aux, mean_rows, d.B, d.H2, d.W2, d.C, auxh, op16, s2);
   return cudaGetLastError();
 }
 
