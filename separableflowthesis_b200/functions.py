@@ -393,14 +393,13 @@ class LookupPairFunction(Function):
     @staticmethod
     def forward(ctx, corr1, corr2, pyramid1, pyramid2, coords, edge1, edge2, levels, radius):
         out1, out2 = MemorySaver.lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels, radius)
+        ctx.cfg = (tuple(corr1.shape), tuple(corr2.shape), levels, radius)
+        ctx.set_materialize_grads(False)
         if edge1 is not None or edge2 is not None:
             ctx.save_for_backward(coords)
-            ctx.cfg = (tuple(corr1.shape), tuple(corr2.shape), levels, radius)
-            ctx.set_materialize_grads(False)
-            if edge1 is None:
-                ctx.mark_non_differentiable(out1)
-            elif edge2 is None:
-                ctx.mark_non_differentiable(out2)
+            # (with coordinates that need a gradient, and get none, both outputs stay differentiable, whatever the volumes need)
+            if not ctx.needs_input_grad[4]:
+                ctx.mark_non_differentiable(*[out for out, edge in ((out1, edge1), (out2, edge2)) if edge is None])
         return out1, out2, edge1, edge2
 
     @staticmethod

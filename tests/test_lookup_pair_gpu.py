@@ -97,6 +97,12 @@ def test_autograd_of_a_chain(cuda_device):
     assert not o1.requires_grad and o2.requires_grad
     (g2,) = torch.autograd.grad((o2 * o2).sum(), [v2])
     assert torch.equal(g2, ref[0][3])
+    # coordinates that need a gradient get none, whatever the volumes need
+    for vols in ((v1.detach(), v2.detach()), (v1, v2.detach()), (v1.detach(), v2)):
+        c = coords[0].clone().requires_grad_(True)
+        o1, o2 = sfb.CorrBlock1D(*vols)(c)
+        got = torch.autograd.grad((o1 * o1).sum() + o2.sum(), [c] + [v for v in vols if v.requires_grad], allow_unused=True)
+        assert got[0] is None and all(x is not None for x in got[1:])
     # chains of two lookups
     block = sfb.CorrBlock1D(v1, v2)
     block.CHAIN = 2
