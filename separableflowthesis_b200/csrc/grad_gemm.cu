@@ -51,6 +51,8 @@
 // Warp roles: warp 0 feature (B operand) producer, warp 1 TMEM allocation + MMA issue, warps 2..9 generate G
 // and, at the end, drain the accumulator (two warps per TMEM lane quarter, alternating 16-column chunks),
 // warp 10 producer of the XU / XV blocks; storing: warp 11 copies the blocks to memory.
+#include <climits>
+
 #include <cuda_bf16.h>
 
 #include "kernels.h"
@@ -652,14 +654,17 @@ __device__ __forceinline__ int grad_level(const int (&first)[LEVELS + 1], int bl
 
 // The parts of a tile in scratch added to the output, in their order, four values to a thread.  A kernel of its own: added up by
 // the CTA that finished a tile last, the 128 KB of every piece came through that one SM.
+// grid (tails * grad_fold_blocks): the levels of a large batch have more tails than grid.y takes.
 constexpr int GG_FOLD_THREADS = 256;
+__host__ __device__ constexpr int grad_fold_blocks(int C) { return (C * (TILE_M / 4) + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS; }
 template <int FORM, int LEVELS>
 __global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const __grid_constant__ GradLaunch<LEVELS> launch) {
-  const int level = grad_level<LEVELS>(launch.first_tail, blockIdx.y);
+  const int C = launch.a[0].d.C, per_tail = grad_fold_blocks(C), t = blockIdx.x / per_tail;   // C is a multiple of 4
+  const int level = grad_level<LEVELS>(launch.first_tail, t);
   const GradArgs& a = launch.a[level];
   if (*reinterpret_cast<volatile int*>(a.status) != 0) return;
-  const int C = a.d.C, tail = LEVELS == 1 ? blockIdx.y : blockIdx.y - launch.first_tail[level];   // C is a multiple of 4
-  const int i = blockIdx.x * GG_FOLD_THREADS + threadIdx.x;   // four neighbours of the parts' layout (grad_part)
+  const int tail = LEVELS == 1 ? t : t - launch.first_tail[level];
+  const int i = (blockIdx.x - t * per_tail) * GG_FOLD_THREADS + threadIdx.x;   // four neighbours of the parts' layout (grad_part)
   if (i >= C * (TILE_M / 4)) return;
   GradSched sc;
   constexpr bool STORED = FORM == GRAD_IMAGE2_STORED;   // tails are halves of a tile
@@ -893,8 +898,9 @@ static cudaError_t launch_one(GradLaunch<LEVELS>& launch, int levels, cudaStream
   kern<<<blocks, gg_threads<FORM>(), smem_bytes, stream>>>(launch, launch.a[0].status);
   if (tails > 0) {
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    const int items = launch.a[0].d.C * (TILE_M / 4);
-    grad_fold_kernel<FORM, LEVELS><<<dim3((items + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS, tails), GG_FOLD_THREADS, 0, stream>>>(launch);
+    const long long fold_blocks = (long long)tails * grad_fold_blocks(launch.a[0].d.C);
+    if (fold_blocks > INT_MAX) return cudaErrorInvalidConfiguration;
+    grad_fold_kernel<FORM, LEVELS><<<(unsigned)fold_blocks, GG_FOLD_THREADS, 0, stream>>>(launch);
   }
   return cudaGetLastError();
 }

@@ -28,3 +28,31 @@ def test_fused_backward(B, Kc, cuda_device):
     G, F1, F2 = G.double(), F1.double(), F2.double()
     assert torch.equal(gF1.double(), (G[..., None] * F2[:, None, None]).sum((3, 4)))
     assert torch.equal(gF2.double(), (G[..., None] * F1[:, :, :, None, None]).sum((1, 2)))
+
+
+# The gradients of image 1 are summed over the levels tile by tile: 16 384 x 4 of 128 pixels and more than 65535 of them.  C = 4 runs with
+# TF32 operands and never hands G over, in parts of the batch or otherwise.
+@pytest.mark.parametrize("B", [16384, 16390])
+def test_pyramid_backward(B, cuda_device):
+    C, H1, W1, Kc, sizes = 4, 16, 25, 1, [(2, 4), (1, 2)]
+    Kt, dev = 2 + Kc, cuda_device
+    g = torch.Generator(device=dev).manual_seed(B)
+    randn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    f1, pyr = randn(B, C, H1, W1), [randn(B, C, h, w) for h, w in sizes]
+    params = [randn(Kc, 2, 3, 3, 3) * 0.2, randn(Kc) * 0.1, randn(Kc, 2, 3, 3, 3) * 0.2, randn(Kc) * 0.1]
+    gu, gv = randn(B, 2 * Kt, 4, H1, W1), randn(B, 2 * Kt, 2, H1, W1)
+
+    def both(part):
+        maps = f1[part].contiguous(), [f2[part].contiguous() for f2 in pyr]
+        sep_u, sep_v, buffer = ops.separation_pyramid_forward(*maps, *params, True, 0.5)
+        return ops.separation_pyramid_backward(*maps, params[0], params[2], sep_u, sep_v, buffer, gu[part].contiguous(), gv[part].contiguous(), 0.5)
+
+    whole = both(slice(None))
+    parts = [both(slice(i, i + 4100)) for i in range(0, B, 4100)]
+    # per sample: the same products, sums of up to 400 or 10 of them in other pieces (2^-23 of the result each)
+    relerr = lambda x, ref: ((x.double() - ref.double()).norm() / ref.double().norm()).item()
+    assert relerr(whole[0], torch.cat([p[0] for p in parts])) < 400 * 2 ** -23
+    for l in range(2):
+        assert relerr(whole[1][l], torch.cat([p[1][l] for p in parts])) < 400 * 2 ** -23
+    for i in (2, 4):   # parameters: sums over the batch, in the order of blocks and of parts (2^-24 of a few thousand terms that cancel)
+        assert relerr(whole[i], sum(p[i].double() for p in parts)) < 1e-4
