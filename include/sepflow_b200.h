@@ -67,7 +67,8 @@ enum {
   SFB_OP_SEPARATION_LEVEL_BACKWARD = 10
 };
 
-/* Scratch bytes an op needs for `shape` (0 if the shape is invalid). */
+/* Scratch bytes an op uses for `shape` (0 if the shape is invalid) with the operands that are set (sfb_set_sweep_operands).  A backward's
+ * include room for the gradient of the volume, which it generates twice where there is none. */
 size_t sfb_workspace_bytes(int op, const sfb_shape* shape);
 
 /* Replaces MemorySaver.max_avg_forward (MemorySaver_cuda.cpp:10-21 -> MemorySaver_kernel_forward.cu:901-949). */
@@ -233,6 +234,9 @@ int sfb_separation_level_backward_fmaps(const float* fmap1, const float* fmap2, 
  * what its averages contribute. */
 size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
                                           int32_t with_argmax, int32_t pooled);
+/* Workspace of the forward (backward = 0) or the backward (1; 2: the least that it takes).  With 16-bit operands the backward's has room
+ * for the gradient of the volume, up to 4 GiB of it at a time: the gradient GEMMs then generate it once and not twice.  It uses what
+ * there is room for, and the size follows the operands that are set (sfb_set_sweep_operands) when it is asked for. */
 size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
                                               int32_t backward);
 int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,

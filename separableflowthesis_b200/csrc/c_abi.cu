@@ -215,6 +215,15 @@ GradArgs with_wait_settings(GradArgs a) {
   return a;
 }
 
+// Operand type of a call's contractions: the process-wide switch (sfb_set_sweep_operands), as OP16_NONE (TF32), OP16_BF16 or OP16_FP16.
+// 16-bit rows must be multiples of 16 bytes for TMA: with FP16 operands, which have the precision of TF32, other shapes run with the
+// latter; with BF16 operands they are refused (operand_mode).
+int op16_of(const Dims& d) {
+  const int m = g_sweep_operands.load();
+  if (d.C % 8 != 0) return OP16_NONE;
+  return m == SFB_OPERANDS_BF16 ? OP16_BF16 : (m == SFB_OPERANDS_FP16 ? OP16_FP16 : OP16_NONE);
+}
+
 struct Workspace {
   int* status;
   float* scales;  // scale slots of the FP16 operand kind (kernels.h, SCALE_*), in the header after the status word
@@ -242,7 +251,8 @@ struct Workspace {
   size_t bytes;        // without the scratch of the tail pieces, which a caller's buffer may lack (the kernels then
   float* part;         // do whole tiles only)
   size_t part_bytes;
-  uint8_t* stored;     // G between the gradient GEMMs, behind the scratch; a buffer may lack it as well (G is then generated twice)
+  uint8_t* stored;     // G between the gradient GEMMs (16-bit operands), behind the scratch; a buffer may lack it as well (G is then
+                       // generated twice)
   size_t stored_bytes;  // the samples that the buffer has room for
 };
 
@@ -289,9 +299,9 @@ WsPlan plan_for(int op, const Dims& d) {
 bool grad_hands_over(const Dims& d, int levels) {
   return d.N2() > 4096 || (d.N2() >= 512 && (long long)d.B * ((d.N1() + TILE_M - 1) / TILE_M) * levels > SM_COUNT);
 }
-// Samples whose G (`bytes` each) is stored at a time: all, as many as fit, or (0) none.
-int grad_chunk(const Dims& d, int levels, size_t bytes) {
-  return grad_hands_over(d, levels) ? (int)std::min<size_t>(d.B, GRAD_STORED_LIMIT / bytes) : 0;
+// Samples whose G (`bytes` each) is stored at a time: all, as many as fit, or (0) none.  With TF32 operands it is generated twice.
+int grad_chunk(const Dims& d, int levels, size_t bytes, int op16) {
+  return op16 != OP16_NONE && grad_hands_over(d, levels) ? (int)std::min<size_t>(d.B, GRAD_STORED_LIMIT / bytes) : 0;
 }
 
 Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
@@ -340,7 +350,7 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   size_t part = 0;
   if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS, false).part_floats);
   if (d.Kc > 0 && plan.sweeps) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
-  const int samples = plan.Rg ? grad_chunk(d, 1, grad_stored_bytes(d, w.n1p)) : 0;
+  const int samples = plan.Rg ? grad_chunk(d, 1, grad_stored_bytes(d, w.n1p), op16_of(d)) : 0;
   if (plan.Rg) {
     for (const int form : {GRAD_IMAGE1, GRAD_IMAGE2}) part = std::max(part, grad_split(d, form).part_floats);
     for (const int n : {samples, samples > 0 ? d.B % samples : 0}) {   // full chunks and what is left
@@ -474,16 +484,10 @@ int map_aux(CUtensorMap* tm, const Dims& d, const void* aux, bool bf16 = false) 
   return make_map(tm, aux, 3, dims, box, CU_TENSOR_MAP_SWIZZLE_128B, bf16);
 }
 
-// Operand type of this call's contractions: the process-wide switch (sfb_set_sweep_operands), as OP16_NONE (TF32),
-// OP16_BF16 or OP16_FP16.
 int operand_mode(const Dims& d, int* op16) {
-  const int m = g_sweep_operands.load();
-  *op16 = m == SFB_OPERANDS_BF16 ? OP16_BF16 : (m == SFB_OPERANDS_FP16 ? OP16_FP16 : OP16_NONE);
-  if (d.C % 8 != 0) {  // 16-bit rows must be multiples of 16 bytes for TMA
-    if (*op16 == OP16_BF16)
-      return fail(SFB_ERR_UNSUPPORTED_SHAPE, "BF16 operands need a feature dimension that is a multiple of 8 (C=%d)", d.C);
-    *op16 = OP16_NONE;  // FP16 and TF32 operands have the same precision: such shapes run with TF32
-  }
+  if (d.C % 8 != 0 && g_sweep_operands.load() == SFB_OPERANDS_BF16)
+    return fail(SFB_ERR_UNSUPPORTED_SHAPE, "BF16 operands need a feature dimension that is a multiple of 8 (C=%d)", d.C);
+  *op16 = op16_of(d);
   return SFB_OK;
 }
 // What the sweeps multiply their outputs by: the inverse of the feature scales of FP16 operands, else nothing.
@@ -1561,14 +1565,50 @@ PyramidWorkspace carve_pyramid_forward(const Pyramid& py, void* base) {
   return p;
 }
 
-// The backward's: attention gradients, gradients of the max/avg channels, GEMM operands and image 2's copies per level, image 1's shared;
-// the gradients of the level's own volumes (gs_u, gs_v) where it is not in place; those of pooled levels of image 2 (gf2).
+// Cuts of the gradient GEMMs of a pyramid whose G is stored `samples` at a time (0: generated twice), for chunks of the batch and the
+// shorter last one, image-1-major and image-2-major; the scratch that the largest takes.
+struct PyramidGradPlan {
+  int samples;
+  TileSplit split[2][2][MAX_FUSED_LEVELS];
+  size_t part_bytes;
+};
+PyramidGradPlan plan_pyramid_grads(const Pyramid& py, int samples) {
+  PyramidGradPlan plan;
+  plan.samples = samples;
+  size_t part = 0;
+  const int B = py.d[0].B, chunk = samples > 0 ? samples : B;
+  for (const int last : {0, 1}) {
+    Dims d[MAX_FUSED_LEVELS];
+    for (int l = 0; l < py.levels; ++l) {
+      d[l] = py.d[l];
+      d[l].B = last ? B % chunk : chunk;
+    }
+    if (d[0].B == 0) continue;
+    for (const int image2 : {0, 1}) {
+      TileSplit* const split = plan.split[last][image2];
+      grad_split_levels(d, py.levels, samples > 0 ? (image2 ? GRAD_IMAGE2_STORED : GRAD_IMAGE1_STORING) : (image2 ? GRAD_IMAGE2 : GRAD_IMAGE1), split);
+      size_t floats = 0;
+      for (int l = 0; l < py.levels; ++l) floats += split[l].part_floats;
+      part = std::max(part, floats);
+    }
+  }
+  plan.part_bytes = align_up(part * sizeof(float), 256);
+  return plan;
+}
+
+// The backward's buffer: the header and the gradients of pooled levels of image 2 (gf2), then two regions of which each is used twice.
+//   first : the copies of the sweep, the attention gradients and the scratch of both; then, once those are through, the GEMMs' operands
+//           and channel-major copies
+//   second: the gradients of the max/avg channels and of the volumes that are not in place (gs_u, gs_v), which the operands are packed
+//           from; then the GEMMs' scratch and G
+// Image 1's copies are shared by the levels.  8 x 135 x 240, C = 256, four channels and levels: 12.9 GB with room for G, 20.2 with all arrays
+// side by side; a level alone takes 8.1, 12.3 with room for G.
 struct PyramidBackward {
   Workspace w[MAX_FUSED_LEVELS];
   float *gs_u[MAX_FUSED_LEVELS], *gs_v[MAX_FUSED_LEVELS], *gf2[MAX_FUSED_LEVELS];
-  int samples;             // whose G of all levels is stored at a time (0: none)
-  size_t bytes;            // without the stored G, which a caller's buffer may lack
-  size_t stored_bytes;
+  size_t second, end;      // where the second region begins, and ends before the GEMMs
+  size_t sample_bytes;     // stored G of a sample
+  size_t bytes(const PyramidGradPlan& plan) const { return std::max(end, second + plan.part_bytes + plan.samples * sample_bytes); }
 };
 PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
   PyramidBackward p;
@@ -1582,61 +1622,75 @@ PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
   const size_t bn = (size_t)d0.B * d0.N1();
   const int n1p = padded_pixels(d0), Kt = 2 + d0.Kc, Rg = 4 + grad_slots(d0.Kc);
   int* const status = reinterpret_cast<int*>(take(WS_HEADER_BYTES / sizeof(float)));
-  float* const F1 = take(bn * d0.C);
-  float* const F1t = take((size_t)d0.B * d0.C * n1p);
-  AttentionDims at[MAX_ATTENTION_JOBS];
   for (int l = 0; l < py.levels; ++l) {
-    const Dims& d = py.d[l];
     Workspace& w = p.w[l];
     w = Workspace{};
     w.status = status;
     w.scales = reinterpret_cast<float*>(reinterpret_cast<char*>(status) + WS_SCALES_OFFSET) + l * SCALE_LEVEL;
     w.n1p = n1p;
+    p.gf2[l] = l == 0 ? nullptr : take((size_t)py.d[l].B * py.d[l].C * py.d[l].N2());
+  }
+  const size_t first = off;
+  float* const F1 = take(bn * d0.C);
+  AttentionDims at[MAX_ATTENTION_JOBS];
+  for (int l = 0; l < py.levels; ++l) {
+    const Dims& d = py.d[l];
+    Workspace& w = p.w[l];
     w.F1r = F1;
     w.F2r = take((size_t)d.B * d.N2() * d.C);
     w.F1h = reinterpret_cast<uint16_t*>(w.F1r);
     w.F2h = reinterpret_cast<uint16_t*>(w.F2r);
+    w.ga_u = take(bn * d.Kc * d.W2);
+    w.ga_v = take(bn * d.Kc * d.H2);
+    at[2 * l] = AttentionDims{d.B, d.Kc, d.W2, d.H1, d.W1};
+    at[2 * l + 1] = AttentionDims{d.B, d.Kc, d.H2, d.H1, d.W1};
+  }
+  TileSplit split[MAX_FUSED_LEVELS];
+  float* const parts = take(pyramid_part_floats(py, chunk_channels(d0.Kc), true, split));
+  float* const at_partial = take(attention_partial_floats(at, 2 * py.levels));
+  const size_t swept = off;
+  off = first;
+  float* const F1t = take((size_t)d0.B * d0.C * n1p);
+  for (int l = 0; l < py.levels; ++l) {
+    const Dims& d = py.d[l];
+    Workspace& w = p.w[l];
+    w.part = parts;
+    w.at_partial = at_partial;
     w.F1t = F1t;
     w.h2p = (d.H2 + GG_UT - 1) / GG_UT * GG_UT;
     w.F2t = take((size_t)d.B * f2t_per_sample(d, w));
     w.gxu = take((size_t)d.B * d.H2 * Rg * n1p);
     w.gxv = take((size_t)d.B * d.W2 * Rg * n1p);
-    w.ga_u = take(bn * d.Kc * d.W2);
-    w.ga_v = take(bn * d.Kc * d.H2);
+  }
+  p.second = off = std::max(swept, off);
+  p.sample_bytes = 0;
+  for (int l = 0; l < py.levels; ++l) {
+    const Dims& d = py.d[l];
+    Workspace& w = p.w[l];
     w.gm_u = take(bn * 2 * d.W2);
     w.gm_v = take(bn * 2 * d.H2);
     p.gs_u[l] = py.in_place[l] ? nullptr : take(bn * Kt * d.W2);
     p.gs_v[l] = py.in_place[l] ? nullptr : take(bn * Kt * d.H2);
-    p.gf2[l] = l == 0 ? nullptr : take((size_t)d.B * d.C * d.N2());
-    at[2 * l] = AttentionDims{d.B, d.Kc, d.W2, d.H1, d.W1};
-    at[2 * l + 1] = AttentionDims{d.B, d.Kc, d.H2, d.H1, d.W1};
+    p.sample_bytes += grad_stored_bytes(d, n1p);
   }
-  p.w[0].at_partial = take(attention_partial_floats(at, 2 * py.levels));
-  TileSplit split[MAX_FUSED_LEVELS];
-  size_t part = pyramid_part_floats(py, chunk_channels(d0.Kc), true, split), stored = 0;
-  for (int l = 0; l < py.levels; ++l) stored += grad_stored_bytes(py.d[l], n1p);
-  p.samples = grad_chunk(d0, py.levels, stored);
-  auto grad_parts = [&](int form, int samples) {
-    Dims d[MAX_FUSED_LEVELS];
-    for (int l = 0; l < py.levels; ++l) {
-      d[l] = py.d[l];
-      d[l].B = samples;
-    }
-    grad_split_levels(d, py.levels, form, split);
-    size_t floats = 0;
-    for (int l = 0; l < py.levels; ++l) floats += split[l].part_floats;
-    part = std::max(part, floats);
-  };
-  for (const int form : {GRAD_IMAGE1, GRAD_IMAGE2}) grad_parts(form, d0.B);
-  for (const int n : {p.samples, p.samples > 0 ? d0.B % p.samples : 0})   // full chunks and what is left
-    for (const int form : {GRAD_IMAGE1_STORING, GRAD_IMAGE2_STORED})
-      if (n > 0) grad_parts(form, n);
-  float* const parts = take(part);
-  for (int l = 0; l < py.levels; ++l) p.w[l].part = parts;
-  p.bytes = off;
-  for (int l = 0; l < py.levels; ++l) p.w[l].stored = reinterpret_cast<uint8_t*>(take(p.samples * grad_stored_bytes(py.d[l], n1p) / sizeof(float)));
-  p.stored_bytes = off - p.bytes;
+  p.end = off;
   return p;
+}
+// The most samples of G at a time that a buffer has room for.  Buffers of pyramid_backward_bytes() have it for all that are wanted.
+PyramidGradPlan pyramid_grad_plan(const Pyramid& py, const PyramidBackward& pb, int op16, size_t room) {
+  for (int n = grad_chunk(py.d[0], py.levels, pb.sample_bytes, op16); n > 0;) {
+    const PyramidGradPlan plan = plan_pyramid_grads(py, n);
+    if (pb.bytes(plan) <= room) return plan;
+    // the scratch may differ with the cut of a smaller chunk, so that its room is looked at again
+    n = std::min<long long>(n - 1, room > pb.second + plan.part_bytes ? (room - pb.second - plan.part_bytes) / pb.sample_bytes : 0);
+  }
+  return plan_pyramid_grads(py, 0);
+}
+// least: without room for G beyond what there is anyway.
+size_t pyramid_backward_bytes(const Pyramid& py, bool least) {
+  const PyramidBackward pb = carve_pyramid_backward(py, nullptr);
+  const size_t twice = pb.bytes(plan_pyramid_grads(py, 0));
+  return least ? twice : std::max(twice, pb.bytes(pyramid_grad_plan(py, pb, op16_of(py.d[0]), SIZE_MAX)));
 }
 
 // The sweeps of all levels: `fill(l, a)` sets a level's views, the rest is common.
@@ -1736,9 +1790,7 @@ size_t sfb_separation_pyramid_workspace_bytes(const sfb_shape* shape, const int3
                                               int32_t backward) {
   Pyramid py;
   if (check_pyramid(shape, H2, W2, levels, &py) != SFB_OK) return 0;
-  if (backward == 0) return carve_pyramid_forward(py, nullptr).bytes;
-  const PyramidBackward pb = carve_pyramid_backward(py, nullptr);
-  return pb.bytes + pb.stored_bytes;
+  return backward == 0 ? carve_pyramid_forward(py, nullptr).bytes : pyramid_backward_bytes(py, backward == 2);
 }
 
 int sfb_separation_pyramid_forward(const float* fmap1, const float* const* fmap2, const int32_t* H2, const int32_t* W2,
@@ -1829,13 +1881,14 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
   if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return fail(SFB_ERR_INVALID_ARGUMENT, "workspace is NULL or not 256-byte aligned");
   const PyramidBackward pb = carve_pyramid_backward(py, workspace);
-  if (workspace_bytes < pb.bytes)
-    return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", workspace_bytes, pb.bytes);
+  int op16;   // read once: it decides the plan, too
+  SFB_TRY(operand_mode(py.d[0], &op16));
+  const PyramidGradPlan plan = pyramid_grad_plan(py, pb, op16, workspace_bytes);
+  if (workspace_bytes < pb.bytes(plan))
+    return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", workspace_bytes, pb.bytes(plan));
   const Dims& d0 = py.d[0];
   const Workspace* const w = pb.w;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int op16;
-  SFB_TRY(operand_mode(d0, &op16));
   const float* maps2[MAX_FUSED_LEVELS];
   float* grads2[MAX_FUSED_LEVELS];
   for (int l = 0; l < levels; ++l) {
@@ -1921,26 +1974,25 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
   }
   SFB_CUDA(timed(KID_PACK, pack_launches(groups.count, d0.B), st, [&] { return launch_pack_interleaved_cf(groups, d0.B, N1, w[0].n1p, st); }));
   SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_channel_major_cf(copies, 1 + levels, d0.B, d0.C, op16, st); }));
-  const int samples = op16 != 0 && workspace_bytes >= pb.bytes + pb.stored_bytes ? pb.samples : 0;   // as in run_grad_pair
-  for (int b0 = 0; b0 < d0.B; b0 += samples > 0 ? samples : d0.B) {
+  // G of as many samples as the workspace takes is generated and stored by one GEMM and read back by the other (run_grad_pair)
+  const int samples = plan.samples, chunk = samples > 0 ? samples : d0.B;
+  for (int b0 = 0; b0 < d0.B; b0 += chunk) {
+    const int here = std::min(chunk, d0.B - b0);
     for (const int form : {samples > 0 ? GRAD_IMAGE1_STORING : GRAD_IMAGE1, samples > 0 ? GRAD_IMAGE2_STORED : GRAD_IMAGE2}) {
       const bool image2_major = grad_is_image2(form);
+      const TileSplit* const split = plan.split[here < chunk ? 1 : 0][image2_major ? 1 : 0];
       GradArgs a[MAX_FUSED_LEVELS];
       GradMaps maps;
-      TileSplit split[MAX_FUSED_LEVELS];
-      Dims d[MAX_FUSED_LEVELS];
-      for (int l = 0; l < levels; ++l) {
-        d[l] = py.d[l];
-        if (samples > 0) d[l].B = std::min(samples, d0.B - b0);
-      }
-      grad_split_levels(d, levels, form, split);
-      float* part = w[0].part;
+      float* part = reinterpret_cast<float*>(static_cast<char*>(workspace) + pb.second);
+      uint8_t* stored = reinterpret_cast<uint8_t*>(part) + plan.part_bytes;
       int part0 = -1, launches = 1;
       for (int l = 0; l < levels; ++l) {
         SFB_TRY(grad_arguments(py.d[l], w[l], op16, GRAD_FUSED, 4 * Q, form, image2_major ? grads2[l] : gfmap1, 1, scale1, &a[l], &maps.y[l],
                                &maps.xu[l], &maps.xv[l]));
-        a[l].d = d[l];
+        a[l].d.B = here;
         a[l].b0 = b0;
+        a[l].stored = stored;
+        stored += samples * grad_stored_bytes(py.d[l], w[l].n1p);
         a[l].whole_tiles = split[l].whole_tiles;
         a[l].pieces = split[l].pieces;
         a[l].parts = split[l].parts;

@@ -19,7 +19,8 @@ from . import _lib
 
 # Scratch buffers handed to the library, one per (device, stream): calls that share a workspace must be ordered on
 # one stream.  A buffer grows to the largest size asked for and is kept for reuse (12.3 GB for a level backward of
-# B=8, 135x240, Kc=4, 4.2 of them for the gradient of the volume, in parts); release_workspaces() drops them.  The lock covers DataParallel-style callers that run the ops
+# B=8, 135x240, Kc=4, 4.2 of them for the gradient of the volume, in parts; 12.9 GB for that of four levels together); release_workspaces()
+# drops them.  The lock covers DataParallel-style callers that run the ops
 # from several threads.
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 _workspaces_lock = threading.Lock()

@@ -6,7 +6,7 @@ import re
 
 import pytest
 
-from separableflowthesis_b200 import _lib, build
+from separableflowthesis_b200 import _lib, build, ops
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -152,3 +152,21 @@ def test_workspace_holds_the_copies_of_one_operand_type(lib):
     copies = 4 * C * (2 * H * W + H + W)    # both images and the mean rows of image 2
     assert lib.sfb_workspace_bytes(_lib.OP_MAX_AVG_FORWARD_CF, ctypes.byref(s)) == 1024 + copies
     assert lib.sfb_workspace_bytes(_lib.OP_COMPRESSION_CF, ctypes.byref(s)) == 1024 + 4 * C * 2 * H * W
+
+
+def test_pyramid_backward_workspace_follows_the_operands(lib):
+    """Room for the gradient of the volume is asked for with 16-bit operands alone, and a buffer of four levels stays below what its
+    arrays would take side by side (8 x 135 x 240, C = 256, four channels: 20.2 GB)."""
+    def sizes(B, H, W, C, Kc, levels, operands):
+        s = _lib.SfbShape(B, H, W, H, W, C, Kc)
+        h, w = [(ctypes.c_int32 * levels)(*[n >> l for l in range(levels)]) for n in (H, W)]
+        with ops.sweep_operands(operands):
+            return [lib.sfb_separation_pyramid_workspace_bytes(ctypes.byref(s), h, w, levels, backward) for backward in (1, 2)]
+
+    for shape in ((2, 48, 64, 256, 2, 4), (8, 48, 64, 256, 2, 3), (8, 135, 240, 256, 4, 4), (8, 135, 240, 256, 4, 1), (2, 135, 240, 128, 4, 2)):
+        (full16, least16), (full32, least32) = sizes(*shape, "fp16"), sizes(*shape, "tf32")
+        assert full32 == least32 == least16 <= full16, shape
+        assert (full16, least16) == tuple(sizes(*shape, "bf16"))
+    assert sizes(8, 48, 64, 256, 2, 1, "fp16")[0] > sizes(8, 48, 64, 256, 2, 1, "tf32")[0]
+    assert sizes(8, 135, 240, 256, 4, 4, "fp16")[0] < 13e9
+    assert sizes(8, 48, 64, 36, 2, 1, "fp16") == sizes(8, 48, 64, 36, 2, 1, "tf32")   # no 16-bit rows: TF32 either way
