@@ -229,9 +229,9 @@ int sfb_separation_level_backward_fmaps(const float* fmap1, const float* fmap2, 
  * above.  SEP_u (B,(2+Kc)*levels,W2[0],H1,W1) and SEP_v (B,(2+Kc)*levels,H2[0],H1,W1) are the concatenated outputs, each level
  * resampled to the displacement range of level 0.  `saved` (256-byte aligned) receives what a backward needs: the levels' own
  * volumes, attention weights and, with_argmax != 0, arg-max indices.
- * Image 2's levels may be made here: with fmap2[1..] NULL they are the 2 x 2 averages of one another (core/corr.py:377-382),
- * `saved` then holds them too (pooled != 0), and a backward with gfmap2[1..] NULL returns the gradient of fmap2[0] alone, with
- * what its averages contribute. */
+ * Image 2's levels may be made here: with fmap2[1..] NULL they are the 2 x 2 averages of one another (core/corr.py:377-382) and
+ * `saved` holds them too (pooled != 0).  A backward with gfmap2[1..] NULL returns the gradient of fmap2[0] alone, with what its
+ * averages contribute, whoever made them. */
 size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
                                           int32_t with_argmax, int32_t pooled);
 /* Workspace of the forward (backward = 0) or the backward (1; 2: the least that it takes).  With 16-bit operands the backward's has room
@@ -253,6 +253,10 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
                                     const float* gSEP_u, const float* gSEP_v, float* gfmap1, float* const* gfmap2,
                                     float* gweight_u, float* gbias_u, float* gweight_v, float* gbias_v,
                                     const sfb_shape* shape, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Those averages by themselves, in one launch: pooled[l-1] (B,C,H >> l,W >> l) for l = 1 .. levels-1, 2 to 4 levels, of fmap2 (B,C,H,W).
+ * The maps need no alignment beyond that of a float. */
+int sfb_pool_levels(const float* fmap2, float* const* pooled, int32_t B, int32_t C, int32_t H, int32_t W, int32_t levels, void* stream);
 
 /* Placement of one pyramid level's volumes into the concatenated outputs of the call site (core/corr.py:459-475:
  * F.interpolate(..., [D0,H1,W1], mode='trilinear', align_corners=True), then torch.cat over levels).  H1, W1 do not

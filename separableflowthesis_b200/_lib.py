@@ -47,7 +47,7 @@ EXPORTED_SYMBOLS = (
     "sfb_lookup4d_forward", "sfb_lookup4d_backward", "sfb_debug_wait_timeout", "sfb_lookup_build_pyramid_pair",
     "sfb_lookup_forward_pair", "sfb_lookup_accumulator_bytes", "sfb_lookup_accumulate_pair", "sfb_lookup_fold_gradient",
     "sfb_separation_pyramid_saved_bytes", "sfb_separation_pyramid_workspace_bytes", "sfb_separation_pyramid_forward",
-    "sfb_separation_pyramid_backward",
+    "sfb_separation_pyramid_backward", "sfb_pool_levels",
 )
 
 
@@ -132,6 +132,8 @@ def load() -> ctypes.CDLL:
     lib.sfb_separation_pyramid_forward.argtypes = [P, P, P, P, I32, ctypes.c_float] + [P] * 7 + [SZ, I32] + tail
     lib.sfb_separation_pyramid_backward.restype = ctypes.c_int
     lib.sfb_separation_pyramid_backward.argtypes = [P, P, P, P, I32, ctypes.c_float] + [P] * 5 + [SZ] + [P] * 8 + tail
+    lib.sfb_pool_levels.restype = ctypes.c_int
+    lib.sfb_pool_levels.argtypes = [P, P] + [I32] * 5 + [P]
     lib.sfb_max_avg_forward_static.restype = ctypes.c_int
     lib.sfb_max_avg_forward_static.argtypes = [P, P, P, P, SH, P]
     lib.sfb_static_scratch_bytes.restype = SZ

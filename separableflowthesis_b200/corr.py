@@ -24,7 +24,7 @@ import torch.nn.functional as F
 
 from .functions import (ComputeMaxArgmaxAvgFunction, ComputeMaxAvgFunction, ComputeSelfCompressionFunction,
                         FusedMaxArgmaxAvgFunction, FusedSelfCompressionFunction, SeparationCompressionCF,
-                        Lookup4dFunction, LookupFunction, LookupPairFunction, LookupVolumeFunction,
+                        Lookup4dFunction, LookupFunction, LookupPairFunction, LookupVolumeFunction, PooledLevelFunction,
                         SeparationLevelFunction, SeparationMaxAvgCF,
                         SeparationPooledPyramidFunction, SeparationPyramidFunction,
                         SeparationState)
@@ -55,27 +55,25 @@ class AlternateCorrBlockSepflow:
         self.num_levels = num_levels
         self.radius = radius
         self.fmap1_l0 = fmap1
-        self._fmap2, self._pyramid, self._grad_mode = fmap2, None, torch.is_grad_enabled()
-        # the call for all levels makes the pyramid itself; whoever reads it gets the tensors
-        if not (2 <= num_levels <= _ops.PYRAMID_MAX_LEVELS and fmap2.is_cuda and fmap2.dtype == torch.float32 and fmap2.dim() == 4
-                and min(fmap2.shape[2:]) >> (num_levels - 1) >= 1):
-            self._build_pyramid()
+        self._fmap2, self._pyramid, self._pooled, self._grad_mode = fmap2, None, None, torch.is_grad_enabled()
+        if (2 <= num_levels <= _ops.PYRAMID_MAX_LEVELS and fmap2.is_cuda and fmap2.dtype == torch.float32 and fmap2.dim() == 4
+                and min(fmap2.shape[2:]) >> (num_levels - 1) >= 1 and fmap2.numel() > 0):
+            # one launch; differentiable tensors for whoever reads them (the call for all levels takes them as they are)
+            self._pooled = _ops.pool_levels(fmap2.detach().contiguous(), num_levels)
+        else:
+            self._pyramid = [fmap2]
+            for _ in range(num_levels - 1):
+                self._pyramid.append(F.avg_pool2d(self._pyramid[-1], 2, stride=2))
         self._channels_last = None
-
-    def _build_pyramid(self):
-        level = self._fmap2
-        levels = [level]
-        with torch.set_grad_enabled(self._grad_mode):   # as the constructor was called
-            for _ in range(self.num_levels - 1):
-                level = F.avg_pool2d(level, 2, stride=2)
-                levels.append(level)
-        self._pyramid = levels
 
     @property
     def pyramid(self):
-        """Image 2's feature maps per level, average-pooled (core/corr.py:377-382)."""
+        """Image 2's feature maps per level, average-pooled as the block was made (core/corr.py:377-382)."""
         if self._pyramid is None:
-            self._build_pyramid()
+            with torch.set_grad_enabled(self._grad_mode):   # as the constructor was called
+                self._pyramid = [self._fmap2]
+                for level in self._pooled:
+                    self._pyramid.append(PooledLevelFunction.apply(self._pyramid[-1], (level,)))
         return self._pyramid
 
     @pyramid.setter
@@ -134,9 +132,9 @@ class AlternateCorrBlockSepflow:
                 and self._one_node_per_level(attention_weights)
                 and attention_weights[0].out_channels <= _ops.PYRAMID_MAX_CHANNELS and batch * (2 + attention_weights[0].out_channels) <= 65535):
             attention1, attention2 = attention_weights
-            return SeparationPooledPyramidFunction.apply(self.support_backward, 1.0 / math.sqrt(fdim), self.num_levels, attention1.weight,
+            return SeparationPooledPyramidFunction.apply(self.support_backward, 1.0 / math.sqrt(fdim), attention1.weight,
                                                          attention1.bias, attention2.weight, attention2.bias,
-                                                         self.fmap1_l0.contiguous(), self._fmap2.contiguous())
+                                                         self.fmap1_l0.contiguous(), self._fmap2.contiguous(), *self._pooled)
         h2, w2 = self.pyramid[0].shape[2:]
         if self._one_node_per_level(attention_weights) and self.num_levels > 1:
             # one node for the whole pyramid: levels are resampled along the displacement axis and written into

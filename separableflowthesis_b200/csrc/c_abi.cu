@@ -1779,6 +1779,26 @@ PixView volume_view(float* base, long long sb, int channel, int D, int N1) {
 
 extern "C" {
 
+int sfb_pool_levels(const float* fmap2, float* const* pooled, int32_t B, int32_t C, int32_t H, int32_t W, int32_t levels, void* stream) {
+  if (levels < 2 || levels > MAX_FUSED_LEVELS)
+    return fail(SFB_ERR_UNSUPPORTED_SHAPE, "levels must be in [2, %d] (got %d)", MAX_FUSED_LEVELS, levels);
+  if (B < 1 || C < 1 || H < 1 || W < 1 || std::min(H, W) >> (levels - 1) < 1)
+    return fail(SFB_ERR_INVALID_ARGUMENT, "%d levels need maps of at least one pixel each (got %d x %d x %d x %d)", levels, B, C, H, W);
+  if ((long long)B * C > INT_MAX || (long long)H * W > INT_MAX) return fail(SFB_ERR_UNSUPPORTED_SHAPE, "maps too large");
+  Dims d[MAX_FUSED_LEVELS];
+  float* out[MAX_FUSED_LEVELS] = {nullptr};
+  bool all = fmap2 != nullptr && pooled != nullptr;
+  for (int l = 0; l < levels; ++l) {
+    d[l] = Dims{B, 1, 1, H >> l, W >> l, C, 0};
+    if (l > 0 && all) out[l] = pooled[l - 1];
+    all = all && (l == 0 || out[l] != nullptr);
+  }
+  if (!all) return fail(SFB_ERR_INVALID_ARGUMENT, "fmap2 and pooled must not be NULL");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_pool_levels(d, levels, fmap2, out, st); }));
+  return SFB_OK;
+}
+
 size_t sfb_separation_pyramid_saved_bytes(const sfb_shape* shape, const int32_t* H2, const int32_t* W2, int32_t levels,
                                           int32_t with_argmax, int32_t pooled) {
   Pyramid py;
@@ -1872,7 +1892,7 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
   bool pooled, grads_pooled;
   SFB_TRY(check_levels(py, reinterpret_cast<const void* const*>(fmap2), "fmap2", &pooled));
   SFB_TRY(check_levels(py, reinterpret_cast<const void* const*>(gfmap2), "gfmap2", &grads_pooled));
-  if (pooled != grads_pooled) return fail(SFB_ERR_INVALID_ARGUMENT, "fmap2 and gfmap2 must both have all levels or both the first alone");
+  if (pooled && !grads_pooled) return fail(SFB_ERR_INVALID_ARGUMENT, "gfmap2 must be the first level alone where fmap2 is");
   if (weight_u == nullptr || weight_v == nullptr || gweight_u == nullptr || gbias_u == nullptr || gweight_v == nullptr ||
       gbias_v == nullptr)
     return fail(SFB_ERR_INVALID_ARGUMENT, "attention weights and their gradient buffers must not be NULL");
@@ -1893,7 +1913,7 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
   float* grads2[MAX_FUSED_LEVELS];
   for (int l = 0; l < levels; ++l) {
     maps2[l] = pooled && l > 0 ? sv.fmap2[l] : fmap2[l];
-    grads2[l] = pooled && l > 0 ? pb.gf2[l] : gfmap2[l];
+    grads2[l] = grads_pooled && l > 0 ? pb.gf2[l] : gfmap2[l];
   }
   SFB_TRY(prepare_pyramid(py, w, fmap1, maps2, nullptr, scale1, false, op16, st));
   const int N1 = d0.N1(), K = d0.Kc, Kt = 2 + K;
@@ -2006,7 +2026,7 @@ int sfb_separation_pyramid_backward(const float* fmap1, const float* const* fmap
       SFB_CUDA(timed(KID_GRAD_FUSED_IMG1 + (image2_major ? 1 : 0), launches, st, [&] { return launch_grad_gemm(a, levels, maps, st); }));
     }
   }
-  if (pooled)
+  if (grads_pooled)
     SFB_CUDA(timed(KID_PREPARE, 1, st, [&] { return launch_unpool_levels(py.d, levels, gfmap2[0], grads2, st); }));
   return SFB_OK;
 }

@@ -284,8 +284,10 @@ struct LevelOperands { float *F2r, *aux; uint16_t *F2h, *auxh; };
 [[nodiscard]] cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, const float* const* fmap2, float scale1,
                               const LevelOperands* out, float* F1r, uint16_t* F1h, int* status, cudaStream_t stream, int op16 = 0,
                               float* scales = nullptr, float* const* pooled = nullptr);
-// With `pooled`, the levels from the second on are made here, pooled[l] (= fmap2[l]) from the first; their gradients g[l] go back to the
-// first's, g0, with:
+// With `pooled`, the levels from the second on are made here, pooled[l] (= fmap2[l]) from the first.  The same without the rest, from and
+// to arrays of any alignment:
+[[nodiscard]] cudaError_t launch_pool_levels(const Dims* d, int levels, const float* fmap2, float* const* pooled, cudaStream_t stream);
+// Gradients g[l] of the averages, added to the first level's, g0:
 [[nodiscard]] cudaError_t launch_unpool_levels(const Dims* d, int levels, float* g0, const float* const* g, cudaStream_t stream);
 // Largest |x| * premul of each array, `samples` runs of n values sb apart, combined into its amax slot (SCALE_* of a level), and then the
 // multipliers that follow from the slots of every level: those of the features or (gradients) those of the gradient operands.

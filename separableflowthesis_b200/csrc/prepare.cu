@@ -217,8 +217,8 @@ pool_levels_kernel(const __grid_constant__ PoolJob job, float* scales) {
   }
 }
 
-static cudaError_t launch_pool_levels(const Dims* d, int levels, const float* fmap1, const float* fmap2, float* const* pooled,
-                                      float premul1, bool magnitudes, float* scales, cudaStream_t stream) {
+static cudaError_t launch_pool(const Dims* d, int levels, const float* fmap1, const float* fmap2, float* const* pooled,
+                               float premul1, bool magnitudes, float* scales, cudaStream_t stream) {
   PoolJob job{};
   job.in = fmap2;
   for (int l = 1; l < levels; ++l) job.out[l - 1] = pooled[l];
@@ -235,11 +235,15 @@ static cudaError_t launch_pool_levels(const Dims* d, int levels, const float* fm
   const long long blocks1 = magnitudes ? (long long)std::max<size_t>(1, std::min<size_t>((job.n1 + per_block - 1) / per_block, 148 * 8)) : 0;
   if (blocks1 + blocks2 > INT_MAX) return cudaErrorInvalidConfiguration;
   job.blocks2 = (int)blocks2;
-  const bool vec = job.W % 4 == 0;
+  const bool vec = job.W % 4 == 0 && reinterpret_cast<uintptr_t>(job.in) % 16 == 0;
   auto kern = magnitudes ? (vec ? pool_levels_kernel<true, true> : pool_levels_kernel<false, true>)
                          : (vec ? pool_levels_kernel<true, false> : pool_levels_kernel<false, false>);
   kern<<<(unsigned)(blocks1 + blocks2), AM_THREADS, 0, stream>>>(job, scales);
   return cudaGetLastError();
+}
+
+cudaError_t launch_pool_levels(const Dims* d, int levels, const float* fmap2, float* const* pooled, cudaStream_t stream) {
+  return launch_pool(d, levels, nullptr, fmap2, pooled, 1.f, false, nullptr, stream);
 }
 
 // Gradient of image 2 from those of its pooled levels, in place on level 0's: every level's gradient spreads evenly over the 2 x 2 entries
@@ -871,7 +875,7 @@ cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, con
   cudaError_t err;
   if (pooled != nullptr) {
     err = clear_header(levels, status, stream);
-    if (err == cudaSuccess) err = launch_pool_levels(d, levels, fmap1, fmap2[0], pooled, scale1, op16 == OP16_FP16 && scales != nullptr, scales, stream);
+    if (err == cudaSuccess) err = launch_pool(d, levels, fmap1, fmap2[0], pooled, scale1, op16 == OP16_FP16 && scales != nullptr, scales, stream);
   } else {
     err = begin_prepare(d, levels, fmap1, fmap2, scale1, status, op16, scales, stream);
   }

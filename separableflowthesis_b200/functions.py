@@ -318,16 +318,16 @@ class SeparationPyramidFunction(Function):
 
 
 class SeparationPooledPyramidFunction(Function):
-    """The same with the pyramid of image 2 made by the library from its first level: ``apply(with_argmax, scale1, levels, weight_u,
-    bias_u, weight_v, bias_v, fmap1, fmap2)`` on CUDA maps, 2 to 4 levels."""
+    """The same for the levels that ``pool_levels`` made of the first one, whose gradient has what they contribute: ``apply(with_argmax,
+    scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, *pooled)`` on CUDA maps, 2 to 4 levels with the first."""
 
     @staticmethod
-    def forward(ctx, with_argmax, scale1, levels, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2):
+    def forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, *pooled):
         params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
-        ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, levels
-        sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, [fmap2], *params, with_argmax, scale1, levels)
+        ctx.with_argmax, ctx.scale1 = with_argmax, scale1
+        sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, [fmap2, *pooled], *params, with_argmax, scale1)
         if with_argmax:
-            ctx.save_for_backward(fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, buffer)
+            ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, buffer, fmap2, *pooled)
         return sep_u, sep_v
 
     @staticmethod
@@ -335,11 +335,26 @@ class SeparationPooledPyramidFunction(Function):
     def backward(ctx, grad_sep_u, grad_sep_v):
         if not ctx.with_argmax:
             raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
-        fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, buffer = ctx.saved_tensors
+        fmap1, weight_u, weight_v, sep_u, sep_v, buffer, *levels = ctx.saved_tensors
         g1, (g2,), gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(
-            fmap1, [fmap2], weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, buffer, grad_sep_u.contiguous(),
-            grad_sep_v.contiguous(), ctx.scale1, ctx.levels)
-        return None, None, None, gw_u, gb_u, gw_v, gb_v, g1, g2
+            fmap1, levels, weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, buffer, grad_sep_u.contiguous(),
+            grad_sep_v.contiguous(), ctx.scale1, pooled=True)
+        return (None, None, gw_u, gb_u, gw_v, gb_v, g1, g2, *[None] * (len(levels) - 1))
+
+
+class PooledLevelFunction(Function):
+    """A level that ``pool_levels`` made of the one before, as a differentiable tensor: ``apply(finer, (level,))`` returns level, with the
+    gradient of avg_pool2d."""
+
+    @staticmethod
+    def forward(ctx, finer, level):
+        ctx.save_for_backward(finer)
+        return level[0]
+
+    @staticmethod
+    def backward(ctx, grad):
+        (finer,) = ctx.saved_tensors
+        return torch.ops.aten.avg_pool2d_backward(grad, finer, [2, 2], [2, 2], [0, 0], False, True, None), None
 
 
 # --------------------------------------------------------------------------------------------------

@@ -527,6 +527,18 @@ def _check_pyramid(fmap1, fmap2_levels, levels):
     return s
 
 
+def pool_levels(fmap2, levels):
+    """The coarser levels of image 2's pyramid, 2 x 2 averages of one another (core/corr.py:377-382), in one launch."""
+    _check(fmap2, "fmap2", torch.float32, 4)
+    B, C, H, W = fmap2.shape
+    out = [torch.empty(B, C, H >> l, W >> l, dtype=torch.float32, device=fmap2.device) for l in range(1, levels)]
+    lib = _lib.load()
+    ptrs = (ctypes.c_void_p * len(out))(*[t.data_ptr() for t in out])
+    with _on(fmap2.device):
+        _raise_on(lib.sfb_pool_levels(fmap2.data_ptr(), ptrs, B, C, H, W, levels, _stream(fmap2.device)), "sfb_pool_levels")
+    return out
+
+
 def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, bias_v, with_argmax, scale1, levels=None):
     """(sep_u, sep_v, saved): separation_level_forward of every level on the model's feature maps, resampled to the displacement range
     of level 0 and concatenated; `saved` is what the backward needs beside the inputs and outputs (one flat buffer).  With one map and the
@@ -556,9 +568,10 @@ def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, 
     return sep_u, sep_v, saved
 
 
-def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, g_sep_u, g_sep_v, scale1, levels=None):
-    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max; with pooled levels
-    the gradient of the one map."""
+def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, g_sep_u, g_sep_v, scale1, levels=None,
+                                pooled=False):
+    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max; where the library made
+    the levels, or they are the first one's ``pool_levels`` (``pooled``), the gradient of the one map."""
     L = levels or len(fmap2_levels)
     s = _check_pyramid(fmap1, fmap2_levels, L)
     dev = fmap1.device
@@ -571,7 +584,7 @@ def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, 
         _check_like(t, name, (s.B, Kt, D, s.H1, s.W1), torch.float32, dev)
     _check(saved, "saved", torch.uint8, 1)
     gF1 = torch.empty_like(fmap1)
-    gF2 = [torch.empty_like(f2) for f2 in fmap2_levels]
+    gF2 = [torch.empty_like(f2) for f2 in (fmap2_levels[:1] if pooled else fmap2_levels)]
     gw_u, gw_v = torch.empty_like(weight_u), torch.empty_like(weight_v)
     gb_u = torch.empty(s.Kc, dtype=torch.float32, device=dev)
     gb_v = torch.empty(s.Kc, dtype=torch.float32, device=dev)

@@ -131,7 +131,7 @@ def test_pooled_levels(shape, operands, cuda_device):
 
 
 def test_block_pyramid_on_demand(cuda_device):
-    """A block makes its pyramid when it is read, with the grad mode it was made in."""
+    """The differentiable levels of a block are made when they are read, with the grad mode the block was made in."""
     import separableflowthesis_b200 as sfb
     f1, pyr, _ = inputs(1, 32, 16, 24, 2, 3, 1, cuda_device)
     f2 = pyr[0].requires_grad_(True)
@@ -144,3 +144,79 @@ def test_block_pyramid_on_demand(cuda_device):
     assert not block.pyramid[1].requires_grad
     with pytest.raises(RuntimeError):
         sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=6)
+
+
+@pytest.mark.parametrize("shape", [(1, 32, 16, 24, 2, 3), (2, 64, 17, 33, 1, 4), (2, 32, 15, 31, 2, 2), (1, 36, 40, 60, 4, 4)])
+@pytest.mark.parametrize("layout", ["contiguous", "channels_last", "off a 16-byte boundary"])
+def test_block_takes_its_pyramid_when_made(shape, layout, cuda_device):
+    """The coarser levels are those of the maps as they are in the constructor (core/corr.py:377-382), whatever is written to them later,
+    and whether or not `pyramid` is read in between; level 0 is the maps themselves."""
+    import separableflowthesis_b200 as sfb
+    B, C, H, W, Kc, levels = shape
+    f1, pyr, params = inputs(B, C, H, W, Kc, levels, H + W, cuda_device)
+    modules = []
+    for i in (0, 2):
+        m = torch.nn.Conv3d(2, Kc, 3, padding=1).to(cuda_device)
+        with torch.no_grad():
+            m.weight.copy_(params[i])
+            m.bias.copy_(params[i + 1])
+        modules.append(m)
+    f2 = pyr[0]
+    if layout == "channels_last":
+        f2 = f2.contiguous(memory_format=torch.channels_last)
+    elif layout != "contiguous":
+        f2 = torch.empty(f2.numel() + 1, device=cuda_device)[1:].view_as(f2).copy_(f2)
+    for read in (False, True):
+        with torch.no_grad():
+            maps = f2.clone() if layout != "off a 16-byte boundary" else torch.empty(f2.numel() + 1, device=cuda_device)[1:].view_as(f2).copy_(f2)
+            block = sfb.AlternateCorrBlockSepflow(f1, maps, None, num_levels=levels)
+            maps.mul_(-0.5)
+            if read:
+                assert all(torch.equal(x, y) for x, y in zip(block.pyramid[1:], pyr[1:])) and block.pyramid[0] is maps
+            if layout == "off a 16-byte boundary":   # the library refuses such a level 0, as it always did
+                with pytest.raises(RuntimeError, match="aligned"):
+                    block(None, sep=True, attention_weights=modules)
+                continue
+            got = block(None, sep=True, attention_weights=modules)
+            want = ops.separation_pyramid_forward(f1, [(-0.5 * pyr[0]).contiguous(), *pyr[1:]], *params, False, 1 / math.sqrt(C))
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("shape", [(1, 32, 16, 24, 2, 3), (2, 64, 17, 33, 1, 4)])
+def test_block_gradients(shape, cuda_device):
+    """One call for all levels and their averages, and the same through the levels as tensors: equal gradients; a write to the maps
+    between forward and backward is noticed; the levels' gradients are avg_pool2d's, to the second derivative."""
+    import separableflowthesis_b200 as sfb
+    B, C, H, W, Kc, levels = shape
+    f1, pyr, _ = inputs(B, C, H, W, Kc, levels, H + W, cuda_device)
+    modules = [torch.nn.Conv3d(2, Kc, 3, padding=1).to(cuda_device) for _ in range(2)]
+    grads = []
+    for read in (False, True):
+        f2 = pyr[0].clone().requires_grad_(True)
+        block = sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=levels, support_backward=True)
+        if read:
+            block.pyramid
+        u, v = block(None, sep=True, attention_weights=modules)
+        grads.append(torch.autograd.grad((u * u).sum() + v.sum(), [f2, modules[0].weight, modules[1].weight]))
+    assert all(relerr(x, y) < 1e-6 for x, y in zip(*grads))
+    for read in (False, True):
+        f2 = pyr[0].clone().requires_grad_(True)
+        block = sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=levels, support_backward=True)
+        if read:
+            block.pyramid
+        loss = sum(x.sum() for x in block(None, sep=True, attention_weights=modules))
+        f2.data.add_(0)   # not tracked
+        with torch.no_grad():
+            f2.add_(0)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            loss.backward()
+    f2 = pyr[0].clone().requires_grad_(True)
+    made = sfb.AlternateCorrBlockSepflow(f1, f2, None, num_levels=levels).pyramid
+    chain = [f2]
+    for _ in range(levels - 1):
+        chain.append(F.avg_pool2d(chain[-1], 2, stride=2))
+    inner = [torch.autograd.grad([(t * t).sum() for t in p], p[1], retain_graph=True)[0] for p in (made, chain)]
+    assert torch.equal(*inner)
+    first = [torch.autograd.grad([(t * t * t).sum() for t in p], f2, create_graph=True)[0] for p in (made, chain)]
+    assert torch.equal(*first)
+    assert torch.equal(*[torch.autograd.grad((g * g).sum(), f2)[0] for g in first])
