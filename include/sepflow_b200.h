@@ -70,6 +70,8 @@ enum {
 /* Scratch bytes an op uses for `shape` (0 if the shape is invalid) with the operands that are set (sfb_set_sweep_operands).  A backward's
  * include room for the gradient of the volume, which it generates twice where there is none. */
 size_t sfb_workspace_bytes(int op, const sfb_shape* shape);
+/* The same without that room. */
+size_t sfb_workspace_least_bytes(int op, const sfb_shape* shape);
 
 /* Replaces MemorySaver.max_avg_forward (MemorySaver_cuda.cpp:10-21 -> MemorySaver_kernel_forward.cu:901-949). */
 int sfb_max_avg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, const sfb_shape* shape,

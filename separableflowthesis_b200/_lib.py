@@ -32,7 +32,7 @@ OP_SEPARATION_LEVEL_BACKWARD = 10
 
 # Every symbol include/sepflow_b200.h declares.
 EXPORTED_SYMBOLS = (
-    "sfb_workspace_bytes", "sfb_max_avg_forward", "sfb_max_argmax_avg_forward",
+    "sfb_workspace_bytes", "sfb_workspace_least_bytes", "sfb_max_avg_forward", "sfb_max_argmax_avg_forward",
     "sfb_max_argmax_avg_backward", "sfb_compression_forward", "sfb_compression_backward",
     "sfb_corr_volume", "sfb_device_status", "sfb_status_string", "sfb_last_error", "sfb_version",
     "sfb_kernel_timing_enable", "sfb_kernel_timing_count", "sfb_kernel_timing_read",
@@ -72,6 +72,8 @@ def load() -> ctypes.CDLL:
     tail = [SH, P, SZ, P]  # shape, workspace, workspace_bytes, stream
     lib.sfb_workspace_bytes.restype = SZ
     lib.sfb_workspace_bytes.argtypes = [ctypes.c_int, SH]
+    lib.sfb_workspace_least_bytes.restype = SZ
+    lib.sfb_workspace_least_bytes.argtypes = [ctypes.c_int, SH]
     for name, nptr in (("sfb_max_avg_forward", 4), ("sfb_max_argmax_avg_forward", 6),
                        ("sfb_max_argmax_avg_backward", 8), ("sfb_compression_forward", 6),
                        ("sfb_compression_backward", 10), ("sfb_corr_volume", 3),

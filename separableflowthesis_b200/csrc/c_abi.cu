@@ -304,7 +304,8 @@ int grad_chunk(const Dims& d, int levels, size_t bytes, int op16) {
   return op16 != OP16_NONE && grad_hands_over(d, levels) ? (int)std::min<size_t>(d.B, GRAD_STORED_LIMIT / bytes) : 0;
 }
 
-Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
+// stores: with room for G where the gradient GEMMs hand it over (else what they need to generate it twice).
+Workspace carve(const Dims& d, void* base, const WsPlan& plan, bool stores = true) {
   Workspace w;
   size_t off = 0;
   char* p = static_cast<char*>(base);
@@ -350,7 +351,7 @@ Workspace carve(const Dims& d, void* base, const WsPlan& plan) {
   size_t part = 0;
   if (plan.aux) part = std::max(part, sweep_split(d, MAXAVG_PART_SLOTS, false).part_floats);
   if (d.Kc > 0 && plan.sweeps) part = std::max(part, sweep_split(d, chunk_channels(d.Kc), true).part_floats);
-  const int samples = plan.Rg ? grad_chunk(d, 1, grad_stored_bytes(d, w.n1p), op16_of(d)) : 0;
+  const int samples = plan.Rg && stores ? grad_chunk(d, 1, grad_stored_bytes(d, w.n1p), op16_of(d)) : 0;
   if (plan.Rg) {
     for (const int form : {GRAD_IMAGE1, GRAD_IMAGE2}) part = std::max(part, grad_split(d, form).part_floats);
     for (const int n : {samples, samples > 0 ? d.B % samples : 0}) {   // full chunks and what is left
@@ -451,6 +452,7 @@ int check_workspace(const Dims& d, void* ws, size_t ws_bytes, int op, Workspace*
   if (ws_bytes < out->bytes)
     return fail(SFB_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, %zu needed", ws_bytes, out->bytes);
   const size_t room = ws_bytes - out->bytes;
+  if (out->stored_bytes > 0 && room < out->part_bytes + grad_stored_bytes(d, out->n1p)) *out = carve(d, ws, plan_for(op, d), false);
   out->stored_bytes = room > out->part_bytes ? std::min(out->stored_bytes, room - out->part_bytes) : 0;
   if (room < out->part_bytes) out->part_bytes = 0;
   return SFB_OK;
@@ -822,7 +824,7 @@ int static_scratch(void** out) {
 
 extern "C" {
 
-size_t sfb_workspace_bytes(int op, const sfb_shape* shape) {
+static size_t workspace_bytes_of(int op, const sfb_shape* shape, bool stores) {
   Dims d;
   if (op < SFB_OP_MAX_AVG_FORWARD || op > SFB_OP_SEPARATION_LEVEL_BACKWARD) return 0;
   const bool need_kc = op == SFB_OP_COMPRESSION_FORWARD || op == SFB_OP_COMPRESSION_BACKWARD ||
@@ -830,9 +832,11 @@ size_t sfb_workspace_bytes(int op, const sfb_shape* shape) {
                        op == SFB_OP_SEPARATION_FEATURE_BACKWARD_CF || op == SFB_OP_SEPARATION_LEVEL_FORWARD ||
                        op == SFB_OP_SEPARATION_LEVEL_BACKWARD;
   if (check_shape(shape, need_kc, &d) != SFB_OK) return 0;
-  const Workspace w = carve(d, nullptr, plan_for(op, d));
+  const Workspace w = carve(d, nullptr, plan_for(op, d), stores);
   return w.bytes + w.part_bytes + w.stored_bytes;
 }
+size_t sfb_workspace_bytes(int op, const sfb_shape* shape) { return workspace_bytes_of(op, shape, true); }
+size_t sfb_workspace_least_bytes(int op, const sfb_shape* shape) { return workspace_bytes_of(op, shape, false); }
 
 int sfb_max_avg_forward(const float* F1, const float* F2, float* MA_u, float* MA_v, const sfb_shape* shape,
                         void* workspace, size_t workspace_bytes, void* stream) {

@@ -234,87 +234,114 @@ class SeparationLevelFunction(Function):
 
 # --------------------------------------------------------------------------------------------------
 # All pyramid levels as one autograd node (core/corr.py:416-475): the maps of up to four levels go to the library in one call, which
-# runs every kernel once for all of them.  Else, per level, the one-call forward from the feature maps, whose volumes are
-# resampled along the displacement axis and written straight into their channel slice of the concatenated outputs (the reference runs
-# F.interpolate per level and torch.cat over levels).
+# runs every kernel once for all of them.  Else, or where there is no memory for what that takes at a time, the one-call forward of a
+# level from the feature maps per level, whose volumes are resampled along the displacement axis and written straight into their channel slice
+# of the concatenated outputs (the reference runs F.interpolate per level and torch.cat over levels).
 def _levels_together(fmap1, fmap2_levels, Kc):
     H2, W2 = fmap2_levels[0].shape[2:]
     return (fmap1.is_cuda and len(fmap2_levels) <= MemorySaver.PYRAMID_MAX_LEVELS and Kc <= MemorySaver.PYRAMID_MAX_CHANNELS
             and all(f.shape[2] <= H2 and f.shape[3] <= W2 for f in fmap2_levels) and fmap1.shape[0] * (2 + Kc) <= 65535)
 
 
+def _levels_forward(fmap1, fmap2_levels, params, with_argmax, scale1):
+    """Level by level: sep_u, sep_v and, for a backward, (sep_u, sep_v, argmax_u, argmax_v, a_u, a_v) per level; volumes that lie in the
+    outputs are None."""
+    B, _, H1, W1 = fmap1.shape
+    H2, W2 = fmap2_levels[0].shape[2:]     # displacement ranges of the outputs (= H1, W1 unless image-1 rows are sharded)
+    L, Kt = len(fmap2_levels), 2 + params[0].shape[0]
+    sep_u = torch.empty(B, Kt * L, W2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
+    sep_v = torch.empty(B, Kt * L, H2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
+    saved = []
+    for l, fmap2 in enumerate(fmap2_levels):
+        if tuple(fmap2.shape[2:]) == (H2, W2):   # displacement range of the output: written in place
+            level = MemorySaver.separation_level_forward(fmap1, fmap2, *params, with_argmax, True, scale1, (sep_u, sep_v, l * Kt))
+        else:
+            level = MemorySaver.separation_level_forward(fmap1, fmap2, *params, with_argmax, True, scale1)
+            MemorySaver.upsample_displacement_into(level[0], sep_u, l * Kt)
+            MemorySaver.upsample_displacement_into(level[1], sep_v, l * Kt)
+        if with_argmax:
+            saved.append(tuple(level))
+    return sep_u, sep_v, saved
+
+
+def _levels_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, gu, gv, scale1):
+    """Gradients of fmap1, [fmap2_l], weight_u, bias_u, weight_v, bias_v from what _levels_forward saved."""
+    Kt = 2 + weight_u.shape[0]
+    total, g2 = None, []
+    for l, (fmap2, (su, sv, am_u, am_v, a_u, a_v)) in enumerate(zip(fmap2_levels, saved)):
+        if su is None:
+            out = MemorySaver.separation_level_backward(fmap1, fmap2, weight_u, weight_v, sep_u, sep_v, am_u, am_v, a_u, a_v, gu, gv, True,
+                                                        scale1, l * Kt)
+        else:
+            gsu = MemorySaver.upsample_displacement_backward(gu, l * Kt, Kt, su.shape[2])
+            gsv = MemorySaver.upsample_displacement_backward(gv, l * Kt, Kt, sv.shape[2])
+            out = MemorySaver.separation_level_backward(fmap1, fmap2, weight_u, weight_v, su, sv, am_u, am_v, a_u, a_v, gsu, gsv, True, scale1)
+        g2.append(out.pop(1))
+        if total is None:
+            total = out
+        else:
+            for t, x in zip(total, out):
+                t += x
+    g1, *gparams = total
+    return (g1, g2, *gparams)
+
+
+def _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2_levels):
+    params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
+    ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, len(fmap2_levels)
+    ctx.together = _levels_together(fmap1, fmap2_levels, weight_u.shape[0])
+    if ctx.together:
+        try:
+            sep_u, sep_v, saved = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
+        except torch.OutOfMemoryError:
+            ctx.together = False   # (not here, where the exception keeps the attempt's tensors)
+    if not ctx.together:
+        sep_u, sep_v, saved = _levels_forward(fmap1, fmap2_levels, params, with_argmax, scale1)
+    if with_argmax:
+        if not ctx.together:   # volumes written in place are saved as the outputs themselves
+            ctx.in_place = [t[0] is None for t in saved]
+        flat = [saved] if ctx.together else [x for t in saved for x in t if x is not None]
+        ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, *flat)
+    return sep_u, sep_v
+
+
+def _pyramid_backward(ctx, grad_sep_u, grad_sep_v, pooled=False):
+    """(g1, [g2_l], parameters'); `pooled`: the one gradient of the first level, with what its averages contribute."""
+    if not ctx.with_argmax:
+        raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
+    L = ctx.levels
+    fmap1, weight_u, weight_v, sep_u, sep_v, *rest = ctx.saved_tensors
+    fmap2_levels, saved = rest[:L], rest[L:]
+    args = fmap1, fmap2_levels, weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v
+    upstream = grad_sep_u.contiguous(), grad_sep_v.contiguous(), ctx.scale1
+    if ctx.together:
+        try:
+            return MemorySaver.separation_pyramid_backward(*args, saved[0], *upstream, pooled=pooled)
+        except torch.OutOfMemoryError:
+            pass
+        saved = MemorySaver.separation_pyramid_saved(saved[0], fmap1, fmap2_levels, weight_u.shape[0], True)
+    else:
+        flat = iter(saved)
+        saved = [tuple(None if in_place and i < 2 else next(flat) for i in range(6)) for in_place in ctx.in_place]
+    g1, g2, *gparams = _levels_backward(*args, saved, *upstream)
+    if pooled:
+        for l in range(L - 1, 0, -1):
+            g2[l - 1] += torch.ops.aten.avg_pool2d_backward(g2[l], fmap2_levels[l - 1], [2, 2], [2, 2], [0, 0], False, True, None)
+        del g2[1:]
+    return (g1, g2, *gparams)
+
+
 class SeparationPyramidFunction(Function):
     @staticmethod
     def forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, *fmap2_levels):
         assert fmap1.is_contiguous() and all(f.is_contiguous() for f in fmap2_levels)
-        params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
-        B, _, H1, W1 = fmap1.shape
-        H2, W2 = fmap2_levels[0].shape[2:]     # displacement ranges of the outputs (= H1, W1 unless image-1 rows are sharded)
-        L, Kt = len(fmap2_levels), 2 + weight_u.shape[0]
-        saved = []
-        ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, L
-        ctx.together = _levels_together(fmap1, fmap2_levels, weight_u.shape[0])
-        if ctx.together:
-            sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
-            if with_argmax:
-                ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, buffer)
-            return sep_u, sep_v
-        sep_u = torch.empty(B, Kt * L, W2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
-        sep_v = torch.empty(B, Kt * L, H2, H1, W1, dtype=fmap1.dtype, device=fmap1.device)
-        for l, fmap2 in enumerate(fmap2_levels):
-            if tuple(fmap2.shape[2:]) == (H2, W2):   # displacement range of the output: written in place
-                su, sv, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(
-                    fmap1, fmap2, *params, with_argmax, True, scale1, (sep_u, sep_v, l * Kt))
-            else:
-                su, sv, am_u, am_v, a_u, a_v = MemorySaver.separation_level_forward(fmap1, fmap2, *params,
-                                                                                    with_argmax, True, scale1)
-                MemorySaver.upsample_displacement_into(su, sep_u, l * Kt)
-                MemorySaver.upsample_displacement_into(sv, sep_v, l * Kt)
-            saved.append((su, sv, am_u, am_v, a_u, a_v))
-        if with_argmax:
-            # volumes written in place are saved as the outputs themselves
-            ctx.in_place = [t[0] is None for t in saved]
-            flat = [x for t in saved for x in t if x is not None]
-            ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, *flat)
-        return sep_u, sep_v
+        return _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2_levels)
 
     @staticmethod
     @once_differentiable
     def backward(ctx, grad_sep_u, grad_sep_v):
-        if not ctx.with_argmax:
-            raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
-        L = ctx.levels
-        fmap1, weight_u, weight_v, sep_u, sep_v = ctx.saved_tensors[:5]
-        fmap2_levels = ctx.saved_tensors[5:5 + L]
-        flat = list(ctx.saved_tensors[5 + L:])
-        wu, wv = weight_u.contiguous(), weight_v.contiguous()
-        gu, gv = grad_sep_u.contiguous(), grad_sep_v.contiguous()
-        if ctx.together:
-            g1, g2, gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(fmap1, fmap2_levels, wu, wv, sep_u, sep_v, flat[0],
-                                                                                     gu, gv, ctx.scale1)
-            return (None, None, gw_u, gb_u, gw_v, gb_v, g1, *g2)
-        Kt = 2 + weight_u.shape[0]
-        g1 = gw_u = gb_u = gw_v = gb_v = None
-        g2 = []
-        for l in range(L):
-            if ctx.in_place[l]:
-                am_u, am_v, a_u, a_v = flat[:4]
-                del flat[:4]
-                out = MemorySaver.separation_level_backward(fmap1, fmap2_levels[l], wu, wv, sep_u, sep_v, am_u, am_v,
-                                                            a_u, a_v, gu, gv, True, ctx.scale1, l * Kt)
-            else:
-                su, sv, am_u, am_v, a_u, a_v = flat[:6]
-                del flat[:6]
-                gsu = MemorySaver.upsample_displacement_backward(gu, l * Kt, Kt, su.shape[2])
-                gsv = MemorySaver.upsample_displacement_backward(gv, l * Kt, Kt, sv.shape[2])
-                out = MemorySaver.separation_level_backward(fmap1, fmap2_levels[l], wu, wv, su, sv, am_u, am_v, a_u,
-                                                            a_v, gsu, gsv, True, ctx.scale1)
-            g2.append(out[1])
-            if l == 0:
-                g1, gw_u, gb_u, gw_v, gb_v = out[0], out[2], out[3], out[4], out[5]
-            else:
-                g1 += out[0]; gw_u += out[2]; gb_u += out[3]; gw_v += out[4]; gb_v += out[5]
-        return (None, None, gw_u, gb_u, gw_v, gb_v, g1, *g2)
+        g1, g2, *gparams = _pyramid_backward(ctx, grad_sep_u, grad_sep_v)
+        return (None, None, *gparams, g1, *g2)
 
 
 class SeparationPooledPyramidFunction(Function):
@@ -322,24 +349,14 @@ class SeparationPooledPyramidFunction(Function):
     scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, *pooled)`` on CUDA maps, 2 to 4 levels with the first."""
 
     @staticmethod
-    def forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, *pooled):
-        params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
-        ctx.with_argmax, ctx.scale1 = with_argmax, scale1
-        sep_u, sep_v, buffer = MemorySaver.separation_pyramid_forward(fmap1, [fmap2, *pooled], *params, with_argmax, scale1)
-        if with_argmax:
-            ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, buffer, fmap2, *pooled)
-        return sep_u, sep_v
+    def forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, *fmap2_levels):
+        return _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2_levels)
 
     @staticmethod
     @once_differentiable
     def backward(ctx, grad_sep_u, grad_sep_v):
-        if not ctx.with_argmax:
-            raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
-        fmap1, weight_u, weight_v, sep_u, sep_v, buffer, *levels = ctx.saved_tensors
-        g1, (g2,), gw_u, gb_u, gw_v, gb_v = MemorySaver.separation_pyramid_backward(
-            fmap1, levels, weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v, buffer, grad_sep_u.contiguous(),
-            grad_sep_v.contiguous(), ctx.scale1, pooled=True)
-        return (None, None, gw_u, gb_u, gw_v, gb_v, g1, g2, *[None] * (len(levels) - 1))
+        g1, (g2,), *gparams = _pyramid_backward(ctx, grad_sep_u, grad_sep_v, pooled=True)
+        return (None, None, *gparams, g1, g2, *[None] * (ctx.levels - 1))
 
 
 class PooledLevelFunction(Function):

@@ -19,11 +19,12 @@ from . import _lib
 
 # Scratch buffers handed to the library, one per (device, stream): calls that share a workspace must be ordered on
 # one stream.  A buffer grows to the largest size asked for and is kept for reuse (12.3 GB for a level backward of
-# B=8, 135x240, Kc=4, 4.2 of them for the gradient of the volume, in parts; 12.9 GB for that of four levels together); release_workspaces()
-# drops them.  The lock covers DataParallel-style callers that run the ops
-# from several threads.
+# B=8, 135x240, Kc=4, 4.2 of them for the gradient of the volume, in parts; 12.9 GB for that of four levels together);
+# release_workspaces() drops them.  The lock covers DataParallel-style callers that run the ops from several threads.
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 _workspaces_lock = threading.Lock()
+# Sizes from which on there was no memory for a buffer: what can do with less does not try them again, until release_workspaces().
+_too_large: Dict[Tuple[int, int], int] = {}
 
 
 # What a call costs on the host decides the small ones, so the device is switched only when another one is current, its stream is
@@ -78,20 +79,49 @@ def _workspace(nbytes: int, device: torch.device, stream: int) -> torch.Tensor:
     with _workspaces_lock:
         ws = _workspaces.get(key)
         if ws is None or ws.numel() < nbytes:
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+            try:
+                ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+            except torch.OutOfMemoryError:
+                if ws is None:
+                    raise
+                # the smaller one goes first (work in flight keeps it: the allocator hands memory on in the order of the stream)
+                ws = None
+                del _workspaces[key]
+                ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
             _workspaces[key] = ws
         return ws
 
 
+def _workspace_or_less(nbytes: int, least, device: torch.device, stream: int, must: bool = True) -> torch.Tensor:
+    """A buffer of nbytes, or where there is no memory for it of least() bytes.  Not `must`: OutOfMemoryError without another attempt at
+    what there was no memory for before."""
+    key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
+    for n, last in ((nbytes, False), (None, True)):
+        if last:
+            n = least()
+        if n >= _too_large.get(key, n + 1) and not (last and must):
+            continue
+        try:
+            return _workspace(n, device, stream)
+        except torch.OutOfMemoryError:
+            with _workspaces_lock:
+                _too_large[key] = min(n, _too_large.get(key, n))
+            if last:
+                raise
+    raise torch.OutOfMemoryError(f"no memory for a workspace of {n} bytes")
+
+
 def release_workspaces(device=None) -> int:
     """Drop the cached scratch buffers (of one device, or of all) and return the bytes released to torch's
-    allocator.  Work already enqueued keeps its buffer alive through torch's stream-ordered allocator only if the
+    allocator.  Sizes that there was no memory for are tried again afterwards.  Work already enqueued keeps its buffer alive through torch's stream-ordered allocator only if the
     caller synchronises first: call this between steps, not while ops are in flight."""
     index = None if device is None else torch.device(device).index
     freed = 0
     with _workspaces_lock:
         for key in [k for k in _workspaces if index is None or k[0] == index]:
             freed += _workspaces.pop(key).numel()
+        for key in [k for k in _too_large if index is None or k[0] == index]:
+            del _too_large[key]
     return freed
 
 
@@ -116,7 +146,7 @@ def _call(name: str, op: int, shape: _lib.SfbShape, device: torch.device, tensor
         if nbytes == 0:
             # run the entry point anyway so that the library reports the precise reason
             nbytes = 256
-        ws = _workspace(nbytes, device, stream)
+        ws = _workspace_or_less(nbytes, lambda: max(lib.sfb_workspace_least_bytes(op, ctypes.byref(shape)), 256), device, stream)
         rc = getattr(lib, name)(*[_ptr(t) for t in tensors], ctypes.byref(shape), ws.data_ptr(), ws.numel(), stream)
         if rc != _lib.SFB_OK:
             raise RuntimeError(f"{name}: {lib.sfb_status_string(rc).decode()}: {lib.sfb_last_error().decode()}")
@@ -594,7 +624,8 @@ def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, 
     shape = ctypes.byref(s)
     with _on(dev):
         stream = _stream(dev)
-        ws = _workspace(max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, 1), 256), dev, stream)
+        size = lambda backward: max(lib.sfb_separation_pyramid_workspace_bytes(shape, H2, W2, L, backward), 256)
+        ws = _workspace_or_less(size(1), lambda: size(2), dev, stream, must=False)
         _raise_on(lib.sfb_separation_pyramid_backward(
             fmap1.data_ptr(), ptrs, H2, W2, L, scale1, weight_u.data_ptr(), weight_v.data_ptr(), sep_u.data_ptr(), sep_v.data_ptr(),
             saved.data_ptr(), saved.numel(), g_sep_u.data_ptr(), g_sep_v.data_ptr(), gF1.data_ptr(), gptrs, gw_u.data_ptr(),
