@@ -96,25 +96,35 @@ def _workspace_or_less(nbytes: int, least, device: torch.device, stream: int, mu
     """A buffer of nbytes, or where there is no memory for it of least() bytes.  Not `must`: OutOfMemoryError without another attempt at
     what there was no memory for before."""
     key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
-    for n, last in ((nbytes, False), (None, True)):
-        if last:
-            n = least()
-        if n >= _too_large.get(key, n + 1) and not (last and must):
-            continue
+
+    def hopeless(n):
+        ws = _workspaces.get(key)
+        return n >= _too_large.get(key, n + 1) and (ws is None or ws.numel() < n)
+
+    def attempt(n):
         try:
             return _workspace(n, device, stream)
         except torch.OutOfMemoryError:
             with _workspaces_lock:
                 _too_large[key] = min(n, _too_large.get(key, n))
-            if last:
-                raise
-    raise torch.OutOfMemoryError(f"no memory for a workspace of {n} bytes")
+            raise
+
+    if not hopeless(nbytes):
+        try:
+            return attempt(nbytes)
+        except torch.OutOfMemoryError:
+            pass
+    n = least()
+    if not must and hopeless(n):
+        raise torch.OutOfMemoryError(f"no memory for a workspace of {n} bytes")
+    return attempt(n)
 
 
 def release_workspaces(device=None) -> int:
     """Drop the cached scratch buffers (of one device, or of all) and return the bytes released to torch's
-    allocator.  Sizes that there was no memory for are tried again afterwards.  Work already enqueued keeps its buffer alive through torch's stream-ordered allocator only if the
-    caller synchronises first: call this between steps, not while ops are in flight."""
+    allocator.  Sizes that there was no memory for are tried again afterwards.  Work already enqueued keeps its buffer
+    alive through torch's stream-ordered allocator only if the caller synchronises first: call this between steps, not
+    while ops are in flight."""
     index = None if device is None else torch.device(device).index
     freed = 0
     with _workspaces_lock:
