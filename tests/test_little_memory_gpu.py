@@ -27,7 +27,7 @@ class Shortage:
 
     def start(self, limit):
         self.limit, self.asked, self.given = limit, [], []
-        ops._too_large.clear()
+        ops.release_workspaces()
 
 
 @pytest.fixture()
