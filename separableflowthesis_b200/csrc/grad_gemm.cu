@@ -846,21 +846,15 @@ void grad_split_levels(const Dims* d, int levels, int form, TileSplit* out) {
   int cut[MAX_FUSED_LEVELS] = {1, 1, 1, 1};
   static_assert(MAX_FUSED_LEVELS == 4, "cut");
   if (all <= 4 * SM_COUNT) {
-    double best = 0;
-    for (int n0 = 1; n0 <= std::min(blocks[0], MAX_PIECES); ++n0) {
-      for (int n1 = 1; n1 <= (image2_major || levels < 2 ? 1 : std::min(n0, blocks[1])); ++n1) {
-        BlockQueue queue;
-        for (int l = 0; l < levels; ++l) {
-          const int n = l == 0 || image2_major ? n0 : (l == 1 ? n1 : 1);
-          queue.add(tiles[l] * n, (double)blocks[l] / n * unit + 8);
-        }
-        const double cost = queue.makespan() + (image2_major && n0 > 1 ? 6.0 : 0.0);
-        if (best == 0 || cost < 0.95 * best) {
-          best = cost;
-          for (int l = 0; l < levels; ++l) cut[l] = l == 0 || image2_major ? n0 : (l == 1 ? n1 : 1);
-        }
+    const auto pieces = [&](int l, int n0, int n1) { return l == 0 || image2_major ? n0 : (l == 1 ? n1 : 1); };
+    const LevelCut c = cheapest_cut(std::min(blocks[0], MAX_PIECES), image2_major || levels < 2 ? 1 : blocks[1], [&](auto& work, int n0, int n1) {
+      for (int l = 0; l < levels; ++l) {
+        const int n = pieces(l, n0, n1);
+        work.add(tiles[l] * n, (double)blocks[l] / n * unit + 8);
       }
-    }
+      return image2_major && n0 > 1 ? 6.0 : 0.0;
+    });
+    for (int l = 0; l < levels; ++l) cut[l] = pieces(l, c.n0, c.n1);
   }
   int parts = -1;   // the image-1-major form: of all levels, less the one that goes to the output
   for (int l = 0; l < levels; ++l) parts += cut[l];

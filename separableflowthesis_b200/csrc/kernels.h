@@ -165,6 +165,46 @@ class BlockQueue {
   int n_ = 1;
 };
 
+// What a makespan is not below: no SM idle, and the longest block.
+class BlockWork {
+ public:
+  void add(int blocks, double length) {
+    if (blocks <= 0) return;
+    total_ += blocks * length;
+    longest_ = std::max(longest_, length);
+  }
+  double bound() const { return std::max(total_ / SM_COUNT, longest_); }
+
+ private:
+  double total_ = 0, longest_ = 0;
+};
+// Host side.  The cut (n0, n1) of the blocks of two groups, 1 <= n0 <= most0 and 1 <= n1 <= min(n0, most1), that clearly (by a twentieth)
+// undercuts the ones before it.  fill(blocks, n0, n1) adds a cut's blocks and returns what the launch costs beside them.  Of up to 136 cuts
+// those whose work alone shows that they do not are left out: the size query of a backward of 2 x 55 x 128 with four levels, four searches, took
+// 130 us with all of them, 7 now.
+struct LevelCut { int n0, n1; };
+template <class Fill>
+LevelCut cheapest_cut(int most0, int most1, Fill&& fill) {
+  LevelCut cut{1, 1};
+  double best = 0;
+  for (int n0 = 1; n0 <= most0; ++n0) {
+    for (int n1 = 1; n1 <= std::min(n0, most1); ++n1) {
+      if (best > 0) {
+        BlockWork work;
+        const double beside = fill(work, n0, n1);
+        if (work.bound() * (1 - 1e-9) + beside >= 0.95 * best) continue;   // (less than the rounding of either)
+      }
+      BlockQueue queue;
+      const double beside = fill(queue, n0, n1), cost = queue.makespan() + beside;
+      if (best == 0 || cost < 0.95 * best) {
+        best = cost;
+        cut = LevelCut{n0, n1};
+      }
+    }
+  }
+  return cut;
+}
+
 // Gradient GEMM.  G = dLoss/dS is generated from two "interleaved" operand sets: for every displacement
 // and image-1 pixel the R4 values (slots) that pixel contributes, in groups of four:
 //   XU (B, H2, R4/4, n1p, 4)  values that depend on (pixel, u);  XV (B, W2, R4/4, n1p, 4)  (pixel, v)

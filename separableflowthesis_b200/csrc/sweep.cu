@@ -887,22 +887,16 @@ void sweep_split_levels(const Dims* d, int levels, int slots, bool sums, TileSpl
     out[l] = TileSplit{tiles, tiles, 1, 0, 0};
   }
   if (tiles > 4 * SM_COUNT) return;
-  int best_cut[2] = {1, 1};
-  double best = 0;
-  for (int n0 = 1; n0 <= std::min(n_vb[0], MAX_PIECES); ++n0) {
-    for (int n1 = 1; n1 <= (levels > 1 ? std::min(n_vb[1], n0) : 1); ++n1) {
-      BlockQueue queue;
-      for (int l = 0; l < levels; ++l) {
-        const int n = l == 0 ? n0 : (l == 1 ? n1 : 1), per = n_vb[l] / n, extra = n_vb[l] - per * n;
-        if (extra > 0) queue.add(tiles * extra, (per + 1) * n_ub[l] + 2);   // (the order inside a level does not matter much)
-        queue.add(tiles * (n - extra), per * n_ub[l] + 2);
-      }
-      const double cost = queue.makespan() + (n0 > 1 || n1 > 1 ? 2.0 : 0.0);
-      if (best == 0 || cost < 0.95 * best) { best = cost; best_cut[0] = n0; best_cut[1] = n1; }
+  const LevelCut cut = cheapest_cut(std::min(n_vb[0], MAX_PIECES), levels > 1 ? n_vb[1] : 1, [&](auto& work, int n0, int n1) {
+    for (int l = 0; l < levels; ++l) {
+      const int n = l == 0 ? n0 : (l == 1 ? n1 : 1), per = n_vb[l] / n, extra = n_vb[l] - per * n;
+      work.add(tiles * extra, (per + 1) * n_ub[l] + 2);   // (the order inside a level does not matter much)
+      work.add(tiles * (n - extra), per * n_ub[l] + 2);
     }
-  }
+    return n0 > 1 || n1 > 1 ? 2.0 : 0.0;
+  });
   for (int l = 0; l < std::min(levels, 2); ++l) {
-    const int n = best_cut[l];
+    const int n = l == 0 ? cut.n0 : cut.n1;
     if (n == 1) continue;
     const int parts = sums ? n_vb[l] - piece_start(n_vb[l], n, 1) : n - 1;
     out[l] = TileSplit{tiles, 0, n, parts, (size_t)tiles * parts * slots * d[l].H2 * TILE_M};
