@@ -58,8 +58,8 @@ class AlternateCorrBlockSepflow:
         self._fmap2, self._pyramid, self._pooled, self._grad_mode = fmap2, None, None, torch.is_grad_enabled()
         if (2 <= num_levels <= _ops.PYRAMID_MAX_LEVELS and fmap2.is_cuda and fmap2.dtype == torch.float32 and fmap2.dim() == 4
                 and min(fmap2.shape[2:]) >> (num_levels - 1) >= 1 and fmap2.numel() > 0):
-            # one launch; differentiable tensors for whoever reads them (the call for all levels takes them as they are)
-            self._pooled = _ops.pool_levels(fmap2.detach().contiguous(), num_levels)
+            # one launch and buffer; differentiable tensors for whoever reads them (the call for all levels takes them as they are)
+            self._pooled = _ops.pool_levels(fmap2 if fmap2.is_contiguous() else fmap2.detach().contiguous(), num_levels)
         else:
             self._pyramid = [fmap2]
             for _ in range(num_levels - 1):
@@ -72,7 +72,7 @@ class AlternateCorrBlockSepflow:
         if self._pyramid is None:
             with torch.set_grad_enabled(self._grad_mode):   # as the constructor was called
                 self._pyramid = [self._fmap2]
-                for level in self._pooled:
+                for level in _ops.pooled_level_views(self._pooled, self._fmap2.shape, self.num_levels):
                     self._pyramid.append(PooledLevelFunction.apply(self._pyramid[-1], (level,)))
         return self._pyramid
 
@@ -132,9 +132,9 @@ class AlternateCorrBlockSepflow:
                 and self._one_node_per_level(attention_weights)
                 and attention_weights[0].out_channels <= _ops.PYRAMID_MAX_CHANNELS and batch * (2 + attention_weights[0].out_channels) <= 65535):
             attention1, attention2 = attention_weights
-            return SeparationPooledPyramidFunction.apply(self.support_backward, 1.0 / math.sqrt(fdim), attention1.weight,
+            return SeparationPooledPyramidFunction.apply(self.support_backward, 1.0 / math.sqrt(fdim), self.num_levels, attention1.weight,
                                                          attention1.bias, attention2.weight, attention2.bias,
-                                                         self.fmap1_l0.contiguous(), self._fmap2.contiguous(), *self._pooled)
+                                                         self.fmap1_l0.contiguous(), self._fmap2.contiguous(), self._pooled)
         h2, w2 = self.pyramid[0].shape[2:]
         if self._one_node_per_level(attention_weights) and self.num_levels > 1:
             # one node for the whole pyramid: levels are resampled along the displacement axis and written into

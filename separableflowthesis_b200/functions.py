@@ -286,45 +286,53 @@ def _levels_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, save
     return (g1, g2, *gparams)
 
 
-def _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2_levels):
+def _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2_levels, levels=None, pooled=None):
+    """`pooled`: fmap2_levels is the first of so many levels, and the others are in that buffer (pool_levels)."""
     params = [t.contiguous() for t in (weight_u, bias_u, weight_v, bias_v)]
-    ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, len(fmap2_levels)
+    ctx.with_argmax, ctx.scale1, ctx.levels = with_argmax, scale1, levels or len(fmap2_levels)
     ctx.together = _levels_together(fmap1, fmap2_levels, weight_u.shape[0])
     if ctx.together:
         try:
-            sep_u, sep_v, saved = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1)
+            sep_u, sep_v, saved = MemorySaver.separation_pyramid_forward(fmap1, fmap2_levels, *params, with_argmax, scale1, levels, pooled)
         except torch.OutOfMemoryError:
             ctx.together = False   # (not here, where the exception keeps the attempt's tensors)
     if not ctx.together:
-        sep_u, sep_v, saved = _levels_forward(fmap1, fmap2_levels, params, with_argmax, scale1)
+        sep_u, sep_v, saved = _levels_forward(fmap1, _all_levels(fmap2_levels, ctx.levels, pooled), params, with_argmax, scale1)
     if with_argmax:
         if not ctx.together:   # volumes written in place are saved as the outputs themselves
             ctx.in_place = [t[0] is None for t in saved]
         flat = [saved] if ctx.together else [x for t in saved for x in t if x is not None]
-        ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, *flat)
+        ctx.save_for_backward(fmap1, weight_u, weight_v, sep_u, sep_v, *fmap2_levels, *([] if pooled is None else [pooled]), *flat)
     return sep_u, sep_v
 
 
-def _pyramid_backward(ctx, grad_sep_u, grad_sep_v, pooled=False):
-    """(g1, [g2_l], parameters'); `pooled`: the one gradient of the first level, with what its averages contribute."""
+def _all_levels(fmap2_levels, levels, pooled):
+    return fmap2_levels if pooled is None else [*fmap2_levels, *MemorySaver.pooled_level_views(pooled, fmap2_levels[0].shape, levels)]
+
+
+def _pyramid_backward(ctx, grad_sep_u, grad_sep_v, is_pooled=False):
+    """(g1, [g2_l], parameters'); `is_pooled`: the one gradient of the first level, with what its averages contribute."""
     if not ctx.with_argmax:
         raise NotImplementedError("max avg backward pass is not implemented: use max argmax avg")
     L = ctx.levels
     fmap1, weight_u, weight_v, sep_u, sep_v, *rest = ctx.saved_tensors
-    fmap2_levels, saved = rest[:L], rest[L:]
-    args = fmap1, fmap2_levels, weight_u.contiguous(), weight_v.contiguous(), sep_u, sep_v
-    upstream = grad_sep_u.contiguous(), grad_sep_v.contiguous(), ctx.scale1
+    given = 1 if is_pooled else L
+    fmap2_levels, pooled, saved = rest[:given], rest[given] if is_pooled else None, rest[given + is_pooled:]
+    wu, wv = weight_u.contiguous(), weight_v.contiguous()
+    gu, gv = grad_sep_u.contiguous(), grad_sep_v.contiguous()
     if ctx.together:
         try:
-            return MemorySaver.separation_pyramid_backward(*args, saved[0], *upstream, pooled=pooled)
+            return MemorySaver.separation_pyramid_backward(fmap1, fmap2_levels, wu, wv, sep_u, sep_v, saved[0], gu, gv, ctx.scale1, L, pooled)
         except torch.OutOfMemoryError:
             pass
+    fmap2_levels = _all_levels(fmap2_levels, L, pooled)
+    if ctx.together:
         saved = MemorySaver.separation_pyramid_saved(saved[0], fmap1, fmap2_levels, weight_u.shape[0], True)
     else:
         flat = iter(saved)
         saved = [tuple(None if in_place and i < 2 else next(flat) for i in range(6)) for in_place in ctx.in_place]
-    g1, g2, *gparams = _levels_backward(*args, saved, *upstream)
-    if pooled:
+    g1, g2, *gparams = _levels_backward(fmap1, fmap2_levels, wu, wv, sep_u, sep_v, saved, gu, gv, ctx.scale1)
+    if is_pooled:
         for l in range(L - 1, 0, -1):
             g2[l - 1] += torch.ops.aten.avg_pool2d_backward(g2[l], fmap2_levels[l - 1], [2, 2], [2, 2], [0, 0], False, True, None)
         del g2[1:]
@@ -346,17 +354,17 @@ class SeparationPyramidFunction(Function):
 
 class SeparationPooledPyramidFunction(Function):
     """The same for the levels that ``pool_levels`` made of the first one, whose gradient has what they contribute: ``apply(with_argmax,
-    scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, *pooled)`` on CUDA maps, 2 to 4 levels with the first."""
+    scale1, levels, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, pooled)`` on CUDA maps, 2 to 4 levels with the first."""
 
     @staticmethod
-    def forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, *fmap2_levels):
-        return _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2_levels)
+    def forward(ctx, with_argmax, scale1, levels, weight_u, bias_u, weight_v, bias_v, fmap1, fmap2, pooled):
+        return _pyramid_forward(ctx, with_argmax, scale1, weight_u, bias_u, weight_v, bias_v, fmap1, [fmap2], levels, pooled)
 
     @staticmethod
     @once_differentiable
     def backward(ctx, grad_sep_u, grad_sep_v):
-        g1, (g2,), *gparams = _pyramid_backward(ctx, grad_sep_u, grad_sep_v, pooled=True)
-        return (None, None, *gparams, g1, g2, *[None] * (ctx.levels - 1))
+        g1, (g2,), *gparams = _pyramid_backward(ctx, grad_sep_u, grad_sep_v, is_pooled=True)
+        return (None, None, None, *gparams, g1, g2, None)
 
 
 class PooledLevelFunction(Function):

@@ -547,44 +547,75 @@ def separation_level_backward(img1_features_l0, img2_features_lk, weight_u, weig
 PYRAMID_MAX_LEVELS, PYRAMID_MAX_CHANNELS = 4, 4
 
 
-def _pyramid_arrays(maps, levels):
-    """Host arrays of an entry point: pointers (NULL for the levels that the library pools itself), heights, widths."""
-    H, W = maps[0].shape[2:]
+def _pyramid_arrays(maps, levels, pooled=None):
+    """Host arrays of an entry point: pointers (of the levels in the buffer of pool_levels, or NULL for those that the library pools itself),
+    heights, widths."""
+    B, C, H, W = maps[0].shape
     sizes = [t.shape[2:] for t in maps] + [(H >> l, W >> l) for l in range(len(maps), levels)]
     ptrs = (ctypes.c_void_p * levels)(*[t.data_ptr() for t in maps])
+    if pooled is not None:
+        for l, at in enumerate(_pooled_offsets(B * C, H, W, levels)[:-1]):
+            ptrs[l + 1] = pooled.data_ptr() + 4 * at
     sizes = (ctypes.c_int32 * (2 * levels))(*[h for h, _ in sizes], *[w for _, w in sizes])
     return ptrs, ctypes.addressof(sizes), ctypes.addressof(sizes) + 4 * levels, sizes
 
 
-def _check_pyramid(fmap1, fmap2_levels, levels):
-    """Shape of a pyramid call.  fmap2_levels: all levels of image 2, or the first alone with the number of `levels`."""
+def _check_pyramid(fmap1, fmap2_levels, levels, pooled=None):
+    """Shape of a pyramid call.  fmap2_levels: all levels of image 2, or the first alone with the number of `levels`, and possibly the
+    buffer of the others."""
     s = None
     for f2 in fmap2_levels:
         level = _check_fmaps(fmap1, f2)
         s = s or level
     if levels != len(fmap2_levels) and (len(fmap2_levels) != 1 or min(s.H2, s.W2) >> (levels - 1) < 1):
         raise RuntimeError(f"{len(fmap2_levels)} maps given for {levels} levels of at least one pixel")
+    if pooled is not None:
+        _check_like(pooled, "pooled", (_pooled_offsets(s.B * s.C, s.H2, s.W2, levels)[-1],), torch.float32, fmap1.device)
     return s
 
 
+def _pooled_offsets(planes, H, W, levels):
+    """Where levels 1, 2, ... begin in the buffer of pool_levels, each on 256 bytes, and its elements."""
+    at, offsets = 0, []
+    for l in range(1, levels):
+        offsets.append(at)
+        at += (planes * (H >> l) * (W >> l) + 63) // 64 * 64
+    return offsets + [at]
+
+
 def pool_levels(fmap2, levels):
-    """The coarser levels of image 2's pyramid, 2 x 2 averages of one another (core/corr.py:377-382), in one launch."""
+    """The coarser levels of image 2's pyramid, 2 x 2 averages of one another (core/corr.py:377-382), in one launch and one buffer
+    (pooled_level_views)."""
     _check(fmap2, "fmap2", torch.float32, 4)
+    dev = fmap2.device
     B, C, H, W = fmap2.shape
-    out = [torch.empty(B, C, H >> l, W >> l, dtype=torch.float32, device=fmap2.device) for l in range(1, levels)]
-    lib = _lib.load()
-    ptrs = (ctypes.c_void_p * len(out))(*[t.data_ptr() for t in out])
-    with _on(fmap2.device):
-        _raise_on(lib.sfb_pool_levels(fmap2.data_ptr(), ptrs, B, C, H, W, levels, _stream(fmap2.device)), "sfb_pool_levels")
+    *offsets, size = _pooled_offsets(B * C, H, W, levels)
+    out = torch.empty(size, dtype=torch.float32, device=dev)
+    base = out.data_ptr()
+    ptrs = (ctypes.c_void_p * (levels - 1))(*[base + 4 * at for at in offsets])
+    with _on(dev):
+        _raise_on(_lib.load().sfb_pool_levels(fmap2.data_ptr(), ptrs, B, C, H, W, levels, _stream(dev)), "sfb_pool_levels")
     return out
 
 
-def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, bias_v, with_argmax, scale1, levels=None):
+def pooled_level_views(pooled, shape, levels):
+    """The levels (B,C,H >> l,W >> l) of maps of that shape in the buffer of pool_levels, as tensors that autograd does not take for views
+    of one another."""
+    B, C, H, W = shape
+    out = []
+    for l, at in enumerate(_pooled_offsets(B * C, H, W, levels)[:-1], 1):
+        h, w = H >> l, W >> l
+        out.append(torch.empty(0, dtype=pooled.dtype, device=pooled.device).set_(pooled.untyped_storage(), pooled.storage_offset() + at,
+                                                                                  (B, C, h, w), (C * h * w, h * w, w, 1)))
+    return out
+
+
+def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, bias_v, with_argmax, scale1, levels=None, pooled=None):
     """(sep_u, sep_v, saved): separation_level_forward of every level on the model's feature maps, resampled to the displacement range
     of level 0 and concatenated; `saved` is what the backward needs beside the inputs and outputs (one flat buffer).  With one map and the
-    number of `levels`, the others are its 2 x 2 averages, made by the library."""
+    number of `levels`, the others are its 2 x 2 averages, those of `pooled` (pool_levels) or made by the library."""
     L = levels or len(fmap2_levels)
-    s = _check_pyramid(fmap1, fmap2_levels, L)
+    s = _check_pyramid(fmap1, fmap2_levels, L, pooled)
     dev = fmap1.device
     s.Kc = _check_attention_params(weight_u, bias_u, "attention1", dev)
     if _check_attention_params(weight_v, bias_v, "attention2", dev) != s.Kc:
@@ -593,9 +624,9 @@ def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, 
     sep_u = torch.empty(s.B, Kt, s.W2, s.H1, s.W1, dtype=torch.float32, device=dev)
     sep_v = torch.empty(s.B, Kt, s.H2, s.H1, s.W1, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L)
-    shape, pooled = ctypes.byref(s), int(L != len(fmap2_levels))
-    saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax), pooled), 256), dtype=torch.uint8,
+    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L, pooled)
+    shape, makes = ctypes.byref(s), int(L != len(fmap2_levels) and pooled is None)
+    saved = torch.empty(max(lib.sfb_separation_pyramid_saved_bytes(shape, H2, W2, L, int(with_argmax), makes), 256), dtype=torch.uint8,
                         device=dev)
     with _on(dev):
         stream = _stream(dev)
@@ -609,11 +640,11 @@ def separation_pyramid_forward(fmap1, fmap2_levels, weight_u, bias_u, weight_v, 
 
 
 def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, sep_v, saved, g_sep_u, g_sep_v, scale1, levels=None,
-                                pooled=False):
-    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max; where the library made
-    the levels, or they are the first one's ``pool_levels`` (``pooled``), the gradient of the one map."""
+                                pooled=None):
+    """(gfmap1, [gfmap2_l], gweight_u, gbias_u, gweight_v, gbias_v) of ``separation_pyramid_forward`` with arg-max; with one map and its
+    averages the gradient of the one map."""
     L = levels or len(fmap2_levels)
-    s = _check_pyramid(fmap1, fmap2_levels, L)
+    s = _check_pyramid(fmap1, fmap2_levels, L, pooled)
     dev = fmap1.device
     _check(weight_u, "attention1.weight", torch.float32, 5)
     s.Kc = weight_u.shape[0]
@@ -624,12 +655,12 @@ def separation_pyramid_backward(fmap1, fmap2_levels, weight_u, weight_v, sep_u, 
         _check_like(t, name, (s.B, Kt, D, s.H1, s.W1), torch.float32, dev)
     _check(saved, "saved", torch.uint8, 1)
     gF1 = torch.empty_like(fmap1)
-    gF2 = [torch.empty_like(f2) for f2 in (fmap2_levels[:1] if pooled else fmap2_levels)]
+    gF2 = [torch.empty_like(f2) for f2 in fmap2_levels]
     gw_u, gw_v = torch.empty_like(weight_u), torch.empty_like(weight_v)
     gb_u = torch.empty(s.Kc, dtype=torch.float32, device=dev)
     gb_v = torch.empty(s.Kc, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L)
+    ptrs, H2, W2, _sizes = _pyramid_arrays(fmap2_levels, L, pooled)
     gptrs = (ctypes.c_void_p * L)(*[t.data_ptr() for t in gF2])
     shape = ctypes.byref(s)
     with _on(dev):

@@ -215,6 +215,9 @@ def test_block_gradients(shape, cuda_device):
     chain = [f2]
     for _ in range(levels - 1):
         chain.append(F.avg_pool2d(chain[-1], 2, stride=2))
+    for p in (made, chain):   # a write to a level reaches neither the others nor the maps
+        p[-1].mul_(1.5)
+    assert all(torch.equal(x, y) for x, y in zip(made, chain))
     inner = [torch.autograd.grad([(t * t).sum() for t in p], p[1], retain_graph=True)[0] for p in (made, chain)]
     assert torch.equal(*inner)
     first = [torch.autograd.grad([(t * t * t).sum() for t in p], f2, create_graph=True)[0] for p in (made, chain)]
