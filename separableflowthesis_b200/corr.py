@@ -24,7 +24,7 @@ import torch.nn.functional as F
 
 from .functions import (ComputeMaxArgmaxAvgFunction, ComputeMaxAvgFunction, ComputeSelfCompressionFunction,
                         FusedMaxArgmaxAvgFunction, FusedSelfCompressionFunction, SeparationCompressionCF,
-                        Lookup4dFunction, LookupFunction, LookupPairFunction, LookupVolumeFunction, PooledLevelFunction,
+                        Lookup4dFunction, LookupPairFunction, LookupVolumeFunction, PooledLevelFunction,
                         SeparationLevelFunction, SeparationMaxAvgCF,
                         SeparationPooledPyramidFunction, SeparationPyramidFunction,
                         SeparationState)
@@ -189,8 +189,8 @@ class CorrBlock1D:
     positions of the FIRST volume are clamped to [-1, 1] before the lookup (core/corr.py:586) and those of the second
     are not; gradients flow to the volumes, not to the coordinates (the model detaches them, core/sepflow.py:192).
 
-    Two float32 volumes on one GPU are looked up by one call for both, and the gradients of the block's calls are summed by
-    the library (LookupPairFunction); everything else goes through the ops for a single volume.
+    Both volumes are looked up by one call, and the gradients of the block's calls are summed by the library
+    (LookupPairFunction).
     """
 
     # Lookups of one chain of gradients.  A chain keeps its lookups' coordinates for as long as the block lives.
@@ -203,14 +203,9 @@ class CorrBlock1D:
         self.radius = radius
         self.corr1 = corr1.contiguous()
         self.corr2 = corr2.contiguous()
-        self._pair = all(c.is_cuda and c.dtype == torch.float32 and c.device == corr1.device for c in (corr1, corr2))
         self._chain = None
         with torch.no_grad():
-            if self._pair:
-                self.pyramid1, self.pyramid2 = _ops.lookup_build_pyramid_pair(self.corr1, self.corr2, num_levels)
-            else:
-                self.pyramid1 = _ops.lookup_build_pyramid(self.corr1, num_levels)
-                self.pyramid2 = _ops.lookup_build_pyramid(self.corr2, num_levels)
+            self.pyramid1, self.pyramid2 = _ops.lookup_build_pyramid_pair(self.corr1, self.corr2, num_levels)
 
     def _edges(self):
         """(needs gradient 1, 2, lookups so far, edge 1, 2) of the chain that the next lookup continues."""
@@ -225,14 +220,10 @@ class CorrBlock1D:
         return chain
 
     def __call__(self, coords):
-        if self._pair and coords.dim() == 4 and coords.shape[1] >= 2:
-            chain = self._edges()
-            edges = chain[3:] if chain is not None else (None, None)
-            out1, out2, *edges = LookupPairFunction.apply(self.corr1, self.corr2, self.pyramid1, self.pyramid2, coords, *edges,
-                                                          self.num_levels, self.radius)
-            if chain is not None:
-                self._chain = (*chain[:2], chain[2] + 1, *edges)
-            return out1, out2
-        out1 = LookupFunction.apply(self.corr1, self.pyramid1, coords[:, 0], self.num_levels, self.radius, True)
-        out2 = LookupFunction.apply(self.corr2, self.pyramid2, coords[:, 1], self.num_levels, self.radius, False)
+        chain = self._edges()
+        edges = chain[3:] if chain is not None else (None, None)
+        out1, out2, *edges = LookupPairFunction.apply(self.corr1, self.corr2, self.pyramid1, self.pyramid2, coords, *edges,
+                                                      self.num_levels, self.radius)
+        if chain is not None:
+            self._chain = (*chain[:2], chain[2] + 1, *edges)
         return out1, out2

@@ -383,26 +383,9 @@ class PooledLevelFunction(Function):
 
 
 # --------------------------------------------------------------------------------------------------
-# Lookup on one aggregated 3D volume (CorrBlock1D, core/corr.py:576-594).  The volume's pyramid is passed in so that
-# it is built once per volume, not once per refinement iteration.  No gradient for the coordinates: the model
-# detaches them before every lookup (core/sepflow.py:192).
-class LookupFunction(Function):
-    @staticmethod
-    def forward(ctx, corr, pyramid, coord, levels, radius, clamp_unit):
-        out = MemorySaver.lookup_forward(corr, pyramid, coord, levels, radius, clamp_unit)
-        ctx.save_for_backward(coord)
-        ctx.cfg = (tuple(corr.shape), levels, radius, clamp_unit)
-        return out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, grad_out):
-        (coord,) = ctx.saved_tensors
-        shape, levels, radius, clamp_unit = ctx.cfg
-        gcorr = MemorySaver.lookup_backward(shape, coord, grad_out.contiguous(), levels, radius, clamp_unit)
-        return gcorr, None, None, None, None, None
-
-
+# Lookups on the two aggregated 3D volumes (CorrBlock1D, core/corr.py:576-594).  The volumes' pyramids are passed in so that they are
+# built once, not once per refinement iteration.  No gradient for the coordinates: the model detaches them (core/sepflow.py:192).
+#
 # A refinement looks up a dozen times on the same two volumes.  Gradients of the volumes themselves, one per lookup, would each be
 # written whole and then added up by autograd.  Instead every lookup takes an edge to its volume (a tensor that stands for
 # the volume's accumulator and holds nothing) and hands it on to the next: in the backward the accumulator comes down that

@@ -118,16 +118,25 @@ def test_corrblock1d_host_logic(golden_dir, monkeypatch):
 
     class OracleOps:
         @staticmethod
-        def lookup_build_pyramid(corr, levels):
-            return None
+        def lookup_build_pyramid_pair(corr1, corr2, levels):
+            return None, None
 
         @staticmethod
-        def lookup_forward(corr, pyramid, coord, levels, radius, clamp_unit):
-            return orc.lookup_forward(corr, coord, levels, radius, clamp_unit)
+        def lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels, radius):
+            return (orc.lookup_forward(corr1, coords[:, 0], levels, radius, True), orc.lookup_forward(corr2, coords[:, 1], levels, radius, False))
 
         @staticmethod
-        def lookup_backward(shape, coord, grad_out, levels, radius, clamp_unit):
-            return orc.lookup_backward(shape, coord, grad_out, levels, radius, clamp_unit)
+        def lookup_accumulator_size(shape, levels, clamp_unit):
+            return torch.Size(shape).numel()   # of the volume itself
+
+        @staticmethod
+        def lookup_accumulate_pair(shape1, shape2, coords, g1, g2, acc1, acc2, levels, radius):
+            acc1 += orc.lookup_backward(shape1, coords[:, 0], g1, levels, radius, True).reshape(-1)
+            acc2 += orc.lookup_backward(shape2, coords[:, 1], g2, levels, radius, False).reshape(-1)
+
+        @staticmethod
+        def lookup_fold_gradient(acc, shape, levels, clamp_unit):
+            return acc.reshape(shape)
 
     monkeypatch.setattr(corr_mod, "_ops", OracleOps)
     monkeypatch.setattr(functions, "MemorySaver", OracleOps)

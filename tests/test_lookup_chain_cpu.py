@@ -1,14 +1,20 @@
-"""CPU: the autograd side of the lookups on both aggregated volumes (LookupPairFunction, LookupVolumeFunction) with the oracle in place
-of the library; the library's own ops are tested in the gpu-marked files."""
+"""CPU: the host side of the lookups on both aggregated volumes (CorrBlock1D, LookupPairFunction, LookupVolumeFunction) with the oracle in
+place of the library; the library's own ops are tested in the gpu-marked files."""
+import os
+
+import numpy as np
 import pytest
 import torch
 
+import separableflowthesis_b200 as sfb
 from oracle import separation_oracle as orc
-from separableflowthesis_b200 import functions
+from separableflowthesis_b200 import corr, functions
 
 
 class PairOps:
     """The pair ops on CPU tensors.  An accumulator holds the gradient of its volume."""
+
+    log = []   # accumulations and folds
 
     @staticmethod
     def lookup_build_pyramid_pair(corr1, corr2, levels):
@@ -24,18 +30,22 @@ class PairOps:
 
     @staticmethod
     def lookup_accumulate_pair(shape1, shape2, coords, g1, g2, acc1, acc2, levels, radius):
+        PairOps.log.append(("accumulate", g1 is not None, g2 is not None))
         for g, acc, shape, axis in ((g1, acc1, shape1, 0), (g2, acc2, shape2, 1)):
             if g is not None:
                 acc += orc.lookup_backward(shape, coords[:, axis], g, levels, radius, axis == 0).reshape(-1)
 
     @staticmethod
     def lookup_fold_gradient(acc, shape, levels, clamp_unit):
+        PairOps.log.append(("fold", clamp_unit))
         return acc.reshape(shape)
 
 
 @pytest.fixture()
 def pair_ops(monkeypatch):
     monkeypatch.setattr(functions, "MemorySaver", PairOps)
+    monkeypatch.setattr(corr, "_ops", PairOps)
+    del PairOps.log[:]
 
 
 LEVELS, RADIUS = 2, 2
@@ -52,7 +62,7 @@ def inputs(needs1, needs2, coords_need, seed=3):
 @pytest.mark.parametrize("needs1,needs2", [(False, False), (True, False), (False, True), (True, True)])
 def test_coordinates_that_need_a_gradient(needs1, needs2, pair_ops):
     """They get none, and neither do volumes that need none; a loss of either output alone can still be differentiated, as with one
-    lookup per volume (LookupFunction)."""
+    lookup per volume."""
     for part in ((0,), (1,), (0, 1)):
         v1, v2, coords = inputs(needs1, needs2, True)
         edges = [functions.LookupVolumeFunction.apply(v, LEVELS, clamp) if v.requires_grad else None for v, clamp in ((v1, True), (v2, False))]
@@ -72,3 +82,47 @@ def test_outputs_of_volumes_without_gradients(pair_ops):
     v1, v2, coords = inputs(False, False, False)
     out1, out2, *_ = functions.LookupPairFunction.apply(v1, v2, None, None, coords, None, None, LEVELS, RADIUS)
     assert not out1.requires_grad and not out2.requires_grad
+
+
+def sequence(block, coords):
+    return [block(c) for c in coords]
+
+
+def test_chain_against_the_reference(golden_dir, pair_ops):
+    """Several lookups of one block, one backward: the outputs and, for the golden upstream gradients of one lookup, the gradients of the
+    reference's own class; accumulated per lookup, folded once per volume."""
+    g = np.load(os.path.join(golden_dir, "lookup1d_b1_dim2_16x24.npz"))
+    load = lambda name: torch.from_numpy(np.ascontiguousarray(g[name])).double()
+    v1, v2, coords = load("corr1").requires_grad_(True), load("corr2").requires_grad_(True), load("coords")
+    block = sfb.CorrBlock1D(v1, v2, num_levels=int(g["levels"]), radius=int(g["radius"]))
+    weights = (1.0, -0.5, 3.0)
+    outs = sequence(block, [coords] * 3)
+    for out1, out2 in outs:
+        assert (out1 - load("out1")).abs().max() < 1e-6 and (out2 - load("out2")).abs().max() < 1e-6
+    sum(w * ((o1 * load("w1")).sum() + (o2 * load("w2")).sum()) for w, (o1, o2) in zip(weights, outs)).backward()
+    assert (v1.grad - sum(weights) * load("g_corr1")).abs().max() < 5e-6
+    assert (v2.grad - sum(weights) * load("g_corr2")).abs().max() < 5e-6
+    assert PairOps.log == [("accumulate", True, True)] * 3 + PairOps.log[3:] and sorted(PairOps.log[3:]) == [("fold", False), ("fold", True)]
+
+
+def test_chain_of_different_lookups(pair_ops):
+    """Lookups that reach the loss with one output, with none, and lookups without grad in between."""
+    v1, v2, _ = inputs(True, True, False)
+    coords = [inputs(False, False, False, seed)[2] for seed in range(4)]
+    block = sfb.CorrBlock1D(v1, v2, num_levels=LEVELS, radius=RADIUS)
+    outs = sequence(block, coords[:2])
+    with torch.no_grad():
+        assert not block(coords[0])[0].requires_grad
+    outs += sequence(block, coords[2:])
+    (outs[0][0].sum() + (outs[2][1] ** 2).sum() + outs[3][0].sum()).backward()
+    lookup = lambda v, i, g, axis: orc.lookup_backward(v.shape, coords[i][:, axis], g, LEVELS, RADIUS, axis == 0)
+    ones = torch.ones_like(outs[0][0])
+    assert torch.allclose(v1.grad, lookup(v1, 0, ones, 0) + lookup(v1, 3, ones, 0), atol=1e-12)
+    assert torch.allclose(v2.grad, lookup(v2, 2, 2 * outs[2][1].detach(), 1), atol=1e-12)
+
+
+def test_volumes_and_coordinates_are_the_ops_business(monkeypatch):
+    """No path around the library: what the pair ops refuse is refused."""
+    v1, v2, coords = inputs(False, False, False)
+    with pytest.raises(RuntimeError, match="CUDA"):
+        sfb.CorrBlock1D(v1, v2)
