@@ -189,8 +189,10 @@ class CorrBlock1D:
     positions of the FIRST volume are clamped to [-1, 1] before the lookup (core/corr.py:586) and those of the second
     are not; gradients flow to the volumes, not to the coordinates (the model detaches them, core/sepflow.py:192).
 
-    Both volumes are looked up by one call, and the gradients of the block's calls are summed by the library
-    (LookupPairFunction).
+    Both volumes are looked up by one call, and the gradients of the block's calls are summed by the library: the lookups of a
+    block are a chain in the autograd graph (LookupPairFunction), and a backward from any of them walks those before it.  One
+    backward for a loss over several lookups, or a backward after every lookup, goes through each lookup once; several lookups with a
+    backward for each behind them go through all those before the one whose loss it is.
     """
 
     # Lookups of one chain of gradients.  A chain keeps its lookups' coordinates for as long as the block lives.
@@ -208,22 +210,23 @@ class CorrBlock1D:
             self.pyramid1, self.pyramid2 = _ops.lookup_build_pyramid_pair(self.corr1, self.corr2, num_levels)
 
     def _edges(self):
-        """(needs gradient 1, 2, lookups so far, edge 1, 2) of the chain that the next lookup continues."""
+        """(needs gradient 1, 2, lookups so far, whether a backward has passed, edge 1, 2) of the chain that the next lookup continues."""
         needs = (self.corr1.requires_grad, self.corr2.requires_grad) if torch.is_grad_enabled() else (False, False)
         if not any(needs):
             return None
         chain = self._chain
-        if chain is None or chain[:2] != needs or chain[2] >= self.CHAIN:
-            edges = [LookupVolumeFunction.apply(c, self.num_levels, clamp) if need else None
+        if chain is None or chain[:2] != needs or chain[2] >= self.CHAIN or chain[3]:
+            passed = []
+            edges = [LookupVolumeFunction.apply(c, self.num_levels, clamp, passed) if need else None
                      for c, clamp, need in ((self.corr1, True, needs[0]), (self.corr2, False, needs[1]))]
-            chain = (*needs, 0, *edges)
+            chain = (*needs, 0, passed, *edges)
         return chain
 
     def __call__(self, coords):
         chain = self._edges()
-        edges = chain[3:] if chain is not None else (None, None)
+        edges = chain[4:] if chain is not None else (None, None)
         out1, out2, *edges = LookupPairFunction.apply(self.corr1, self.corr2, self.pyramid1, self.pyramid2, coords, *edges,
                                                       self.num_levels, self.radius)
         if chain is not None:
-            self._chain = (*chain[:2], chain[2] + 1, *edges)
+            self._chain = (*chain[:2], chain[2] + 1, chain[3], *edges)
         return out1, out2

@@ -391,11 +391,13 @@ class PooledLevelFunction(Function):
 # the volume's accumulator and holds nothing) and hands it on to the next: in the backward the accumulator comes down that
 # chain, each lookup adds its windows to it, and the volume's node folds it into the gradient, once.
 class LookupVolumeFunction(Function):
-    """Start of a volume's chain: ``apply(corr, levels, clamp_unit)`` -> edge."""
+    """Start of a volume's chain: ``apply(corr, levels, clamp_unit, passed)`` -> edge.  A backward that has come down the chain appends to
+    the list ``passed``: a lookup after it begins a chain of its own, and does not take later backwards through the earlier lookups."""
 
     @staticmethod
-    def forward(ctx, corr, levels, clamp_unit):
+    def forward(ctx, corr, levels, clamp_unit, passed):
         ctx.cfg = (tuple(corr.shape), levels, clamp_unit)
+        ctx.passed = passed
         ctx.set_materialize_grads(False)
         return torch.empty_strided((MemorySaver.lookup_accumulator_size(corr.shape, levels, clamp_unit),), (0,), dtype=corr.dtype,
                                    device=corr.device)
@@ -403,10 +405,12 @@ class LookupVolumeFunction(Function):
     @staticmethod
     @once_differentiable
     def backward(ctx, acc):
+        if not ctx.passed:
+            ctx.passed.append(True)
         if acc is None:
-            return None, None, None
+            return None, None, None, None
         shape, levels, clamp_unit = ctx.cfg
-        return MemorySaver.lookup_fold_gradient(acc.contiguous(), shape, levels, clamp_unit), None, None
+        return MemorySaver.lookup_fold_gradient(acc.contiguous(), shape, levels, clamp_unit), None, None, None
 
 
 class LookupPairFunction(Function):

@@ -65,7 +65,7 @@ def test_coordinates_that_need_a_gradient(needs1, needs2, pair_ops):
     lookup per volume."""
     for part in ((0,), (1,), (0, 1)):
         v1, v2, coords = inputs(needs1, needs2, True)
-        edges = [functions.LookupVolumeFunction.apply(v, LEVELS, clamp) if v.requires_grad else None for v, clamp in ((v1, True), (v2, False))]
+        edges = [functions.LookupVolumeFunction.apply(v, LEVELS, clamp, []) if v.requires_grad else None for v, clamp in ((v1, True), (v2, False))]
         outs = functions.LookupPairFunction.apply(v1, v2, None, None, coords, *edges, LEVELS, RADIUS)[:2]
         assert outs[0].requires_grad and outs[1].requires_grad
         sum((outs[i] * outs[i]).sum() for i in part).backward()
@@ -119,6 +119,31 @@ def test_chain_of_different_lookups(pair_ops):
     ones = torch.ones_like(outs[0][0])
     assert torch.allclose(v1.grad, lookup(v1, 0, ones, 0) + lookup(v1, 3, ones, 0), atol=1e-12)
     assert torch.allclose(v2.grad, lookup(v2, 2, 2 * outs[2][1].detach(), 1), atol=1e-12)
+
+
+@pytest.mark.parametrize("retain", [False, True])
+def test_backward_after_every_lookup(retain, pair_ops, monkeypatch):
+    """Each goes through its own lookup alone."""
+    walked = []
+    backward = functions.LookupPairFunction.backward
+
+    def counted(ctx, *grads):
+        walked.append(1)
+        return backward(ctx, *grads)
+
+    monkeypatch.setattr(functions.LookupPairFunction, "backward", staticmethod(counted))
+    v1, v2, _ = inputs(True, True, False)
+    block = sfb.CorrBlock1D(v1, v2, num_levels=LEVELS, radius=RADIUS)
+    for i in range(4):
+        coords = inputs(False, False, False, i)[2]
+        o1, o2 = block(coords)
+        g1, g2 = torch.autograd.grad([(o1 * o1).sum() + o2.sum()], [v1, v2], retain_graph=retain)
+        assert torch.equal(g1, orc.lookup_backward(v1.shape, coords[:, 0], 2 * o1.detach(), LEVELS, RADIUS, True))
+        assert torch.equal(g2, orc.lookup_backward(v2.shape, coords[:, 1], torch.ones_like(o2), LEVELS, RADIUS, False))
+    assert len(walked) == 4
+    outs = sequence(block, [coords] * 3)   # and a chain goes on where there was none
+    sum(o1.sum() + o2.sum() for o1, o2 in outs).backward()
+    assert len(walked) == 7
 
 
 def test_volumes_and_coordinates_are_the_ops_business(monkeypatch):
