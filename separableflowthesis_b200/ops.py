@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import math
 import os
 import threading
@@ -570,17 +571,20 @@ def _check_pyramid(fmap1, fmap2_levels, levels, pooled=None):
     if levels != len(fmap2_levels) and (len(fmap2_levels) != 1 or min(s.H2, s.W2) >> (levels - 1) < 1):
         raise RuntimeError(f"{len(fmap2_levels)} maps given for {levels} levels of at least one pixel")
     if pooled is not None:
-        _check_like(pooled, "pooled", (_pooled_offsets(s.B * s.C, s.H2, s.W2, levels)[-1],), torch.float32, fmap1.device)
+        _check(pooled, "pooled", torch.float32, 1)
+        if pooled.numel() != _pooled_offsets(s.B * s.C, s.H2, s.W2, levels)[-1] or pooled.device != fmap1.device:
+            raise RuntimeError("pooled is not the buffer of these levels (pool_levels)")
     return s
 
 
+@functools.lru_cache(maxsize=64)
 def _pooled_offsets(planes, H, W, levels):
     """Where levels 1, 2, ... begin in the buffer of pool_levels, each on 256 bytes, and its elements."""
     at, offsets = 0, []
     for l in range(1, levels):
         offsets.append(at)
         at += (planes * (H >> l) * (W >> l) + 63) // 64 * 64
-    return offsets + [at]
+    return (*offsets, at)
 
 
 def pool_levels(fmap2, levels):
