@@ -1682,7 +1682,7 @@ PyramidBackward carve_pyramid_backward(const Pyramid& py, void* base) {
 }
 // The most samples of G at a time that a buffer has room for.  Buffers of pyramid_backward_bytes() have it for all that are wanted.
 PyramidGradPlan pyramid_grad_plan(const Pyramid& py, const PyramidBackward& pb, int op16, size_t room) {
-  for (int n = grad_chunk(py.d[0], py.levels, pb.sample_bytes, op16); n > 0;) {
+  for (int n = pb.end <= room ? grad_chunk(py.d[0], py.levels, pb.sample_bytes, op16) : 0; n > 0;) {
     const PyramidGradPlan plan = plan_pyramid_grads(py, n);
     if (pb.bytes(plan) <= room) return plan;
     // the scratch may differ with the cut of a smaller chunk, so that its room is looked at again

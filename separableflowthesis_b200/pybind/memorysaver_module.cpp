@@ -28,6 +28,7 @@ namespace {
 struct Abi {
   void* handle = nullptr;
   decltype(&sfb_workspace_bytes) workspace_bytes = nullptr;
+  decltype(&sfb_workspace_least_bytes) workspace_least_bytes = nullptr;
   decltype(&sfb_max_avg_forward) max_avg_forward = nullptr;
   decltype(&sfb_max_argmax_avg_forward) max_argmax_avg_forward = nullptr;
   decltype(&sfb_max_argmax_avg_backward) max_argmax_avg_backward = nullptr;
@@ -64,6 +65,7 @@ void load_abi() {
   g_abi.member = reinterpret_cast<decltype(g_abi.member)>(dlsym(g_abi.handle, symbol)); \
   TORCH_CHECK(g_abi.member != nullptr, "MemorySaver: libsepflow_b200.so lacks ", symbol)
   SFB_RESOLVE(workspace_bytes, "sfb_workspace_bytes");
+  SFB_RESOLVE(workspace_least_bytes, "sfb_workspace_least_bytes");
   SFB_RESOLVE(max_avg_forward, "sfb_max_avg_forward");
   SFB_RESOLVE(max_argmax_avg_forward, "sfb_max_argmax_avg_forward");
   SFB_RESOLVE(max_argmax_avg_backward, "sfb_max_argmax_avg_backward");
@@ -109,16 +111,41 @@ void check_attention(sfb_shape& s, const at::Tensor& A_u, const at::Tensor& A_v,
 
 // ---- workspace cache ---------------------------------------------------------------------------------
 std::mutex g_ws_mu;
-std::map<std::pair<int, void*>, at::Tensor> g_ws;
+struct CachedWorkspace {
+  at::Tensor buffer;
+  size_t too_large = SIZE_MAX;   // from this size on there was no memory: calls that can do with less do not ask for it again
+};
+std::map<std::pair<int, void*>, CachedWorkspace> g_ws;
+
+// Grows the buffer; the smaller one goes where there is no room for both (work in flight keeps it: the allocator hands memory on in the
+// order of the stream).
+void grow(CachedWorkspace& ws, size_t bytes, const at::Device& dev) {
+  if (ws.buffer.defined() && static_cast<size_t>(ws.buffer.numel()) >= bytes) return;
+  const auto options = at::TensorOptions().dtype(at::kByte).device(dev);
+  try {
+    ws.buffer = at::empty({static_cast<int64_t>(bytes)}, options);
+  } catch (const c10::OutOfMemoryError&) {
+    if (!ws.buffer.defined()) throw;
+    ws.buffer.reset();
+    ws.buffer = at::empty({static_cast<int64_t>(bytes)}, options);
+  }
+}
 
 at::Tensor workspace(int op, const sfb_shape& s, const at::Device& dev, cudaStream_t stream) {
   size_t bytes = g_abi.workspace_bytes(op, &s);
   if (bytes == 0) bytes = 256;  // the entry point then reports the precise reason
   std::lock_guard<std::mutex> lk(g_ws_mu);
-  at::Tensor& ws = g_ws[{dev.index(), static_cast<void*>(stream)}];
-  if (!ws.defined() || static_cast<size_t>(ws.numel()) < bytes)
-    ws = at::empty({static_cast<int64_t>(bytes)}, at::TensorOptions().dtype(at::kByte).device(dev));
-  return ws;
+  CachedWorkspace& ws = g_ws[{dev.index(), static_cast<void*>(stream)}];
+  const size_t least = bytes == 256 ? bytes : g_abi.workspace_least_bytes(op, &s);
+  if (least < bytes && bytes >= ws.too_large) bytes = least;
+  try {
+    grow(ws, bytes, dev);
+  } catch (const c10::OutOfMemoryError&) {
+    if (least >= bytes) throw;
+    ws.too_large = bytes;
+    grow(ws, least, dev);
+  }
+  return ws.buffer;
 }
 
 void raise_on(int rc, const char* name) {

@@ -117,3 +117,33 @@ def test_pyramid(shape, read, operands, shortage, cuda_device, monkeypatch):
                 assert relerr(x, ref) < H * W / 8 * 2 ** -23 + 2e-5, (short_forward, limit)
         with pytest.raises(torch.OutOfMemoryError):
             step(False, 1000)
+
+
+def test_native_module(cuda_device):
+    """The MemorySaver module asks torch's allocator itself, which is given room for the smaller buffer alone."""
+    from separableflowthesis_b200 import build
+    module = build.load_pybind_module()
+    B, H, W, C, Kc = 3, 65, 64, 64, 2
+    g = torch.Generator().manual_seed(1)
+    ints = lambda lo, hi, *s: torch.randint(lo, hi + 1, s, generator=g).float().to(cuda_device)
+    args = [ints(-2, 2, B, H, W, C), ints(-2, 2, B, H, W, C), ints(0, 2, B, H, W, Kc, W), ints(0, 2, B, H, W, Kc, H), ints(-2, 2, B, H, W, Kc, H),
+            ints(-2, 2, B, H, W, Kc, W)]
+    want = ops.compression_backward(*args)
+    shape = _lib.SfbShape(B, H, W, H, W, C, Kc)
+    full, least = [f(_lib.OP_COMPRESSION_BACKWARD, shape) for f in (_lib.load().sfb_workspace_bytes, _lib.load().sfb_workspace_least_bytes)]
+    assert least + 2 ** 26 < full
+    ops.release_workspaces()
+    stream = torch.cuda.Stream()   # whose buffer the module does not have yet
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total, before = torch.cuda.get_device_properties(cuda_device).total_memory, torch.cuda.memory_reserved()
+    try:
+        torch.cuda.set_per_process_memory_fraction((before + full) / total)   # the outputs want some of it, too
+        with torch.cuda.stream(stream):
+            for _ in range(2):
+                got = module.compression_backward(*args)
+                assert all(torch.equal(x, y) for x, y in zip(got, want))
+        torch.cuda.synchronize()
+        assert least <= torch.cuda.memory_reserved() - before < full
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
