@@ -9,9 +9,9 @@
 // warps (short columns: the softmax ends the walk).
 //
 // Two things decide the speed of such a walk, and both are handled explicitly:
-//  * latency: a thread needs plane e+1 only after it is done with plane e, so on its own it has one plane of
-//    loads in flight.  Each thread therefore prefetches its neighbourhoods a few planes ahead with cp.async into
-//    a ring of shared-memory slots that only it reads (no block barrier), see PlaneRing.
+//  * latency: a thread needs plane e+1 only after it is done with plane e, so planes are fetched a few ahead: the tiled form
+//    (calls with a status word) into a ring of tiles that a block shares, see PlaneFeed; the gather form, every thread its
+//    own neighbourhoods with cp.async, see PlaneRing.
 //  * operand bandwidth: all threads multiply by the same 54*Kc filter weights.  Reading them from shared memory
 //    costs a 32-lane register write per weight, more than the FMA they feed; instead the weights of the (up to
 //    four) channels being processed are staged in __constant__ memory, where an FMA reads them as an operand.
@@ -25,6 +25,7 @@
 //   weight grads: gW[k,c,tap] = sum X(shifted by tap) * gL, per-block partial sums, reduced in a fixed order by
 //                 a second kernel (bit-reproducible; no floating-point atomics)
 #include <climits>
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 
@@ -37,9 +38,28 @@ constexpr int AT_THREADS = 128;
 constexpr int AT_TAPS = 27;
 constexpr int AT_KC = 4;  // channels per launch of the forward / logit-gradient kernels and per constant-memory stage
 
-// Filter weights (k, c, td, th, tw) of the channels the running kernel works on, of both modules.
-constexpr int AT_WEIGHTS = AT_KC * 2 * AT_TAPS;
-__constant__ float c_att_weights[2 * AT_WEIGHTS];
+// Filter weights of the channels the running kernel works on, of both modules, in the order in which the kernel reads them, so that
+// weights which are used together lie in one 16-byte word (stage_weights_kernel).  n = 3 * th + tw is the neighbour a value comes
+// from: of the forward's tap (th, tw), of the input gradients' tap (2 - th, 2 - tw).
+constexpr int AT_WEIGHTS = 3 * AT_KC * 20;
+__constant__ float4 c_att_weights[2 * AT_WEIGHTS / 4];
+__host__ __device__ constexpr int forward_weight(int k, int c, int td, int n) { return ((td * 2 + c) * 9 + n) * AT_KC + k; }
+__host__ __device__ constexpr int input_grad_weight(int k, int c, int td, int n) { return (td * AT_KC + k) * 20 + n * 2 + c; }
+static_assert(forward_weight(AT_KC - 1, 1, 2, 8) < AT_WEIGHTS && input_grad_weight(AT_KC - 1, 1, 2, 8) < AT_WEIGHTS, "weights staged");
+template <int MODULE>
+__device__ __forceinline__ float att_weight(int i) { return reinterpret_cast<const float*>(c_att_weights)[MODULE * AT_WEIGHTS + i]; }
+
+struct StageWeights {
+  const float* weight[2];   // (k, c, td, th, tw), `channels` of them; null where no job uses the module
+  int channels;
+  bool input_grad;
+};
+__device__ float g_att_weights[2 * AT_WEIGHTS];   // on their way into constant memory
+__global__ void __launch_bounds__(AT_KC * 2 * AT_TAPS) stage_weights_kernel(const __grid_constant__ StageWeights s) {
+  const int m = blockIdx.x, i = threadIdx.x, k = i / (2 * AT_TAPS), c = i / AT_TAPS & 1, tap = i % AT_TAPS, td = tap / 9, n = tap % 9;
+  if (s.weight[m] == nullptr || k >= s.channels) return;
+  g_att_weights[m * AT_WEIGHTS + (s.input_grad ? input_grad_weight(k, c, td, 8 - n) : forward_weight(k, c, td, n))] = __ldg(s.weight[m] + i);
+}
 
 // Jobs of a launch: blocks first[j] .. first[j+1]-1 belong to job j.
 struct JobBlocks {
@@ -198,9 +218,9 @@ __device__ __forceinline__ void logits_walk_gather(const LogitsJobs::Job& job, f
         const float xv = *ring.slot(s, c * 9 + n);
 #pragma unroll
         for (int k = 0; k < KC; ++k) {
-          acc[2][k] = fmaf(xv, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + n], acc[2][k]);
-          acc[1][k] = fmaf(xv, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 9 + n], acc[1][k]);
-          acc[0][k] = fmaf(xv, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
+          acc[2][k] = fmaf(xv, att_weight<MODULE>(forward_weight(k, c, 0, n)), acc[2][k]);
+          acc[1][k] = fmaf(xv, att_weight<MODULE>(forward_weight(k, c, 1, n)), acc[1][k]);
+          acc[0][k] = fmaf(xv, att_weight<MODULE>(forward_weight(k, c, 2, n)), acc[0][k]);
         }
       }
     if (e > d0) emit(e - 1);
@@ -232,135 +252,222 @@ attention_logits_kernel(const __grid_constant__ LogitsJobs jobs, int Kc, int k0,
   if (SOFT) softmax_columns<KC>(job, Kc, k0, b, p, (size_t)N1);
 }
 
-// ---- logits, pixel tiles fetched by TMA -----------------------------------------------------------------
-// A block owns a tile of AT_TW x AT_TH image-1 pixels.  A producer warp fetches, plane by plane, the tile of both
-// input channels with its one-pixel halo as ONE tiled TMA load into a ring of stages (the box starts 4 pixels to the
-// left so that its x coordinate is a multiple of 16 bytes; pixels outside the image arrive as zeros, which is the
-// convolution's zero padding), and the 128 pixel threads read their 18 neighbours from shared memory at constant
-// offsets.  Against the gather above this removes the 18 per-thread copies per plane and their address arithmetic,
-// which were a third of the instructions of an issue-bound kernel.  Needs W1 % 4 == 0 (TMA strides are multiples of
-// 16 bytes).  grid of ceil(W1/32) * ceil(H1/4) * B * pieces blocks per job, block 128 + 32.
-constexpr int AT_TW = 32, AT_TH = 4;
-constexpr int AT_BOX_W = AT_TW + 8, AT_BOX_H = AT_TH + 2;
-constexpr int AT_TSTAGES = 6;
+// ---- logits, pixel tiles in shared memory -------------------------------------------------------------------
+// A block owns a tile of AT_TW x AT_TILE_ROWS image-1 pixels; a thread does AT_ROWS pixels of a column, one below the other.  The tile of both input
+// channels with its one-pixel halo comes in plane by plane through a ring of stages (PlaneFeed), a few planes ahead, and the threads read
+// their neighbours from shared memory at constant offsets.  Pixels outside the image are zeros = the convolution's padding.
+// A plane e adds to the outputs e - 1, e and e + 1: `older` (e - 1, complete after this plane), `newer` (e), and e + 1, which starts from the
+// bias.  Each takes over from the one before it in its first multiply-add, so nothing is moved from plane to plane.
+// Bound: FP32 issue.  Every pixel takes 54 multiply-adds per channel and plane with weights that are the same for all: they are operands from
+// constant memory (uniform registers), which a multiply-add takes at full rate, where one with three registers takes 1.2 to 1.6 cycles and a
+// packed one needs its weights moved to registers first (measured; 173 us instead of 118 for the logits below).  With one pixel to a thread
+// multiply-adds were 40 % of the instructions; four share a loaded weight, 18 of 36 neighbours, addresses and barrier: 75 %.  Two or three
+// pixels are within 5 % of it, with two channels slower (88 and 81 us instead of 69).  Logits of four levels: 1 x 55 x 128, four channels
+// 51 -> 33 us, 4 x 55 x 128 168 -> 103, 1 x 135 x 240 427 -> 238, 3 x 47 x 155 (three channels, copies) 121 -> 85; 8 x 47 x 156, one level,
+// two channels 96 -> 69.  The loop is 17 KB of instructions at four channels; what is left above the multiply-adds is fetching them, and barriers.
+// grid of ceil(W1/32) * ceil(H1/16) * B * pieces blocks per job, block 128.
+enum Feed : int { FEED_COPIES = 0, FEED_TMA = 1 };
+constexpr int AT_TW = 32, AT_WARPS = AT_THREADS / 32;
+constexpr int AT_BOX_W = AT_TW + 8;   // both forms: pixel w0 lies at column 4
+constexpr int AT_ROWS = 4, AT_TILE_ROWS = AT_WARPS * AT_ROWS;   // of a thread, of a tile
+constexpr int AT_STAGE_BYTES = 46 * 1024, AT_MAX_STAGES = 6;   // ring of a block
 
-// A TMA destination in shared memory must be 128-byte aligned; one channel's tile is 960 bytes, so every stage is
-// padded to a multiple of 128.
-constexpr uint32_t AT_TILE_BYTES = AT_BOX_H * AT_BOX_W * sizeof(float);
+// A TMA destination in shared memory must be 128-byte aligned, so every stage is padded to a multiple of 128.
 template <int NCH>
 struct alignas(128) AttentionTileStage {
-  float v[NCH][AT_BOX_H][AT_BOX_W];
+  float v[NCH][AT_TILE_ROWS + 2][AT_BOX_W];
 };
+constexpr int at_stages(size_t stage_bytes) {
+  return AT_STAGE_BYTES / (int)stage_bytes < AT_MAX_STAGES ? AT_STAGE_BYTES / (int)stage_bytes : AT_MAX_STAGES;
+}
 template <int NCH>
 struct AttentionTileSmem {
-  AttentionTileStage<NCH> x[AT_TSTAGES];
-  uint64_t full[AT_TSTAGES];
-  uint64_t empty[AT_TSTAGES];
+  static constexpr int STAGES = at_stages(sizeof(AttentionTileStage<NCH>));
+  AttentionTileStage<NCH> x[STAGES];
+  uint64_t full[STAGES];
   WaitCtl ctl;
 };
+static_assert(AttentionTileSmem<AT_KC>::STAGES >= 3, "planes in flight");
 
 // A block of a job: its pixel tile, sample and piece of the walk.
 struct TileBlock {
   int w0, h0, b, piece;
 };
+template <int ROWS>
 __device__ __forceinline__ TileBlock tile_block(int r, int B, int H1, int W1) {
-  const int tx = (W1 + AT_TW - 1) / AT_TW, tiles = tx * ((H1 + AT_TH - 1) / AT_TH);
+  const int tx = (W1 + AT_TW - 1) / AT_TW, tiles = tx * ((H1 + ROWS - 1) / ROWS);
   const int z = r / tiles, t = r - z * tiles, ty = t / tx;
-  return TileBlock{(t - ty * tx) * AT_TW, ty * AT_TH, z % B, z / B};
+  return TileBlock{(t - ty * tx) * AT_TW, ty * ROWS, z % B, z / B};
 }
 struct TileMaps {
   CUtensorMap m[MAX_ATTENTION_JOBS];
 };
 
-// The planes e0 .. e0 + n_planes - 1 of a tile, one box of `channel0` .. per plane.
-template <int NCH, class Smem>
-__device__ __forceinline__ void tile_producer(Smem& sm, const CUtensorMap* tm, const TileBlock& t, int e0, int n_planes, int channel0,
-                                              int* status) {
-  for (int i = 0; i < n_planes; ++i) {
-    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-    if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) return;
-    mbar_expect_tx(&sm.full[s], NCH * AT_TILE_BYTES);
-    tma_load_5d(sm.x[s].v, tm, &sm.full[s], t.w0 - 4, t.h0 - 1, e0 + i, channel0, t.b);
+// Copies by all WARPS warps of a block of a plane's tile of NCH channels (`src`: channel 0; channels `channel_stride` apart, of which
+// `channels` exist) with a halo of HALO pixels, a row per instruction.  Pixels and channels that do not exist become zeros.
+template <int NCH, int ROWS, int WIDTH, int HALO, int WARPS>
+__device__ __forceinline__ void copy_tile(float (&dst)[NCH][ROWS][WIDTH], const float* src, size_t channel_stride, int channels, int h0,
+                                          int w0, int H1, int W1) {
+  constexpr int COL0 = HALO != 0 ? 4 : 0;   // column of pixel w0
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 - HALO + warp, w = w0 + lane;
+  const float* const at = src + (ptrdiff_t)h * W1 + w;   // dereferenced where the pixel exists
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const bool column = c < channels && w < W1;
+    const float* row = at + c * channel_stride;
+#pragma unroll
+    for (int r = 0; r < ROWS; r += WARPS, row += WARPS * W1) {
+      if (ROWS % WARPS != 0 && r + WARPS > ROWS && r + warp >= ROWS) break;
+      const bool ok = column && (unsigned)(h + r) < (unsigned)H1;
+      cp_async4(&dst[c][r + warp][COL0 + lane], ok ? row : src, ok);
+    }
+  }
+  if (HALO == 0) return;
+  for (int i = threadIdx.x; i < NCH * ROWS * 2; i += WARPS * 32) {   // the columns on either side
+    const int c = i / (ROWS * 2), r = (i >> 1) % ROWS, hh = h0 - HALO + r, ww = (i & 1) != 0 ? w0 + AT_TW : w0 - 1;
+    const bool ok = c < channels && (unsigned)hh < (unsigned)H1 && (unsigned)ww < (unsigned)W1;
+    cp_async4(&dst[c][r][(i & 1) != 0 ? COL0 + AT_TW : COL0 - 1], ok ? src + c * channel_stride + hh * W1 + ww : src, ok);
   }
 }
 
-template <int KC, int MODULE>   // false: a wait ran out
-__device__ __forceinline__ bool logits_walk_tiled(AttentionTileSmem<2>& sm, const LogitsJobs::Job& job, const TileBlock& t, int Kc, int k0,
-                                                  int d0, int d1, int e0, int n_planes, int ty, int tx, int H1, int W1, int* status) {
-  const int D = job.D, h = t.h0 + ty, w = t.w0 + tx;
-  const bool valid = h < H1 && w < W1;
-  const size_t plane = (size_t)H1 * W1;
-  float* out = job.a + ((size_t)t.b * Kc + k0) * D * plane + (size_t)(valid ? h * W1 + w : 0);
+// The planes e0 .. e0 + n_planes - 1 of a tile, channels channel0 .. channel0 + NCH - 1 of each, to all threads of a block.  Where W1 is a
+// multiple of 4 and the tensor 16-byte aligned (TMA strides and addresses), a plane is ONE tiled TMA load, whose box starts 4 pixels
+// to the left so that its x coordinate is a multiple of 16 bytes; else 4-byte cp.async copies by all threads.  One barrier per plane: it
+// says that the plane is there for all, and that the stage of the one before has been read.  (With a warp of its own as the producer, and
+// stages handed back through mbarriers, a fifth of the instructions were polls and a plane's copies took that warp longer than the others its
+// arithmetic: 1 x 135 x 240 275 us instead of 250, 3 x 47 x 155 127 instead of 119, its weight gradients 290 instead of 151.)
+template <int NCH, int FEED>
+struct PlaneFeed {
+  static constexpr int STAGES = AttentionTileSmem<NCH>::STAGES;
+  AttentionTileSmem<NCH>& sm;
+  const CUtensorMap* tm;
+  const float* src;   // copies: first channel of the sample, plane e0; channels `channel_stride` apart, `channels` of them
+  size_t channel_stride;
+  int channels, e0, n_planes, channel0, H1, W1;
+  TileBlock t;
+  int* status;
 
-  float bk[KC], acc[3][KC];
+  __device__ __forceinline__ void fetch(int i) {
+    if constexpr (FEED == FEED_TMA) {
+      if (threadIdx.x == 0 && i < n_planes) {
+        const int s = i % STAGES;
+        mbar_expect_tx(&sm.full[s], sizeof(sm.x[s].v));
+        tma_load_5d(sm.x[s].v, tm, &sm.full[s], t.w0 - 4, t.h0 - 1, e0 + i, channel0, t.b);
+      }
+    } else {
+      if (i < n_planes)
+        copy_tile<NCH, AT_TILE_ROWS + 2, AT_BOX_W, 1, AT_WARPS>(sm.x[i % STAGES].v, src + (size_t)i * H1 * W1, channel_stride, channels,
+                                                                   t.h0, t.w0, H1, W1);
+      cp_async_commit();   // a group per plane, also where there is none
+    }
+  }
+  __device__ __forceinline__ void start() {
+    for (int i = 0; i < STAGES - 1; ++i) fetch(i);
+  }
+  // Plane i, or null in all threads when a wait ran out.
+  __device__ __forceinline__ const AttentionTileStage<NCH>* plane(int i) {
+    if constexpr (FEED == FEED_TMA) {
+      const bool ok = mbar_wait(&sm.full[i % STAGES], (i / STAGES) & 1u, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
+      fence_proxy_async_smem();   // this thread's reads of the stage that is filled again are over
+      if (!__syncthreads_and(ok)) return nullptr;
+    } else {
+      cp_async_wait<STAGES - 2>();
+      __syncthreads();
+    }
+    fetch(i + STAGES - 1);
+    return &sm.x[i % STAGES];
+  }
+};
+
+template <int KC, int MODULE, int FEED>   // false: a wait ran out
+__device__ __forceinline__ bool logits_walk_tiled(PlaneFeed<2, FEED>& feed, const LogitsJobs::Job& job, int Kc, int k0, int d0, int d1) {
+  constexpr int R = AT_ROWS;
+  const int D = job.D, H1 = feed.H1, W1 = feed.W1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = feed.t.h0 + warp * R, w = feed.t.w0 + lane;
+  const int rows = w < W1 ? min(R, H1 - h) : 0;   // of this thread; may be <= 0
+  const bool warp_has_rows = h < H1;
+  const size_t plane = (size_t)H1 * W1;
+  float* const out = job.a + ((size_t)feed.t.b * Kc + k0) * D * plane;   // the same for the whole block
+  const uint32_t p = rows > 0 ? (uint32_t)(h * W1 + w) : 0u;
+
+  float bk[KC], older[KC][R], newer[KC][R];
 #pragma unroll
   for (int k = 0; k < KC; ++k) {
     bk[k] = __ldg(job.bias + k0 + k);
-    acc[0][k] = acc[1][k] = acc[2][k] = bk[k];
+#pragma unroll
+    for (int r = 0; r < R; ++r) older[k][r] = newer[k][r] = bk[k];
   }
-  auto emit = [&](int d) {  // logit d is complete in acc[0]
+  auto emit = [&](int d) {
 #pragma unroll
     for (int k = 0; k < KC; ++k)
-      if (valid) out[((size_t)k * D + d) * plane] = acc[0][k];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r < rows) (out + ((size_t)k * D + d) * plane + r * W1)[p] = older[k][r];
   };
-  for (int i = 0; i < n_planes; ++i) {  // plane e feeds logits e+1 (tap td=0), e (td=1), e-1 (td=2)
-    const int e = e0 + i;
-    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-    if (!mbar_wait_warp(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE)) return false;
-    float xv[2][9];
+  for (int i = 0; i < feed.n_planes; ++i) {
+    const int e = feed.e0 + i;
+    const auto* stage = feed.plane(i);
+    if (stage == nullptr) return false;
+    if (!warp_has_rows) continue;
+    float x[2][R + 2][3];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int n = 0; n < 9; ++n) xv[c][n] = sm.x[s].v[c][ty + n / 3][tx + 3 + n % 3];
-    hand_back_stage(&sm.empty[s], tx);   // the neighbourhoods are in registers
+      for (int r = 0; r < R + 2; ++r)
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
+        for (int j = 0; j < 3; ++j) x[c][r][j] = stage->v[c][warp * R + r][lane + 3 + j];
+    auto taps = [&](auto td, float (&a)[KC][R], auto&& from) {   // a = from + taps
 #pragma unroll
-      for (int n = 0; n < 9; ++n) {
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int k = 0; k < KC; ++k) {
-          acc[2][k] = fmaf(xv[c][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + n], acc[2][k]);
-          acc[1][k] = fmaf(xv[c][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 9 + n], acc[1][k]);
-          acc[0][k] = fmaf(xv[c][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + 18 + n], acc[0][k]);
-        }
-      }
-    if (e > d0) emit(e - 1);
+        for (int n = 0; n < 9; ++n)
 #pragma unroll
-    for (int k = 0; k < KC; ++k) { acc[0][k] = acc[1][k]; acc[1][k] = acc[2][k]; acc[2][k] = bk[k]; }
+          for (int k = 0; k < KC; ++k) {
+            const float wt = att_weight<MODULE>(forward_weight(k, c, decltype(td)::value, n));
+#pragma unroll
+            for (int r = 0; r < R; ++r) a[k][r] = fmaf(x[c][r + n / 3][n % 3], wt, c == 0 && n == 0 ? from(k, r) : a[k][r]);
+          }
+    };
+    if (e > d0) {
+      taps(std::integral_constant<int, 2>{}, older, [&](int k, int r) { return older[k][r]; });
+      emit(e - 1);
+    }
+    if (e >= d0 && e < d1) taps(std::integral_constant<int, 1>{}, older, [&](int k, int r) { return newer[k][r]; });
+    if (e + 1 < d1) taps(std::integral_constant<int, 0>{}, newer, [&](int k, int) { return bk[k]; });
   }
-  if (d1 == D) emit(D - 1);
+  if (d1 == D && warp_has_rows) emit(D - 1);
   return true;
 }
 
-template <int KC, bool SOFT>
-__global__ void __launch_bounds__(AT_THREADS + 32)
+template <int KC, bool SOFT, int FEED>
+__global__ void __launch_bounds__(AT_THREADS)
 attention_logits_tiled_kernel(const __grid_constant__ TileMaps maps, const __grid_constant__ LogitsJobs jobs, int Kc, int k0, int B,
                               int H1, int W1, int* status) {
   if (!cta_has_work(status)) return;
   __shared__ __align__(128) AttentionTileSmem<2> sm;
   const int ji = job_of(jobs.blocks, blockIdx.x);
   const LogitsJobs::Job& job = jobs.j[ji];
-  const TileBlock t = tile_block(blockIdx.x - jobs.blocks.first[ji], B, H1, W1);
+  const TileBlock t = tile_block<AT_TILE_ROWS>(blockIdx.x - jobs.blocks.first[ji], B, H1, W1);
   const int d0 = t.piece * job.dc, d1 = min(d0 + job.dc, job.D);
   const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, job.D) - e0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t plane = (size_t)H1 * W1;
+  PlaneFeed<2, FEED> feed{sm, &maps.m[ji], job.x + (size_t)t.b * job.x_sb + e0 * plane, job.D * plane, 2, e0, n_planes, 0, H1, W1, t, status};
   if (threadIdx.x == 0) {
-    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
+    if (FEED == FEED_TMA) {
+      for (int s = 0; s < feed.STAGES; ++s) mbar_init(&sm.full[s], 1);
+      prefetch_tensormap(feed.tm);
+    }
     wait_ctl_init(&sm.ctl, 0);
     fence_barrier_init();
-    prefetch_tensormap(&maps.m[ji]);
   }
   __syncthreads();
-  if (warp == AT_THREADS / 32) {
-    if (lane == 0) tile_producer<2>(sm, &maps.m[ji], t, e0, n_planes, 0, status);
-    __syncwarp();
-  } else {
-    bool ok = true;
-    by_module(job.module, [&](auto m) {
-      ok = logits_walk_tiled<KC, decltype(m)::value>(sm, job, t, Kc, k0, d0, d1, e0, n_planes, warp, lane, H1, W1, status);
-    });
-    const int h = t.h0 + warp, w = t.w0 + lane;
-    if (SOFT && ok && h < H1 && w < W1) softmax_columns<KC>(job, Kc, k0, t.b, h * W1 + w, (size_t)H1 * W1);
+  feed.start();
+  bool ok = true;
+  by_module(job.module, [&](auto m) { ok = logits_walk_tiled<KC, decltype(m)::value>(feed, job, Kc, k0, d0, d1); });
+  if (SOFT && ok) {
+    const int warp = threadIdx.x >> 5, w = t.w0 + (threadIdx.x & 31);
+    if (w < W1)
+      for (int h = t.h0 + warp * AT_ROWS; h < min(t.h0 + (warp + 1) * AT_ROWS, H1); ++h) softmax_columns<KC>(job, Kc, k0, t.b, h * W1 + w, plane);
   }
   __syncthreads();
   if (wait_ctl_aborted(&sm.ctl)) {
@@ -440,12 +547,12 @@ attention_softmax_kernel(const __grid_constant__ SoftmaxJobs jobs, int N1, unsig
 
 // Tensor map over a channels-first tensor (B, nch, D, H1, W1) whose samples are `sb` elements apart; the box is one
 // plane's pixel tile of `box_ch` channels, with the stencil's halo or without.
-static cudaError_t tile_map(CUtensorMap* tm, const float* x, long long sb, int nch, int box_ch, const AttentionDims& d,
+static cudaError_t tile_map(CUtensorMap* tm, const float* x, long long sb, int nch, int box_ch, const AttentionDims& d, int rows,
                             bool halo) {
   const uint64_t N1 = (uint64_t)d.H1 * d.W1;
   const uint64_t dims[5] = {(uint64_t)d.W1, (uint64_t)d.H1, (uint64_t)d.D, (uint64_t)nch, (uint64_t)d.B};
   const uint64_t strides[4] = {(uint64_t)d.W1 * 4, N1 * 4, (uint64_t)d.D * N1 * 4, (uint64_t)sb * 4};
-  const uint32_t box[5] = {(uint32_t)(halo ? AT_BOX_W : AT_TW), (uint32_t)(halo ? AT_BOX_H : AT_TH), 1, (uint32_t)box_ch, 1};
+  const uint32_t box[5] = {(uint32_t)(halo ? AT_BOX_W : AT_TW), (uint32_t)(rows + (halo ? 2 : 0)), 1, (uint32_t)box_ch, 1};
   return encode_plain_map(tm, x, 5, dims, strides, box);
 }
 static bool tileable(const AttentionDims& d, const void* x, long long sb) {
@@ -612,14 +719,12 @@ __device__ __forceinline__ void input_grad_walk_gather(const InputGradJobs::Job&
     for (int k = 0; k < KC; ++k)
 #pragma unroll
       for (int n = 0; n < 9; ++n) {
-        // neighbour n = (nh, nw) holds gL at (h + nh - 1, w + nw - 1), which meets tap th = 2 - nh, tw = 2 - nw
-        const int t = (2 - n / 3) * 3 + (2 - n % 3);
         const float v = *ring.slot(s, k * 9 + n);
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int td = 0; td < 3; ++td)
-            acc[c][td] = fmaf(v, c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + td * 9 + t], acc[c][td]);
+            acc[c][td] = fmaf(v, att_weight<MODULE>(input_grad_weight(k, c, td, n)), acc[c][td]);
       }
     if (e > d0) emit(e - 1);
 #pragma unroll
@@ -783,203 +888,260 @@ attention_reduce_partials_kernel(const __grid_constant__ PartialSums sums) {
   if (threadIdx.x == 0) sums.out[j][i] = red[0];
 }
 
-// ---- input and weight gradients, pixel tiles fetched by TMA -------------------------------------------------
+// ---- input and weight gradients, pixel tiles in shared memory ---------------------------------------------
 // Same arithmetic as the two gather kernels above with the tile scheme of attention_logits_tiled_kernel.
-// Input gradients: the stage holds the tile (with halo) of the KC logit-gradient channels of one plane.
-template <int KC, int MODULE>
-__device__ __forceinline__ void input_grad_walk_tiled(AttentionTileSmem<KC>& sm, const InputGradJobs::Job& job, const TileBlock& t,
-                                                      int accumulate, int k0, int d0, int d1, int e0, int n_planes, int ty, int tx, int H1,
-                                                      int W1, int* status) {
-  const int D = job.D, h = t.h0 + ty, w = t.w0 + tx;
-  const bool valid = h < H1 && w < W1;
-  const size_t plane = (size_t)H1 * W1, p = valid ? (size_t)h * W1 + w : 0;
-  float* o0 = job.gx + (size_t)t.b * 2 * D * plane + p;
-  const float* ad = job.add != nullptr && k0 == 0 ? job.add + (size_t)t.b * job.add_sb + p : nullptr;
-  float acc[2][3];  // [c][output d = e-1, e, e+1]
+// Input gradients: the stage holds the tile (with halo) of the KC logit-gradient channels of one plane.  Bound like the logits.
+// 8 x 47 x 156, two channels, one level: 122 -> 82 us; 3 x 47 x 155, three channels, four levels (copies) 157 -> 98; 8 x 135 x 240, four
+// channels 1.76 -> 1.42 ms; 2 x 48 x 64, two channels, four levels 19 -> 13.
+template <int KC, int MODULE, int FEED>
+__device__ __forceinline__ void input_grad_walk_tiled(PlaneFeed<KC, FEED>& feed, const InputGradJobs::Job& job, int accumulate, int k0,
+                                                      int d0, int d1) {
+  constexpr int R = AT_ROWS;
+  const int D = job.D, H1 = feed.H1, W1 = feed.W1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = feed.t.h0 + warp * R, w = feed.t.w0 + lane;
+  const int rows = w < W1 ? min(R, H1 - h) : 0;   // of this thread; may be <= 0
+  const bool warp_has_rows = h < H1;
+  const size_t plane = (size_t)H1 * W1;
+  const uint32_t p = rows > 0 ? (uint32_t)(h * W1 + w) : 0u;
+  float* const o0 = job.gx + (size_t)feed.t.b * 2 * D * plane;   // the same for the whole block
+  // what the sums are added to: the given addend, for a later chunk of channels the earlier ones' sums
+  const float* const before = accumulate ? o0 : (job.add != nullptr ? job.add + (size_t)feed.t.b * job.add_sb : nullptr);
+  float older[2][R], newer[2][R], addend[2][R];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) acc[c][0] = acc[c][1] = acc[c][2] = 0.f;
-  auto emit = [&](int d) {
-    if (!valid) return;
+  for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const size_t i = ((size_t)c * D + d) * plane;
-      float v = acc[c][0];
-      if (ad != nullptr) v += __ldg(ad + i);
-      if (accumulate) v += o0[i];
-      o0[i] = v;
-    }
+    for (int r = 0; r < R; ++r) older[c][r] = newer[c][r] = 0.f;
+  auto fetch = [&](int d) {   // asked for a plane's arithmetic before it is needed
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        addend[c][r] = before != nullptr && r < rows ? (before + ((size_t)c * D + d) * plane + r * W1)[p] : 0.f;
   };
-  for (int i = 0; i < n_planes; ++i) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
-    const int e = e0 + i;
-    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-    if (!mbar_wait_warp(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE)) return;
-    float v[KC][9];
+  auto emit = [&](int d) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r < rows) (o0 + ((size_t)c * D + d) * plane + r * W1)[p] = older[c][r] + addend[c][r];
+  };
+  for (int i = 0; i < feed.n_planes; ++i) {  // plane e of gL feeds gX planes e-1 (td=0), e (td=1), e+1 (td=2)
+    const int e = feed.e0 + i;
+    if (e > d0) fetch(e - 1);
+    const auto* stage = feed.plane(i);
+    if (stage == nullptr) return;
+    if (!warp_has_rows) continue;
+    float v[KC][R + 2][3];
 #pragma unroll
     for (int k = 0; k < KC; ++k)
 #pragma unroll
-      for (int n = 0; n < 9; ++n) v[k][n] = sm.x[s].v[k][ty + n / 3][tx + 3 + n % 3];
-    hand_back_stage(&sm.empty[s], tx);
+      for (int r = 0; r < R + 2; ++r)
 #pragma unroll
-    for (int k = 0; k < KC; ++k)
+        for (int j = 0; j < 3; ++j) v[k][r][j] = stage->v[k][warp * R + r][lane + 3 + j];
+    auto taps = [&](auto td, float (&a)[2][R], auto&& from) {   // a = from + taps
 #pragma unroll
-      for (int n = 0; n < 9; ++n) {
-        // neighbour n = (nh, nw) holds gL at (h + nh - 1, w + nw - 1), which meets tap th = 2 - nh, tw = 2 - nw
-        const int tap = (2 - n / 3) * 3 + (2 - n % 3);
+      for (int k = 0; k < KC; ++k)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int n = 0; n < 9; ++n)
 #pragma unroll
-          for (int td = 0; td < 3; ++td)
-            acc[c][td] = fmaf(v[k][n], c_att_weights[MODULE * AT_WEIGHTS + (k * 2 + c) * AT_TAPS + td * 9 + tap], acc[c][td]);
-      }
-    if (e > d0) emit(e - 1);
+          for (int c = 0; c < 2; ++c) {
+            const float wt = att_weight<MODULE>(input_grad_weight(k, c, decltype(td)::value, n));
 #pragma unroll
-    for (int c = 0; c < 2; ++c) { acc[c][0] = acc[c][1]; acc[c][1] = acc[c][2]; acc[c][2] = 0.f; }
+            for (int r = 0; r < R; ++r) a[c][r] = fmaf(v[k][r + n / 3][n % 3], wt, k == 0 && n == 0 ? from(c, r) : a[c][r]);
+          }
+    };
+    if (e > d0) {
+      taps(std::integral_constant<int, 0>{}, older, [&](int c, int r) { return older[c][r]; });
+      emit(e - 1);
+    }
+    if (e >= d0 && e < d1) taps(std::integral_constant<int, 1>{}, older, [&](int c, int r) { return newer[c][r]; });
+    if (e + 1 < d1) taps(std::integral_constant<int, 2>{}, newer, [&](int, int) { return 0.f; });
   }
-  if (d1 == D) emit(D - 1);
+  if (d1 == D) {
+    fetch(D - 1);
+    emit(D - 1);
+  }
 }
 
-template <int KC>
-__global__ void __launch_bounds__(AT_THREADS + 32)
-attention_input_grad_tiled_kernel(const __grid_constant__ TileMaps maps, const __grid_constant__ InputGradJobs jobs, int accumulate, int k0,
-                                  int B, int H1, int W1, int* status) {
+template <int KC, int FEED>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_input_grad_tiled_kernel(const __grid_constant__ TileMaps maps, const __grid_constant__ InputGradJobs jobs, int accumulate, int Kc,
+                                  int k0, int B, int H1, int W1, int* status) {
   if (!cta_has_work(status)) return;
   __shared__ __align__(128) AttentionTileSmem<KC> sm;
   const int ji = job_of(jobs.blocks, blockIdx.x);
   const InputGradJobs::Job& job = jobs.j[ji];
-  const TileBlock t = tile_block(blockIdx.x - jobs.blocks.first[ji], B, H1, W1);
+  const TileBlock t = tile_block<AT_TILE_ROWS>(blockIdx.x - jobs.blocks.first[ji], B, H1, W1);
   const int d0 = t.piece * job.dc, d1 = min(d0 + job.dc, job.D);
   const int e0 = max(d0 - 1, 0), n_planes = min(d1 + 1, job.D) - e0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t plane = (size_t)H1 * W1;
+  PlaneFeed<KC, FEED> feed{sm, &maps.m[ji], job.gl + (((size_t)t.b * Kc + k0) * job.D + e0) * plane, job.D * plane, Kc - k0, e0, n_planes, k0,
+                              H1, W1, t, status};
   if (threadIdx.x == 0) {
-    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], AT_THREADS / 32); }
+    if (FEED == FEED_TMA) {
+      for (int s = 0; s < feed.STAGES; ++s) mbar_init(&sm.full[s], 1);
+      prefetch_tensormap(feed.tm);
+    }
     wait_ctl_init(&sm.ctl, 0);
     fence_barrier_init();
-    prefetch_tensormap(&maps.m[ji]);
   }
   __syncthreads();
-  if (warp == AT_THREADS / 32) {
-    if (lane == 0) tile_producer<KC>(sm, &maps.m[ji], t, e0, n_planes, k0, status);
-    __syncwarp();
-  } else {
-    by_module(job.module, [&](auto m) {
-      input_grad_walk_tiled<KC, decltype(m)::value>(sm, job, t, accumulate, k0, d0, d1, e0, n_planes, warp, lane, H1, W1, status);
-    });
-  }
+  feed.start();
+  by_module(job.module, [&](auto m) { input_grad_walk_tiled<KC, decltype(m)::value>(feed, job, accumulate, k0, d0, d1); });
   __syncthreads();
   if (wait_ctl_aborted(&sm.ctl)) {
     let_copies_land();
   }
 }
 
-// Weight gradients: warps 0-3 own input channel 0, warps 4-7 input channel 1, each thread KW output channels of its
-// pixel; the stage holds the tile (with halo) of plane e of both X channels and the tile (without halo) of plane e+1 of
+// Weight gradients: half of the warps own input channel 0, the others input channel 1, each thread KW output channels of its WG_ROWS
+// pixels; the stage holds the tile (with halo) of plane e of both X channels and the tile (without halo) of plane e+1 of
 // the KW logit-gradient channels, which the two halves share.  The sums of two output channels are one packed pair
-// (fma.rn.f32x2 with the X value in both halves), which halves the multiply-add instructions; KW odd leaves one
-// channel on scalar ones.  A piece is `dc` planes of X.
-// grid (ceil(W1/32) * ceil(H1/4) * B * pieces blocks per job, chunks of KW channels); partial: of the module, (Kc * 2 * 27, rows).
-constexpr int WG_WARPS = 8;
+// (fma.rn.f32x2 with the X value in both halves), which halves the multiply-add instructions.  Several pixels to a thread share the X
+// values they read; with two channels to a thread the sums leave registers for three blocks on an SM (with four there was one, of eight warps).
+// 8 x 47 x 156, two channels, one level: 151 -> 73 us; 3 x 47 x 155, three channels, four levels (copies) 193 -> 151; 8 x 135 x 240, four
+// channels 1.67 -> 1.34 ms; 2 x 48 x 64, two channels, four levels 32 -> 15.  Bound: the FMA pipe (2.25 cycles for a packed multiply-add with
+// an operand kept) and issue beside it.  Logit gradients of three planes are
+// held, in registers whose roles rotate over three planes of the loop.  A piece is `dc` planes of X.
+// TMA loads are issued by a warp of their own; copies by all warps, which then meet at a barrier per plane as in PlaneFeed.
+// grid (ceil(W1/32) * ceil(H1/8) * B * pieces blocks per job, chunks of KW channels), block wg_threads(FEED); partial: of the module,
+// (Kc * 2 * 27, rows).
+constexpr int WG_GROUPS = 2, WG_WARPS = 2 * WG_GROUPS, WG_ROWS = 4, WG_TILE_ROWS = WG_GROUPS * WG_ROWS, WG_MAX_CHANNELS = 2;
+constexpr int wg_channels(int Kc) { return Kc < WG_MAX_CHANNELS ? Kc : WG_MAX_CHANNELS; }   // of a thread
 template <int KW>
 struct WeightGradTileSmem {
   struct alignas(128) Stage {   // both parts are TMA destinations: 128-byte aligned
-    alignas(128) float x[2][AT_BOX_H][AT_BOX_W];
-    alignas(128) float g[KW][AT_TH][AT_TW];
-  } st[AT_TSTAGES];
-  uint64_t full[AT_TSTAGES];
-  uint64_t empty[AT_TSTAGES];
+    alignas(128) float x[2][WG_TILE_ROWS + 2][AT_BOX_W];
+    alignas(128) float g[KW][WG_TILE_ROWS][AT_TW];
+  };
+  static constexpr int STAGES = at_stages(sizeof(Stage));
+  Stage st[STAGES];
+  uint64_t full[STAGES];
+  uint64_t empty[STAGES];
   WaitCtl ctl;
   float red[WG_WARPS * KW * AT_TAPS];
 };
 
-template <int KW>
-__global__ void __launch_bounds__(WG_WARPS * 32 + 32, 1)
+__host__ __device__ constexpr int wg_threads(int feed) { return WG_WARPS * 32 + (feed == FEED_TMA ? 32 : 0); }
+template <int KW, int FEED>
+__global__ void __launch_bounds__(wg_threads(FEED), 3)
 attention_weight_grad_tiled_kernel(const __grid_constant__ TileMaps maps_x, const __grid_constant__ TileMaps maps_gl,
                                    const __grid_constant__ WeightGradJobs jobs, int Kc, int B, int H1, int W1, int* status) {
   if (!cta_has_work(status)) return;
   __shared__ __align__(128) WeightGradTileSmem<KW> sm;
-  constexpr int KP = KW / 2;   // packed channel pairs
+  constexpr int R = WG_ROWS, STAGES = WeightGradTileSmem<KW>::STAGES;
   const int ji = job_of(jobs.blocks, blockIdx.x), r = blockIdx.x - jobs.blocks.first[ji];
   const WeightGradJobs::Job& job = jobs.j[ji];
-  const TileBlock tb = tile_block(r, B, H1, W1);
+  const TileBlock tb = tile_block<WG_TILE_ROWS>(r, B, H1, W1);
   const int w0 = tb.w0, h0 = tb.h0, b = tb.b, k0 = blockIdx.y * KW, D = job.D;
   const float* __restrict__ const gl = job.gl;
   const CUtensorMap *const tm_x = &maps_x.m[ji], *const tm_gl = &maps_gl.m[ji];
   const int e0 = tb.piece * job.dc, n_planes = min(job.dc, D - e0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t plane = (size_t)H1 * W1;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < AT_TSTAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], WG_WARPS); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], WG_WARPS); }
     wait_ctl_init(&sm.ctl, 0);
     fence_barrier_init();
-    prefetch_tensormap(tm_x);
-    prefetch_tensormap(tm_gl);
+    if (FEED == FEED_TMA) {
+      prefetch_tensormap(tm_x);
+      prefetch_tensormap(tm_gl);
+    }
   }
   __syncthreads();
-  if (warp == WG_WARPS) {  // producer
-    if (lane == 0) {
-      for (int i = 0; i < n_planes; ++i) {
-        const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
-        mbar_expect_tx(&sm.full[s], 2 * AT_TILE_BYTES + KW * AT_TH * AT_TW * (uint32_t)sizeof(float));
-        tma_load_5d(sm.st[s].x, tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
-        tma_load_5d(sm.st[s].g, tm_gl, &sm.full[s], w0, h0, e0 + i + 1, k0, b);  // plane D, channels >= Kc read as zero
-      }
+  auto copy_plane = [&](int i) {
+    if (i < n_planes) {
+      auto& st = sm.st[i % STAGES];
+      copy_tile<2, WG_TILE_ROWS + 2, AT_BOX_W, 1, WG_WARPS>(st.x, job.x + (size_t)b * job.x_sb + (size_t)(e0 + i) * plane, D * plane, 2, h0, w0, H1,
+                                                            W1);
+      const bool has_next = e0 + i + 1 < D;
+      copy_tile<KW, WG_TILE_ROWS, AT_TW, 0, WG_WARPS>(st.g, gl + (((size_t)b * Kc + k0) * D + (has_next ? e0 + i + 1 : 0)) * plane, D * plane,
+                                                      has_next ? Kc - k0 : 0, h0, w0, H1, W1);
+    }
+    cp_async_commit();   // a group per plane, also where there is none
+  };
+  if constexpr (FEED == FEED_COPIES) {
+    for (int i = 0; i < STAGES - 1; ++i) copy_plane(i);
+  } else if (warp == WG_WARPS) {  // producer
+    if (lane != 0) return;
+    for (int i = 0; i < n_planes; ++i) {
+      const uint32_t s = i % STAGES, ph = (i / STAGES) & 1u;
+      if (!mbar_wait(&sm.empty[s], ph ^ 1u, &sm.ctl, status, DEV_TIMEOUT_PRODUCER)) { let_copies_land(); break; }
+      mbar_expect_tx(&sm.full[s], sizeof(sm.st[s].x) + sizeof(sm.st[s].g));
+      tma_load_5d(sm.st[s].x, tm_x, &sm.full[s], w0 - 4, h0 - 1, e0 + i, 0, b);
+      tma_load_5d(sm.st[s].g, tm_gl, &sm.full[s], w0, h0, e0 + i + 1, k0, b);  // plane D, channels >= Kc read as zero
     }
     return;
   }
-  const int tx = lane, ty = warp & 3, c = warp >> 2;
-  const int h = h0 + ty, w = w0 + tx;
-  const bool valid = h < H1 && w < W1;
-  const size_t plane = (size_t)H1 * W1;
-  uint64_t acc2[KP > 0 ? KP * AT_TAPS : 1];         // [pair][td][neighbour]
-  float acc1[(KW & 1) != 0 ? AT_TAPS : 1];          // the odd channel
+  const int q = warp % WG_GROUPS, c = warp / WG_GROUPS;
+  const int h = h0 + q * R, w = w0 + lane, rows = w < W1 ? min(R, H1 - h) : 0;
+  using Value = std::conditional_t<KW == 2, uint64_t, float>;   // a value of all channels of the thread
+  auto mul_add = [](Value g, float v, Value a) -> Value {
+    if constexpr (KW == 2) return fma2(pack2(v, v), g, a);
+    else return fmaf(v, g, a);
+  };
+  Value acc[AT_TAPS];   // [td * 9 + neighbour]
 #pragma unroll
-  for (int i = 0; i < KP * AT_TAPS; ++i) acc2[i] = 0ull;
-  if constexpr ((KW & 1) != 0) {
+  for (int i = 0; i < AT_TAPS; ++i) acc[i] = Value(0);
+  Value g[3][R];        // gL of plane d in g[(d - e0 + 3) % 3]
 #pragma unroll
-    for (int i = 0; i < AT_TAPS; ++i) acc1[i] = 0.f;
-  }
-  float g_prev[KW], g_cur[KW], g_next[KW];
+  for (int rr = 0; rr < R; ++rr) {
+    float before[2], here[2];
 #pragma unroll
-  for (int k = 0; k < KW; ++k) {
-    const bool ok = valid && k0 + k < Kc;
-    const float* gp = gl + (((size_t)b * Kc + (ok ? k0 + k : 0)) * D + e0) * plane + (ok ? (size_t)h * W1 + w : 0);
-    g_prev[k] = (ok && e0 > 0) ? __ldg(gp - plane) : 0.f;
-    g_cur[k] = ok ? __ldg(gp) : 0.f;
+    for (int k = 0; k < KW; ++k) {
+      const bool ok = rr < rows && k0 + k < Kc;
+      const float* gp = gl + (((size_t)b * Kc + (ok ? k0 + k : 0)) * D + e0) * plane + (ok ? (size_t)(h + rr) * W1 + w : 0);
+      before[k] = (ok && e0 > 0) ? __ldg(gp - plane) : 0.f;
+      here[k] = ok ? __ldg(gp) : 0.f;
+    }
+    if constexpr (KW == 2) {
+      g[2][rr] = pack2(before[0], before[1]);
+      g[0][rr] = pack2(here[0], here[1]);
+    } else {
+      g[2][rr] = before[0];
+      g[0][rr] = here[0];
+    }
   }
   bool alive = true;
-  for (int i = 0; i < n_planes; ++i) {  // plane e of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2)
-    const uint32_t s = i % AT_TSTAGES, ph = (i / AT_TSTAGES) & 1u;
-    const bool ok = mbar_wait(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE);
-    if (!__all_sync(0xffffffffu, ok)) { let_copies_land(); alive = false; break; }
-    float v[9];
-#pragma unroll
-    for (int n = 0; n < 9; ++n) v[n] = sm.st[s].x[c][ty + n / 3][tx + 3 + n % 3];
-#pragma unroll
-    for (int k = 0; k < KW; ++k) g_next[k] = sm.st[s].g[k][ty][tx];
-    hand_back_stage(&sm.empty[s], lane);
-#pragma unroll
-    for (int q = 0; q < KP; ++q) {
-      const uint64_t gn = pack2(g_next[2 * q], g_next[2 * q + 1]), gc = pack2(g_cur[2 * q], g_cur[2 * q + 1]),
-                     gp = pack2(g_prev[2 * q], g_prev[2 * q + 1]);
-#pragma unroll
-      for (int n = 0; n < 9; ++n) {
-        const uint64_t vv = pack2(v[n], v[n]);
-        acc2[q * AT_TAPS + n] = fma2(gn, vv, acc2[q * AT_TAPS + n]);
-        acc2[q * AT_TAPS + 9 + n] = fma2(gc, vv, acc2[q * AT_TAPS + 9 + n]);
-        acc2[q * AT_TAPS + 18 + n] = fma2(gp, vv, acc2[q * AT_TAPS + 18 + n]);
-      }
-    }
-    if constexpr ((KW & 1) != 0) {
-#pragma unroll
-      for (int n = 0; n < 9; ++n) {
-        acc1[n] = fmaf(g_next[KW - 1], v[n], acc1[n]);
-        acc1[9 + n] = fmaf(g_cur[KW - 1], v[n], acc1[9 + n]);
-        acc1[18 + n] = fmaf(g_prev[KW - 1], v[n], acc1[18 + n]);
-      }
+  auto plane_sums = [&](int i, auto phase) -> bool {   // plane e0 + i of X meets gL at d = e+1 (td=0), e (td=1), e-1 (td=2); i % 3 == phase
+    constexpr int P = decltype(phase)::value;
+    const uint32_t s = i % STAGES, ph = (i / STAGES) & 1u;
+    if constexpr (FEED == FEED_TMA) {
+      if (!mbar_wait_warp(&sm.full[s], ph, &sm.ctl, status, DEV_TIMEOUT_EPILOGUE)) { let_copies_land(); return false; }
+    } else {
+      cp_async_wait<STAGES - 2>();
+      named_bar_sync(1, WG_WARPS * 32);   // the plane is there for all, and the one before has been read
+      copy_plane(i + STAGES - 1);
     }
 #pragma unroll
-    for (int k = 0; k < KW; ++k) { g_prev[k] = g_cur[k]; g_cur[k] = g_next[k]; }
+    for (int rr = 0; rr < R; ++rr) {
+      if constexpr (KW == 2) g[(P + 1) % 3][rr] = pack2(sm.st[s].g[0][q * R + rr][lane], sm.st[s].g[1][q * R + rr][lane]);
+      else g[(P + 1) % 3][rr] = sm.st[s].g[0][q * R + rr][lane];
+    }
+#pragma unroll
+    for (int y = 0; y < R + 2; ++y)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const float v = sm.st[s].x[c][q * R + y][lane + 3 + j];
+#pragma unroll
+        for (int th = 0; th < 3; ++th) {   // the pixel in row y - th sees the value as its neighbour (th, j)
+          if (y - th < 0 || y - th >= R) continue;
+#pragma unroll
+          for (int td = 0; td < 3; ++td) {
+            Value& a = acc[td * 9 + th * 3 + j];
+            a = mul_add(g[(P + 4 - td) % 3][y - th], v, a);
+          }
+        }
+      }
+    if constexpr (FEED == FEED_TMA) hand_back_stage(&sm.empty[s], lane);
+    return true;
+  };
+  for (int i = 0; i < n_planes && alive; i += 3) {
+    alive = plane_sums(i, std::integral_constant<int, 0>{});
+    if (alive && i + 1 < n_planes) alive = plane_sums(i + 1, std::integral_constant<int, 1>{});
+    if (alive && i + 2 < n_planes) alive = plane_sums(i + 2, std::integral_constant<int, 2>{});
   }
-  // reduce over the 128 pixel threads of each input channel (named barrier 1: the producer warp has left);
+  // reduce over the threads of each input channel (named barrier 1: the producer warp has left);
   // column (k, c, td, n) goes to row (k0 + k) * 54 + c * 27 + td * 9 + n of the partial sums
   auto put = [&](int i, float sum) {
     if (!alive) sum = 0.f;
@@ -988,28 +1150,26 @@ attention_weight_grad_tiled_kernel(const __grid_constant__ TileMaps maps_x, cons
     if (lane == 0) sm.red[warp * KW * AT_TAPS + i] = sum;
   };
 #pragma unroll
-  for (int q = 0; q < KP; ++q)
-#pragma unroll
-    for (int t = 0; t < AT_TAPS; ++t) {
+  for (int t = 0; t < AT_TAPS; ++t) {
+    if constexpr (KW == 2) {
       float lo, hi;
-      unpack2(acc2[q * AT_TAPS + t], lo, hi);
-      put(2 * q * AT_TAPS + t, lo);
-      put((2 * q + 1) * AT_TAPS + t, hi);
+      unpack2(acc[t], lo, hi);
+      put(t, lo);
+      put(AT_TAPS + t, hi);
+    } else {
+      put(t, acc[t]);
     }
-  if constexpr ((KW & 1) != 0) {
-#pragma unroll
-    for (int t = 0; t < AT_TAPS; ++t) put((KW - 1) * AT_TAPS + t, acc1[t]);
   }
   named_bar_sync(1, WG_WARPS * 32);
-  const size_t rows = job.rows;
+  const size_t n_rows = job.rows;
   float* dst = job.partial + job.row0 + r;
   for (int i = threadIdx.x; i < 2 * KW * AT_TAPS; i += WG_WARPS * 32) {
     const int cc = i / (KW * AT_TAPS), j = i - cc * KW * AT_TAPS, k = j / AT_TAPS, t = j - k * AT_TAPS;
     if (k0 + k >= Kc) continue;
     float sum = 0.f;
 #pragma unroll
-    for (int wv = 0; wv < 4; ++wv) sum += sm.red[(cc * 4 + wv) * KW * AT_TAPS + j];
-    dst[(((size_t)(k0 + k) * 2 + cc) * AT_TAPS + t) * rows] = sum;
+    for (int wv = 0; wv < WG_GROUPS; ++wv) sum += sm.red[(cc * WG_GROUPS + wv) * KW * AT_TAPS + j];
+    dst[(((size_t)(k0 + k) * 2 + cc) * AT_TAPS + t) * n_rows] = sum;
   }
 }
 
@@ -1024,7 +1184,8 @@ struct WeightStage {
   cudaEvent_t done[AT_MAX_DEVICES] = {nullptr};
   cudaStream_t last[AT_MAX_DEVICES] = {nullptr};
   bool used[AT_MAX_DEVICES] = {false};
-  void* address[AT_MAX_DEVICES] = {nullptr};   // of c_att_weights
+  void* constant[AT_MAX_DEVICES] = {nullptr};   // addresses of c_att_weights and g_att_weights
+  void* ordered[AT_MAX_DEVICES] = {nullptr};
 } g_stage;
 
 class StagedWeights {
@@ -1034,14 +1195,22 @@ class StagedWeights {
     if (err_ == cudaSuccess && (dev_ < 0 || dev_ >= AT_MAX_DEVICES)) err_ = cudaErrorInvalidDevice;
     if (err_ != cudaSuccess) return;
     if (g_stage.done[dev_] == nullptr) err_ = cudaEventCreateWithFlags(&g_stage.done[dev_], cudaEventDisableTiming);
-    if (err_ == cudaSuccess && g_stage.address[dev_] == nullptr) err_ = cudaGetSymbolAddress(&g_stage.address[dev_], c_att_weights);
+    if (err_ == cudaSuccess && g_stage.ordered[dev_] == nullptr) {
+      err_ = cudaGetSymbolAddress(&g_stage.constant[dev_], c_att_weights);
+      if (err_ == cudaSuccess) err_ = cudaGetSymbolAddress(&g_stage.ordered[dev_], g_att_weights);
+    }
     if (err_ == cudaSuccess && g_stage.used[dev_] && g_stage.last[dev_] != st_)
       err_ = cudaStreamWaitEvent(st_, g_stage.done[dev_], 0);
   }
-  cudaError_t put(const float* device_weights, int channels, int module = 0) {  // weights of `channels` <= AT_KC channels
+  // Weights of channels k0 .. k0 + channels - 1 (at most AT_KC) of both modules.
+  cudaError_t put(const AttentionModules& modules, int k0, int channels, bool input_grad) {
     if (err_ != cudaSuccess) return err_;
-    err_ = cudaMemcpyAsync(static_cast<float*>(g_stage.address[dev_]) + module * AT_WEIGHTS, device_weights,
-                           (size_t)channels * 2 * AT_TAPS * sizeof(float), cudaMemcpyDeviceToDevice, st_);
+    StageWeights s{{nullptr, nullptr}, channels, input_grad};
+    for (int m = 0; m < 2; ++m)
+      if (modules.weight[m] != nullptr) s.weight[m] = modules.weight[m] + (size_t)k0 * 2 * AT_TAPS;
+    stage_weights_kernel<<<2, AT_KC * 2 * AT_TAPS, 0, st_>>>(s);
+    err_ = cudaGetLastError();
+    if (err_ == cudaSuccess) err_ = cudaMemcpyAsync(g_stage.constant[dev_], g_stage.ordered[dev_], sizeof(c_att_weights), cudaMemcpyDeviceToDevice, st_);
     return err_;
   }
   ~StagedWeights() {
@@ -1063,30 +1232,73 @@ class StagedWeights {
 // ---- launchers ---------------------------------------------------------------------------------------
 static dim3 pixel_grid(const AttentionDims& d) { return dim3((d.H1 * d.W1 + AT_THREADS - 1) / AT_THREADS, d.B); }
 
-static size_t tile_count(const AttentionDims& d) {
-  return (size_t)((d.W1 + AT_TW - 1) / AT_TW) * ((d.H1 + AT_TH - 1) / AT_TH);
-}
-// Displacements per block of a stencil walk: enough blocks (AT_BLOCKS_TARGET) to fill the 148 SMs several times over,
+static size_t tile_count(const AttentionDims& d, int rows) { return (size_t)((d.W1 + AT_TW - 1) / AT_TW) * ((d.H1 + rows - 1) / rows); }
+// Blocks of a job whose walks are not cut, in the tiled form and in the gather form (callers without a status word).
+static size_t form_blocks(const AttentionDims& d, bool tiled) { return (tiled ? tile_count(d, AT_TILE_ROWS) : (size_t)pixel_grid(d).x) * d.B; }
+// Displacements per block of a walk of the gather form: enough blocks (AT_BLOCKS_TARGET) to fill the 148 SMs several times over,
 // but at least AT_MIN_WALK displacements, because every block also reads a plane on either side of its own.
 // The weight gradients pay for a reduction over the block at the end of a walk as well and keep one or two blocks on an
 // SM, hence fewer and longer pieces.
 constexpr int AT_BLOCKS_TARGET = 148 * 8, AT_MIN_WALK = 8;
 constexpr int WG_BLOCKS_TARGET = 148 * 3, WG_MIN_WALK = 16;
-// The jobs of a launch fill the SMs together, with walks of about the same length: `total` is the sum of their D.  (Every job with as
-// many pieces as if it were the only one of its size, 1 x 55 x 128 with four levels and channels spent the last half of its logits on a few
-// long walks: 56 us, 50 now.)
-static int walk_length(size_t blocks, int D, int total, int target = AT_BLOCKS_TARGET, int min_walk = AT_MIN_WALK) {
+static int even_walk(int D, int dc) {   // the walks of a column of D, cut into pieces of at most dc
+  const int pieces = (D + dc - 1) / dc;
+  return (D + pieces - 1) / pieces;
+}
+static int gather_walk(size_t blocks, int D, int total, int target = AT_BLOCKS_TARGET, int min_walk = AT_MIN_WALK) {
   const int pieces = (int)((target + blocks - 1) / blocks);   // of all jobs
-  const int dc = std::max((total + pieces - 1) / pieces, min_walk), own = (D + dc - 1) / dc;
-  return (D + own - 1) / own;
+  return even_walk(D, std::max((total + pieces - 1) / pieces, min_walk));
 }
-// Displacements per block of the weight gradients' walk, and the blocks of a job (partial sums of a weight).
-static int weight_walk(const AttentionDims& d, int total, bool tiled) {
-  return walk_length((tiled ? tile_count(d) : 2 * (size_t)pixel_grid(d).x) * d.B, d.D, total, WG_BLOCKS_TARGET, WG_MIN_WALK);
+// Longest piece of the tiled walks, for all jobs of a launch (same blocks, columns of D[0 .. n-1]), on `slots` blocks at a time.  Pieces are cut
+// so that all of them make one round of the slots, or two, ...: with k rounds a launch takes between the work of a slot and k times its longest
+// piece.  A piece costs `extra` planes beside its own: the planes on either side of it, whose values it needs in part, its start and end.
+static int tiled_walk(size_t blocks, const int* D, int n, int slots, double extra) {
+  int most = 1, total = 0;
+  for (int i = 0; i < n; ++i) {
+    most = std::max(most, D[i]);
+    total += D[i];
+  }
+  auto pieces = [&](int dc) {
+    double count = 0;
+    for (int i = 0; i < n; ++i) count += (D[i] + dc - 1) / dc;
+    return count * blocks;
+  };
+  double best = 0;
+  int walk = most;
+  for (int rounds = 1; rounds <= 8; ++rounds) {
+    const double room = (double)rounds * slots;
+    int dc = std::max(1, (int)((double)blocks * total / room));
+    while (dc < most && pieces(dc) > room) dc += 1 + dc / 16;
+    dc = even_walk(most, std::min(dc, most));
+    const double count = pieces(dc), work = ((double)blocks * total + count * extra) / slots;
+    const double cost = 0.5 * (work + std::max(work, std::ceil(count / slots) * (dc + extra)));
+    if (best == 0 || cost < 0.98 * best) {
+      best = cost;
+      walk = dc;
+    }
+  }
+  return walk;
 }
-static size_t weight_rows(const AttentionDims& d, int total, bool tiled) {
-  const int dc = weight_walk(d, total, tiled);
-  return (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * ((d.D + dc - 1) / dc);
+// Blocks on an SM of the tiled kernels (registers), and what a piece costs beside its planes.
+constexpr double AT_PIECE_EXTRA = 3.0, WG_PIECE_EXTRA = 8.0;
+constexpr int WG_SLOTS = 3 * SM_COUNT;
+// Displacements per block of the weight gradients' walks, and the blocks of a job (partial sums of a weight).
+struct WeightWalks {
+  int dc[MAX_ATTENTION_JOBS];
+  size_t rows[MAX_ATTENTION_JOBS];
+};
+static WeightWalks weight_walks(const AttentionDims* d, int count, bool tiled) {
+  WeightWalks r{};
+  int D[MAX_ATTENTION_JOBS], total = 0;
+  for (int i = 0; i < count; ++i) total += D[i] = d[i].D;
+  const size_t blocks = tiled ? tile_count(d[0], WG_TILE_ROWS) * d[0].B : form_blocks(d[0], false);
+  const int chunks = (d[0].Kc + wg_channels(d[0].Kc) - 1) / wg_channels(d[0].Kc);
+  const int walk = tiled ? tiled_walk(blocks * chunks, D, count, WG_SLOTS, WG_PIECE_EXTRA) : 0;
+  for (int i = 0; i < count; ++i) {
+    r.dc[i] = tiled ? even_walk(D[i], walk) : gather_walk(2 * blocks, D[i], total, WG_BLOCKS_TARGET, WG_MIN_WALK);
+    r.rows[i] = blocks * ((D[i] + r.dc[i] - 1) / r.dc[i]);
+  }
+  return r;
 }
 // The softmax backward: pixels of a block by the length of the column (attention_logit_grad_kernel).
 static int logit_grad_pixels(int D) { return D <= 8 ? lg_pixels(1) : D <= 16 ? lg_pixels(2) : D <= 32 ? lg_pixels(4) : 32; }
@@ -1095,10 +1307,8 @@ static size_t bias_rows(const AttentionDims& d) { return (size_t)d.B * ((d.H1 * 
 // Bias partials per block of the softmax backward, weight partials per block of the weight gradients, whichever form they take.
 size_t attention_partial_floats(const AttentionDims* d, int count) {
   size_t floats = 0;
-  int total = 0;
-  for (int i = 0; i < count; ++i) total += d[i].D;
-  for (int i = 0; i < count; ++i)
-    floats += d[i].Kc * (bias_rows(d[i]) + 2 * AT_TAPS * std::max(weight_rows(d[i], total, true), weight_rows(d[i], total, false)));
+  const WeightWalks tiled = weight_walks(d, count, true), gather = weight_walks(d, count, false);
+  for (int i = 0; i < count; ++i) floats += d[i].Kc * (bias_rows(d[i]) + 2 * AT_TAPS * std::max(tiled.rows[i], gather.rows[i]));
   return floats;
 }
 
@@ -1141,34 +1351,55 @@ static cudaError_t launch_softmax(const AttentionJob* job, int count, cudaStream
   return launch_softmax_class<0>(job, count, 32, INT_MAX, st);
 }
 
+// Displacements per block of the walks of a launch (logits or input gradients).  A column short enough for the walks to end with its softmax is
+// not cut by launches that have two blocks per SM without it.
+struct Walks {
+  int dc[MAX_ATTENTION_JOBS];
+  bool soft;   // all columns end with their softmax
+};
 template <class Job>
-static int total_D(const Job* job, int count) {
-  int total = 0;
-  for (int i = 0; i < count; ++i) total += job[i].d.D;
-  return total;
+static Walks stencil_walks(const Job* job, int count, bool tiled, int blocks_per_sm, bool with_softmax) {
+  Walks r{};
+  int D[MAX_ATTENTION_JOBS], total = 0;
+  for (int i = 0; i < count; ++i) total += D[i] = job[i].d.D;
+  const size_t blocks = form_blocks(job[0].d, tiled);
+  const int walk = tiled ? tiled_walk(blocks, D, count, blocks_per_sm * SM_COUNT, AT_PIECE_EXTRA) : 0;
+  r.soft = with_softmax;
+  for (int i = 0; i < count; ++i) {
+    const bool whole = with_softmax && D[i] <= AT_SOFT_MAX && blocks * count >= 2 * SM_COUNT;
+    r.dc[i] = whole ? D[i] : (tiled ? even_walk(D[i], walk) : gather_walk(blocks, D[i], total));
+    r.soft = r.soft && D[i] <= AT_SOFT_MAX && r.dc[i] == D[i];
+  }
+  return r;
 }
-// Displacements per block of the forward's walk, and whether the walks of a launch end with the softmax of their columns.  A column
-// short enough for that is not cut by launches that have two blocks per SM without it.
-static int forward_walk(const AttentionDims& d, int jobs, int total, bool tiled) {
-  const size_t blocks = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
-  return d.D <= AT_SOFT_MAX && blocks * jobs >= 2 * SM_COUNT ? d.D : walk_length(blocks, d.D, total);
+// The order of a launch's jobs: the longest pieces first, so that the short ones fill the end.
+static void by_length(const Walks& walks, int count, int* order) {
+  for (int i = 0; i < count; ++i) {
+    int at = i;
+    for (; at > 0 && walks.dc[order[at - 1]] < walks.dc[i]; --at) order[at] = order[at - 1];
+    order[at] = i;
+  }
 }
-static bool softmax_in_walk(const AttentionJob* job, int count, bool tiled) {
-  const int total = total_D(job, count);
-  for (int i = 0; i < count; ++i)
-    if (job[i].d.D > AT_SOFT_MAX || forward_walk(job[i].d, count, total, tiled) < job[i].d.D) return false;
-  return true;
+// Blocks of the tiled walks on an SM (registers).
+static int logits_per_sm(int Kc) { return Kc >= 3 ? 4 : 6; }
+static int input_grad_per_sm(int Kc) { return Kc >= 3 ? 3 : 5; }
+static bool logits_by_tma(const AttentionJob* job, int count) {
+  bool tma = true;
+  for (int i = 0; i < count; ++i) tma = tma && tileable(job[i].d, job[i].x, job[i].x_sb);
+  return tma;
 }
-static bool all_tileable(const AttentionJob* job, int count, const int* status) {
-  bool ok = status != nullptr;
-  for (int i = 0; i < count; ++i) ok = ok && tileable(job[i].d, job[i].x, job[i].x_sb);
-  return ok;
+// f(integral constant) of a number of channels
+template <class F>
+static void by_channels(int kc, F&& f) {
+  if (kc == 1) f(std::integral_constant<int, 1>{});
+  else if (kc == 2) f(std::integral_constant<int, 2>{});
+  else if (kc == 3) f(std::integral_constant<int, 3>{});
+  else f(std::integral_constant<int, 4>{});
 }
 
 int attention_forward_launches(const AttentionJob* job, int count, const int* status) {
-  const bool tiled = all_tileable(job, count, status);
-  int n = (job[0].d.Kc + AT_KC - 1) / AT_KC;
-  if (softmax_in_walk(job, count, tiled)) return n;
+  int n = 2 * ((job[0].d.Kc + AT_KC - 1) / AT_KC);   // the weights' staging and the walks per chunk of channels
+  if (stencil_walks(job, count, status != nullptr, logits_per_sm(job[0].d.Kc), true).soft) return n;
   for (int i = 0; i < count; ++i) {
     bool first = true;   // of its class of lengths
     for (int k = 0; k < i; ++k) first = first && softmax_class(job[k].d.D) != softmax_class(job[i].d.D);
@@ -1180,22 +1411,25 @@ int attention_forward_launches(const AttentionJob* job, int count, const int* st
 cudaError_t launch_attention_forward(const AttentionJob* job, int count, const AttentionModules& modules, cudaStream_t st, int* status) {
   if (count < 1 || count > MAX_ATTENTION_JOBS) return cudaErrorInvalidValue;
   const AttentionDims& d = job[0].d;
-  const bool tiled = all_tileable(job, count, status);
-  const bool soft = softmax_in_walk(job, count, tiled);
+  const bool tiled = status != nullptr, tma = tiled && logits_by_tma(job, count);
+  const Walks walks = stencil_walks(job, count, tiled, logits_per_sm(d.Kc), true);
+  const bool soft = walks.soft;
+  int order[MAX_ATTENTION_JOBS];
+  by_length(walks, count, order);
   TileMaps maps;
   LogitsJobs jobs{};
   unsigned long long blocks = 0;
   for (int i = 0; i < MAX_ATTENTION_JOBS; ++i) {
     jobs.blocks.first[i] = (int)blocks;
     if (i >= count) continue;
-    const AttentionJob& j = job[i];
-    if (tiled) {
-      cudaError_t err = tile_map(&maps.m[i], j.x, j.x_sb, 2, 2, j.d, true);
+    const AttentionJob& j = job[order[i]];
+    if (tma) {
+      cudaError_t err = tile_map(&maps.m[i], j.x, j.x_sb, 2, 2, j.d, AT_TILE_ROWS, true);
       if (err != cudaSuccess) return err;
     }
-    const int dc = forward_walk(j.d, count, total_D(job, count), tiled);
+    const int dc = walks.dc[order[i]];
     jobs.j[i] = LogitsJobs::Job{j.x, j.x_sb, modules.bias[j.module], j.a, j.d.D, dc, j.module};
-    blocks += (unsigned long long)(tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B * ((j.d.D + dc - 1) / dc);
+    blocks += (unsigned long long)form_blocks(d, tiled) * ((j.d.D + dc - 1) / dc);
     if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
   }
   jobs.blocks.first[MAX_ATTENTION_JOBS] = (int)blocks;
@@ -1203,25 +1437,23 @@ cudaError_t launch_attention_forward(const AttentionJob* job, int count, const A
     StagedWeights staged(st);
     for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
       const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC;
-      for (int m = 0; m < 2; ++m) {
-        if (modules.weight[m] == nullptr) continue;
-        cudaError_t err = staged.put(modules.weight[m] + (size_t)k0 * 2 * AT_TAPS, kc, m);
-        if (err != cudaSuccess) return err;
-      }
-      if (tiled) {
-#define SFB_AT_FWD_T(KC) (soft ? attention_logits_tiled_kernel<KC, true> : attention_logits_tiled_kernel<KC, false>)<<<(unsigned)blocks, AT_THREADS + 32, 0, st>>>(maps, jobs, d.Kc, k0, d.B, d.H1, d.W1, status)
-        if (kc == 1) SFB_AT_FWD_T(1); else if (kc == 2) SFB_AT_FWD_T(2); else if (kc == 3) SFB_AT_FWD_T(3); else SFB_AT_FWD_T(4);
-#undef SFB_AT_FWD_T
-        continue;
-      }
-#define SFB_AT_FWD(KC) (soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>)<<<(unsigned)blocks, AT_THREADS, 0, st>>>(jobs, d.Kc, k0, d.B, d.H1, d.W1)
-      if (kc == 1) SFB_AT_FWD(1); else if (kc == 2) SFB_AT_FWD(2); else if (kc == 3) SFB_AT_FWD(3); else SFB_AT_FWD(4);
-#undef SFB_AT_FWD
+      cudaError_t err = staged.put(modules, k0, kc, false);
+      if (err != cudaSuccess) return err;
+      by_channels(kc, [&](auto c) {
+        constexpr int KC = decltype(c)::value;
+        if (!tiled) {
+          (soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>)<<<(unsigned)blocks, AT_THREADS, 0, st>>>(
+              jobs, d.Kc, k0, d.B, d.H1, d.W1);
+          return;
+        }
+        auto kernel = tma ? (soft ? attention_logits_tiled_kernel<KC, true, FEED_TMA> : attention_logits_tiled_kernel<KC, false, FEED_TMA>)
+                          : (soft ? attention_logits_tiled_kernel<KC, true, FEED_COPIES> : attention_logits_tiled_kernel<KC, false, FEED_COPIES>);
+        kernel<<<(unsigned)blocks, AT_THREADS, 0, st>>>(maps, jobs, d.Kc, k0, d.B, d.H1, d.W1, status);
+      });
+      if ((err = cudaGetLastError()) != cudaSuccess) return err;
     }
   }
-  cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess || soft) return err;
-  return launch_softmax(job, count, st);
+  return soft ? cudaSuccess : launch_softmax(job, count, st);
 }
 
 template <int KC>
@@ -1283,7 +1515,7 @@ static cudaError_t launch_logit_grad(const AttentionGradJob* job, const PartialP
 }
 
 int attention_backward_launches(const AttentionGradJob* job, int count) {
-  int n = (job[0].d.Kc + AT_KC - 1) / AT_KC + 2;   // input gradients per chunk of channels, weight gradients, the reduction
+  int n = 2 * ((job[0].d.Kc + AT_KC - 1) / AT_KC) + 2;   // staging and input gradients per chunk of channels, weight gradients, the reduction
   for (int i = 0; i < count; ++i) {
     bool first = true;   // of its class of lengths
     for (int k = 0; k < i; ++k) first = first && logit_grad_class(job[k].d.D) != logit_grad_class(job[i].d.D);
@@ -1296,10 +1528,14 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
                                       const AttentionGradients& grads, float* partial, cudaStream_t st, int* status) {
   if (count < 1 || count > MAX_ATTENTION_JOBS) return cudaErrorInvalidValue;
   const AttentionDims& d = job[0].d;
-  const int N1 = d.H1 * d.W1, total = total_D(job, count);
+  const int N1 = d.H1 * d.W1;
   auto g_sb = [&](const AttentionGradJob& j) { return (long long)d.Kc * j.d.D * N1; };
-  bool tiled = status != nullptr;
-  for (int i = 0; i < count; ++i) tiled = tiled && tileable(job[i].d, job[i].x, job[i].x_sb) && tileable(job[i].d, job[i].g, g_sb(job[i]));
+  const bool tiled = status != nullptr;
+  bool tma = tiled;
+  for (int i = 0; i < count; ++i) tma = tma && tileable(job[i].d, job[i].x, job[i].x_sb) && tileable(job[i].d, job[i].g, g_sb(job[i]));
+  AttentionDims dims[MAX_ATTENTION_JOBS];
+  for (int i = 0; i < count; ++i) dims[i] = job[i].d;
+  const WeightWalks weights = weight_walks(dims, count, tiled);
 
   // partial sums: per module the bias partials (Kc, rows), then the weight partials (Kc * 54, rows)
   PartialPlace place[MAX_ATTENTION_JOBS];
@@ -1312,7 +1548,7 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
       place[i].bias_row0 = brows;
       place[i].weight_row0 = wrows;
       brows += (int)bias_rows(job[i].d);
-      wrows += (int)weight_rows(job[i].d, total, tiled);
+      wrows += (int)weights.rows[i];
     }
     float *const bias = partial, *const weight = bias + (size_t)brows * d.Kc;
     partial = weight + (size_t)wrows * d.Kc * 2 * AT_TAPS;
@@ -1334,69 +1570,71 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
   cudaError_t err = launch_logit_grad(job, place, count, st);
   if (err != cudaSuccess) return err;
   {
+    const Walks walks = stencil_walks(job, count, tiled, input_grad_per_sm(d.Kc), false);
+    int order[MAX_ATTENTION_JOBS];
+    by_length(walks, count, order);
     InputGradJobs jobs{};
     unsigned long long blocks = 0;
     for (int i = 0; i <= MAX_ATTENTION_JOBS; ++i) {
       jobs.blocks.first[i] = (int)blocks;
       if (i >= count) continue;
-      const size_t tiles = (tiled ? tile_count(d) : (size_t)pixel_grid(d).x) * d.B;
-      const int dc = walk_length(tiles, job[i].d.D, total);
-      jobs.j[i] = InputGradJobs::Job{job[i].g, job[i].add, job[i].add_sb, job[i].gx, job[i].d.D, dc, job[i].module};
-      blocks += (unsigned long long)tiles * ((job[i].d.D + dc - 1) / dc);
+      const AttentionGradJob& j = job[order[i]];
+      const int dc = walks.dc[order[i]];
+      jobs.j[i] = InputGradJobs::Job{j.g, j.add, j.add_sb, j.gx, j.d.D, dc, j.module};
+      blocks += (unsigned long long)form_blocks(d, tiled) * ((j.d.D + dc - 1) / dc);
       if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
     }
     StagedWeights staged(st);
     for (int k0 = 0; k0 < d.Kc; k0 += AT_KC) {
       const int kc = d.Kc - k0 < AT_KC ? d.Kc - k0 : AT_KC, accumulate = k0 == 0 ? 0 : 1;
-      for (int m = 0; m < 2; ++m) {
-        if (modules.weight[m] == nullptr) continue;
-        err = staged.put(modules.weight[m] + (size_t)k0 * 2 * AT_TAPS, kc, m);
-        if (err != cudaSuccess) return err;
-      }
-      if (tiled) {
-        TileMaps maps;
+      if ((err = staged.put(modules, k0, kc, true)) != cudaSuccess) return err;
+      TileMaps maps;
+      if (tma) {
         for (int i = 0; i < count; ++i) {
-          err = tile_map(&maps.m[i], job[i].g, g_sb(job[i]), d.Kc, kc, job[i].d, true);
+          const AttentionGradJob& j = job[order[i]];
+          err = tile_map(&maps.m[i], j.g, g_sb(j), d.Kc, kc, j.d, AT_TILE_ROWS, true);
           if (err != cudaSuccess) return err;
         }
-#define SFB_AT_IG_T(KC) attention_input_grad_tiled_kernel<KC><<<(unsigned)blocks, AT_THREADS + 32, 0, st>>>(maps, jobs, accumulate, k0, d.B, d.H1, d.W1, status)
-        if (kc == 1) SFB_AT_IG_T(1); else if (kc == 2) SFB_AT_IG_T(2); else if (kc == 3) SFB_AT_IG_T(3); else SFB_AT_IG_T(4);
-#undef SFB_AT_IG_T
-        continue;
       }
-      if (kc == 1) err = launch_input_grad<1>((unsigned)blocks, jobs, accumulate, d, k0, st);
-      else if (kc == 2) err = launch_input_grad<2>((unsigned)blocks, jobs, accumulate, d, k0, st);
-      else if (kc == 3) err = launch_input_grad<3>((unsigned)blocks, jobs, accumulate, d, k0, st);
-      else err = launch_input_grad<4>((unsigned)blocks, jobs, accumulate, d, k0, st);
+      by_channels(kc, [&](auto c) {
+        constexpr int KC = decltype(c)::value;
+        if (!tiled) {
+          err = launch_input_grad<KC>((unsigned)blocks, jobs, accumulate, d, k0, st);
+          return;
+        }
+        (tma ? attention_input_grad_tiled_kernel<KC, FEED_TMA> : attention_input_grad_tiled_kernel<KC, FEED_COPIES>)
+            <<<(unsigned)blocks, AT_THREADS, 0, st>>>(maps, jobs, accumulate, d.Kc, k0, d.B, d.H1, d.W1, status);
+        err = cudaGetLastError();
+      });
       if (err != cudaSuccess) return err;
     }
   }
-  const int kw = d.Kc >= 4 ? 4 : d.Kc, chunks = (d.Kc + kw - 1) / kw;
+  const int kw = tiled ? wg_channels(d.Kc) : std::min(d.Kc, 4), chunks = (d.Kc + kw - 1) / kw;
   WeightGradJobs jobs{};
   unsigned long long blocks = 0;
   TileMaps maps_x, maps_gl;
   for (int i = 0; i <= MAX_ATTENTION_JOBS; ++i) {
     jobs.blocks.first[i] = (int)blocks;
     if (i >= count) continue;
-    jobs.j[i] = WeightGradJobs::Job{job[i].x, job[i].x_sb, job[i].g, place[i].weight, job[i].d.D, weight_walk(job[i].d, total, tiled),
+    jobs.j[i] = WeightGradJobs::Job{job[i].x, job[i].x_sb, job[i].g, place[i].weight, job[i].d.D, weights.dc[i],
                                     place[i].weight_row0, place[i].weight_rows};
-    blocks += weight_rows(job[i].d, total, tiled);
+    blocks += weights.rows[i];
     if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-    if (tiled) {
-      err = tile_map(&maps_x.m[i], job[i].x, job[i].x_sb, 2, 2, job[i].d, true);
-      if (err == cudaSuccess) err = tile_map(&maps_gl.m[i], job[i].g, g_sb(job[i]), d.Kc, kw, job[i].d, false);
+    if (tma) {
+      err = tile_map(&maps_x.m[i], job[i].x, job[i].x_sb, 2, 2, job[i].d, WG_TILE_ROWS, true);
+      if (err == cudaSuccess) err = tile_map(&maps_gl.m[i], job[i].g, g_sb(job[i]), d.Kc, kw, job[i].d, WG_TILE_ROWS, false);
       if (err != cudaSuccess) return err;
     }
   }
-  if (tiled) {
-#define SFB_AT_WG_T(KW) attention_weight_grad_tiled_kernel<KW><<<dim3((unsigned)blocks, chunks), WG_WARPS * 32 + 32, 0, st>>>(maps_x, maps_gl, jobs, d.Kc, d.B, d.H1, d.W1, status)
-    if (kw == 1) SFB_AT_WG_T(1); else if (kw == 2) SFB_AT_WG_T(2); else if (kw == 3) SFB_AT_WG_T(3); else SFB_AT_WG_T(4);
-#undef SFB_AT_WG_T
-  } else {
-#define SFB_AT_WG(KW) attention_weight_grad_kernel<KW><<<dim3((unsigned)blocks, 2 * chunks), AT_THREADS, 0, st>>>(jobs, d.Kc, d.B, d.H1, d.W1)
-    if (kw == 1) SFB_AT_WG(1); else if (kw == 2) SFB_AT_WG(2); else if (kw == 3) SFB_AT_WG(3); else SFB_AT_WG(4);
-#undef SFB_AT_WG
-  }
+  by_channels(kw, [&](auto c) {
+    constexpr int KW = decltype(c)::value;
+    if (!tiled) {
+      attention_weight_grad_kernel<KW><<<dim3((unsigned)blocks, 2 * chunks), AT_THREADS, 0, st>>>(jobs, d.Kc, d.B, d.H1, d.W1);
+    } else if constexpr (KW <= WG_MAX_CHANNELS) {
+      (tma ? attention_weight_grad_tiled_kernel<KW, FEED_TMA> : attention_weight_grad_tiled_kernel<KW, FEED_COPIES>)
+          <<<dim3((unsigned)blocks, chunks), wg_threads(tma ? FEED_TMA : FEED_COPIES), 0, st>>>(maps_x, maps_gl, jobs, d.Kc, d.B, d.H1, d.W1, status);
+    }
+  });
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
   attention_reduce_partials_kernel<<<columns, RP_THREADS, 0, st>>>(sums);
   return cudaGetLastError();

@@ -389,9 +389,9 @@ struct AttentionJob {
   long long x_sb;
   float* a;
 };
-// `status` (optional): a device status word for bounded waits.  With it, and when W1 is a multiple of 4 and every x is
-// 16-byte aligned, the kernels fetch their pixel tiles (with the stencil's halo, zero-filled outside the image) by
-// TMA; otherwise every thread gathers its own neighbourhood.
+// `status` (optional): a device status word for bounded waits.  With it blocks work on pixel tiles in shared memory (with the
+// stencil's halo, zeros outside the image), fetched by TMA when W1 is a multiple of 4 and every x is 16-byte aligned, else
+// by copies; without it every thread gathers its own neighbourhood.
 [[nodiscard]] cudaError_t launch_attention_forward(const AttentionJob* jobs, int count, const AttentionModules& modules,
                                      cudaStream_t stream, int* status = nullptr);
 int attention_forward_launches(const AttentionJob* jobs, int count, const int* status);  // its kernels
