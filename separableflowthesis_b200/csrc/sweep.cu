@@ -66,10 +66,15 @@ constexpr uint32_t SW_TMEM_COLS = 512;
 // 64 KB (16-bit) five.
 constexpr int SW_MAX_STAGES = 6;
 constexpr uint32_t SW_RING_BYTES = MAX_KB * SW_F1_BLOCK_BYTES + 3 * SW_STAGE_BYTES;   // image-1 tile and ring together
-__device__ __forceinline__ uint32_t sw_stages(int nkb) {
-  const uint32_t n = (SW_RING_BYTES - nkb * SW_F1_BLOCK_BYTES) / SW_STAGE_BYTES;
+__device__ __forceinline__ uint32_t sw_stages(int nkb, uint32_t row_bytes) {
+  const uint32_t n = (SW_RING_BYTES - row_bytes - nkb * SW_F1_BLOCK_BYTES) / SW_STAGE_BYTES;
   return n < SW_MAX_STAGES ? n : SW_MAX_STAGES;
 }
+// Row sums on their way to memory (the compression with KC channels, TMA rows): behind the ring, two buffers per epilogue warp of the
+// rows x channels of 32 pixels that it has of a tile.
+__host__ __device__ constexpr int sw_channels(int KC) { return KC == 1 ? 1 : 2; }           // of a thread
+__host__ __device__ constexpr int sw_rows(int KC) { return KC <= 2 ? SWEEP_UT / 2 : SWEEP_UT; }   // with one or two channels the two groups share a tile's rows
+__host__ __device__ constexpr uint32_t sw_row_bytes(int KC) { return 2 * SW_EPI_WARPS * sw_rows(KC) * sw_channels(KC) * 32 * sizeof(float); }
 static_assert(SW_NACC * SW_TILE_N <= 512, "accumulators exceed TMEM");
 static_assert(SW_NMERGE > SW_NACC, "a warpgroup can run SW_NACC tiles ahead of the other");
 
@@ -142,11 +147,11 @@ __device__ __forceinline__ SweepSched sweep_sched(const SweepArgs& a, int block)
 // ---------------------------------------------------------------------------------- producer
 template <bool NARROW>
 __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const CUtensorMap* tm_f1,
-                               const CUtensorMap* tm_f2, const CUtensorMap* tm_aux) {
+                               const CUtensorMap* tm_f2, const CUtensorMap* tm_aux, uint32_t row_bytes) {
   const int kel = a.op16 ? 2 * KBLK : KBLK;  // channels in one 128-byte row
   mbar_expect_tx(&sm.f1_full, sc.nkb * SW_F1_BLOCK_BYTES);
   for (int kb = 0; kb < sc.nkb; ++kb) tma_load_3d(sm.f1(kb), tm_f1, &sm.f1_full, kb * kel, sc.m0, sc.b);
-  const uint32_t n_stages = sw_stages(sc.nkb);
+  const uint32_t n_stages = sw_stages(sc.nkb, row_bytes);
   uint32_t s = 0, ph = 0;
   int vb = sc.vb0, ub = 0;
   for (int t = 0; t < sc.t_total; ++t) {
@@ -166,13 +171,13 @@ __device__ void sweep_producer(SweepSmem& sm, const SweepArgs& a, const SweepSch
 }
 
 // ---------------------------------------------------------------------------------- MMA issuer
-__device__ void sweep_mma(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc) {
+__device__ void sweep_mma(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, uint32_t row_bytes) {
   constexpr uint32_t idesc_tf32 = make_idesc_tf32(TILE_M, SW_TILE_N, false, false);
   const uint32_t idesc_16 = make_idesc_op16(a.op16, TILE_M, SW_TILE_N);  // BF16 or FP16 operands
   const bool op16 = a.op16 != 0;
   if (!mbar_wait(&sm.f1_full, 0, &sm.ctl, a.status, DEV_TIMEOUT_MMA)) return;
   tc_fence_after();
-  const uint32_t n_stages = sw_stages(sc.nkb);
+  const uint32_t n_stages = sw_stages(sc.nkb, row_bytes);
   uint32_t s = 0, ph = 0;
   for (int t = 0; t < sc.t_total; ++t) {
     const uint32_t acc = t % SW_NACC, aph = (t / SW_NACC) & 1u;
@@ -473,6 +478,11 @@ __device__ __forceinline__ void fma2_tmem(uint64_t& acc, uint32_t lo, uint32_t h
   asm volatile("{\n\t.reg .b64 s;\n\tmov.b64 s, {%1, %2};\n\tfma.rn.f32x2 %0, s, %3, %0;\n\t}" : "+l"(acc) : "r"(lo), "r"(hi), "l"(w));
 }
 
+// Where the row sums of a level go by TMA: the output, and the scratch of later pieces.  (pixel, displacement, channel, sample or part)
+struct RowMaps {
+  CUtensorMap out, part;
+};
+
 // Compression sums.  A thread does CPT channels of its pixel.  With three or four channels the two groups take two each and read
 // whole tiles; with one or two (SPLIT) both do all of them and share a tile's rows, and the column sums of a block are put
 // together at its end.
@@ -489,8 +499,10 @@ __device__ __forceinline__ void fma2_tmem(uint64_t& acc, uint32_t lo, uint32_t h
 // sums are not moved around at every tile (450 of 1860 instructions per warp and tile were moves); the row weights of the
 // next tile are asked for before the wait for this one.  135 x 240, one pair, four channels: 897 -> 717 us (8 pairs, two
 // sweeps: 14.2 -> 10.9 ms); 8 x 47 x 156, two channels: 337 -> 290 us.
-template <int CPT, bool SPLIT, bool CUT, bool NARROW>
-__device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e) {
+template <int KC, bool CUT, bool NARROW, bool TMA_ROWS>
+__device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const SweepSched& sc, const EpiCtx& e, const RowMaps* maps) {
+  constexpr int CPT = sw_channels(KC);
+  constexpr bool SPLIT = KC <= 2;
   using T = Tile<NARROW>;
   constexpr int VT = T::VT, HALVES = T::HALVES;
   constexpr int NR = SPLIT ? T::RW : T::UT;      // tile rows of this thread
@@ -517,6 +529,14 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
     part_step = (uint32_t)a.part_slots * H2 * TILE_M;
   }
   const int row0 = SPLIT ? e.wg * T::RW : 0;
+  // TMA_ROWS: a tile's row sums go to one of the warp's two buffers, from where a TMA store (first column block, and every one of a later
+  // piece) or add takes them to memory.  A buffer is used again, and a row added to again, when the copies of two tiles ago are complete
+  // (of one row block: of the tile before), so the sums of a row are added up in the order of its column blocks.  With red.global from the
+  // registers the sixteen of a warp and tile, their 64-bit addresses and conditions took an eighth of the launch (135 x 240, one pair, four
+  // levels and channels 965 -> 860 us, 4 x 55 x 128 228 -> 203; 8 x 47 x 156, one level, two channels, both sweeps 514 -> 487).
+  const int warp = e.wg * 4 + (e.p - e.lane - sc.m0) / 32;
+  float* const row_buffer = reinterpret_cast<float*>(sm.ring + SW_RING_BYTES - sw_row_bytes(KC)) + warp * (2 * NR * CPT * 32) + e.lane;
+  const bool later_piece = CUT && sc.piece > 0;
   float av[CPT][NR];   // w_v of the coming tile's rows (past the image: the last row's)
   auto load_av = [&](int u0) {
 #pragma unroll
@@ -557,7 +577,15 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         rows[c] = e.valid && c < n_ch ? nu : 0;
         dst[c] = ou + u0 * ousd + c * ouss;
       }
+      float* const to_rows = row_buffer + (t & 1) * (NR * CPT * 32);
       if (!epi_wait(sm, a, t)) return;
+      if constexpr (TMA_ROWS) {
+        if (e.lane == 0) {
+          if (sc.n_ub > 1) bulk_wait<1>();
+          else bulk_wait<0>();
+        }
+        __syncwarp();
+      }
       const uint32_t tacc = e.tbase + (t % SW_NACC) * SW_TILE_N + row0 * VT;
       uint32_t s[2][16];
       uint64_t r2[CPT];
@@ -581,12 +609,23 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
         if (h == HALVES - 1) {
 #pragma unroll
           for (int c = 0; c < CPT; ++c, dst[c - 1] += ousd) {
-            if (rows[c] > ul) {
+            if constexpr (TMA_ROWS) {
+              to_rows[(c * NR + ul) * 32] = sum2(r2[c]) * e.osc;
+            } else if (rows[c] > ul) {
               const float x = sum2(r2[c]) * e.osc;
               if (first) *dst[c] = x;
               else atomicAdd(dst[c], x);
             }
           }
+        }
+      }
+      if constexpr (TMA_ROWS) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (e.lane == 0 && e.valid && nu > 0) {
+          if (later_piece) tma_store_4d(&maps->part, to_rows, e.p - sc.m0, u0, k_first, sc.tail * a.parts + vb - sc.part_vb0);
+          else if (first) tma_store_4d(&maps->out, to_rows, e.p, u0, k, sc.b);
+          else tma_add_4d(&maps->out, to_rows, e.p, u0, k, sc.b);
         }
       }
     }
@@ -640,6 +679,7 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
       if (!(e.wg == 0 ? merge(std::integral_constant<int, 0>{}) : merge(std::integral_constant<int, 1>{}))) return;
     }
   }
+  if (TMA_ROWS && e.lane == 0) bulk_wait_all();
 }
 
 // Test aid: writes the dense volume of a (small) problem so the tensor-core plumbing can be checked alone.
@@ -679,6 +719,7 @@ __device__ void epilogue_dump(SweepSmem& sm, const SweepArgs& a, const SweepSche
 template <int LEVELS>
 struct SweepLaunch {
   CUtensorMap f1, f2[LEVELS], aux[LEVELS];
+  RowMaps rows[LEVELS];
   SweepArgs a[LEVELS];
   int first_block[LEVELS + 1], first_tail[LEVELS + 1];   // of the sweep and of the fold; levels that do not exist have none
 };
@@ -705,7 +746,8 @@ __device__ __forceinline__ void by_tile_form(const SweepArgs& a, F&& f) {
 // pixel tile beside 28), and the finest leaves SMs idle in its last wave, which their tiles fill.  Both sweeps of four levels with their
 // folds, levels one after the other and together (us, four channels, FP16): 1 x 55 x 128 172 and 134, 4 x 55 x 128 422 and 360,
 // 1 x 135 x 240 1675 and 1558.
-template <int MODE, bool CUT, int KC, int FORM, int LEVELS>
+// TMA_ROWS (compression): the row sums go to memory by TMA (wide tiles; narrow ones of a pyramid's levels do not).
+template <int MODE, bool CUT, int KC, int FORM, int LEVELS, bool TMA_ROWS>
 __global__ void __launch_bounds__(SW_THREADS, 1)
 sweep_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch, int* status) {
   if (!cta_has_work(status)) return;
@@ -750,15 +792,16 @@ sweep_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch, int* status) {
   };
   // The two kinds of warps do not meet in common code again: what follows here is compiled for SW_REGS_ISSUE registers, what
   // follows there for SW_REGS_EPI.
+  constexpr uint32_t row_bytes = TMA_ROWS ? sw_row_bytes(KC) : 0;
   if (warp < 4) {
     set_max_registers<SW_REGS_ISSUE, false>();
     by_tile_form<FORM>(a, [&](auto narrow) {
       constexpr bool NARROW = decltype(narrow)::value;
       const SweepSched sc = sweep_sched<MODE, CUT, NARROW>(a, block);
       if (warp == 0) {
-        if (lane == 0) sweep_producer<NARROW>(sm, a, sc, tm_f1, tm_f2, tm_aux);
+        if (lane == 0) sweep_producer<NARROW>(sm, a, sc, tm_f1, tm_f2, tm_aux, row_bytes);
       } else if (warp == 1) {
-        if (lane == 0) sweep_mma(sm, a, sc);
+        if (lane == 0) sweep_mma(sm, a, sc, row_bytes);
       }
     });
     __syncwarp();
@@ -783,7 +826,7 @@ sweep_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch, int* status) {
     e.osc = a.out_scale != nullptr ? __ldg(a.out_scale) : 1.f;
     if constexpr (MODE == SWEEP_MAXAVG) epilogue_maxavg<false, CUT, NARROW>(sm, a, sc, e);
     else if constexpr (MODE == SWEEP_MAXARGAVG) epilogue_maxavg<true, CUT, NARROW>(sm, a, sc, e);
-    else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC == 1 ? 1 : 2, KC <= 2, CUT, NARROW>(sm, a, sc, e);
+    else if constexpr (MODE == SWEEP_COMPRESS) epilogue_compress<KC, CUT, NARROW, TMA_ROWS && !NARROW>(sm, a, sc, e, &launch.rows[level]);
     else epilogue_dump<NARROW>(sm, a, sc, e);
   });
   __syncwarp();
@@ -903,9 +946,33 @@ void sweep_split_levels(const Dims* d, int levels, int slots, bool sums, TileSpl
   }
 }
 
-template <int MODE, bool CUT, int KC, int FORM, int LEVELS>
+// Maps of the row sums of a level.  Not all views have the alignment that a tensor map asks for (planes of a multiple of 4 pixels); and with
+// TF32 operands the image-1 tile leaves no room for the buffers beside a ring of three stages.
+static bool row_maps(const SweepArgs& a, int rows, int channels, RowMaps* maps, cudaError_t* err) {
+  const auto aligned = [](long long elements) { return elements % 4 == 0; };
+  if ((reinterpret_cast<uintptr_t>(a.ou.base) & 15u) != 0 || !aligned(a.ou.sb) || !aligned(a.ou.sd) || !aligned(a.ou.ss)) return false;
+  const uint32_t box[4] = {32, (uint32_t)rows, (uint32_t)channels, 1};
+  const uint64_t dims[4] = {(uint64_t)a.n_valid, (uint64_t)a.d.H2, (uint64_t)(a.k0 + a.kc), (uint64_t)a.d.B};
+  const uint64_t strides[3] = {a.ou.sd * 4ull, a.ou.ss * 4ull, (uint64_t)a.ou.sb * 4ull};
+  if ((*err = encode_plain_map(&maps->out, a.ou.base, 4, dims, strides, box)) != cudaSuccess) return false;
+  if (a.pieces == 1) return true;
+  const int tails = a.d.B * ((a.d.N1() + TILE_M - 1) / TILE_M) - a.whole_tiles;
+  const uint64_t part_dims[4] = {TILE_M, (uint64_t)a.d.H2, (uint64_t)a.part_slots, (uint64_t)tails * a.parts};
+  const uint64_t part_strides[3] = {TILE_M * 4ull, a.d.H2 * (TILE_M * 4ull), (uint64_t)a.part_slots * a.d.H2 * (TILE_M * 4ull)};
+  return (*err = encode_plain_map(&maps->part, a.part, 4, part_dims, part_strides, box)) == cudaSuccess;
+}
+
+template <int MODE, bool CUT, int KC, int FORM, int LEVELS, bool TMA_ROWS = false>
 static cudaError_t launch_one(SweepLaunch<LEVELS>& launch, int levels, cudaStream_t stream) {
-  auto kern = sweep_kernel<MODE, CUT, KC, FORM, LEVELS>;
+  if constexpr (MODE == SWEEP_COMPRESS && FORM != TILES_NARROW && !TMA_ROWS) {
+    bool tma = launch.a[0].op16 != 0;
+    cudaError_t err = cudaSuccess;
+    for (int l = 0; l < levels && tma; ++l)
+      tma = launch.a[l].narrow || row_maps(launch.a[l], sw_rows(KC), sw_channels(KC), &launch.rows[l], &err);
+    if (err != cudaSuccess) return err;
+    if (tma) return launch_one<MODE, CUT, KC, FORM, LEVELS, true>(launch, levels, stream);
+  }
+  auto kern = sweep_kernel<MODE, CUT, KC, FORM, LEVELS, TMA_ROWS>;
   static DeviceOnce configured;  // the attribute is per device and stays set
   cudaError_t err = configured.run([&] {
     // A kernel that was compiled for fewer registers than the split takes would wait in setmaxnreg.inc without a limit.
