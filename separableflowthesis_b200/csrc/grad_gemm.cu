@@ -141,15 +141,6 @@ struct GradSched {
 template <int Q>
 struct Slots {
   float f[4 * Q];
-  // global memory: group q of this pixel is `group_stride` floats after group q-1.  Loads of one float each: a 16-byte load
-  // would put the four slots of a column into neighbouring registers, and then a slot of all columns into the same register
-  // bank as their sums, which costs every other multiply-add a cycle (9.5 against 8.5 ms at 8 x 135 x 240).
-  __device__ __forceinline__ void load_global(const float* p, size_t group_stride, bool ok) {
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) f[4 * q + k] = ok ? __ldg(p + q * group_stride + k) : 0.f;
-  }
   // shared memory block [group][pixel][4]
   __device__ __forceinline__ void load_shared(const float* p, int group_stride) {
 #pragma unroll
@@ -159,6 +150,39 @@ struct Slots {
     }
   }
 };
+
+// The slots of N columns from column v0 on (p: of column 0, a column `column_stride` floats after the one before, group q
+// `group_stride` floats after group q-1); zero past column W - 1.  As 16-byte loads that are all under way before the first value is
+// used; with one load per value, and columns waiting for one another, a CTA took some 12,000 cycles for the slots of 16 columns (three groups, every 34
+// blocks at 8 x 135 x 240; 6,100 with two groups, every 12 blocks at 8 x 47 x 156), and every CTA asks for them at about the same time:
+// operand_producer brings them into L2 before that, which leaves 6,800 and 3,700.  The selection also moves every value to a register of
+// its own: a 16-byte load puts the four slots of a column into neighbouring registers, and then a slot of all columns lies in the same
+// register bank as their sums, which costs every other multiply-add a cycle.  Image-1-major GEMMs, 8 x 47 x 156 (BF16) 403 -> 383 us,
+// 3 x 47 x 155 (TF32) 333 -> 320, 8 x 135 x 240 within 2 %.
+template <int Q, int N>
+__device__ __forceinline__ void load_columns(Slots<Q> (&xv)[N], const float* p, size_t column_stride, size_t group_stride, int v0, int W) {
+  float4 raw[N][Q];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float* column = p + (size_t)min(v0 + i, W - 1) * column_stride;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const float4* src = reinterpret_cast<const float4*>(column + q * group_stride);
+      asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(raw[i][q].x), "=f"(raw[i][q].y), "=f"(raw[i][q].z), "=f"(raw[i][q].w) : "l"(src));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const bool ok = v0 + i < W;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      xv[i].f[4 * q] = ok ? raw[i][q].x : 0.f;
+      xv[i].f[4 * q + 1] = ok ? raw[i][q].y : 0.f;
+      xv[i].f[4 * q + 2] = ok ? raw[i][q].z : 0.f;
+      xv[i].f[4 * q + 3] = ok ? raw[i][q].w : 0.f;
+    }
+  }
+}
 
 // TF32 rounding of a value that goes straight to the tensor core: tcgen05.mma kind::tf32 ignores the low 13
 // mantissa bits, so adding half a TF32 ulp is all it takes (round_tf32 without the mask).
@@ -221,11 +245,7 @@ __device__ void generator_image1(GradSmem<Q, FORM>& sm, const GradArgs& a, const
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t so = t % Cfg::NXU, pho = (t / Cfg::NXU) & 1u;
     const int vbase = vb * GG_VT + vh * GG_VH;
-    if (ub2 == 0 || t == 0) {
-#pragma unroll
-      for (int i = 0; i < GG_VH; ++i)
-        xv[i].load_global(xv_p + (size_t)(vbase + i) * row_stride, group_stride, vbase + i < W2);
-    }
+    if (ub2 == 0 || t == 0) load_columns(xv, xv_p, row_stride, group_stride, vbase, W2);
     if (!mbar_wait_warp(&sm.xu_full[so], pho, &sm.ctl, a.status, DEV_TIMEOUT_GENERATOR)) return;
     float g[GG_UT][GG_VH];
 #pragma unroll
@@ -422,7 +442,11 @@ __device__ void operand_producer(GradSmem<Q, FORM>& sm, const GradArgs& a, const
   using Cfg = GradCfg<Q, FORM>;
   using Smem = GradSmem<Q, FORM>;
   constexpr int I2MAJOR = grad_is_image2(FORM) ? 1 : 0;
-  int ub2 = I2MAJOR == 0 ? sc.t0 % sc.n_ub2 : 0;
+  int vb = 0, ub2 = 0;
+  if (I2MAJOR == 0) { vb = sc.t0 / sc.n_ub2; ub2 = sc.t0 - vb * sc.n_ub2; }
+  const size_t xv_group = (size_t)a.n1p * 4;
+  const float* const xv_p = a.xv + (size_t)sc.b * a.d.W2 * Q * xv_group + (size_t)sc.m0 * 4;
+  const int ahead = min(sc.n_ub2, GG_VT), quiet = sc.n_ub2 - ahead;   // the last blocks of a column of blocks, and the ones before
   for (int t = 0; t < sc.n_blocks; ++t) {
     const uint32_t su = t % Cfg::NXU, phu = (t / Cfg::NXU) & 1u;
     if (!mbar_wait(&sm.xu_empty[su], phu ^ 1u, &sm.ctl, a.status, DEV_TIMEOUT_PRODUCER)) return;
@@ -430,7 +454,14 @@ __device__ void operand_producer(GradSmem<Q, FORM>& sm, const GradArgs& a, const
     if (I2MAJOR == 0) {
       tma_load_4d(sm.xu[su], tm_xu, &sm.xu_full[su], sc.m0 * 4, 0, ub2 * GG_UT, sc.b);
       tma_load_4d(sm.xu[su] + Smem::XU_FLOATS / 2, tm_xu, &sm.xu_full[su], (sc.m0 + 64) * 4, 0, ub2 * GG_UT, sc.b);
-      if (++ub2 == sc.n_ub2) ub2 = 0;
+      // The (pixel, v) slots of the next 16 columns, which all CTAs read at about the same time, are brought into L2 a few columns per block.
+      if (ub2 >= quiet) {
+        const int v0 = (vb + 1) * GG_VT + (ub2 - quiet) * GG_VT / ahead, v1 = min((vb + 1) * GG_VT + (ub2 - quiet + 1) * GG_VT / ahead, a.d.W2);
+        for (int v = v0; v < v1; ++v)
+#pragma unroll
+          for (int q = 0; q < Q; ++q) bulk_prefetch_l2(xv_p + ((size_t)v * Q + q) * xv_group, TILE_M * 16);
+      }
+      if (++ub2 == sc.n_ub2) { ub2 = 0; ++vb; }
     } else {
       tma_load_4d(sm.xu[su], tm_xu, &sm.xu_full[su], (sc.t0 + t) * GG_KJ * 4, 0, sc.u0, sc.b);
       const uint32_t sv = t % Cfg::NXV, phv = (t / Cfg::NXV) & 1u;

@@ -162,6 +162,10 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// Contiguous global bytes on their way into L2 (16-byte aligned, a multiple of 16 bytes).
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {   // a bulk group of its own
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(dst),
                "r"(smem_u32(src)), "r"(bytes)
