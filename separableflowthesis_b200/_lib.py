@@ -163,6 +163,22 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native module with the host side of the lookups (``pybind/host_module.cpp``), bound to the library's entry points."""
+    global _host
+    if _host is None:
+        from . import build
+        lib, module = load(), build.load_host_module()
+        module.bind(*[ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in (
+            "sfb_lookup_pyramid_bytes", "sfb_lookup_build_pyramid_pair", "sfb_lookup_forward_pair", "sfb_lookup_accumulator_bytes",
+            "sfb_lookup_accumulate_pair", "sfb_status_string", "sfb_last_error")])
+        _host = module
+    return _host
+
+
 def kernel_timing(enable: bool) -> None:
     """Start (True) or stop (False) a fresh per-kernel timing measurement."""
     load().sfb_kernel_timing_enable(1 if enable else 0)

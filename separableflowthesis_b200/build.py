@@ -57,43 +57,67 @@ PYBIND_SRC = os.path.join(PYBIND_DIR, "memorysaver_module.cpp")
 PYBIND_OUT = os.path.join(PYBIND_DIR, "MemorySaver.so")
 
 
-def build_pybind_module(force: bool = False) -> str:
-    """Compile ``pybind/memorysaver_module.cpp`` into ``pybind/MemorySaver.so``: a native Python module with the five
-    names of the reference's pybind11 module (libs/MemorySaver/src/MemorySaver_cuda.cpp:105-112) over the C ABI.
-    Host code only (g++ with torch's headers); it finds ``libsepflow_b200.so`` at import time."""
-    deps = [PYBIND_SRC, os.path.join(PKG_DIR, "..", "include", "sepflow_b200.h")]
-    if not force and os.path.exists(PYBIND_OUT) and all(os.path.getmtime(PYBIND_OUT) > os.path.getmtime(d) for d in deps):
-        return PYBIND_OUT
+HOST_SRC = os.path.join(PYBIND_DIR, "host_module.cpp")
+HOST_OUT = os.path.join(PYBIND_DIR, "sfb_host.so")
+
+
+def _build_extension(src: str, out: str, name: str, force: bool) -> str:
+    """Host code only (g++ with torch's headers)."""
+    deps = [src, os.path.join(PKG_DIR, "..", "include", "sepflow_b200.h")]
+    if not force and os.path.exists(out) and all(os.path.getmtime(out) > os.path.getmtime(d) for d in deps):
+        return out
     import sysconfig
     import torch
     from torch.utils import cpp_extension
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", "-DTORCH_EXTENSION_NAME=MemorySaver",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-DTORCH_EXTENSION_NAME={name}",
            "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     for inc in cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda_home, "include")]:
         cmd += ["-I", inc]
-    cmd += [PYBIND_SRC, "-o", PYBIND_OUT, "-L", lib_dir, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
+    cmd += [src, "-o", out, "-L", lib_dir, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
             "-L", os.path.join(cuda_home, "lib64"), "-lcudart", "-ldl", f"-Wl,-rpath,{lib_dir}"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError("building the MemorySaver module failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr[-4000:])
-    return PYBIND_OUT
+        raise RuntimeError(f"building the {name} module failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr[-4000:])
+    return out
 
 
-def load_pybind_module():
-    """Import ``pybind/MemorySaver.so`` as the module ``MemorySaver`` (what the reference imports from
-    ``libs/MemorySaver/build/lib``)."""
+def _load_extension(path: str, name: str):
     import importlib.util
     import torch  # noqa: F401  (the module links against libtorch)
-    if not os.path.exists(PYBIND_OUT):
-        raise RuntimeError(f"{PYBIND_OUT} is missing: build it with `python -m separableflowthesis_b200.build`")
-    spec = importlib.util.spec_from_file_location("MemorySaver", PYBIND_OUT)
+    if not os.path.exists(path):
+        raise RuntimeError(f"{path} is missing: build it with `python -m separableflowthesis_b200.build`")
+    spec = importlib.util.spec_from_file_location(name, path)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
     return mod
 
 
+def build_pybind_module(force: bool = False) -> str:
+    """Compile ``pybind/memorysaver_module.cpp`` into ``pybind/MemorySaver.so``: a native Python module with the five
+    names of the reference's pybind11 module (libs/MemorySaver/src/MemorySaver_cuda.cpp:105-112) over the C ABI.
+    It finds ``libsepflow_b200.so`` at import time."""
+    return _build_extension(PYBIND_SRC, PYBIND_OUT, "MemorySaver", force)
+
+
+def build_host_module(force: bool = False) -> str:
+    """Compile ``pybind/host_module.cpp`` into ``pybind/sfb_host.so``: the host side of the lookups on the aggregated volumes, which
+    the ops call (``_lib.host``)."""
+    return _build_extension(HOST_SRC, HOST_OUT, "sfb_host", force)
+
+
+def load_pybind_module():
+    """Import ``pybind/MemorySaver.so`` as the module ``MemorySaver`` (what the reference imports from
+    ``libs/MemorySaver/build/lib``)."""
+    return _load_extension(PYBIND_OUT, "MemorySaver")
+
+
+def load_host_module():
+    return _load_extension(HOST_OUT, "sfb_host")
+
+
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
     print(build_pybind_module(force="--force" in sys.argv))
+    print(build_host_module(force="--force" in sys.argv))

@@ -21,6 +21,7 @@ import math
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from .functions import (ComputeMaxArgmaxAvgFunction, ComputeMaxAvgFunction, ComputeSelfCompressionFunction,
                         FusedMaxArgmaxAvgFunction, FusedSelfCompressionFunction, SeparationCompressionCF,
@@ -179,6 +180,11 @@ class AlternateCorrBlockSepflow:
         return Lookup4dFunction.apply(coords.to(F1.dtype).contiguous(), self.radius, scale, F1, *F2_levels)
 
 
+def _transforms_active() -> bool:
+    """Whether torch.func transforms or forward-mode derivatives are: those are for the autograd Function to see (and to refuse)."""
+    return torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+
+
 class CorrBlock1D:
     """Lookup on the two aggregated 3D cost volumes: a drop-in for ``CorrBlock1D`` of the reference
     (core/corr.py:513-624).  corr1 (B,dim,W2,H1,W1) is read with the x component of the coordinates, corr2
@@ -224,6 +230,8 @@ class CorrBlock1D:
 
     def __call__(self, coords):
         chain = self._edges()
+        if chain is None and not (torch.is_grad_enabled() and coords.requires_grad) and not _transforms_active():
+            return _ops.lookup_forward_pair(self.corr1, self.corr2, self.pyramid1, self.pyramid2, coords, self.num_levels, self.radius)
         edges = chain[4:] if chain is not None else (None, None)
         out1, out2, *edges = LookupPairFunction.apply(self.corr1, self.corr2, self.pyramid1, self.pyramid2, coords, *edges,
                                                       self.num_levels, self.radius)

@@ -799,61 +799,15 @@ def lookup_backward(corr_shape, coord, grad_out, levels=4, radius=4, clamp_unit=
 
 
 # Both aggregated volumes of a model at once: corr1 (B,dim,D1,H1,W1), read with coords[:, 0] and clamped positions, and corr2
-# (B,dim,D2,H1,W1), read with coords[:, 1].
-def _pair_sizes(shape1, shape2):
-    B, dim, D1, H1, W1 = shape1
-    if len(shape2) != 5 or tuple(shape2[:2]) != (B, dim) or tuple(shape2[3:]) != (H1, W1):
-        raise RuntimeError(f"the volumes differ in more than their displacements: {tuple(shape1)} and {tuple(shape2)}")
-    return B, dim, D1, shape2[2], H1, W1
-
-
-def _check_pair_volumes(corr1, corr2):
-    _check_volume(corr1)
-    _check_volume(corr2)
-    if corr1.device != corr2.device:
-        raise RuntimeError(f"corr1 is on {corr1.device}, corr2 on {corr2.device}")
-    return _pair_sizes(corr1.shape, corr2.shape)
-
-
-def _check_coords_pair(coords, B, H1, W1, dev):
-    """Strides between the samples and the components of coords (B, 2 or more, H1, W1)."""
-    if not (coords.is_cuda and coords.dtype == torch.float32 and coords.dim() == 4 and coords.device == dev
-            and coords.shape[0] == B and coords.shape[1] >= 2 and coords.shape[2] == H1 and coords.shape[3] == W1):
-        raise RuntimeError(f"coords must be a CUDA float32 tensor of shape {(B, 2, H1, W1)} on {dev}")
-    sb, sc, sh, sw = coords.stride()
-    if (sw != 1 and W1 > 1) or (sh != W1 and H1 > 1):
-        raise RuntimeError("coords must be contiguous within a component of a sample")
-    return sb, sc
-
-
+# (B,dim,D2,H1,W1), read with coords[:, 1].  Checks, outputs and the call are native (pybind/host_module.cpp).
 def lookup_build_pyramid_pair(corr1, corr2, levels: int):
     """lookup_build_pyramid of both volumes, in one launch."""
-    B, dim, D1, D2, H1, W1 = _check_pair_volumes(corr1, corr2)
-    lib = _lib.load()
-    pyr = [torch.empty(max(lib.sfb_lookup_pyramid_bytes(B, dim, D, H1, W1, levels) // 4, 1), dtype=torch.float32, device=corr1.device)
-           for D in (D1, D2)]
-    with _on(corr1.device):
-        stream = _stream(corr1.device)
-        _raise_on(lib.sfb_lookup_build_pyramid_pair(corr1.data_ptr(), pyr[0].data_ptr(), corr2.data_ptr(), pyr[1].data_ptr(), B, dim,
-                                                    D1, D2, H1, W1, levels, stream), "sfb_lookup_build_pyramid_pair")
-    return pyr
+    return _lib.host().lookup_build_pyramid_pair(corr1, corr2, levels)
 
 
 def lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels=4, radius=4):
     """(lookup_forward(corr1, pyramid1, coords[:, 0], clamp_unit=True), lookup_forward(corr2, pyramid2, coords[:, 1])), in one launch."""
-    B, dim, D1, D2, H1, W1 = _check_pair_volumes(corr1, corr2)
-    dev = corr1.device
-    sb, sc = _check_coords_pair(coords, B, H1, W1, dev)
-    size = (B, levels * dim * (2 * radius + 1), H1, W1)
-    out1 = torch.empty(size, dtype=torch.float32, device=dev)
-    out2 = torch.empty(size, dtype=torch.float32, device=dev)
-    lib = _lib.load()
-    with _on(dev):
-        stream = _stream(dev)
-        _raise_on(lib.sfb_lookup_forward_pair(corr1.data_ptr(), pyramid1.data_ptr(), corr2.data_ptr(), pyramid2.data_ptr(),
-                                              coords.data_ptr(), sb, sc, out1.data_ptr(), out2.data_ptr(), B, dim, D1, D2, H1, W1,
-                                              levels, radius, stream), "sfb_lookup_forward_pair")
-    return out1, out2
+    return _lib.host().lookup_forward_pair(corr1, corr2, pyramid1, pyramid2, coords, levels, radius)
 
 
 def lookup_accumulator_size(corr_shape, levels, clamp_unit) -> int:
@@ -864,20 +818,7 @@ def lookup_accumulator_size(corr_shape, levels, clamp_unit) -> int:
 def lookup_accumulate_pair(shape1, shape2, coords, gout1, gout2, acc1, acc2, levels=4, radius=4) -> None:
     """Adds the gradients of one lookup_forward_pair to the volumes' accumulators (flat tensors of lookup_accumulator_size elements),
     in place.  gout1 and acc1, or gout2 and acc2, may both be None."""
-    B, dim, D1, D2, H1, W1 = _pair_sizes(shape1, shape2)
-    dev = coords.device
-    sb, sc = _check_coords_pair(coords, B, H1, W1, dev)
-    for gout, acc, shape, clamp in ((gout1, acc1, shape1, True), (gout2, acc2, shape2, False)):
-        if gout is not None:
-            _check_like(gout, "grad_out", (B, levels * dim * (2 * radius + 1), H1, W1), torch.float32, dev)
-            _check_like(acc, "accumulator", (lookup_accumulator_size(shape, levels, clamp),), torch.float32, dev)
-    lib = _lib.load()
-    with _on(dev):
-        stream = _stream(dev)
-        _raise_on(lib.sfb_lookup_accumulate_pair(
-            gout1.data_ptr() if gout1 is not None else None, gout2.data_ptr() if gout2 is not None else None, coords.data_ptr(), sb,
-            sc, acc1.data_ptr() if gout1 is not None else None, acc2.data_ptr() if gout2 is not None else None, B, dim, D1, D2, H1,
-            W1, levels, radius, stream), "sfb_lookup_accumulate_pair")
+    _lib.host().lookup_accumulate_pair(shape1, shape2, coords, gout1, gout2, acc1, acc2, levels, radius)
 
 
 def lookup_fold_gradient(acc, corr_shape, levels=4, clamp_unit=False) -> torch.Tensor:
