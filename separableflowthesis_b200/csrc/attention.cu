@@ -56,6 +56,7 @@ struct StageWeights {
 };
 __device__ float g_att_weights[2 * AT_WEIGHTS];   // on their way into constant memory
 __global__ void __launch_bounds__(AT_KC * 2 * AT_TAPS) stage_weights_kernel(const __grid_constant__ StageWeights s) {
+  follow_previous_kernel();
   const int m = blockIdx.x, i = threadIdx.x, k = i / (2 * AT_TAPS), c = i / AT_TAPS & 1, tap = i % AT_TAPS, td = tap / 9, n = tap % 9;
   if (s.weight[m] == nullptr || k >= s.channels) return;
   g_att_weights[m * AT_WEIGHTS + (s.input_grad ? input_grad_weight(k, c, td, 8 - n) : forward_weight(k, c, td, n))] = __ldg(s.weight[m] + i);
@@ -241,6 +242,7 @@ __device__ __forceinline__ void softmax_columns(const LogitsJobs::Job& job, int 
 template <int KC, bool SOFT>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_logits_kernel(const __grid_constant__ LogitsJobs jobs, int Kc, int k0, int B, int H1, int W1) {
+  follow_previous_kernel();
   __shared__ float ring_mem[FW_STAGES * 18 * AT_THREADS];
   const int ji = job_of(jobs.blocks, blockIdx.x);
   const LogitsJobs::Job& job = jobs.j[ji];
@@ -490,6 +492,7 @@ struct SoftmaxJobs {
 template <int V>
 __global__ void __launch_bounds__(SM_THREADS, V == 0 ? 8 : (V <= 8 ? 6 : (V <= 20 ? 3 : 2)))
 attention_softmax_kernel(const __grid_constant__ SoftmaxJobs jobs, int N1, unsigned pixel_blocks) {
+  follow_previous_kernel();
   __shared__ float red[2][SM_GROUPS][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int ji = job_of(jobs.blocks, blockIdx.x), D = jobs.D[ji];
@@ -582,6 +585,7 @@ __host__ __device__ constexpr int lg_pixels(int G) { return lg_warps(G) / G * 32
 template <int G, int V, int MIN_BLOCKS>
 __global__ void __launch_bounds__(32 * lg_warps(G), MIN_BLOCKS)
 attention_logit_grad_kernel(const __grid_constant__ LogitGradJobs jobs, int Kc, int N1, unsigned pixel_blocks) {
+  follow_previous_kernel();
   const int ji = job_of(jobs.blocks, blockIdx.x);
   const LogitGradJobs::Job& job = jobs.j[ji];
   const float* __restrict__ const a = job.a;
@@ -736,6 +740,7 @@ __device__ __forceinline__ void input_grad_walk_gather(const InputGradJobs::Job&
 template <int KC>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_input_grad_kernel(const __grid_constant__ InputGradJobs jobs, int accumulate, int Kc, int k0, int B, int H1, int W1) {
+  follow_previous_kernel();
   extern __shared__ float ring_dyn[];
   const int ji = job_of(jobs.blocks, blockIdx.x);
   const InputGradJobs::Job& job = jobs.j[ji];
@@ -766,6 +771,7 @@ struct WeightGradJobs {
 template <int KW>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_weight_grad_kernel(const __grid_constant__ WeightGradJobs jobs, int Kc, int B, int H1, int W1) {
+  follow_previous_kernel();
   const int ji = job_of(jobs.blocks, blockIdx.x);
   const WeightGradJobs::Job& job = jobs.j[ji];
   const float* __restrict__ const x = job.x;
@@ -870,6 +876,7 @@ struct PartialSums {
 };
 __global__ void __launch_bounds__(RP_THREADS)
 attention_reduce_partials_kernel(const __grid_constant__ PartialSums sums) {
+  follow_previous_kernel();
   __shared__ float red[RP_THREADS];
   int j = 0;
 #pragma unroll
@@ -1208,7 +1215,7 @@ class StagedWeights {
     StageWeights s{{nullptr, nullptr}, channels, input_grad};
     for (int m = 0; m < 2; ++m)
       if (modules.weight[m] != nullptr) s.weight[m] = modules.weight[m] + (size_t)k0 * 2 * AT_TAPS;
-    stage_weights_kernel<<<2, AT_KC * 2 * AT_TAPS, 0, st_>>>(s);
+    launch_next(stage_weights_kernel, 2, AT_KC * 2 * AT_TAPS, 0, st_, s);
     err_ = cudaGetLastError();
     if (err_ == cudaSuccess) err_ = cudaMemcpyAsync(g_stage.constant[dev_], g_stage.ordered[dev_], sizeof(c_att_weights), cudaMemcpyDeviceToDevice, st_);
     return err_;
@@ -1331,7 +1338,7 @@ static cudaError_t launch_softmax_class(const AttentionJob* job, int count, int 
   }
   if (n == 0) return cudaSuccess;
   for (; n <= MAX_ATTENTION_JOBS; ++n) jobs.blocks.first[n] = (int)blocks;
-  attention_softmax_kernel<V><<<(unsigned)blocks, SM_THREADS, 0, st>>>(jobs, d.H1 * d.W1, pb);
+  launch_next(attention_softmax_kernel<V>, (unsigned)blocks, SM_THREADS, 0, st, jobs, d.H1 * d.W1, pb);
   return cudaGetLastError();
 }
 static int softmax_class(int D) {   // largest values per warp of a class; 0: any
@@ -1442,13 +1449,13 @@ cudaError_t launch_attention_forward(const AttentionJob* job, int count, const A
       by_channels(kc, [&](auto c) {
         constexpr int KC = decltype(c)::value;
         if (!tiled) {
-          (soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>)<<<(unsigned)blocks, AT_THREADS, 0, st>>>(
-              jobs, d.Kc, k0, d.B, d.H1, d.W1);
+          launch_next(soft ? attention_logits_kernel<KC, true> : attention_logits_kernel<KC, false>, (unsigned)blocks, AT_THREADS, 0, st, jobs,
+                      d.Kc, k0, d.B, d.H1, d.W1);
           return;
         }
         auto kernel = tma ? (soft ? attention_logits_tiled_kernel<KC, true, FEED_TMA> : attention_logits_tiled_kernel<KC, false, FEED_TMA>)
                           : (soft ? attention_logits_tiled_kernel<KC, true, FEED_COPIES> : attention_logits_tiled_kernel<KC, false, FEED_COPIES>);
-        kernel<<<(unsigned)blocks, AT_THREADS, 0, st>>>(maps, jobs, d.Kc, k0, d.B, d.H1, d.W1, status);
+        launch_next(kernel, (unsigned)blocks, AT_THREADS, 0, st, maps, jobs, d.Kc, k0, d.B, d.H1, d.W1, status);
       });
       if ((err = cudaGetLastError()) != cudaSuccess) return err;
     }
@@ -1466,7 +1473,7 @@ static cudaError_t launch_input_grad(unsigned blocks, const InputGradJobs& jobs,
         [&] { return cudaFuncSetAttribute(attention_input_grad_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
     if (err != cudaSuccess) return err;
   }
-  attention_input_grad_kernel<KC><<<blocks, AT_THREADS, smem, st>>>(jobs, accumulate, d.Kc, k0, d.B, d.H1, d.W1);
+  launch_next(attention_input_grad_kernel<KC>, blocks, AT_THREADS, smem, st, jobs, accumulate, d.Kc, k0, d.B, d.H1, d.W1);
   return cudaGetLastError();
 }
 
@@ -1494,7 +1501,7 @@ static cudaError_t launch_logit_grad_class(const AttentionGradJob* job, const Pa
   }
   if (n == 0) return cudaSuccess;
   for (; n <= MAX_ATTENTION_JOBS; ++n) jobs.blocks.first[n] = (int)blocks;
-  attention_logit_grad_kernel<G, V, MIN_BLOCKS><<<(unsigned)blocks, 32 * lg_warps(G), 0, st>>>(jobs, d.Kc, d.H1 * d.W1, pb);
+  launch_next(attention_logit_grad_kernel<G, V, MIN_BLOCKS>, (unsigned)blocks, 32 * lg_warps(G), 0, st, jobs, d.Kc, d.H1 * d.W1, pb);
   return cudaGetLastError();
 }
 static int logit_grad_class(int D) {
@@ -1602,8 +1609,8 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
           err = launch_input_grad<KC>((unsigned)blocks, jobs, accumulate, d, k0, st);
           return;
         }
-        (tma ? attention_input_grad_tiled_kernel<KC, FEED_TMA> : attention_input_grad_tiled_kernel<KC, FEED_COPIES>)
-            <<<(unsigned)blocks, AT_THREADS, 0, st>>>(maps, jobs, accumulate, d.Kc, k0, d.B, d.H1, d.W1, status);
+        launch_next(tma ? attention_input_grad_tiled_kernel<KC, FEED_TMA> : attention_input_grad_tiled_kernel<KC, FEED_COPIES>, (unsigned)blocks,
+                    AT_THREADS, 0, st, maps, jobs, accumulate, d.Kc, k0, d.B, d.H1, d.W1, status);
         err = cudaGetLastError();
       });
       if (err != cudaSuccess) return err;
@@ -1629,14 +1636,15 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
   by_channels(kw, [&](auto c) {
     constexpr int KW = decltype(c)::value;
     if (!tiled) {
-      attention_weight_grad_kernel<KW><<<dim3((unsigned)blocks, 2 * chunks), AT_THREADS, 0, st>>>(jobs, d.Kc, d.B, d.H1, d.W1);
+      launch_next(attention_weight_grad_kernel<KW>, dim3((unsigned)blocks, 2 * chunks), AT_THREADS, 0, st, jobs, d.Kc, d.B, d.H1, d.W1);
     } else if constexpr (KW <= WG_MAX_CHANNELS) {
-      (tma ? attention_weight_grad_tiled_kernel<KW, FEED_TMA> : attention_weight_grad_tiled_kernel<KW, FEED_COPIES>)
-          <<<dim3((unsigned)blocks, chunks), wg_threads(tma ? FEED_TMA : FEED_COPIES), 0, st>>>(maps_x, maps_gl, jobs, d.Kc, d.B, d.H1, d.W1, status);
+      launch_next(tma ? attention_weight_grad_tiled_kernel<KW, FEED_TMA> : attention_weight_grad_tiled_kernel<KW, FEED_COPIES>,
+                  dim3((unsigned)blocks, chunks), wg_threads(tma ? FEED_TMA : FEED_COPIES), 0, st, maps_x, maps_gl, jobs, d.Kc, d.B, d.H1, d.W1,
+                  status);
     }
   });
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
-  attention_reduce_partials_kernel<<<columns, RP_THREADS, 0, st>>>(sums);
+  launch_next(attention_reduce_partials_kernel, columns, RP_THREADS, 0, st, sums);
   return cudaGetLastError();
 }
 

@@ -690,6 +690,7 @@ constexpr int GG_FOLD_THREADS = 256;
 __host__ __device__ constexpr int grad_fold_blocks(int C) { return (C * (TILE_M / 4) + GG_FOLD_THREADS - 1) / GG_FOLD_THREADS; }
 template <int FORM, int LEVELS>
 __global__ void __launch_bounds__(GG_FOLD_THREADS) grad_fold_kernel(const __grid_constant__ GradLaunch<LEVELS> launch) {
+  follow_previous_kernel();
   const int C = launch.a[0].d.C, per_tail = grad_fold_blocks(C), t = blockIdx.x / per_tail;   // C is a multiple of 4
   const int level = grad_level<LEVELS>(launch.first_tail, t);
   const GradArgs& a = launch.a[level];
@@ -920,12 +921,12 @@ static cudaError_t launch_one(GradLaunch<LEVELS>& launch, int levels, cudaStream
   }
   launch.first_block[LEVELS] = blocks;
   launch.first_tail[LEVELS] = tails;
-  kern<<<blocks, gg_threads<FORM>(), smem_bytes, stream>>>(launch, launch.a[0].status);
+  launch_next(kern, blocks, gg_threads<FORM>(), smem_bytes, stream, launch, launch.a[0].status);
   if (tails > 0) {
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     const long long fold_blocks = (long long)tails * grad_fold_blocks(launch.a[0].d.C);
     if (fold_blocks > INT_MAX) return cudaErrorInvalidConfiguration;
-    grad_fold_kernel<FORM, LEVELS><<<(unsigned)fold_blocks, GG_FOLD_THREADS, 0, stream>>>(launch);
+    launch_next(grad_fold_kernel<FORM, LEVELS>, (unsigned)fold_blocks, GG_FOLD_THREADS, 0, stream, launch);
   }
   return cudaGetLastError();
 }

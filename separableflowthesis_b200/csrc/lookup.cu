@@ -13,6 +13,7 @@
 // times on the same two volumes and wants the sum of their gradients: the lookups of a pair of volumes add their windows to one
 // accumulator per level (lookup_accumulate_kernel), which is folded once (lookup_gradient_fold_kernel).
 #include "kernels.h"
+#include "sm100_primitives.cuh"
 
 namespace sfb {
 
@@ -45,6 +46,7 @@ struct LookupPyramids { LookupLevelsMut v[2]; };
 template <int VEC>
 __global__ void __launch_bounds__(LK_THREADS)
 lookup_pyramid_kernel(const __grid_constant__ LookupPyramids vols, int base, int levels, int row_blocks, int N1) {
+  follow_previous_kernel();
   typedef typename LkVec<VEC>::type V;
   const int p = (blockIdx.x * LK_THREADS + threadIdx.x) * VEC;
   const int vol = blockIdx.y / row_blocks, r0 = (blockIdx.y - vol * row_blocks) * LK_PROWS;
@@ -100,6 +102,7 @@ constexpr int LK_WARPS = 4;
 template <int TAPS>
 __global__ void __launch_bounds__(32 * LK_WARPS, TAPS > 0 ? 5 : 0)
 lookup_forward_kernel(const __grid_constant__ LookupVolumes vols, int dim, int N1, int levels, int radius) {
+  follow_previous_kernel();
   const int p = (blockIdx.x * blockDim.z + threadIdx.z) * 32 + threadIdx.x, b = blockIdx.y;
   if (p >= N1) return;
   const LookupVolume& lv = vols.v[blockIdx.z];
@@ -141,6 +144,7 @@ lookup_forward_kernel(const __grid_constant__ LookupVolumes vols, int dim, int N
 __global__ void lookup_backward_kernel(const LookupLevelsMut gl, const float* __restrict__ coord, long long coord_sb,
                                        const float* __restrict__ gout, int dim, int N1, int levels, int radius,
                                        int clamp_unit) {
+  follow_previous_kernel();
   const int p = blockIdx.x * LK_THREADS + threadIdx.x, b = blockIdx.y;
   if (p >= N1) return;
   const float c = __ldg(coord + (size_t)b * coord_sb + p);
@@ -169,6 +173,7 @@ __global__ void lookup_backward_kernel(const LookupLevelsMut gl, const float* __
 // evenly over the 2^l entries it averaged; entries dropped by the floor of an odd size get none).
 // grid (ceil(N1/128), D, planes)
 __global__ void lookup_fold_kernel(const LookupLevelsMut gl, int N1, int levels) {
+  follow_previous_kernel();
   const int p = blockIdx.x * LK_THREADS + threadIdx.x, i = blockIdx.y;
   if (p >= N1) return;
   float acc = 0.f, scale = 1.f;
@@ -202,6 +207,7 @@ __global__ void __launch_bounds__(32 * LK_BWARPS)
 lookup_backward_window_kernel(const float* __restrict__ coord, long long coord_sb, const float* __restrict__ gout,
                               float* __restrict__ gcorr, int dim, int D, int N1, int levels, int radius,
                               int clamp_unit) {
+  follow_previous_kernel();
   __shared__ float win[LOOKUP_MAX_LEVELS][LK_WIN][32];
   __shared__ int wbase[LOOKUP_MAX_LEVELS][32];
   constexpr int MAX_TAPS = TAPS > 0 ? TAPS : 2 * LK_RMAX + 1;
@@ -283,6 +289,7 @@ struct LookupAccumulators { LookupAccumulator v[2]; };
 template <bool WINDOW, int TAPS>
 __global__ void __launch_bounds__(32 * LK_WARPS)
 lookup_accumulate_kernel(const __grid_constant__ LookupAccumulators vols, int dim, int N1, int levels, int radius) {
+  follow_previous_kernel();
   __shared__ float win_mem[WINDOW ? LK_WARPS : 1][LK_WIN][32];
   constexpr int MAX_TAPS = TAPS > 0 ? TAPS : 2 * LK_RMAX + 1;
   const int p = (blockIdx.x * blockDim.z + threadIdx.z) * 32 + threadIdx.x;
@@ -346,6 +353,7 @@ lookup_accumulate_kernel(const __grid_constant__ LookupAccumulators vols, int di
 template <int VEC>
 __global__ void __launch_bounds__(LK_THREADS)
 lookup_gradient_fold_kernel(const __grid_constant__ LookupAccumulator lv, float* __restrict__ gcorr, int levels, int N1) {
+  follow_previous_kernel();
   typedef typename LkVec<VEC>::type V;
   const int p = (blockIdx.x * LK_THREADS + threadIdx.x) * VEC, r0 = blockIdx.y * LK_PROWS, D = lv.D[0];
   if (p >= N1) return;
@@ -407,7 +415,7 @@ static cudaError_t launch_pyramids(const LookupDims* d, const float* const* corr
     for (int v = 0; v < volumes; ++v) D = std::max(D, vols.v[v].D[base]);
     const int row_blocks = (D + LK_PROWS - 1) / LK_PROWS;
     const dim3 grid((N1 + px - 1) / px, volumes * row_blocks, d[0].B * d[0].dim);
-    (vec ? lookup_pyramid_kernel<4> : lookup_pyramid_kernel<1>)<<<grid, LK_THREADS, 0, st>>>(vols, base, levels, row_blocks, N1);
+    launch_next((vec ? lookup_pyramid_kernel<4> : lookup_pyramid_kernel<1>), grid, LK_THREADS, 0, st, vols, base, levels, row_blocks, N1);
   }
   return cudaGetLastError();
 }
@@ -437,7 +445,7 @@ static cudaError_t launch_forward(const LookupDims* d, const LookupCall* c, int 
   const int N1 = d[0].H1 * d[0].W1;
   const dim3 block = level_block(d[0].levels), grid(pixel_blocks(N1, block), d[0].B, volumes);
   auto kern = d[0].radius == LK_RMAX ? lookup_forward_kernel<2 * LK_RMAX + 1> : lookup_forward_kernel<0>;
-  kern<<<grid, block, 0, st>>>(vols, d[0].dim, N1, d[0].levels, d[0].radius);
+  launch_next(kern, grid, block, 0, st, vols, d[0].dim, N1, d[0].levels, d[0].radius);
   return cudaGetLastError();
 }
 cudaError_t launch_lookup_forward(const LookupDims& d, const LookupCall& c, cudaStream_t st) { return launch_forward(&d, &c, 1, st); }
@@ -475,7 +483,7 @@ cudaError_t launch_lookup_accumulate(const LookupDims* d, const LookupGradient* 
   auto kern = radius == LK_RMAX  ? lookup_accumulate_kernel<true, 2 * LK_RMAX + 1>
               : radius < LK_RMAX ? lookup_accumulate_kernel<true, 0>
                                  : lookup_accumulate_kernel<false, 0>;
-  kern<<<grid, block, 0, st>>>(vols, d[0].dim, N1, d[0].levels, radius);
+  launch_next(kern, grid, block, 0, st, vols, d[0].dim, N1, d[0].levels, radius);
   return cudaGetLastError();
 }
 
@@ -486,7 +494,7 @@ cudaError_t launch_lookup_gradient_fold(const LookupDims& d, const float* acc, f
   const bool vec = lk_vec4(N1, {acc, gcorr});
   const int px = LK_THREADS * (vec ? 4 : 1);
   const dim3 grid((N1 + px - 1) / px, (d.D + LK_PROWS - 1) / LK_PROWS, d.B * d.dim);
-  (vec ? lookup_gradient_fold_kernel<4> : lookup_gradient_fold_kernel<1>)<<<grid, LK_THREADS, 0, st>>>(a, gcorr, d.levels, N1);
+  launch_next((vec ? lookup_gradient_fold_kernel<4> : lookup_gradient_fold_kernel<1>), grid, LK_THREADS, 0, st, a, gcorr, d.levels, N1);
   return cudaGetLastError();
 }
 
@@ -496,7 +504,7 @@ cudaError_t launch_lookup_backward(const LookupDims& d, const float* gout, const
   if (d.radius <= LK_RMAX) {
     const dim3 wgrid((N1 + 31) / 32, d.B * d.dim);
     auto kern = d.radius == LK_RMAX ? lookup_backward_window_kernel<2 * LK_RMAX + 1> : lookup_backward_window_kernel<0>;
-    kern<<<wgrid, 32 * LK_BWARPS, 0, st>>>(coord, coord_sb, gout, gcorr, d.dim, d.D, N1, d.levels, d.radius, clamp_unit);
+    launch_next(kern, wgrid, 32 * LK_BWARPS, 0, st, coord, coord_sb, gout, gcorr, d.dim, d.D, N1, d.levels, d.radius, clamp_unit);
     return cudaGetLastError();
   }
   LookupLevelsMut gl;
@@ -509,11 +517,11 @@ cudaError_t launch_lookup_backward(const LookupDims& d, const float* gout, const
     if (err != cudaSuccess) return err;
   }
   const dim3 grid((N1 + LK_THREADS - 1) / LK_THREADS, d.B);
-  lookup_backward_kernel<<<grid, LK_THREADS, 0, st>>>(gl, coord, coord_sb, gout, d.dim, N1, d.levels, d.radius,
+  launch_next(lookup_backward_kernel, grid, LK_THREADS, 0, st, gl, coord, coord_sb, gout, d.dim, N1, d.levels, d.radius,
                                                      clamp_unit);
   if (d.levels > 1) {
     const dim3 fgrid((N1 + LK_THREADS - 1) / LK_THREADS, d.D, d.B * d.dim);
-    lookup_fold_kernel<<<fgrid, LK_THREADS, 0, st>>>(gl, N1, d.levels);
+    launch_next(lookup_fold_kernel, fgrid, LK_THREADS, 0, st, gl, N1, d.levels);
   }
   return cudaGetLastError();
 }

@@ -195,6 +195,7 @@ template <int NQ, int LP, bool FULL>
 __global__ void __launch_bounds__(L4_THREADS, 2)
 lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                         float* __restrict__ out, int H1, int W1, int C, int radius, int levels, float scale) {
+  follow_previous_kernel();
   __shared__ float s_S[L4_WARPS][L4_PX][L4_BMAX];
   __shared__ float s_out[L4_WIN * L4_WIN][L4_TILE + 1];
   __shared__ int s_rows[L4_WARPS][L4_BMAX];
@@ -440,6 +441,7 @@ __global__ void __launch_bounds__(L4_BTHREADS, 2)
 lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                          const float* __restrict__ gout, float* __restrict__ gF1, int H1, int W1, int C, int radius,
                          int levels, int limit, float scale) {
+  follow_previous_kernel();
   __shared__ L4Tile s_tile;
   __shared__ __align__(16) float s_gS[L4_BBOX + 4][L4_BPX];     // gradient of (position, pixel), scaled; positions without any are left out
   __shared__ __align__(16) int s_rows[L4_BBOX + 4];             // their image-2 rows
@@ -631,6 +633,7 @@ __global__ void __launch_bounds__(L4_APART, 4)
 lookup4d_backward_apart_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                                const float* __restrict__ gout, float* __restrict__ gF1, int H1, int W1, int C, int radius,
                                int levels, int limit, float scale) {
+  follow_previous_kernel();
   __shared__ L4Tile s_tile;
   __shared__ float s_gS[L4_APART_WARPS][L4_PX][L4_BMAX];
   __shared__ float s_g[L4_WIN * L4_WIN][L4_BPX + 1];
@@ -730,6 +733,7 @@ lookup4d_backward_apart_kernel(const float* __restrict__ F1, Lookup4dLevels lv, 
 
 // Zeros for the reductions, all levels in one launch (C is a multiple of 4 and the pointers are 16-byte aligned).
 __global__ void __launch_bounds__(256) lookup4d_clear_kernel(Lookup4dLevels lv, int B, int C) {
+  follow_previous_kernel();
   float4* const p = reinterpret_cast<float4*>(lv.g2[blockIdx.y]);
   const size_t n = (size_t)B * lv.H2[blockIdx.y] * lv.W2[blockIdx.y] * (C / 4);
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -755,7 +759,7 @@ cudaError_t launch_lookup4d_forward(const Lookup4dDims& d, const float* F1, cons
   const Lookup4dLevels lv = make_levels(d, F2, nullptr);
   const dim3 grid(l4_tiles(d), d.levels, d.B);
 #define SFB_L4_FWD(NQ, LP)                                                                                                             \
-  (d.C == NQ * 4 * LP ? lookup4d_forward_kernel<NQ, LP, true> : lookup4d_forward_kernel<NQ, LP, false>)<<<grid, L4_THREADS, 0, stream>>>( \
+  launch_next((d.C == NQ * 4 * LP ? lookup4d_forward_kernel<NQ, LP, true> : lookup4d_forward_kernel<NQ, LP, false>), grid, L4_THREADS, 0, stream, \
       F1, lv, coords, out, d.H1, d.W1, d.C, d.radius, d.levels, scale)
   switch ((d.C + 63) / 64) {
     case 1: SFB_L4_FWD(1, 16); break;
@@ -778,18 +782,20 @@ cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, con
   const Lookup4dLevels lv = make_levels(d, F2, gF2);
   size_t largest = 0;
   for (int l = 0; l < d.levels; ++l) largest = std::max(largest, (size_t)d.B * d.H2[l] * d.W2[l] * (d.C / 4));
-  lookup4d_clear_kernel<<<dim3((unsigned)std::min<size_t>((largest + 1023) / 1024, 148 * 8), d.levels), 256, 0, stream>>>(lv, d.B, d.C);
+  launch_next(lookup4d_clear_kernel, dim3((unsigned)std::min<size_t>((largest + 1023) / 1024, 148 * 8), d.levels), 256, 0, stream, lv, d.B, d.C);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const dim3 grid((unsigned)((d.W1 + L4_BT - 1) / L4_BT) * (unsigned)((d.H1 + L4_BT - 1) / L4_BT), 1, d.B);   // per tile
   const int limit = l4_tile_limit(d.radius);
   if (limit > 0) {
     const dim3 whole(grid.x, (unsigned)((d.C + L4_BTHREADS - 1) / L4_BTHREADS), d.B);
-    lookup4d_backward_kernel<<<whole, L4_BTHREADS, 0, stream>>>(F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale);
+    launch_next(lookup4d_backward_kernel, whole, L4_BTHREADS, 0, stream, F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
-#define SFB_L4_BWD(NCH) lookup4d_backward_apart_kernel<NCH><<<grid, L4_APART, 0, stream>>>(F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale)
+#define SFB_L4_BWD(NCH)                                                                                                                 \
+  launch_next(lookup4d_backward_apart_kernel<NCH>, grid, L4_APART, 0, stream, F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, \
+              limit, scale)
   switch ((d.C + 127) / 128) {
     case 1: SFB_L4_BWD(1); break;
     case 2: SFB_L4_BWD(2); break;

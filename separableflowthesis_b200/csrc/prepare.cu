@@ -66,6 +66,7 @@ struct AbsmaxJobs {
 };
 __global__ void __launch_bounds__(AM_THREADS)
 absmax_kernel(const __grid_constant__ AbsmaxJobs jobs, float* scales, int levels, int gradients) {
+  follow_previous_kernel();
   __shared__ float red[AM_THREADS / 32];
   int job = 0;
 #pragma unroll
@@ -125,6 +126,7 @@ static_assert(MAX_FUSED_LEVELS == 4, "8 x 8 pixels are one of the coarsest level
 template <bool VEC, bool MAGNITUDES>
 __global__ void __launch_bounds__(AM_THREADS)
 pool_levels_kernel(const __grid_constant__ PoolJob job, float* scales) {
+  follow_previous_kernel();
   constexpr int SLOTS = MAX_FUSED_LEVELS + 1;   // magnitudes of the levels of image 2, of image 1
   float m[SLOTS];
 #pragma unroll
@@ -241,7 +243,7 @@ static cudaError_t launch_pool(const Dims* d, int levels, const float* fmap1, co
   const bool vec = job.W % 4 == 0 && reinterpret_cast<uintptr_t>(job.in) % 16 == 0;
   auto kern = magnitudes ? (vec ? pool_levels_kernel<true, true> : pool_levels_kernel<false, true>)
                          : (vec ? pool_levels_kernel<true, false> : pool_levels_kernel<false, false>);
-  kern<<<(unsigned)(blocks1 + blocks2), AM_THREADS, 0, stream>>>(job, scales);
+  launch_next(kern, (unsigned)(blocks1 + blocks2), AM_THREADS, 0, stream, job, scales);
   return cudaGetLastError();
 }
 
@@ -259,6 +261,7 @@ struct UnpoolJob {
 };
 __global__ void __launch_bounds__(256)
 unpool_levels_kernel(const __grid_constant__ UnpoolJob job) {
+  follow_previous_kernel();
   const int H = job.H, W = job.W, quads = (W + 3) / 4;
   const int i = blockIdx.x * 256 + threadIdx.x, y = i / quads, x0 = (i - y * quads) * 4;
   if (y >= H) return;
@@ -291,7 +294,7 @@ cudaError_t launch_unpool_levels(const Dims* d, int levels, float* g0, const flo
   const long long planes = (long long)d[0].B * d[0].C;
   for (long long p0 = 0; p0 < planes; p0 += 65535) {
     const unsigned n = (unsigned)std::min<long long>(planes - p0, 65535);
-    unpool_levels_kernel<<<dim3((unsigned)(((long long)quads * job.H + 255) / 256), n), 256, 0, stream>>>(job);
+    launch_next(unpool_levels_kernel, dim3((unsigned)(((long long)quads * job.H + 255) / 256), n), 256, 0, stream, job);
     if (cudaError_t err = cudaGetLastError(); err != cudaSuccess) return err;
     job.g0 += (size_t)n * d[0].N2();
     for (int l = 1; l < levels; ++l) job.g[l - 1] += (size_t)n * d[l].N2();
@@ -317,7 +320,7 @@ cudaError_t launch_absmax(const AbsmaxSource* src, int count, float* scales, int
     blocks += (long long)jobs.blocks[i] * jobs.src[i].samples;
     if (blocks > INT_MAX) return cudaErrorInvalidConfiguration;
   }
-  absmax_kernel<<<(unsigned)blocks, AM_THREADS, 0, stream>>>(jobs, scales, levels, gradients ? 1 : 0);
+  launch_next(absmax_kernel, (unsigned)blocks, AM_THREADS, 0, stream, jobs, scales, levels, gradients ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -360,6 +363,7 @@ constexpr int FM_GROUPS = 4, FM_QUADS = 64;
 __global__ void __launch_bounds__(FM_GROUPS * FM_QUADS)
 round_means_kernel(const RoundJob j1, const RoundJob j2, int copies1, int copies2, const float* __restrict__ F2, float* __restrict__ aux, int mean_rows,
                    int B, int H2, int W2, int C, uint16_t* __restrict__ auxh, int op16, const float* __restrict__ scale16) {
+  follow_previous_kernel();
   __shared__ float4 red[FM_GROUPS][FM_QUADS];
   const int block = (int)blockIdx.x - mean_rows * B;
   if (block >= 0) {
@@ -420,6 +424,7 @@ struct MeansJobs {
 template <int NV>
 __global__ void __launch_bounds__(256)
 f2_means_cf_kernel(const __grid_constant__ MeansJobs jobs, int C, int op16) {
+  follow_previous_kernel();
   const MeansJobs::Job& job = jobs.j[blockIdx.z];
   const float* const fmap2 = job.fmap2;
   float* const aux = job.aux;
@@ -526,6 +531,7 @@ __device__ __forceinline__ Patch patch_of(const PatchJobs& jobs, int n1p, int& j
 }
 
 __global__ void pack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
+  follow_previous_kernel();
   __shared__ uint32_t tile[PACK_PX][33];
   int ji;
   const Patch t = patch_of(jobs, n1p, ji);
@@ -548,6 +554,7 @@ __global__ void pack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int 
 }
 
 __global__ void unpack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
+  follow_previous_kernel();
   __shared__ uint32_t tile[PACK_PX][33];
   int ji;
   const Patch t = patch_of(jobs, n1p, ji);
@@ -577,7 +584,7 @@ static cudaError_t launch_patches(Kernel kern, const PatchJob* job, int count, i
     if (i < count) blocks += (long long)((job[i].D + 31) / 32) * (n1p / PACK_PX) * B * job[i].K;
     if (blocks > INT_MAX) return cudaErrorInvalidConfiguration;
   }
-  kern<<<(unsigned)blocks, dim3(32, 8), 0, stream>>>(jobs, N1, n1p);
+  launch_next(kern, (unsigned)blocks, dim3(32, 8), 0, stream, jobs, N1, n1p);
   return cudaGetLastError();
 }
 cudaError_t launch_pack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream) {
@@ -592,6 +599,7 @@ cudaError_t launch_unpack(const PatchJob* jobs, int count, int B, int N1, int n1
 // launch.  grid (ceil(largest D/32), n1p/32, groups * B), block (32, 8).
 __global__ void __launch_bounds__(256)
 pack_interleaved_kernel(const __grid_constant__ PackGroups groups, int B, int N1, int n1p) {
+  follow_previous_kernel();
   constexpr int RS = 32 * 33 + 32 / 4;  // slot stride chosen so that the interleaved read below is conflict-free
   __shared__ uint32_t tile[4 * RS];
   const int gi = blockIdx.z / B, b = blockIdx.z - gi * B;
@@ -650,7 +658,7 @@ static cudaError_t launch_groups(const PackGroups& groups, int B, Launch&& launc
 
 cudaError_t launch_pack_interleaved(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream) {
   return launch_groups(groups, B, [&](const PackGroups& some, int D) {
-    pack_interleaved_kernel<<<dim3((D + 31) / 32, n1p / 32, some.count * B), dim3(32, 8), 0, stream>>>(some, B, N1, n1p);
+    launch_next(pack_interleaved_kernel, dim3((D + 31) / 32, n1p / 32, some.count * B), dim3(32, 8), 0, stream, some, B, N1, n1p);
   });
 }
 
@@ -666,6 +674,7 @@ constexpr int PI_DB = 4;
 
 __global__ void __launch_bounds__(256)
 pack_interleaved_cf_kernel(const __grid_constant__ PackGroups groups, int B, int N1, int n1p) {
+  follow_previous_kernel();
   const int gi = blockIdx.z / B, b = blockIdx.z - gi * B;
   const PackGroup& g = groups.g[gi];
   const int p = blockIdx.x * 256 + threadIdx.x, d0 = blockIdx.y * PI_DB, D = g.D;
@@ -705,7 +714,7 @@ pack_interleaved_cf_kernel(const __grid_constant__ PackGroups groups, int B, int
 
 cudaError_t launch_pack_interleaved_cf(const PackGroups& groups, int B, int N1, int n1p, cudaStream_t stream) {
   return launch_groups(groups, B, [&](const PackGroups& some, int D) {
-    pack_interleaved_cf_kernel<<<dim3((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, some.count * B), 256, 0, stream>>>(some, B, N1, n1p);
+    launch_next(pack_interleaved_cf_kernel, dim3((n1p + 255) / 256, (D + PI_DB - 1) / PI_DB, some.count * B), 256, 0, stream, some, B, N1, n1p);
   });
 }
 
@@ -720,6 +729,7 @@ struct TransposeJobs {
 };
 __global__ void __launch_bounds__(256)
 transpose_round_kernel(const __grid_constant__ TransposeJobs jobs, int C, int op16) {
+  follow_previous_kernel();
   __shared__ float tile[64][33];
   int image = 0;
 #pragma unroll
@@ -762,6 +772,7 @@ struct MapCopies {
 __host__ __device__ inline int map_copy_channel(const MapCopy& c) { return c.blocked ? (c.width + 15) / 16 * c.pitch * 16 : c.pitch; }
 __global__ void __launch_bounds__(256)
 channel_major_cf_kernel(const __grid_constant__ MapCopies copies, int C, int op16) {
+  follow_previous_kernel();
   int ci = 0;
 #pragma unroll
   for (int i = 1; i < MAX_MAP_COPIES; ++i) ci = (int)blockIdx.x >= copies.first[i] ? i : ci;
@@ -809,7 +820,7 @@ cudaError_t launch_channel_major_cf(const MapCopy* copy, int count, int B, int C
     copies.first[i] = i < count ? blocks : INT_MAX;
     if (i < count) blocks += (map_copy_channel(copy[i]) / 2 + 256 * CM_PAIRS - 1) / (256 * CM_PAIRS);
   }
-  channel_major_cf_kernel<<<dim3(blocks, C, B), 256, 0, stream>>>(copies, C, op16);
+  launch_next(channel_major_cf_kernel, dim3(blocks, C, B), 256, 0, stream, copies, C, op16);
   return cudaGetLastError();
 }
 
@@ -823,6 +834,7 @@ __host__ __device__ inline int map_copy_columns(const MapCopy& c) { return c.blo
 __host__ __device__ inline int map_copy_rows(const MapCopy& c) { return c.blocked ? c.pitch : 1; }
 template <typename T>
 __global__ void channel_major_kernel(const MapCopy c1, const MapCopy c2, int blocks1, int C, int op16) {
+  follow_previous_kernel();
   __shared__ float tile[32][33];
   const bool first = (int)blockIdx.x < blocks1;
   const MapCopy& c = first ? c1 : c2;
@@ -850,8 +862,8 @@ __global__ void channel_major_kernel(const MapCopy c1, const MapCopy c2, int blo
 cudaError_t launch_channel_major(const MapCopy& c1, const MapCopy& c2, int B, int C, int op16, cudaStream_t stream) {
   auto blocks = [](const MapCopy& c) { return (map_copy_columns(c) + 31) / 32 * map_copy_rows(c); };
   const dim3 grid(blocks(c1) + blocks(c2), (C + 31) / 32, B), block(32, 8);
-  if (op16) channel_major_kernel<uint16_t><<<grid, block, 0, stream>>>(c1, c2, blocks(c1), C, op16);
-  else channel_major_kernel<float><<<grid, block, 0, stream>>>(c1, c2, blocks(c1), C, 0);
+  if (op16) launch_next(channel_major_kernel<uint16_t>, grid, block, 0, stream, c1, c2, blocks(c1), C, op16);
+  else launch_next(channel_major_kernel<float>, grid, block, 0, stream, c1, c2, blocks(c1), C, 0);
   return cudaGetLastError();
 }
 
@@ -896,7 +908,7 @@ cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, con
       jobs.j[1 + l] = TransposeJob{fmap2[l], out[l].F2r, out[l].F2h, scaled ? scales + l * SCALE_LEVEL + SCALE_F2 : nullptr, 1.f, d[l].N2()};
       blocks += (d[l].N2() + 31) / 32;
     }
-    transpose_round_kernel<<<dim3(blocks, (C + 63) / 64, B), dim3(32, 8), 0, stream>>>(jobs, C, op16);
+    launch_next(transpose_round_kernel, dim3(blocks, (C + 63) / 64, B), dim3(32, 8), 0, stream, jobs, C, op16);
   }
   if (out[0].aux != nullptr || out[0].auxh != nullptr) {
     MeansJobs jobs;
@@ -912,7 +924,7 @@ cudaError_t launch_prepare_cf(const Dims* d, int levels, const float* fmap1, con
                 : W2 <= 128 ? f2_means_cf_kernel<4>
                 : W2 <= 256 ? f2_means_cf_kernel<8>
                             : f2_means_cf_kernel<0>;
-    kern<<<dim3(C, B, levels), 256, 0, stream>>>(jobs, C, op16);
+    launch_next(kern, dim3(C, B, levels), 256, 0, stream, jobs, C, op16);
   }
   return cudaGetLastError();
 }
@@ -935,7 +947,8 @@ cudaError_t launch_prepare(const Dims& d, const float* F1, const float* F2, floa
   const int mean_rows = means ? d.H2 + d.W2 : 0;
   const long long grid = (long long)mean_rows * d.B + c1 + c2;
   if (grid > INT_MAX) return cudaErrorInvalidConfiguration;
-  round_means_kernel<<<(unsigned)grid, threads, 0, stream>>>(j1, j2, (int)c1, (int)c2, F2, aux, mean_rows, d.B, d.H2, d.W2, d.C, auxh, op16, s2);
+  launch_next(round_means_kernel, (unsigned)grid, threads, 0, stream, j1, j2, (int)c1, (int)c2, F2, aux, mean_rows, d.B, d.H2, d.W2, d.C, auxh,
+              op16, s2);
   return cudaGetLastError();
 }
 

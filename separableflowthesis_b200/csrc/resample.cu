@@ -8,6 +8,7 @@
 #include <climits>
 
 #include "kernels.h"
+#include "sm100_primitives.cuh"
 
 namespace sfb {
 
@@ -58,6 +59,7 @@ __device__ __forceinline__ void rs_store(float* p, const float4& v, int n) {
 template <bool VEC>
 __global__ void __launch_bounds__(RS_THREADS)
 upsample_displacement_kernel(const __grid_constant__ ResampleJobs jobs, int K, int N1) {
+  follow_previous_kernel();
   constexpr int DB = VEC ? RS_DB : RS_DB1;
   int ji = 0;
 #pragma unroll
@@ -105,6 +107,7 @@ struct ResampleAdjointJobs {
 template <bool CUT, int PX>
 __global__ void __launch_bounds__(RS_THREADS)
 upsample_displacement_adjoint_kernel(const __grid_constant__ ResampleAdjointJobs jobs, int K, int N1) {
+  follow_previous_kernel();
   int ji = 0;
 #pragma unroll
   for (int i = 1; i < MAX_RESAMPLE_JOBS; ++i) ji = (int)blockIdx.z >= jobs.first[i] ? i : ji;
@@ -202,7 +205,7 @@ cudaError_t launch_upsample_displacement(const ResampleJob* job, int count, int 
   }
   const dim3 grid((N1 + RS_THREADS * RS_PX - 1) / (RS_THREADS * RS_PX), rows, B * K);
   auto kern = vec ? upsample_displacement_kernel<true> : upsample_displacement_kernel<false>;
-  kern<<<grid, RS_THREADS, 0, st>>>(jobs, K, N1);
+  launch_next(kern, grid, RS_THREADS, 0, st, jobs, K, N1);
   return cudaGetLastError();
 }
 
@@ -224,7 +227,7 @@ cudaError_t launch_upsample_displacement_adjoint(const ResampleAdjointJob* job, 
   const int px = cut || (long long)blocks * B * K * count < RS_WIDE_FROM ? 1 : RS_PX;
   auto kern = cut ? upsample_displacement_adjoint_kernel<true, 1>
                   : (px == 1 ? upsample_displacement_adjoint_kernel<false, 1> : upsample_displacement_adjoint_kernel<false, RS_PX>);
-  kern<<<dim3((N1 + RS_THREADS * px - 1) / (RS_THREADS * px), B * K, pieces), RS_THREADS, 0, st>>>(jobs, K, N1);
+  launch_next(kern, dim3((N1 + RS_THREADS * px - 1) / (RS_THREADS * px), B * K, pieces), RS_THREADS, 0, st, jobs, K, N1);
   return cudaGetLastError();
 }
 

@@ -29,10 +29,19 @@ __device__ __forceinline__ void wait_ctl_init(WaitCtl* ctl, unsigned long long l
   ctl->abort_flag = 0;
   ctl->limit_ns = limit_ns != 0 ? limit_ns : WAIT_LIMIT_NS;
 }
+// Every kernel of the library begins with this (the ones with bounded waits in cta_has_work).  The host launches it while the kernel before it in the
+// stream may still be running (launch_next in kernels.h): its CTAs become resident where there is room and wait here, in hardware, until that
+// kernel is complete and its writes are visible.  Past the wait the next kernel may be launched in the same way; it in turn waits for this one.
+__device__ __forceinline__ void follow_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
 // Whether a wait of the launch has run out already, in which case a CTA that starts now does nothing.  One read for the whole
 // CTA (every thread calls it, before any barrier or register split is set up): CTAs that give up write the word at any time,
 // and warps that read it for themselves could part ways, some of them gone and the others waiting for them.
 __device__ __forceinline__ bool cta_has_work(const int* status) {
+  follow_previous_kernel();
   const int gave_up = threadIdx.x == 0 ? *reinterpret_cast<const volatile int*>(status) : 0;
   return __syncthreads_or(gave_up) == 0;
 }

@@ -841,6 +841,7 @@ sweep_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch, int* status) {
 constexpr int FOLD_ROWS = 4;
 template <int MODE, int LEVELS>
 __global__ void __launch_bounds__(TILE_M) sweep_fold_kernel(const __grid_constant__ SweepLaunch<LEVELS> launch) {
+  follow_previous_kernel();
   constexpr bool SUM = MODE == SWEEP_COMPRESS, ARG = MODE == SWEEP_MAXARGAVG;
   const int level = level_of<LEVELS>(launch.first_tail, blockIdx.y);
   const SweepArgs& a = launch.a[level];
@@ -997,11 +998,12 @@ static cudaError_t launch_one(SweepLaunch<LEVELS>& launch, int levels, cudaStrea
   }
   launch.first_block[LEVELS] = blocks;
   launch.first_tail[LEVELS] = tails;
-  kern<<<blocks, SW_THREADS, SW_SMEM_BYTES, stream>>>(launch, launch.a[0].status);
+  // kern<<<blocks, SW_THREADS, SW_SMEM_BYTES, stream>>>(launch, status), early
+  launch_next(kern, blocks, SW_THREADS, SW_SMEM_BYTES, stream, launch, launch.a[0].status);
   if constexpr (CUT) {
     if (tails == 0) return cudaGetLastError();
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    sweep_fold_kernel<MODE, LEVELS><<<dim3((rows + FOLD_ROWS - 1) / FOLD_ROWS, tails), TILE_M, 0, stream>>>(launch);
+    launch_next(sweep_fold_kernel<MODE, LEVELS>, dim3((rows + FOLD_ROWS - 1) / FOLD_ROWS, tails), TILE_M, 0, stream, launch);
   }
   return cudaGetLastError();
 }
