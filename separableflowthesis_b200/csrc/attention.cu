@@ -478,73 +478,124 @@ attention_logits_tiled_kernel(const __grid_constant__ TileMaps maps, const __gri
 }
 
 // ---- softmax over d, in place -------------------------------------------------------------------------------
-// A block owns 32 consecutive pixels of one (sample, channel); warp g takes displacements g, g + 8, ... and keeps its
-// V = ceil(D / 8) values in registers, so that every logit is read once and every weight written once (HBM-bound, all
+// A block owns 32 * VEC consecutive pixels of one (sample, channel); warp g takes displacements g, g + 8, ... and keeps its
+// V = ceil(D / 8) values of VEC pixels in registers, so that every logit is read once and every weight written once (HBM-bound, all
 // loads of a thread in flight together).  V = 0: any D, the values are read again in each of the three walks.  The
-// order of the sums depends on D only.  grid of ceil(N1/32) * planes (= B * Kc) blocks per job, block 256.
+// order of the sums depends on D only.  grid of ceil(N1/(32*VEC)) * planes (= B * Kc) blocks per job, block 256.
+// VEC: neighbouring pixels of a lane, moved by one access (planes of a multiple of VEC pixels, 16-byte aligned): with one, the
+// accesses' addresses and the two exchanges between warps cost as much as the data.  Inference at four levels, both
+// modules: 4 x 55 x 128 689 -> 678 us, 1 x 135 x 240 2384 -> 2357 (four pixels only up to V = 8: 682 and 2364).
 constexpr int SM_THREADS = SM_GROUPS * 32;
 struct SoftmaxJobs {
   JobBlocks blocks;
   float* a[MAX_ATTENTION_JOBS];
   int D[MAX_ATTENTION_JOBS];
 };
+template <int VEC> struct SoftmaxVec { float f[VEC]; };
+template <int VEC>
+__device__ __forceinline__ SoftmaxVec<VEC> load_pixels(const float* p) {
+  SoftmaxVec<VEC> v;
+  if constexpr (VEC == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v.f[0] = t.x; v.f[1] = t.y; v.f[2] = t.z; v.f[3] = t.w;
+  } else if constexpr (VEC == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    v.f[0] = t.x; v.f[1] = t.y;
+  } else {
+    v.f[0] = *p;
+  }
+  return v;
+}
+template <int VEC>
+__device__ __forceinline__ void store_pixels(float* p, const SoftmaxVec<VEC>& v) {
+  if constexpr (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v.f[0], v.f[1], v.f[2], v.f[3]);
+  else if constexpr (VEC == 2) *reinterpret_cast<float2*>(p) = make_float2(v.f[0], v.f[1]);
+  else *p = v.f[0];
+}
 
-template <int V>
-__global__ void __launch_bounds__(SM_THREADS, V == 0 ? 8 : (V <= 8 ? 6 : (V <= 20 ? 3 : 2)))
+template <int V, int VEC>
+__global__ void __launch_bounds__(SM_THREADS, V == 0 ? 8 : (V * VEC <= 8 ? 6 : (V * VEC <= 20 ? 3 : 2)))
 attention_softmax_kernel(const __grid_constant__ SoftmaxJobs jobs, int N1, unsigned pixel_blocks) {
   follow_previous_kernel();
-  __shared__ float red[2][SM_GROUPS][32];
+  __shared__ SoftmaxVec<VEC> red[2][SM_GROUPS][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int ji = job_of(jobs.blocks, blockIdx.x), D = jobs.D[ji];
   const unsigned block = blockIdx.x - jobs.blocks.first[ji], row = block / pixel_blocks;
-  const int p = (int)(block - row * pixel_blocks) * 32 + lane;
+  const int p = ((int)(block - row * pixel_blocks) * 32 + lane) * VEC;
   const bool in = p < N1;
   float* base = jobs.a[ji] + (size_t)row * D * N1 + (in ? p : 0);
   constexpr int NV = V > 0 ? V : 1;
-  float v[NV];
-  float m = -INFINITY;
+  SoftmaxVec<VEC> v[NV], m, l;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) m.f[j] = -INFINITY;
   if constexpr (V > 0) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const int d = g + i * SM_GROUPS;
-      v[i] = in && d < D ? base[(size_t)d * N1] : -INFINITY;
+      if (in && d < D) {
+        v[i] = load_pixels<VEC>(base + (size_t)d * N1);
+      } else {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) v[i].f[j] = -INFINITY;
+      }
     }
 #pragma unroll
-    for (int i = 0; i < V; ++i) m = fmaxf(m, v[i]);
+    for (int i = 0; i < V; ++i)
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) m.f[j] = fmaxf(m.f[j], v[i].f[j]);
   } else {
-    for (int d = g; d < D; d += SM_GROUPS) m = fmaxf(m, in ? base[(size_t)d * N1] : 0.f);
+    for (int d = g; d < D; d += SM_GROUPS) m.f[0] = fmaxf(m.f[0], in ? base[(size_t)d * N1] : 0.f);
   }
   red[0][g][lane] = m;
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < SM_GROUPS; ++i) m = fmaxf(m, red[0][i][lane]);
-  float l = 0.f;
+  for (int i = 0; i < SM_GROUPS; ++i) {
+    const SoftmaxVec<VEC> other = red[0][i][lane];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) m.f[j] = fmaxf(m.f[j], other.f[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) l.f[j] = 0.f;
   if constexpr (V > 0) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       if (g + i * SM_GROUPS < D) {
-        v[i] = __expf(v[i] - m);
-        l += v[i];
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+          v[i].f[j] = __expf(v[i].f[j] - m.f[j]);
+          l.f[j] += v[i].f[j];
+        }
       }
     }
   } else {
-    for (int d = g; d < D; d += SM_GROUPS) l += __expf((in ? base[(size_t)d * N1] : 0.f) - m);
+    for (int d = g; d < D; d += SM_GROUPS) l.f[0] += __expf((in ? base[(size_t)d * N1] : 0.f) - m.f[0]);
   }
   red[1][g][lane] = l;
   __syncthreads();
-  l = 0.f;
 #pragma unroll
-  for (int i = 0; i < SM_GROUPS; ++i) l += red[1][i][lane];
-  const float inv = 1.f / l;
+  for (int j = 0; j < VEC; ++j) l.f[j] = 0.f;
+#pragma unroll
+  for (int i = 0; i < SM_GROUPS; ++i) {
+    const SoftmaxVec<VEC> other = red[1][i][lane];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) l.f[j] += other.f[j];
+  }
+  SoftmaxVec<VEC> inv;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) inv.f[j] = 1.f / l.f[j];
   if (!in) return;
   if constexpr (V > 0) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const int d = g + i * SM_GROUPS;
-      if (d < D) base[(size_t)d * N1] = v[i] * inv;
+      if (d < D) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) v[i].f[j] *= inv.f[j];
+        store_pixels<VEC>(base + (size_t)d * N1, v[i]);
+      }
     }
   } else {
-    for (int d = g; d < D; d += SM_GROUPS) base[(size_t)d * N1] = __expf(base[(size_t)d * N1] - m) * inv;
+    for (int d = g; d < D; d += SM_GROUPS) base[(size_t)d * N1] = __expf(base[(size_t)d * N1] - m.f[0]) * inv.f[0];
   }
 }
 
@@ -1320,11 +1371,11 @@ size_t attention_partial_floats(const AttentionDims* d, int count) {
 }
 
 // Columns of a class of lengths are done by one launch.
-template <int V>
-static cudaError_t launch_softmax_class(const AttentionJob* job, int count, int above, int upto, cudaStream_t st) {
+template <int V, int VEC>
+static cudaError_t launch_softmax_jobs(const AttentionJob* job, int count, int above, int upto, cudaStream_t st) {
   SoftmaxJobs jobs{};
   const AttentionDims& d = job[0].d;
-  const unsigned pb = (unsigned)((d.H1 * d.W1 + 31) / 32);
+  const unsigned pb = (unsigned)((d.H1 * d.W1 + 32 * VEC - 1) / (32 * VEC));
   unsigned long long blocks = 0;
   int n = 0;
   for (int i = 0; i < count; ++i) {
@@ -1338,8 +1389,22 @@ static cudaError_t launch_softmax_class(const AttentionJob* job, int count, int 
   }
   if (n == 0) return cudaSuccess;
   for (; n <= MAX_ATTENTION_JOBS; ++n) jobs.blocks.first[n] = (int)blocks;
-  launch_next(attention_softmax_kernel<V>, (unsigned)blocks, SM_THREADS, 0, st, jobs, d.H1 * d.W1, pb);
+  launch_next(attention_softmax_kernel<V, VEC>, (unsigned)blocks, SM_THREADS, 0, st, jobs, d.H1 * d.W1, pb);
   return cudaGetLastError();
+}
+// Pixels of a lane: as many as the values of a thread leave registers for (128 of them, two blocks per SM), in launches that
+// have a block for every SM all the same.  Two at V <= 32 spill and gained nothing over one.
+template <int V>
+static cudaError_t launch_softmax_class(const AttentionJob* job, int count, int above, int upto, cudaStream_t st) {
+  constexpr int VEC = V == 0 || V > 24 ? 1 : (V <= 16 ? 4 : 2);
+  if constexpr (VEC > 1) {
+    const AttentionDims& d = job[0].d;
+    const long long N1 = (long long)d.H1 * d.W1;
+    bool wide = N1 % VEC == 0 && N1 / (32 * VEC) * d.B * d.Kc >= SM_COUNT;
+    for (int i = 0; i < count; ++i) wide = wide && (reinterpret_cast<uintptr_t>(job[i].a) & 15u) == 0;
+    if (wide) return launch_softmax_jobs<V, VEC>(job, count, above, upto, st);
+  }
+  return launch_softmax_jobs<V, 1>(job, count, above, upto, st);
 }
 static int softmax_class(int D) {   // largest values per warp of a class; 0: any
   const int v = (D + SM_GROUPS - 1) / SM_GROUPS;
