@@ -19,8 +19,8 @@
 // Backward (features only: the model detaches the coordinates, core/sepflow.py:193): the gradient of a pixel's window is
 // spread back onto the integer positions (each takes from at most four window entries); gF1 is the sum over positions of
 // that times the image-2 row, gF2 of a position the sum over pixels of the same times the pixel's row.  The channel is a
-// free index of both, so a lane owns one channel for all pixels of a 4 x 4 tile, and the box of all their windows is
-// walked once: an image-2 row is read, and reduced into L2, once per tile.  Tiles whose windows lie too far apart take
+// free index of both, so a lane owns two channels for all pixels of a 4 x 4 tile, and the box of all their windows is
+// walked once: an image-2 row is read, and reduced into L2, once per tile and level.  Tiles whose windows lie too far apart take
 // the forward's walks, with one 16-byte vector reduction per lane (red.global.add.v4.f32) and position.
 #include <algorithm>
 #include <climits>
@@ -285,14 +285,16 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
 // ---- backward ---------------------------------------------------------------------------------------------
 constexpr int L4_BT = 4;                        // tile of 4 x 4 pixels
 constexpr int L4_BPX = L4_BT * L4_BT;
+constexpr int L4_BCH = 256;                      // channels of a CTA, two a lane
 constexpr int L4_BBOX = 384;                    // positions of the largest box walked for the whole tile
-constexpr int L4_BTHREADS = 256, L4_BWARPS = L4_BTHREADS / 32;
-// Largest box of a tile for windows of a radius.  A level of a whole tile takes 1.2 us per position plus 35, where four walks of 2 x 2 pixels take
+constexpr int L4_BTHREADS = 128, L4_BWARPS = L4_BTHREADS / 32;
+// Largest box of a tile for windows of a radius.  A level of a whole tile took 1.2 us per position plus 35 (a tenth less since), where four walks of 2 x 2 pixels take
 // 0.85 (2 x 55 x 128, C = 256); those have (2r + 3)^2 positions each in a smooth field and (2r + 4)^2 or more where the tile's box is near the
 // limit: radius 4 382, 3 256, 2 153.  With (2r + 3)^2 a field with noise of half a pixel took 337 us at radius 3, 2 x 2 pixels alone 299, 220 with
 // this.  Radius 1 and 0 walk 2 x 2 pixels only.
 inline int l4_tile_limit(int radius) { return radius < 2 ? 0 : std::min(L4_BBOX, (4 * (2 * radius + 4) * (2 * radius + 4) - 41) * 5 / 7); }
-static_assert(L4_BTHREADS <= L4_BBOX && L4_BBOX % 4 == 0, "partial sums of warps that share channels; steps of four positions");
+static_assert(2 * L4_BTHREADS <= L4_BBOX && L4_BBOX % 4 == 0, "partial sums of warps that share channels; steps of four positions");
+static_assert(L4_BCH == L4_BWARPS * 64, "a warp has 64 channels");
 
 __device__ __forceinline__ void red_add_v4(float* addr, uint64_t lo, uint64_t hi) {
   float x, y, z, w;
@@ -431,13 +433,43 @@ __device__ __forceinline__ void l4_nonfinite(const float (*gS)[L4_BPX], const in
   }
 }
 
-// Every CTA walks all levels of its tile, so that gF1 is stored once.  Warp w owns channels 32 (w % groups) .. of the CTA's 256; warps
-// beyond the channels share out the positions.  Bound by FP32 issue: 32 multiply-adds of some 45 instructions per warp and position (packed
-// pairs with three different operands take 3 cycles, no gain over two scalar ones).  With a walk per 2 x 2 pixels, lanes splitting
-// the channels, each walk reduced its own 140 positions of 1 KB into L2: 2 x 55 x 128 pixels at C = 256, four levels, radius 4 took 416 us;
-// 278 now.
-// grid (ceil(W1/4) * ceil(H1/4), ceil(C/256), B)
-__global__ void __launch_bounds__(L4_BTHREADS, 2)
+// The levels of a tile are done by two CTAs, the pairs 0 and 3, 1 and 2 (and so on) about alike in length.
+__host__ __device__ constexpr int l4_parts(int levels) { return levels > 1 ? 2 : 1; }
+__device__ __forceinline__ int l4_part(int level) { return (level + 1) >> 1 & 1; }
+
+// A lane's CH consecutive channels.
+template <int CH> struct L4Channels { float f[CH]; };
+template <int CH>
+__device__ __forceinline__ L4Channels<CH> l4_load_channels(const float* p) {
+  L4Channels<CH> v;
+  if constexpr (CH == 2) {
+    const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+    v.f[0] = t.x;
+    v.f[1] = t.y;
+  } else {
+    v.f[0] = __ldg(p);
+  }
+  return v;
+}
+template <int CH>
+__device__ __forceinline__ void l4_add_channels(float* p, const float (&v)[CH]) {
+  if constexpr (CH == 2) asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v[0]), "f"(v[1]) : "memory");
+  else atomicAdd(p, v[0]);
+}
+
+// A CTA walks half the levels of its tile; gF1 is cleared and the two sums added to it (either order gives the same bits; one level: stored).
+// Warp w owns channels 32 CH (w % groups) .. of the CTA's 256; warps beyond the channels share out the positions.  Bound by FP32 issue: 32
+// multiply-adds per channel and position at 1.3 cycles or so (packed pairs with three different operands take 3 cycles, no gain over two
+// scalar ones).  CH: a gradient's 16 bytes come back to 32 lanes at 128 bytes a cycle and SM, so with one channel a lane shared memory
+// took 16 cycles of a position where the multiply-adds take 11; with two they serve twice the products (one where there are no more than 32
+// channels).  Three CTAs: 128 registers for four spill (2 x 55 x 128 pixels at C = 256, four levels, radius 4: 315 us).
+// Two CTAs a tile: tiles alone, as in the last wave, left an SM with four warps (1 x 60 x 160: 1429 -> 1369 us for four
+// iterations forward and backward, with one channel and 8 warps a tile 1385).
+// With a walk per 2 x 2 pixels, lanes splitting the channels, each walk reduced its own 140 positions of 1 KB into L2: the first size took
+// 416 us; 280 with one channel a lane, 252 now.
+// grid (ceil(W1/4) * ceil(H1/4), ceil(C/256) * l4_parts, B)
+template <int CH>
+__global__ void __launch_bounds__(L4_BTHREADS, 3)
 lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                          const float* __restrict__ gout, float* __restrict__ gF1, int H1, int W1, int C, int radius,
                          int levels, int limit, float scale) {
@@ -460,20 +492,28 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
   const bool in = lane < L4_BPX && h0 + lane / L4_BT < H1 && w0 + lane % L4_BT < W1;
   const unsigned mask = __ballot_sync(0xffffffffu, in);
   const size_t tile = ((size_t)b * N1 + (size_t)h0 * W1 + w0) * C;
-  const int c0 = (int)blockIdx.y * L4_BTHREADS, groups = min(L4_BWARPS, (C - c0 + 31) / 32), sharers = L4_BWARPS / groups;
-  const int c = c0 + w % groups * 32 + lane, share = w / groups;
+  constexpr int WARP_CH = 32 * CH;
+  const int parts = l4_parts(levels), part = (int)blockIdx.y % parts;
+  const int c0 = (int)blockIdx.y / parts * L4_BCH, groups = min(L4_BWARPS, (C - c0 + WARP_CH - 1) / WARP_CH), sharers = L4_BWARPS / groups;
+  const int c = c0 + w % groups * WARP_CH + lane * CH, share = w / groups;
   const bool mine = c < C && share < sharers;
-  float f1[L4_BPX], gf1[L4_BPX];
+  float f1[CH][L4_BPX], gf1[CH][L4_BPX];
   bool finite1 = true;
 #pragma unroll
   for (int px = 0; px < L4_BPX; ++px) {
     const bool ok = mine && h0 + px / L4_BT < H1 && w0 + px % L4_BT < W1;
-    f1[px] = ok ? __ldg(F1 + tile + ((size_t)(px / L4_BT) * W1 + px % L4_BT) * C + c) : 0.f;
-    finite1 &= isfinite(f1[px]);
-    gf1[px] = 0.f;
+    L4Channels<CH> v{};
+    if (ok) v = l4_load_channels<CH>(F1 + tile + ((size_t)(px / L4_BT) * W1 + px % L4_BT) * C + c);
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      f1[k][px] = v.f[k];
+      finite1 &= isfinite(v.f[k]);
+      gf1[k][px] = 0.f;
+    }
   }
   if (!l4_tile(s_tile, coords, lv, levels, b, h0, w0, H1, W1, radius, limit)) return;   // lookup4d_backward_apart_kernel does it
   for (int level = 0; level < levels; ++level) {
+    if (parts > 1 && l4_part(level) != part) continue;
     const int H2 = lv.H2[level], W2 = lv.W2[level];
     const L4Box box = s_tile.box[level];
     const int nq = box.bw * box.bh;
@@ -560,46 +600,56 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
     const char* const F2c = reinterpret_cast<const char*>(lv.f2[level] + (size_t)b * H2 * W2 * C + c);
     char* const G2c = reinterpret_cast<char*>(lv.g2[level] + (size_t)b * H2 * W2 * C + c);
     const uint32_t row_bytes = 4 * C;
-    const auto f2_at = [&](int r) { return __ldg(reinterpret_cast<const float*>(F2c + (uint64_t)row_bytes * (uint32_t)r)); };
-    const auto add_at = [&](int r, float v) { atomicAdd(reinterpret_cast<float*>(G2c + (uint64_t)row_bytes * (uint32_t)r), v); };
+    const auto f2_row = [&](int r) { return reinterpret_cast<const float*>(F2c + (uint64_t)row_bytes * (uint32_t)r); };
+    const auto g2_row = [&](int r) { return reinterpret_cast<float*>(G2c + (uint64_t)row_bytes * (uint32_t)r); };
     // four positions a step; the next step's rows are requested before this one's are used
     int next_r[4];
-    float next_f[4];
+    L4Channels<CH> next_f[4];
     const auto fetch = [&](int q0) {
       if (q0 >= padded) return;
       *reinterpret_cast<int4*>(next_r) = *reinterpret_cast<const int4*>(&s_rows[q0]);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) next_f[k] = f2_at(next_r[k]);
+      for (int k = 0; k < 4; ++k) next_f[k] = l4_load_channels<CH>(f2_row(next_r[k]));
     };
     fetch(share * 4);
 #pragma unroll 2
     for (int q0 = share * 4; q0 < padded; q0 += sharers * 4) {
       int r[4];
-      float f[4];
+      L4Channels<CH> f[4];
+      float magnitude = 0.f;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         r[k] = next_r[k];
         f[k] = next_f[k];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) magnitude += fabsf(f[k].f[i]);
       }
       fetch(q0 + sharers * 4);
-      if (!finite1 || !isfinite((fabsf(f[0]) + fabsf(f[1])) + (fabsf(f[2]) + fabsf(f[3])))) {
-        l4_nonfinite(s_gS, s_rows, q0, f1, gf1, f2_at, add_at);
+      if (!finite1 || !isfinite(magnitude)) {
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+          l4_nonfinite(s_gS, s_rows, q0, f1[i], gf1[i], [&](int at) { return __ldg(f2_row(at) + i); },
+                       [&](int at, float v) { atomicAdd(g2_row(at) + i, v); });
         continue;
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        float g2[4];
+        float g2[CH][4], total[CH];
 #pragma unroll
         for (int p4 = 0; p4 < L4_BPX; p4 += 4) {
           const float4 t = *reinterpret_cast<const float4*>(&s_gS[q0 + k][p4]);
           const float g[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            gf1[p4 + i] = fmaf(g[i], f[k], gf1[p4 + i]);
-            g2[i] = p4 == 0 ? g[i] * f1[i] : fmaf(g[i], f1[p4 + i], g2[i]);
-          }
+          for (int j = 0; j < CH; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              gf1[j][p4 + i] = fmaf(g[i], f[k].f[j], gf1[j][p4 + i]);
+              g2[j][i] = p4 == 0 ? g[i] * f1[j][i] : fmaf(g[i], f1[j][p4 + i], g2[j][i]);
+            }
         }
-        add_at(r[k], (g2[0] + g2[1]) + (g2[2] + g2[3]));
+#pragma unroll
+        for (int j = 0; j < CH; ++j) total[j] = (g2[j][0] + g2[j][1]) + (g2[j][2] + g2[j][3]);
+        l4_add_channels<CH>(g2_row(r[k]), total);
       }
     }
   }
@@ -607,19 +657,34 @@ lookup4d_backward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const 
     __syncthreads();
     if (mine && share > 0) {
 #pragma unroll
-      for (int px = 0; px < L4_BPX; ++px) s_gS[threadIdx.x][px] = gf1[px];
+      for (int j = 0; j < CH; ++j)
+#pragma unroll
+        for (int px = 0; px < L4_BPX; ++px) s_gS[threadIdx.x + j * L4_BTHREADS][px] = gf1[j][px];
     }
     __syncthreads();
     if (mine && share == 0) {
       for (int k = 1; k < sharers; ++k)
 #pragma unroll
-        for (int px = 0; px < L4_BPX; ++px) gf1[px] += s_gS[threadIdx.x + k * groups * 32][px];
+        for (int j = 0; j < CH; ++j)
+#pragma unroll
+          for (int px = 0; px < L4_BPX; ++px) gf1[j][px] += s_gS[threadIdx.x + k * groups * 32 + j * L4_BTHREADS][px];
     }
   }
   if (mine && share == 0) {
 #pragma unroll
     for (int px = 0; px < L4_BPX; ++px)
-      if (h0 + px / L4_BT < H1 && w0 + px % L4_BT < W1) gF1[tile + ((size_t)(px / L4_BT) * W1 + px % L4_BT) * C + c] = gf1[px];
+      if (h0 + px / L4_BT < H1 && w0 + px % L4_BT < W1) {
+        float* const dst = gF1 + tile + ((size_t)(px / L4_BT) * W1 + px % L4_BT) * C + c;
+        float sum[CH];
+#pragma unroll
+        for (int j = 0; j < CH; ++j) sum[j] = gf1[j][px];
+        if (parts > 1) {
+          l4_add_channels<CH>(dst, sum);
+        } else {
+#pragma unroll
+          for (int j = 0; j < CH; ++j) dst[j] = sum[j];
+        }
+      }
   }
 }
 
@@ -731,11 +796,15 @@ lookup4d_backward_apart_kernel(const float* __restrict__ F1, Lookup4dLevels lv, 
     }
 }
 
-// Zeros for the reductions, all levels in one launch (C is a multiple of 4 and the pointers are 16-byte aligned).
-__global__ void __launch_bounds__(256) lookup4d_clear_kernel(Lookup4dLevels lv, int B, int C) {
+// Zeros for the reductions, all arrays in one launch (C is a multiple of 4 and the pointers are 16-byte aligned).
+struct L4Clear {
+  float* p[LOOKUP_MAX_LEVELS + 1];
+  size_t quads[LOOKUP_MAX_LEVELS + 1];
+};
+__global__ void __launch_bounds__(256) lookup4d_clear_kernel(L4Clear clear) {
   follow_previous_kernel();
-  float4* const p = reinterpret_cast<float4*>(lv.g2[blockIdx.y]);
-  const size_t n = (size_t)B * lv.H2[blockIdx.y] * lv.W2[blockIdx.y] * (C / 4);
+  float4* const p = reinterpret_cast<float4*>(clear.p[blockIdx.y]);
+  const size_t n = clear.quads[blockIdx.y];
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
@@ -780,16 +849,24 @@ cudaError_t launch_lookup4d_backward(const Lookup4dDims& d, const float* F1, con
                                      const float* coords, const float* gout, float* gF1, float* const* gF2,
                                      float scale, cudaStream_t stream) {
   const Lookup4dLevels lv = make_levels(d, F2, gF2);
+  const int limit = l4_tile_limit(d.radius), parts = l4_parts(d.levels);
+  L4Clear clear{};
+  int arrays = 0;
   size_t largest = 0;
-  for (int l = 0; l < d.levels; ++l) largest = std::max(largest, (size_t)d.B * d.H2[l] * d.W2[l] * (d.C / 4));
-  launch_next(lookup4d_clear_kernel, dim3((unsigned)std::min<size_t>((largest + 1023) / 1024, 148 * 8), d.levels), 256, 0, stream, lv, d.B, d.C);
+  const auto add = [&](float* p, size_t quads) {
+    clear.p[arrays] = p;
+    clear.quads[arrays++] = quads;
+    largest = std::max(largest, quads);
+  };
+  for (int l = 0; l < d.levels; ++l) add(gF2[l], (size_t)d.B * d.H2[l] * d.W2[l] * (d.C / 4));
+  if (limit > 0 && parts > 1) add(gF1, (size_t)d.B * d.H1 * d.W1 * (d.C / 4));
+  launch_next(lookup4d_clear_kernel, dim3((unsigned)std::min<size_t>((largest + 1023) / 1024, 148 * 8), arrays), 256, 0, stream, clear);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const dim3 grid((unsigned)((d.W1 + L4_BT - 1) / L4_BT) * (unsigned)((d.H1 + L4_BT - 1) / L4_BT), 1, d.B);   // per tile
-  const int limit = l4_tile_limit(d.radius);
   if (limit > 0) {
-    const dim3 whole(grid.x, (unsigned)((d.C + L4_BTHREADS - 1) / L4_BTHREADS), d.B);
-    launch_next(lookup4d_backward_kernel, whole, L4_BTHREADS, 0, stream, F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale);
+    const dim3 whole(grid.x, (unsigned)((d.C + L4_BCH - 1) / L4_BCH * parts), d.B);
+    launch_next(d.C > 32 ? lookup4d_backward_kernel<2> : lookup4d_backward_kernel<1>, whole, L4_BTHREADS, 0, stream, F1, lv, coords, gout, gF1, d.H1, d.W1, d.C, d.radius, d.levels, limit, scale);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
