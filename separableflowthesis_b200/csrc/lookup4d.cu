@@ -13,7 +13,7 @@
 // mostly overlap because neighbouring pixels move alike, visits the bounding box of their windows once, and uses every
 // loaded image-2 row for all of them (their feature rows in registers, lanes split the channels).  Partial sums of 32
 // (position, pixel) pairs are reduced together with a 31-shuffle transpose.  When the windows lie far apart (a motion
-// boundary) the walk is done for fewer pixels at a time.  A CTA covers 8 x 4 pixels and stages its outputs in shared
+// boundary) the walk is done for fewer pixels at a time.  A CTA covers 8 x 2 pixels and stages its outputs in shared
 // memory, so that the (B, levels*(2r+1)^2, H1, W1) result is written in runs of eight pixels (a 32-byte sector).
 //
 // Backward (features only: the model detaches the coordinates, core/sepflow.py:193): the gradient of a pixel's window is
@@ -30,12 +30,11 @@
 
 namespace sfb {
 
-constexpr int L4_TW = 8, L4_TH = 4;            // image-1 pixels of a CTA: two-dimensional, so that windows overlap
+constexpr int L4_TW = 8, L4_TH = 2;            // image-1 pixels of a CTA: two-dimensional, so that windows overlap
 constexpr int L4_TILE = L4_TW * L4_TH;
 constexpr int L4_RMAX = 4;
 constexpr int L4_WIN = 2 * L4_RMAX + 1;        // window side
 constexpr int L4_SIDE = 2 * L4_RMAX + 2;       // integer positions under a window, per side
-static_assert(L4_TILE == 32, "the output staging assumes 32 pixels per CTA");
 
 struct Lookup4dLevels {
   const float* f2[LOOKUP_MAX_LEVELS];   // level l: (B, H2_l, W2_l, C)
@@ -138,12 +137,13 @@ __device__ __forceinline__ void l4_fill_rows(int* rows, const L4Box& box, int H2
 }
 
 // ---- forward ----------------------------------------------------------------------------------------------
-// A CTA owns 8 x 4 pixels at one level, a warp 2 x 2 of them: one walk over the box of their windows with the four
+// A CTA owns 8 x 2 pixels at one level, a warp 2 x 2 of them: one walk over the box of their windows with the four
 // pixels' feature rows in registers (lanes split the channels).  Bound by instruction issue: the products are packed
 // pairs and the positions come from a table.
-constexpr int L4_THREADS = 256;
+constexpr int L4_THREADS = 128;
 constexpr int L4_WARPS = L4_THREADS / 32;
 constexpr int L4_PX = 4;
+static_assert(L4_TW == 2 * L4_WARPS && L4_TH == 2, "2 x 2 pixels a warp");
 constexpr int L4_BMAX = 224;                   // largest box a four-pixel walk accepts
 static_assert(L4_SIDE * L4_SIDE <= L4_BMAX && L4_BMAX % 32 == 0, "one pixel's positions must fit the table");
 
@@ -189,10 +189,11 @@ __device__ __forceinline__ void l4_box_products(const L4Quad (&f1)[NPX][NQ], con
 }
 
 // Two packed multiply-adds per 4 channels, pixel and position, and the reductions, bound the forward: 2 x 55 x 128 at C = 256, four
-// levels, radius 4 takes 172 us with 32 lanes a position, 148 with 16.
-// grid (ceil(W1/8) * ceil(H1/4), levels, B)
+// levels, radius 4 takes 172 us with 32 lanes a position, 148 with 16.  Four CTAs of 8 x 2 pixels per SM instead of two of 8 x 4 wait for less
+// at their ends and beginnings: six of them 951 -> 912 us (1 x 60 x 160 664 -> 638; 4 x 4 pixels 936 and 652).
+// grid (ceil(W1/8) * ceil(H1/2), levels, B)
 template <int NQ, int LP, bool FULL>
-__global__ void __launch_bounds__(L4_THREADS, 2)
+__global__ void __launch_bounds__(L4_THREADS, 4)
 lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const float* __restrict__ coords,
                         float* __restrict__ out, int H1, int W1, int C, int radius, int levels, float scale) {
   follow_previous_kernel();
@@ -209,8 +210,8 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
   const int tiles_x = (W1 + L4_TW - 1) / L4_TW;
   const int h0 = (int)(blockIdx.x / tiles_x) * L4_TH, w0 = (int)(blockIdx.x % tiles_x) * L4_TW;
   const int win = 2 * radius + 1;
-  // warp w: columns 2*(w%4) .., rows 2*(w/4) .. of the tile; its pixel px: column px%2, row px/2
-  const int ph = h0 + 2 * (w >> 2), pw = w0 + 2 * (w & 3);
+  // warp w: columns 2*w, 2*w + 1 of the tile; its pixel px: column px%2, row px/2
+  const int ph = h0, pw = w0 + 2 * w;
 
   L4Pixel geo{0.f, 0.f, 0, 0};
   const int mh = ph + ((lane >> 1) & 1), mw = pw + (lane & 1);
@@ -272,7 +273,7 @@ lookup4d_forward_kernel(const float* __restrict__ F1, Lookup4dLevels lv, const f
       const float* S = s_S[w][px] + (g.y + bb - radius - oy) * sbw + (g.x + a - radius - ox);
       const float top = S[0] + fx * (S[1] - S[0]);
       const float bot = S[sbw] + fx * (S[sbw + 1] - S[sbw]);
-      s_out[o][(2 * (w >> 2) + px / 2) * L4_TW + 2 * (w & 3) + px % 2] = top + fy * (bot - top);
+      s_out[o][px / 2 * L4_TW + 2 * w + px % 2] = top + fy * (bot - top);
     }
   }
   __syncthreads();
