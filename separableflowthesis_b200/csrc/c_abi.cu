@@ -543,10 +543,10 @@ cudaError_t prepare_operands(const Dims& d, const Workspace& w, const Features& 
   return f.fmaps ? launch_prepare_cf(&d, 1, f.F1, &f.F2, f.scale1, &out, F1r, F1h, w.status, st, op16, w.scales)
                  : launch_prepare(d, f.F1, f.F2, F1r, F2r, aux, w.status, st, F1h, F2h, auxh, op16, w.scales);
 }
-// Launches of the above: FP16 operands add the search for the magnitudes; pixel-major features have copies and mean rows in one.
+// Launches of the above: the header is cleared; FP16 operands add the search for the magnitudes; pixel-major features have copies and mean rows in one.
 int prepare_launches(const Workspace& w, bool fmaps, bool with_aux, int op16) {
   const bool copies = !op16 || w.F1h != nullptr;
-  return (fmaps ? (copies ? 1 : 0) + (with_aux ? 1 : 0) : (copies || with_aux ? 1 : 0)) + (op16 == OP16_FP16 ? 1 : 0);
+  return 1 + (fmaps ? (copies ? 1 : 0) + (with_aux ? 1 : 0) : (copies || with_aux ? 1 : 0)) + (op16 == OP16_FP16 ? 1 : 0);
 }
 #define SFB_PREPARE(f, with_aux) \
   SFB_CUDA(timed(KID_PREPARE, prepare_launches(w, (f).fmaps, with_aux, (f).op16), st, [&] { return prepare_operands(d, w, f, with_aux, st); }))

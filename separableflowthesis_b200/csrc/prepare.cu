@@ -867,8 +867,15 @@ cudaError_t launch_channel_major(const MapCopy& c1, const MapCopy& c2, int B, in
   return cudaGetLastError();
 }
 
+// Zeros for the workspace header.  A kernel: launches wait for a memory operation as a whole, with the device idle on either side of it (drop-in
+// operators 2 x 48 x 64, four calls, 387 -> 375 us, infer 1 x 55 x 128 238 -> 236).  grid 1, block 32.
+__global__ void __launch_bounds__(32) clear_header_kernel(int* words, int n) {
+  follow_previous_kernel();
+  for (int i = threadIdx.x; i < n; i += 32) words[i] = 0;
+}
 static cudaError_t clear_header(int levels, int* status, cudaStream_t stream) {
-  return cudaMemsetAsync(status, 0, WS_SCALES_OFFSET + (size_t)levels * SCALE_LEVEL * sizeof(float), stream);
+  launch_next(clear_header_kernel, 1, 32, 0, stream, status, (int)(WS_SCALES_OFFSET / sizeof(int)) + levels * SCALE_LEVEL);
+  return cudaGetLastError();
 }
 // Clears the workspace header (status word, scale slots) and, for FP16 operands, finds the feature scales.
 static cudaError_t begin_prepare(const Dims* d, int levels, const float* F1, const float* const* F2, float premul1, int* status, int op16,
