@@ -506,13 +506,15 @@ f2_means_cf_kernel(const __grid_constant__ MeansJobs jobs, int C, int op16) {
 }
 
 // Tiled transposes between the reference's per-pixel layout (B, N1, K, D) (displacement d fastest) and the
-// packed layout (B, D, R, n1p) (pixel fastest) the kernels use.  A block moves a patch of 128 pixels x 32
+// packed layout (B, D, R, n1p) (pixel fastest) the kernels use.  A block moves a patch of 128 pixels (PX) x 32
 // displacements through shared memory so that both sides are coalesced; every thread keeps 16 loads in flight,
 // and the displacement tiles are the fastest so that blocks running together read neighbouring
 // 128-byte pieces of the same rows.  One launch for all tensors of a call (a launch of a small one is mostly latency: the four outputs of
 // 2 x 48 x 64 took 31 us in four launches, 10 in one).
-// grid: ceil(D/32) * n1p/128 * B*K blocks per tensor, block (32, 8).
-constexpr int PACK_PX = 128;
+// Launches of less than four such blocks per SM move 32 pixels a block: they are over sooner than a block's instructions for sixteen loads and stores
+// have been fetched (drop-in operators 2 x 48 x 64, three conversions and two packs, 365 -> 349 us; up to 16 blocks per SM
+// 4 x 48 x 64 with three channels takes 577 instead of 562).
+// grid: ceil(D/32) * n1p/PX * B*K blocks per tensor, block (32, 8).
 struct PatchJobs {
   PatchJob j[MAX_PATCH_JOBS];
   int first[MAX_PATCH_JOBS];   // blocks; tensors that do not exist start past the end of the grid
@@ -520,26 +522,28 @@ struct PatchJobs {
 struct Patch {
   int b, k, d0, p0;
 };
+template <int PX>
 __device__ __forceinline__ Patch patch_of(const PatchJobs& jobs, int n1p, int& job) {
   job = 0;
 #pragma unroll
   for (int i = 1; i < MAX_PATCH_JOBS; ++i) job = (int)blockIdx.x >= jobs.first[i] ? i : job;
   const PatchJob& j = jobs.j[job];
-  const int r = blockIdx.x - jobs.first[job], nd = (j.D + 31) / 32, np = n1p / PACK_PX;
+  const int r = blockIdx.x - jobs.first[job], nd = (j.D + 31) / 32, np = n1p / PX;
   const int q = r / nd, z = q / np, b = z / j.K;
-  return Patch{b, z - b * j.K, (r - q * nd) * 32, (q - z * np) * PACK_PX};
+  return Patch{b, z - b * j.K, (r - q * nd) * 32, (q - z * np) * PX};
 }
 
-__global__ void pack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
+template <int PX>
+__global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
   follow_previous_kernel();
-  __shared__ uint32_t tile[PACK_PX][33];
+  __shared__ uint32_t tile[PX][33];
   int ji;
-  const Patch t = patch_of(jobs, n1p, ji);
+  const Patch t = patch_of<PX>(jobs, n1p, ji);
   const PatchJob& j = jobs.j[ji];
   const int tx = threadIdx.x, ty = threadIdx.y, D = j.D;
   const uint32_t* src = static_cast<const uint32_t*>(j.pixels) + (((size_t)t.b * N1 + t.p0) * j.Kpix + j.k0 + t.k) * D + t.d0 + tx;
 #pragma unroll
-  for (int i = ty; i < PACK_PX; i += 8) {
+  for (int i = ty; i < PX; i += 8) {
     uint32_t v = 0;
     if (t.p0 + i < N1 && t.d0 + tx < D) v = __ldg(src + (size_t)i * j.Kpix * D);
     tile[i][tx] = v;
@@ -547,51 +551,60 @@ __global__ void pack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int 
   __syncthreads();
   uint32_t* dst = reinterpret_cast<uint32_t*>(j.packed) + (((size_t)t.b * D + t.d0) * j.R + j.r0 + t.k) * n1p + t.p0;
 #pragma unroll
-  for (int i = ty; i < 32 * (PACK_PX / 32); i += 8) {
-    const int d = i / (PACK_PX / 32), p = (i % (PACK_PX / 32)) * 32 + tx;
+  for (int i = ty; i < 32 * (PX / 32); i += 8) {
+    const int d = i / (PX / 32), p = (i % (PX / 32)) * 32 + tx;
     if (t.d0 + d < D) dst[(size_t)d * j.R * n1p + p] = tile[p][d];
   }
 }
 
-__global__ void unpack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
+template <int PX>
+__global__ void __launch_bounds__(256) unpack_kernel(const __grid_constant__ PatchJobs jobs, int N1, int n1p) {
   follow_previous_kernel();
-  __shared__ uint32_t tile[PACK_PX][33];
+  __shared__ uint32_t tile[PX][33];
   int ji;
-  const Patch t = patch_of(jobs, n1p, ji);
+  const Patch t = patch_of<PX>(jobs, n1p, ji);
   const PatchJob& j = jobs.j[ji];
   const int tx = threadIdx.x, ty = threadIdx.y, D = j.D;
   const uint32_t* src = reinterpret_cast<const uint32_t*>(j.packed) + (((size_t)t.b * D + t.d0) * j.R + j.r0 + t.k) * n1p + t.p0;
 #pragma unroll
-  for (int i = ty; i < 32 * (PACK_PX / 32); i += 8) {
-    const int d = i / (PACK_PX / 32), p = (i % (PACK_PX / 32)) * 32 + tx;
+  for (int i = ty; i < 32 * (PX / 32); i += 8) {
+    const int d = i / (PX / 32), p = (i % (PX / 32)) * 32 + tx;
     tile[p][d] = t.d0 + d < D ? __ldg(src + (size_t)d * j.R * n1p + p) : 0u;
   }
   __syncthreads();
   uint32_t* dst = static_cast<uint32_t*>(const_cast<void*>(j.pixels)) + (((size_t)t.b * N1 + t.p0) * j.Kpix + j.k0 + t.k) * D + t.d0 + tx;
 #pragma unroll
-  for (int i = ty; i < PACK_PX; i += 8)
+  for (int i = ty; i < PX; i += 8)
     if (t.p0 + i < N1 && t.d0 + tx < D) dst[(size_t)i * j.Kpix * D] = tile[i][tx];
 }
 
 template <class Kernel>
-static cudaError_t launch_patches(Kernel kern, const PatchJob* job, int count, int B, int N1, int n1p, cudaStream_t stream) {
-  if (count < 1 || count > MAX_PATCH_JOBS) return cudaErrorInvalidValue;
+static cudaError_t launch_patches(Kernel kern, int px, const PatchJob* job, int count, int B, int N1, int n1p, cudaStream_t stream) {
   PatchJobs jobs;
   long long blocks = 0;
   for (int i = 0; i < MAX_PATCH_JOBS; ++i) {
     jobs.j[i] = job[i < count ? i : 0];
     jobs.first[i] = i < count ? (int)blocks : INT_MAX;
-    if (i < count) blocks += (long long)((job[i].D + 31) / 32) * (n1p / PACK_PX) * B * job[i].K;
+    if (i < count) blocks += (long long)((job[i].D + 31) / 32) * (n1p / px) * B * job[i].K;
     if (blocks > INT_MAX) return cudaErrorInvalidConfiguration;
   }
   launch_next(kern, (unsigned)blocks, dim3(32, 8), 0, stream, jobs, N1, n1p);
   return cudaGetLastError();
 }
+static bool short_patches(const PatchJob* job, int count, int B, int n1p) {
+  long long blocks = 0;   // of 128 pixels
+  for (int i = 0; i < count; ++i) blocks += (long long)((job[i].D + 31) / 32) * (n1p / 128) * B * job[i].K;
+  return blocks < 4 * SM_COUNT;
+}
 cudaError_t launch_pack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream) {
-  return launch_patches(pack_kernel, jobs, count, B, N1, n1p, stream);
+  if (count < 1 || count > MAX_PATCH_JOBS) return cudaErrorInvalidValue;
+  if (short_patches(jobs, count, B, n1p)) return launch_patches(pack_kernel<32>, 32, jobs, count, B, N1, n1p, stream);
+  return launch_patches(pack_kernel<128>, 128, jobs, count, B, N1, n1p, stream);
 }
 cudaError_t launch_unpack(const PatchJob* jobs, int count, int B, int N1, int n1p, cudaStream_t stream) {
-  return launch_patches(unpack_kernel, jobs, count, B, N1, n1p, stream);
+  if (count < 1 || count > MAX_PATCH_JOBS) return cudaErrorInvalidValue;
+  if (short_patches(jobs, count, B, n1p)) return launch_patches(unpack_kernel<32>, 32, jobs, count, B, N1, n1p, stream);
+  return launch_patches(unpack_kernel<128>, 128, jobs, count, B, N1, n1p, stream);
 }
 
 // Interleaved pack of groups of four slots: every block transposes a 32-pixel x 32-displacement patch of each of a group's sources through

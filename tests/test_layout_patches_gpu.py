@@ -1,0 +1,29 @@
+"""The transposes between the reference's layout and the library's, in patches of 32 pixels (small launches) and of 128: a batch
+whose tensors take the long ones against its samples alone, which take the short ones."""
+import pytest
+import torch
+
+from separableflowthesis_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H1,W1", [(9, 14), (8, 16), (11, 3), (25, 31)])
+@pytest.mark.parametrize("H2,W2", [(31, 33), (32, 64), (65, 5)])
+def test_batch_and_its_samples(H1, W1, H2, W2, cuda_device):
+    K = 3
+    # patches of 128 pixels x 32 displacements: at least four per SM in the batch, fewer in a sample
+    per_sample = -(-H1 * W1 // 128) * (-(-H2 // 32) + -(-W2 // 32)) * 2
+    assert per_sample * K < 4 * 148
+    B = -(-4 * 148 // per_sample)
+    g = torch.Generator(device=cuda_device).manual_seed(H1 * W2)
+    randn = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
+    F1, F2 = randn(B, H1, W1, 16), randn(B, H2, W2, 16)
+    a_u, a_v = randn(B, H1, W1, K, W2).softmax(-1), randn(B, H1, W1, K, H2).softmax(-1)
+    with ops.sweep_operands("bf16"):   # no scales, which are of a call's whole tensors
+        batch = [*ops.max_argmax_avg_forward(F1, F2), *ops.compression_forward(F1, F2, a_u, a_v)]
+        for b in {0, B // 2, B - 1}:
+            f1, f2, w_u, w_v = [t[b:b + 1].clone() for t in (F1, F2, a_u, a_v)]
+            alone = [*ops.max_argmax_avg_forward(f1, f2), *ops.compression_forward(f1, f2, w_u, w_v)]
+            for x, y in zip(batch, alone):
+                assert torch.equal(x[b:b + 1], y)
