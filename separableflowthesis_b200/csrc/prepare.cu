@@ -841,39 +841,47 @@ cudaError_t launch_channel_major_cf(const MapCopy* copy, int count, int B, int C
 //   blocked = 0: dst (B, C, pitch), pixel index = row*width + x (image 1: rows = 1, width = N1, pitch = n1p)
 //   blocked = 1: dst (B, C, ceil(width/16), pitch, 16): columns in blocks of 16, so that the 4 rows x 16 columns of one
 //                K block of the image-1-major GEMM are 64 consecutive values (image 2: pitch = H2 rounded up to 4)
-// Padding is zero.  32 x 32 tiles through shared memory, both images in one launch; grid (sum over the images of tiles of their padded
-// rows, ceil(C/32), B), block (32, 8).
+// Padding is zero.  Tiles of CMK_PX pixels x 32 channels through shared memory, both images in one launch; grid (sum over the images of tiles of
+// their padded rows, ceil(C/32), B), block (32, 8).  A thread has eight
+// loads under way and stores two pixels at once; with tiles of 32 pixels, one to a store, the drop-in operators took 348 us instead of 346 at
+// 2 x 48 x 64, 3024 instead of 2978 at 8 x 47 x 156 (BF16) and 5767 instead of 5692 at 1 x 135 x 240.
 __host__ __device__ inline int map_copy_columns(const MapCopy& c) { return c.blocked ? (c.width + 15) / 16 * 16 : c.pitch; }   // of a padded row
 __host__ __device__ inline int map_copy_rows(const MapCopy& c) { return c.blocked ? c.pitch : 1; }
+constexpr int CMK_PX = 64;
 template <typename T>
-__global__ void channel_major_kernel(const MapCopy c1, const MapCopy c2, int blocks1, int C, int op16) {
+__global__ void __launch_bounds__(256) channel_major_kernel(const MapCopy c1, const MapCopy c2, int blocks1, int C, int op16) {
   follow_previous_kernel();
-  __shared__ float tile[32][33];
+  __shared__ float tile[CMK_PX][33];
   const bool first = (int)blockIdx.x < blocks1;
   const MapCopy& c = first ? c1 : c2;
   const float sc16 = (op16 == OP16_FP16 && c.scale16 != nullptr) ? __ldg(c.scale16) : 1.f;
-  const int columns = map_copy_columns(c), per_row = (columns + 31) / 32, r = blockIdx.x - (first ? 0 : blocks1);
-  const int row = r / per_row, x0 = (r - row * per_row) * 32, c0 = blockIdx.y * 32, b = blockIdx.z;
+  const int columns = map_copy_columns(c), per_row = (columns + CMK_PX - 1) / CMK_PX, r = blockIdx.x - (first ? 0 : blocks1);
+  const int row = r / per_row, x0 = (r - row * per_row) * CMK_PX, c0 = blockIdx.y * 32, b = blockIdx.z;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const float* src = c.src + (((size_t)b * c.rows + row) * c.width + x0) * C + c0 + tx;
 #pragma unroll
-  for (int j = ty; j < 32; j += 8) tile[j][tx] = (row < c.rows && x0 + j < c.width && c0 + tx < C) ? __ldg(src + (size_t)j * C) : 0.f;
+  for (int j = ty; j < CMK_PX; j += 8) tile[j][tx] = (row < c.rows && x0 + j < c.width && c0 + tx < C) ? __ldg(src + (size_t)j * C) : 0.f;
   __syncthreads();
   const size_t per_channel = (size_t)map_copy_rows(c) * columns;
-  const int x = x0 + tx;
+  const int x = x0 + 2 * tx;   // and x + 1, next to it: columns and blocks of them are even
+  if (x >= columns) return;
   const size_t off = c.blocked ? ((size_t)(x >> 4) * c.pitch + row) * 16 + (x & 15) : (size_t)x;
   T* dst = static_cast<T*>(c.dst) + ((size_t)b * C + c0) * per_channel + off;
 #pragma unroll
   for (int j = ty; j < 32; j += 8) {
-    if (c0 + j < C && x < columns) {
-      if constexpr (sizeof(T) == 2) dst[(size_t)j * per_channel] = to_op16(tile[tx][j] * sc16, op16);
-      else dst[(size_t)j * per_channel] = tile[tx][j];
+    if (c0 + j >= C) return;
+    const float lo = tile[2 * tx][j], hi = tile[2 * tx + 1][j];
+    T* const at = dst + (size_t)j * per_channel;
+    if constexpr (sizeof(T) == 2) {
+      *reinterpret_cast<uint32_t*>(at) = op16 == OP16_FP16 ? pack_fp16x2(lo * sc16, hi * sc16) : pack_bf16x2(lo * sc16, hi * sc16);
+    } else {
+      *reinterpret_cast<float2*>(at) = make_float2(lo, hi);
     }
   }
 }
 
 cudaError_t launch_channel_major(const MapCopy& c1, const MapCopy& c2, int B, int C, int op16, cudaStream_t stream) {
-  auto blocks = [](const MapCopy& c) { return (map_copy_columns(c) + 31) / 32 * map_copy_rows(c); };
+  auto blocks = [](const MapCopy& c) { return (map_copy_columns(c) + CMK_PX - 1) / CMK_PX * map_copy_rows(c); };
   const dim3 grid(blocks(c1) + blocks(c2), (C + 31) / 32, B), block(32, 8);
   if (op16) launch_next(channel_major_kernel<uint16_t>, grid, block, 0, stream, c1, c2, blocks(c1), C, op16);
   else launch_next(channel_major_kernel<float>, grid, block, 0, stream, c1, c2, blocks(c1), C, 0);
