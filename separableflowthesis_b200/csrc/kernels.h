@@ -34,18 +34,28 @@ struct DeviceOnce {
 // channels 1 x 48 x 64 47.2 -> 40.0 us, inference 1 x 55 x 128 with four levels 262 -> 239, 4 x 55 x 128 697 -> 687, the drop-in operators of a
 // training step 2 x 48 x 64 409 -> 384, twelve lookups 4 x 55 x 128 135 -> 114.
 template <class... Params, class... Args>
-void launch_next(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Args&&... args) {
-  cudaLaunchAttribute early{};
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
+void launch_with(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = shared_bytes;
   config.stream = stream;
-  config.attrs = &early;
-  config.numAttrs = 1;
+  config.attrs = &attribute;
+  config.numAttrs = early ? 1 : 0;
   (void)cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+template <class... Params, class... Args>
+void launch_next(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Args&&... args) {
+  launch_with(true, kernel, grid, block, shared_bytes, stream, std::forward<Args>(args)...);
+}
+// The same when the device is empty again: for few long blocks behind a kernel that holds the SMs unevenly, which would come to lie two to an SM
+// while others have none.
+template <class... Params, class... Args>
+void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Args&&... args) {
+  launch_with(false, kernel, grid, block, shared_bytes, stream, std::forward<Args>(args)...);
 }
 
 // Problem size of one op call (one pyramid level).  N1 = H1*W1 image-1 pixels, N2 = H2*W2.
