@@ -180,18 +180,20 @@ __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t 
                "r"(smem_u32(src)), "r"(bytes)
                : "memory");
 }
-// A box of a tensor map stored, or added (FP32), from shared memory; what lies outside the tensor is left out.  A bulk group of its own.
+// A box of a tensor map stored, or added (FP32), from shared memory; what lies outside the tensor is left out.  Belongs to the bulk group that the
+// thread commits next.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* tm, const void* src, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n\tcp.async.bulk.commit_group;" ::"l"(tm),
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(tm),
                "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
 __device__ __forceinline__ void tma_add_4d(const CUtensorMap* tm, const void* src, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n\tcp.async.bulk.commit_group;" ::
-                   "l"(tm),
+  asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(tm),
                "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
+// This thread's copies since its last group are one; without any, a group that is complete at once.
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Until all but the last N of this thread's bulk groups have read their shared memory / are complete.
 template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 template <int N> __device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }

@@ -531,7 +531,9 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
   const int row0 = SPLIT ? e.wg * T::RW : 0;
   // TMA_ROWS: a tile's row sums go to one of the warp's two buffers, from where a TMA store (first column block, and every one of a later
   // piece) or add takes them to memory.  A buffer is used again, and a row added to again, when the copies of two tiles ago are complete
-  // (of one row block: of the tile before), so the sums of a row are added up in the order of its column blocks.  With red.global from the
+  // (of one row block: of the tile before), so the sums of a row are added up in the order of its column blocks.  Every tile is a bulk group,
+  // also one of which a group of warps has no row (SPLIT, 1 to 4 rows in the last block): without it the wait for all groups but the last
+  // would leave the one of two tiles ago under way.  With red.global from the
   // registers the sixteen of a warp and tile, their 64-bit addresses and conditions took an eighth of the launch (135 x 240, one pair, four
   // levels and channels 965 -> 860 us, 4 x 55 x 128 228 -> 203; 8 x 47 x 156, one level, two channels, both sweeps 514 -> 487).
   const int warp = e.wg * 4 + (e.p - e.lane - sc.m0) / 32;
@@ -622,11 +624,12 @@ __device__ void epilogue_compress(SweepSmem& sm, const SweepArgs& a, const Sweep
       if constexpr (TMA_ROWS) {
         fence_proxy_async_smem();
         __syncwarp();
-        if (e.lane == 0 && e.valid && nu > 0) {
+        if (e.lane == 0 && (!SPLIT || nu > 0) && e.valid) {
           if (later_piece) tma_store_4d(&maps->part, to_rows, e.p - sc.m0, u0, k_first, sc.tail * a.parts + vb - sc.part_vb0);
           else if (first) tma_store_4d(&maps->out, to_rows, e.p, u0, k, sc.b);
           else tma_add_4d(&maps->out, to_rows, e.p, u0, k, sc.b);
         }
+        bulk_commit();   // in every tile: the wait above counts groups (by all lanes: in lane 0's branch the 135 x 240 launch takes 866 us, not 860)
       }
     }
     float cv[CPT][VT];
