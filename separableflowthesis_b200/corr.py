@@ -181,8 +181,9 @@ class AlternateCorrBlockSepflow:
 
 
 def _transforms_active() -> bool:
-    """Whether torch.func transforms or forward-mode derivatives are: those are for the autograd Function to see (and to refuse)."""
-    return torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+    """Whether torch.func transforms, forward-mode derivatives or a trace are: those are for the autograd Function to see (transforms and
+    derivatives to refuse, a trace to record: of a call past it, it would record the allocation of the outputs alone)."""
+    return torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch.jit.is_tracing()
 
 
 class CorrBlock1D:

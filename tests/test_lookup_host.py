@@ -59,6 +59,28 @@ def test_transforms_and_forward_mode_reach_the_function(block):
     assert entered
 
 
+def test_traces_reach_the_function(block):
+    """A trace would record a direct call as the allocation of its outputs, without the lookup."""
+    coords = torch.zeros(1, 2, 4, 5)
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda c: block(c), (coords,), check_trace=False)
+        assert "LookupPairFunction" in str(traced.graph)
+        out1, out2 = traced(coords)
+    assert torch.equal(out1, torch.zeros_like(out1)) and torch.equal(out2, torch.ones_like(out2))
+
+
+@pytest.mark.gpu
+def test_a_trace_looks_up(cuda_device):
+    g = torch.Generator().manual_seed(1)
+    v1, v2 = torch.randn(1, 1, 24, 16, 24, generator=g).to(cuda_device), torch.randn(1, 1, 16, 16, 24, generator=g).to(cuda_device)
+    first, then = (torch.rand(1, 2, 16, 24, generator=g).to(cuda_device) * 10 for _ in range(2))
+    lookup = sfb.CorrBlock1D(v1, v2, num_levels=2, radius=2)
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda c: lookup(c), (first,), check_trace=False)
+        for got, want in zip(traced(then), lookup(then)):
+            assert torch.equal(got, want)
+
+
 def test_cpu_tensors_are_refused():
     v1, v2, coords = torch.zeros(1, 1, 16, 16, 16), torch.zeros(1, 1, 16, 16, 16), torch.zeros(1, 2, 16, 16)
     with pytest.raises(RuntimeError, match="CUDA"):
