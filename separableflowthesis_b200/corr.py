@@ -182,8 +182,12 @@ class AlternateCorrBlockSepflow:
 
 def _transforms_active() -> bool:
     """Whether torch.func transforms, forward-mode derivatives or a trace are: those are for the autograd Function to see (transforms and
-    derivatives to refuse, a trace to record: of a call past it, it would record the allocation of the outputs alone)."""
-    return torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch.jit.is_tracing()
+    derivatives to refuse, a trace to record: of a call past it, it would record the allocation of the outputs alone).  The first two
+    have no public switch; a torch without these names counts as active."""
+    try:
+        return torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch.jit.is_tracing()
+    except AttributeError:
+        return True
 
 
 class CorrBlock1D:

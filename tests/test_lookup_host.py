@@ -59,6 +59,13 @@ def test_transforms_and_forward_mode_reach_the_function(block):
     assert entered
 
 
+@pytest.mark.parametrize("owner, name", [(torch._C, "_are_functorch_transforms_active"), (torch.autograd.forward_ad, "_current_level")])
+def test_a_torch_without_the_switches_counts_as_active(monkeypatch, owner, name):
+    assert not corr._transforms_active()
+    monkeypatch.delattr(owner, name)
+    assert corr._transforms_active()
+
+
 def test_traces_reach_the_function(block):
     """A trace would record a direct call as the allocation of its outputs, without the lookup."""
     coords = torch.zeros(1, 2, 4, 5)
