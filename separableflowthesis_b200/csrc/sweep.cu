@@ -1001,7 +1001,6 @@ static cudaError_t launch_one(SweepLaunch<LEVELS>& launch, int levels, cudaStrea
   }
   launch.first_block[LEVELS] = blocks;
   launch.first_tail[LEVELS] = tails;
-  // kern<<<blocks, SW_THREADS, SW_SMEM_BYTES, stream>>>(launch, status), early
   launch_next(kern, blocks, SW_THREADS, SW_SMEM_BYTES, stream, launch, launch.a[0].status);
   if constexpr (CUT) {
     if (tails == 0) return cudaGetLastError();

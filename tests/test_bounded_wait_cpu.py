@@ -34,13 +34,14 @@ def test_a_cta_leaves_early_as_a_whole():
 def test_a_register_split_is_checked_against_the_compiled_kernel():
     """setmaxnreg.inc waits for registers of the CTA's launch; a kernel compiled for fewer than the split adds up to must be
     refused by the host."""
-    sources = [open(os.path.join(build.CSRC, name)).read() for name in build.SOURCES]
+    sources = [re.sub(r"//.*", "", open(os.path.join(build.CSRC, name)).read()) for name in build.SOURCES]
     split = [text for text in sources if "set_max_registers<" in text]
     assert len(split) == 1
     host = split[0][split[0].index("static cudaError_t launch_one("):]
     host = host[:host.index("\n}")]
-    order = [host.index(s) for s in ("cudaFuncGetAttributes(&built, kern)", "register_split_fits(built.numRegs)", "kern<<<")]
+    order = [host.index(s) for s in ("cudaFuncGetAttributes(&built, kern)", "register_split_fits(built.numRegs)", "launch_next(kern,")]
     assert order == sorted(order)
+    assert len(re.findall(r"launch_\w+\(kern\b", split[0])) == 1 and host.count("auto kern = sweep_kernel<") == split[0].count("= sweep_kernel<") == 1
 
 
 def test_a_cta_that_gives_up_lets_its_copies_land():
