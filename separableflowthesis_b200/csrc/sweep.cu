@@ -63,10 +63,10 @@ constexpr uint32_t SW_STAGE_BYTES = SW_TILE_N * KBLK * 4;
 constexpr uint32_t SW_F1_BLOCK_BYTES = TILE_M * KBLK * 4;
 constexpr uint32_t SW_TMEM_COLS = 512;
 // Image-2 blocks (32 KB) in flight: what the resident image-1 tile leaves.  128 KB of it (TF32, 256 channels) leave three,
-// 64 KB (16-bit) five.
+// 64 KB (16-bit) five, and four beside the 8 to 32 KB of row sums on their way to memory (compression, TMA rows).
 constexpr int SW_MAX_STAGES = 6;
 constexpr uint32_t SW_RING_BYTES = MAX_KB * SW_F1_BLOCK_BYTES + 3 * SW_STAGE_BYTES;   // image-1 tile and ring together
-__device__ __forceinline__ uint32_t sw_stages(int nkb, uint32_t row_bytes) {
+__host__ __device__ constexpr uint32_t sw_stages(int nkb, uint32_t row_bytes) {
   const uint32_t n = (SW_RING_BYTES - row_bytes - nkb * SW_F1_BLOCK_BYTES) / SW_STAGE_BYTES;
   return n < SW_MAX_STAGES ? n : SW_MAX_STAGES;
 }
@@ -75,6 +75,7 @@ __device__ __forceinline__ uint32_t sw_stages(int nkb, uint32_t row_bytes) {
 __host__ __device__ constexpr int sw_channels(int KC) { return KC == 1 ? 1 : 2; }           // of a thread
 __host__ __device__ constexpr int sw_rows(int KC) { return KC <= 2 ? SWEEP_UT / 2 : SWEEP_UT; }   // with one or two channels the two groups share a tile's rows
 __host__ __device__ constexpr uint32_t sw_row_bytes(int KC) { return 2 * SW_EPI_WARPS * sw_rows(KC) * sw_channels(KC) * 32 * sizeof(float); }
+static_assert(sw_stages((MAX_KB + 1) / 2, sw_row_bytes(4)) >= 3 && sw_row_bytes(4) >= sw_row_bytes(2), "image-2 blocks in flight beside the row sums");
 static_assert(SW_NACC * SW_TILE_N <= 512, "accumulators exceed TMEM");
 static_assert(SW_NMERGE > SW_NACC, "a warpgroup can run SW_NACC tiles ahead of the other");
 
