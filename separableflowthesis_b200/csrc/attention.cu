@@ -1064,6 +1064,7 @@ attention_input_grad_tiled_kernel(const __grid_constant__ TileMaps maps, const _
 // TMA loads are issued by a warp of their own; copies by all warps, which then meet at a barrier per plane as in PlaneFeed.
 // grid (ceil(W1/32) * ceil(H1/8) * B * pieces blocks per job, chunks of KW channels), block wg_threads(FEED); partial: of the module,
 // (Kc * 2 * 27, rows).
+constexpr int WG_PER_SM = 3;   // blocks on an SM, by the launch bounds; the number by which walks are cut, whose partial sums size the workspace
 constexpr int WG_GROUPS = 2, WG_WARPS = 2 * WG_GROUPS, WG_ROWS = 4, WG_TILE_ROWS = WG_GROUPS * WG_ROWS, WG_MAX_CHANNELS = 2;
 constexpr int wg_channels(int Kc) { return Kc < WG_MAX_CHANNELS ? Kc : WG_MAX_CHANNELS; }   // of a thread
 template <int KW>
@@ -1082,7 +1083,7 @@ struct WeightGradTileSmem {
 
 __host__ __device__ constexpr int wg_threads(int feed) { return WG_WARPS * 32 + (feed == FEED_TMA ? 32 : 0); }
 template <int KW, int FEED>
-__global__ void __launch_bounds__(wg_threads(FEED), 3)
+__global__ void __launch_bounds__(wg_threads(FEED), WG_PER_SM)
 attention_weight_grad_tiled_kernel(const __grid_constant__ TileMaps maps_x, const __grid_constant__ TileMaps maps_gl,
                                    const __grid_constant__ WeightGradJobs jobs, int Kc, int B, int H1, int W1, int* status) {
   if (!cta_has_work(status)) return;
@@ -1337,9 +1338,8 @@ static int tiled_walk(size_t blocks, const int* D, int n, int slots, double extr
   }
   return walk;
 }
-// Blocks on an SM of the tiled kernels (registers), and what a piece costs beside its planes.
+// What a piece costs beside its planes.
 constexpr double AT_PIECE_EXTRA = 3.0, WG_PIECE_EXTRA = 8.0;
-constexpr int WG_SLOTS = 3 * SM_COUNT;
 // Displacements per block of the weight gradients' walks, and the blocks of a job (partial sums of a weight).
 struct WeightWalks {
   int dc[MAX_ATTENTION_JOBS];
@@ -1351,7 +1351,7 @@ static WeightWalks weight_walks(const AttentionDims* d, int count, bool tiled) {
   for (int i = 0; i < count; ++i) total += D[i] = d[i].D;
   const size_t blocks = tiled ? tile_count(d[0], WG_TILE_ROWS) * d[0].B : form_blocks(d[0], false);
   const int chunks = (d[0].Kc + wg_channels(d[0].Kc) - 1) / wg_channels(d[0].Kc);
-  const int walk = tiled ? tiled_walk(blocks * chunks, D, count, WG_SLOTS, WG_PIECE_EXTRA) : 0;
+  const int walk = tiled ? tiled_walk(blocks * chunks, D, count, WG_PER_SM * SM_COUNT, WG_PIECE_EXTRA) : 0;
   for (int i = 0; i < count; ++i) {
     r.dc[i] = tiled ? even_walk(D[i], walk) : gather_walk(2 * blocks, D[i], total, WG_BLOCKS_TARGET, WG_MIN_WALK);
     r.rows[i] = blocks * ((D[i] + r.dc[i] - 1) / r.dc[i]);
@@ -1444,22 +1444,6 @@ static Walks stencil_walks(const Job* job, int count, bool tiled, int blocks_per
   }
   return r;
 }
-// The order of a launch's jobs: the longest pieces first, so that the short ones fill the end.
-static void by_length(const Walks& walks, int count, int* order) {
-  for (int i = 0; i < count; ++i) {
-    int at = i;
-    for (; at > 0 && walks.dc[order[at - 1]] < walks.dc[i]; --at) order[at] = order[at - 1];
-    order[at] = i;
-  }
-}
-// Blocks of the tiled walks on an SM (registers).
-static int logits_per_sm(int Kc) { return Kc >= 3 ? 4 : 6; }
-static int input_grad_per_sm(int Kc) { return Kc >= 3 ? 3 : 5; }
-static bool logits_by_tma(const AttentionJob* job, int count) {
-  bool tma = true;
-  for (int i = 0; i < count; ++i) tma = tma && tileable(job[i].d, job[i].x, job[i].x_sb);
-  return tma;
-}
 // f(integral constant) of a number of channels
 template <class F>
 static void by_channels(int kc, F&& f) {
@@ -1469,9 +1453,58 @@ static void by_channels(int kc, F&& f) {
   else f(std::integral_constant<int, 4>{});
 }
 
+// Blocks on an SM of a tiled kernel (AT_THREADS threads, static shared memory), as it was compiled: 3 to 5 of the forms that copy, 3 to 8 of those by
+// TMA.  Written down as 4 or 6 (logits, three channels and more, or fewer) and 3 or 5 (input gradients) for both forms, where a round of the
+// slots was none: logits 1 x 135 x 241, one level, four channels (3 on an SM) 205 -> 163 us, 1 x 55 x 127, two channels (4) 17.0 -> 14.3; input
+// gradients 4 x 55 x 128, four levels, three channels (4) 129 -> 95.  104 sizes, one and four levels, one to four channels: 2.7 % less for
+// either kernel; up to a tenth more where rounds of fewer blocks happened to fit (4 x 55 x 128, one level, three channels: logits 49 -> 54).
+// Asked once per kernel and device.
+template <auto KERNEL>
+static int blocks_per_sm() {
+  static std::atomic<int> known[AT_MAX_DEVICES];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= AT_MAX_DEVICES) return 1;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n == 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, AT_THREADS, 0) == cudaSuccess)
+    known[dev].store(n, std::memory_order_relaxed);
+  return std::max(n, 1);
+}
+// The order of a launch's jobs: the longest pieces first, so that the short ones fill the end.
+static void by_length(const Walks& walks, int count, int* order) {
+  for (int i = 0; i < count; ++i) {
+    int at = i;
+    for (; at > 0 && walks.dc[order[at - 1]] < walks.dc[i]; --at) order[at] = order[at - 1];
+    order[at] = i;
+  }
+}
+static bool logits_by_tma(const AttentionJob* job, int count) {
+  bool tma = true;
+  for (int i = 0; i < count; ++i) tma = tma && tileable(job[i].d, job[i].x, job[i].x_sb);
+  return tma;
+}
+static Walks logits_walks(const AttentionJob* job, int count, bool tiled, bool tma) {
+  int per_sm = 0;
+  if (tiled)
+    by_channels(std::min(job[0].d.Kc, AT_KC), [&](auto c) {
+      constexpr int KC = decltype(c)::value;
+      per_sm = tma ? blocks_per_sm<attention_logits_tiled_kernel<KC, false, FEED_TMA>>()
+                   : blocks_per_sm<attention_logits_tiled_kernel<KC, false, FEED_COPIES>>();
+    });
+  return stencil_walks(job, count, tiled, per_sm, true);
+}
+static Walks input_grad_walks(const AttentionGradJob* job, int count, bool tiled, bool tma) {
+  int per_sm = 0;
+  if (tiled)
+    by_channels(std::min(job[0].d.Kc, AT_KC), [&](auto c) {
+      constexpr int KC = decltype(c)::value;
+      per_sm = tma ? blocks_per_sm<attention_input_grad_tiled_kernel<KC, FEED_TMA>>() : blocks_per_sm<attention_input_grad_tiled_kernel<KC, FEED_COPIES>>();
+    });
+  return stencil_walks(job, count, tiled, per_sm, false);
+}
+
 int attention_forward_launches(const AttentionJob* job, int count, const int* status) {
   int n = 2 * ((job[0].d.Kc + AT_KC - 1) / AT_KC);   // the weights' staging and the walks per chunk of channels
-  if (stencil_walks(job, count, status != nullptr, logits_per_sm(job[0].d.Kc), true).soft) return n;
+  if (logits_walks(job, count, status != nullptr, status != nullptr && logits_by_tma(job, count)).soft) return n;
   for (int i = 0; i < count; ++i) {
     bool first = true;   // of its class of lengths
     for (int k = 0; k < i; ++k) first = first && softmax_class(job[k].d.D) != softmax_class(job[i].d.D);
@@ -1484,7 +1517,7 @@ cudaError_t launch_attention_forward(const AttentionJob* job, int count, const A
   if (count < 1 || count > MAX_ATTENTION_JOBS) return cudaErrorInvalidValue;
   const AttentionDims& d = job[0].d;
   const bool tiled = status != nullptr, tma = tiled && logits_by_tma(job, count);
-  const Walks walks = stencil_walks(job, count, tiled, logits_per_sm(d.Kc), true);
+  const Walks walks = logits_walks(job, count, tiled, tma);
   const bool soft = walks.soft;
   int order[MAX_ATTENTION_JOBS];
   by_length(walks, count, order);
@@ -1642,7 +1675,7 @@ cudaError_t launch_attention_backward(const AttentionGradJob* job, int count, co
   cudaError_t err = launch_logit_grad(job, place, count, st);
   if (err != cudaSuccess) return err;
   {
-    const Walks walks = stencil_walks(job, count, tiled, input_grad_per_sm(d.Kc), false);
+    const Walks walks = input_grad_walks(job, count, tiled, tma);
     int order[MAX_ATTENTION_JOBS];
     by_length(walks, count, order);
     InputGradJobs jobs{};
