@@ -289,11 +289,14 @@ constexpr int L4_BPX = L4_BT * L4_BT;
 constexpr int L4_BCH = 256;                      // channels of a CTA, two a lane
 constexpr int L4_BBOX = 384;                    // positions of the largest box walked for the whole tile
 constexpr int L4_BTHREADS = 128, L4_BWARPS = L4_BTHREADS / 32;
-// Largest box of a tile for windows of a radius.  A level of a whole tile took 1.2 us per position plus 35 (a tenth less since), where four walks of 2 x 2 pixels take
-// 0.85 (2 x 55 x 128, C = 256); those have (2r + 3)^2 positions each in a smooth field and (2r + 4)^2 or more where the tile's box is near the
-// limit: radius 4 382, 3 256, 2 153.  With (2r + 3)^2 a field with noise of half a pixel took 337 us at radius 3, 2 x 2 pixels alone 299, 220 with
-// this.  Radius 1 and 0 walk 2 x 2 pixels only.
-inline int l4_tile_limit(int radius) { return radius < 2 ? 0 : std::min(L4_BBOX, (4 * (2 * radius + 4) * (2 * radius + 4) - 41) * 5 / 7); }
+// Largest box of a tile for windows of a radius: what the table holds.  One level of 2 x 55 x 128 pixels at C = 256 takes 0.48 us per position plus
+// 40 as whole tiles, 0.9 per position of a 2 x 2 pixels' box plus 34 as four walks of those, so a uniform spread would draw the line at boxes of
+// 256 positions (radius 4), 155 (3) and 80 (2).  But a field's tiles differ, and those left apart are a second launch of few long blocks: both lie above
+// either alone.  Four levels, smooth motion with objects of another one: all tiles apart 325 us (radius 3) and 226 (2), with limits of 256 and 153
+// 380 and 262, with this 219 and 163; noise of 1, 1.5, 2 and 3 pixels, radius 2: 219, 239, 267, 306 apart, 255, 237, 303, 317 with 153,
+// 168, 181, 196, 360 with this.  (Blocks of 2 x 3 pixels with motions 4 apart, no two alike, lose: 282 -> 355 and 233 -> 265.)
+// Radius 1 and 0 walk 2 x 2 pixels only: whole tiles gain 5 % at C = 256 in a smooth field, and lose 15 at 128.
+inline int l4_tile_limit(int radius) { return radius < 2 ? 0 : L4_BBOX; }
 static_assert(2 * L4_BTHREADS <= L4_BBOX && L4_BBOX % 4 == 0, "partial sums of warps that share channels; steps of four positions");
 static_assert(L4_BCH == L4_BWARPS * 64, "a warp has 64 channels");
 

@@ -68,3 +68,10 @@ def test_infinity_reaches_its_windows_only(where, cuda_device):
             for x in range(W):
                 hit[y, x] = x + 2 <= 2 <= x + 7 and y + 2 <= 4 <= y + 7
         assert torch.isfinite(a2).all() and not torch.isfinite(a1[0, ..., 5][hit]).any() and torch.isfinite(a1[0, ..., 5][~hit]).all()
+
+
+# boxes on both sides of the table's 384 positions at smaller radii: (3 * step + 2r + 2)^2 and one more per side
+@pytest.mark.parametrize("C", [36, 256])
+@pytest.mark.parametrize("radius,step", [(3, 3), (3, 4), (2, 3), (2, 4), (2, 5)])
+def test_largest_boxes_of_smaller_radii(radius, step, C, cuda_device):
+    test_box_sizes(radius, step, C, cuda_device)
